@@ -1,0 +1,80 @@
+"""Shapes at the edges of the tensor-core kernels' tiles, through the public calls, against the CPU oracle: head widths
+that no tile has (padded to the next wider one), sequences shorter than a tile of query rows, and windows of a prompt
+at an offset.  Tolerance: the stated bar of this path, |got - ref| <= 1e-5 + 1e-4 |ref|, element-wise."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def close(got, ref, what):
+    got, ref = got.cpu().numpy().astype(np.float64), np.asarray(ref, np.float64)
+    assert got.shape == ref.shape, what
+    bad = ~(np.abs(got - ref) <= 1e-5 + 1e-4 * np.abs(ref))
+    assert not bad.any(), (what, int(bad.sum()), float(np.nanmax(np.abs(got - ref))))
+
+
+def normal(oracle, shape, stream):
+    return oracle.fill_normal(shape, 93, stream)
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D", [
+    (2, 33, 4, 2, 36), (1, 64, 3, 1, 40), (1, 1, 4, 2, 64), (2, 65, 4, 4, 60), (1, 2, 2, 1, 128), (1, 127, 4, 2, 68),
+    (2, 129, 6, 2, 80), (1, 32, 4, 1, 124), (1, 100, 4, 2, 132), (1, 63, 2, 2, 200), (1, 257, 2, 1, 252), (3, 31, 8, 2, 256),
+])
+def test_widths_and_short_sequences(zt, oracle, B, T, H, Hkv, D):
+    q, k, v, do = (normal(oracle, (B, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv, H)))
+    tq, tk, tv, tdo = (torch.from_numpy(x).cuda() for x in (q, k, v, do))
+    ws = zt.BackwardWorkspace(B, T, H, Hkv, D)
+    o, lse = zt.attention_forward(tq, tk, tv, H, Hkv, D, want_lse=True, keep=ws)
+    grads = zt.attention_backward(tq, tk, tv, o, lse, tdo, H, Hkv, D, workspace=ws, kept=ws.token != 0)
+    torch.cuda.synchronize()
+    assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+    for b in range(B):
+        ro, rl = oracle.attention_forward(q[b], k[b], v[b], H, Hkv, D, want_lse=True, threads=4)
+        ref = oracle.attention_backward(q[b], k[b], v[b], do[b], H, Hkv, D, threads=4)
+        for name, got, want in zip(("out", "lse", "dq", "dk", "dv"), (o, lse, *grads), (ro, rl, *ref)):
+            close(got[b], want, f"{name}[{b}]")
+
+
+@pytest.mark.parametrize("T,q_offset,ctx,H,Hkv,D", [
+    (33, 1, 40, 4, 2, 32), (64, 63, 127, 3, 1, 64), (128, 64, 192, 4, 1, 80), (200, 313, 600, 8, 2, 128),
+    (129, 511, 700, 6, 3, 96), (40, 0, 64, 2, 2, 192), (70, 250, 320, 4, 2, 256), (96, 1000, 1500, 32, 8, 128),
+    # many key tiles: the row sums leave the tensor core's accumulator every sixteen of them
+    (129, 2900, 3100, 2, 1, 128), (300, 2100, 2400, 4, 1, 64), (40, 1500, 1540, 2, 1, 256),
+])
+def test_windows_of_a_prompt(zt, oracle, T, q_offset, ctx, H, Hkv, D):
+    """device.Attn.forward_at: rows at q_offset over the first q_offset + T keys; what lies beyond is never read."""
+    q = normal(oracle, (T, H * D), 0)
+    n_keys = q_offset + T
+    k, v = (normal(oracle, (n_keys, Hkv * D), i) for i in (1, 2))
+    holder = zt.Attn(ctx, H, Hkv, D)
+    holder.k.fill_(float("nan")), holder.v.fill_(float("nan")), holder.q.zero_()
+    for name, x in (("q", q), ("k", k), ("v", v)):
+        holder.upload(getattr(holder, name), x)
+    holder.forward_at(1, 64, q_offset, n_keys, T)
+    torch.cuda.synchronize()
+    assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0
+    ref = oracle.attention_forward_at(q, k, v, H, Hkv, D, q_offset, n_keys)
+    got = holder.out[: q.size].view(q.shape)
+    close(got, ref, "window")
+    # the CUDA-core kernels served these calls with rounded f32 sums: as a whole no further off than they are
+    assert float(np.linalg.norm(got.cpu().numpy() - ref) / np.linalg.norm(ref)) <= 5e-6
+
+
+@pytest.mark.parametrize("T,H,Hkv,D,pos", [(70, 4, 2, 40, 3), (150, 2, 1, 136, 0), (90, 2, 2, 68, 5)])
+def test_rope_at_widths_between_the_tiles(zt, oracle, T, H, Hkv, D, pos):
+    """Halves that are multiples of four ride in the pre-pass; others are rotated before it."""
+    q, k, v, do = (normal(oracle, (1, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv, H)))
+    tq, tk, tv, tdo = (torch.from_numpy(x).cuda() for x in (q, k, v, do))
+    ws = zt.RopeWorkspace(1, T, H, Hkv, D)
+    o, lse = zt.attention_forward_rope(tq, tk, tv, H, Hkv, D, pos=pos, workspace=ws, want_lse=True)
+    dq, dk, dv = zt.attention_backward_rope(tq, tk, tv, o, lse, tdo, H, Hkv, D, pos=pos, workspace=ws, kept=ws.token != 0)
+    torch.cuda.synchronize()
+    assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0
+    qr, kr = oracle.rope_forward(q[0], pos, D), oracle.rope_forward(k[0], pos, D)
+    close(o[0], oracle.attention_forward(qr, kr, v[0], H, Hkv, D), "out")
+    rdq, rdk, rdv = oracle.attention_backward(qr, kr, v[0], do[0], H, Hkv, D)
+    for name, got, want in (("dq", dq, oracle.rope_backward(rdq, pos, D)), ("dk", dk, oracle.rope_backward(rdk, pos, D)), ("dv", dv, rdv)):
+        close(got[0], want, name)

@@ -73,6 +73,7 @@ struct PrepassTensor {
     uint32_t *amax;   // [batch][width / cols_per_group] bit patterns of max |x|, zeroed by the caller
     __half *planes;   // [2][batch][T][width / src_head * dst_head]
     int width, cols_per_group;
+    int rows;                // rows of x per sequence that are converted
     int src_head, dst_head;  // a head's columns in x and in the planes: 32 -> 64 pads each head with zeros
     const float2 *rope;      // null, or the (cos, sin) table [T][src_head / 2]: x is rotated on its way in
 };
@@ -95,7 +96,7 @@ __device__ __forceinline__ float4 prepass_load(const PrepassTensor &t, const flo
 }
 struct PrepassArgs {
     PrepassTensor t[4];
-    int n, batch, T;
+    int n, batch;
 };
 constexpr int kPrepassRows = 32;      // rows of one sequence per absmax CTA
 constexpr int kPrepassMaxGroups = 256;
@@ -109,8 +110,9 @@ __global__ void __launch_bounds__(256) bwd_absmax_kernel(const PrepassArgs a) {
     const int w4 = t.width / 4, n_groups = t.width / t.cols_per_group;
     for (int i = threadIdx.x; i < n_groups; i += 256) gmax[i] = 0u;
     __syncthreads();
-    const int r1 = min(r0 + kPrepassRows, a.T);
-    const float4 *base = reinterpret_cast<const float4 *>(t.x + (long long)b * a.T * t.width);
+    if (r0 >= t.rows) return;
+    const int r1 = min(r0 + kPrepassRows, t.rows);
+    const float4 *base = reinterpret_cast<const float4 *>(t.x + (long long)b * t.rows * t.width);
     for (int c4 = threadIdx.x; c4 < w4; c4 += 256) {
         float m = 0.f;
 #pragma unroll 8
@@ -137,10 +139,10 @@ __global__ void __launch_bounds__(256) bwd_split_kernel(const PrepassArgs a) {
     if (t.src_head != t.dst_head) {
         // zero-padded heads: walk the planes' float4s, fetch the source's where there is one
         const int w4s = t.width / 4, w4d = t.width / t.src_head * t.dst_head / 4;
-        const long long seq4d = (long long)a.T * w4d;
+        const long long seq4d = (long long)t.rows * w4d;
         const long long first = (long long)blockIdx.x * kSplitPerCta;
         if (first >= seq4d) return;
-        const float4 *src = reinterpret_cast<const float4 *>(t.x) + (long long)b * a.T * w4s;
+        const float4 *src = reinterpret_cast<const float4 *>(t.x) + (long long)b * t.rows * w4s;
         uint2 *hp = reinterpret_cast<uint2 *>(t.planes) + b * seq4d;
         uint2 *lp = hp + (long long)a.batch * seq4d;
         const uint32_t *amax = t.amax + b * n_groups;
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(256) bwd_split_kernel(const PrepassArgs a) {
         return;
     }
     const int w4 = t.width / 4;
-    const long long seq4 = (long long)a.T * w4;  // float4 per sequence
+    const long long seq4 = (long long)t.rows * w4;  // float4 per sequence
     const long long first = (long long)blockIdx.x * kSplitPerCta;
     if (first >= seq4) return;
     const float4 *src = reinterpret_cast<const float4 *>(t.x) + b * seq4;
@@ -200,16 +202,15 @@ __global__ void __launch_bounds__(256) bwd_split_kernel(const PrepassArgs a) {
 
 // Both passes for the tensors in `a` (amax already zeroed).
 inline int launch_prepass(const PrepassArgs &a, cudaStream_t stream) {
-    int wmax = 0, wmax_src = 0;
+    int rows = 0;
+    long long seq4 = 0;
     for (int i = 0; i < a.n; ++i) {
-        const int wd = a.t[i].width / a.t[i].src_head * a.t[i].dst_head;
-        wmax = wd > wmax ? wd : wmax;
-        wmax_src = a.t[i].width > wmax_src ? a.t[i].width : wmax_src;
+        const long long s4 = (long long)a.t[i].rows * (a.t[i].width / a.t[i].src_head * a.t[i].dst_head / 4);
+        seq4 = s4 > seq4 ? s4 : seq4;
+        rows = a.t[i].rows > rows ? a.t[i].rows : rows;
     }
-    (void)wmax_src;
-    const dim3 ga((unsigned)((a.T + kPrepassRows - 1) / kPrepassRows), (unsigned)a.batch, (unsigned)a.n);
+    const dim3 ga((unsigned)((rows + kPrepassRows - 1) / kPrepassRows), (unsigned)a.batch, (unsigned)a.n);
     if (ZT_LAUNCH("bwd_absmax_kernel", stream, (bwd_absmax_kernel<<<ga, 256, 0, stream>>>(a)))) return 1;
-    const long long seq4 = (long long)a.T * (wmax / 4);
     const dim3 gs((unsigned)((seq4 + kSplitPerCta - 1) / kSplitPerCta), (unsigned)a.batch, (unsigned)a.n);
     return ZT_LAUNCH("bwd_split_kernel", stream, (bwd_split_kernel<<<gs, 256, 0, stream>>>(a)));
 }
@@ -275,7 +276,7 @@ struct BwdParams {
     float *dq, *dk, *dv;
     PeerList dq_peers;       // dq is also stored here (same element index), see zt_common.cuh
     int batch, T, n_heads, n_kv_heads;
-    int dim_out;     // the tensors' head_dim: the tile's D, or 32 under a tile padded to 64
+    int dim_out;     // the tensors' head_dim, at most the tile's D
     const float2 *rope_t;  // null, or the (cos, sin) table transposed, [dim_out / 2][T]: dq leaves as R^T of what was computed
     float scale, scale_log2;
     float p_scale;  // P is multiplied by this power of two before its 16-bit split
@@ -753,7 +754,7 @@ __global__ void __launch_bounds__(kKvThreads, 1)
                         }
                     }
                 }
-                if (c0 + c < p.dim_out) {  // (a padded tile's upper columns are not the tensor's)
+                if (c0 + c + 4 * j8 < p.dim_out) {  // (a padded tile's upper columns are not the tensor's)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         if (key - j8 + i >= p.T) continue;
@@ -1280,7 +1281,7 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
 
 inline bool tc_bwd_supported(int batch, int T, int dim, const void *q, const void *k, const void *v,
                              const void *dout, const void *dq, const void *dk, const void *dv) {
-    if (!(dim == 32 || dim == 64 || dim == 96 || dim == 128) || T < 128 || batch < 1) return false;
+    if (!tc_takes_dim(dim) || dim > 128 || T < 1 || batch < 1) return false;
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(q) || !al(k) || !al(v) || !al(dout) || !al(dq) || !al(dk) || !al(dv)) return false;
     const DeviceInfo *d = device_info();
@@ -1310,12 +1311,6 @@ inline int launch_bwd_tc_d(const BwdMaps &m, const BwdParams &p, cudaStream_t st
 }
 
 }  // namespace tcb
-
-// head_dim 32 runs on the 64-wide tiles and head_dim 96 on the 128-wide ones: the planes carry every head
-// zero-padded to the tile's width (at 32 the MMAs would cost the same at half the width, see the clock floor
-// above; at 96 a quarter of the tensor work is padding), outputs keep their own width.  The kernels write
-// their outputs in 32-column (128-wide tiles) or 16/32-column (64-wide) pieces, which is why only these two.
-inline int tc_tile_dim(int dim) { return dim == 32 ? 64 : (dim == 96 ? 128 : (dim == 192 ? 256 : dim)); }
 
 inline size_t tc_bwd_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     return tcb::bwd_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).total_bytes;

@@ -1,4 +1,4 @@
-// The backward at head_dim 64 and 128 (and 32, 96 padded to them) as ONE tensor-core kernel: dK, dV and dQ from one
+// The backward at tile widths 64 and 128 (every head_dim up to 128, padded to them) as ONE tensor-core kernel: dK, dV and dQ from one
 // computation of S^T and dP^T.
 //
 // tc_bwd.cuh computes S and dP twice: once in the dK/dV kernel (a CTA per 128 keys, query tiles walked) and
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                         }
                     }
                 }
-                if (c0 + c < p.dim_out) {
+                if (c0 + c + 4 * j8 < p.dim_out) {  // (a padded tile's upper columns are not the tensor's)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         if (key - j8 + i >= p.T) continue;
@@ -631,7 +631,7 @@ inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &
 
 }  // namespace tcf
 
-// Which backward a head_dim-`dim` call takes: the fused kernel at tile widths 64 and 128 (head_dim 32 ... 128) unless the
+// Which backward a head_dim-`dim` call takes: the fused kernel at tile widths 64 and 128 (head_dim up to 128) unless the
 // two-kernel form is asked for (zt_attn_set_path(8)) or dq must also be stored into peers' memory (the fused
 // kernel adds partial sums into dq, which a plain peer store cannot follow).
 inline bool tc_bwd_takes_fused(int dim, bool two_kernels, const PeerList *dq_peers) {
@@ -665,13 +665,13 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
         return refuse("could not clear the backward workspace header");
     }
     PrepassArgs pa{};
-    pa.batch = batch, pa.T = T;
-    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, dim, td, nullptr};
+    pa.batch = batch;
+    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, T, dim, td, nullptr};
     pa.n = 1;
     if (!qkv_planes_kept) {
-        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, dim, td, rope};
-        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, dim, td, rope};
-        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, dim, td, nullptr};
+        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, rope};
+        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, T, dim, td, rope};
+        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, T, dim, td, nullptr};
         pa.n = 4;
     }
     if (launch_prepass(pa, stream)) return 1;

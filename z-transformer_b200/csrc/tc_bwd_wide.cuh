@@ -1,4 +1,4 @@
-// Causal GQA attention backward at head_dim 256 (and 192 zero-padded to it) on the tensor cores.
+// Causal GQA attention backward at head_dim 256 (and 132 ... 252 zero-padded to it) on the tensor cores.
 //
 // What it computes: autograd.attentionBackward (src/autograd.zig:636-842) for a batch, as tc_bwd.cuh does:
 //     P = exp(S - lse),  dP = dO V^T,  dS = P (dP - delta),  dV = P^T dO,  dK = scale dS^T Q,  dQ = scale dS K
@@ -822,7 +822,7 @@ inline WideWorkspace wide_workspace(void *ws, int batch, int T, int n_heads, int
 
 inline bool tc_bwd_wide_supported(int batch, int T, int n_heads, int n_kv_heads, int dim, const void *q, const void *k,
                                   const void *v, const void *dout, const void *dq, const void *dk, const void *dv) {
-    if (!(dim == 192 || dim == 256) || T < 128 || batch < 1) return false;
+    if (!tc_takes_dim(dim) || dim <= 128 || T < 1 || batch < 1) return false;
     if (wide_unit_cap(batch, T, n_heads, n_kv_heads) == 0) return false;
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(q) || !al(k) || !al(v) || !al(dout) || !al(dq) || !al(dk) || !al(dv)) return false;
@@ -864,13 +864,13 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         return refuse("could not clear the backward's outputs and workspace header");
     }
     PrepassArgs pa{};
-    pa.batch = batch, pa.T = T;
-    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, dim, td, nullptr};
+    pa.batch = batch;
+    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, T, dim, td, nullptr};
     pa.n = 1;
     if (!qkv_planes_kept) {
-        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, dim, td, nullptr};
-        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, dim, td, nullptr};
-        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, dim, td, nullptr};
+        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, nullptr};
+        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, T, dim, td, nullptr};
+        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, T, dim, td, nullptr};
         pa.n = 4;
     }
     if (launch_prepass(pa, stream)) return 1;

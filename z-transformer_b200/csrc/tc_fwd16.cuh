@@ -42,6 +42,7 @@ struct Shared {
     uint32_t tmem_base;
     volatile int abort;
     float fin_m[2][128], fin_l[2][128];  // each set's reference maximum and sum, for the final merge
+    float fin_f[2][128];                 // what has been flushed of its O is relative to this maximum (-inf: nothing)
 };
 
 struct Params {
@@ -49,7 +50,9 @@ struct Params {
     const uint32_t *amax_q, *amax_k, *amax_v;   // [B, Hkv]
     float *out, *lse;                           // lse may be null
     int batch, T, n_heads, n_kv_heads;
-    int dim_out;  // the tensors' head_dim: the tile's D, or 32 under a tile padded to 64
+    int q_offset;  // query row r stands at position q_offset + r of the keys: it sees keys 0 .. q_offset + r
+    int flush_tiles;  // O leaves the tensor core's accumulator every so many key tiles; 0: never (see flush_row)
+    int dim_out;  // the tensors' head_dim, at most the tile's D
     int ahead;    // attn_fwd_tc16 prefetches the query tile of the block this many places on in launch order; 0: none
     float scale_log2;
     // When set, the epilogue also leaves out as f16 hi/lo planes ([2][B][T][H * dim_out], one power-of-two scale per
@@ -119,6 +122,46 @@ __device__ __forceinline__ float row_exp32(const uint32_t (&r)[32], int key0, in
     return sum;
 }
 
+// The tensor core adds into its f32 accumulator with truncation, which over n key tiles of 64 costs O about
+// n 2.3e-7 of its size, always toward zero (1.4e-5 measured at 4096 keys in one accumulator).  With p.flush_tiles set,
+// O leaves TMEM every so many tiles and is summed with rounding in memory: in the row of out, which the finished row
+// overwrites at the end.  16 tiles hold the error at 3.7e-6 whatever the context, for 64 KB through L2 per 32000
+// clocks of MMAs.  Set for windows of a prompt, every row of which runs over the whole context behind it; over a whole
+// sequence the rows that see few keys carry the result's norm.
+constexpr int kFlushKeyTiles = 16;
+// Four columns of the running sum: the first flush starts it, `f` moves it to the current reference maximum.
+__device__ __forceinline__ float4 flush_sum4(const float *at, float f, bool first, float4 o) {
+    if (first) return o;
+    const float4 g = *reinterpret_cast<const float4 *>(at);
+    o.x = fmaf(g.x, f, o.x), o.y = fmaf(g.y, f, o.y), o.z = fmaf(g.z, f, o.z), o.w = fmaf(g.w, f, o.w);
+    return o;
+}
+// Where a row's running sum is kept: columns [0, D/2) and [D/2, D); `width` columns of it (the rest are padding), null
+// when the row is not the tensor's.
+struct FlushRow {
+    float *lower, *upper;
+    int width;
+    template <int D>
+    __device__ __forceinline__ float *at(int c) const { return c < D / 2 ? lower + c : upper + (c - D / 2); }
+};
+// O's columns [0, D) of this thread's row, at TMEM `taddr`, into its running sum.
+template <int D>
+__device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, float f, bool first) {
+#pragma unroll 1
+    for (int c = 0; c < D; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(taddr + c, r);
+        tmem_wait_ld();
+        if (row.lower == nullptr) continue;
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+            if (c + i >= row.width) break;
+            float *at = row.at<D>(c + i);
+            *reinterpret_cast<float4 *>(at) = flush_sum4(at, f, first, make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])));
+        }
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_fwd_tc16(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
@@ -139,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int g = h / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
-    const int n_tiles = (rows_end + BN - 1) / BN;
+    const int n_tiles = (p.q_offset + rows_end + BN - 1) / BN;
     const int B = p.batch;
 
     if (threadIdx.x == 0) {
@@ -260,11 +303,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t vh = v_u32 + (uint32_t)(s * 2 * KP);
                 const uint64_t mvh = desc_mnmajor_16b(vh, BN * 128), mvl = desc_mnmajor_16b(vh + KP, BN * 128);
                 const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
+                const bool fresh = j < 2 || (p.flush_tiles > 0 && (j >> 1) % p.flush_tiles == 0);  // (O was flushed before tile j)
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
                     const uint32_t ac = (uint32_t)(32 * (kk >> 1) + (kk & 1) * 8);
                     const uint64_t dvh = desc_advance(mvh, kk * 2048), dvl = desc_advance(mvl, kk * 2048);
-                    mma_ts_f16(tmem + cO, tmem + cS + ac, dvh, id_o, (j > 1 || kk > 0) ? 1 : 0);
+                    mma_ts_f16(tmem + cO, tmem + cS + ac, dvh, id_o, (!fresh || kk > 0) ? 1 : 0);
                     mma_ts_f16(tmem + cO, tmem + cS + ac, dvl, id_o, 1);
                     mma_ts_f16(tmem + cO, tmem + cS + ac + 16, dvh, id_o, 1);
                 }
@@ -283,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the key tiles of its parity, with a reference maximum, a sum and an O accumulator of its own;
         // the two partial softmaxes are merged at the end.  Nothing a set does waits on the other's tile.
         const int tid = threadIdx.x & 127, set = threadIdx.x >> 7;
-        const int t = t0 + tid;
+        const int t = t0 + tid, pos = p.q_offset + t;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         bool ok = true;
         {
@@ -307,6 +351,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         const float cs = p.scale_log2 / (mq * mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
+        float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
+        // where the sets keep flushed sums: set 0 in out, set 1 in the two planes of the query row, which this CTA alone
+        // reads and has in TMEM by now (a forward that flushes keeps no planes for a backward)
+        FlushRow row0{nullptr, nullptr, p.dim_out}, row1{nullptr, nullptr, D};
+        if (p.flush_tiles > 0 && t < p.T) {
+            row0.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
+            row0.upper = row0.lower + D / 2;
+            __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * D + (long long)h * D;
+            row1.lower = reinterpret_cast<float *>(planes);
+            row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * D);
+        }
         for (int j = set; ok && j < n_tiles; j += 2) {
             if (!__all_sync(0xffffffffu, fwait(&sh->s_full[set], (uint32_t)((j >> 1) & 1), sh))) {
                 fgive_up(sh, 45);
@@ -315,23 +370,25 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_after();
             const int s0 = j * BN;
-            const bool diag = (s0 + BN - 1 > t0) && !ZT_DEFECT(1);
+            const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32(tmem + lane_base + cS, r0);
             tmem_ld32(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
             float mt = -INFINITY;
-            if (diag) mt = row_max32<true>(r1, s0 + 32, t, row_max32<true>(r0, s0, t, mt));
-            else mt = row_max32<false>(r1, s0 + 32, t, row_max32<false>(r0, s0, t, mt));
+            if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
+            else mt = row_max32<false>(r1, s0 + 32, pos, row_max32<false>(r0, s0, pos, mt));
             mt *= cs;  // cs > 0
             float factor = 1.f;
+            const float m_old = m_ref;
             if ((mt > m_ref + kRescaleThreshold || m_ref == -INFINITY) && mt != -INFINITY) {
                 factor = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - mt);
                 m_ref = mt;
             }
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
-            if (j > 1 && __any_sync(0xffffffffu, factor != 1.f)) {
+            const bool flush = p.flush_tiles > 0 && j > 1 && (j >> 1) % p.flush_tiles == 0;
+            if (j > 1 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
                 // this set's O may only be touched once its previous P.V (tile j-2) has retired
                 if (!__all_sync(0xffffffffu, fwait(&sh->pv_done[set], (uint32_t)(((j >> 1) - 1) & 1), sh))) {
                     fgive_up(sh, 46);
@@ -339,14 +396,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 }
                 tc_fence_after();
+                if (flush) {
+                    const bool first = m_flushed == -INFINITY;
+                    flush_row<D>(tmem + lane_base + cO, set == 0 ? row0 : row1, first ? 0.f : ex2(m_flushed - m_old), first);
+                    m_flushed = m_old;
+                } else {
 #pragma unroll 1
-                for (int c = 0; c < D; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem + lane_base + cO + c, r);
-                    tmem_wait_ld();
+                    for (int c = 0; c < D; c += 32) {
+                        uint32_t r[32];
+                        tmem_ld32(tmem + lane_base + cO + c, r);
+                        tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
-                    tmem_st32(tmem + lane_base + cO + c, r);
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
+                        tmem_st32(tmem + lane_base + cO + c, r);
+                    }
                 }
             }
             // l is kept in P's units (times kPScale), like O
@@ -354,10 +417,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             float psum;
             {
                 uint32_t ph[16], pl[16];
-                psum = diag ? row_exp32<true>(r0, s0, t, cs, off, ph, pl) : row_exp32<false>(r0, s0, t, cs, off, ph, pl);
+                psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
                 tmem_st16(tmem + lane_base + cS, ph);
                 tmem_st16(tmem + lane_base + cS + 16, pl);
-                psum += diag ? row_exp32<true>(r1, s0 + 32, t, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, t, cs, off, ph, pl);
+                psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
                 tmem_st16(tmem + lane_base + cS + 32, ph);
                 tmem_st16(tmem + lane_base + cS + 48, pl);
             }
@@ -369,6 +432,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---- merge the two partial softmaxes
         sh->fin_m[set][tid] = m_ref;
         sh->fin_l[set][tid] = l;
+        sh->fin_f[set][tid] = m_flushed;
         asm volatile("bar.sync 1, 256;" ::: "memory");  // the 256 softmax threads
         if (ok && !__all_sync(0xffffffffu, fwait(&sh->all_done, 0, sh))) {
             fgive_up(sh, 48);
@@ -384,10 +448,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float m0 = sh->fin_m[0][tid], l0 = sh->fin_l[0][tid];
             const float m1 = two ? sh->fin_m[1][tid] : -INFINITY, l1 = two ? sh->fin_l[1][tid] : 0.f;
             const float mm = fmaxf(m0, m1);  // m0 is finite: key 0 is visible to every row
-            const float w0 = ex2(m0 - mm), w1 = (m1 == -INFINITY) ? 0.f : ex2(m1 - mm);
+            // (the merge is a running-maximum correction too, the only one where each set has a single tile)
+            const float w0 = ZT_DEFECT(3) ? 1.f : ex2(m0 - mm), w1 = (m1 == -INFINITY) ? 0.f : (ZT_DEFECT(3) ? 1.f : ex2(m1 - mm));
             const float lsum = w0 * l0 + w1 * l1;
             const float inv = 1.f / (lsum * mv);  // lsum, like O, carries kPScale
             const float f0 = w0 * inv, f1 = w1 * inv;
+            const float s0 = sh->fin_f[0][tid], s1 = sh->fin_f[1][tid];
+            const bool add0 = s0 != -INFINITY && row0.lower != nullptr, add1 = s1 != -INFINITY && row1.lower != nullptr;
+            const float g0 = add0 ? ex2(s0 - m0) : 0.f, g1 = add1 ? ex2(s1 - m1) : 0.f;
             // set s merges columns [s D/2, (s+1) D/2) of the row
             uint8_t *srow = sK + tid * (D * 4);
 #pragma unroll 1
@@ -398,12 +466,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tmem_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                    float4 o4;
-                    o4.x = __uint_as_float(ra[i]) * f0, o4.y = __uint_as_float(ra[i + 1]) * f0;
-                    o4.z = __uint_as_float(ra[i + 2]) * f0, o4.w = __uint_as_float(ra[i + 3]) * f0;
+                    const int col = set * (D / 2) + c + i;
+                    float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
+                    if (add0 && col < row0.width) o4 = flush_sum4(row0.at<D>(col), g0, false, o4);
+                    o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
-                        o4.x += __uint_as_float(rb[i]) * f1, o4.y += __uint_as_float(rb[i + 1]) * f1;
-                        o4.z += __uint_as_float(rb[i + 2]) * f1, o4.w += __uint_as_float(rb[i + 3]) * f1;
+                        float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
+                        if (add1) x4 = flush_sum4(row1.at<D>(col), g1, false, x4);
+                        o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     const int ch = (set * (D / 2) + c + i) >> 2;
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;
@@ -440,13 +510,13 @@ struct Workspace {
     size_t total_bytes, amax_bytes;
 };
 
-inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim) {
+inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset = 0) {
     Workspace w{};
     const size_t n_amax = (size_t)batch * n_kv_heads;
     w.amax_bytes = (3 * n_amax * sizeof(uint32_t) + 1023) / 1024 * 1024;
     auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
     const size_t qh = (size_t)2 * batch * T * n_heads * dim * sizeof(__half);
-    const size_t kh = (size_t)2 * batch * T * n_kv_heads * dim * sizeof(__half);
+    const size_t kh = (size_t)2 * batch * (q_offset + T) * n_kv_heads * dim * sizeof(__half);
     char *c = static_cast<char *>(base);
     w.amax_q = reinterpret_cast<uint32_t *>(c), w.amax_k = w.amax_q + n_amax, w.amax_v = w.amax_k + n_amax;
     size_t off = w.amax_bytes;
@@ -477,15 +547,12 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
 
 }  // namespace tcf16
 
-inline size_t tc_fwd16_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
-    return tcf16::workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).total_bytes;
+inline size_t tc_fwd16_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset = 0) {
+    return tcf16::workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim), q_offset).total_bytes;
 }
 
-inline bool tc_fwd16_supported(int batch, int T, int dim, int q_offset, int n_keys, const void *q, const void *k,
-                               const void *v, const void *out) {
-    if (!(dim == 32 || dim == 64 || dim == 96 || dim == 128 || dim == 192 || dim == 256) || q_offset != 0 || n_keys != T ||
-        T < 128 || batch < 1)
-        return false;
+inline bool tc_fwd16_supported(int batch, int T, int dim, const void *q, const void *k, const void *v, const void *out) {
+    if (!tc_takes_dim(dim) || T < kTcForwardMinRows || batch < 1) return false;
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(q) || !al(k) || !al(v) || !al(out)) return false;
     const DeviceInfo *d = device_info();
@@ -494,14 +561,16 @@ inline bool tc_fwd16_supported(int batch, int T, int dim, int q_offset, int n_ke
 
 // `in_backward_workspace`: lay the planes out where the backward's workspace keeps them (tc_bwd.cuh
 // bwd_workspace), so that a backward given the same workspace can use them as they are.
+// q_offset: the query rows are a window of the sequence that starts there (batch 1; k and v hold at least q_offset + T
+// rows, of which the later ones are not read).
 // out_planes (optional): where the kernel also leaves out as f16 hi/lo planes, [2][batch][T][n_heads * dim] halves.
 inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float *out, float *lse, void *ws,
                            int batch, int T, int n_heads, int n_kv_heads, int dim, cudaStream_t stream,
                            const float2 *rope = nullptr, bool in_backward_workspace = false, int variant = 0,
-                           __half *out_planes = nullptr, const PeerList *out_peers = nullptr) {
+                           __half *out_planes = nullptr, const PeerList *out_peers = nullptr, int q_offset = 0) {
     using namespace tcb;
-    const int td = tc_tile_dim(dim);  // the kernel's D; the planes' head width (head_dim 32 is zero-padded to 64)
-    tcf16::Workspace w = tcf16::workspace(ws, batch, T, n_heads, n_kv_heads, td);
+    const int td = tc_tile_dim(dim);  // the kernel's D; the planes' head width
+    tcf16::Workspace w = tcf16::workspace(ws, batch, T, n_heads, n_kv_heads, td, q_offset);
     if (in_backward_workspace) {
         const BwdWorkspace bw = bwd_workspace(ws, batch, T, n_heads, n_kv_heads, td);
         w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;  // contiguous; amax_do follows
@@ -511,28 +580,29 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     const int group = n_heads / n_kv_heads;
     const int wq_src = n_heads * dim, wkv_src = n_kv_heads * dim;
     const int wkv = n_kv_heads * td;
+    const int n_seen = q_offset + T;  // key rows that some query row sees
     if (cudaMemsetAsync(w.amax_q, 0, w.amax_bytes, stream) != cudaSuccess) {
         cudaGetLastError();
         return refuse("could not clear the forward workspace header");
     }
     PrepassArgs pa{};
-    pa.n = 3, pa.batch = batch, pa.T = T;
-    pa.t[0] = {q, w.amax_q, w.q_planes, wq_src, group * dim, dim, td, rope};
-    pa.t[1] = {k, w.amax_k, w.k_planes, wkv_src, dim, dim, td, rope};
-    pa.t[2] = {v, w.amax_v, w.v_planes, wkv_src, dim, dim, td, nullptr};
+    pa.n = 3, pa.batch = batch;
+    pa.t[0] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, rope};
+    pa.t[1] = {k, w.amax_k, w.k_planes, wkv_src, dim, n_seen, dim, td, rope};
+    pa.t[2] = {v, w.amax_v, w.v_planes, wkv_src, dim, n_seen, dim, td, nullptr};
     if (launch_prepass(pa, stream)) return 1;
     if (td == 256) {
-        // head_dim 256 (and 192 padded to it): one head per CTA, K fetched block by block (attn_fwd_tc16x)
+        // head_dim 256 (and those padded to it): one head per CTA, K fetched block by block (attn_fwd_tc16x)
         CUtensorMap kmap, vmap, qmap;
-        if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, T, wkv, 64, 64) ||
-            !make_half_tile_map(&vmap, w.v_planes, 2 * batch, T, wkv, td, 64) ||
+        if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, 64, 64) ||
+            !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
             !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
             return refuse("the TMA tensor maps for the forward could not be encoded.");
         tcf16::Params p{};
         p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
         p.out = out, p.lse = lse;
         p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-        p.dim_out = dim;
+        p.dim_out = dim, p.q_offset = q_offset, p.flush_tiles = q_offset > 0 ? tcf16::kFlushKeyTiles : 0;
         p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
         if (out_peers) p.out_peers = *out_peers;
         p.scale_log2 = kLog2e / sqrtf((float)dim);
@@ -543,15 +613,15 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     // and that still gives every SM a CTA, one head per CTA (attn_fwd_tc16) otherwise; 1: one head per CTA;
     // 2: two heads per CTA whatever the number of CTAs (the group must be even).
     CUtensorMap kmap, vmap, qmap;
-    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, T, wkv, td, 64) ||
-        !make_half_tile_map(&vmap, w.v_planes, 2 * batch, T, wkv, td, 64) ||
+    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td, 64) ||
+        !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
         !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
     tcf16::Params p{};
     p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
     p.out = out, p.lse = lse;
     p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-    p.dim_out = dim;
+    p.dim_out = dim, p.q_offset = q_offset, p.flush_tiles = q_offset > 0 ? tcf16::kFlushKeyTiles : 0;
     p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
     if (out_peers) p.out_peers = *out_peers;
     p.ahead = device_info() ? device_info()->sm_count : 0;  // one CTA per SM

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int g = h0 / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
-    const int n_tiles = (rows_end + BN - 1) / BN;
+    const int n_tiles = (p.q_offset + rows_end + BN - 1) / BN;
     const int B = p.batch;
 
     if (threadIdx.x == 0) {
@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             };
             // P.V of head `hd`, tile j (V tile j has landed)
             auto issue_pv = [&](int hd, int j) {
+                const bool fresh = j == 0 || (p.flush_tiles > 0 && j % p.flush_tiles == 0);  // (O was flushed before tile j)
                 const uint32_t vh = v_u32 + (uint32_t)((j & 1) * 2 * KP);
                 const uint64_t mvh = desc_mnmajor_16b(vh, BN * 128), mvl = desc_mnmajor_16b(vh + KP, BN * 128);
                 const uint32_t cS = cS0 + hd * BN, cO = cO0 + hd * D;
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int kk = 0; kk < BN / 16; ++kk) {
                     const uint32_t ac = (uint32_t)(32 * (kk >> 1) + (kk & 1) * 8);
                     const uint64_t dvh = desc_advance(mvh, kk * 2048), dvl = desc_advance(mvl, kk * 2048);
-                    mma_ts_f16(tmem + cO, tmem + cS + ac, dvh, id_o, (j > 0 || kk > 0) ? 1 : 0);
+                    mma_ts_f16(tmem + cO, tmem + cS + ac, dvh, id_o, (!fresh || kk > 0) ? 1 : 0);
                     mma_ts_f16(tmem + cO, tmem + cS + ac, dvl, id_o, 1);
                     mma_ts_f16(tmem + cO, tmem + cS + ac + 16, dvh, id_o, 1);
                 }
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int tid = threadIdx.x & 127, set = threadIdx.x >> 7;
         const int lane = threadIdx.x & 31;
         const int h = h0 + set;
-        const int t = t0 + tid;
+        const int t = t0 + tid, pos = p.q_offset + t;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         bool ok = true;
         {
@@ -223,6 +224,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         const float cs = p.scale_log2 / (mq * mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
+        float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
+        FlushRow row{nullptr, nullptr, p.dim_out};
+        if (p.flush_tiles > 0 && t < p.T) {
+            row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
+            row.upper = row.lower + D / 2;
+        }
         for (int j = 0; ok && j < n_tiles; ++j) {
             if (!__all_sync(0xffffffffu, gwait(&sh->s_full[set], (uint32_t)(j & 1), sh))) {
                 ggive_up(sh, 45);
@@ -231,23 +238,25 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_after();
             const int s0 = j * BN;
-            const bool diag = (s0 + BN - 1 > t0) && !ZT_DEFECT(1);
+            const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32(tmem + lane_base + cS, r0);
             tmem_ld32(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
             float mt = -INFINITY;
-            if (diag) mt = row_max32<true>(r1, s0 + 32, t, row_max32<true>(r0, s0, t, mt));
-            else mt = row_max32<false>(r1, s0 + 32, t, row_max32<false>(r0, s0, t, mt));
+            if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
+            else mt = row_max32<false>(r1, s0 + 32, pos, row_max32<false>(r0, s0, pos, mt));
             mt *= cs;  // cs > 0
             float factor = 1.f;
+            const float m_old = m_ref;
             if ((mt > m_ref + kRescaleThreshold || m_ref == -INFINITY) && mt != -INFINITY) {
                 factor = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - mt);
                 m_ref = mt;
             }
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
-            if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
+            const bool flush = p.flush_tiles > 0 && j > 0 && j % p.flush_tiles == 0;
+            if (j > 0 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
                 // this head's O may only be touched once its previous P.V has retired
                 if (!__all_sync(0xffffffffu, gwait(&sh->pv_done[set], (uint32_t)((j - 1) & 1), sh))) {
                     ggive_up(sh, 46);
@@ -255,14 +264,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 }
                 tc_fence_after();
+                if (flush) {
+                    const bool first = m_flushed == -INFINITY;
+                    flush_row<D>(tmem + lane_base + cO, row, first ? 0.f : ex2(m_flushed - m_old), first);
+                    m_flushed = m_old;
+                } else {
 #pragma unroll 1
-                for (int c = 0; c < D; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem + lane_base + cO + c, r);
-                    tmem_wait_ld();
+                    for (int c = 0; c < D; c += 32) {
+                        uint32_t r[32];
+                        tmem_ld32(tmem + lane_base + cO + c, r);
+                        tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
-                    tmem_st32(tmem + lane_base + cO + c, r);
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
+                        tmem_st32(tmem + lane_base + cO + c, r);
+                    }
                 }
             }
             // l is kept in P's units (times kPScale), like O
@@ -270,10 +285,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             float psum;
             {
                 uint32_t ph[16], pl[16];
-                psum = diag ? row_exp32<true>(r0, s0, t, cs, off, ph, pl) : row_exp32<false>(r0, s0, t, cs, off, ph, pl);
+                psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
                 tmem_st16(tmem + lane_base + cS, ph);
                 tmem_st16(tmem + lane_base + cS + 16, pl);
-                psum += diag ? row_exp32<true>(r1, s0 + 32, t, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, t, cs, off, ph, pl);
+                psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
                 tmem_st16(tmem + lane_base + cS + 32, ph);
                 tmem_st16(tmem + lane_base + cS + 48, pl);
             }
@@ -293,6 +308,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
+            const bool add = m_flushed != -INFINITY && row.lower != nullptr;
+            const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * (D * 4);
 #pragma unroll 1
             for (int c = 0; c < D; c += 32) {
@@ -301,9 +318,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tmem_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                    float4 o4;
-                    o4.x = __uint_as_float(ra[i]) * inv, o4.y = __uint_as_float(ra[i + 1]) * inv;
-                    o4.z = __uint_as_float(ra[i + 2]) * inv, o4.w = __uint_as_float(ra[i + 3]) * inv;
+                    float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
+                    if (add && c + i < row.width) o4 = flush_sum4(row.at<D>(c + i), ff, false, o4);
+                    o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     const int ch = (c + i) >> 2;
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;
                 }

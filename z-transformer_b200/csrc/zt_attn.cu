@@ -101,10 +101,10 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
 #ifndef ZT_NO_TC
     const int path = g_path.load();
     if ((path == 0 || path == 6 || path == 7 || path == 8) && n_kv_heads <= tcb::kPrepassMaxGroups &&
-        tc_fwd16_supported(batch, T, dim, q_offset, n_keys, q, k, v, out)) {
+        tc_fwd16_supported(batch, T, dim, q, k, v, out)) {
         // The f16-split forward keeps its operand planes in the per-device arena (no entry point
         // of the forward takes a workspace); see device_arena for when that allocates.
-        const size_t need = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+        const size_t need = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim, q_offset);
         bool in_capture = false;
         void *arena = device_arena(need, stream, &in_capture);
         if (in_capture)
@@ -112,7 +112,7 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
                           "stream is being captured: call zt_attn_reserve for the shape before the capture.", need);
         if (arena)
             return launch_fwd_tc16(q, k, v, out, lse, arena, batch, T, n_heads, n_kv_heads, dim, stream, nullptr, false,
-                                   path == 6 ? 1 : (path == 7 ? 2 : 0));
+                                   path == 6 ? 1 : (path == 7 ? 2 : 0), nullptr, nullptr, q_offset);
     }
     if ((path == 0 || path == 2 || path == 6 || path == 7 || path == 8) &&
         tc_fwd_supported(batch, T, n_heads, n_kv_heads, dim, q_offset, n_keys, q, k, v, out)) {
@@ -131,10 +131,11 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
 
 static size_t backward_workspace(int batch, int T, int n_heads, int n_kv_heads, int dim) {
 #ifndef ZT_NO_TC
-    if ((dim == 32 || dim == 64 || dim == 96 || dim == 128) && T >= 128)
-        return tc_bwd_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
-    // head_dim 192 and 256: the planes of the fused form, then a row-scaled copy of Q's and the planes of P and dS
-    if ((dim == 192 || dim == 256) && T >= 128) return tc_bwd_wide_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+    if (tc_takes_dim(dim)) {
+        if (dim <= 128) return tc_bwd_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+        // wider heads: the planes of the fused form, then a row-scaled copy of Q's and the planes of P and dS
+        return tc_bwd_wide_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+    }
 #endif
     (void)batch, (void)n_heads, (void)n_kv_heads;
     return 0;
@@ -345,8 +346,7 @@ int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     if (need_device()) return 1;
     size_t need = kArenaBytes;  // the decode-shaped forward's partial results
 #ifndef ZT_NO_TC
-    if (n_kv_heads <= tcb::kPrepassMaxGroups && T >= 128 &&
-        (dim == 32 || dim == 64 || dim == 96 || dim == 128 || dim == 192 || dim == 256)) {
+    if (n_kv_heads <= tcb::kPrepassMaxGroups && tc_takes_dim(dim)) {
         const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
         const size_t b = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
         need = f > need ? f : need;
@@ -528,7 +528,7 @@ static int forward_keep_impl(const float *q, const float *k, const float *v, flo
     const int keep_path = g_path.load();
     if ((keep_path == 0 || keep_path == 6 || keep_path == 7 || keep_path == 8) && need > 0 && workspace && workspace_bytes >= need &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
-        tc_fwd16_supported(batch, T, dim, 0, T, q, k, v, out)) {
+        tc_fwd16_supported(batch, T, dim, q, k, v, out)) {
         if (launch_fwd_tc16(q, k, v, out, lse, workspace, batch, T, n_heads, n_kv_heads, dim, s, nullptr, true,
                             keep_path == 6 ? 1 : (keep_path == 7 ? 2 : 0), nullptr, out_peers))
             return 1;
@@ -684,8 +684,9 @@ static int forward_rope_impl(const float *q, const float *k, const float *v, flo
     drop_kept_planes(w.inner);
     if (launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
 #ifndef ZT_NO_TC
-    if ((g_path.load() == 0 || g_path.load() == 8) && n_kv_heads <= tcb::kPrepassMaxGroups &&
-        tc_fwd16_supported(batch, T, dim, 0, T, q, k, v, out) &&
+    // (the pre-pass rotates four elements at a time: a head's halves must be multiples of four)
+    if ((g_path.load() == 0 || g_path.load() == 8) && n_kv_heads <= tcb::kPrepassMaxGroups && dim % 8 == 0 &&
+        tc_fwd16_supported(batch, T, dim, q, k, v, out) &&
         w.inner_bytes >= tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim)) {
         // the planes (rotated q and k among them) go where the backward keeps its own: the rope backward that
         // follows with the same workspace, tensors, pos and theta converts only dout
@@ -732,12 +733,12 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     if (launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
     bool fused = false, dq_in_kernel = false;
 #ifndef ZT_NO_TC
-    fused = g_path.load() != 1 && w.inner_bytes > 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
+    fused = g_path.load() != 1 && w.inner_bytes > 0 && dim % 8 == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
             tcb::tc_bwd_supported(batch, T, dim, q, k, v, dout, dq, dk, dv);
-    // the dQ kernel's epilogue rotates whole 16- or 32-column pieces: not at head_dim 96, whose halves are 48 wide;
+    // the dQ kernel's epilogue rotates whole 16- or 32-column pieces: only where a head's half is made of them;
     // and the fused backward adds partial sums into dq, which can only be rotated once they are complete
     const bool two_kernels = g_path.load() == 8;
-    dq_in_kernel = fused && dim != 96 && !tc_bwd_takes_fused(dim, two_kernels, nullptr);
+    dq_in_kernel = fused && (dim == 32 || dim == 64 || dim == 128) && !tc_bwd_takes_fused(dim, two_kernels, nullptr);
     if (fused && launch_delta(out, dout, delta, tcb::bwd_workspace(w.inner, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).rnorm,
                               (long long)batch * T * n_heads, dim, s))
         return 1;
@@ -748,8 +749,8 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     if (!fused) {
         if (launch_rope_apply(q, w.q_rot, w.table, batch, T, n_heads * dim, dim, false, s)) return 1;
         if (launch_rope_apply(k, w.k_rot, w.table, batch, T, n_kv_heads * dim, dim, false, s)) return 1;
-        // (head_dim 192 and 256 take the unfused tensor-core form, which wants the inner workspace)
-        const bool wide = dim == 192 || dim == 256;
+        // (the wide heads take the unfused tensor-core form, which wants the inner workspace)
+        const bool wide = dim > 128 || dim % 8 != 0;
         if (backward_impl(w.q_rot, w.k_rot, v, out, lse, delta, dout, dq, dk, dv, wide ? w.inner : nullptr,
                           wide ? w.inner_bytes : 0, batch, T, n_heads, n_kv_heads, dim, s))
             return 1;
@@ -803,8 +804,8 @@ int check_proj(const void *workspace, size_t workspace_bytes, int batch, int T, 
 // planes of x [batch][rows][width] with one scale per batch item
 int proj_planes(const float *x, uint32_t *amax, __half *planes, int batch, int rows, int width, cudaStream_t s) {
     tcb::PrepassArgs pa{};
-    pa.n = 1, pa.batch = batch, pa.T = rows;
-    pa.t[0] = {x, amax, planes, width, width, width, width, nullptr};
+    pa.n = 1, pa.batch = batch;
+    pa.t[0] = {x, amax, planes, width, width, rows, width, width, nullptr};
     return tcb::launch_prepass(pa, s);
 }
 #endif
