@@ -1,0 +1,455 @@
+// The pre-pass of the tensor-core kernels: f32 tensors -> f16 hi/lo operand planes with a power-of-two scale per
+// (sequence, group of heads), and beside them what the backward wants to know about the rows of dout.
+//
+// Two launches for all tensors of a call, both bound by HBM (or, for small calls, by launch latency):
+//   pass_stats_kernel    reads every tensor once.  Per block: max |x| and, where asked, the largest row norm; per row of
+//                        dout its norm and delta = sum_j dout out.  A block leaves its two maxima in a slot of its own
+//                        (no atomics and nothing to clear beforehand).
+//   pass_planes_kernel   reads the slots of its (sequence, group) -- at most 1024 of them --, publishes the maxima for
+//                        the attention kernels, and writes the planes (rotating q and k on the way where rope is asked
+//                        for), the row-scaled copy of q's planes for dK, and the zeros of outputs that are summed in memory.
+// Both work on units, one head of one row, held by 8, 16 or 32 lanes; a lane has four units in flight.  A block's units
+// belong to one (sequence, group); the split into blocks aims at 2048 blocks per tensor (14 an SM; 4096 and 1024 were
+// 1-2 % slower, 512 more) of at least eight units a lane group.
+// Before (one kernel per quantity: two for the planes, one each for delta, v's norms, dout's norms, the row-scaled
+// copy, and up to four memsets; 13 launches a step where there are 6 now): batch 8, T 512, 32/8 heads of 64, forward
+// and backward, 175 us, now 115; T 1024, heads of 256, 740 us, now 540; T 4096, heads of 128, 1370 us, now 1270.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "rope_kernels.cuh"
+#include "zt_common.cuh"
+
+namespace zt {
+namespace tcb {
+
+// ---- scaling --------------------------------------------------------------------------------------
+// The power of two that moves a block's largest magnitude into [2^14, 2^15).  `bits` is the f32
+// bit pattern of max |x| (non-negative, so it orders like an integer).
+__host__ __device__ inline float block_mult(uint32_t bits) {
+    const int ex = (int)((bits >> 23) & 0xff);  // biased exponent: |x| in [2^(ex-127), 2^(ex-126))
+    if (ex == 0 || ex == 0xff) return 1.0f;      // zero/subnormal block, or inf/nan: leave alone
+    int e = 14 - (ex - 127);                     // |x| * 2^e in [2^14, 2^15)
+    if (e > 126) e = 126;
+    if (e < -126) e = -126;
+    uint32_t out = (uint32_t)(e + 127) << 23;
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(out);
+#else
+    float f;
+    memcpy(&f, &out, 4);
+    return f;
+#endif
+}
+// pow2_for(x, top): the power of two c with x c in [2^(top-1), 2^top); 1 when x is zero or not finite.
+__device__ __forceinline__ float pow2_for(float x, int top) {
+    if (!(x > 0.f) || !(x < 3.0e38f)) return 1.0f;
+    int e;
+    frexpf(x, &e);  // x = m 2^e, m in [0.5, 1)
+    int k = top - e;
+    k = k > 120 ? 120 : (k < -120 ? -120 : k);
+    return __uint_as_float((uint32_t)(k + 127) << 23);
+}
+// Row t's scale of dS (cq) and what divides row t of the second copy of Q (1 / rel): both powers of two.
+constexpr float kRowBoostMax = 4096.f;  // a row's scale is at most this many times the group's smallest
+__device__ __forceinline__ float ds_group_scale(uint32_t rnmax_bits, uint32_t vnmax_bits) {
+    return pow2_for(2.02f * __uint_as_float(rnmax_bits) * __uint_as_float(vnmax_bits), 14);
+}
+__device__ __forceinline__ void ds_row_scale(float rnorm_t, uint32_t rnmax_bits, uint32_t vnmax_bits, float &cq, float &rel) {
+    const float cmin = ds_group_scale(rnmax_bits, vnmax_bits);
+    const float x = 2.02f * rnorm_t * __uint_as_float(vnmax_bits);
+    float c = (x > 0.f && x < 3.0e38f) ? pow2_for(x, 14) : cmin;
+    c = fminf(fmaxf(c, cmin), cmin * kRowBoostMax);
+    if (!(c < 3.0e38f)) c = cmin;
+    cq = c;
+    rel = cmin / c;
+}
+
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// (a, b) -> packed h pair and packed l pair: one paired conversion each way instead of two single ones
+__device__ __forceinline__ void split_pack(float a, float b, uint32_t &hw, uint32_t &lw) {
+    const __half2 hh = __floats2half2_rn(a, b);
+    const float2 back = __half22float2(hh);
+    hw = *reinterpret_cast<const uint32_t *>(&hh);
+    lw = pack_half2(a - back.x, b - back.y);
+}
+
+// ---- the two launches -------------------------------------------------------------------------------
+constexpr int kPrepassMaxGroups = 256;
+constexpr int kPassThreads = 256, kStatsStages = 4, kPassUnroll = 4;
+constexpr int kPassTargetBlocks = 2048, kPassMaxSlots = 1024, kPassMaxTensors = 5;
+constexpr int kFillPerBlock = 4096;  // float4
+
+struct PassTensor {
+    const float *x;          // [batch][rows][heads * dim]; null: no f32 source, see q_planes
+    const float *o;          // with delta: the tensor it is formed with
+    float *delta, *rnorm;    // [batch][rows][heads], or null
+    __half *planes;          // [2][batch][rows][heads * td], or null
+    uint2 *part;             // [batch * groups][slots] (max |x|, largest row norm) as f32 bit patterns
+    uint32_t *amax, *nmax;   // [batch * groups]: where the maxima are published; nmax null: not wanted
+    const float2 *rope;      // null, or the (cos, sin) table [rows][dim / 2]: x is rotated on its way into the planes
+    // the copy of the planes with row t times rel(t) (ds_row_scale, from rnorm and the largest row norms of dout and v),
+    // or null; made from x's planes as they pass, or from q_planes where x is null
+    __half *qs;
+    const __half *q_planes;
+    const uint2 *dn_part, *vn_part;  // dout's slots; v's, or null: v's norms are published already
+    const uint32_t *vn_final;
+    int dn_slots, vn_slots;
+    int batch, rows, heads, group;  // heads per row, heads per group
+    int slots, per_block;           // blocks per (sequence, group), units per block
+    int first;                      // first block of this tensor
+};
+struct PassArgs {
+    PassTensor t[kPassMaxTensors];
+    float4 *fill[3];
+    long long fill_n4[3];
+    int fill_first[4];  // first block of each region; [n_fill]: one past the last
+    int n, n_stats, n_fill, dim, td;
+};
+
+struct PassUnit {  // where a block stands
+    int z, bg, slot, b, g, begin, end;
+};
+__device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int blk) {
+    PassUnit w;
+    w.z = 0;
+    while (w.z + 1 < n && blk >= a.t[w.z + 1].first) ++w.z;
+    const PassTensor &t = a.t[w.z];
+    const int groups = t.heads / t.group, i = blk - t.first;
+    w.bg = i / t.slots, w.slot = i - w.bg * t.slots;
+    w.b = w.bg / groups, w.g = w.bg - w.b * groups;
+    w.begin = w.slot * t.per_block;
+    w.end = min(w.begin + t.per_block, t.rows * t.group);
+    return w;
+}
+
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool in) {
+    const int bytes = in ? 16 : 0;  // (0: the 16 bytes are filled with zeros and src is not read)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// LP lanes hold a unit, NC float4 each.  The loads run kStages - 1 steps of U units ahead through slots of shared memory
+// that belong to one thread each (so nothing but the thread's own copies is waited for): held in registers instead,
+// the loads of a step would stall on the arithmetic of the step before (heads of 256, batch 8, T 1024: 4.1 TB/s against 5.4).
+template <int LP, int NC>
+__global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_constant__ PassArgs a) {
+    constexpr int NG = kPassThreads / LP, U = 2 / NC, S = kStatsStages;
+    extern __shared__ __align__(16) float4 ring[];  // [S][U][NC][2][kPassThreads]
+    __shared__ float red[2][kPassThreads / 32];
+    const PassUnit w = pass_locate(a, a.n_stats, (int)blockIdx.x);
+    const PassTensor &t = a.t[w.z];
+    const int gi = threadIdx.x / LP, li = threadIdx.x % LP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool rows_out = t.delta != nullptr, norms = rows_out || t.nmax != nullptr;
+    const int n4 = a.dim >> 2, group = t.group, heads = t.heads;
+    const long long first = (long long)w.b * t.rows * heads + w.g * group;  // the (sequence, group)'s first unit
+    const float4 *xb = reinterpret_cast<const float4 *>(t.x) + first * n4 + li;
+    const float4 *ob = reinterpret_cast<const float4 *>(rows_out ? t.o : t.x) + first * n4 + li;
+    const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(ring + threadIdx.x);
+    const int n_steps = (w.end - w.begin + NG * U - 1) / (NG * U);
+    const auto place = [&](int step, int k) -> int {  // the unit's index within the (sequence, group), or -1
+        const int u = w.begin + gi + (step * U + k) * NG;
+        return u < w.end ? (u / group) * (heads - group) + u : -1;  // r heads + (u - r group)
+    };
+    const auto fetch = [&](int step) {
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int at = place(step, k);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const bool in = step < n_steps && at >= 0 && li + LP * c < n4;
+                const long long off = in ? (long long)at * n4 + LP * c : 0;
+                const uint32_t dst = slot0 + (uint32_t)((((step % S) * U + k) * NC + c) * 2 * kPassThreads * 16);
+                copy16_async(dst, xb + off, in);
+                if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    pdl_wait();
+    pdl_launch();
+#pragma unroll
+    for (int i = 0; i < S - 1; ++i) fetch(i);
+    float amax = 0.f, nmax = 0.f;
+    for (int step = 0; step < n_steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        float sq[U], de[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            sq[k] = 0.f, de[k] = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float4 *at = ring + (((step % S) * U + k) * NC + c) * 2 * kPassThreads + threadIdx.x;
+                const float4 x = at[0];
+                amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+                sq[k] = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq[k]))));
+                if (rows_out) {
+                    const float4 o = at[kPassThreads];
+                    de[k] = fmaf(x.x, o.x, fmaf(x.y, o.y, fmaf(x.z, o.z, fmaf(x.w, o.w, de[k]))));
+                }
+            }
+        }
+        fetch(step + S - 1);
+        if (!norms) continue;
+#pragma unroll
+        for (int off = LP / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], off);
+                if (rows_out) de[k] += __shfl_xor_sync(0xffffffffu, de[k], off);
+            }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const float norm = sqrtf(sq[k]);
+            nmax = fmaxf(nmax, norm);
+            const int at = place(step, k);
+            if (rows_out && li == 0 && at >= 0) t.delta[first + at] = de[k], t.rnorm[first + at] = norm;
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+        nmax = fmaxf(nmax, __shfl_xor_sync(0xffffffffu, nmax, off));
+    }
+    if (lane == 0) red[0][warp] = amax, red[1][warp] = nmax;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 1; i < kPassThreads / 32; ++i) amax = fmaxf(amax, red[0][i]), nmax = fmaxf(nmax, red[1][i]);
+        t.part[(long long)w.bg * t.slots + w.slot] = make_uint2(__float_as_uint(amax), __float_as_uint(nmax));
+    }
+}
+
+// The largest of `slots` pairs, by the whole block, in every thread.  (f32 bit patterns of non-negative numbers order
+// like integers.)
+__device__ __forceinline__ uint2 pass_reduce(const uint2 *part, int slots, uint2 *red) {
+    uint2 m = make_uint2(0u, 0u);
+    for (int i = threadIdx.x; i < slots; i += kPassThreads) {
+        const uint2 v = part[i];
+        m.x = max(m.x, v.x), m.y = max(m.y, v.y);
+    }
+    m.x = __reduce_max_sync(0xffffffffu, m.x), m.y = __reduce_max_sync(0xffffffffu, m.y);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = red[0];
+#pragma unroll
+    for (int i = 1; i < kPassThreads / 32; ++i) m.x = max(m.x, red[i].x), m.y = max(m.y, red[i].y);
+    __syncthreads();
+    return m;
+}
+
+// Four elements times m into the planes at `hi` (null: not wanted) and, times rel as well, into the row-scaled copy.
+__device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long plane, float4 v, float m, float rel) {
+    uint2 hw, lw;
+    split_pack(v.x * m, v.y * m, hw.x, lw.x);
+    split_pack(v.z * m, v.w * m, hw.y, lw.y);
+    if (hi) *reinterpret_cast<uint2 *>(hi) = hw, *reinterpret_cast<uint2 *>(hi + plane) = lw;
+    if (qs == nullptr) return;
+    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&hw.x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&hw.y));
+    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&lw.x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&lw.y));
+    split_pack((h0.x + l0.x) * rel, (h0.y + l0.y) * rel, hw.x, lw.x);
+    split_pack((h1.x + l1.x) * rel, (h1.y + l1.y) * rel, hw.y, lw.y);
+    *reinterpret_cast<uint2 *>(qs) = hw, *reinterpret_cast<uint2 *>(qs + plane) = lw;
+}
+
+// LP lanes hold a unit of the planes (td columns), NC chunks of four columns each.
+template <int LP, int NC>
+__global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
+    constexpr int NG = kPassThreads / LP, U = kPassUnroll;
+    pdl_wait();
+    pdl_launch();
+    const int blk = (int)blockIdx.x;
+    if (blk >= a.fill_first[0]) {
+        int f = 0;
+        while (f + 1 < a.n_fill && blk >= a.fill_first[f + 1]) ++f;
+        const long long i0 = (long long)(blk - a.fill_first[f]) * kFillPerBlock;
+#pragma unroll
+        for (int k = 0; k < kFillPerBlock / kPassThreads; ++k) {
+            const long long i = i0 + k * kPassThreads + threadIdx.x;
+            if (i < a.fill_n4[f]) a.fill[f][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        return;
+    }
+    __shared__ uint2 red[kPassThreads / 32];
+    const PassUnit w = pass_locate(a, a.n, blk);
+    const PassTensor &t = a.t[w.z];
+    const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
+    const long long plane = (long long)t.batch * t.rows * t.heads * a.td;
+    const int n4 = a.dim >> 2;
+    uint32_t dn = 0u, vn = 0u;
+    if (t.qs) {
+        dn = pass_reduce(t.dn_part + (long long)w.bg * t.dn_slots, t.dn_slots, red).y;
+        vn = t.vn_part ? pass_reduce(t.vn_part + (long long)w.bg * t.vn_slots, t.vn_slots, red).y : t.vn_final[w.bg];
+    }
+    const auto locate = [&](int u, int &r) -> long long {
+        r = u / t.group;
+        return u < w.end ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
+    };
+    const auto row_rel = [&](long long at) -> float {
+        float cq, rel;
+        ds_row_scale(__ldg(t.rnorm + at), dn, vn, cq, rel);
+        return rel;
+    };
+    if (t.x == nullptr) {
+        for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+            uint2 h[U][NC], l[U][NC];
+            long long at[U];
+            float rel[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                int r;
+                at[k] = locate(u0 + k * NG + gi, r);
+                rel[k] = at[k] < 0 ? 1.f : row_rel(at[k]);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const __half *src = t.q_planes + (at[k] < 0 ? 0 : at[k]) * a.td + (li + LP * c) * 4;
+                    h[k][c] = __ldg(reinterpret_cast<const uint2 *>(src));
+                    l[k][c] = __ldg(reinterpret_cast<const uint2 *>(src + plane));
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].y));
+                    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].y));
+                    // (a sum of the two pieces splits into these very pieces again)
+                    if (at[k] >= 0)
+                        store_split4(nullptr, t.qs + at[k] * a.td + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel[k]);
+                }
+        }
+        return;
+    }
+    const uint2 top = pass_reduce(t.part + (long long)w.bg * t.slots, t.slots, red);
+    if (w.slot == 0 && threadIdx.x == 0) {
+        t.amax[w.bg] = top.x;
+        if (t.nmax) t.nmax[w.bg] = top.y;
+    }
+    const float m = block_mult(top.x);
+    if (t.rope == nullptr) {
+        for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+            float4 x[U][NC];
+            long long at[U];
+            float rel[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                int r;
+                at[k] = locate(u0 + k * NG + gi, r);
+                rel[k] = t.qs && at[k] >= 0 ? row_rel(at[k]) : 1.f;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const int ch = li + LP * c;
+                    x[k][c] = (at[k] >= 0 && ch < n4) ? __ldg(reinterpret_cast<const float4 *>(t.x + at[k] * a.dim) + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const long long to = at[k] * a.td + (li + LP * c) * 4;
+                    if (at[k] >= 0) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel[k]);
+                }
+        }
+        return;
+    }
+    // rotated: a lane of the head's lower half takes a chunk and its partner half a head on (a head's halves are
+    // multiples of four wide), so that every element and every table entry is fetched once
+    const int half = a.dim >> 1, h4 = half >> 2;
+    for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            int r;
+            const long long at = locate(u0 + k * NG + gi, r);
+            if (at < 0) break;
+            const float rel = t.qs ? row_rel(at) : 1.f;
+            const auto put = [&](int col, float4 v) {
+                const long long to = at * a.td + col;
+                store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, v, m, rel);
+            };
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int ch = li + LP * c;
+                if (ch < h4) {
+                    const float4 *src = reinterpret_cast<const float4 *>(t.x + at * a.dim);
+                    const float4 lo = __ldg(src + ch), hi = __ldg(src + h4 + ch);
+                    const float4 *cs = reinterpret_cast<const float4 *>(t.rope + (long long)r * half) + 2 * ch;
+                    const float4 p = __ldg(cs), q = __ldg(cs + 1);  // four (cos, sin) pairs
+                    float4 lr, hr;
+                    lr.x = rope_elem(lo.x, hi.x, make_float2(p.x, p.y), false, false), hr.x = rope_elem(hi.x, lo.x, make_float2(p.x, p.y), true, false);
+                    lr.y = rope_elem(lo.y, hi.y, make_float2(p.z, p.w), false, false), hr.y = rope_elem(hi.y, lo.y, make_float2(p.z, p.w), true, false);
+                    lr.z = rope_elem(lo.z, hi.z, make_float2(q.x, q.y), false, false), hr.z = rope_elem(hi.z, lo.z, make_float2(q.x, q.y), true, false);
+                    lr.w = rope_elem(lo.w, hi.w, make_float2(q.z, q.w), false, false), hr.w = rope_elem(hi.w, lo.w, make_float2(q.z, q.w), true, false);
+                    put(ch * 4, lr), put(half + ch * 4, hr);
+                } else if (ch >= n4) {
+                    put(ch * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+                }
+            }
+        }
+    }
+}
+
+// ---- host side --------------------------------------------------------------------------------------
+// Slots of one tensor of `bg` (sequence, group) pairs: what pass_slots() below can ask for.
+inline size_t pass_part_bytes(size_t bg) { return (bg > (size_t)kPassTargetBlocks ? bg : (size_t)kPassTargetBlocks) * sizeof(uint2); }
+
+// Adds a tensor (x or q_planes set by the caller afterwards where they are not plain) to the launch.
+inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, int heads, int group, uint2 *part, uint32_t *amax,
+                            uint32_t *nmax, __half *planes) {
+    PassTensor &t = a.t[a.n++];
+    t = PassTensor{};
+    t.x = x, t.batch = batch, t.rows = rows, t.heads = heads, t.group = group;
+    t.part = part, t.amax = amax, t.nmax = nmax, t.planes = planes;
+    const long long bg = (long long)batch * (heads / group), units = (long long)rows * group;
+    const int lanes = a.dim <= 32 ? 8 : (a.dim <= 64 ? 16 : 32);
+    const long long step = (long long)kPassThreads / lanes * 8;  // eight units a lane group at least
+    long long slots = kPassTargetBlocks / bg;
+    slots = slots > kPassMaxSlots ? kPassMaxSlots : (slots < 1 ? 1 : slots);
+    const long long most = (units + step - 1) / step;
+    if (slots > most) slots = most;
+    long long per = (units + slots - 1) / slots;
+    per = (per + step - 1) / step * step;
+    t.per_block = (int)per;
+    t.slots = (int)((units + per - 1) / per);
+    return t;
+}
+inline void pass_fill(PassArgs &a, float *dst, long long n) {
+    a.fill[a.n_fill] = reinterpret_cast<float4 *>(dst), a.fill_n4[a.n_fill++] = n / 4;
+}
+// Both launches.  The tensors with an f32 source come first in a.t.
+inline int launch_pass(PassArgs &a, cudaStream_t stream) {
+    long long blocks = 0, stats = 0;
+    a.n_stats = 0;
+    for (int i = 0; i < a.n; ++i) {
+        PassTensor &t = a.t[i];
+        t.first = (int)blocks;
+        blocks += (long long)t.batch * (t.heads / t.group) * t.slots;
+        if (t.x) a.n_stats = i + 1, stats = blocks;
+    }
+    a.fill_first[0] = (int)blocks;
+    for (int f = 0; f < a.n_fill; ++f) {
+        blocks += (a.fill_n4[f] + kFillPerBlock - 1) / kFillPerBlock;
+        a.fill_first[f + 1] = (int)blocks;
+    }
+    if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
+    int rc;
+    const dim3 gs((unsigned)stats), gp((unsigned)blocks), th(kPassThreads);
+    constexpr size_t smem = (size_t)kStatsStages * 2 * 2 * kPassThreads * sizeof(float4);
+    const auto stats_launch = [&](auto *kernel) -> int {
+        if (optin_smem((const void *)kernel, smem)) return 1;
+        return launch_pdl("pass_stats_kernel", kernel, gs, th, smem, stream, a);
+    };
+    if (a.dim <= 32) rc = stats_launch(pass_stats_kernel<8, 1>);
+    else if (a.dim <= 64) rc = stats_launch(pass_stats_kernel<16, 1>);
+    else if (a.dim <= 128) rc = stats_launch(pass_stats_kernel<32, 1>);
+    else rc = stats_launch(pass_stats_kernel<32, 2>);
+    if (rc) return rc;
+    if (a.td == 64) return launch_pdl("pass_planes_kernel", pass_planes_kernel<16, 1>, gp, th, 0, stream, a);
+    if (a.td == 128) return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 1>, gp, th, 0, stream, a);
+    return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 2>, gp, th, 0, stream, a);
+}
+
+}  // namespace tcb
+}  // namespace zt

@@ -16,9 +16,8 @@
 // maximum lose relative (not absolute) precision; the parity tests bound the effect.
 //
 // Kernels:
-//   bwd_absmax / bwd_split   per-(sequence, KV group) max |x| of q, k, v, dout; then the h and l
-//                            planes of each tensor ([2][B][T][W] halves) in the workspace.  One
-//                            launch of each for all tensors.
+//   pass_stats / pass_planes (prepass.cuh) per-(sequence, KV group) max |x| of q, k, v, dout, delta and the row
+//                            norms of dout; then the h and l planes of each tensor ([2][B][T][W] halves).
 //   attn_bwd_dkdv_tc         one CTA per (128 keys, KV head, sequence): S^T = K Q^T and
 //                            dP^T = V dO^T per 64-row query tile of every head of the group,
 //                            P^T and dS^T written back to TMEM as packed halves,
@@ -37,6 +36,7 @@
 
 #include <cuda_fp16.h>
 
+#include "prepass.cuh"
 #include "rope_kernels.cuh"
 #include "tc_common.cuh"
 #include "tc_fwd.cuh"
@@ -46,217 +46,6 @@ namespace zt {
 namespace tcb {
 
 using namespace tc;
-
-// ---- scaling --------------------------------------------------------------------------------------
-// The power of two that moves a block's largest magnitude into [2^14, 2^15).  `bits` is the f32
-// bit pattern of max |x| (non-negative, so it orders like an integer).
-__host__ __device__ inline float block_mult(uint32_t bits) {
-    const int ex = (int)((bits >> 23) & 0xff);  // biased exponent: |x| in [2^(ex-127), 2^(ex-126))
-    if (ex == 0 || ex == 0xff) return 1.0f;      // zero/subnormal block, or inf/nan: leave alone
-    int e = 14 - (ex - 127);                     // |x| * 2^e in [2^14, 2^15)
-    if (e > 126) e = 126;
-    if (e < -126) e = -126;
-    uint32_t out = (uint32_t)(e + 127) << 23;
-#if defined(__CUDA_ARCH__)
-    return __uint_as_float(out);
-#else
-    float f;
-    memcpy(&f, &out, 4);
-    return f;
-#endif
-}
-
-// The pre-pass over up to four tensors in one launch each: max |x| per (sequence, column group), then
-// the 16-bit planes.  Tensor z is [batch][T][width] floats; its groups are `cols_per_group` columns wide.
-struct PrepassTensor {
-    const float *x;
-    uint32_t *amax;   // [batch][width / cols_per_group] bit patterns of max |x|, zeroed by the caller
-    __half *planes;   // [2][batch][T][width / src_head * dst_head]
-    int width, cols_per_group;
-    int rows;                // rows of x per sequence that are converted
-    int src_head, dst_head;  // a head's columns in x and in the planes: 32 -> 64 pads each head with zeros
-    const float2 *rope;      // null, or the (cos, sin) table [T][src_head / 2]: x is rotated on its way in
-};
-
-// Four consecutive elements of row r starting at column c of tensor t, rotated if the tensor asks for it.
-// A head's halves are multiples of four wide, so the four partners are one float4 too.
-__device__ __forceinline__ float4 prepass_load(const PrepassTensor &t, const float4 *row4, int r, int c) {
-    const float4 v = __ldg(row4 + c / 4);
-    if (t.rope == nullptr) return v;
-    const int half = t.src_head / 2;
-    const int w = c % t.src_head;
-    const bool upper = w >= half;
-    const float4 o = __ldg(row4 + (upper ? c - half : c + half) / 4);
-    const float4 *cs = reinterpret_cast<const float4 *>(t.rope + (long long)r * half + (upper ? w - half : w));
-    const float4 a = __ldg(cs), b = __ldg(cs + 1);  // four (cos, sin) pairs
-    float4 out;
-    out.x = rope_elem(v.x, o.x, make_float2(a.x, a.y), upper, false), out.y = rope_elem(v.y, o.y, make_float2(a.z, a.w), upper, false);
-    out.z = rope_elem(v.z, o.z, make_float2(b.x, b.y), upper, false), out.w = rope_elem(v.w, o.w, make_float2(b.z, b.w), upper, false);
-    return out;
-}
-struct PrepassArgs {
-    PrepassTensor t[4];
-    int n, batch;
-};
-constexpr int kPrepassRows = 32;      // rows of one sequence per absmax CTA
-constexpr int kPrepassMaxGroups = 256;
-
-// grid (ceil(T / kPrepassRows), batch, n tensors).  A thread keeps to its columns, so its group is fixed
-// and the row loop is nothing but independent loads.
-__global__ void __launch_bounds__(256) bwd_absmax_kernel(const PrepassArgs a) {
-    __shared__ uint32_t gmax[kPrepassMaxGroups];
-    const PrepassTensor t = a.t[blockIdx.z];
-    const int b = blockIdx.y, r0 = blockIdx.x * kPrepassRows;
-    const int w4 = t.width / 4, n_groups = t.width / t.cols_per_group;
-    for (int i = threadIdx.x; i < n_groups; i += 256) gmax[i] = 0u;
-    __syncthreads();
-    if (r0 >= t.rows) return;
-    const int r1 = min(r0 + kPrepassRows, t.rows);
-    const float4 *base = reinterpret_cast<const float4 *>(t.x + (long long)b * t.rows * t.width);
-    for (int c4 = threadIdx.x; c4 < w4; c4 += 256) {
-        float m = 0.f;
-#pragma unroll 8
-        for (int r = r0; r < r1; ++r) {
-            // (a tensor that will be rotated is measured unrotated: a rotated pair is at most sqrt(2) times its
-            // larger element, and the scale leaves a factor of two below the f16 range)
-            const float4 v = __ldg(base + (long long)r * w4 + c4);
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        }
-        atomicMax(&gmax[(c4 * 4) / t.cols_per_group], __float_as_uint(m));
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_groups; i += 256)
-        if (gmax[i]) atomicMax(t.amax + b * n_groups + i, gmax[i]);
-}
-
-// x -> planes h = f16(x m), l = f16(x m - h).  grid (ceil(T width / 4 / 2048), batch, n tensors): a CTA
-// converts 2048 consecutive float4 of one sequence, eight per thread.
-constexpr int kSplitPerCta = 2048;
-__global__ void __launch_bounds__(256) bwd_split_kernel(const PrepassArgs a) {
-    const PrepassTensor t = a.t[blockIdx.z];
-    const int b = blockIdx.y;
-    const int n_groups = t.width / t.cols_per_group;
-    if (t.src_head != t.dst_head) {
-        // zero-padded heads: walk the planes' float4s, fetch the source's where there is one
-        const int w4s = t.width / 4, w4d = t.width / t.src_head * t.dst_head / 4;
-        const long long seq4d = (long long)t.rows * w4d;
-        const long long first = (long long)blockIdx.x * kSplitPerCta;
-        if (first >= seq4d) return;
-        const float4 *src = reinterpret_cast<const float4 *>(t.x) + (long long)b * t.rows * w4s;
-        uint2 *hp = reinterpret_cast<uint2 *>(t.planes) + b * seq4d;
-        uint2 *lp = hp + (long long)a.batch * seq4d;
-        const uint32_t *amax = t.amax + b * n_groups;
-#pragma unroll
-        for (int k = 0; k < kSplitPerCta / 256; ++k) {
-            const long long i = first + k * 256 + threadIdx.x;
-            if (i >= seq4d) break;
-            const int r = (int)(i / w4d);
-            const int cd = (int)(i - (long long)r * w4d) * 4;      // column in the planes
-            const int head = cd / t.dst_head, within = cd - head * t.dst_head;
-            uint2 hw = make_uint2(0u, 0u), lw = make_uint2(0u, 0u);
-            if (within < t.src_head) {
-                const int cs = head * t.src_head + within;          // column in x
-                const float m = block_mult(amax[cs / t.cols_per_group]);
-                const float4 v = prepass_load(t, src + (long long)r * w4s, r, cs);
-                const float s[4] = {v.x * m, v.y * m, v.z * m, v.w * m};
-                __half h[4], l[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    h[e] = __float2half_rn(s[e]);
-                    l[e] = __float2half_rn(s[e] - __half2float(h[e]));
-                }
-                hw = *reinterpret_cast<const uint2 *>(h), lw = *reinterpret_cast<const uint2 *>(l);
-            }
-            hp[i] = hw, lp[i] = lw;
-        }
-        return;
-    }
-    const int w4 = t.width / 4;
-    const long long seq4 = (long long)t.rows * w4;  // float4 per sequence
-    const long long first = (long long)blockIdx.x * kSplitPerCta;
-    if (first >= seq4) return;
-    const float4 *src = reinterpret_cast<const float4 *>(t.x) + b * seq4;
-    uint2 *hp = reinterpret_cast<uint2 *>(t.planes) + b * seq4;
-    uint2 *lp = hp + (long long)a.batch * seq4;
-    const uint32_t *amax = t.amax + b * n_groups;
-    const unsigned col0 = (unsigned)(first % w4);
-#pragma unroll
-    for (int k = 0; k < kSplitPerCta / 256; ++k) {
-        const int o = k * 256 + threadIdx.x;
-        const long long i = first + o;
-        if (i >= seq4) break;
-        const unsigned c4 = (col0 + (unsigned)o) % (unsigned)w4;
-        const float m = block_mult(amax[(c4 * 4u) / (unsigned)t.cols_per_group]);
-        const float4 v = t.rope ? prepass_load(t, src + (i - c4), (int)((i - c4) / w4), (int)(c4 * 4u)) : __ldg(src + i);
-        const float s[4] = {v.x * m, v.y * m, v.z * m, v.w * m};
-        __half h[4], l[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            h[e] = __float2half_rn(s[e]);
-            l[e] = __float2half_rn(s[e] - __half2float(h[e]));
-        }
-        hp[i] = *reinterpret_cast<const uint2 *>(h);
-        lp[i] = *reinterpret_cast<const uint2 *>(l);
-    }
-}
-
-// Both passes for the tensors in `a` (amax already zeroed).
-inline int launch_prepass(const PrepassArgs &a, cudaStream_t stream) {
-    int rows = 0;
-    long long seq4 = 0;
-    for (int i = 0; i < a.n; ++i) {
-        const long long s4 = (long long)a.t[i].rows * (a.t[i].width / a.t[i].src_head * a.t[i].dst_head / 4);
-        seq4 = s4 > seq4 ? s4 : seq4;
-        rows = a.t[i].rows > rows ? a.t[i].rows : rows;
-    }
-    const dim3 ga((unsigned)((rows + kPrepassRows - 1) / kPrepassRows), (unsigned)a.batch, (unsigned)a.n);
-    if (ZT_LAUNCH("bwd_absmax_kernel", stream, (bwd_absmax_kernel<<<ga, 256, 0, stream>>>(a)))) return 1;
-    const dim3 gs((unsigned)((seq4 + kSplitPerCta - 1) / kSplitPerCta), (unsigned)a.batch, (unsigned)a.n);
-    return ZT_LAUNCH("bwd_split_kernel", stream, (bwd_split_kernel<<<gs, 256, 0, stream>>>(a)));
-}
-
-// max over the rows s of |v[b, s, kv, :]| (Euclidean), per (sequence, KV head).  grid (ceil(T / 256), n_kv_heads,
-// batch), 8 warps; a warp walks 32 rows of the block's 256 and keeps a running maximum, the block then makes ONE
-// atomic: thousands of atomics on the same word serialise in L2 (a warp per row took 0.2 ms at the headline shape).
-// vnmax holds f32 bit patterns (non-negative, so they order like integers), zeroed by the caller.
-__global__ void __launch_bounds__(256) bwd_vnorm_kernel(const float *__restrict__ v, uint32_t *__restrict__ vnmax,
-                                                        int T, int n_kv_heads, int dim) {
-    __shared__ float wmax[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kv = blockIdx.y, b = blockIdx.z;
-    const int r0 = blockIdx.x * 256 + warp * 32;
-    float best = 0.f;
-    for (int r = r0; r < r0 + 32 && r < T; ++r) {
-        const float *x = v + (((long long)b * T + r) * n_kv_heads + kv) * dim;
-        float acc = 0.f;
-        for (int j = lane; j < dim; j += 32) {
-            const float e = __ldg(x + j);
-            acc = fmaf(e, e, acc);
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        best = fmaxf(best, acc);
-    }
-    if (lane == 0) wmax[warp] = best;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float m = wmax[0];
-        for (int i = 1; i < 8; ++i) m = fmaxf(m, wmax[i]);
-        // (an Inf or NaN row: sqrt keeps it, and the scale built from it falls back to 1)
-        atomicMax(vnmax + b * n_kv_heads + kv, __float_as_uint(sqrtf(m)));
-    }
-}
-
-__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
-    const __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t *>(&h);
-}
-// (a, b) -> packed h pair and packed l pair: one paired conversion each way instead of two single ones
-__device__ __forceinline__ void split_pack(float a, float b, uint32_t &hw, uint32_t &lw) {
-    const __half2 hh = __floats2half2_rn(a, b);
-    const float2 back = __half22float2(hh);
-    hw = *reinterpret_cast<const uint32_t *>(&hh);
-    lw = pack_half2(a - back.x, b - back.y);
-}
 
 __device__ __forceinline__ void red_add_v4(float *addr, float4 v) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
@@ -269,7 +58,7 @@ struct BwdParams {
     const __half *k_planes, *v_planes;   // dkdv kernel: the hi planes of K and V are read straight into TMEM
     const __half *q_planes, *do_planes;  // dq kernel: Q, dO planes read straight into TMEM
     const uint32_t *amax_q, *amax_k, *amax_v, *amax_do;  // [B, Hkv] bit patterns of max |x|
-    const float *rnorm;      // [B, T, H] Euclidean norm of each row of dout (bwd_rownorm_kernel)
+    const float *rnorm;      // [B, T, H] Euclidean norm of each row of dout (pass_stats_kernel)
     const uint32_t *vnmax;   // [B, Hkv] bit pattern of the largest Euclidean norm of a row of v
     uint32_t *dsmax;         // [B, Hkv] bit pattern of max |dS| (true units): written by the dQ kernel, read by dK/dV;
                              // for the fused kernel the same words hold the largest row norm of dout instead
@@ -296,16 +85,6 @@ struct BwdParams {
 //    bounded: the dQ kernel, which runs first, records the largest |dS| it formed in each (sequence, KV group),
 //    and the dK/dV kernel places that value an eighth below the top of the range (its own dS differs from the
 //    dQ kernel's by rounding only).
-// pow2_below_top(x, top): the power of two c with x c in [2^(top-1), 2^top); 1 when x is zero or not finite.
-__device__ __forceinline__ float pow2_for(float x, int top) {
-    if (!(x > 0.f) || !(x < 3.0e38f)) return 1.0f;
-    int e;
-    frexpf(x, &e);  // x = m 2^e, m in [0.5, 1)
-    int k = top - e;
-    k = k > 120 ? 120 : (k < -120 ? -120 : k);
-    return __uint_as_float((uint32_t)(k + 127) << 23);
-}
-
 // The dK/dV kernel's walk over (query tile, head of the group), and where its TMEM accumulators
 // are flushed to memory.
 //
@@ -1254,13 +1033,13 @@ struct BwdWorkspace {
     __half *q_planes, *do_planes, *k_planes, *v_planes;
     float *rnorm;  // [batch, T, n_heads]
     __half *qs_planes;  // the row-scaled copy of q's planes (the fused and the wide-head backward read it for dK)
-    size_t total_bytes, amax_bytes;
+    uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
+    size_t total_bytes;
 };
 
 inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim) {
     BwdWorkspace w{};
     const size_t n_amax = (size_t)batch * n_kv_heads;
-    w.amax_bytes = (6 * n_amax * sizeof(uint32_t) + 1023) / 1024 * 1024;
     const size_t qh = (size_t)2 * batch * T * n_heads * dim * sizeof(__half);
     const size_t kh = (size_t)2 * batch * T * n_kv_heads * dim * sizeof(__half);
     auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
@@ -1268,7 +1047,8 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
     w.amax_q = reinterpret_cast<uint32_t *>(c);
     w.amax_k = w.amax_q + n_amax, w.amax_v = w.amax_k + n_amax, w.amax_do = w.amax_v + n_amax;
     w.vnmax = w.amax_do + n_amax, w.dsmax = w.vnmax + n_amax;
-    size_t off = w.amax_bytes;
+    size_t off = up(6 * n_amax * sizeof(uint32_t));
+    for (int i = 0; i < 4; ++i) w.part[i] = reinterpret_cast<uint2 *>(c + off), off += up(pass_part_bytes(n_amax));
     w.q_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.do_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.k_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
@@ -1277,6 +1057,20 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
     w.qs_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.total_bytes = off;
     return w;
+}
+
+// The pre-pass of a backward: a.t[0] is dout and, unless their planes were kept, a.t[1 .. 3] are q, k, v.  want_qs: the
+// row-scaled copy of q's planes, want_q: q's planes themselves.
+inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs, bool want_q, bool kept, cudaStream_t stream) {
+    if (!kept && !want_q) a.t[1].planes = nullptr;
+    if (want_qs) {
+        const PassTensor &g = a.t[0];
+        PassTensor &t = kept ? pass_add(a, nullptr, g.batch, g.rows, g.heads, g.group, nullptr, nullptr, nullptr, nullptr) : a.t[1];
+        t.qs = w.qs_planes, t.rnorm = w.rnorm, t.dn_part = g.part, t.dn_slots = g.slots;
+        if (kept) t.q_planes = w.q_planes, t.vn_final = w.vnmax;
+        else t.vn_part = a.t[3].part, t.vn_slots = a.t[3].slots;
+    }
+    return launch_pass(a, stream);
 }
 
 inline bool tc_bwd_supported(int batch, int T, int dim, const void *q, const void *k, const void *v,

@@ -22,7 +22,7 @@
 // with A in TMEM every 52 clocks where two threads together reach the pipe's 32.
 //  * the scale of dS: no dQ kernel runs first to measure the largest |dS| of a KV group.  dS is scaled per
 //    query row (column of dS^T), as the dQ kernel did, and the row's factor is moved onto Q for dK: the Q tiles
-//    this kernel reads are the row-scaled copy (tc_bwd_wide.cuh: wide_qscaled_kernel), row t divided by a power
+//    this kernel reads are the row-scaled copy (prepass.cuh), row t divided by a power
 //    of two rel(t) in [1, 2^12].  S^T = K Q~^T is multiplied back per column by the row threads (exact), dK is
 //    sum_t (dS cq(t)) (Q / rel(t)) with one scale, dQ^T's column t leaves times 1 / cq(t).
 #pragma once
@@ -34,8 +34,6 @@ namespace tcf {
 
 using namespace tc;
 using namespace tcb;
-using tcw::wide_group_scale;
-using tcw::wide_row_scale;
 
 struct FusedShared {
     uint64_t full_q[2], free_q[2], full_g, free_g;
@@ -114,12 +112,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     const int bg = b * p.n_kv_heads + g;
     const float mq = block_mult(p.amax_q[bg]), mk = block_mult(p.amax_k[bg]);
     const float mv = block_mult(p.amax_v[bg]), mdo = block_mult(p.amax_do[bg]);
     const uint32_t rn_bits = p.dsmax[bg], vn_bits = p.vnmax[bg];  // (the header's last array holds max |dout row| here)
-    const float cmin = wide_group_scale(rn_bits, vn_bits);
+    const float cmin = ds_group_scale(rn_bits, vn_bits);
 
     if (warp == kKvRowWarps) {
         // ------------------------------------------------------------------ TMA producer
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             const long long idx = ((long long)b * p.T + t) * p.n_heads + g * group + w.hh;
             if (set == 0) return __ldg(p.lse + idx) * kLog2e - lse_shift;
             float cq, rel;
-            wide_row_scale(__ldg(p.rnorm + idx), rn_bits, vn_bits, cq, rel);
+            ds_row_scale(__ldg(p.rnorm + idx), rn_bits, vn_bits, cq, rel);
             if (set == 1) return ZT_DEFECT(13) ? 0.f : __ldg(p.delta + idx) * cq / p.p_scale;
             if (set == 2) return cs_over_cmin * cq;
             return cq * inv_dov;
@@ -621,7 +621,7 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     if (optin_smem((const void *)attn_bwd_fused_tc<D>, smem)) return 1;
     const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
-    return ZT_LAUNCH("attn_bwd_fused_tc", stream, (attn_bwd_fused_tc<D><<<grid, kFusedThreads, smem, stream>>>(k128, v128, qs64, g64, p)));
+    return launch_pdl("attn_bwd_fused_tc", attn_bwd_fused_tc<D>, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
 }
 inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
                             const BwdParams &p, cudaStream_t stream) {
@@ -639,10 +639,11 @@ inline bool tc_bwd_takes_fused(int dim, bool two_kernels, const PeerList *dq_pee
     return (td == 64 || td == 128) && !two_kernels && !(dq_peers && dq_peers->n > 0);
 }
 
-// delta and the row norms of dout (workspace rnorm) must already be there.  dq, dk, dv are assigned.
+// delta (= sum_j dout out, per row) is formed here; dq, dk, dv are assigned.  `out` may alias dq: it has been read when
+// dq is first written.
 // rope_t: only with the two-kernel form (the fused kernel's dq takes its rotation in a pass of its own, by the caller).
-inline int launch_bwd_tc(const float *q, const float *k, const float *v, const float *dout, const float *lse,
-                         const float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
+inline int launch_bwd_tc(const float *q, const float *k, const float *v, const float *out, const float *dout,
+                         const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
                          int n_heads, int n_kv_heads, int dim, cudaStream_t stream, const float2 *rope = nullptr,
                          const float2 *rope_t = nullptr, bool qkv_planes_kept = false, const PeerList *dq_peers = nullptr,
                          bool two_kernels = false) {
@@ -652,45 +653,28 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     if (fused && rope_t) return refuse("internal: the fused backward does not rotate dq.");
     const BwdWorkspace w = bwd_workspace(workspace, batch, T, n_heads, n_kv_heads, td);
     const int group = n_heads / n_kv_heads;
-    const int wq_src = n_heads * dim, wkv_src = n_kv_heads * dim;
     const int wq = n_heads * td, wkv = n_kv_heads * td;
-    // With the planes of q, k, v kept by the forward (and their maxima beside them), only dout is converted.
+    // With the planes of q, k, v kept by the forward (their maxima and v's largest row norm beside them), only dout is
+    // converted.  The header's last array holds the largest row norm of dout for the fused kernel, max |dS| (which its
+    // dQ kernel finds) for the two kernels.
     const size_t n_amax = (size_t)batch * n_kv_heads;
-    // (with kept planes the maxima of q, k, v stay; those of dout, the row norms of v and the header's last array --
-    // max |dS| for the two kernels, the largest row norm of dout for the fused one -- start from zero)
-    if (cudaMemsetAsync(qkv_planes_kept ? w.amax_do : w.amax_q, 0,
-                        qkv_planes_kept ? 3 * n_amax * sizeof(uint32_t) : w.amax_bytes, stream) != cudaSuccess ||
-        (fused && cudaMemsetAsync(dq, 0, (size_t)batch * T * wq_src * sizeof(float), stream) != cudaSuccess)) {
+    if (!fused && cudaMemsetAsync(w.dsmax, 0, n_amax * sizeof(uint32_t), stream) != cudaSuccess) {
         cudaGetLastError();
         return refuse("could not clear the backward workspace header");
     }
-    PrepassArgs pa{};
-    pa.batch = batch;
-    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, T, dim, td, nullptr};
-    pa.n = 1;
-    if (!qkv_planes_kept) {
-        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, rope};
-        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, T, dim, td, rope};
-        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, T, dim, td, nullptr};
-        pa.n = 4;
-    }
-    if (launch_prepass(pa, stream)) return 1;
+    PassArgs pa{};
+    pa.dim = dim, pa.td = td;
     {
-        const dim3 gv((unsigned)((T + 255) / 256), (unsigned)n_kv_heads, (unsigned)batch);
-        if (ZT_LAUNCH("bwd_vnorm_kernel", stream, (bwd_vnorm_kernel<<<gv, 256, 0, stream>>>(v, w.vnmax, T, n_kv_heads, dim))))
-            return 1;
+        PassTensor &t = pass_add(pa, dout, batch, T, n_heads, group, w.part[3], w.amax_do, fused ? w.dsmax : nullptr, w.do_planes);
+        t.o = out, t.delta = delta, t.rnorm = w.rnorm;
     }
-    if (fused) {
-        // the largest row norm of dout per KV group, then Q's planes with every row divided by its share of the scale of dS
-        const dim3 gr((unsigned)((T + 63) / 64), (unsigned)batch);
-        if (ZT_LAUNCH("wide_rnmax_kernel", stream, (tcw::wide_rnmax_kernel<<<gr, 256, 0, stream>>>(w.rnorm, w.dsmax, T, n_heads, n_kv_heads))))
-            return 1;
-        const long long n8 = (long long)batch * T * wq / 8;
-        if (ZT_LAUNCH("wide_qscaled_kernel", stream,
-                      (tcw::wide_qscaled_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(w.q_planes, w.qs_planes, w.rnorm, w.dsmax,
-                                                                                                  w.vnmax, batch, T, n_heads, n_kv_heads, td))))
-            return 1;
+    if (!qkv_planes_kept) {
+        pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
+        pass_add(pa, k, batch, T, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
+        pass_add(pa, v, batch, T, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     }
+    if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
+    if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
     BwdMaps m;
     if (!make_half_tile_map(&m.k128, w.k_planes, 2 * batch, T, wkv, td, 128) ||
         !make_half_tile_map(&m.v128, w.v_planes, 2 * batch, T, wkv, td, 128) ||

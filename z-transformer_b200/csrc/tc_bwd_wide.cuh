@@ -36,6 +36,8 @@ namespace tcw {
 using namespace tc;
 using tcb::block_mult;
 using tcb::kDsBound;
+using tcb::ds_group_scale;
+using tcb::ds_row_scale;
 using tcb::pow2_for;
 using tcb::split_pack;
 
@@ -45,7 +47,6 @@ constexpr int kSB = 4 * kTB;       // a stage: A hi, A lo, B hi, B lo
 constexpr int kScoreThreads = 10 * 32;  // TMA producer, MMA issuer, eight epilogue warps
 constexpr int kTriThreads = 6 * 32;     // TMA producer, MMA issuer, four epilogue warps
 constexpr int kPiece = 1024;            // contraction depth of one CTA of gemm_tri
-constexpr float kRowBoostMax = 4096.f;  // a row's scale is at most this many times the group's smallest
 
 struct WideShared {
     uint64_t full[kStages], freed[kStages], all_done, staged;
@@ -77,68 +78,6 @@ struct WideParams {
     int which;                         // gemm_tri<1>: 0 dK (dS and the row-scaled Q), 1 dV (P and dO)
     float scale, scale_log2, p_scale;
 };
-
-// Row t's scale of dS (cq) and what divides row t of the second copy of Q (1 / rel): both powers of two.
-__device__ __forceinline__ float wide_group_scale(uint32_t rnmax_bits, uint32_t vnmax_bits) {
-    return pow2_for(2.02f * __uint_as_float(rnmax_bits) * __uint_as_float(vnmax_bits), 14);
-}
-__device__ __forceinline__ void wide_row_scale(float rnorm_t, uint32_t rnmax_bits, uint32_t vnmax_bits, float &cq, float &rel) {
-    const float cmin = wide_group_scale(rnmax_bits, vnmax_bits);
-    const float x = 2.02f * rnorm_t * __uint_as_float(vnmax_bits);
-    float c = (x > 0.f && x < 3.0e38f) ? pow2_for(x, 14) : cmin;
-    c = fminf(fmaxf(c, cmin), cmin * kRowBoostMax);
-    if (!(c < 3.0e38f)) c = cmin;
-    cq = c;
-    rel = cmin / c;
-}
-
-// rnmax[b, g] = the largest row norm of dout over the rows and the heads of KV group g.  grid (ceil(T / 64), B).
-__global__ void __launch_bounds__(256) wide_rnmax_kernel(const float *__restrict__ rnorm, uint32_t *__restrict__ rnmax,
-                                                         int T, int n_heads, int n_kv_heads) {
-    __shared__ uint32_t gmax[tcb::kPrepassMaxGroups];
-    const int b = blockIdx.y, group = n_heads / n_kv_heads;
-    for (int i = threadIdx.x; i < n_kv_heads; i += 256) gmax[i] = 0u;
-    __syncthreads();
-    const long long r0 = (long long)blockIdx.x * 64, r1 = r0 + 64 < T ? r0 + 64 : T;
-    const long long n = (r1 - r0) * n_heads;
-    const float *base = rnorm + ((long long)b * T + r0) * n_heads;
-    for (long long i = threadIdx.x; i < n; i += 256) {
-        const float x = __ldg(base + i);
-        if (x > 0.f) atomicMax(&gmax[(int)(i % n_heads) / group], __float_as_uint(x));
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_kv_heads; i += 256)
-        if (gmax[i]) atomicMax(rnmax + b * n_kv_heads + i, gmax[i]);
-}
-
-// The second copy of Q's planes: row t of head h times rel(t, h).  A thread converts eight elements.
-__global__ void __launch_bounds__(256) wide_qscaled_kernel(const __half *__restrict__ q_planes, __half *__restrict__ qs_planes,
-                                                           const float *__restrict__ rnorm, const uint32_t *__restrict__ rnmax,
-                                                           const uint32_t *__restrict__ vnmax, int batch, int T, int n_heads,
-                                                           int n_kv_heads, int td) {
-    const long long per_plane = (long long)batch * T * n_heads * td;
-    const long long i8 = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (i8 * 8 >= per_plane) return;
-    const long long e = i8 * 8;
-    const long long rowhead = e / td;  // (b * T + t) * n_heads + h
-    const int h = (int)(rowhead % n_heads);
-    const int b = (int)(rowhead / ((long long)T * n_heads));
-    const int g = h / (n_heads / n_kv_heads);
-    float cq, rel;
-    wide_row_scale(__ldg(rnorm + rowhead), rnmax[b * n_kv_heads + g], vnmax[b * n_kv_heads + g], cq, rel);
-    const uint4 hw = __ldg(reinterpret_cast<const uint4 *>(q_planes + e));
-    const uint4 lw = __ldg(reinterpret_cast<const uint4 *>(q_planes + per_plane + e));
-    const uint32_t hs[4] = {hw.x, hw.y, hw.z, hw.w}, ls[4] = {lw.x, lw.y, lw.z, lw.w};
-    uint32_t ho[4], lo[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&hs[j]));
-        const float2 c = __half22float2(*reinterpret_cast<const __half2 *>(&ls[j]));
-        split_pack((a.x + c.x) * rel, (a.y + c.y) * rel, ho[j], lo[j]);
-    }
-    *reinterpret_cast<uint4 *>(qs_planes + e) = make_uint4(ho[0], ho[1], ho[2], ho[3]);
-    *reinterpret_cast<uint4 *>(qs_planes + per_plane + e) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-}
 
 // ---------------------------------------------------------------------------------------------------
 // P and dS of one 128 x 128 tile.  grid (tiles at or below the diagonal, units of the chunk), 320 threads.
@@ -177,6 +116,8 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -243,7 +184,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]), mdo = block_mult(p.amax_do[b * p.n_kv_heads + g]);
         const long long ridx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + h;
         float cq = 1.f, rel = 1.f;
-        if (t < p.T) wide_row_scale(__ldg(p.rnorm + ridx), p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g], cq, rel);
+        if (t < p.T) ds_row_scale(__ldg(p.rnorm + ridx), p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g], cq, rel);
         const float cs = p.scale_log2 / (mq * mk);
         // P leaves times p_scale: the factor rides in the exponent
         const float lse2 = (t < p.T) ? __ldg(p.lse + ridx) * kLog2e - log2f(p.p_scale) : 0.f;
@@ -412,6 +353,8 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -526,7 +469,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         const float mv = block_mult(p.amax_v[bg]), mdo = block_mult(p.amax_do[bg]);
         const long long ridx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + h;
         float cq = 1.f, rel = 1.f;
-        if (t < p.T) wide_row_scale(__ldg(p.rnorm + ridx), p.rnmax[bg], p.vnmax[bg], cq, rel);
+        if (t < p.T) ds_row_scale(__ldg(p.rnorm + ridx), p.rnmax[bg], p.vnmax[bg], cq, rel);
         const float cs = p.scale_log2 / (mq * mk);
         const float lse2 = (t < p.T) ? __ldg(p.lse + ridx) * kLog2e - log2f(p.p_scale) : 0.f;
         const float c1 = cq / (mdo * mv * p.p_scale);
@@ -641,7 +584,10 @@ __global__ void __launch_bounds__(kTriThreads, 1)
         if (k_begin < m0) k_begin = m0;
     }
     if (k_end > p.Tp) k_end = p.Tp;
-    if (k_begin >= k_end || m0 >= p.T) return;  // (the whole CTA: nothing has been set up yet)
+    if (k_begin >= k_end || m0 >= p.T) {  // (the whole CTA: nothing has been set up yet)
+        pdl_wait();
+        return;
+    }
     const int n_steps = (k_end - k_begin) / 64;
 
     if (threadIdx.x == 0) {
@@ -657,6 +603,8 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -726,11 +674,11 @@ __global__ void __launch_bounds__(kTriThreads, 1)
         if (MODE == 0) {
             float cq = 1.f, rel = 1.f;
             if (t < p.T)
-                wide_row_scale(__ldg(p.rnorm + ((long long)b * p.T + t) * p.n_heads + h), p.rnmax[b * p.n_kv_heads + g],
+                ds_row_scale(__ldg(p.rnorm + ((long long)b * p.T + t) * p.n_heads + h), p.rnmax[b * p.n_kv_heads + g],
                                p.vnmax[b * p.n_kv_heads + g], cq, rel);
             f = p.scale / (cq * block_mult(p.amax_k[b * p.n_kv_heads + g]));
         } else if (p.which == 0) {
-            f = p.scale / (wide_group_scale(p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g]) *
+            f = p.scale / (ds_group_scale(p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g]) *
                            block_mult(p.amax_q[b * p.n_kv_heads + g]));
         } else {
             f = 1.0f / (p.p_scale * block_mult(p.amax_do[b * p.n_kv_heads + g]));
@@ -839,9 +787,10 @@ inline size_t tc_bwd_wide_workspace_bytes(int batch, int T, int n_heads, int n_k
     return tcw::wide_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).total_bytes;
 }
 
-// delta and the row norms of dout (workspace .base.rnorm) must already be there.  dq, dk, dv are assigned.
-inline int launch_bwd_wide(const float *q, const float *k, const float *v, const float *dout, const float *lse,
-                           const float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
+// delta (= sum_j dout out, per row) is formed here; dq, dk, dv are assigned.  `out` may alias dq: it has been read when
+// dq is first written.
+inline int launch_bwd_wide(const float *q, const float *k, const float *v, const float *out, const float *dout,
+                           const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
                            int n_heads, int n_kv_heads, int dim, cudaStream_t stream, bool qkv_planes_kept = false,
                            bool tile_scores = false) {
     using namespace tcb;
@@ -850,44 +799,23 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     const WideWorkspace ww = wide_workspace(workspace, batch, T, n_heads, n_kv_heads, td);
     const BwdWorkspace &w = ww.base;
     const int group = n_heads / n_kv_heads;
-    const int wq_src = n_heads * dim, wkv_src = n_kv_heads * dim;
     const int wq = n_heads * td, wkv = n_kv_heads * td;
-    const size_t n_amax = (size_t)batch * n_kv_heads;
-    // (with kept planes the maxima of q, k, v stay; those of dout and the two norms start from zero.  The header's
-    // last array holds the largest row norm of dout here.)
-    if (cudaMemsetAsync(qkv_planes_kept ? w.amax_do : w.amax_q, 0,
-                        qkv_planes_kept ? 3 * n_amax * sizeof(uint32_t) : w.amax_bytes, stream) != cudaSuccess ||
-        cudaMemsetAsync(dq, 0, (size_t)batch * T * wq_src * sizeof(float), stream) != cudaSuccess ||
-        cudaMemsetAsync(dk, 0, (size_t)batch * T * wkv_src * sizeof(float), stream) != cudaSuccess ||
-        cudaMemsetAsync(dv, 0, (size_t)batch * T * wkv_src * sizeof(float), stream) != cudaSuccess) {
-        cudaGetLastError();
-        return refuse("could not clear the backward's outputs and workspace header");
-    }
-    PrepassArgs pa{};
-    pa.batch = batch;
-    pa.t[0] = {dout, w.amax_do, w.do_planes, wq_src, group * dim, T, dim, td, nullptr};
-    pa.n = 1;
-    if (!qkv_planes_kept) {
-        pa.t[1] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, nullptr};
-        pa.t[2] = {k, w.amax_k, w.k_planes, wkv_src, dim, T, dim, td, nullptr};
-        pa.t[3] = {v, w.amax_v, w.v_planes, wkv_src, dim, T, dim, td, nullptr};
-        pa.n = 4;
-    }
-    if (launch_prepass(pa, stream)) return 1;
-    uint32_t *rnmax = w.dsmax;
+    PassArgs pa{};
+    pa.dim = dim, pa.td = td;
+    uint32_t *rnmax = w.dsmax;  // (the header's last array)
     {
-        const dim3 gv((unsigned)((T + 255) / 256), (unsigned)n_kv_heads, (unsigned)batch);
-        if (ZT_LAUNCH("bwd_vnorm_kernel", stream, (bwd_vnorm_kernel<<<gv, 256, 0, stream>>>(v, w.vnmax, T, n_kv_heads, dim))))
-            return 1;
-        const dim3 gr((unsigned)((T + 63) / 64), (unsigned)batch);
-        if (ZT_LAUNCH("wide_rnmax_kernel", stream, (wide_rnmax_kernel<<<gr, 256, 0, stream>>>(w.rnorm, rnmax, T, n_heads, n_kv_heads))))
-            return 1;
-        const long long n8 = (long long)batch * T * wq / 8;
-        if (ZT_LAUNCH("wide_qscaled_kernel", stream,
-                      (wide_qscaled_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(w.q_planes, w.qs_planes, w.rnorm, rnmax,
-                                                                                             w.vnmax, batch, T, n_heads, n_kv_heads, td))))
-            return 1;
+        PassTensor &t = pass_add(pa, dout, batch, T, n_heads, group, w.part[3], w.amax_do, rnmax, w.do_planes);
+        t.o = out, t.delta = delta, t.rnorm = w.rnorm;
     }
+    if (!qkv_planes_kept) {
+        pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes);
+        pass_add(pa, k, batch, T, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes);
+        pass_add(pa, v, batch, T, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
+    }
+    pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
+    pass_fill(pa, dk, (long long)batch * T * n_kv_heads * dim);
+    pass_fill(pa, dv, (long long)batch * T * n_kv_heads * dim);
+    if (launch_pass_backward(pa, w, true, true, qkv_planes_kept, stream)) return 1;
     const int Tp = ww.Tp, cap = ww.unit_cap;
     CUtensorMap q_k, k_k, g_k, v_k;      // K-major 128-row tiles of one 64-column block: the scores' operands
     CUtensorMap k_n, qs_n, g_n;          // N-major tiles (64 contraction rows x the head's 256 columns): B of the three products
@@ -927,22 +855,19 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         p.unit0 = unit0;
         if (tile_scores) {
             const dim3 gs((unsigned)(nt * (nt + 1) / 2), (unsigned)units);
-            if (ZT_LAUNCH("bwd_wide_scores", stream, (bwd_wide_scores<<<gs, kScoreThreads, smem, stream>>>(q_k, k_k, g_k, v_k, p))))
-                return 1;
+            if (launch_pdl("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
         } else {
             const dim3 gs((unsigned)units, (unsigned)nt);
-            if (ZT_LAUNCH("bwd_wide_scores_res", stream,
-                          (bwd_wide_scores_res<<<gs, kScoreThreads, smem_r, stream>>>(q_k, k_k, g_k, v_k, p))))
-                return 1;
+            if (launch_pdl("bwd_wide_scores_res", bwd_wide_scores_res, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
         }
         p.out = dq, p.which = 0;
         const dim3 gq((unsigned)nt, (unsigned)(units * p.pieces));
-        if (ZT_LAUNCH("gemm_tri_dq", stream, (gemm_tri<0><<<gq, kTriThreads, smem_t, stream>>>(ds_k, k_n, p)))) return 1;
+        if (launch_pdl("gemm_tri_dq", gemm_tri<0>, gq, dim3(kTriThreads), smem_t, stream, ds_k, k_n, p)) return 1;
         const dim3 gk((unsigned)nt, (unsigned)(units * p.pieces));  // (units = KV groups x heads of a group)
         p.out = dk, p.which = 0;
-        if (ZT_LAUNCH("gemm_tri_dk", stream, (gemm_tri<1><<<gk, kTriThreads, smem_t, stream>>>(ds_m, qs_n, p)))) return 1;
+        if (launch_pdl("gemm_tri_dk", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, ds_m, qs_n, p)) return 1;
         p.out = dv, p.which = 1;
-        if (ZT_LAUNCH("gemm_tri_dv", stream, (gemm_tri<1><<<gk, kTriThreads, smem_t, stream>>>(p_m, g_n, p)))) return 1;
+        if (launch_pdl("gemm_tri_dv", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, p_m, g_n, p)) return 1;
     }
     return 0;
 }

@@ -6,7 +6,7 @@
 // an f16 term is half a TF32 MMA, operands take half the bytes (three K and three V tiles, hi and
 // lo, fit in shared memory), and two S tiles and two O accumulators fit in TMEM.
 //
-//   bwd_absmax / bwd_split   (tc_bwd.cuh) q, k, v -> f16 hi/lo planes with a power-of-two scale
+//   the pre-pass             (prepass.cuh) q, k, v -> f16 hi/lo planes with a power-of-two scale
 //                            per (sequence, KV group), in a workspace.
 //   TMA warp        K and V hi/lo tiles of 64 keys, a ring of three slots each: a K tile is free
 //                   once its S has retired, two tiles before its V.
@@ -202,6 +202,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
     const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
@@ -506,20 +508,22 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 struct Workspace {
     uint32_t *amax_q, *amax_k, *amax_v;
+    uint32_t *vnmax;  // (in the backward's layout: the largest row norm of v, which the backward wants; else null)
+    uint2 *part[3];   // the pre-pass's slots
     __half *q_planes, *k_planes, *v_planes;
-    size_t total_bytes, amax_bytes;
+    size_t total_bytes;
 };
 
 inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset = 0) {
     Workspace w{};
     const size_t n_amax = (size_t)batch * n_kv_heads;
-    w.amax_bytes = (3 * n_amax * sizeof(uint32_t) + 1023) / 1024 * 1024;
     auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
     const size_t qh = (size_t)2 * batch * T * n_heads * dim * sizeof(__half);
     const size_t kh = (size_t)2 * batch * (q_offset + T) * n_kv_heads * dim * sizeof(__half);
     char *c = static_cast<char *>(base);
     w.amax_q = reinterpret_cast<uint32_t *>(c), w.amax_k = w.amax_q + n_amax, w.amax_v = w.amax_k + n_amax;
-    size_t off = w.amax_bytes;
+    size_t off = up(3 * n_amax * sizeof(uint32_t));
+    for (int i = 0; i < 3; ++i) w.part[i] = reinterpret_cast<uint2 *>(c + off), off += up(tcb::pass_part_bytes(n_amax));
     w.q_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.k_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
@@ -534,7 +538,7 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     if (optin_smem((const void *)attn_fwd_tc16<D>, smem)) return 1;
     const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
-    return ZT_LAUNCH("attn_fwd_tc16", stream, (attn_fwd_tc16<D><<<grid, kThreads, smem, stream>>>(kmap, vmap, qmap, p)));
+    return launch_pdl("attn_fwd_tc16", attn_fwd_tc16<D>, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
 // (tc_fwd16x.cuh)
@@ -573,24 +577,20 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     tcf16::Workspace w = tcf16::workspace(ws, batch, T, n_heads, n_kv_heads, td, q_offset);
     if (in_backward_workspace) {
         const BwdWorkspace bw = bwd_workspace(ws, batch, T, n_heads, n_kv_heads, td);
-        w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;  // contiguous; amax_do follows
-        w.amax_bytes = 3 * (size_t)batch * n_kv_heads * sizeof(uint32_t);
+        w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;
+        w.vnmax = bw.vnmax;
+        for (int i = 0; i < 3; ++i) w.part[i] = bw.part[i];
         w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes;
     }
     const int group = n_heads / n_kv_heads;
-    const int wq_src = n_heads * dim, wkv_src = n_kv_heads * dim;
     const int wkv = n_kv_heads * td;
     const int n_seen = q_offset + T;  // key rows that some query row sees
-    if (cudaMemsetAsync(w.amax_q, 0, w.amax_bytes, stream) != cudaSuccess) {
-        cudaGetLastError();
-        return refuse("could not clear the forward workspace header");
-    }
-    PrepassArgs pa{};
-    pa.n = 3, pa.batch = batch;
-    pa.t[0] = {q, w.amax_q, w.q_planes, wq_src, group * dim, T, dim, td, rope};
-    pa.t[1] = {k, w.amax_k, w.k_planes, wkv_src, dim, n_seen, dim, td, rope};
-    pa.t[2] = {v, w.amax_v, w.v_planes, wkv_src, dim, n_seen, dim, td, nullptr};
-    if (launch_prepass(pa, stream)) return 1;
+    PassArgs pa{};
+    pa.dim = dim, pa.td = td;
+    pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
+    pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
+    pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
+    if (launch_pass(pa, stream)) return 1;
     if (td == 256) {
         // head_dim 256 (and those padded to it): one head per CTA, K fetched block by block (attn_fwd_tc16x)
         CUtensorMap kmap, vmap, qmap;

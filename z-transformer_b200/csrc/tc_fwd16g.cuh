@@ -78,6 +78,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
     const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
@@ -354,7 +356,7 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     if (optin_smem((const void *)attn_fwd_tc16g<D>, smem)) return 1;
     const dim3 grid((unsigned)(p.n_heads / 2), (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
-    return ZT_LAUNCH("attn_fwd_tc16g", stream, (attn_fwd_tc16g<D><<<grid, kThreads, smem, stream>>>(kmap, vmap, qmap, p)));
+    return launch_pdl("attn_fwd_tc16g", attn_fwd_tc16g<D>, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

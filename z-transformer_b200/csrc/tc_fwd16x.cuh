@@ -91,6 +91,8 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    pdl_wait();
+    pdl_launch();
 
     const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
     const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
@@ -355,7 +357,7 @@ inline int launch_x(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     const size_t smem = 3 * (size_t)(2 * 64 * 256 * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
     if (optin_smem((const void *)attn_fwd_tc16x, smem)) return 1;
     const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
-    return ZT_LAUNCH("attn_fwd_tc16x", stream, (attn_fwd_tc16x<<<grid, kThreadsX, smem, stream>>>(kmap, vmap, qmap, p)));
+    return launch_pdl("attn_fwd_tc16x", attn_fwd_tc16x, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

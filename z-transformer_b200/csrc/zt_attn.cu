@@ -217,10 +217,7 @@ static int backward_impl(const float *q, const float *k, const float *v, const f
         workspace_bytes >= backward_workspace(batch, T, n_heads, n_kv_heads, dim) &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
         n_kv_heads <= tcb::kPrepassMaxGroups && tcb::tc_bwd_supported(batch, T, dim, q, k, v, dout, dq, dk, dv)) {
-        // the tensor-core kernels also want each row's |dout| (their scale of dS): the same pass writes it
-        float *rnorm = tcb::bwd_workspace(workspace, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).rnorm;
-        if (launch_delta(out, dout, delta, rnorm, (long long)batch * T * n_heads, dim, stream)) return 1;
-        return launch_bwd_tc(q, k, v, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads,
+        return launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads,
                              dim, stream, nullptr, nullptr, kept, dq_peers, g_path.load() == 8);
     }
     const size_t wide_need = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
@@ -228,16 +225,14 @@ static int backward_impl(const float *q, const float *k, const float *v, const f
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
         !(dq_peers && dq_peers->n > 0) &&
         tcw::tc_bwd_wide_supported(batch, T, n_heads, n_kv_heads, dim, q, k, v, dout, dq, dk, dv)) {
-        float *rnorm = tcw::wide_workspace(workspace, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).base.rnorm;
-        if (launch_delta(out, dout, delta, rnorm, (long long)batch * T * n_heads, dim, stream)) return 1;
-        return launch_bwd_wide(q, k, v, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads, dim,
+        return launch_bwd_wide(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads, dim,
                                stream, kept, g_path.load() == 8);
     }
 #endif
     if (dq_peers && dq_peers->n > 0)
         return refuse("peer copies of dq are written by the tensor-core backward only, which does not take this shape.");
     (void)workspace, (void)workspace_bytes, (void)kept;
-    if (launch_delta(out, dout, delta, nullptr, (long long)batch * T * n_heads, dim, stream)) return 1;
+    if (launch_delta(out, dout, delta, (long long)batch * T * n_heads, dim, stream)) return 1;
     SimtBwdParams p{};
     p.q = q, p.k = k, p.v = v, p.dout = dout, p.lse = lse, p.delta = delta;
     p.dq = dq, p.dk = dk, p.dv = dv;
@@ -739,10 +734,7 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     // and the fused backward adds partial sums into dq, which can only be rotated once they are complete
     const bool two_kernels = g_path.load() == 8;
     dq_in_kernel = fused && (dim == 32 || dim == 64 || dim == 128) && !tc_bwd_takes_fused(dim, two_kernels, nullptr);
-    if (fused && launch_delta(out, dout, delta, tcb::bwd_workspace(w.inner, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).rnorm,
-                              (long long)batch * T * n_heads, dim, s))
-        return 1;
-    if (fused && launch_bwd_tc(q, k, v, dout, lse, delta, dq, dk, dv, w.inner, batch, T, n_heads, n_kv_heads, dim, s,
+    if (fused && launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, w.inner, batch, T, n_heads, n_kv_heads, dim, s,
                                w.table, dq_in_kernel ? w.table_t : nullptr, kept, nullptr, two_kernels))
         return 1;
 #endif
@@ -766,15 +758,18 @@ namespace {
 struct ProjWorkspace {
     uint32_t *amax_ctx, *amax_w, *amax_dy;  // [batch], [1], [batch]
     __half *ctx_planes, *w_planes, *dy_planes;
-    size_t total_bytes, header_bytes;
+    uint2 *part_ctx, *part_w, *part_dy;     // the pre-pass's slots
+    size_t total_bytes;
 };
 ProjWorkspace proj_workspace(void *base, int batch, int T, int k, int n) {
     auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
     ProjWorkspace w{};
     char *c = static_cast<char *>(base);
     w.amax_ctx = reinterpret_cast<uint32_t *>(c), w.amax_w = w.amax_ctx + batch, w.amax_dy = w.amax_w + 1;
-    w.header_bytes = up((size_t)(2 * batch + 1) * sizeof(uint32_t));
-    size_t off = w.header_bytes;
+    size_t off = up((size_t)(2 * batch + 1) * sizeof(uint32_t));
+    w.part_ctx = reinterpret_cast<uint2 *>(c + off), off += up(tcb::pass_part_bytes(batch));
+    w.part_w = reinterpret_cast<uint2 *>(c + off), off += up(tcb::pass_part_bytes(1));
+    w.part_dy = reinterpret_cast<uint2 *>(c + off), off += up(tcb::pass_part_bytes(batch));
     w.ctx_planes = reinterpret_cast<__half *>(c + off), off += up((size_t)2 * batch * T * k * sizeof(__half));
     w.w_planes = reinterpret_cast<__half *>(c + off), off += up((size_t)2 * k * n * sizeof(__half));
     w.dy_planes = reinterpret_cast<__half *>(c + off), off += up((size_t)2 * batch * T * n * sizeof(__half));
@@ -801,12 +796,10 @@ int check_proj(const void *workspace, size_t workspace_bytes, int batch, int T, 
 #endif
 }
 #ifndef ZT_NO_TC
-// planes of x [batch][rows][width] with one scale per batch item
-int proj_planes(const float *x, uint32_t *amax, __half *planes, int batch, int rows, int width, cudaStream_t s) {
-    tcb::PrepassArgs pa{};
-    pa.n = 1, pa.batch = batch;
-    pa.t[0] = {x, amax, planes, width, width, rows, width, width, nullptr};
-    return tcb::launch_prepass(pa, s);
+// The planes of x [batch][rows][width] with one scale per batch item: 64 columns count as a head of the pre-pass.
+void add_proj_planes(tcb::PassArgs &a, const float *x, int batch, int rows, int width, uint2 *part, uint32_t *amax, __half *planes) {
+    a.dim = 64, a.td = 64;
+    tcb::pass_add(a, x, batch, rows, width / 64, width / 64, part, amax, nullptr, planes);
 }
 #endif
 }  // namespace
@@ -828,22 +821,20 @@ __global__ void seq_amax_kernel(const uint32_t *__restrict__ amax_v, uint32_t *_
 // y = ctx . w.  ctx_planes_from: null (ctx is converted here), or the [batch, n_kv_heads] maxima of v that scaled the
 // planes the attention kernel has already left in the workspace.
 static int proj_forward_impl(const float *ctx, const float *w, float *y, void *workspace, int batch, int T, int k, int n,
-                             cudaStream_t s, bool header_cleared, const uint32_t *ctx_planes_from, int n_kv_heads) {
+                             cudaStream_t s, const uint32_t *ctx_planes_from, int n_kv_heads) {
 #ifndef ZT_NO_TC
     const ProjWorkspace ws = proj_workspace(workspace, batch, T, k, n);
     const int pieces = (k + tcg::kPiece - 1) / tcg::kPiece;
-    if ((!header_cleared && cudaMemsetAsync(ws.amax_ctx, 0, ws.header_bytes, s) != cudaSuccess) ||
-        (pieces > 1 && cudaMemsetAsync(y, 0, (size_t)batch * T * n * sizeof(float), s) != cudaSuccess)) {
-        cudaGetLastError();
-        return refuse("could not clear the projection's buffers");
-    }
+    tcb::PassArgs pa{};
+    add_proj_planes(pa, w, 1, k, n, ws.part_w, ws.amax_w, ws.w_planes);
     if (ctx_planes_from) {
         if (ZT_LAUNCH("seq_amax_kernel", s, (seq_amax_kernel<<<(unsigned)batch, 1, 0, s>>>(ctx_planes_from, ws.amax_ctx, n_kv_heads))))
             return 1;
-    } else if (proj_planes(ctx, ws.amax_ctx, ws.ctx_planes, batch, T, k, s)) {
-        return 1;
+    } else {
+        add_proj_planes(pa, ctx, batch, T, k, ws.part_ctx, ws.amax_ctx, ws.ctx_planes);
     }
-    if (proj_planes(w, ws.amax_w, ws.w_planes, 1, k, n, s)) return 1;
+    if (pieces > 1) tcb::pass_fill(pa, y, (long long)batch * T * n);  // (the pieces are added in memory)
+    if (tcb::launch_pass(pa, s)) return 1;
     CUtensorMap amap, bmap;
     if (!tcg::make_plane_map(&amap, ws.ctx_planes, 2 * batch, T, k, 1, 128) ||   // rows x K, K-major
         !tcg::make_plane_map(&bmap, ws.w_planes, 2, k, n, 2, 64))                // K x N, N-major
@@ -863,7 +854,7 @@ int zt_proj_forward(const float *ctx, const float *w, float *y, void *workspace,
     g_last_error[0] = 0;
     if (!ctx || !w || !y) return refuse("a null device pointer was passed.");
     if (check_proj(workspace, workspace_bytes, batch, T, k, n)) return 1;
-    return proj_forward_impl(ctx, w, y, workspace, batch, T, k, n, (cudaStream_t)stream, false, nullptr, 0);
+    return proj_forward_impl(ctx, w, y, workspace, batch, T, k, n, (cudaStream_t)stream, nullptr, 0);
 }
 
 int zt_attn_block_forward(const float *q, const float *k, const float *v, const float *wo, float *ctx, float *lse, float *y,
@@ -880,10 +871,6 @@ int zt_attn_block_forward(const float *q, const float *k, const float *v, const 
     cudaStream_t s = (cudaStream_t)stream;
 #ifndef ZT_NO_TC
     const ProjWorkspace pw = proj_workspace(proj_workspace_, batch, T, kdim, d_model);
-    if (cudaMemsetAsync(pw.amax_ctx, 0, pw.header_bytes, s) != cudaSuccess) {
-        cudaGetLastError();
-        return refuse("could not clear the projection's buffers");
-    }
     bool planes_written = false;
     if (forward_rope_impl(q, k, v, ctx, lse, rope_ws, rope_ws_bytes, batch, T, n_heads, n_kv_heads, dim, pos,
                           theta, stream, host_token, pw.ctx_planes, &planes_written))
@@ -893,7 +880,7 @@ int zt_attn_block_forward(const float *q, const float *k, const float *v, const 
         const RopeWorkspace rw = rope_workspace(rope_ws, batch, T, n_heads, n_kv_heads, dim);
         from = tcb::bwd_workspace(rw.inner, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).amax_v;
     }
-    return proj_forward_impl(ctx, wo, y, proj_workspace_, batch, T, kdim, d_model, s, true, from, n_kv_heads);
+    return proj_forward_impl(ctx, wo, y, proj_workspace_, batch, T, kdim, d_model, s, from, n_kv_heads);
 #else
     (void)s, (void)lse, (void)rope_ws, (void)rope_ws_bytes, (void)pos, (void)theta;
     return 1;
@@ -910,14 +897,12 @@ int zt_proj_backward(const float *ctx, const float *w, const float *dy, float *d
     const ProjWorkspace ws = proj_workspace(workspace, batch, T, k, n);
     const int pieces_in = (n + tcg::kPiece - 1) / tcg::kPiece;   // inputGrad contracts over n
     const int pieces_w = (T + tcg::kPiece - 1) / tcg::kPiece;    // weightGrad contracts over a sequence's rows
-    if (cudaMemsetAsync(ws.amax_ctx, 0, ws.header_bytes, s) != cudaSuccess ||
-        (pieces_in > 1 && cudaMemsetAsync(dctx, 0, (size_t)batch * T * k * sizeof(float), s) != cudaSuccess)) {
-        cudaGetLastError();
-        return refuse("could not clear the projection's buffers");
-    }
-    if (proj_planes(ctx, ws.amax_ctx, ws.ctx_planes, batch, T, k, s)) return 1;
-    if (proj_planes(w, ws.amax_w, ws.w_planes, 1, k, n, s)) return 1;
-    if (proj_planes(dy, ws.amax_dy, ws.dy_planes, batch, T, n, s)) return 1;
+    tcb::PassArgs pa{};
+    add_proj_planes(pa, ctx, batch, T, k, ws.part_ctx, ws.amax_ctx, ws.ctx_planes);
+    add_proj_planes(pa, w, 1, k, n, ws.part_w, ws.amax_w, ws.w_planes);
+    add_proj_planes(pa, dy, batch, T, n, ws.part_dy, ws.amax_dy, ws.dy_planes);
+    if (pieces_in > 1) tcb::pass_fill(pa, dctx, (long long)batch * T * k);
+    if (tcb::launch_pass(pa, s)) return 1;
     CUtensorMap dy_k, w_k, ctx_m, dy_n;
     if (!tcg::make_plane_map(&dy_k, ws.dy_planes, 2 * batch, T, n, 1, 128) ||   // A: rows x N, K-major (contraction over n)
         !tcg::make_plane_map(&w_k, ws.w_planes, 2, k, n, 1, 128) ||             // B: w's rows are dctx's columns, K-major

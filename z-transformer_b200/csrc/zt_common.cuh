@@ -89,6 +89,30 @@ inline void prof_end(int idx, const char *name, cudaStream_t stream) {
         return ::zt::launch_failed(name " launch");           \
     }())
 
+// ---- launches that overlap the end of the kernel before them -------------------------------------
+// Programmatic dependent launch: the grid may be set up while the kernel before it in the stream still runs.  Every
+// kernel launched this way calls pdl_wait() in every block before it touches global memory -- it returns once the
+// kernel before has completed and its writes are visible, so the stream's order is what it always was -- and
+// pdl_launch() as soon as its own successor may be set up.  On a chain of 5-10 us kernels this takes 1-2 us off
+// each gap.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline int launch_pdl(const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                      const A &...args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    const int pi = prof_begin(stream);
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    prof_end(pi, name, stream);
+    return launch_failed(name);
+}
+
 // ---- per-device facts, asked once per device --------------------------------
 struct DeviceInfo {
     int known = 0;
