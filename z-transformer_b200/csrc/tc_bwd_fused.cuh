@@ -621,7 +621,7 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     if (optin_smem((const void *)attn_bwd_fused_tc<D>, smem)) return 1;
     const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
-    return launch_pdl("attn_bwd_fused_tc", attn_bwd_fused_tc<D>, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
+    return launch_after("attn_bwd_fused_tc", attn_bwd_fused_tc<D>, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
 }
 inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
                             const BwdParams &p, cudaStream_t stream) {

@@ -855,19 +855,19 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         p.unit0 = unit0;
         if (tile_scores) {
             const dim3 gs((unsigned)(nt * (nt + 1) / 2), (unsigned)units);
-            if (launch_pdl("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
         } else {
             const dim3 gs((unsigned)units, (unsigned)nt);
-            if (launch_pdl("bwd_wide_scores_res", bwd_wide_scores_res, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores_res", bwd_wide_scores_res, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
         }
         p.out = dq, p.which = 0;
         const dim3 gq((unsigned)nt, (unsigned)(units * p.pieces));
-        if (launch_pdl("gemm_tri_dq", gemm_tri<0>, gq, dim3(kTriThreads), smem_t, stream, ds_k, k_n, p)) return 1;
+        if (launch_after("gemm_tri_dq", gemm_tri<0>, gq, dim3(kTriThreads), smem_t, stream, ds_k, k_n, p)) return 1;
         const dim3 gk((unsigned)nt, (unsigned)(units * p.pieces));  // (units = KV groups x heads of a group)
         p.out = dk, p.which = 0;
-        if (launch_pdl("gemm_tri_dk", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, ds_m, qs_n, p)) return 1;
+        if (launch_after("gemm_tri_dk", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, ds_m, qs_n, p)) return 1;
         p.out = dv, p.which = 1;
-        if (launch_pdl("gemm_tri_dv", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, p_m, g_n, p)) return 1;
+        if (launch_after("gemm_tri_dv", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, p_m, g_n, p)) return 1;
     }
     return 0;
 }

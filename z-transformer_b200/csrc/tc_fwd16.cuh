@@ -51,7 +51,7 @@ struct Params {
     float *out, *lse;                           // lse may be null
     int batch, T, n_heads, n_kv_heads;
     int q_offset;  // query row r stands at position q_offset + r of the keys: it sees keys 0 .. q_offset + r
-    int flush_tiles;  // O leaves the tensor core's accumulator every so many key tiles; 0: never (see flush_row)
+    bool flush;    // O leaves the tensor core's accumulator every kFlushKeyTiles key tiles (see flush_row)
     int dim_out;  // the tensors' head_dim, at most the tile's D
     int ahead;    // attn_fwd_tc16 prefetches the query tile of the block this many places on in launch order; 0: none
     float scale_log2;
@@ -123,7 +123,7 @@ __device__ __forceinline__ float row_exp32(const uint32_t (&r)[32], int key0, in
 }
 
 // The tensor core adds into its f32 accumulator with truncation, which over n key tiles of 64 costs O about
-// n 2.3e-7 of its size, always toward zero (1.4e-5 measured at 4096 keys in one accumulator).  With p.flush_tiles set,
+// n 2.3e-7 of its size, always toward zero (1.4e-5 measured at 4096 keys in one accumulator).  With FLUSH
 // O leaves TMEM every so many tiles and is summed with rounding in memory: in the row of out, which the finished row
 // overwrites at the end.  16 tiles hold the error at 3.7e-6 whatever the context, for 64 KB through L2 per 32000
 // clocks of MMAs.  Set for windows of a prompt, every row of which runs over the whole context behind it; over a whole
@@ -162,7 +162,7 @@ __device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, f
     }
 }
 
-template <int D>
+template <int D, bool FLUSH>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_fwd_tc16(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                   const __grid_constant__ CUtensorMap qmap, const Params p) {
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t vh = v_u32 + (uint32_t)(s * 2 * KP);
                 const uint64_t mvh = desc_mnmajor_16b(vh, BN * 128), mvl = desc_mnmajor_16b(vh + KP, BN * 128);
                 const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
-                const bool fresh = j < 2 || (p.flush_tiles > 0 && (j >> 1) % p.flush_tiles == 0);  // (O was flushed before tile j)
+                const bool fresh = j < 2 || (FLUSH && (j >> 1) % kFlushKeyTiles == 0);  // (O was flushed before tile j)
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
                     const uint32_t ac = (uint32_t)(32 * (kk >> 1) + (kk & 1) * 8);
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // where the sets keep flushed sums: set 0 in out, set 1 in the two planes of the query row, which this CTA alone
         // reads and has in TMEM by now (a forward that flushes keeps no planes for a backward)
         FlushRow row0{nullptr, nullptr, p.dim_out}, row1{nullptr, nullptr, D};
-        if (p.flush_tiles > 0 && t < p.T) {
+        if (FLUSH && t < p.T) {
             row0.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row0.upper = row0.lower + D / 2;
             __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * D + (long long)h * D;
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
-            const bool flush = p.flush_tiles > 0 && j > 1 && (j >> 1) % p.flush_tiles == 0;
+            const bool flush = FLUSH && j > 1 && (j >> 1) % kFlushKeyTiles == 0;
             if (j > 1 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
                 // this set's O may only be touched once its previous P.V (tile j-2) has retired
                 if (!__all_sync(0xffffffffu, fwait(&sh->pv_done[set], (uint32_t)(((j >> 1) - 1) & 1), sh))) {
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float inv = 1.f / (lsum * mv);  // lsum, like O, carries kPScale
             const float f0 = w0 * inv, f1 = w1 * inv;
             const float s0 = sh->fin_f[0][tid], s1 = sh->fin_f[1][tid];
-            const bool add0 = s0 != -INFINITY && row0.lower != nullptr, add1 = s1 != -INFINITY && row1.lower != nullptr;
+            const bool add0 = FLUSH && s0 != -INFINITY && row0.lower != nullptr, add1 = FLUSH && s1 != -INFINITY && row1.lower != nullptr;
             const float g0 = add0 ? ex2(s0 - m0) : 0.f, g1 = add1 ? ex2(s1 - m1) : 0.f;
             // set s merges columns [s D/2, (s+1) D/2) of the row
             uint8_t *srow = sK + tid * (D * 4);
@@ -536,9 +536,10 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
                     cudaStream_t stream) {
     size_t smem = 12 * (size_t)(64 * D * 2) + sizeof(Shared) + 1024;
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    if (optin_smem((const void *)attn_fwd_tc16<D>, smem)) return 1;
+    const auto kernel = p.flush ? attn_fwd_tc16<D, true> : attn_fwd_tc16<D, false>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
-    return launch_pdl("attn_fwd_tc16", attn_fwd_tc16<D>, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
 // (tc_fwd16x.cuh)
@@ -602,7 +603,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
         p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
         p.out = out, p.lse = lse;
         p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-        p.dim_out = dim, p.q_offset = q_offset, p.flush_tiles = q_offset > 0 ? tcf16::kFlushKeyTiles : 0;
+        p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
         p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
         if (out_peers) p.out_peers = *out_peers;
         p.scale_log2 = kLog2e / sqrtf((float)dim);
@@ -621,7 +622,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
     p.out = out, p.lse = lse;
     p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-    p.dim_out = dim, p.q_offset = q_offset, p.flush_tiles = q_offset > 0 ? tcf16::kFlushKeyTiles : 0;
+    p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
     p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
     if (out_peers) p.out_peers = *out_peers;
     p.ahead = device_info() ? device_info()->sm_count : 0;  // one CTA per SM

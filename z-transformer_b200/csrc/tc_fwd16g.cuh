@@ -37,7 +37,7 @@ __device__ __forceinline__ void ggive_up(SharedG *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-template <int D>
+template <int D, bool FLUSH>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_fwd_tc16g(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                    const __grid_constant__ CUtensorMap qmap, const Params p) {
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             };
             // P.V of head `hd`, tile j (V tile j has landed)
             auto issue_pv = [&](int hd, int j) {
-                const bool fresh = j == 0 || (p.flush_tiles > 0 && j % p.flush_tiles == 0);  // (O was flushed before tile j)
+                const bool fresh = j == 0 || (FLUSH && j % kFlushKeyTiles == 0);  // (O was flushed before tile j)
                 const uint32_t vh = v_u32 + (uint32_t)((j & 1) * 2 * KP);
                 const uint64_t mvh = desc_mnmajor_16b(vh, BN * 128), mvl = desc_mnmajor_16b(vh + KP, BN * 128);
                 const uint32_t cS = cS0 + hd * BN, cO = cO0 + hd * D;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         FlushRow row{nullptr, nullptr, p.dim_out};
-        if (p.flush_tiles > 0 && t < p.T) {
+        if (FLUSH && t < p.T) {
             row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row.upper = row.lower + D / 2;
         }
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
-            const bool flush = p.flush_tiles > 0 && j > 0 && j % p.flush_tiles == 0;
+            const bool flush = FLUSH && j > 0 && j % kFlushKeyTiles == 0;
             if (j > 0 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
                 // this head's O may only be touched once its previous P.V has retired
                 if (!__all_sync(0xffffffffu, gwait(&sh->pv_done[set], (uint32_t)((j - 1) & 1), sh))) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
-            const bool add = m_flushed != -INFINITY && row.lower != nullptr;
+            const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * (D * 4);
 #pragma unroll 1
@@ -354,9 +354,10 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
                       cudaStream_t stream) {
     size_t smem = 14 * (size_t)(64 * D * 2) + sizeof(SharedG);
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    if (optin_smem((const void *)attn_fwd_tc16g<D>, smem)) return 1;
+    const auto kernel = p.flush ? attn_fwd_tc16g<D, true> : attn_fwd_tc16g<D, false>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)(p.n_heads / 2), (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
-    return launch_pdl("attn_fwd_tc16g", attn_fwd_tc16g<D>, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16g", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

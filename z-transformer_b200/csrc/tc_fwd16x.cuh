@@ -50,6 +50,7 @@ __device__ __forceinline__ void xgive_up(SharedX *sh, int code) {
 
 // kmap: K planes with a box of ONE 64-column block x 64 keys; vmap: V planes, four blocks x 64 keys; qmap: Q planes,
 // four blocks x 128 rows.
+template <bool FLUSH>
 __global__ void __launch_bounds__(kThreadsX, 1)
     attn_fwd_tc16x(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                    const __grid_constant__ CUtensorMap qmap, const Params p) {
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             };
             // P.V of tile j
             auto issue_pv = [&](int j) {
-                const bool fresh = j == 0 || (p.flush_tiles > 0 && j % p.flush_tiles == 0);  // (O was flushed before tile j)
+                const bool fresh = j == 0 || (FLUSH && j % kFlushKeyTiles == 0);  // (O was flushed before tile j)
                 const uint64_t mvh = desc_mnmajor_16b(v_u32, BN * 128), mvl = desc_mnmajor_16b(v_u32 + KP, BN * 128);
                 const uint32_t cS = cS0 + (j & 1) * BN;
 #pragma unroll
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         FlushRow row{nullptr, nullptr, p.dim_out};
-        if (p.flush_tiles > 0 && t < p.T) {
+        if (FLUSH && t < p.T) {
             row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row.upper = row.lower + D / 2;
         }
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             }
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
-            const bool flush = p.flush_tiles > 0 && j > 0 && j % p.flush_tiles == 0;
+            const bool flush = FLUSH && j > 0 && j % kFlushKeyTiles == 0;
             if (j > 0 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
                 // O may only be touched once the previous P.V has retired
                 if (!__all_sync(0xffffffffu, xwait(&sh->pv_done, (uint32_t)((j - 1) & 1), sh))) {
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
-            const bool add = m_flushed != -INFINITY && row.lower != nullptr;
+            const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * (D * 4);
 #pragma unroll 1
@@ -355,9 +356,10 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 inline int launch_x(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
                     cudaStream_t stream) {
     const size_t smem = 3 * (size_t)(2 * 64 * 256 * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
-    if (optin_smem((const void *)attn_fwd_tc16x, smem)) return 1;
+    const auto kernel = p.flush ? attn_fwd_tc16x<true> : attn_fwd_tc16x<false>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
-    return launch_pdl("attn_fwd_tc16x", attn_fwd_tc16x, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

@@ -222,7 +222,7 @@ inline int launch_gemm(const CUtensorMap &amap, const CUtensorMap &bmap, const G
     const size_t smem = gemm_smem_bytes();
     if (optin_smem((const void *)gemm_f16split_tc<A_MN, B_MN>, smem)) return 1;
     const dim3 grid((unsigned)((p.m_rows + 127) / 128), (unsigned)((p.n_cols + 127) / 128), (unsigned)(p.batch * p.pieces));
-    return launch_pdl("gemm_f16split_tc", gemm_f16split_tc<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, amap, bmap, p);
+    return launch_after("gemm_f16split_tc", gemm_f16split_tc<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, amap, bmap, p);
 }
 
 }  // namespace tcg
