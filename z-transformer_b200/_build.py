@@ -9,6 +9,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libztattn.so")
 HOST_LIB_PATH = os.path.join(HERE, "libzthost.so")
+# the native host side of the Python calls, a CPython extension over torch's C++ API
+TORCH_EXT_PATH = os.path.join(HERE, "_zt_torch.so")
 HARNESS_PATH = os.path.join(HERE, "zt_attn_harness")
 # the negative-control build: the same sources with defect switches compiled into the kernels (-DZT_DEFECTS)
 DEFECTS_LIB_PATH = os.path.join(HERE, "libztattn_defects.so")
@@ -39,9 +41,25 @@ def _sources() -> list[str]:
     return out
 
 
+def _build_torch_ext(src: str) -> None:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    include, lib = os.path.join(root, "include"), os.path.join(root, "lib")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    subprocess.check_call([
+        shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        "-isystem", include, "-isystem", os.path.join(include, "torch", "csrc", "api", "include"),
+        "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
+        "-o", TORCH_EXT_PATH, src, "-L" + HERE, "-lztattn", "-Wl,-rpath,$ORIGIN",
+        "-L" + lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
     """nvcc -> libztattn.so (kernels + C ABI), libzthost.so (C++ host mirror + its C shim, when its
-    source exists) and the zt_attn_harness program."""
+    source exists), _zt_torch.so (the Python calls' host side) and the zt_attn_harness program."""
     srcs = _sources()
     if force or _stale(LIB_PATH, srcs):
         cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH, os.path.join(CSRC, "zt_attn.cu"), "-lcuda"]
@@ -54,6 +72,9 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
                "-o", HOST_LIB_PATH, host_src, "-L" + HERE, "-lztattn",
                "-Xlinker", "-rpath", "-Xlinker", "$ORIGIN"]
         subprocess.check_call(cmd)
+    ext_src = os.path.join(CSRC, "host", "zt_torch.cpp")
+    if force or _stale(TORCH_EXT_PATH, [ext_src, srcs[0]]):
+        _build_torch_ext(ext_src)
     harness_src = os.path.join(CSRC, "zt_harness.cpp")
     if os.path.exists(harness_src) and (force or _stale(HARNESS_PATH, srcs)):
         # the twin-directory harness: a host program over the C ABI (csrc/zt_harness.cpp)

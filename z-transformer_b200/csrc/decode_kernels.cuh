@@ -12,8 +12,11 @@
 //   * a row is read once and dotted against every query head of the group held
 //     in registers; lane-group shuffles finish each dot;
 //   * online softmax in the log2 domain per lane group, merged across lane
-//     groups by shuffles, across warps through shared memory, and across chunks
-//     by a second small kernel (log-sum-exp combine).
+//     groups by shuffles, across warps through shared memory, and across the blocks of
+//     a sequence's KV head either inside a thread-block cluster (its blocks divide the
+//     keys evenly and read each other's sums from shared memory: one launch, nothing
+//     in global memory) or, for contexts too long for that, by a second small
+//     kernel over partial results in the workspace (log-sum-exp combine).
 //
 // Algorithmic bytes per sequence step: n_keys * 2 * n_kv_heads * dim * 4 (K and V
 // once each) plus q and out.
@@ -24,6 +27,7 @@
 namespace zt {
 
 constexpr int kDecodeThreads = 256;
+constexpr int kMaxCluster = 8;
 constexpr int kDecodeHeaderBytes = 256;  // workspace header: bad-sequence counter
 
 struct DecodeParams {
@@ -35,6 +39,7 @@ struct DecodeParams {
     float *part_acc;   // [batch, n_heads, max_chunks, dim]
     int *bad_count;    // in the workspace header
     int batch, n_ctx, n_heads, n_kv_heads, dim, chunk, max_chunks, n_sub;
+    int cluster;  // blocks per cluster in the one-launch form
     long long cache_batch_stride;  // elements between two sequences' caches
     float scale_log2;
 };
@@ -45,6 +50,32 @@ __device__ __forceinline__ float4 ldg_stream(const float *ptr) {
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                  : "l"(ptr));
     return v;
+}
+
+// ---- thread-block clusters ----------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// A float of block `rank`'s shared memory, at the place that `addr` has in this block's.
+__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
+    float v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n"
+                 : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+
+// How many sequences name no valid prefix: counted by one block, so that nothing has to be cleared beforehand.
+__device__ __forceinline__ void count_bad_sequences(const DecodeParams &p) {
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    if (p.n_keys)
+        for (int i = threadIdx.x; i < p.batch; i += blockDim.x)
+            if (p.n_keys[i] < 1 || p.n_keys[i] > p.n_ctx) atomicAdd(&total, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) *p.bad_count = total;
 }
 
 template <int NCH, int GP>
@@ -58,7 +89,9 @@ struct DecodeCfg {
 
 // LPK lanes share one key row; each lane holds NCH float4 chunks of it (chunk index
 // li + LPK * c); GP query heads are processed per pass.
-template <int LPK, int NCH, int GP>
+// CLUSTER: the blocks of a cluster (x) divide the sequence's keys evenly and finish the rows among themselves;
+// otherwise block x takes the x-th chunk of p.chunk keys and leaves a partial result.
+template <int LPK, int NCH, int GP, bool CLUSTER>
 __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks)
     decode_splitk_kernel(const DecodeParams p) {
     constexpr int U = DecodeCfg<NCH, GP>::kUnroll;
@@ -67,15 +100,27 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks
     extern __shared__ float smem[];
 
     const int b = blockIdx.z;
-    const int nk = p.n_keys ? p.n_keys[b] : p.n_keys_all;
-    if (nk < 1 || nk > p.n_ctx) return;  // reported by the combine kernel
-    const int c0 = blockIdx.x * p.chunk;
-    if (c0 >= nk) return;
-    const int c1 = (c0 + p.chunk < nk) ? c0 + p.chunk : nk;
     const int group = p.n_heads / p.n_kv_heads;
     const int g = blockIdx.y / p.n_sub, sub = blockIdx.y - g * p.n_sub;
     const int h0 = g * group + sub * GP;
     const int nh = (group - sub * GP) < GP ? (group - sub * GP) : GP;
+    pdl_wait();
+    pdl_launch();
+    if (CLUSTER && blockIdx.x == 0 && blockIdx.y == 0 && b == 0) count_bad_sequences(p);
+    const int nk = p.n_keys ? p.n_keys[b] : p.n_keys_all;
+    if (nk < 1 || nk > p.n_ctx) {
+        // decode.attnStep refuses an empty prefix (src/decode.zig:350); on the device the refusal is a NaN row plus
+        // a count the host can read.  (Two launches: the combine kernel writes the rows.)
+        if (CLUSTER && blockIdx.x == 0) {
+            for (int i = threadIdx.x; i < nh * p.dim; i += kDecodeThreads) p.out[((long long)b * p.n_heads + h0) * p.dim + i] = __int_as_float(0x7fc00000);
+            if (p.lse && threadIdx.x < nh) p.lse[(long long)b * p.n_heads + h0 + threadIdx.x] = __int_as_float(0x7fc00000);
+        }
+        return;  // (the whole cluster)
+    }
+    const int chunk = CLUSTER ? (nk + p.cluster - 1) / p.cluster : p.chunk;
+    const int c0 = blockIdx.x * chunk;
+    if (!CLUSTER && c0 >= nk) return;
+    const int c1 = (c0 + chunk < nk) ? c0 + chunk : nk;  // (a cluster's last blocks may have no key: c0 >= c1)
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int li = lane % LPK;
@@ -236,25 +281,57 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks
             lsum = fmaf(src[1], cw, lsum);
             a = fmaf(src[4 + j], cw, a);
         }
-        const long long slot = ((long long)b * p.n_heads + h0 + hh) * p.max_chunks + blockIdx.x;
-        p.part_acc[slot * dim + j] = a;
-        if (j == 0) p.part_ml[slot] = make_float2(mx, lsum);
+        if (CLUSTER) {
+            float *blk = smem + NW * GP * rec + hh * rec;  // the block's own sums, for its cluster to read
+            blk[4 + j] = a;
+            if (j == 0) blk[0] = mx, blk[1] = lsum;
+        } else {
+            const long long slot = ((long long)b * p.n_heads + h0 + hh) * p.max_chunks + blockIdx.x;
+            p.part_acc[slot * dim + j] = a;
+            if (j == 0) p.part_ml[slot] = make_float2(mx, lsum);
+        }
     }
+    if (!CLUSTER) return;
+    cluster_arrive();
+    cluster_wait();
+    const int cs = p.cluster;
+    const uint32_t blk0 = (uint32_t)__cvta_generic_to_shared(smem + NW * GP * rec);
+    for (int idx = blockIdx.x * kDecodeThreads + threadIdx.x; idx < nh * dim; idx += cs * kDecodeThreads) {
+        const int hh = idx / dim, j = idx - hh * dim;
+        const uint32_t at = blk0 + (uint32_t)(hh * rec) * 4u;
+        float mr[kMaxCluster], mx = -INFINITY;  // (block 0 of a cluster has keys: the maximum is finite)
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+            mr[r] = r < cs ? ld_cluster(at, r) : -INFINITY;
+            mx = fmaxf(mx, mr[r]);
+        }
+        float lsum = 0.f, acc_j = 0.f;
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+            if (r >= cs) break;
+            const float w = (mr[r] == -INFINITY) ? 0.f : ex2(mr[r] - mx);
+            lsum = fmaf(ld_cluster(at + 4u, r), w, lsum);
+            acc_j = fmaf(ld_cluster(at + 4u * (4 + j), r), w, acc_j);
+        }
+        const long long row = (long long)b * p.n_heads + h0 + hh;
+        p.out[row * dim + j] = acc_j / lsum;
+        if (p.lse && j == 0) p.lse[row] = (mx + log2f(lsum)) * kLn2;
+    }
+    cluster_arrive();  // nobody's shared memory goes away while others read it
+    cluster_wait();
 }
 
 // Log-sum-exp combine of a sequence's chunks.  grid (n_heads, batch), block 128.
 __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams p) {
     const int h = blockIdx.x, b = blockIdx.y;
+    pdl_wait();
+    pdl_launch();
+    if (h == 0 && b == 0) count_bad_sequences(p);
     const int nk = p.n_keys ? p.n_keys[b] : p.n_keys_all;
     float *orow = p.out + ((long long)b * p.n_heads + h) * p.dim;
     if (nk < 1 || nk > p.n_ctx) {
-        // decode.attnStep refuses an empty prefix (src/decode.zig:350); on the device the
-        // refusal is a NaN row plus a count the host can read.
         for (int j = threadIdx.x; j < p.dim; j += blockDim.x) orow[j] = __int_as_float(0x7fc00000);
-        if (threadIdx.x == 0) {
-            if (p.lse) p.lse[(long long)b * p.n_heads + h] = __int_as_float(0x7fc00000);
-            if (h == 0) atomicAdd(p.bad_count, 1);
-        }
+        if (threadIdx.x == 0 && p.lse) p.lse[(long long)b * p.n_heads + h] = __int_as_float(0x7fc00000);
         return;
     }
     const int nchunks = (nk + p.chunk - 1) / p.chunk;
@@ -277,10 +354,14 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
         p.lse[(long long)b * p.n_heads + h] = (mx + log2f(lsum)) * kLn2;
 }
 
-// kv_cache.Layer.append for a batch (src/kv_cache.zig:88-95).  grid (batch), block 256.
-__global__ void kv_append_kernel(float *k_cache, float *v_cache, int *n_keys, const float *k_new,
-                                 const float *v_new, int *full_count, int n_ctx, int width) {
+// kv_cache.Layer.append for a batch (src/kv_cache.zig:88-95).  grid (batch), block 256.  VEC: four floats at a time (the
+// rows of both caches and of the new rows start on 16-byte boundaries).
+template <bool VEC>
+__global__ void __launch_bounds__(256) kv_append_kernel(float *k_cache, float *v_cache, int *n_keys, const float *k_new,
+                                                        const float *v_new, int *full_count, int n_ctx, int width) {
     const int b = blockIdx.x;
+    pdl_wait();
+    pdl_launch();
     const int len = n_keys[b];
     if (len < 0 || len >= n_ctx) {  // Error.Full: nothing is written, nothing advances
         if (threadIdx.x == 0 && full_count) atomicAdd(full_count, 1);
@@ -288,9 +369,14 @@ __global__ void kv_append_kernel(float *k_cache, float *v_cache, int *n_keys, co
     }
     float *kd = k_cache + ((long long)b * n_ctx + len) * width;
     float *vd = v_cache + ((long long)b * n_ctx + len) * width;
-    for (int j = threadIdx.x; j < width; j += blockDim.x) {
-        kd[j] = k_new[(long long)b * width + j];
-        vd[j] = v_new[(long long)b * width + j];
+    const float *ks = k_new + (long long)b * width, *vs = v_new + (long long)b * width;
+    if (VEC) {
+        for (int j = threadIdx.x * 4; j < width; j += 1024) {
+            const float4 kx = *reinterpret_cast<const float4 *>(ks + j), vx = *reinterpret_cast<const float4 *>(vs + j);
+            *reinterpret_cast<float4 *>(kd + j) = kx, *reinterpret_cast<float4 *>(vd + j) = vx;
+        }
+    } else {
+        for (int j = threadIdx.x; j < width; j += 256) kd[j] = ks[j], vd[j] = vs[j];
     }
     __syncthreads();
     if (threadIdx.x == 0) n_keys[b] = len + 1;
@@ -300,6 +386,7 @@ __global__ void kv_append_kernel(float *k_cache, float *v_cache, int *n_keys, co
 
 struct DecodePlan {
     int lpk, nch, gp, n_sub, chunk, max_chunks;
+    int cluster;  // blocks per (sequence, KV head, pass) in the one-launch form; 0: two launches
     size_t ml_bytes, acc_bytes, total_bytes;
 };
 
@@ -327,6 +414,14 @@ inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads,
     if (chunk > 1024) chunk = 1024;
     pl.chunk = (int)chunk;
     pl.max_chunks = (n_ctx + pl.chunk - 1) / pl.chunk;
+    // One launch where clusters of at most eight blocks find an SM slot each at once (two blocks an SM) and a block's
+    // share stays below 768 keys; 32/8 heads of 128, us a call: one sequence, 512 keys 6.9 against 12.9, 2048 keys 11.1
+    // against 18.4, 8192 keys 39.4 against 35.6; four sequences, 2048 keys 19.4 against 30.7; sixteen (a second wave of
+    // clusters), 512 keys 34.0 against 27.5.  (Clusters of sixteen start late: 36.7 where eight take 19.4.)
+    const long long slots = target_blocks / 4;
+    long long cs = 1;
+    while (cs < kMaxCluster && 2 * cs * units <= slots && n_ctx > 64 * cs) cs *= 2;
+    pl.cluster = (cs * units <= slots && n_ctx <= 768 * cs) ? (int)cs : 0;
     pl.ml_bytes = (size_t)batch * n_heads * pl.max_chunks * sizeof(float2);
     pl.ml_bytes = (pl.ml_bytes + 255) / 256 * 256;
     pl.acc_bytes = (size_t)batch * n_heads * pl.max_chunks * dim * sizeof(float);
@@ -336,11 +431,18 @@ inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads,
 
 template <int LPK, int NCH, int GP>
 inline int launch_decode_inst(const DecodeParams &p, cudaStream_t stream) {
-    const size_t smem = (size_t)(kDecodeThreads / 32) * GP * (p.dim + 4) * sizeof(float);
-    if (optin_smem((const void *)decode_splitk_kernel<LPK, NCH, GP>, smem)) return 1;
-    dim3 grid((unsigned)p.max_chunks, (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
-    return ZT_LAUNCH("decode_splitk_kernel", stream,
-                     (decode_splitk_kernel<LPK, NCH, GP><<<grid, kDecodeThreads, smem, stream>>>(p)));
+    if (p.cluster == 0) {
+        const size_t smem = (size_t)(kDecodeThreads / 32) * GP * (p.dim + 4) * sizeof(float);
+        const auto kernel = decode_splitk_kernel<LPK, NCH, GP, false>;
+        if (optin_smem((const void *)kernel, smem)) return 1;
+        const dim3 grid((unsigned)p.max_chunks, (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
+        return launch_pdl("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p);
+    }
+    const size_t smem = (size_t)(kDecodeThreads / 32 + 1) * GP * (p.dim + 4) * sizeof(float);
+    const auto kernel = decode_splitk_kernel<LPK, NCH, GP, true>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
+    const dim3 grid((unsigned)p.cluster, (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
+    return launch_pdl_cluster("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p.cluster, p);
 }
 
 template <int LPK, int NCH>
@@ -352,17 +454,13 @@ inline int launch_decode_gp(const DecodeParams &p, int gp, cudaStream_t stream) 
     }
 }
 
-// Split-K pass followed by the combine, both on `stream`.
+// One launch, or the split-K pass followed by the combine, on `stream`.
 inline int launch_decode(DecodeParams p, const DecodePlan &pl, void *workspace, cudaStream_t stream) {
     char *ws = static_cast<char *>(workspace);
     p.bad_count = reinterpret_cast<int *>(ws);
     p.part_ml = reinterpret_cast<float2 *>(ws + kDecodeHeaderBytes);
     p.part_acc = reinterpret_cast<float *>(ws + kDecodeHeaderBytes + pl.ml_bytes);
-    p.chunk = pl.chunk, p.max_chunks = pl.max_chunks, p.n_sub = pl.n_sub;
-    if (cudaMemsetAsync(ws, 0, kDecodeHeaderBytes, stream) != cudaSuccess) {
-        cudaGetLastError();
-        return refuse("could not clear the decode workspace header");
-    }
+    p.chunk = pl.chunk, p.max_chunks = pl.max_chunks, p.n_sub = pl.n_sub, p.cluster = pl.cluster;
     int rc;
     if (pl.lpk == 8) rc = launch_decode_gp<8, 1>(p, pl.gp, stream);
     else if (pl.nch == 1) rc = launch_decode_gp<16, 1>(p, pl.gp, stream);
@@ -371,9 +469,9 @@ inline int launch_decode(DecodeParams p, const DecodePlan &pl, void *workspace, 
     else rc = launch_decode_gp<16, 4>(p, pl.gp, stream);
     if (rc) return rc;
     g_last_path = "decode-splitk";
+    if (pl.cluster) return 0;
     const dim3 cgrid((unsigned)p.n_heads, (unsigned)p.batch);
-    return ZT_LAUNCH("decode_combine_kernel", stream,
-                     decode_combine_kernel<<<cgrid, 128, 0, stream>>>(p));
+    return launch_pdl("decode_combine_kernel", decode_combine_kernel, cgrid, dim3(128), 0, stream, p);
 }
 
 }  // namespace zt

@@ -1002,8 +1002,7 @@ int zt_attn_decode_static(const float *q, const float *k_cache, const float *v_c
     p.batch = batch, p.n_ctx = n_ctx, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads, p.dim = dim;
     p.cache_batch_stride = (long long)n_ctx * n_kv_heads * dim;
     p.scale_log2 = kLog2e / sqrtf((float)dim);
-    // launch_decode clears the scratch's header (the bad-sequence counter) on `stream` first;
-    // every other word of the scratch that the combine step reads is written by this call.
+    // every word of the scratch that the combine step or the host reads is written by this call
     return launch_decode(p, pl, scratch, (cudaStream_t)stream);
 }
 
@@ -1030,9 +1029,10 @@ int zt_kv_append(float *k_cache, float *v_cache, int *n_keys, const float *k_new
     if (need_device()) return 1;
     g_last_path = "kv-append";
     cudaStream_t s = (cudaStream_t)stream;
-    return ZT_LAUNCH("kv_append_kernel", s,
-                     kv_append_kernel<<<(unsigned)batch, 256, 0, s>>>(k_cache, v_cache, n_keys, k_new, v_new,
-                                                                      full_count, n_ctx, n_kv_heads * dim));
+    const int width = n_kv_heads * dim;
+    const bool vec = width % 4 == 0 && aligned16(k_cache) && aligned16(v_cache) && aligned16(k_new) && aligned16(v_new);
+    return launch_pdl("kv_append_kernel", vec ? kv_append_kernel<true> : kv_append_kernel<false>, dim3((unsigned)batch), dim3(256), 0, s,
+                      k_cache, v_cache, n_keys, k_new, v_new, full_count, n_ctx, width);
 }
 
 }  // extern "C"

@@ -127,13 +127,34 @@ inline const DeviceInfo *device_info() {
     return &d;
 }
 
+// Function attributes are set once per (kernel, device, value): asking the driver on every launch costs more host time
+// than the launch's own bookkeeping.  Returns whether `value` is already known to hold.
+inline bool attribute_known(const void *fn, int attr, size_t value, bool record) {
+    struct Entry { const void *fn; int dev, attr; size_t value; };
+    static std::vector<Entry> known;
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    for (Entry &e : known)
+        if (e.fn == fn && e.dev == dev && e.attr == attr) {
+            if (record && value > e.value) e.value = value;
+            return value <= e.value;
+        }
+    if (record) known.push_back(Entry{fn, dev, attr, value});
+    return record;
+}
+
 // Opt a kernel into more than 48 KiB of dynamic shared memory; a refusal, not an exit
 // (src/cuda/attn_kernels.cu:822-830).
 inline int optin_smem(const void *fn, size_t bytes) {
-    if (bytes <= 48u * 1024u) return 0;
+    if (bytes <= 48u * 1024u || attribute_known(fn, (int)cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, false)) return 0;
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) return 0;
+    if (e == cudaSuccess) {
+        attribute_known(fn, (int)cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, true);
+        return 0;
+    }
     return refuse("the device would not grant %zu bytes of shared memory per block: %s", bytes,
                   cudaGetErrorString(e));
 }
@@ -147,6 +168,24 @@ inline int launch_pdl(const char *name, void (*kernel)(P...), dim3 grid, dim3 bl
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
     cfg.attrs = attr, cfg.numAttrs = 1;
+    const int pi = prof_begin(stream);
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    prof_end(pi, name, stream);
+    return launch_failed(name);
+}
+
+// The same for a grid of thread-block clusters of `cluster` blocks along x.
+template <typename... P, typename... A>
+inline int launch_pdl_cluster(const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              int cluster, const A &...args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+    cfg.attrs = attr, cfg.numAttrs = 2;
     const int pi = prof_begin(stream);
     cudaLaunchKernelEx(&cfg, kernel, args...);
     prof_end(pi, name, stream);

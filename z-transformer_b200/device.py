@@ -152,9 +152,12 @@ class Attn:
 
     def forward_at(self, group_q: int, max_tile: int, q_offset: int, n_keys: int, t: int) -> None:
         """device.zig:387-398."""
-        import torch
         forward_bounds(self.c_t, q_offset, n_keys, t)
         b = self._buf
+        if _lib.native().forward_at(b["q"], b["k"], b["v"], b["out"], t, self.c_heads, self.c_kv_heads, self.c_dim,
+                                    group_q, max_tile, q_offset, n_keys):
+            return
+        import torch
         with torch.cuda.device(self.device):
             rc = _lib.load().zt_attn_forward(b["q"].data_ptr(), b["k"].data_ptr(), b["v"].data_ptr(),
                                              b["out"].data_ptr(), t, self.c_heads, self.c_kv_heads,

@@ -41,10 +41,11 @@ class Layer:
         """Start from given per-sequence fill counts (a ragged batch whose rows were written directly)."""
         import torch
         lens = torch.as_tensor(lens, dtype=torch.int32)
-        if lens.shape != (self.batch,) or int(lens.min()) < 0 or int(lens.max()) > self.n_ctx:
+        low, high = map(int, torch.aminmax(lens)) if lens.shape == (self.batch,) else (-1, 0)
+        if low < 0 or high > self.n_ctx:
             raise DimensionMismatch("kv_cache.Layer.set_lens")
-        self._len_bound = int(lens.max())
-        self.len.copy_(lens.to(self.len.device))
+        self._len_bound = high
+        self.len.copy_(lens)
 
     def check_append(self, k_rows, v_rows) -> None:
         """Every refusal of append, made without writing anything: widths, placement, and Full."""
@@ -62,6 +63,9 @@ class Layer:
     def append(self, k_rows, v_rows) -> None:
         """One new row per sequence ([batch, width]); refuses, writing nothing, when any
         sequence is full or a width is wrong (src/kv_cache.zig:88-95)."""
+        if self._len_bound < self.n_ctx and _lib.native().kv_append(self.k, self.v, self.len, k_rows, v_rows, self._full):
+            self._len_bound += 1
+            return
         self.check_append(k_rows, v_rows)
         self._append_unchecked(k_rows, v_rows)
 

@@ -8,7 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from ._build import LIB_PATH
+from ._build import LIB_PATH, TORCH_EXT_PATH
 
 _vp, _i, _sz, _d = C.c_void_p, C.c_int, C.c_size_t, C.c_double
 
@@ -74,6 +74,27 @@ def load():
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The native host side of the per-step calls (csrc/host/zt_torch.cpp); raises when it has not been built."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries are what the extension links against)
+        load()
+        if not os.path.exists(TORCH_EXT_PATH):
+            raise RuntimeError(f"{TORCH_EXT_PATH} is missing: build it with `python -c \"import __graft_entry__ as g; g.build()\"`.")
+        loader = importlib.machinery.ExtensionFileLoader("_zt_torch", TORCH_EXT_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_zt_torch", loader))
+        loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def last_error() -> str:

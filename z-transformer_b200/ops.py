@@ -56,6 +56,14 @@ def attention_forward(q, k, v, n_heads, n_kv_heads, head_dim, *, want_lse=False,
     keep: a BackwardWorkspace of this shape; the forward's operand planes of q, k, v are left in it, and a
     backward given it with kept=True (the caller's word that q, k, v were not written in between) skips
     converting them again."""
+    if keep is None or keep.shape == (*q.shape[:2], n_heads, n_kv_heads, head_dim):
+        done = _lib.native().attention_forward(q, k, v, n_heads, n_kv_heads, head_dim, want_lse,
+                                               None if keep is None else keep.buf, 0 if keep is None else keep.nbytes)
+        if done:
+            if keep is not None:
+                keep.token = done[2]
+            return done[:2] if want_lse else done[0]
+    # (2-D tensors, and whatever has to be refused)
     import torch
     _head_config(n_heads, n_kv_heads, head_dim)
     squeeze = q.dim() == 2
@@ -99,6 +107,16 @@ def attention_backward(q, k, v, out, lse, dout, n_heads, n_kv_heads, head_dim, *
     workspace: a BackwardWorkspace of this shape (one is allocated per call otherwise).
     kept: the workspace was the `keep` of the forward of these very q, k, v and they have not been written
     since: the backward then uses the planes the forward left there (refused if they are gone)."""
+    if workspace is not None and workspace.shape == (*q.shape[:2], n_heads, n_kv_heads, head_dim):
+        token = workspace.token if kept else 0
+        done = _lib.native().attention_backward(q, k, v, n_heads, n_kv_heads, head_dim, out, lse, dout, workspace.buf,
+                                                workspace.nbytes, token)
+        if done is not None:
+            if kept:
+                workspace.token = 0
+            if not done:
+                raise ConfigRefused(_lib.last_error())
+            return done
     import torch
     _head_config(n_heads, n_kv_heads, head_dim)
     squeeze = q.dim() == 2
@@ -294,9 +312,16 @@ class AttentionBlock:
         """y = (attention(rope(q), rope(k), v)) . wo.  fused: one call of zt_attn_block_forward (the attention
         kernel's epilogue leaves ctx as the projection's operand planes); otherwise the two calls one after the
         other -- same numbers, one more pass over ctx."""
+        B, T, H, Hkv, D = self.shape
+        if fused and q.shape[:2] == (B, T) and wo.shape[-1:] == (self.d_model,):
+            done = _lib.native().block_forward(q, k, v, H, Hkv, D, wo, self.rope_ws.buf, self.rope_ws.nbytes,
+                                               self.proj_ws.buf, self.proj_ws.nbytes, pos, self.theta)
+            if done:
+                y, ctx, lse, self.rope_ws.token = done
+                self.saved = (q, k, v, wo, ctx, lse, pos)
+                return y
         import ctypes
         import torch
-        B, T, H, Hkv, D = self.shape
         if not fused:
             ctx, lse = attention_forward_rope(q, k, v, H, Hkv, D, pos=pos, theta=self.theta, workspace=self.rope_ws,
                                               want_lse=True)
@@ -329,6 +354,13 @@ class AttentionBlock:
         q, k, v, wo, ctx, lse, pos = self.saved
         self.saved = None
         B, T, H, Hkv, D = self.shape
+        done = _lib.native().block_backward(q, k, v, H, Hkv, D, wo, ctx, lse, dy, dwo, self.rope_ws.buf, self.rope_ws.nbytes,
+                                            self.proj_ws.buf, self.proj_ws.nbytes, pos, self.theta, self.rope_ws.token)
+        if done is not None:
+            self.rope_ws.token = 0
+            if not done:
+                raise ConfigRefused(_lib.last_error())
+            return done
         dctx = proj_backward(ctx, wo, dy, dwo, workspace=self.proj_ws)
         return attention_backward_rope(q, k, v, ctx, lse, dctx, H, Hkv, D, pos=pos, theta=self.theta,
                                        workspace=self.rope_ws, kept=self.rope_ws.token != 0)
@@ -356,6 +388,11 @@ class DecodeWorkspace:
 def decode_attention(q, k_cache, v_cache, n_keys, n_heads, n_kv_heads, head_dim, *, workspace=None,
                      want_lse=False, out=None):
     """decode.attnStep for a batch: q [B, H*D], caches [B, n_ctx, Hkv*D], n_keys int32 [B]."""
+    if workspace is not None:
+        done = _lib.native().decode(q, k_cache, v_cache, n_keys, n_heads, n_kv_heads, head_dim, workspace.buf,
+                                    workspace.nbytes, out, want_lse)
+        if done:
+            return done if want_lse else done[0]
     import torch
     _head_config(n_heads, n_kv_heads, head_dim)
     _need_cuda_f32(q, k_cache, v_cache)
