@@ -7,8 +7,8 @@
 //   * split-K over the context: block (chunk, kv head, sequence) reads a fixed-size
 //     chunk of keys, so ragged lengths balance by themselves and a short batch
 //     still fills the machine;
-//   * a K/V row is read by a group of LPK lanes as 128-bit, fully coalesced,
-//     no-L1-allocate loads, several keys in flight per lane before any is used;
+//   * a K/V row is read by a group of LPK lanes as 128-bit, fully coalesced asynchronous
+//     copies into shared memory, several steps ahead of their use;
 //   * a row is read once and dotted against every query head of the group held
 //     in registers; lane-group shuffles finish each dot;
 //   * online softmax in the log2 domain per lane group, merged across lane
@@ -44,14 +44,6 @@ struct DecodeParams {
     float scale_log2;
 };
 
-__device__ __forceinline__ float4 ldg_stream(const float *ptr) {
-    float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(ptr));
-    return v;
-}
-
 // ---- thread-block clusters ----------------------------------------------------------------------
 __device__ __forceinline__ void cluster_arrive() {
     __syncwarp();
@@ -78,26 +70,43 @@ __device__ __forceinline__ void count_bad_sequences(const DecodeParams &p) {
     if (threadIdx.x == 0) *p.bad_count = total;
 }
 
-template <int NCH, int GP>
+constexpr float kNoKey = -3.402823466e38f;  // the running maximum before the first key
+constexpr float kDecodeLazy = 8.f;          // a maximum moves when it is outgrown by 2^8
+
+template <int LPK, int NCH, int GP>
 struct DecodeCfg {
-    // Keys in flight per lane group, and blocks per SM, from a register estimate:
-    // K and V staging (8 floats per chunk per key) + q and accumulators (8 per chunk per head).
-    static constexpr int kUnroll = (NCH >= 3 || NCH * GP >= 8) ? 2 : 4;
-    static constexpr int kRegEstimate = kUnroll * NCH * 8 + GP * NCH * 8 + 28;
-    static constexpr int kMinBlocks = kRegEstimate > 124 ? 1 : 2;
+    // Keys a lane group takes per step: at most as many (key, head) pairs as it has lanes, and 128 bytes a thread.
+    static constexpr int kUnroll = (4 / NCH < 1 ? 1 : 4 / NCH) * GP > LPK ? LPK / GP : (4 / NCH < 1 ? 1 : 4 / NCH);
+    // Blocks per SM from a register estimate (q and accumulators: 8 floats per chunk per head), stages from what is left
+    // of shared memory (96 KB or 192 KB a block).
+    static constexpr int kMinBlocks = GP * NCH * 8 + 56 > 128 ? 1 : 2;
+    static constexpr int kStageBytes = kDecodeThreads * kUnroll * NCH * 2 * 16;
+    static constexpr int kFit = (kMinBlocks == 2 ? 96 : 192) * 1024 / kStageBytes;
+    static constexpr int kStages = kFit > 8 ? 8 : kFit;
 };
 
 // LPK lanes share one key row; each lane holds NCH float4 chunks of it (chunk index
 // li + LPK * c); GP query heads are processed per pass.
 // CLUSTER: the blocks of a cluster (x) divide the sequence's keys evenly and finish the rows among themselves;
 // otherwise block x takes the x-th chunk of p.chunk keys and leaves a partial result.
+//
+// The loads run kStages - 1 steps ahead through slots of shared memory that belong to one thread each, filled by
+// cp.async and waited for by that thread alone: no barrier in the loop, and the memory system always has 64 KB a block
+// to work on.  (Held in registers, a step's loads could not go out before the step before had been used up: batch 64, 8192
+// keys, 32/8 heads of 128 took 785 us, 5.5 TB/s; now 636 us, 6.75 TB/s.)
+// The U GP dots of a step are summed over the lane group by exchanging halves -- V - 1 + log2(LPK / V) shuffles instead of
+// V log2(LPK) -- which leaves each lane the sum of one (key, head) pair; that lane alone takes the exponential and keeps
+// the head's maximum and its share of the denominator, and hands P out to the others.
 template <int LPK, int NCH, int GP, bool CLUSTER>
-__global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks)
+__global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<LPK, NCH, GP>::kMinBlocks)
     decode_splitk_kernel(const DecodeParams p) {
-    constexpr int U = DecodeCfg<NCH, GP>::kUnroll;
+    using Cfg = DecodeCfg<LPK, NCH, GP>;
+    constexpr int U = Cfg::kUnroll, S = Cfg::kStages;
+    constexpr int V = U * GP, SP = LPK / V;                // (key, head) pairs of a step; lanes that end up with the same one
     constexpr int GPW = 32 / LPK;                          // lane groups per warp
     constexpr int NG = (kDecodeThreads / 32) * GPW;        // lane groups per block
-    extern __shared__ float smem[];
+    static_assert(V <= LPK && (V & (V - 1)) == 0, "a lane for every pair");
+    extern __shared__ __align__(16) float smem[];          // the ring; the merge's records afterwards
 
     const int b = blockIdx.z;
     const int group = p.n_heads / p.n_kv_heads;
@@ -127,6 +136,31 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks
     const int gi = warp * GPW + lane / LPK;
     const int dim = p.dim, n_chunks4 = dim >> 2;
     const long long kvw = (long long)p.n_kv_heads * dim;
+    const long long first = b * p.cache_batch_stride + (long long)(c0 + gi) * kvw + (long long)g * dim + li * 4;
+    const float *kb = p.k_cache + first, *vb = p.v_cache + first;
+    const int n_mine = c1 - c0 - gi;  // this lane group's keys are the i < n_mine with i a multiple of NG
+    const int n_steps = c1 > c0 ? (c1 - c0 + NG * U - 1) / (NG * U) : 0;
+    const float4 *ring = reinterpret_cast<const float4 *>(smem) + threadIdx.x;  // [S][U][NCH][2][threads]
+    const uint32_t ring_u32 = (uint32_t)__cvta_generic_to_shared(ring);
+    const auto fetch = [&](int step) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = (step * U + u) * NG;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                const bool in = i < n_mine && li + LPK * c < n_chunks4;
+                const long long off = (long long)i * kvw + LPK * c * 4;
+                const uint32_t dst = ring_u32 + (uint32_t)((((step % S) * U + u) * NCH + c) * 2 * kDecodeThreads * 16);
+                copy16_async(dst, in ? kb + off : p.k_cache, in);
+                copy16_async(dst + kDecodeThreads * 16, in ? vb + off : p.v_cache, in);
+            }
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < S - 1; ++i) {
+        if (i < n_steps) fetch(i);
+        copy_async_commit();
+    }
 
     // This lane's slices of the group's query rows, pre-multiplied by log2(e)/sqrt(dim).
     float4 qr[GP][NCH];
@@ -144,86 +178,95 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<NCH, GP>::kMinBlocks
             qr[hh][c] = x;
         }
 
-    float m[GP], l[GP];
+    // of the pair this lane ends up with, key `own / GP` of a step and head `own % GP`:
+    const int own_key = (li / SP) / GP * NG;
+    float m_own = kNoKey, l_own = 0.f;
     float4 acc[GP][NCH];
 #pragma unroll
-    for (int hh = 0; hh < GP; ++hh) {
-        m[hh] = -INFINITY, l[hh] = 0.f;
+    for (int hh = 0; hh < GP; ++hh)
 #pragma unroll
         for (int c = 0; c < NCH; ++c) acc[hh][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-
-    const float *kb = p.k_cache + b * p.cache_batch_stride + (long long)g * dim;
-    const float *vb = p.v_cache + b * p.cache_batch_stride + (long long)g * dim;
 
     // The trip count is the same for every lane of the block (the shuffles below name the
     // whole warp); a lane group whose keys run out early carries -inf scores instead.
-    for (int base = c0; base < c1; base += NG * U) {
-        const int s = base + gi;
-        float4 kf[U][NCH], vf[U][NCH];
-        // all loads of this step are issued before any is consumed
+    for (int step = 0; step < n_steps; ++step) {
+        copy_async_wait<S - 2>();
+        if (step + S - 1 < n_steps) fetch(step + S - 1);  // into the slot that step - 1 has used up
+        copy_async_commit();
+        const float4 *slot = ring + (step % S) * (U * NCH * 2 * kDecodeThreads);
+        float d[V];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int key = s + u * NG;
+#pragma unroll
+            for (int hh = 0; hh < GP; ++hh) d[u * GP + hh] = 0.f;
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
-                const int ch = li + LPK * c;
-                if (key < c1 && ch < n_chunks4) {
-                    kf[u][c] = ldg_stream(kb + (long long)key * kvw + ch * 4);
-                    vf[u][c] = ldg_stream(vb + (long long)key * kvw + ch * 4);
-                } else {
-                    kf[u][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    vf[u][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 kf = slot[(u * NCH + c) * 2 * kDecodeThreads];
+#pragma unroll
+                for (int hh = 0; hh < GP; ++hh) {
+                    float &x = d[u * GP + hh];
+                    x = fmaf(kf.x, qr[hh][c].x, x), x = fmaf(kf.y, qr[hh][c].y, x);
+                    x = fmaf(kf.z, qr[hh][c].z, x), x = fmaf(kf.w, qr[hh][c].w, x);
                 }
             }
         }
-        float sc[U][GP];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int n = V / 2, off = LPK / 2; off > 0; n >>= 1, off >>= 1) {
+            if (n > 0) {
+                const bool up = (lane & off) != 0;
+#pragma unroll
+                for (int i = 0; i < n; ++i) {
+                    const float send = up ? d[i] : d[i + n], keep = up ? d[i + n] : d[i];
+                    d[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+            } else {
+                d[0] += __shfl_xor_sync(0xffffffffu, d[0], off);
+            }
+        }
+        const float sc = (step * U * NG + own_key < n_mine) ? d[0] : -INFINITY;
+        if (__any_sync(0xffffffffu, sc > m_own + kDecodeLazy)) {
+            float mx = fmaxf(m_own, sc);
+#pragma unroll
+            for (int off = SP * GP; off < LPK; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            const float f = ex2(m_own - mx);
+            l_own *= f, m_own = mx;
 #pragma unroll
             for (int hh = 0; hh < GP; ++hh) {
-                float d = 0.f;
+                const float fh = __shfl_sync(0xffffffffu, f, hh * SP, LPK);
 #pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    d = fmaf(kf[u][c].x, qr[hh][c].x, d);
-                    d = fmaf(kf[u][c].y, qr[hh][c].y, d);
-                    d = fmaf(kf[u][c].z, qr[hh][c].z, d);
-                    d = fmaf(kf[u][c].w, qr[hh][c].w, d);
-                }
-#pragma unroll
-                for (int off = LPK / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-                sc[u][hh] = (s + u * NG < c1) ? d : -INFINITY;
+                for (int c = 0; c < NCH; ++c) acc[hh][c].x *= fh, acc[hh][c].y *= fh, acc[hh][c].z *= fh, acc[hh][c].w *= fh;
             }
+        }
+        const float p_own = ex2(sc - m_own);  // exp2(-inf) = 0 for absent keys
+        l_own += p_own;
 #pragma unroll
-        for (int hh = 0; hh < GP; ++hh) {
-            float mx = m[hh];
+        for (int u = 0; u < U; ++u) {
+            float pe[GP];
 #pragma unroll
-            for (int u = 0; u < U; ++u) mx = fmaxf(mx, sc[u][hh]);
-            // With no real key so far mx is -inf; subtracting 0 instead keeps every
-            // exponent at -inf (factor 0) rather than -inf - -inf (NaN).
-            const float mxs = (mx == -INFINITY) ? 0.f : mx;
-            const float corr = ex2(m[hh] - mxs);
-            m[hh] = mx;
-            float ls = l[hh] * corr;
+            for (int hh = 0; hh < GP; ++hh) pe[hh] = __shfl_sync(0xffffffffu, p_own, (u * GP + hh) * SP, LPK);
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
-                acc[hh][c].x *= corr, acc[hh][c].y *= corr, acc[hh][c].z *= corr, acc[hh][c].w *= corr;
-            }
+                const float4 vf = slot[((u * NCH + c) * 2 + 1) * kDecodeThreads];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const float pe = ex2(sc[u][hh] - mxs);  // exp2(-inf) = 0 for absent keys
-                ls += pe;
-#pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    acc[hh][c].x = fmaf(pe, vf[u][c].x, acc[hh][c].x);
-                    acc[hh][c].y = fmaf(pe, vf[u][c].y, acc[hh][c].y);
-                    acc[hh][c].z = fmaf(pe, vf[u][c].z, acc[hh][c].z);
-                    acc[hh][c].w = fmaf(pe, vf[u][c].w, acc[hh][c].w);
+                for (int hh = 0; hh < GP; ++hh) {
+                    acc[hh][c].x = fmaf(pe[hh], vf.x, acc[hh][c].x), acc[hh][c].y = fmaf(pe[hh], vf.y, acc[hh][c].y);
+                    acc[hh][c].z = fmaf(pe[hh], vf.z, acc[hh][c].z), acc[hh][c].w = fmaf(pe[hh], vf.w, acc[hh][c].w);
                 }
             }
-            l[hh] = ls;
         }
     }
+    copy_async_wait<0>();
+    // every lane of the group learns every head's maximum and denominator
+#pragma unroll
+    for (int off = SP * GP; off < LPK; off <<= 1) l_own += __shfl_xor_sync(0xffffffffu, l_own, off);
+    float m[GP], l[GP];
+#pragma unroll
+    for (int hh = 0; hh < GP; ++hh) {
+        const float mo = __shfl_sync(0xffffffffu, m_own, hh * SP, LPK);
+        m[hh] = mo == kNoKey ? -INFINITY : mo;
+        l[hh] = __shfl_sync(0xffffffffu, l_own, hh * SP, LPK);
+    }
+    __syncthreads();  // the ring's slots are the merge's records from here on
 
     // Merge the lane groups of a warp.  A group that saw no key has m = -inf, l = 0.
 #pragma unroll
@@ -337,15 +380,20 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
     const int nchunks = (nk + p.chunk - 1) / p.chunk;
     const long long slot0 = ((long long)b * p.n_heads + h) * p.max_chunks;
     float mx = -INFINITY;
-    for (int c = 0; c < nchunks; ++c) mx = fmaxf(mx, p.part_ml[slot0 + c].x);
+    for (int c = threadIdx.x & 31; c < nchunks; c += 32) mx = fmaxf(mx, p.part_ml[slot0 + c].x);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     float lsum = 0.f;
-    for (int c = 0; c < nchunks; ++c) {
+    for (int c = threadIdx.x & 31; c < nchunks; c += 32) {
         const float2 ml = p.part_ml[slot0 + c];
         lsum = fmaf(ml.y, ex2(ml.x - mx), lsum);
     }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
     const float inv = 1.f / lsum;
     for (int j = threadIdx.x; j < p.dim; j += blockDim.x) {
         float a = 0.f;
+#pragma unroll 8
         for (int c = 0; c < nchunks; ++c)
             a = fmaf(p.part_acc[(slot0 + c) * p.dim + j], ex2(p.part_ml[slot0 + c].x - mx), a);
         orow[j] = a * inv;
@@ -431,18 +479,15 @@ inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads,
 
 template <int LPK, int NCH, int GP>
 inline int launch_decode_inst(const DecodeParams &p, cudaStream_t stream) {
-    if (p.cluster == 0) {
-        const size_t smem = (size_t)(kDecodeThreads / 32) * GP * (p.dim + 4) * sizeof(float);
-        const auto kernel = decode_splitk_kernel<LPK, NCH, GP, false>;
-        if (optin_smem((const void *)kernel, smem)) return 1;
-        const dim3 grid((unsigned)p.max_chunks, (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
-        return launch_pdl("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p);
-    }
-    const size_t smem = (size_t)(kDecodeThreads / 32 + 1) * GP * (p.dim + 4) * sizeof(float);
-    const auto kernel = decode_splitk_kernel<LPK, NCH, GP, true>;
+    using Cfg = DecodeCfg<LPK, NCH, GP>;
+    size_t smem = (size_t)Cfg::kStages * Cfg::kStageBytes;
+    const size_t merge = (size_t)(kDecodeThreads / 32 + 1) * GP * (p.dim + 4) * sizeof(float);
+    if (smem < merge) smem = merge;
+    const auto kernel = p.cluster ? decode_splitk_kernel<LPK, NCH, GP, true> : decode_splitk_kernel<LPK, NCH, GP, false>;
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)p.cluster, (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
-    return launch_pdl_cluster("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p.cluster, p);
+    const dim3 grid((unsigned)(p.cluster ? p.cluster : p.max_chunks), (unsigned)(p.n_kv_heads * p.n_sub), (unsigned)p.batch);
+    if (p.cluster) return launch_pdl_cluster("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p.cluster, p);
+    return launch_pdl("decode_splitk_kernel", kernel, grid, dim3(kDecodeThreads), smem, stream, p);
 }
 
 template <int LPK, int NCH>

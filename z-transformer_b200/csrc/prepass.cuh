@@ -127,11 +127,6 @@ __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int bl
     return w;
 }
 
-__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool in) {
-    const int bytes = in ? 16 : 0;  // (0: the 16 bytes are filled with zeros and src is not read)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-
 // LP lanes hold a unit, NC float4 each.  The loads run kStages - 1 steps of U units ahead through slots of shared memory
 // that belong to one thread each (so nothing but the thread's own copies is waited for): held in registers instead,
 // the loads of a step would stall on the arithmetic of the step before (heads of 256, batch 8, T 1024: 4.1 TB/s against 5.4).
@@ -167,7 +162,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
                 if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        copy_async_commit();
     };
     pdl_wait();
     pdl_launch();
@@ -175,7 +170,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     for (int i = 0; i < S - 1; ++i) fetch(i);
     float amax = 0.f, nmax = 0.f;
     for (int step = 0; step < n_steps; ++step) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        copy_async_wait<S - 2>();
         float sq[U], de[U];
 #pragma unroll
         for (int k = 0; k < U; ++k) {
