@@ -22,6 +22,8 @@ def normal(oracle, shape, stream):
 @pytest.mark.parametrize("B,T,H,Hkv,D", [
     (2, 33, 4, 2, 36), (1, 64, 3, 1, 40), (1, 1, 4, 2, 64), (2, 65, 4, 4, 60), (1, 2, 2, 1, 128), (1, 127, 4, 2, 68),
     (2, 129, 6, 2, 80), (1, 32, 4, 1, 124), (1, 100, 4, 2, 132), (1, 63, 2, 2, 200), (1, 257, 2, 1, 252), (3, 31, 8, 2, 256),
+    # few key tiles for the chip: the backward's walk is split by heads, then by ranges of query tiles
+    (1, 1000, 4, 2, 64), (1, 700, 3, 3, 40), (2, 300, 8, 1, 128), (1, 1100, 2, 1, 72),
 ])
 def test_widths_and_short_sequences(zt, oracle, B, T, H, Hkv, D):
     q, k, v, do = (normal(oracle, (B, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv, H)))
@@ -43,6 +45,9 @@ def test_widths_and_short_sequences(zt, oracle, B, T, H, Hkv, D):
     (129, 511, 700, 6, 3, 96), (40, 0, 64, 2, 2, 192), (70, 250, 320, 4, 2, 256), (96, 1000, 1500, 32, 8, 128),
     # many key tiles: the row sums leave the tensor core's accumulator every sixteen of them
     (129, 2900, 3100, 2, 1, 128), (300, 2100, 2400, 4, 1, 64), (40, 1500, 1540, 2, 1, 256),
+    # few rows: the keys are split over the chip (parts that some rows see nothing of, parts that sum in memory too)
+    (2, 700, 702, 4, 2, 64), (16, 3000, 3016, 2, 1, 96), (150, 5000, 5200, 4, 4, 64), (100, 2500, 2600, 2, 2, 256),
+    (700, 1, 701, 2, 1, 64), (250, 9000, 9250, 8, 2, 40),
 ])
 def test_windows_of_a_prompt(zt, oracle, T, q_offset, ctx, H, Hkv, D):
     """device.Attn.forward_at: rows at q_offset over the first q_offset + T keys; what lies beyond is never read."""
@@ -61,6 +66,18 @@ def test_windows_of_a_prompt(zt, oracle, T, q_offset, ctx, H, Hkv, D):
     close(got, ref, "window")
     # the CUDA-core kernels served these calls with rounded f32 sums: as a whole no further off than they are
     assert float(np.linalg.norm(got.cpu().numpy() - ref) / np.linalg.norm(ref)) <= 5e-6
+
+
+def test_split_launches_are_reproducible(zt, oracle):
+    """Parts are put together in a fixed order: out, lse, dk and dv come out bit for bit the same (dq is summed in memory)."""
+    T, H, Hkv, D = 900, 4, 1, 64
+    q, k, v, do = (torch.from_numpy(normal(oracle, (1, T, w * D), i)).cuda() for i, w in enumerate((H, Hkv, Hkv, H)))
+    runs = []
+    for _ in range(2):
+        o, lse = zt.attention_forward(q, k, v, H, Hkv, D, want_lse=True)
+        runs.append((o, lse, *zt.attention_backward(q, k, v, o, lse, do, H, Hkv, D)[1:]))
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("T,H,Hkv,D,pos", [(70, 4, 2, 40, 3), (150, 2, 1, 136, 0), (90, 2, 2, 68, 5)])

@@ -40,6 +40,7 @@
 #include "rope_kernels.cuh"
 #include "tc_common.cuh"
 #include "tc_fwd.cuh"
+#include "tc_split.cuh"
 #include "zt_common.cuh"
 
 namespace zt {
@@ -68,6 +69,8 @@ struct BwdParams {
     int dim_out;     // the tensors' head_dim, at most the tile's D
     const float2 *rope_t;  // null, or the (cos, sin) table transposed, [dim_out / 2][T]: dq leaves as R^T of what was computed
     float scale, scale_log2;
+    BwdParts parts;     // how the walk of a key tile is split; more than one part: dk, dv are the first part's,
+    long long dkv_part; // and this many elements lie between two parts'
     float p_scale;  // P is multiplied by this power of two before its 16-bit split
 };
 
@@ -1034,6 +1037,7 @@ struct BwdWorkspace {
     float *rnorm;  // [batch, T, n_heads]
     __half *qs_planes;  // the row-scaled copy of q's planes (the fused and the wide-head backward read it for dK)
     uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
+    float *parts;       // partial results of a split forward, then of a split backward (tc_split.cuh)
     size_t total_bytes;
 };
 
@@ -1055,6 +1059,8 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.rnorm = reinterpret_cast<float *>(c + off), off += up((size_t)batch * T * n_heads * sizeof(float));
     w.qs_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
+    const size_t pf = fwd_parts_floats(batch, T, n_heads, dim, 0), pb = dim <= 128 ? bwd_parts_floats(batch, T, n_heads, n_kv_heads, dim) : 0;
+    w.parts = reinterpret_cast<float *>(c + off), off += up((pf > pb ? pf : pb) * sizeof(float));
     w.total_bytes = off;
     return w;
 }

@@ -79,14 +79,26 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     FusedShared *sh = reinterpret_cast<FusedShared *>(sG + 2 * QP);
 
     const int warp = threadIdx.x >> 5;
-    const int g = blockIdx.x, kt = (int)blockIdx.y, b = blockIdx.z;
+    const int g = blockIdx.x, kt = (int)blockIdx.y, b = (int)blockIdx.z / p.parts.n(), part = (int)blockIdx.z - b * p.parts.n();
     const int group = p.n_heads / p.n_kv_heads;
     const int s0 = kt * 128;
-    const int n_q = (p.T + BQ - 1) / BQ, qi0 = s0 / BQ;
+    // this CTA's part of the walk: heads [head0, head0 + n_heads_mine) and query tiles [qi0, n_q)
+    const int n_heads_mine = group / p.parts.heads, head0 = g * group + part / p.parts.ranges * n_heads_mine;
+    int n_q = (p.T + BQ - 1) / BQ, qi0 = s0 / BQ;
+    if (p.parts.ranges > 1) {
+        const int per = (n_q - qi0 + p.parts.ranges - 1) / p.parts.ranges;
+        qi0 += part % p.parts.ranges * per;
+        if (qi0 >= n_q) {
+            pdl_wait();
+            pdl_launch();
+            return;  // (the whole CTA: nothing has been set up yet)
+        }
+        n_q = qi0 + per < n_q ? qi0 + per : n_q;
+    }
     const int per_head = n_q - qi0;
-    const int n_it = group * per_head;
+    const int n_it = n_heads_mine * per_head;
     const int B = p.batch;
-    Walk walk(group, per_head, qi0, n_q);
+    Walk walk(n_heads_mine, per_head, qi0, n_q);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) mbar_init(&sh->full_q[i], 1), mbar_init(&sh->free_q[i], 1);
@@ -136,7 +148,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 const int j = n_ql, s = j & 1;
                 // (its slot was last read by dK(j - 2))
                 if (j >= 2 && !fwait(&sh->free_q[s], (uint32_t)((((j >> 1) - 1) & 1)), sh)) { fgive_up(sh, 61), live = false; return; }
-                const int h = g * group + wq.hh, row = wq.qi * BQ;
+                const int h = head0 + wq.hh, row = wq.qi * BQ;
                 mbar_arrive_expect_tx(&sh->full_q[s], 2 * QP);
                 tma_load_4d(sQ + s * 2 * QP, &qmap, &sh->full_q[s], 0, row, h * NB, b);
                 tma_load_4d(sQ + s * 2 * QP + QP, &qmap, &sh->full_q[s], 0, row, h * NB, B + b);
@@ -146,7 +158,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 const int j = n_gl;
                 // (the one slot was last read by dV(j - 1))
                 if (j >= 1 && !fwait(&sh->free_g, (uint32_t)((j - 1) & 1), sh)) { fgive_up(sh, 61), live = false; return; }
-                const int h = g * group + wg.hh, row = wg.qi * BQ;
+                const int h = head0 + wg.hh, row = wg.qi * BQ;
                 mbar_arrive_expect_tx(&sh->full_g, 2 * QP);
                 tma_load_4d(sG, &gmap, &sh->full_g, 0, row, h * NB, b);
                 tma_load_4d(sG + QP, &gmap, &sh->full_g, 0, row, h * NB, B + b);
@@ -362,7 +374,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             if (tid >= 64 || it >= n_it) return 0.f;
             const int t = w.qi * BQ + tid;
             if (t >= p.T) return 0.f;
-            const long long idx = ((long long)b * p.T + t) * p.n_heads + g * group + w.hh;
+            const long long idx = ((long long)b * p.T + t) * p.n_heads + head0 + w.hh;
             if (set == 0) return __ldg(p.lse + idx) * kLog2e - lse_shift;
             float cq, rel;
             ds_row_scale(__ldg(p.rnorm + idx), rn_bits, vn_bits, cq, rel);
@@ -391,7 +403,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             const uint32_t acc = tmem + lane_base + (set < 2 ? cDV : cDK) + c0;
             const int j8 = lane & 7;
             const long long wo = (long long)p.n_kv_heads * p.dim_out;
-            float *dst = (set < 2 ? p.dv : p.dk) + ((long long)b * p.T + (key - j8)) * wo + (long long)g * p.dim_out + c0 + 4 * j8;
+            const int mine = (int)blockIdx.z - b * p.parts.n();  // (`part`, without a register held for it)
+            float *dst = (set < 2 ? p.dv : p.dk) + mine * p.dkv_part + ((long long)b * p.T + (key - j8)) * wo + (long long)g * p.dim_out + c0 + 4 * j8;
             const float f = set < 2 ? 1.0f / (p.p_scale * mdo) : p.scale / (mq * cmin);
 #pragma unroll 1
             for (int c = 0; c < D / 2; c += 32) {
@@ -474,7 +487,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                     float4 a;
                     a.x = __uint_as_float(r[4 * q4]) * fq[q4], a.y = __uint_as_float(r[4 * q4 + 1]) * fq[q4];
                     a.z = __uint_as_float(r[4 * q4 + 2]) * fq[q4], a.w = __uint_as_float(r[4 * q4 + 3]) * fq[q4];
-                    red_add_v4(p.dq + ((long long)b * p.T + t) * wq + (long long)(g * group + prev_hh) * p.dim_out + d0, a);
+                    red_add_v4(p.dq + ((long long)b * p.T + t) * wq + (long long)(head0 + prev_hh) * p.dim_out + d0, a);
                 }
             }
         };
@@ -620,7 +633,7 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
     size_t smem = fused_smem_bytes<D>();
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     if (optin_smem((const void *)attn_bwd_fused_tc<D>, smem)) return 1;
-    const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
+    const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)(p.batch * p.parts.n()));
     return launch_after("attn_bwd_fused_tc", attn_bwd_fused_tc<D>, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
 }
 inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
@@ -676,15 +689,16 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
     if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
     BwdMaps m;
-    if (!make_half_tile_map(&m.k128, w.k_planes, 2 * batch, T, wkv, td, 128) ||
-        !make_half_tile_map(&m.v128, w.v_planes, 2 * batch, T, wkv, td, 128) ||
-        !make_half_tile_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, wq, td, 64) ||
-        !make_half_tile_map(&m.g64, w.do_planes, 2 * batch, T, wq, td, 64) ||
-        !make_half_tile_map(&m.k64, w.k_planes, 2 * batch, T, wkv, td, 64) ||
-        !make_half_tile_map(&m.v64, w.v_planes, 2 * batch, T, wkv, td, 64) ||
-        !make_half_tile_map(&m.q128, w.q_planes, 2 * batch, T, wq, td, 128) ||
-        !make_half_tile_map(&m.g128, w.do_planes, 2 * batch, T, wq, td, 128))
-        return refuse("the TMA tensor maps for the backward could not be encoded.");
+    bool maps = make_half_tile_map(&m.k128, w.k_planes, 2 * batch, T, wkv, td, 128) &&
+                make_half_tile_map(&m.v128, w.v_planes, 2 * batch, T, wkv, td, 128) &&
+                make_half_tile_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, wq, td, 64) &&
+                make_half_tile_map(&m.g64, w.do_planes, 2 * batch, T, wq, td, 64);
+    if (!fused)
+        maps = maps && make_half_tile_map(&m.k64, w.k_planes, 2 * batch, T, wkv, td, 64) &&
+               make_half_tile_map(&m.v64, w.v_planes, 2 * batch, T, wkv, td, 64) &&
+               make_half_tile_map(&m.q128, w.q_planes, 2 * batch, T, wq, td, 128) &&
+               make_half_tile_map(&m.g128, w.do_planes, 2 * batch, T, wq, td, 128);
+    if (!maps) return refuse("the TMA tensor maps for the backward could not be encoded.");
     BwdParams p{};
     p.lse = lse, p.delta = delta;
     p.k_planes = w.k_planes, p.v_planes = w.v_planes, p.q_planes = w.q_planes, p.do_planes = w.do_planes;
@@ -700,7 +714,14 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     // dS is scaled inside the kernels (see "The scale of dS" in tc_bwd.cuh and the head of this file).
     p.p_scale = ldexpf(1.0f, 10);
     g_last_path = "tcgen05";
-    if (fused) return tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream);
+    if (fused) {
+        p.parts = bwd_parts(batch, T, n_heads, n_kv_heads);
+        if (p.parts.n() == 1) return tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream);
+        const long long n = (long long)batch * T * n_kv_heads * dim;
+        p.dk = w.parts, p.dv = w.parts + n, p.dkv_part = 2 * n;
+        if (tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream)) return 1;
+        return launch_bwd_join(w.parts, dk, dv, batch, T, n_kv_heads * dim, p.parts, stream);
+    }
     return td == 64 ? launch_bwd_tc_d<64>(m, p, stream) : launch_bwd_tc_d<128>(m, p, stream);
 }
 

@@ -302,10 +302,11 @@ __device__ __forceinline__ float tf32_round(float x) {
 // 0.45 ms here.
 inline int tc_tile_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : 256); }
 inline bool tc_takes_dim(int dim) { return dim % 4 == 0 && dim >= 32 && dim <= 256; }
-// Query rows from which the forward goes to the tensor cores: up to 32 rows the CUDA-core forward is one launch of
-// one row tile and the quicker of the two (32/8 heads of 128: 17 us against 28 at 32 rows, 29.5 against 28.5 at 48,
-// 57 against 31 at 127).  The backward has no such line: 47 against 111 us at 2 rows already.
-constexpr int kTcForwardMinRows = 33;
+// Keys from which the forward goes to the tensor cores: up to 32 the CUDA-core forward is one launch of one row and one
+// key tile and the quicker of the two (32/8 heads of 128: 17 us against 28 at 32 rows, 29.5 against 28.5 at 48, 57
+// against 31 at 127; a key tile more costs it 13 us, however few the rows).  The backward has no such line: 47
+// against 111 us at 2 rows already.
+constexpr int kTcForwardMinKeys = 33;
 
 // ---- host: tensor maps through the driver entry point (no link-time libcuda dependency) ---------
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

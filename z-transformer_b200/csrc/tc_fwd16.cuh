@@ -51,6 +51,8 @@ struct Params {
     float *out, *lse;                           // lse may be null
     int batch, T, n_heads, n_kv_heads;
     int q_offset;  // query row r stands at position q_offset + r of the keys: it sees keys 0 .. q_offset + r
+    int parts;     // CTAs along a query tile's keys; with more than one, out and lse are the parts' (see tc_split.cuh):
+    long long out_part, lse_part;  // elements from one part's to the next
     bool flush;    // O leaves the tensor core's accumulator every kFlushKeyTiles key tiles (see flush_row)
     int dim_out;  // the tensors' head_dim, at most the tile's D
     int ahead;    // attn_fwd_tc16 prefetches the query tile of the block this many places on in launch order; 0: none
@@ -178,11 +180,23 @@ __global__ void __launch_bounds__(kThreads, 1)
     // launch order (x fastest): a head's query tiles, late (long) ones first.  (Starting the heads of a sequence
     // tile by tile instead, which would shorten the tail, measured 3 % slower.)
     const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int h = blockIdx.y, b = (int)blockIdx.z / p.parts, part = (int)blockIdx.z - b * p.parts;
     const int g = h / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
-    const int n_tiles = (p.q_offset + rows_end + BN - 1) / BN;
+    int n_tiles = (p.q_offset + rows_end + BN - 1) / BN, jb = 0;  // key tiles of this CTA, and the first of them
+    if (p.parts > 1) {
+        const int per = (n_tiles + p.parts - 1) / p.parts;
+        jb = part * per;
+        n_tiles = n_tiles - jb < per ? n_tiles - jb : per;
+        if (n_tiles <= 0) {
+            pdl_wait();
+            pdl_launch();
+            if (threadIdx.x < 128 && t0 + threadIdx.x < p.T)
+                p.lse[part * p.lse_part + ((long long)b * p.T + t0 + threadIdx.x) * p.n_heads + h] = -INFINITY;
+            return;  // (the whole CTA: nothing has been set up yet)
+        }
+    }
     const int B = p.batch;
 
     if (threadIdx.x == 0) {
@@ -236,16 +250,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int s = j % 3;
                 if (j >= 3 && !fwait(&sh->free_k[s], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { fgive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_k[s], 2 * KP);
-                tma_load_4d(sK + s * 2 * KP, &kmap, &sh->full_k[s], 0, j * BN, g * NB, b);
-                tma_load_4d(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], 0, j * BN, g * NB, B + b);
+                tma_load_4d(sK + s * 2 * KP, &kmap, &sh->full_k[s], 0, (jb + j) * BN, g * NB, b);
+                tma_load_4d(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], 0, (jb + j) * BN, g * NB, B + b);
                 ++n_k;
             };
             auto load_v = [&](int j) {
                 const int s = j % 3;
                 if (j >= 3 && !fwait(&sh->free_v[s], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { fgive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v[s], 2 * KP);
-                tma_load_4d(sV + s * 2 * KP, &vmap, &sh->full_v[s], 0, j * BN, g * NB, b);
-                tma_load_4d(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], 0, j * BN, g * NB, B + b);
+                tma_load_4d(sV + s * 2 * KP, &vmap, &sh->full_v[s], 0, (jb + j) * BN, g * NB, b);
+                tma_load_4d(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], 0, (jb + j) * BN, g * NB, B + b);
                 ++n_v;
             };
             const int first = n_tiles < 3 ? n_tiles : 3;
@@ -358,11 +372,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         // reads and has in TMEM by now (a forward that flushes keeps no planes for a backward)
         FlushRow row0{nullptr, nullptr, p.dim_out}, row1{nullptr, nullptr, D};
         if (FLUSH && t < p.T) {
-            row0.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
+            row0.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row0.upper = row0.lower + D / 2;
-            __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * D + (long long)h * D;
-            row1.lower = reinterpret_cast<float *>(planes);
-            row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * D);
+            if (p.parts > 1) {  // (whose parts share the query rows: behind the parts' rows)
+                row1.lower = row0.lower + p.parts * p.out_part, row1.upper = row1.lower + D / 2;
+                row1.width = p.dim_out;
+            } else {
+                __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * D + (long long)h * D;
+                row1.lower = reinterpret_cast<float *>(planes);
+                row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * D);
+            }
         }
         for (int j = set; ok && j < n_tiles; j += 2) {
             if (!__all_sync(0xffffffffu, fwait(&sh->s_full[set], (uint32_t)((j >> 1) & 1), sh))) {
@@ -371,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 break;
             }
             tc_fence_after();
-            const int s0 = j * BN;
+            const int s0 = (jb + j) * BN;
             const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32(tmem + lane_base + cS, r0);
@@ -449,11 +468,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool two = n_tiles > 1;  // set 1 has an accumulator only then
             const float m0 = sh->fin_m[0][tid], l0 = sh->fin_l[0][tid];
             const float m1 = two ? sh->fin_m[1][tid] : -INFINITY, l1 = two ? sh->fin_l[1][tid] : 0.f;
-            const float mm = fmaxf(m0, m1);  // m0 is finite: key 0 is visible to every row
+            // (finite where the CTA has all the keys, key 0 being visible to every row; a part may hold none that a row sees)
+            const float mm = fmaxf(fmaxf(m0, m1), -3.0e38f);
             // (the merge is a running-maximum correction too, the only one where each set has a single tile)
             const float w0 = ZT_DEFECT(3) ? 1.f : ex2(m0 - mm), w1 = (m1 == -INFINITY) ? 0.f : (ZT_DEFECT(3) ? 1.f : ex2(m1 - mm));
             const float lsum = w0 * l0 + w1 * l1;
-            const float inv = 1.f / (lsum * mv);  // lsum, like O, carries kPScale
+            const float inv = lsum == 0.f ? 0.f : 1.f / (lsum * mv);  // lsum, like O, carries kPScale
             const float f0 = w0 * inv, f1 = w1 * inv;
             const float s0 = sh->fin_f[0][tid], s1 = sh->fin_f[1][tid];
             const bool add0 = FLUSH && s0 != -INFINITY && row0.lower != nullptr, add1 = FLUSH && s1 != -INFINITY && row1.lower != nullptr;
@@ -474,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
                         float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
-                        if (add1) x4 = flush_sum4(row1.at<D>(col), g1, false, x4);
+                        if (add1 && col < row1.width) x4 = flush_sum4(row1.at<D>(col), g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     const int ch = (set * (D / 2) + c + i) >> 2;
@@ -482,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
             if (set == 0 && p.lse && t < p.T)
-                p.lse[((long long)b * p.T + t) * p.n_heads + h] = (mm + log2f(lsum) - 7.0f) * kLn2;
+                p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (mm + log2f(lsum) - 7.0f) * kLn2;
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (!sh->abort) {
@@ -496,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int r = warp * 16 + i + lane / CH;
                 const float4 o4 = *reinterpret_cast<const float4 *>(sK + r * (D * 4) + ((ch ^ (r & (CH - 1))) << 4));
                 if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
-                    store_out4(p, ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
+                    store_out4(p, part * p.out_part + ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
             }
         }
     }
@@ -511,6 +531,7 @@ struct Workspace {
     uint32_t *vnmax;  // (in the backward's layout: the largest row norm of v, which the backward wants; else null)
     uint2 *part[3];   // the pre-pass's slots
     __half *q_planes, *k_planes, *v_planes;
+    float *parts;     // of a forward split along the keys
     size_t total_bytes;
 };
 
@@ -527,6 +548,7 @@ inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_h
     w.q_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.k_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
+    w.parts = reinterpret_cast<float *>(c + off), off += up(fwd_parts_floats(batch, T, n_heads, dim, q_offset) * sizeof(float));
     w.total_bytes = off;
     return w;
 }
@@ -538,7 +560,7 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     const auto kernel = p.flush ? attn_fwd_tc16<D, true> : attn_fwd_tc16<D, false>;
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
+    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
     return launch_after("attn_fwd_tc16", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
@@ -556,8 +578,8 @@ inline size_t tc_fwd16_workspace_bytes(int batch, int T, int n_heads, int n_kv_h
     return tcf16::workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim), q_offset).total_bytes;
 }
 
-inline bool tc_fwd16_supported(int batch, int T, int dim, const void *q, const void *k, const void *v, const void *out) {
-    if (!tc_takes_dim(dim) || T < kTcForwardMinRows || batch < 1) return false;
+inline bool tc_fwd16_supported(int batch, int T, int q_offset, int dim, const void *q, const void *k, const void *v, const void *out) {
+    if (!tc_takes_dim(dim) || q_offset + T < kTcForwardMinKeys || batch < 1) return false;
     auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     if (!al(q) || !al(k) || !al(v) || !al(out)) return false;
     const DeviceInfo *d = device_info();
@@ -581,7 +603,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
         w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;
         w.vnmax = bw.vnmax;
         for (int i = 0; i < 3; ++i) w.part[i] = bw.part[i];
-        w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes;
+        w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes, w.parts = bw.parts;
     }
     const int group = n_heads / n_kv_heads;
     const int wkv = n_kv_heads * td;
@@ -592,32 +614,12 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
     pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     if (launch_pass(pa, stream)) return 1;
-    if (td == 256) {
-        // head_dim 256 (and those padded to it): one head per CTA, K fetched block by block (attn_fwd_tc16x)
-        CUtensorMap kmap, vmap, qmap;
-        if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, 64, 64) ||
-            !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
-            !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
-            return refuse("the TMA tensor maps for the forward could not be encoded.");
-        tcf16::Params p{};
-        p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
-        p.out = out, p.lse = lse;
-        p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-        p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
-        p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
-        if (out_peers) p.out_peers = *out_peers;
-        p.scale_log2 = kLog2e / sqrtf((float)dim);
-        g_last_path = "tcgen05";
-        return tcf16::launch_x(kmap, vmap, qmap, p, stream);
-    }
-    // variant 0: two heads of a KV group per CTA (attn_fwd_tc16g) when the group has an even number of query heads
-    // and that still gives every SM a CTA, one head per CTA (attn_fwd_tc16) otherwise; 1: one head per CTA;
-    // 2: two heads per CTA whatever the number of CTAs (the group must be even).
-    CUtensorMap kmap, vmap, qmap;
-    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td, 64) ||
+    CUtensorMap kmap, vmap, qmap;  // (the widest tile fetches K block by block, see attn_fwd_tc16x)
+    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td == 256 ? 64 : td, 64) ||
         !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
         !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
+    const int sms = split_sm_count();
     tcf16::Params p{};
     p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
     p.out = out, p.lse = lse;
@@ -625,15 +627,26 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
     p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
     if (out_peers) p.out_peers = *out_peers;
-    p.ahead = device_info() ? device_info()->sm_count : 0;  // one CTA per SM
+    p.ahead = sms;  // one CTA per SM
     p.scale_log2 = kLog2e / sqrtf((float)dim);
+    p.parts = variant == 0 && !out_planes && p.out_peers.n == 0 ? fwd_parts(batch, T, n_heads, q_offset) : 1;
+    const long long rows = (long long)batch * T * n_heads;
+    if (p.parts > 1) {
+        p.out = w.parts, p.out_part = rows * dim;
+        p.lse = w.parts + p.parts * (q_offset > 0 ? 2 : 1) * p.out_part, p.lse_part = rows;
+    }
     g_last_path = "tcgen05";
-    // two heads per CTA halve the number of CTAs: not when that leaves SMs without one
+    // variant 0: two heads of a KV group per CTA (attn_fwd_tc16g) when the group has an even number of query heads
+    // and that still gives every SM a CTA (half as many CTAs), one head per CTA (attn_fwd_tc16) otherwise; 1: one head
+    // per CTA; 2: two heads per CTA whatever the number of CTAs (the group must be even).
     const long long pair_ctas = (long long)((T + 127) / 128) * (n_heads / 2) * batch;
-    if ((variant == 0 || variant == 2) && (n_heads / n_kv_heads) % 2 == 0 &&
-        (variant == 2 || (device_info() && pair_ctas >= device_info()->sm_count)))
-        return td == 64 ? tcf16::launch_g_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_g_d<128>(kmap, vmap, qmap, p, stream);
-    return td == 64 ? tcf16::launch_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_d<128>(kmap, vmap, qmap, p, stream);
+    const bool pairs = td != 256 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
+    int rc;
+    if (td == 256) rc = tcf16::launch_x(kmap, vmap, qmap, p, stream);
+    else if (pairs) rc = td == 64 ? tcf16::launch_g_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_g_d<128>(kmap, vmap, qmap, p, stream);
+    else rc = td == 64 ? tcf16::launch_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_d<128>(kmap, vmap, qmap, p, stream);
+    if (rc || p.parts == 1) return rc;
+    return launch_fwd_join(p.out, p.lse, out, lse, rows, dim, p.parts, stream);
 }
 
 }  // namespace zt

@@ -67,11 +67,23 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     const int warp = threadIdx.x >> 5;
     // launch order (x fastest): a head's query tiles, late (long) ones first
     const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int h = blockIdx.y, b = (int)blockIdx.z / p.parts, part = (int)blockIdx.z - b * p.parts;
     const int g = h / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
-    const int n_tiles = (p.q_offset + rows_end + BN - 1) / BN;
+    int n_tiles = (p.q_offset + rows_end + BN - 1) / BN, jb = 0;  // key tiles of this CTA, and the first of them
+    if (p.parts > 1) {
+        const int per = (n_tiles + p.parts - 1) / p.parts;
+        jb = part * per;
+        n_tiles = n_tiles - jb < per ? n_tiles - jb : per;
+        if (n_tiles <= 0) {
+            pdl_wait();
+            pdl_launch();
+            if (threadIdx.x < 128 && t0 + threadIdx.x < p.T)
+                p.lse[part * p.lse_part + ((long long)b * p.T + t0 + threadIdx.x) * p.n_heads + h] = -INFINITY;
+            return;  // (the whole CTA: nothing has been set up yet)
+        }
+    }
     const int B = p.batch;
 
     if (threadIdx.x == 0) {
@@ -112,15 +124,15 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             auto load_k_block = [&](int j, int c) {
                 if (j >= 1 && !xwait(&sh->free_k[c], (uint32_t)((j - 1) & 1), sh)) { xgive_up(sh, 61), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_k[c], 2 * KB);
-                tma_load_4d(sK + c * 2 * KB, &kmap, &sh->full_k[c], 0, j * BN, g * NB + c, b);
-                tma_load_4d(sK + c * 2 * KB + KB, &kmap, &sh->full_k[c], 0, j * BN, g * NB + c, B + b);
+                tma_load_4d(sK + c * 2 * KB, &kmap, &sh->full_k[c], 0, (jb + j) * BN, g * NB + c, b);
+                tma_load_4d(sK + c * 2 * KB + KB, &kmap, &sh->full_k[c], 0, (jb + j) * BN, g * NB + c, B + b);
                 ++n_k;
             };
             auto load_v = [&](int j) {
                 if (j >= 1 && !xwait(&sh->free_v, (uint32_t)((j - 1) & 1), sh)) { xgive_up(sh, 61), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v, 2 * KP);
-                tma_load_4d(sV, &vmap, &sh->full_v, 0, j * BN, g * NB, b);
-                tma_load_4d(sV + KP, &vmap, &sh->full_v, 0, j * BN, g * NB, B + b);
+                tma_load_4d(sV, &vmap, &sh->full_v, 0, (jb + j) * BN, g * NB, b);
+                tma_load_4d(sV + KP, &vmap, &sh->full_v, 0, (jb + j) * BN, g * NB, B + b);
                 ++n_v;
             };
             for (int c = 0; c < NB; ++c) load_k_block(0, c);
@@ -229,7 +241,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         FlushRow row{nullptr, nullptr, p.dim_out};
         if (FLUSH && t < p.T) {
-            row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
+            row.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row.upper = row.lower + D / 2;
         }
         for (int j = 0; ok && j < n_tiles; ++j) {
@@ -239,7 +251,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 break;
             }
             tc_fence_after();
-            const int s0 = j * BN;
+            const int s0 = (jb + j) * BN;
             const uint32_t cS = cS0 + (j & 1) * BN;
             const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
@@ -310,7 +322,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         uint8_t *stage = smem_raw;
         if (ok) {
             tc_fence_after();
-            const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
+            const float inv = l == 0.f ? 0.f : 1.f / (l * mv);  // l, like O, carries kPScale (0: a part without a key the row sees)
             const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * (D * 4);
@@ -328,7 +340,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & 31)) << 4)) = o4;
                 }
             }
-            if (p.lse && t < p.T) p.lse[((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
+            if (p.lse && t < p.T) p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
         }
         mbar_arrive_warp(&sh->staged);
         if (__all_sync(0xffffffffu, xwait(&sh->staged, 0, sh)) && !sh->abort) {
@@ -343,7 +355,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                     const int ch = half * 32 + lane;
                     const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * (D * 4) + ((ch ^ (r & 31)) << 4));
                     if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
-                        store_out4(p, ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
+                        store_out4(p, part * p.out_part + ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
                 }
             }
         }
@@ -358,7 +370,7 @@ inline int launch_x(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     const size_t smem = 3 * (size_t)(2 * 64 * 256 * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
     const auto kernel = p.flush ? attn_fwd_tc16x<true> : attn_fwd_tc16x<false>;
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)p.batch);
+    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
     return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
 }
 

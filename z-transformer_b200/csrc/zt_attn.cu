@@ -101,7 +101,7 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
 #ifndef ZT_NO_TC
     const int path = g_path.load();
     if ((path == 0 || path == 6 || path == 7 || path == 8) && n_kv_heads <= tcb::kPrepassMaxGroups &&
-        tc_fwd16_supported(batch, T, dim, q, k, v, out)) {
+        tc_fwd16_supported(batch, T, q_offset, dim, q, k, v, out)) {
         // The f16-split forward keeps its operand planes in the per-device arena (no entry point
         // of the forward takes a workspace); see device_arena for when that allocates.
         const size_t need = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim, q_offset);
@@ -342,7 +342,9 @@ int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     size_t need = kArenaBytes;  // the decode-shaped forward's partial results
 #ifndef ZT_NO_TC
     if (n_kv_heads <= tcb::kPrepassMaxGroups && tc_takes_dim(dim)) {
-        const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+        // (and, for windows of the sequence, the partial rows of a forward that is split until every SM has a block)
+        const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim) +
+                         (size_t)split_sm_count() * 128 * (2 * tc_tile_dim(dim) + 1) * sizeof(float);
         const size_t b = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
         need = f > need ? f : need;
         need = b > need ? b : need;
@@ -523,7 +525,7 @@ static int forward_keep_impl(const float *q, const float *k, const float *v, flo
     const int keep_path = g_path.load();
     if ((keep_path == 0 || keep_path == 6 || keep_path == 7 || keep_path == 8) && need > 0 && workspace && workspace_bytes >= need &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
-        tc_fwd16_supported(batch, T, dim, q, k, v, out)) {
+        tc_fwd16_supported(batch, T, 0, dim, q, k, v, out)) {
         if (launch_fwd_tc16(q, k, v, out, lse, workspace, batch, T, n_heads, n_kv_heads, dim, s, nullptr, true,
                             keep_path == 6 ? 1 : (keep_path == 7 ? 2 : 0), nullptr, out_peers))
             return 1;
@@ -681,7 +683,7 @@ static int forward_rope_impl(const float *q, const float *k, const float *v, flo
 #ifndef ZT_NO_TC
     // (the pre-pass rotates four elements at a time: a head's halves must be multiples of four)
     if ((g_path.load() == 0 || g_path.load() == 8) && n_kv_heads <= tcb::kPrepassMaxGroups && dim % 8 == 0 &&
-        tc_fwd16_supported(batch, T, dim, q, k, v, out) &&
+        tc_fwd16_supported(batch, T, 0, dim, q, k, v, out) &&
         w.inner_bytes >= tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim)) {
         // the planes (rotated q and k among them) go where the backward keeps its own: the rope backward that
         // follows with the same workspace, tensors, pos and theta converts only dout
