@@ -4,7 +4,9 @@
 // fixed order, so results stay reproducible.
 // B200, us before -> after: forward of a window of 64 rows at 4000 keys, 8/2 heads of 128, 92 -> 33; 300 rows at 8000
 // keys, 12/4 heads of 64, 151 -> 55; 128 rows at 8000 keys, 32/8 heads of 256, 610 -> 225; forward and backward of one
-// sequence, 32/8 heads of 128, T 500 175 -> 96, T 1000 323 -> 228; 4/2 heads of 32, T 2000 211 -> 105.
+// sequence, 32/8 heads of 128, T 500 175 -> 96, T 1000 323 -> 228; 4/2 heads of 32, T 2000 211 -> 105;
+// 4/2 heads of 64, T 8000 813 -> 526 (126 blocks, half of them walking less than half of the longest); batch 4,
+// 16/4 heads of 80, T 1000 373 -> 359.
 #pragma once
 
 #include "tc_common.cuh"
@@ -34,24 +36,35 @@ inline size_t fwd_parts_floats(int batch, int T, int n_heads, int dim, int q_off
     return n < 2 ? 0 : n * rows * ((q_offset > 0 ? 2 : 1) * (size_t)dim + 1);
 }
 
-// Parts of the backward's walk: heads x ranges of query tiles.  A part keeps four steps (a query tile of 64 rows of one
-// head each) of the longest walk.
+// Parts of the backward's walk: heads x ranges of query tiles.  A step is a query tile of 64 rows of one head.
 struct BwdParts {
     int heads, ranges;
     __host__ __device__ int n() const { return heads * ranges; }
 };
+// The split with the shortest schedule, in steps: a launch ends with its longest block, or once all blocks' steps have been
+// shared out with half a block left over at the end (the walks are of all lengths, longest first); a block costs three
+// steps beside its walk, putting the parts together two and their traffic one per 45 blocks.  Parts keep four steps of
+// the longest walk, and a launch two blocks an SM (which bounds the partial results: 38 MB at most).
 inline BwdParts bwd_parts(int batch, int T, int n_heads, int n_kv_heads) {
-    const long long ctas = (long long)n_kv_heads * ((T + 127) / 128) * batch;
-    const int group = n_heads / n_kv_heads, tiles = (T + 63) / 64;
-    const long long most = (long long)group * tiles / 4, fit = split_sm_count() / ctas;
-    const int want = (int)(fit < most ? fit : most);
-    BwdParts p{1, 1};
-    if (want < 2) return p;
-    for (int h = 1; h <= group && h <= want; ++h)
-        if (group % h == 0) p.heads = h;
-    p.ranges = want / p.heads < tiles / 2 ? want / p.heads : tiles / 2;
-    if (p.ranges < 1) p.ranges = 1;
-    return p;
+    const int group = n_heads / n_kv_heads, tiles = (T + 63) / 64, sms = split_sm_count();
+    const long long key_tiles = (T + 127) / 128, ctas = n_kv_heads * key_tiles * batch;
+    const double walks = (double)group * (tiles * key_tiles - key_tiles * (key_tiles - 1)) * n_kv_heads * batch;  // all blocks' steps
+    BwdParts best{1, 1};
+    if (ctas > 2 * sms) return best;
+    double best_cost = 0.;
+    for (int h = 1; h <= group; ++h) {
+        if (group % h != 0) continue;
+        for (int r = 1; r == 1 || r <= tiles / 2; ++r) {
+            const int n = h * r;
+            if (n > 1 && (n * ctas > 2 * sms || (long long)group * tiles < 4LL * n)) break;
+            const double longest = (double)(group / h) * ((tiles + r - 1) / r) + 3, shared = (walks + 3. * n * ctas) / sms + longest / 2;
+            double cost = n * ctas <= sms || longest > shared ? longest : shared;
+            if (n > 1) cost += 2 + n * ctas / 45.;
+            // (of equals the split by heads: a part of a range also flushes its accumulators once per head)
+            if ((h == 1 && r == 1) || cost <= best_cost) best = BwdParts{h, r}, best_cost = cost;
+        }
+    }
+    return best;
 }
 inline size_t bwd_parts_floats(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     const int n = bwd_parts(batch, T, n_heads, n_kv_heads).n();
