@@ -95,3 +95,26 @@ def test_rope_at_widths_between_the_tiles(zt, oracle, T, H, Hkv, D, pos):
     rdq, rdk, rdv = oracle.attention_backward(qr, kr, v[0], do[0], H, Hkv, D)
     for name, got, want in (("dq", dq, oracle.rope_backward(rdq, pos, D)), ("dk", dk, oracle.rope_backward(rdk, pos, D)), ("dv", dv, rdv)):
         close(got[0], want, name)
+
+
+@pytest.mark.parametrize("B,T,k,n", [(1, 1000, 1088, 1216), (2, 1100, 1600, 1536)])
+def test_projection_on_wide_tiles(zt, oracle, B, T, k, n):
+    """Large enough for the 128 x 256 tiles (the second in all three products, several to a block), with tails in rows
+    and columns, a half of a tile beyond the columns, and contractions cut into pieces.  The reference reduces in f32, so
+    the gate is its own, relative to the tensor's largest magnitude (src/train.zig:706)."""
+    ctx, dy = normal(oracle, (B, T, k), 0), normal(oracle, (B, T, n), 1)
+    wo, dwo0 = normal(oracle, (k, n), 2) / np.float32(np.sqrt(k)), normal(oracle, (k, n), 3)
+    tctx, two, tdy, tdwo = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (ctx, wo, dy, dwo0))
+    ws = zt.ProjWorkspace(B, T, k, n)
+    y = zt.proj_forward(tctx, two, workspace=ws)
+    dctx = zt.proj_backward(tctx, two, tdy, tdwo, workspace=ws)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0
+    ref_dwo = dwo0.copy()
+    pairs = []
+    for b in range(B):
+        pairs += [(y[b], oracle.matmul(ctx[b], wo, threads=8)), (dctx[b], oracle.input_grad(dy[b], wo, threads=8))]
+        oracle.weight_grad(ref_dwo, ctx[b], dy[b], threads=8)
+    for got, ref in pairs + [(tdwo, ref_dwo)]:
+        err = np.abs(got.cpu().numpy().astype(np.float64) - ref)
+        assert float(np.where(np.isnan(err), np.inf, err).max()) <= 1e-4 * float(np.abs(ref).max())
