@@ -12,8 +12,8 @@
 //   bwd_wide_scores   one CTA per (128 query rows, 128 keys) tile at or below the diagonal of one (sequence,
 //                     head): S = Q K^T and dP = dO V^T over the head's 256 columns into two TMEM accumulators,
 //                     then P and dS, split, into the scratch planes [T, T] of that head;
-//   gemm_tri<0>       dQ = scale dS K: 128 x 256 output tiles (the whole head), contraction over the keys a query tile sees;
-//   gemm_tri<1>       dK = scale sum_h dS^T Q and dV = sum_h P^T dO: contraction over the query rows at or after
+//   wide_products     dQ = scale dS K: 128 x 256 output tiles (the whole head), contraction over the keys a query tile sees;
+//                     dK = scale sum_h dS^T Q and dV = sum_h P^T dO: contraction over the query rows at or after
 //                     the key tile, every head of the KV group adding into the same output.
 // Contractions longer than 1024 are cut into pieces that separate CTAs add with red.global.add.f32 (the tensor
 // core adds into its accumulator with truncation; see tc_gemm.cuh), so dq, dk, dv are zeroed first.
@@ -46,7 +46,7 @@ constexpr int kTB = 128 * 64 * 2;  // bytes of one plane of an operand tile
 constexpr int kSB = 4 * kTB;       // a stage: A hi, A lo, B hi, B lo
 constexpr int kScoreThreads = 10 * 32;  // TMA producer, MMA issuer, eight epilogue warps
 constexpr int kTriThreads = 6 * 32;     // TMA producer, MMA issuer, four epilogue warps
-constexpr int kPiece = 1024;            // contraction depth of one CTA of gemm_tri
+constexpr int kPiece = 1024;            // contraction depth of one unit of wide_products
 
 struct WideShared {
     uint64_t full[kStages], freed[kStages], all_done, staged;
@@ -70,12 +70,11 @@ struct WideParams {
     const uint32_t *amax_q, *amax_k, *amax_v, *amax_do;  // [B, Hkv] bit patterns of max |x|
     const uint32_t *vnmax, *rnmax;     // [B, Hkv] bit patterns: largest row norm of v, of dout (over the group's heads)
     __half *p_planes, *ds_planes;      // [2][unit_cap][Tp][Tp]: hi planes of the chunk's units, then lo planes
-    float *out;                        // gemm_tri: dq, dk or dv
+    float *dq, *dk, *dv;
     int batch, T, Tp, n_heads, n_kv_heads;
     int dim_out, td;                   // the tensors' head_dim, the planes' (256)
     int unit0, unit_cap;               // the chunk: units (b * n_heads + h) from unit0; planes allocated for unit_cap
-    int pieces;                        // gemm_tri: pieces of kPiece along one head's contraction
-    int which;                         // gemm_tri<1>: 0 dK (dS and the row-scaled Q), 1 dV (P and dO)
+    int units, pieces;                 // wide_products: units of the chunk, pieces of kPiece along one head's contraction
     float scale, scale_log2, p_scale;
 };
 
@@ -546,59 +545,80 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
 inline size_t res_smem_bytes() { return (size_t)14 * (128 * 64 * 2) + sizeof(ResShared); }
 
 // ---------------------------------------------------------------------------------------------------
-// The three products that read the planes.  128 x 256 output tiles (a head's whole width, so that a tile of the
-// planes is read once), 64-deep steps, B always the tensor whose rows are the contraction index ([T, width] planes
-// read as N-major tiles).
-//   MODE 0: dQ.  grid (query tiles, units x pieces).  A = dS planes, K-major; contraction over keys
-//           [piece * 1024, min((m + 1) * 128, (piece + 1) * 1024)); row t leaves times scale / (cq(t) mk).
-//   MODE 1: dK (which 0) or dV (which 1).  grid (key tiles, KV groups of the chunk x heads of a group x pieces).  A = dS or P planes read M-major (rows are the contraction index: query rows); contraction
-//           over query rows [max(m * 128, piece * 1024), min(Tp, (piece + 1) * 1024)).
-// Every tile is added to the output (red.global.add.v4.f32), which the host has zeroed.
+// The three products that read the planes, in one launch of persistent blocks.  128 x 256 output tiles (a head's whole
+// width, so that a tile of the planes is read once), 64-deep steps, B always the tensor whose rows are the contraction
+// index ([T, width] planes read as N-major tiles).
+//   dQ      A = dS planes, K-major; contraction over keys [piece * 1024, min((m + 1) * 128, (piece + 1) * 1024)); row t leaves
+//           times scale / (cq(t) mk).
+//   dK, dV  A = dS or P planes read M-major (rows are the contraction index: query rows); contraction over query rows
+//           [max(m * 128, piece * 1024), min(Tp, (piece + 1) * 1024)); every head of a group adds into its KV head.
+// Every tile is added to the output (red.global.add.v4.f32), which the pre-pass has zeroed.
+// A unit is one (product, head of the chunk, piece, tile): nine steps of MMAs on average at T 1024, about as long as its
+// prologue and epilogue together when each was a block of its own.  So a block walks its share of the units with two
+// accumulators in TMEM (all 512 columns), loads run ahead across units, and a unit's epilogue -- straight from TMEM to
+// memory, rows regrouped among eight lanes -- runs under the next one's MMAs.  A head's tiles are consecutive units:
+// blocks that run together share its operands in L2.
+// Us, three launches of a block per unit -> this: batch 8, T 1024, 32/8 heads of 256 809 -> 777 (bound by DRAM: the planes are
+// 3 GB written and read there); forward and backward at batch 4, T 300, 8/2 heads 129 -> 111, one sequence of T 500, 4/2
+// heads of 160 130 -> 102.
 // ---------------------------------------------------------------------------------------------------
-template <int MODE>
+struct TriShared {
+    uint64_t full[2], freed[2], acc_full[2], acc_free[2];
+    uint32_t tmem_base;
+    volatile int abort;
+};
+__device__ __forceinline__ bool twait(uint64_t *bar, uint32_t parity, TriShared *sh) {
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((i & 255u) == 255u && sh->abort) return false;
+    }
+    return false;
+}
+__device__ __forceinline__ void tgive_up(TriShared *sh, int code) {
+    sh->abort = code;
+    atomicMax(&g_tc_status, code);
+}
+struct TriUnit {
+    int which, u, m0, b, h, k_begin, n_steps;  // which: 0 dQ, 1 dK, 2 dV; n_steps <= 0: nothing to do
+    __device__ __forceinline__ TriUnit(const WideParams &p, int i) {
+        const int nt = p.Tp / 128, m = i % nt, r = i / nt % (p.units * p.pieces);
+        which = i / (nt * p.units * p.pieces);
+        u = r / p.pieces;
+        const int piece = r - u * p.pieces, ug = p.unit0 + u;
+        b = ug / p.n_heads, h = ug - b * p.n_heads;
+        m0 = m * 128;
+        k_begin = piece * kPiece;
+        int k_end = k_begin + kPiece;
+        if (which == 0) k_end = k_end < m0 + 128 ? k_end : m0 + 128;
+        else k_begin = k_begin > m0 ? k_begin : m0;
+        k_end = k_end < p.Tp ? k_end : p.Tp;
+        n_steps = (k_end - k_begin) / 64;
+    }
+};
+
 __global__ void __launch_bounds__(kTriThreads, 1)
-    gemm_tri(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const WideParams p) {
-    constexpr bool A_MN = MODE == 1;
+    wide_products(const __grid_constant__ CUtensorMap ds_k, const __grid_constant__ CUtensorMap ds_m, const __grid_constant__ CUtensorMap p_m,
+                  const __grid_constant__ CUtensorMap k_n, const __grid_constant__ CUtensorMap qs_n, const __grid_constant__ CUtensorMap g_n,
+                  const WideParams p, int n_units) {
     // a stage: A hi, A lo (128 x 64 halves each) and B hi, B lo (64 contraction rows x 256 columns each, as four
-    // 64-column blocks of 8 KB): 96 KB; two stages.  The whole head width per CTA: an A tile is read once for it.
-    constexpr int kBT = 64 * 256 * 2, kStage = 2 * kTB + 2 * kBT, kSt = 2;
+    // 64-column blocks of 8 KB): 96 KB; two stages
+    constexpr int kBT = 64 * 256 * 2, kStage = 2 * kTB + 2 * kBT;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    WideShared *sh = reinterpret_cast<WideShared *>(smem_raw + kSt * kStage);
+    TriShared *sh = reinterpret_cast<TriShared *>(smem_raw + 2 * kStage);
     const int warp = threadIdx.x >> 5;
-    const int m0 = blockIdx.x * 128;
     const int group = p.n_heads / p.n_kv_heads;
-    int u, piece;
-    if (MODE == 0) {
-        u = (int)blockIdx.y / p.pieces, piece = (int)blockIdx.y % p.pieces;
-    } else {
-        const int cg = (int)blockIdx.y / (group * p.pieces), rem = (int)blockIdx.y % (group * p.pieces);
-        u = cg * group + rem / p.pieces, piece = rem % p.pieces;
-    }
-    const int ug = p.unit0 + u;
-    const int b = ug / p.n_heads, h = ug % p.n_heads, g = h / group;
     const int B = p.batch;
-    int k_begin = piece * kPiece, k_end = k_begin + kPiece;
-    if (MODE == 0) {
-        if (k_end > m0 + 128) k_end = m0 + 128;
-    } else {
-        if (k_begin < m0) k_begin = m0;
-    }
-    if (k_end > p.Tp) k_end = p.Tp;
-    if (k_begin >= k_end || m0 >= p.T) {  // (the whole CTA: nothing has been set up yet)
-        pdl_wait();
-        return;
-    }
-    const int n_steps = (k_end - k_begin) / 64;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kSt; ++i) mbar_init(&sh->full[i], 1), mbar_init(&sh->freed[i], 1);
-        mbar_init(&sh->all_done, 1);
-        mbar_init(&sh->staged, 4);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh->full[i], 1), mbar_init(&sh->freed[i], 1);
+            mbar_init(&sh->acc_full[i], 1), mbar_init(&sh->acc_free[i], 4);
+        }
         sh->abort = (smem_u32(smem_raw) & 1023u) ? 84 : 0;
         if (sh->abort) atomicMax(&g_tc_status, 84);
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(&sh->tmem_base, 256);
+    if (warp == 1) tmem_alloc(&sh->tmem_base, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -609,126 +629,141 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (elect_one() && !sh->abort) {
-            tma_prefetch_desc(&amap), tma_prefetch_desc(&bmap);
-            // B's column blocks: the head's (MODE 0: the KV head's) 256 columns
-            const int bblk = ((MODE == 0 ? g : h) * p.td) / 64;
-            int issued = 0;
-            for (int s = 0; s < n_steps; ++s) {
-                const int st = s % kSt, k0 = k_begin + s * 64;
-                if (s >= kSt && !wwait(&sh->freed[st], (uint32_t)(((s / kSt) & 1) ^ 1), sh)) { wgive_up(sh, 85); break; }
-                uint8_t *base = smem_raw + st * kStage;
-                mbar_arrive_expect_tx(&sh->full[st], kStage);
-                if (A_MN) {  // rows = query rows (contraction), columns = keys (M): 64 rows x two 64-column blocks
-                    tma_load_4d(base, &amap, &sh->full[st], 0, k0, m0 / 64, u);
-                    tma_load_4d(base + kTB, &amap, &sh->full[st], 0, k0, m0 / 64, p.unit_cap + u);
-                } else {     // rows = query rows (M), columns = keys (contraction): 128 rows x one block
-                    tma_load_4d(base, &amap, &sh->full[st], 0, m0, k0 / 64, u);
-                    tma_load_4d(base + kTB, &amap, &sh->full[st], 0, m0, k0 / 64, p.unit_cap + u);
+            tma_prefetch_desc(&ds_k), tma_prefetch_desc(&ds_m), tma_prefetch_desc(&p_m);
+            tma_prefetch_desc(&k_n), tma_prefetch_desc(&qs_n), tma_prefetch_desc(&g_n);
+            int it = 0;  // steps issued
+            for (int i = blockIdx.x; i < n_units && !sh->abort; i += gridDim.x) {
+                const TriUnit w(p, i);
+                const CUtensorMap *am = w.which == 0 ? &ds_k : w.which == 1 ? &ds_m : &p_m;
+                const CUtensorMap *bm = w.which == 0 ? &k_n : w.which == 1 ? &qs_n : &g_n;
+                // B's column blocks: the head's (dQ: the KV head's) columns
+                const int bblk = (w.which == 0 ? w.h / group : w.h) * p.td / 64;
+                for (int s = 0; s < w.n_steps; ++s, ++it) {
+                    const int st = it & 1, k0 = w.k_begin + s * 64;
+                    if (it >= 2 && !twait(&sh->freed[st], (uint32_t)(((it >> 1) & 1) ^ 1), sh)) { tgive_up(sh, 85); break; }
+                    uint8_t *base = smem_raw + st * kStage;
+                    mbar_arrive_expect_tx(&sh->full[st], kStage);
+                    // dK, dV: 64 query rows x two 64-key blocks; dQ: 128 query rows x one block
+                    const int c1 = w.which ? k0 : w.m0, c2 = (w.which ? w.m0 : k0) / 64;
+                    tma_load_4d(base, am, &sh->full[st], 0, c1, c2, w.u);
+                    tma_load_4d(base + kTB, am, &sh->full[st], 0, c1, c2, p.unit_cap + w.u);
+                    tma_load_4d(base + 2 * kTB, bm, &sh->full[st], 0, k0, bblk, w.b);
+                    tma_load_4d(base + 2 * kTB + kBT, bm, &sh->full[st], 0, k0, bblk, B + w.b);
                 }
-                tma_load_4d(base + 2 * kTB, &bmap, &sh->full[st], 0, k0, bblk, b);
-                tma_load_4d(base + 2 * kTB + kBT, &bmap, &sh->full[st], 0, k0, bblk, B + b);
-                ++issued;
             }
             if (sh->abort)
-                for (int s = (issued > kSt ? issued - kSt : 0); s < issued; ++s)
-                    mbar_wait(&sh->full[s % kSt], (uint32_t)((s / kSt) & 1));
+                for (int s = (it > 2 ? it - 2 : 0); s < it; ++s) mbar_wait(&sh->full[s & 1], (uint32_t)((s >> 1) & 1));
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (elect_one()) {
-            constexpr uint32_t idesc = idesc_f16(128, 256, A_MN, true);
+        if (elect_one() && !sh->abort) {
             const uint32_t s_u32 = smem_u32(smem_raw);
-            bool ok = !sh->abort;
-            for (int s = 0; ok && s < n_steps; ++s) {
-                const int st = s % kSt;
-                if (!wwait(&sh->full[st], (uint32_t)((s / kSt) & 1), sh)) { wgive_up(sh, 86); ok = false; break; }
-                tc_fence_after();
-                const uint32_t base = s_u32 + (uint32_t)(st * kStage);
-                const uint64_t ah = A_MN ? desc_mnmajor_16b(base, 64 * 128) : desc_kmajor(base);
-                const uint64_t al = A_MN ? desc_mnmajor_16b(base + kTB, 64 * 128) : desc_kmajor(base + kTB);
-                const uint64_t bh = desc_mnmajor_16b(base + 2 * kTB, 64 * 128);
-                const uint64_t bl = desc_mnmajor_16b(base + 2 * kTB + kBT, 64 * 128);
+            int it = 0, n = 0;  // steps, units with something to do
+            for (int i = blockIdx.x; i < n_units && !sh->abort; i += gridDim.x) {
+                const TriUnit w(p, i);
+                if (w.n_steps <= 0) continue;
+                const uint32_t idesc = w.which ? idesc_f16(128, 256, true, true) : idesc_f16(128, 256, false, true);
+                const uint32_t a_step = w.which ? 2048 : 32;
+                const uint32_t acc = tmem + (n & 1) * 256;
+                if (n >= 2 && !twait(&sh->acc_free[n & 1], (uint32_t)(((n >> 1) & 1) ^ 1), sh)) { tgive_up(sh, 86); break; }
+                for (int s = 0; s < w.n_steps; ++s, ++it) {
+                    const int st = it & 1;
+                    if (!twait(&sh->full[st], (uint32_t)((it >> 1) & 1), sh)) { tgive_up(sh, 86); break; }
+                    tc_fence_after();
+                    const uint32_t base = s_u32 + (uint32_t)(st * kStage);
+                    const uint64_t ah = w.which ? desc_mnmajor_16b(base, 64 * 128) : desc_kmajor(base);
+                    const uint64_t al = w.which ? desc_mnmajor_16b(base + kTB, 64 * 128) : desc_kmajor(base + kTB);
+                    const uint64_t bh = desc_mnmajor_16b(base + 2 * kTB, 64 * 128);
+                    const uint64_t bl = desc_mnmajor_16b(base + 2 * kTB + kBT, 64 * 128);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const uint32_t ao = A_MN ? kk * 2048 : kk * 32, bo = kk * 2048;
-                    const uint64_t dah = desc_advance(ah, ao), dal = desc_advance(al, ao);
-                    const uint64_t dbh = desc_advance(bh, bo), dbl = desc_advance(bl, bo);
-                    mma_ss_f16(tmem, dah, dbh, idesc, (s > 0 || kk > 0) ? 1 : 0);
-                    mma_ss_f16(tmem, dah, dbl, idesc, 1);
-                    mma_ss_f16(tmem, dal, dbh, idesc, 1);
+                    for (int kk = 0; kk < 4; ++kk) {
+                        const uint64_t dah = desc_advance(ah, kk * a_step), dal = desc_advance(al, kk * a_step);
+                        const uint64_t dbh = desc_advance(bh, kk * 2048), dbl = desc_advance(bl, kk * 2048);
+                        mma_ss_f16(acc, dah, dbh, idesc, (s > 0 || kk > 0) ? 1 : 0);
+                        mma_ss_f16(acc, dah, dbl, idesc, 1);
+                        mma_ss_f16(acc, dal, dbh, idesc, 1);
+                    }
+                    mma_commit(&sh->freed[st]);
                 }
-                mma_commit(&sh->freed[st]);
+                mma_commit(&sh->acc_full[n & 1]);
+                ++n;
             }
-            if (ok) mma_commit(&sh->all_done);
         }
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue: a thread per output row
-        const int lane = threadIdx.x & 31;
+        const int lane = threadIdx.x & 31, j8 = lane & 7;
         const int lane_grp = warp & 3;
-        const int row = lane_grp * 32 + lane;
         const uint32_t lane_base = (uint32_t)(lane_grp * 32) << 16;
-        const int t = m0 + row;  // MODE 0: the query row; MODE 1: the key
-        float f;
-        if (MODE == 0) {
-            float cq = 1.f, rel = 1.f;
-            if (t < p.T)
-                ds_row_scale(__ldg(p.rnorm + ((long long)b * p.T + t) * p.n_heads + h), p.rnmax[b * p.n_kv_heads + g],
-                               p.vnmax[b * p.n_kv_heads + g], cq, rel);
-            f = p.scale / (cq * block_mult(p.amax_k[b * p.n_kv_heads + g]));
-        } else if (p.which == 0) {
-            f = p.scale / (ds_group_scale(p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g]) *
-                           block_mult(p.amax_q[b * p.n_kv_heads + g]));
-        } else {
-            f = 1.0f / (p.p_scale * block_mult(p.amax_do[b * p.n_kv_heads + g]));
-        }
-        bool ok = __all_sync(0xffffffffu, wwait(&sh->all_done, 0, sh));
-        if (!ok) wgive_up(sh, 87);
-        uint8_t *stage = smem_raw;  // rows go through shared memory: 128 rows x 1024 bytes, chunk c of row r at c ^ (r & 31)
-        if (ok) {
+        int n = 0;
+        for (int i = blockIdx.x; i < n_units; i += gridDim.x) {
+            const TriUnit w(p, i);
+            if (w.n_steps <= 0) continue;
+            const int g = w.h / group, bg = w.b * p.n_kv_heads + g;
+            const int t = w.m0 + lane_grp * 32 + lane;  // dQ: the query row; dK, dV: the key
+            float f;
+            if (w.which == 0) {
+                float cq = 1.f, rel = 1.f;
+                if (t < p.T) ds_row_scale(__ldg(p.rnorm + ((long long)w.b * p.T + t) * p.n_heads + w.h), p.rnmax[bg], p.vnmax[bg], cq, rel);
+                f = p.scale / (cq * block_mult(p.amax_k[bg]));
+            } else if (w.which == 1) {
+                f = p.scale / (ds_group_scale(p.rnmax[bg], p.vnmax[bg]) * block_mult(p.amax_q[bg]));
+            } else {
+                f = 1.0f / (p.p_scale * block_mult(p.amax_do[bg]));
+            }
+            if (!__all_sync(0xffffffffu, twait(&sh->acc_full[n & 1], (uint32_t)((n >> 1) & 1), sh))) { tgive_up(sh, 87); break; }
             tc_fence_after();
-            uint8_t *srow = stage + row * 1024;
+            const long long ld = (long long)(w.which == 0 ? p.n_heads : p.n_kv_heads) * p.dim_out;
+            const int row0 = t - j8;  // the first of this lane's eight rows
+            float *dst = (w.which == 0 ? p.dq : w.which == 1 ? p.dk : p.dv) + ((long long)w.b * p.T + row0) * ld +
+                         (long long)(w.which == 0 ? w.h : g) * p.dim_out + 4 * j8;
 #pragma unroll 1
             for (int c = 0; c < 256; c += 32) {
                 uint32_t r[32];
-                tmem_ld32(tmem + lane_base + c, r);
+                tmem_ld32(tmem + lane_base + (n & 1) * 256 + c, r);
                 tmem_wait_ld();
+                if (c + 32 == 256) {  // all read: the MMAs may have the buffer while the last columns are on their way
+                    tc_fence_before();
+                    mbar_arrive_warp_relaxed(&sh->acc_free[n & 1]);
+                }
+                if (c >= p.dim_out) continue;
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    float4 o4;
-                    o4.x = __uint_as_float(r[i]) * f, o4.y = __uint_as_float(r[i + 1]) * f;
-                    o4.z = __uint_as_float(r[i + 2]) * f, o4.w = __uint_as_float(r[i + 3]) * f;
-                    const int ch = (c + i) >> 2;
-                    *reinterpret_cast<float4 *>(srow + ((ch ^ (row & 31)) << 4)) = o4;
+                for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * f);
+                // eight lanes transpose their 8 x 8 blocks of float4: lane j gets the j-th float4 of eight rows, and an
+                // instruction covers four rows' 128-byte runs
+#pragma unroll
+                for (int M = 4; M >= 1; M >>= 1) {
+                    const bool up = (lane & M) != 0;
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        if (m & M) continue;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const uint32_t send = up ? r[4 * m + e] : r[4 * (m ^ M) + e];
+                            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, M);
+                            if (up) r[4 * m + e] = recv;
+                            else r[4 * (m ^ M) + e] = recv;
+                        }
+                    }
+                }
+                if (c + 4 * j8 < p.dim_out) {  // (a padded tile's upper columns are not the tensor's)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (row0 + e < p.T)
+                            tcb::red_add_v4(dst + (long long)e * ld + c, make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]),
+                                                                                    __uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3])));
                 }
             }
-        }
-        mbar_arrive_warp(&sh->staged);
-        if (__all_sync(0xffffffffu, wwait(&sh->staged, 0, sh)) && !sh->abort) {
-            const int heads_out = MODE == 0 ? p.n_heads : p.n_kv_heads, head_out = MODE == 0 ? h : g;
-            const long long ld = (long long)heads_out * p.dim_out;
-            const int wrow0 = (warp - 2) * 32;
-#pragma unroll 4
-            for (int i = 0; i < 32; ++i) {
-                const int r = wrow0 + i;
-                if (m0 + r >= p.T) continue;
-                float *dst = p.out + ((long long)b * p.T + m0 + r) * ld + (long long)head_out * p.dim_out;
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int ch = half * 32 + lane;
-                    const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * 1024 + ((ch ^ (r & 31)) << 4));
-                    if (ch * 4 < p.dim_out) tcb::red_add_v4(dst + ch * 4, o4);
-                }
-            }
+            ++n;
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 256);
+    if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-inline size_t tri_smem_bytes() { return (size_t)2 * (2 * kTB + 2 * 64 * 256 * 2) + sizeof(WideShared); }
+inline size_t tri_smem_bytes() { return (size_t)2 * (2 * kTB + 2 * 64 * 256 * 2) + sizeof(TriShared); }
 
 // ---- host side ----------------------------------------------------------------------------------------
 
@@ -834,7 +869,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     const size_t smem = wide_smem_bytes();
     const size_t smem_t = tri_smem_bytes(), smem_r = res_smem_bytes();
     if (optin_smem((const void *)bwd_wide_scores, smem) || optin_smem((const void *)bwd_wide_scores_res, smem_r) ||
-        optin_smem((const void *)gemm_tri<0>, smem_t) || optin_smem((const void *)gemm_tri<1>, smem_t))
+        optin_smem((const void *)wide_products, smem_t))
         return 1;
     WideParams p{};
     p.lse = lse, p.delta = delta, p.rnorm = w.rnorm;
@@ -844,6 +879,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     p.batch = batch, p.T = T, p.Tp = Tp, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
     p.dim_out = dim, p.td = td;
     p.unit_cap = cap;
+    p.dq = dq, p.dk = dk, p.dv = dv;
     p.pieces = (Tp + kPiece - 1) / kPiece;
     p.scale = 1.0f / sqrtf((float)dim), p.scale_log2 = kLog2e / sqrtf((float)dim);
     p.p_scale = ldexpf(1.0f, 10);
@@ -860,14 +896,11 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
             const dim3 gs((unsigned)units, (unsigned)nt);
             if (launch_after("bwd_wide_scores_res", bwd_wide_scores_res, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
         }
-        p.out = dq, p.which = 0;
-        const dim3 gq((unsigned)nt, (unsigned)(units * p.pieces));
-        if (launch_after("gemm_tri_dq", gemm_tri<0>, gq, dim3(kTriThreads), smem_t, stream, ds_k, k_n, p)) return 1;
-        const dim3 gk((unsigned)nt, (unsigned)(units * p.pieces));  // (units = KV groups x heads of a group)
-        p.out = dk, p.which = 0;
-        if (launch_after("gemm_tri_dk", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, ds_m, qs_n, p)) return 1;
-        p.out = dv, p.which = 1;
-        if (launch_after("gemm_tri_dv", gemm_tri<1>, gk, dim3(kTriThreads), smem_t, stream, p_m, g_n, p)) return 1;
+        p.units = units;
+        const long long n_units = 3LL * nt * units * p.pieces;
+        const dim3 gp((unsigned)(n_units < split_sm_count() ? n_units : split_sm_count()));
+        if (launch_after("wide_products", wide_products, gp, dim3(kTriThreads), smem_t, stream, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
+            return 1;
     }
     return 0;
 }
