@@ -9,7 +9,9 @@
 //                        the attention kernels, and writes the planes (rotating q and k on the way where rope is asked
 //                        for), the row-scaled copy of q's planes for dK, and the zeros of outputs that are summed in memory.
 // Both work on units, one head of one row, held by 8, 16 or 32 lanes; a lane has four units in flight.  A block's units
-// belong to one (sequence, group); the split into blocks aims at 2048 blocks per tensor (14 an SM; 4096 and 1024 were
+// belong to one (sequence, group), of which its blocks take turns: blocks that run together read and write one stretch
+// of memory, not a stretch each (the first
+// pass at T 4096, heads of 128: 460 us, with the turns 417).  The split into blocks aims at 2048 blocks per tensor (14 an SM; 4096 and 1024 were
 // 1-2 % slower, 512 more) of at least eight units a lane group.
 // Before (one kernel per quantity: two for the planes, one each for delta, v's norms, dout's norms, the row-scaled
 // copy, and up to four memsets; 13 launches a step where there are 6 now): batch 8, T 512, 32/8 heads of 64, forward
@@ -100,7 +102,7 @@ struct PassTensor {
     const uint32_t *vn_final;
     int dn_slots, vn_slots;
     int batch, rows, heads, group;  // heads per row, heads per group
-    int slots, per_block;           // blocks per (sequence, group), units per block
+    int slots;                      // blocks per (sequence, group)
     int first;                      // first block of this tensor
 };
 struct PassArgs {
@@ -112,7 +114,7 @@ struct PassArgs {
 };
 
 struct PassUnit {  // where a block stands
-    int z, bg, slot, b, g, begin, end;
+    int z, bg, slot, b, g, units;
 };
 __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int blk) {
     PassUnit w;
@@ -120,10 +122,11 @@ __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int bl
     while (w.z + 1 < n && blk >= a.t[w.z + 1].first) ++w.z;
     const PassTensor &t = a.t[w.z];
     const int groups = t.heads / t.group, i = blk - t.first;
-    w.bg = i / t.slots, w.slot = i - w.bg * t.slots;
-    w.b = w.bg / groups, w.g = w.bg - w.b * groups;
-    w.begin = w.slot * t.per_block;
-    w.end = min(w.begin + t.per_block, t.rows * t.group);
+    // (the groups of the same rows are neighbours: blocks that run together cover whole rows)
+    const int rest = i / groups;
+    w.g = i - rest * groups, w.b = rest / t.slots, w.slot = rest - w.b * t.slots;
+    w.bg = w.b * groups + w.g;
+    w.units = t.rows * t.group;
     return w;
 }
 
@@ -132,7 +135,7 @@ __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int bl
 // the loads of a step would stall on the arithmetic of the step before (heads of 256, batch 8, T 1024: 4.1 TB/s against 5.4).
 template <int LP, int NC>
 __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_constant__ PassArgs a) {
-    constexpr int NG = kPassThreads / LP, U = 2 / NC, S = kStatsStages;
+    constexpr int NG = kPassThreads / LP, U = 1, S = kStatsStages;
     extern __shared__ __align__(16) float4 ring[];  // [S][U][NC][2][kPassThreads]
     __shared__ float red[2][kPassThreads / 32];
     const PassUnit w = pass_locate(a, a.n_stats, (int)blockIdx.x);
@@ -144,10 +147,10 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     const float4 *xb = reinterpret_cast<const float4 *>(t.x) + first * n4 + li;
     const float4 *ob = reinterpret_cast<const float4 *>(rows_out ? t.o : t.x) + first * n4 + li;
     const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(ring + threadIdx.x);
-    const int n_steps = (w.end - w.begin + NG * U - 1) / (NG * U);
+    const int stride = t.slots * NG * U, n_steps = (w.units - w.slot * NG * U + stride - 1) / stride;
     const auto place = [&](int step, int k) -> int {  // the unit's index within the (sequence, group), or -1
-        const int u = w.begin + gi + (step * U + k) * NG;
-        return u < w.end ? (u / group) * (heads - group) + u : -1;  // r heads + (u - r group)
+        const int u = step * stride + (w.slot * U + k) * NG + gi;
+        return u < w.units ? (u / group) * (heads - group) + u : -1;  // r heads + (u - r group)
     };
     const auto fetch = [&](int step) {
 #pragma unroll
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
     const auto locate = [&](int u, int &r) -> long long {
         r = u / t.group;
-        return u < w.end ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
+        return u < w.units ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
     };
     const auto row_rel = [&](long long at) -> float {
         float cq, rel;
@@ -289,7 +292,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
         return rel;
     };
     if (t.x == nullptr) {
-        for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+        for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
             uint2 h[U][NC], l[U][NC];
             long long at[U];
             float rel[U];
@@ -325,7 +328,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
     const float m = block_mult(top.x);
     if (t.rope == nullptr) {
-        for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+        for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
             float4 x[U][NC];
             long long at[U];
             float rel[U];
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     // rotated: a lane of the head's lower half takes a chunk and its partner half a head on (a head's halves are
     // multiples of four wide), so that every element and every table entry is fetched once
     const int half = a.dim >> 1, h4 = half >> 2;
-    for (int u0 = w.begin; u0 < w.end; u0 += NG * U) {
+    for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
 #pragma unroll
         for (int k = 0; k < U; ++k) {
             int r;
@@ -404,10 +407,7 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
     slots = slots > kPassMaxSlots ? kPassMaxSlots : (slots < 1 ? 1 : slots);
     const long long most = (units + step - 1) / step;
     if (slots > most) slots = most;
-    long long per = (units + slots - 1) / slots;
-    per = (per + step - 1) / step * step;
-    t.per_block = (int)per;
-    t.slots = (int)((units + per - 1) / per);
+    t.slots = (int)slots;
     return t;
 }
 inline void pass_fill(PassArgs &a, float *dst, long long n) {
@@ -431,7 +431,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
     int rc;
     const dim3 gs((unsigned)stats), gp((unsigned)blocks), th(kPassThreads);
-    constexpr size_t smem = (size_t)kStatsStages * 2 * 2 * kPassThreads * sizeof(float4);
+    const size_t smem = (size_t)kStatsStages * (a.dim > 128 ? 2 : 1) * 2 * kPassThreads * sizeof(float4);
     const auto stats_launch = [&](auto *kernel) -> int {
         if (optin_smem((const void *)kernel, smem)) return 1;
         return launch_pdl("pass_stats_kernel", kernel, gs, th, smem, stream, a);

@@ -61,7 +61,8 @@ __host__ __device__ constexpr size_t fused_smem_bytes() {
 
 // grid (n_kv_heads, ceil(T / 128), batch), 608 threads: 16 row warps, a TMA warp, two MMA warps.
 constexpr int kFusedThreads = (kKvRowWarps + 3) * 32;
-template <int D>
+// PARTS: the walk is split (tc_split.cuh).  A variant of its own: the whole walk is 1 % slower with the code in it.
+template <int D, bool PARTS>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     attn_bwd_fused_tc(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                       const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap gmap,
@@ -79,13 +80,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     FusedShared *sh = reinterpret_cast<FusedShared *>(sG + 2 * QP);
 
     const int warp = threadIdx.x >> 5;
-    const int g = blockIdx.x, kt = (int)blockIdx.y, b = (int)blockIdx.z / p.parts.n(), part = (int)blockIdx.z - b * p.parts.n();
+    const int g = blockIdx.x, kt = (int)blockIdx.y, b = PARTS ? (int)blockIdx.z / p.parts.n() : (int)blockIdx.z;
+    const int part = PARTS ? (int)blockIdx.z - b * p.parts.n() : 0;
     const int group = p.n_heads / p.n_kv_heads;
     const int s0 = kt * 128;
     // this CTA's part of the walk: heads [head0, head0 + n_heads_mine) and query tiles [qi0, n_q)
-    const int n_heads_mine = group / p.parts.heads, head0 = g * group + part / p.parts.ranges * n_heads_mine;
+    const int n_heads_mine = PARTS ? group / p.parts.heads : group;
+    const int head0 = PARTS ? g * group + part / p.parts.ranges * n_heads_mine : g * group;
     int n_q = (p.T + BQ - 1) / BQ, qi0 = s0 / BQ;
-    if (p.parts.ranges > 1) {
+    if (PARTS && p.parts.ranges > 1) {
         const int per = (n_q - qi0 + p.parts.ranges - 1) / p.parts.ranges;
         qi0 += part % p.parts.ranges * per;
         if (qi0 >= n_q) {
@@ -403,8 +406,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             const uint32_t acc = tmem + lane_base + (set < 2 ? cDV : cDK) + c0;
             const int j8 = lane & 7;
             const long long wo = (long long)p.n_kv_heads * p.dim_out;
-            const int mine = (int)blockIdx.z - b * p.parts.n();  // (`part`, without a register held for it)
-            float *dst = (set < 2 ? p.dv : p.dk) + mine * p.dkv_part + ((long long)b * p.T + (key - j8)) * wo + (long long)g * p.dim_out + c0 + 4 * j8;
+            const int mine = PARTS ? (int)blockIdx.z - b * p.parts.n() : 0;  // (`part`, without a register held for it)
+            float *dst = (set < 2 ? p.dv : p.dk) + (PARTS ? mine * p.dkv_part : 0) + ((long long)b * p.T + (key - j8)) * wo + (long long)g * p.dim_out + c0 + 4 * j8;
             const float f = set < 2 ? 1.0f / (p.p_scale * mdo) : p.scale / (mq * cmin);
 #pragma unroll 1
             for (int c = 0; c < D / 2; c += 32) {
@@ -632,9 +635,10 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
                               const BwdParams &p, cudaStream_t stream) {
     size_t smem = fused_smem_bytes<D>();
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    if (optin_smem((const void *)attn_bwd_fused_tc<D>, smem)) return 1;
+    const auto kernel = p.parts.n() > 1 ? attn_bwd_fused_tc<D, true> : attn_bwd_fused_tc<D, false>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)(p.batch * p.parts.n()));
-    return launch_after("attn_bwd_fused_tc", attn_bwd_fused_tc<D>, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
+    return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
 }
 inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
                             const BwdParams &p, cudaStream_t stream) {

@@ -145,10 +145,10 @@ inline bool attribute_known(const void *fn, int attr, size_t value, bool record)
     return record;
 }
 
-// Opt a kernel into more than 48 KiB of dynamic shared memory; a refusal, not an exit
+// Opt a kernel into more than 46 KiB of dynamic shared memory (the static kind counts against the 48 too); a refusal, not an exit
 // (src/cuda/attn_kernels.cu:822-830).
 inline int optin_smem(const void *fn, size_t bytes) {
-    if (bytes <= 48u * 1024u || attribute_known(fn, (int)cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, false)) return 0;
+    if (bytes <= 46u * 1024u || attribute_known(fn, (int)cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, false)) return 0;
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess) {
