@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<LPK, NCH, GP>::kMinB
     const int nh = (group - sub * GP) < GP ? (group - sub * GP) : GP;
     pdl_wait();
     pdl_launch();
-    if (CLUSTER && blockIdx.x == 0 && blockIdx.y == 0 && b == 0) count_bad_sequences(p);
+    const bool counts = CLUSTER && blockIdx.x == 0 && blockIdx.y == 0 && b == 0;  // (last of all: off every row's path)
     const int nk = p.n_keys ? p.n_keys[b] : p.n_keys_all;
     if (nk < 1 || nk > p.n_ctx) {
         // decode.attnStep refuses an empty prefix (src/decode.zig:350); on the device the refusal is a NaN row plus
@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<LPK, NCH, GP>::kMinB
             for (int i = threadIdx.x; i < nh * p.dim; i += kDecodeThreads) p.out[((long long)b * p.n_heads + h0) * p.dim + i] = __int_as_float(0x7fc00000);
             if (p.lse && threadIdx.x < nh) p.lse[(long long)b * p.n_heads + h0 + threadIdx.x] = __int_as_float(0x7fc00000);
         }
+        if (counts) count_bad_sequences(p);
         return;  // (the whole cluster)
     }
     const int chunk = CLUSTER ? (nk + p.cluster - 1) / p.cluster : p.chunk;
@@ -342,25 +343,28 @@ __global__ void __launch_bounds__(kDecodeThreads, DecodeCfg<LPK, NCH, GP>::kMinB
     for (int idx = blockIdx.x * kDecodeThreads + threadIdx.x; idx < nh * dim; idx += cs * kDecodeThreads) {
         const int hh = idx / dim, j = idx - hh * dim;
         const uint32_t at = blk0 + (uint32_t)(hh * rec) * 4u;
-        float mr[kMaxCluster], mx = -INFINITY;  // (block 0 of a cluster has keys: the maximum is finite)
+        float mr[kMaxCluster], lr[kMaxCluster], ar[kMaxCluster], mx = -INFINITY;  // (block 0 has keys: the maximum is finite)
 #pragma unroll
-        for (int r = 0; r < kMaxCluster; ++r) {
+        for (int r = 0; r < kMaxCluster; ++r) {  // all of them on their way at once
             mr[r] = r < cs ? ld_cluster(at, r) : -INFINITY;
-            mx = fmaxf(mx, mr[r]);
+            lr[r] = r < cs ? ld_cluster(at + 4u, r) : 0.f;
+            ar[r] = r < cs ? ld_cluster(at + 4u * (4 + j), r) : 0.f;
         }
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) mx = fmaxf(mx, mr[r]);
         float lsum = 0.f, acc_j = 0.f;
 #pragma unroll
         for (int r = 0; r < kMaxCluster; ++r) {
-            if (r >= cs) break;
             const float w = (mr[r] == -INFINITY) ? 0.f : ex2(mr[r] - mx);
-            lsum = fmaf(ld_cluster(at + 4u, r), w, lsum);
-            acc_j = fmaf(ld_cluster(at + 4u * (4 + j), r), w, acc_j);
+            lsum = fmaf(lr[r], w, lsum);
+            acc_j = fmaf(ar[r], w, acc_j);
         }
         const long long row = (long long)b * p.n_heads + h0 + hh;
         p.out[row * dim + j] = acc_j / lsum;
         if (p.lse && j == 0) p.lse[row] = (mx + log2f(lsum)) * kLn2;
     }
     cluster_arrive();  // nobody's shared memory goes away while others read it
+    if (counts) count_bad_sequences(p);
     cluster_wait();
 }
 
@@ -369,12 +373,13 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
     const int h = blockIdx.x, b = blockIdx.y;
     pdl_wait();
     pdl_launch();
-    if (h == 0 && b == 0) count_bad_sequences(p);
+    const bool counts = h == 0 && b == 0;
     const int nk = p.n_keys ? p.n_keys[b] : p.n_keys_all;
     float *orow = p.out + ((long long)b * p.n_heads + h) * p.dim;
     if (nk < 1 || nk > p.n_ctx) {
         for (int j = threadIdx.x; j < p.dim; j += blockDim.x) orow[j] = __int_as_float(0x7fc00000);
         if (threadIdx.x == 0 && p.lse) p.lse[(long long)b * p.n_heads + h] = __int_as_float(0x7fc00000);
+        if (counts) count_bad_sequences(p);
         return;
     }
     const int nchunks = (nk + p.chunk - 1) / p.chunk;
@@ -400,6 +405,7 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(const DecodeParams 
     }
     if (p.lse && threadIdx.x == 0)
         p.lse[(long long)b * p.n_heads + h] = (mx + log2f(lsum)) * kLn2;
+    if (counts) count_bad_sequences(p);
 }
 
 // kv_cache.Layer.append for a batch (src/kv_cache.zig:88-95).  grid (batch), block 256.  VEC: four floats at a time (the

@@ -221,22 +221,40 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     }
 }
 
-// The largest of `slots` pairs, by the whole block, in every thread.  (f32 bit patterns of non-negative numbers order
-// like integers.)
-__device__ __forceinline__ uint2 pass_reduce(const uint2 *part, int slots, uint2 *red) {
-    uint2 m = make_uint2(0u, 0u);
-    for (int i = threadIdx.x; i < slots; i += kPassThreads) {
-        const uint2 v = part[i];
-        m.x = max(m.x, v.x), m.y = max(m.y, v.y);
+// The maxima a block of the second launch needs, from the slots the first one left: its own tensor's and, for the row-scaled
+// copy, the largest row norms of dout and v.  (f32 bit patterns of non-negative numbers order like integers.)
+struct PassTops {
+    uint32_t amax, nmax, dn, vn;
+};
+__device__ __forceinline__ PassTops pass_tops(const PassTensor &t, int bg, uint4 *red) {
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    if (t.x) {
+        const uint2 *part = t.part + (long long)bg * t.slots;
+        for (int i = threadIdx.x; i < t.slots; i += kPassThreads) {
+            const uint2 v = part[i];
+            m.x = max(m.x, v.x), m.y = max(m.y, v.y);
+        }
+    }
+    if (t.qs) {
+        const uint2 *part = t.dn_part + (long long)bg * t.dn_slots;
+        for (int i = threadIdx.x; i < t.dn_slots; i += kPassThreads) m.z = max(m.z, part[i].y);
+        if (t.vn_part) {
+            const uint2 *vp = t.vn_part + (long long)bg * t.vn_slots;
+            for (int i = threadIdx.x; i < t.vn_slots; i += kPassThreads) m.w = max(m.w, vp[i].y);
+        } else {
+            m.w = t.vn_final[bg];
+        }
     }
     m.x = __reduce_max_sync(0xffffffffu, m.x), m.y = __reduce_max_sync(0xffffffffu, m.y);
+    m.z = __reduce_max_sync(0xffffffffu, m.z), m.w = __reduce_max_sync(0xffffffffu, m.w);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
-    m = red[0];
 #pragma unroll
-    for (int i = 1; i < kPassThreads / 32; ++i) m.x = max(m.x, red[i].x), m.y = max(m.y, red[i].y);
-    __syncthreads();
-    return m;
+    for (int i = 0; i < kPassThreads / 32; ++i) {
+        const uint4 v = red[i];
+        m.x = max(m.x, v.x), m.y = max(m.y, v.y), m.z = max(m.z, v.z), m.w = max(m.w, v.w);
+    }
+    return PassTops{m.x, m.y, m.z, m.w};
 }
 
 // Four elements times m into the planes at `hi` (null: not wanted) and, times rel as well, into the row-scaled copy.
@@ -256,7 +274,7 @@ __device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long p
 // LP lanes hold a unit of the planes (td columns), NC chunks of four columns each.
 template <int LP, int NC>
 __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
-    constexpr int NG = kPassThreads / LP, U = kPassUnroll;
+    constexpr int NG = kPassThreads / LP, U = kPassUnroll / NC;
     pdl_wait();
     pdl_launch();
     const int blk = (int)blockIdx.x;
@@ -271,36 +289,34 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
         }
         return;
     }
-    __shared__ uint2 red[kPassThreads / 32];
+    __shared__ uint4 red[kPassThreads / 32];
     const PassUnit w = pass_locate(a, a.n, blk);
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
     const long long plane = (long long)t.batch * t.rows * t.heads * a.td;
     const int n4 = a.dim >> 2;
-    uint32_t dn = 0u, vn = 0u;
-    if (t.qs) {
-        dn = pass_reduce(t.dn_part + (long long)w.bg * t.dn_slots, t.dn_slots, red).y;
-        vn = t.vn_part ? pass_reduce(t.vn_part + (long long)w.bg * t.vn_slots, t.vn_slots, red).y : t.vn_final[w.bg];
-    }
     const auto locate = [&](int u, int &r) -> long long {
         r = u / t.group;
         return u < w.units ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
     };
+    PassTops tops{};
     const auto row_rel = [&](long long at) -> float {
         float cq, rel;
-        ds_row_scale(__ldg(t.rnorm + at), dn, vn, cq, rel);
+        ds_row_scale(__ldg(t.rnorm + at), tops.dn, tops.vn, cq, rel);
         return rel;
     };
+    // (the first units' loads go out before the maxima are waited for: many blocks have no second units)
+    const int stride = t.slots * NG * U;
     if (t.x == nullptr) {
-        for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
-            uint2 h[U][NC], l[U][NC];
-            long long at[U];
-            float rel[U];
+        uint2 h[U][NC], l[U][NC];
+        float rn[U];
+        long long at[U];
+        const auto load = [&](int u0) {
 #pragma unroll
             for (int k = 0; k < U; ++k) {
                 int r;
                 at[k] = locate(u0 + k * NG + gi, r);
-                rel[k] = at[k] < 0 ? 1.f : row_rel(at[k]);
+                rn[k] = __ldg(t.rnorm + (at[k] < 0 ? 0 : at[k]));
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const __half *src = t.q_planes + (at[k] < 0 ? 0 : at[k]) * a.td + (li + LP * c) * 4;
@@ -308,55 +324,71 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                     l[k][c] = __ldg(reinterpret_cast<const uint2 *>(src + plane));
                 }
             }
+        };
+        int u0 = w.slot * NG * U;
+        load(u0);
+        tops = pass_tops(t, w.bg, red);
+        for (; u0 < w.units;) {
 #pragma unroll
-            for (int k = 0; k < U; ++k)
+            for (int k = 0; k < U; ++k) {
+                float cq, rel;
+                ds_row_scale(rn[k], tops.dn, tops.vn, cq, rel);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].y));
                     const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].y));
                     // (a sum of the two pieces splits into these very pieces again)
                     if (at[k] >= 0)
-                        store_split4(nullptr, t.qs + at[k] * a.td + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel[k]);
+                        store_split4(nullptr, t.qs + at[k] * a.td + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel);
                 }
+            }
+            u0 += stride;
+            if (u0 < w.units) load(u0);
         }
         return;
     }
-    const uint2 top = pass_reduce(t.part + (long long)w.bg * t.slots, t.slots, red);
+    float4 x[U][NC];
+    long long at[U];
+    const auto load = [&](int u0) {
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            int r;
+            at[k] = locate(u0 + k * NG + gi, r);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int ch = li + LP * c;
+                x[k][c] = (at[k] >= 0 && ch < n4) ? __ldg(reinterpret_cast<const float4 *>(t.x + at[k] * a.dim) + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    };
+    int u0 = w.slot * NG * U;
+    if (t.rope == nullptr) load(u0);
+    tops = pass_tops(t, w.bg, red);
     if (w.slot == 0 && threadIdx.x == 0) {
-        t.amax[w.bg] = top.x;
-        if (t.nmax) t.nmax[w.bg] = top.y;
+        t.amax[w.bg] = tops.amax;
+        if (t.nmax) t.nmax[w.bg] = tops.nmax;
     }
-    const float m = block_mult(top.x);
+    const float m = block_mult(tops.amax);
     if (t.rope == nullptr) {
-        for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
-            float4 x[U][NC];
-            long long at[U];
-            float rel[U];
+        for (; u0 < w.units;) {
 #pragma unroll
             for (int k = 0; k < U; ++k) {
-                int r;
-                at[k] = locate(u0 + k * NG + gi, r);
-                rel[k] = t.qs && at[k] >= 0 ? row_rel(at[k]) : 1.f;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int ch = li + LP * c;
-                    x[k][c] = (at[k] >= 0 && ch < n4) ? __ldg(reinterpret_cast<const float4 *>(t.x + at[k] * a.dim) + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < U; ++k)
+                const float rel = t.qs && at[k] >= 0 ? row_rel(at[k]) : 1.f;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const long long to = at[k] * a.td + (li + LP * c) * 4;
-                    if (at[k] >= 0) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel[k]);
+                    if (at[k] >= 0) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel);
                 }
+            }
+            u0 += stride;
+            if (u0 < w.units) load(u0);
         }
         return;
     }
     // rotated: a lane of the head's lower half takes a chunk and its partner half a head on (a head's halves are
     // multiples of four wide), so that every element and every table entry is fetched once
     const int half = a.dim >> 1, h4 = half >> 2;
-    for (int u0 = w.slot * NG * U; u0 < w.units; u0 += t.slots * NG * U) {
+    for (; u0 < w.units; u0 += stride) {
 #pragma unroll
         for (int k = 0; k < U; ++k) {
             int r;

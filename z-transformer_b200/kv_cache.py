@@ -45,7 +45,9 @@ class Layer:
         if low < 0 or high > self.n_ctx:
             raise DimensionMismatch("kv_cache.Layer.set_lens")
         self._len_bound = high
-        self.len.copy_(lens)
+        # from ordinary host memory that is ours, the copy has been taken off the host when the call returns: nothing waits
+        # for the GPU (given the caller's tensor, pinned perhaps, it would have to)
+        self.len.copy_(lens.clone() if lens.device.type == "cpu" else lens, non_blocking=True)
 
     def check_append(self, k_rows, v_rows) -> None:
         """Every refusal of append, made without writing anything: widths, placement, and Full."""
