@@ -274,7 +274,7 @@ __device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long p
 // LP lanes hold a unit of the planes (td columns), NC chunks of four columns each.
 template <int LP, int NC>
 __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
-    constexpr int NG = kPassThreads / LP, U = kPassUnroll / NC;
+    constexpr int NG = kPassThreads / LP, U = (kPassUnroll + NC - 1) / NC;
     pdl_wait();
     pdl_launch();
     const int blk = (int)blockIdx.x;
@@ -463,7 +463,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
     int rc;
     const dim3 gs((unsigned)stats), gp((unsigned)blocks), th(kPassThreads);
-    const size_t smem = (size_t)kStatsStages * (a.dim > 128 ? 2 : 1) * 2 * kPassThreads * sizeof(float4);
+    const size_t smem = (size_t)kStatsStages * (a.dim <= 128 ? 1 : (a.dim <= 192 ? 3 : 2)) * 2 * kPassThreads * sizeof(float4);
     const auto stats_launch = [&](auto *kernel) -> int {
         if (optin_smem((const void *)kernel, smem)) return 1;
         return launch_pdl("pass_stats_kernel", kernel, gs, th, smem, stream, a);
@@ -471,10 +471,12 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     if (a.dim <= 32) rc = stats_launch(pass_stats_kernel<8, 1>);
     else if (a.dim <= 64) rc = stats_launch(pass_stats_kernel<16, 1>);
     else if (a.dim <= 128) rc = stats_launch(pass_stats_kernel<32, 1>);
+    else if (a.dim <= 192) rc = stats_launch(pass_stats_kernel<16, 3>);
     else rc = stats_launch(pass_stats_kernel<32, 2>);
     if (rc) return rc;
     if (a.td == 64) return launch_pdl("pass_planes_kernel", pass_planes_kernel<16, 1>, gp, th, 0, stream, a);
     if (a.td == 128) return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 1>, gp, th, 0, stream, a);
+    if (a.td == 192) return launch_pdl("pass_planes_kernel", pass_planes_kernel<16, 3>, gp, th, 0, stream, a);
     return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 2>, gp, th, 0, stream, a);
 }
 

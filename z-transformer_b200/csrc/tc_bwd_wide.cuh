@@ -1,4 +1,4 @@
-// Causal GQA attention backward at head_dim 256 (and 132 ... 252 zero-padded to it) on the tensor cores.
+// Causal GQA attention backward at head_dim 192 and 256 (132 ... 252 zero-padded to the next of them) on the tensor cores.
 //
 // What it computes: autograd.attentionBackward (src/autograd.zig:636-842) for a batch, as tc_bwd.cuh does:
 //     P = exp(S - lse),  dP = dO V^T,  dS = P (dP - delta),  dV = P^T dO,  dK = scale dS^T Q,  dQ = scale dS K
@@ -72,7 +72,7 @@ struct WideParams {
     __half *p_planes, *ds_planes;      // [2][unit_cap][Tp][Tp]: hi planes of the chunk's units, then lo planes
     float *dq, *dk, *dv;
     int batch, T, Tp, n_heads, n_kv_heads;
-    int dim_out, td;                   // the tensors' head_dim, the planes' (256)
+    int dim_out, td;                   // the tensors' head_dim, the planes' (192 or 256)
     int unit0, unit_cap;               // the chunk: units (b * n_heads + h) from unit0; planes allocated for unit_cap
     int units, pieces;                 // wide_products: units of the chunk, pieces of kPiece along one head's contraction
     float scale, scale_log2, p_scale;
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
 // grid (units of the chunk, query tiles), 320 threads.
 // ---------------------------------------------------------------------------------------------------
 struct ResShared {
-    uint64_t full[3], freed[3], qh_full, ql_full, a_ready, s_full, s_free, dp_full, dp_free;
+    uint64_t full[4], freed[4], qh_full, ql_full, a_ready, s_full, s_free, dp_full, dp_free;
     uint32_t tmem_base;
     volatile int abort;
 };
@@ -316,15 +316,21 @@ __device__ __forceinline__ void store_rows_quad(__half *dst, long long ld, const
         *reinterpret_cast<uint4 *>(dst + i * ld + j * 8) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
 }
 
+// Slots of the ring of K and V blocks: what shared memory leaves beside the lo planes of Q and dO.
+template <int D>
+__host__ __device__ constexpr int res_slots() { return D == 256 ? 3 : 4; }
+
+template <int D>
 __global__ void __launch_bounds__(kScoreThreads, 1)
     bwd_wide_scores_res(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                         const __grid_constant__ CUtensorMap gmap, const __grid_constant__ CUtensorMap vmap, const WideParams p) {
+    constexpr int NB = D / 64, NR = res_slots<D>();
     constexpr int BT = 128 * 64 * 2;          // one 64-column block of a 128-row tile, one plane: 16 KB
     constexpr int cQh = 0, cGh = 128, cS = 256, cDP = 384;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t *sQl = smem_raw, *sGl = smem_raw + 4 * BT;   // lo planes of Q and dO: four blocks each (hi planes first, staged)
-    uint8_t *ring = smem_raw + 8 * BT;                   // slot s: block hi, block lo at ring + s * 2 BT + {0, 1} BT
-    ResShared *sh = reinterpret_cast<ResShared *>(ring + 3 * 2 * BT);
+    uint8_t *sQl = smem_raw, *sGl = smem_raw + NB * BT;   // lo planes of Q and dO: NB blocks each (hi planes first, staged)
+    uint8_t *ring = smem_raw + 2 * NB * BT;                   // slot s: block hi, block lo at ring + s * 2 BT + {0, 1} BT
+    ResShared *sh = reinterpret_cast<ResShared *>(ring + NR * 2 * BT);
     const int warp = threadIdx.x >> 5;
     // launch order (x fastest): every unit's last query tile, then every unit's last but one, ...: the longest
     // walks of the whole launch start first, so its tail is a fraction of a short walk
@@ -335,10 +341,10 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
     const int group = p.n_heads / p.n_kv_heads, g = h / group;
     const int B = p.batch;
     const int n_tiles = m + 1;
-    const int n_blocks = 8 * n_tiles;  // per tile: K's four blocks, then V's
+    const int n_blocks = 2 * NB * n_tiles;  // per tile: K's blocks, then V's
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 3; ++i) mbar_init(&sh->full[i], 1), mbar_init(&sh->freed[i], 1);
+        for (int i = 0; i < NR; ++i) mbar_init(&sh->full[i], 1), mbar_init(&sh->freed[i], 1);
         mbar_init(&sh->qh_full, 1), mbar_init(&sh->ql_full, 1);
         mbar_init(&sh->a_ready, 8);
         mbar_init(&sh->s_full, 1), mbar_init(&sh->s_free, 8);
@@ -360,39 +366,40 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         if (elect_one() && !sh->abort) {
             tma_prefetch_desc(&qmap), tma_prefetch_desc(&kmap), tma_prefetch_desc(&gmap), tma_prefetch_desc(&vmap);
             // the hi planes first, into the lo planes' place, until the row threads have moved them to TMEM
-            mbar_arrive_expect_tx(&sh->qh_full, 8 * BT);
-            for (int blk = 0; blk < 4; ++blk) {
-                tma_load_4d(sQl + blk * BT, &qmap, &sh->qh_full, 0, m0, h * 4 + blk, b);
-                tma_load_4d(sGl + blk * BT, &gmap, &sh->qh_full, 0, m0, h * 4 + blk, b);
+            mbar_arrive_expect_tx(&sh->qh_full, 2 * NB * BT);
+            for (int blk = 0; blk < NB; ++blk) {
+                tma_load_4d(sQl + blk * BT, &qmap, &sh->qh_full, 0, m0, h * NB + blk, b);
+                tma_load_4d(sGl + blk * BT, &gmap, &sh->qh_full, 0, m0, h * NB + blk, b);
             }
             int issued = 0;
             bool live = true;
             auto load_block = [&](int j) {
-                const int st = j % 3;
-                if (j >= 3 && !rwait(&sh->freed[st], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { rgive_up(sh, 91), live = false; return; }
-                const int n = j >> 3, blk = j & 3;
-                const bool is_v = (j & 4) != 0;
+                const int st = j % NR;
+                if (j >= NR && !rwait(&sh->freed[st], (uint32_t)(((j / NR) & 1) ^ 1), sh)) { rgive_up(sh, 91), live = false; return; }
+                const int n = j / (2 * NB), in_tile = j - n * 2 * NB;
+                const bool is_v = in_tile >= NB;
+                const int blk = is_v ? in_tile - NB : in_tile;
                 const CUtensorMap *mp = is_v ? &vmap : &kmap;
                 uint8_t *base = ring + st * 2 * BT;
                 mbar_arrive_expect_tx(&sh->full[st], 2 * BT);
-                tma_load_4d(base, mp, &sh->full[st], 0, n * 128, g * 4 + blk, b);
-                tma_load_4d(base + BT, mp, &sh->full[st], 0, n * 128, g * 4 + blk, B + b);
+                tma_load_4d(base, mp, &sh->full[st], 0, n * 128, g * NB + blk, b);
+                tma_load_4d(base + BT, mp, &sh->full[st], 0, n * 128, g * NB + blk, B + b);
                 ++issued;
             };
-            for (int j = 0; j < 3 && j < n_blocks; ++j) load_block(j);
+            for (int j = 0; j < NR && j < n_blocks; ++j) load_block(j);
             if (!rwait(&sh->a_ready, 0, sh)) rgive_up(sh, 91), live = false;
             if (live) {
-                mbar_arrive_expect_tx(&sh->ql_full, 8 * BT);
-                for (int blk = 0; blk < 4; ++blk) {
-                    tma_load_4d(sQl + blk * BT, &qmap, &sh->ql_full, 0, m0, h * 4 + blk, B + b);
-                    tma_load_4d(sGl + blk * BT, &gmap, &sh->ql_full, 0, m0, h * 4 + blk, B + b);
+                mbar_arrive_expect_tx(&sh->ql_full, 2 * NB * BT);
+                for (int blk = 0; blk < NB; ++blk) {
+                    tma_load_4d(sQl + blk * BT, &qmap, &sh->ql_full, 0, m0, h * NB + blk, B + b);
+                    tma_load_4d(sGl + blk * BT, &gmap, &sh->ql_full, 0, m0, h * NB + blk, B + b);
                 }
             }
-            for (int j = 3; live && j < n_blocks; ++j) load_block(j);
+            for (int j = NR; live && j < n_blocks; ++j) load_block(j);
             if (sh->abort) {
                 mbar_wait(&sh->qh_full, 0);
                 if (live) mbar_wait(&sh->ql_full, 0);
-                for (int j = (issued > 3 ? issued - 3 : 0); j < issued; ++j) mbar_wait(&sh->full[j % 3], (uint32_t)((j / 3) & 1));
+                for (int j = (issued > NR ? issued - NR : 0); j < issued; ++j) mbar_wait(&sh->full[j % NR], (uint32_t)((j / NR) & 1));
             }
         }
         __syncwarp();
@@ -413,9 +420,9 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
                     tc_fence_after();
                     const uint32_t acc = tmem + (prod ? cDP : cS), a_hi = tmem + (prod ? cGh : cQh);
                     const uint32_t a_lo = prod ? gl_u32 : ql_u32;
-                    for (int blk = 0; blk < 4; ++blk, ++j) {
-                        const int st = j % 3;
-                        if (!rwait(&sh->full[st], (uint32_t)((j / 3) & 1), sh)) { rgive_up(sh, 94); ok = false; break; }
+                    for (int blk = 0; blk < NB; ++blk, ++j) {
+                        const int st = j % NR;
+                        if (!rwait(&sh->full[st], (uint32_t)((j / NR) & 1), sh)) { rgive_up(sh, 94); ok = false; break; }
                         tc_fence_after();
                         const uint32_t base = ring_u32 + (uint32_t)(st * 2 * BT);
                         const uint64_t bh = desc_kmajor(base), bl = desc_kmajor(base + BT);
@@ -450,7 +457,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
             if (!__all_sync(0xffffffffu, rwait(&sh->qh_full, 0, sh))) rgive_up(sh, 95), ok = false;
             const uint8_t *src = (half ? sGl : sQl) + row * 128;
 #pragma unroll 1
-            for (int blk = 0; blk < 4; ++blk) {
+            for (int blk = 0; blk < NB; ++blk) {
                 uint32_t r[32];
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
@@ -542,12 +549,13 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
-inline size_t res_smem_bytes() { return (size_t)14 * (128 * 64 * 2) + sizeof(ResShared); }
+template <int D>
+inline size_t res_smem_bytes() { return (size_t)(2 * D / 64 + 2 * res_slots<D>()) * (128 * 64 * 2) + sizeof(ResShared); }
 
 // ---------------------------------------------------------------------------------------------------
 // The three products that read the planes, in one launch of persistent blocks.  128 x 256 output tiles (a head's whole
 // width, so that a tile of the planes is read once), 64-deep steps, B always the tensor whose rows are the contraction
-// index ([T, width] planes read as N-major tiles).
+// index ([T, width] planes read as N-major tiles).  (128 x 192 tiles, where the planes are 192 columns wide a head.)
 //   dQ      A = dS planes, K-major; contraction over keys [piece * 1024, min((m + 1) * 128, (piece + 1) * 1024)); row t leaves
 //           times scale / (cq(t) mk).
 //   dK, dV  A = dS or P planes read M-major (rows are the contraction index: query rows); contraction over query rows
@@ -596,13 +604,14 @@ struct TriUnit {
     }
 };
 
+template <int D>
 __global__ void __launch_bounds__(kTriThreads, 1)
     wide_products(const __grid_constant__ CUtensorMap ds_k, const __grid_constant__ CUtensorMap ds_m, const __grid_constant__ CUtensorMap p_m,
                   const __grid_constant__ CUtensorMap k_n, const __grid_constant__ CUtensorMap qs_n, const __grid_constant__ CUtensorMap g_n,
                   const WideParams p, int n_units) {
-    // a stage: A hi, A lo (128 x 64 halves each) and B hi, B lo (64 contraction rows x 256 columns each, as four
-    // 64-column blocks of 8 KB): 96 KB; two stages
-    constexpr int kBT = 64 * 256 * 2, kStage = 2 * kTB + 2 * kBT;
+    // a stage: A hi, A lo (128 x 64 halves each) and B hi, B lo (64 contraction rows x D columns each, in
+    // 64-column blocks of 8 KB): 96 KB at D = 256; two stages
+    constexpr int kBT = 64 * D * 2, kStage = 2 * kTB + 2 * kBT;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     TriShared *sh = reinterpret_cast<TriShared *>(smem_raw + 2 * kStage);
     const int warp = threadIdx.x >> 5;
@@ -637,7 +646,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
                 const CUtensorMap *am = w.which == 0 ? &ds_k : w.which == 1 ? &ds_m : &p_m;
                 const CUtensorMap *bm = w.which == 0 ? &k_n : w.which == 1 ? &qs_n : &g_n;
                 // B's column blocks: the head's (dQ: the KV head's) columns
-                const int bblk = (w.which == 0 ? w.h / group : w.h) * p.td / 64;
+                const int bblk = (w.which == 0 ? w.h / group : w.h) * (D / 64);
                 for (int s = 0; s < w.n_steps; ++s, ++it) {
                     const int st = it & 1, k0 = w.k_begin + s * 64;
                     if (it >= 2 && !twait(&sh->freed[st], (uint32_t)(((it >> 1) & 1) ^ 1), sh)) { tgive_up(sh, 85); break; }
@@ -663,7 +672,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
             for (int i = blockIdx.x; i < n_units && !sh->abort; i += gridDim.x) {
                 const TriUnit w(p, i);
                 if (w.n_steps <= 0) continue;
-                const uint32_t idesc = w.which ? idesc_f16(128, 256, true, true) : idesc_f16(128, 256, false, true);
+                const uint32_t idesc = w.which ? idesc_f16(128, D, true, true) : idesc_f16(128, D, false, true);
                 const uint32_t a_step = w.which ? 2048 : 32;
                 const uint32_t acc = tmem + (n & 1) * 256;
                 if (n >= 2 && !twait(&sh->acc_free[n & 1], (uint32_t)(((n >> 1) & 1) ^ 1), sh)) { tgive_up(sh, 86); break; }
@@ -719,11 +728,11 @@ __global__ void __launch_bounds__(kTriThreads, 1)
             float *dst = (w.which == 0 ? p.dq : w.which == 1 ? p.dk : p.dv) + ((long long)w.b * p.T + row0) * ld +
                          (long long)(w.which == 0 ? w.h : g) * p.dim_out + 4 * j8;
 #pragma unroll 1
-            for (int c = 0; c < 256; c += 32) {
+            for (int c = 0; c < D; c += 32) {
                 uint32_t r[32];
                 tmem_ld32(tmem + lane_base + (n & 1) * 256 + c, r);
                 tmem_wait_ld();
-                if (c + 32 == 256) {  // all read: the MMAs may have the buffer while the last columns are on their way
+                if (c + 32 == D) {  // all read: the MMAs may have the buffer while the last columns are on their way
                     tc_fence_before();
                     mbar_arrive_warp_relaxed(&sh->acc_free[n & 1]);
                 }
@@ -763,7 +772,8 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-inline size_t tri_smem_bytes() { return (size_t)2 * (2 * kTB + 2 * 64 * 256 * 2) + sizeof(TriShared); }
+template <int D>
+inline size_t tri_smem_bytes() { return (size_t)2 * (2 * kTB + 2 * 64 * D * 2) + sizeof(TriShared); }
 
 // ---- host side ----------------------------------------------------------------------------------------
 
@@ -859,17 +869,20 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         !make_half_tile_map(&k_k, w.k_planes, 2 * batch, T, wkv, 64, 128) ||
         !make_half_tile_map(&g_k, w.do_planes, 2 * batch, T, wq, 64, 128) ||
         !make_half_tile_map(&v_k, w.v_planes, 2 * batch, T, wkv, 64, 128) ||
-        !make_half_tile_map(&k_n, w.k_planes, 2 * batch, T, wkv, 256, 64) ||
-        !make_half_tile_map(&qs_n, w.qs_planes, 2 * batch, T, wq, 256, 64) ||
-        !make_half_tile_map(&g_n, w.do_planes, 2 * batch, T, wq, 256, 64) ||
+        !make_half_tile_map(&k_n, w.k_planes, 2 * batch, T, wkv, td, 64) ||
+        !make_half_tile_map(&qs_n, w.qs_planes, 2 * batch, T, wq, td, 64) ||
+        !make_half_tile_map(&g_n, w.do_planes, 2 * batch, T, wq, td, 64) ||
         !make_half_tile_map(&ds_k, ww.ds_planes, 2 * cap, Tp, Tp, 64, 128) ||
         !make_half_tile_map(&ds_m, ww.ds_planes, 2 * cap, Tp, Tp, 128, 64) ||
         !make_half_tile_map(&p_m, ww.p_planes, 2 * cap, Tp, Tp, 128, 64))
         return refuse("the TMA tensor maps for the wide-head backward could not be encoded.");
     const size_t smem = wide_smem_bytes();
-    const size_t smem_t = tri_smem_bytes(), smem_r = res_smem_bytes();
-    if (optin_smem((const void *)bwd_wide_scores, smem) || optin_smem((const void *)bwd_wide_scores_res, smem_r) ||
-        optin_smem((const void *)wide_products, smem_t))
+    const size_t smem_t = td == 192 ? tri_smem_bytes<192>() : tri_smem_bytes<256>();
+    const size_t smem_r = td == 192 ? res_smem_bytes<192>() : res_smem_bytes<256>();
+    const auto scores = td == 192 ? bwd_wide_scores_res<192> : bwd_wide_scores_res<256>;
+    const auto products = td == 192 ? wide_products<192> : wide_products<256>;
+    if (optin_smem((const void *)bwd_wide_scores, smem) || optin_smem((const void *)scores, smem_r) ||
+        optin_smem((const void *)products, smem_t))
         return 1;
     WideParams p{};
     p.lse = lse, p.delta = delta, p.rnorm = w.rnorm;
@@ -894,12 +907,12 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
             if (launch_after("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
         } else {
             const dim3 gs((unsigned)units, (unsigned)nt);
-            if (launch_after("bwd_wide_scores_res", bwd_wide_scores_res, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores_res", scores, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
         }
         p.units = units;
         const long long n_units = 3LL * nt * units * p.pieces;
         const dim3 gp((unsigned)(n_units < split_sm_count() ? n_units : split_sm_count()));
-        if (launch_after("wide_products", wide_products, gp, dim3(kTriThreads), smem_t, stream, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
+        if (launch_after("wide_products", products, gp, dim3(kTriThreads), smem_t, stream, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
             return 1;
     }
     return 0;

@@ -294,13 +294,16 @@ __device__ __forceinline__ float tf32_round(float x) {
 }  // namespace tc
 
 // ---- host: which shapes the tensor-core kernels take ------------------------------------------------
-// They have tiles of 64, 128 and 256 columns; a head of any other width runs on the next wider tile.  The operand
+// They have tiles of 64, 128, 192 and 256 columns; a head of any other width runs on the next wider tile.  The operand
 // planes carry every head zero-padded to the tile's width, outputs keep their own (rows leave in 16-byte chunks,
 // hence the multiple of four).  The padding costs at most half of the tensor work (head_dim 68 on 128 columns;
 // below 64 an MMA of half the width or depth costs the same clocks anyway), and what it replaces is the CUDA-core
 // kernels at a thirtieth of the rate: head_dim 80, batch 4, T 1000, 16/4 heads, forward and backward 7.6 ms there,
-// 0.45 ms here.
-inline int tc_tile_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : 256); }
+// 0.45 ms here.  192 columns lie between because 132 ... 192 padded to 256 paid a third more MMAs, plane bytes and
+// operand traffic for nothing: us on 256 -> on 192 columns, 16/4 heads of 192, forward and backward of batch 4, T 1024
+// 611 -> 526, forward of batch 4, T 2048 562 -> 486, a window of 512 rows at 3584 165 -> 128; 8/2 heads of 160,
+// batch 2, T 4096 1633 -> 1443.
+inline int tc_tile_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : (dim <= 192 ? 192 : 256)); }
 inline bool tc_takes_dim(int dim) { return dim % 4 == 0 && dim >= 32 && dim <= 256; }
 // Keys from which the forward goes to the tensor cores: up to 32 the CUDA-core forward is one launch of one row and one
 // key tile and the quicker of the two (32/8 heads of 128: 17 us against 28 at 32 rows, 29.5 against 28.5 at 48, 57

@@ -565,7 +565,8 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
 }
 
 // (tc_fwd16x.cuh)
-inline int launch_x(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
+template <int D>
+inline int launch_x_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
                     cudaStream_t stream);
 // (tc_fwd16g.cuh)
 template <int D>
@@ -615,7 +616,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     if (launch_pass(pa, stream)) return 1;
     CUtensorMap kmap, vmap, qmap;  // (the widest tile fetches K block by block, see attn_fwd_tc16x)
-    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td == 256 ? 64 : td, 64) ||
+    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td > 128 ? 64 : td, 64) ||
         !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
         !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
@@ -640,9 +641,10 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     // and that still gives every SM a CTA (half as many CTAs), one head per CTA (attn_fwd_tc16) otherwise; 1: one head
     // per CTA; 2: two heads per CTA whatever the number of CTAs (the group must be even).
     const long long pair_ctas = (long long)((T + 127) / 128) * (n_heads / 2) * batch;
-    const bool pairs = td != 256 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
+    const bool pairs = td <= 128 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
     int rc;
-    if (td == 256) rc = tcf16::launch_x(kmap, vmap, qmap, p, stream);
+    if (td == 256) rc = tcf16::launch_x_d<256>(kmap, vmap, qmap, p, stream);
+    else if (td == 192) rc = tcf16::launch_x_d<192>(kmap, vmap, qmap, p, stream);
     else if (pairs) rc = td == 64 ? tcf16::launch_g_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_g_d<128>(kmap, vmap, qmap, p, stream);
     else rc = td == 64 ? tcf16::launch_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_d<128>(kmap, vmap, qmap, p, stream);
     if (rc || p.parts == 1) return rc;

@@ -1,4 +1,4 @@
-// attn_fwd_tc16x: the f16-split forward for head widths up to 256 (head_dim 256, and 192 zero-padded to it).
+// attn_fwd_tc16x<D>: the f16-split forward for head widths above 128, on tiles of D = 192 or 256 columns.
 //
 // At 256 columns a head no longer fits the layout of attn_fwd_tc16 / tc16g: one O accumulator alone is 256 of
 // the 512 TMEM columns, and a 64-key K or V tile (hi and lo planes) is 64 KB.  This kernel keeps their
@@ -6,21 +6,20 @@
 // O += Ph.Vh + Ph.Vl + Pl.Vh, online softmax in the log2 domain with a lazily moved maximum) and changes
 // what the sizes force:
 //   CTA    128 query rows of ONE head; 6 warps: four softmax warps (a thread per row, every key tile), TMA, MMA.
-//   TMEM   [0, 128) Q hi as the A operand, [128, 384) O, [384, 512) two S/P tiles of 64 columns.
-//   smem   Q lo (64 KB; an SS MMA for the Ql.Kh term), ONE K tile and ONE V tile (64 KB each) = 192 KB.
-//   K      is a ring of its four 64-column blocks rather than of whole tiles: S contracts over the blocks one
+//   TMEM   [0, 128) Q hi as the A operand, [128, 128 + D) O, [384, 512) two S/P tiles of 64 columns.
+//   smem   Q lo (an SS MMA for the Ql.Kh term), ONE K tile and ONE V tile, 64 KB each at D = 256.
+//   K      is a ring of its 64-column blocks rather than of whole tiles: S contracts over the blocks one
 //          after the other, a block is free as soon as its twelve MMAs have retired and the same block of the
 //          next tile is fetched into it while the later blocks are still being read.  So S(j+1) can follow
 //          S(j) at once although there is room for one K tile only.
 //   MMA    S(0) S(1) | P.V(0) S(2) | P.V(1) S(3) | ...: the softmax of tile j+1 runs under P.V(j) and S(j+2).
 //          V(j+1) is fetched while S(j+2) runs.
-// Per 64-key tile the tensor core issues 48 MMAs of N = 64 for S and 12 of N = 256 for P.V.
+// Per 64-key tile the tensor core issues 12 MMAs of N = 64 per block for S and 12 of N = D for P.V: heads of 132 to 192
+// columns on a tile of 192 issue three quarters of what they cost padded to 256.
 // The Q hi tile reaches TMEM through V's slot (TMA, then the row threads); the rows leave through the K and V
-// slots (128 KB), a row per store instruction.  Every wait is bounded; a wait that gives up raises g_tc_status.
+// slots, a row in two store instructions.  Every wait is bounded; a wait that gives up raises g_tc_status.
 //
-// The backward at these widths has no tensor-core form: dK and dV are two 256-column accumulators, and K, V, Q and
-// dO tiles of 64 rows are 64 KB each with their lo planes -- neither fits beside the other.  It stays on the
-// CUDA-core kernels.
+// The backward at these widths: tc_bwd_wide.cuh.
 #pragma once
 
 #include "tc_fwd16.cuh"
@@ -48,19 +47,19 @@ __device__ __forceinline__ void xgive_up(SharedX *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-// kmap: K planes with a box of ONE 64-column block x 64 keys; vmap: V planes, four blocks x 64 keys; qmap: Q planes,
-// four blocks x 128 rows.
-template <bool FLUSH>
+// kmap: K planes with a box of ONE 64-column block x 64 keys; vmap: V planes, the head's D / 64 blocks x 64 keys; qmap:
+// Q planes, the head's blocks x 128 rows.
+template <int D, bool FLUSH>
 __global__ void __launch_bounds__(kThreadsX, 1)
     attn_fwd_tc16x(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                    const __grid_constant__ CUtensorMap qmap, const Params p) {
-    constexpr int D = 256, NB = 4, BN = 64;
+    constexpr int NB = D / 64, BN = 64;
     constexpr int KB = BN * 128;        // bytes of one 64-column block of one plane of a key tile (8 KB)
-    constexpr int KP = NB * KB;         // one plane of a key tile (32 KB); a K or V tile is 2 KP
+    constexpr int KP = NB * KB;         // one plane of a key tile (32 KB at 256 columns); a K or V tile is 2 KP
     constexpr int QB = 128 * 128;       // one block of one plane of the 128-row query tile (16 KB)
     constexpr int cQh = 0, cO = 128, cS0 = 384;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // K: block c of the tile at sK + c * 2 KB (hi, then lo); V: hi plane, lo plane; Q lo: four blocks
+    // K: block c of the tile at sK + c * 2 KB (hi, then lo); V: hi plane, lo plane; Q lo: NB blocks
     uint8_t *sK = smem_raw, *sV = sK + 2 * KP, *sQl = sV + 2 * KP;
     SharedX *sh = reinterpret_cast<SharedX *>(sQl + NB * QB);
 
@@ -87,7 +86,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     const int B = p.batch;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; ++i) mbar_init(&sh->full_k[i], 1), mbar_init(&sh->free_k[i], 1);
+        for (int i = 0; i < NB; ++i) mbar_init(&sh->full_k[i], 1), mbar_init(&sh->free_k[i], 1);
         mbar_init(&sh->full_v, 1), mbar_init(&sh->free_v, 1);
         mbar_init(&sh->a_ready, 4);
         mbar_init(&sh->q_full, 1), mbar_init(&sh->ql_full, 1);
@@ -317,8 +316,8 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             ok = false;
         }
         // The rows go to global memory through shared memory (the K and V slots are idle once all_done completes):
-        // 128 rows x 1 KB; a row per store instruction instead of 32.
-        // (16-byte chunk c of row r sits at chunk c ^ (r & 31))
+        // 128 rows of 4 D bytes; a row in two store instructions instead of 32.
+        // (16-byte chunk c of row r sits at chunk c ^ (r & 15): a row is a multiple of sixteen chunks)
         uint8_t *stage = smem_raw;
         if (ok) {
             tc_fence_after();
@@ -337,7 +336,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                     if (add && c + i < row.width) o4 = flush_sum4(row.at<D>(c + i), ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     const int ch = (c + i) >> 2;
-                    *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & 31)) << 4)) = o4;
+                    *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & 15)) << 4)) = o4;
                 }
             }
             if (p.lse && t < p.T) p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
@@ -346,14 +345,15 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         if (__all_sync(0xffffffffu, xwait(&sh->staged, 0, sh)) && !sh->abort) {
             const long long wo = (long long)p.n_heads * p.dim_out;
             const float mo = p.o_planes ? out_plane_mult(p, b) : 1.f;
-            // a warp stores its 32 rows; a row is 64 chunks: two instructions of 32 lanes each
+            // a warp stores its 32 rows; a row is 48 or 64 chunks: two instructions
 #pragma unroll 4
             for (int i = 0; i < 32; ++i) {
                 const int r = warp * 32 + i;
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     const int ch = half * 32 + lane;
-                    const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * (D * 4) + ((ch ^ (r & 31)) << 4));
+                    if (ch >= D / 4) continue;
+                    const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * (D * 4) + ((ch ^ (r & 15)) << 4));
                     if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
                         store_out4(p, part * p.out_part + ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
                 }
@@ -365,10 +365,11 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     if (warp == 5) tmem_dealloc(tmem, 512);
 }
 
-inline int launch_x(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
+template <int D>
+inline int launch_x_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
                     cudaStream_t stream) {
-    const size_t smem = 3 * (size_t)(2 * 64 * 256 * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
-    const auto kernel = p.flush ? attn_fwd_tc16x<true> : attn_fwd_tc16x<false>;
+    const size_t smem = 3 * (size_t)(2 * 64 * D * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
+    const auto kernel = p.flush ? attn_fwd_tc16x<D, true> : attn_fwd_tc16x<D, false>;
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
     return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
