@@ -62,7 +62,7 @@ __host__ __device__ constexpr size_t fused_smem_bytes() {
 // grid (n_kv_heads, ceil(T / 128), batch), 608 threads: 16 row warps, a TMA warp, two MMA warps.
 constexpr int kFusedThreads = (kKvRowWarps + 3) * 32;
 // PARTS: the walk is split (tc_split.cuh).  A variant of its own: the whole walk is 1 % slower with the code in it.
-template <int D, bool PARTS>
+template <int D, bool PARTS, bool PAD>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     attn_bwd_fused_tc(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                       const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap gmap,
@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         // dP^T / dS^T and dQ^T.  What crosses between them goes through the row threads' barriers.
         if (elect_one()) {
             constexpr uint32_t id_s = idesc_f16(128, BQ, false, false);   // S^T: A = K, B = the query tile, both K-major
-            constexpr uint32_t id_a = idesc_f16(128, D, false, true);     // dV: A in TMEM, B the dO tile N-major
+            const int steps = PAD ? head_steps(p.dim_out) : D / 16;
+            const uint32_t id_a = idesc_f16(128, 16 * steps, false, true);  // dV: A in TMEM, B the dO tile N-major
             bool ok = !sh->abort && fwait(&sh->k_full, 0, sh);
             if (!ok) fgive_up(sh, 62);
             tc_fence_after();
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 const uint64_t bqh = desc_kmajor(qh), bql = desc_kmajor(qh + QP);
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
+                    if (PAD && kk >= steps) break;
                     const uint32_t ao = (uint32_t)((kk >> 2) * (128 * 128) + (kk & 3) * 32);
                     const uint32_t bo = (uint32_t)((kk >> 2) * (BQ * 128) + (kk & 3) * 32);
                     const uint64_t dkh = desc_advance(bkh, ao), dkl = desc_advance(bkl, ao);
@@ -268,7 +270,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         // ------------------------------------------------------------------ MMA issuer of the dS side: dP^T, dK, dQ^T
         if (elect_one()) {
             constexpr uint32_t id_s = idesc_f16(128, BQ, false, false);   // dP^T: A = V (TMEM hi, shared lo), B = the dO tile K-major
-            constexpr uint32_t id_a = idesc_f16(128, D, false, true);     // dK: A in TMEM, B the query tile N-major
+            const int steps = PAD ? head_steps(p.dim_out) : D / 16;
+            const uint32_t id_a = idesc_f16(128, 16 * steps, false, true);  // dK: A in TMEM, B the query tile N-major
             constexpr uint32_t id_q = idesc_f16(128, BQ, true, true);     // dQ^T: A = K read M-major, B = dS^T N-major
             bool ok = !sh->abort && fwait(&sh->k_full, 0, sh) && fwait(&sh->a_ready, 0, sh);
             if (!ok) fgive_up(sh, 62);
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 const uint64_t bgh = desc_kmajor(g_u32), bgl = desc_kmajor(g_u32 + QP);
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
+                    if (PAD && kk >= steps) break;
                     const uint32_t ao = (uint32_t)((kk >> 2) * (128 * 128) + (kk & 3) * 32);
                     const uint32_t bo = (uint32_t)((kk >> 2) * (BQ * 128) + (kk & 3) * 32);
                     const uint64_t dvl = desc_advance(bvl, ao);
@@ -635,7 +639,7 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
                               const BwdParams &p, cudaStream_t stream) {
     size_t smem = fused_smem_bytes<D>();
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    const auto kernel = p.parts.n() > 1 ? attn_bwd_fused_tc<D, true> : attn_bwd_fused_tc<D, false>;
+    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused_tc<D, parts.value, pad.value>; }, p.parts.n() > 1, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)(p.batch * p.parts.n()));
     return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);

@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             constexpr uint32_t idesc = idesc_f16(128, 128, false, false);
+            const int steps = head_steps(p.dim_out);
             bool ok = !sh->abort && rwait(&sh->a_ready, 0, sh) && rwait(&sh->ql_full, 0, sh);
             if (!ok) rgive_up(sh, 92);
             tc_fence_after();
@@ -429,6 +430,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
                         const uint64_t al = desc_kmajor(a_lo + (uint32_t)(blk * BT));
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
+                            if (blk * 4 + kk >= steps) break;
                             const uint64_t dbh = desc_advance(bh, kk * 32), dbl = desc_advance(bl, kk * 32);
                             const uint32_t at = a_hi + (uint32_t)((blk * 4 + kk) * 8);
                             mma_ts_f16(acc, at, dbh, idesc, (blk > 0 || kk > 0) ? 1 : 0);
@@ -672,7 +674,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
             for (int i = blockIdx.x; i < n_units && !sh->abort; i += gridDim.x) {
                 const TriUnit w(p, i);
                 if (w.n_steps <= 0) continue;
-                const uint32_t idesc = w.which ? idesc_f16(128, D, true, true) : idesc_f16(128, D, false, true);
+                const uint32_t idesc = idesc_f16(128, 16 * head_steps(p.dim_out), w.which != 0, true);
                 const uint32_t a_step = w.which ? 2048 : 32;
                 const uint32_t acc = tmem + (n & 1) * 256;
                 if (n >= 2 && !twait(&sh->acc_free[n & 1], (uint32_t)(((n >> 1) & 1) ^ 1), sh)) { tgive_up(sh, 86); break; }

@@ -7,10 +7,12 @@
 // protocol mistake costs a wrong answer and a status word, never a hung GPU.
 #pragma once
 
+
 #include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 namespace zt {
 namespace tc {
@@ -233,6 +235,18 @@ __device__ __forceinline__ uint64_t desc_mnmajor_16b(uint32_t addr, uint32_t blo
 __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, bool a_mn_major, bool b_mn_major) {
     return (1u << 4) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+// What of a tile's columns an MMA has to cover for a head of `dim` of them: sixteen-column steps where they are the
+// contraction, columns where they are N.  The padding beyond is zeros that only cost time: at 80 columns on a tile of 128,
+// three steps of eight in S and dP and three eighths of N in the products that leave in head columns.
+__host__ __device__ constexpr int head_steps(int dim) { return (dim + 15) >> 4; }
+// The variant of a kernel template that two flags choose.  (Kernels whose MMA-issuing threads are on the critical path have
+// the padded form as a variant of its own: the check of every step cost heads that fill their tile 0.9 %.)
+template <class F>
+inline auto with_flags(F pick, bool a, bool b) {
+    using std::true_type, std::false_type;
+    return a ? (b ? pick(true_type{}, true_type{}) : pick(true_type{}, false_type{}))
+             : (b ? pick(false_type{}, true_type{}) : pick(false_type{}, false_type{}));
 }
 __device__ __forceinline__ void mma_ts_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                            uint32_t accumulate) {

@@ -37,7 +37,7 @@ __device__ __forceinline__ void ggive_up(SharedG *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-template <int D, bool FLUSH>
+template <int D, bool FLUSH, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
     attn_fwd_tc16g(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                    const __grid_constant__ CUtensorMap qmap, const Params p) {
@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             constexpr uint32_t id_s = idesc_f16(128, BN, false, false);
-            constexpr uint32_t id_o = idesc_f16(128, D, false, true);
+            const int steps = PAD ? head_steps(p.dim_out) : D / 16;
+            const uint32_t id_o = idesc_f16(128, 16 * steps, false, true);
             bool ok = gwait(&sh->a_ready, 0, sh) && gwait(&sh->ql_full, 0, sh);
             if (!ok) ggive_up(sh, 42);
             tc_fence_after();
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t cS = cS0 + hd * BN, cQ = cQh + hd * W2;
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
+                    if (PAD && kk >= steps) break;
                     const uint32_t ao = (uint32_t)((kk >> 2) * (128 * 128) + (kk & 3) * 32);
                     const uint32_t bo = (uint32_t)((kk >> 2) * (BN * 128) + (kk & 3) * 32);
                     const uint64_t dkh = desc_advance(bkh, bo), dkl = desc_advance(bkl, bo);
@@ -354,7 +356,7 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
                       cudaStream_t stream) {
     size_t smem = 14 * (size_t)(64 * D * 2) + sizeof(SharedG);
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    const auto kernel = p.flush ? attn_fwd_tc16g<D, true> : attn_fwd_tc16g<D, false>;
+    const auto kernel = with_flags([](auto flush, auto pad) { return attn_fwd_tc16g<D, flush.value, pad.value>; }, p.flush, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)(p.n_heads / 2), (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
     return launch_after("attn_fwd_tc16g", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);

@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             constexpr uint32_t id_s = idesc_f16(128, BN, false, false);
-            constexpr uint32_t id_o = idesc_f16(128, D, false, true);
+            const int steps = head_steps(p.dim_out);
+            const uint32_t id_o = idesc_f16(128, 16 * steps, false, true);
             bool ok = xwait(&sh->a_ready, 0, sh) && xwait(&sh->ql_full, 0, sh);
             if (!ok) xgive_up(sh, 62);
             tc_fence_after();
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         const int kk = c * 4 + ks;
+                        if (kk >= steps) break;
                         const uint64_t dkh = desc_advance(bkh, ks * 32), dkl = desc_advance(bkl, ks * 32);
                         mma_ts_f16(tmem + cS, tmem + cQh + kk * 8, dkh, id_s, kk > 0);
                         mma_ts_f16(tmem + cS, tmem + cQh + kk * 8, dkl, id_s, 1);
