@@ -26,6 +26,8 @@ def normal(oracle, shape, stream):
     (1, 1000, 4, 2, 64), (1, 700, 3, 3, 40), (2, 300, 8, 1, 128), (1, 1100, 2, 1, 72),
     # the 192-column tile: its narrowest and widest heads, several key tiles a block, more than one piece of a contraction
     (1, 385, 3, 3, 132), (2, 300, 4, 2, 192), (1, 1290, 2, 1, 188),
+    # planes narrower than the tile, on either side of where they become so
+    (1, 300, 4, 2, 32), (2, 200, 2, 1, 72), (1, 200, 2, 2, 96), (1, 200, 4, 2, 100),
 ])
 def test_widths_and_short_sequences(zt, oracle, B, T, H, Hkv, D):
     q, k, v, do = (normal(oracle, (B, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv, H)))
@@ -51,6 +53,8 @@ def test_widths_and_short_sequences(zt, oracle, B, T, H, Hkv, D):
     (2, 700, 702, 4, 2, 64), (16, 3000, 3016, 2, 1, 96), (150, 5000, 5200, 4, 4, 64), (100, 2500, 2600, 2, 2, 256),
     (700, 1, 701, 2, 1, 64), (250, 9000, 9250, 8, 2, 40),
     (300, 2100, 2400, 4, 1, 192), (100, 2500, 2600, 2, 2, 160),
+    # not split, and the planes narrower than the tile: one of the two running sums lives in the query rows' planes
+    (40, 2100, 2140, 76, 76, 72),
 ])
 def test_windows_of_a_prompt(zt, oracle, T, q_offset, ctx, H, Hkv, D):
     """device.Attn.forward_at: rows at q_offset over the first q_offset + T keys; what lies beyond is never read."""

@@ -90,7 +90,7 @@ struct PassTensor {
     const float *x;          // [batch][rows][heads * dim]; null: no f32 source, see q_planes
     const float *o;          // with delta: the tensor it is formed with
     float *delta, *rnorm;    // [batch][rows][heads], or null
-    __half *planes;          // [2][batch][rows][heads * td], or null
+    __half *planes;          // [2][batch][rows][heads * pd], or null
     uint2 *part;             // [batch * groups][slots] (max |x|, largest row norm) as f32 bit patterns
     uint32_t *amax, *nmax;   // [batch * groups]: where the maxima are published; nmax null: not wanted
     const float2 *rope;      // null, or the (cos, sin) table [rows][dim / 2]: x is rotated on its way into the planes
@@ -110,7 +110,7 @@ struct PassArgs {
     float4 *fill[3];
     long long fill_n4[3];
     int fill_first[4];  // first block of each region; [n_fill]: one past the last
-    int n, n_stats, n_fill, dim, td;
+    int n, n_stats, n_fill, dim, pd;  // dim: columns of a head in the tensors; pd: in the planes (plane_dim)
 };
 
 struct PassUnit {  // where a block stands
@@ -271,7 +271,7 @@ __device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long p
     *reinterpret_cast<uint2 *>(qs) = hw, *reinterpret_cast<uint2 *>(qs + plane) = lw;
 }
 
-// LP lanes hold a unit of the planes (td columns), NC chunks of four columns each.
+// LP lanes hold a unit of the planes (pd columns), NC chunks of four columns each.
 template <int LP, int NC>
 __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
     constexpr int NG = kPassThreads / LP, U = (kPassUnroll + NC - 1) / NC;
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     const PassUnit w = pass_locate(a, a.n, blk);
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
-    const long long plane = (long long)t.batch * t.rows * t.heads * a.td;
+    const long long plane = (long long)t.batch * t.rows * t.heads * a.pd;
     const int n4 = a.dim >> 2;
     const auto locate = [&](int u, int &r) -> long long {
         r = u / t.group;
@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                 rn[k] = __ldg(t.rnorm + (at[k] < 0 ? 0 : at[k]));
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const __half *src = t.q_planes + (at[k] < 0 ? 0 : at[k]) * a.td + (li + LP * c) * 4;
+                    const int col = (li + LP * c) * 4;
+                    const __half *src = t.q_planes + (at[k] < 0 ? 0 : at[k]) * a.pd + (col < a.pd ? col : 0);
                     h[k][c] = __ldg(reinterpret_cast<const uint2 *>(src));
                     l[k][c] = __ldg(reinterpret_cast<const uint2 *>(src + plane));
                 }
@@ -338,8 +339,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                     const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].y));
                     const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].y));
                     // (a sum of the two pieces splits into these very pieces again)
-                    if (at[k] >= 0)
-                        store_split4(nullptr, t.qs + at[k] * a.td + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel);
+                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd)
+                        store_split4(nullptr, t.qs + at[k] * a.pd + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel);
                 }
             }
             u0 += stride;
@@ -376,8 +377,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                 const float rel = t.qs && at[k] >= 0 ? row_rel(at[k]) : 1.f;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const long long to = at[k] * a.td + (li + LP * c) * 4;
-                    if (at[k] >= 0) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel);
+                    const long long to = at[k] * a.pd + (li + LP * c) * 4;
+                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel);
                 }
             }
             u0 += stride;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
             if (at < 0) break;
             const float rel = t.qs ? row_rel(at) : 1.f;
             const auto put = [&](int col, float4 v) {
-                const long long to = at * a.td + col;
+                const long long to = at * a.pd + col;
                 store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, v, m, rel);
             };
 #pragma unroll
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                     lr.z = rope_elem(lo.z, hi.z, make_float2(q.x, q.y), false, false), hr.z = rope_elem(hi.z, lo.z, make_float2(q.x, q.y), true, false);
                     lr.w = rope_elem(lo.w, hi.w, make_float2(q.z, q.w), false, false), hr.w = rope_elem(hi.w, lo.w, make_float2(q.z, q.w), true, false);
                     put(ch * 4, lr), put(half + ch * 4, hr);
-                } else if (ch >= n4) {
+                } else if (ch >= n4 && ch * 4 < a.pd) {
                     put(ch * 4, make_float4(0.f, 0.f, 0.f, 0.f));
                 }
             }
@@ -463,21 +464,21 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
     int rc;
     const dim3 gs((unsigned)stats), gp((unsigned)blocks), th(kPassThreads);
-    const size_t smem = (size_t)kStatsStages * (a.dim <= 128 ? 1 : (a.dim <= 192 ? 3 : 2)) * 2 * kPassThreads * sizeof(float4);
-    const auto stats_launch = [&](auto *kernel) -> int {
-        if (optin_smem((const void *)kernel, smem)) return 1;
-        return launch_pdl("pass_stats_kernel", kernel, gs, th, smem, stream, a);
+    // lanes x chunks of four columns that a unit takes: the tightest that holds it
+    const auto both = [&](auto lanes, auto chunks) -> int {
+        constexpr int LP = lanes.value, NC = chunks.value;
+        const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
+        if (optin_smem((const void *)pass_stats_kernel<LP, NC>, smem)) return 1;
+        rc = launch_pdl("pass_stats_kernel", pass_stats_kernel<LP, NC>, gs, th, smem, stream, a);
+        return rc ? rc : launch_pdl("pass_planes_kernel", pass_planes_kernel<LP, NC>, gp, th, 0, stream, a);
     };
-    if (a.dim <= 32) rc = stats_launch(pass_stats_kernel<8, 1>);
-    else if (a.dim <= 64) rc = stats_launch(pass_stats_kernel<16, 1>);
-    else if (a.dim <= 128) rc = stats_launch(pass_stats_kernel<32, 1>);
-    else if (a.dim <= 192) rc = stats_launch(pass_stats_kernel<16, 3>);
-    else rc = stats_launch(pass_stats_kernel<32, 2>);
-    if (rc) return rc;
-    if (a.td == 64) return launch_pdl("pass_planes_kernel", pass_planes_kernel<16, 1>, gp, th, 0, stream, a);
-    if (a.td == 128) return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 1>, gp, th, 0, stream, a);
-    if (a.td == 192) return launch_pdl("pass_planes_kernel", pass_planes_kernel<16, 3>, gp, th, 0, stream, a);
-    return launch_pdl("pass_planes_kernel", pass_planes_kernel<32, 2>, gp, th, 0, stream, a);
+    using std::integral_constant;
+    if (a.pd <= 32) return both(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+    if (a.pd <= 64) return both(integral_constant<int, 16>{}, integral_constant<int, 1>{});
+    if (a.pd <= 96) return both(integral_constant<int, 8>{}, integral_constant<int, 3>{});
+    if (a.pd <= 128) return both(integral_constant<int, 32>{}, integral_constant<int, 1>{});
+    if (a.pd <= 192) return both(integral_constant<int, 16>{}, integral_constant<int, 3>{});
+    return both(integral_constant<int, 32>{}, integral_constant<int, 2>{});
 }
 
 }  // namespace tcb

@@ -148,22 +148,6 @@ struct Walk {
     }
 };
 
-// One row of `words` packed-half words from global memory into TMEM columns [col, col + words).
-template <int WORDS>
-__device__ __forceinline__ void row_to_tmem(const __half *src, bool valid, uint32_t taddr) {
-#pragma unroll 1
-    for (int c = 0; c < WORDS; c += 32) {
-        uint32_t r[32];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (valid) v = __ldg(reinterpret_cast<const uint4 *>(src) + (c + i) / 4);
-            r[i] = v.x, r[i + 1] = v.y, r[i + 2] = v.z, r[i + 3] = v.w;
-        }
-        tmem_st32(taddr + c, r);
-    }
-}
-
 // ---------------------------------------------------------------------------------------------------
 // dK, dV.  grid (ceil(T / 128), n_kv_heads, batch), 576 threads: 16 row warps, a TMA warp, an MMA warp.
 //
@@ -206,12 +190,13 @@ __host__ __device__ constexpr size_t kv_smem_bytes() {
 }
 
 // 16 packed-half words of one row from global memory into TMEM columns [taddr, taddr + 16).
-__device__ __forceinline__ void row_to_tmem16(const __half *src, bool valid, uint32_t taddr) {
+// (`chunks`: how many of the four 16-byte chunks are the row's; zeros beyond)
+__device__ __forceinline__ void row_to_tmem16(const __half *src, int chunks, uint32_t taddr) {
     uint32_t r[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (valid) v = __ldg(reinterpret_cast<const uint4 *>(src) + i / 4);
+        if (i / 4 < chunks) v = __ldg(reinterpret_cast<const uint4 *>(src) + i / 4);
         r[i] = v.x, r[i + 1] = v.y, r[i + 2] = v.z, r[i + 3] = v.w;
     }
     tmem_st16(taddr, r);
@@ -225,6 +210,7 @@ __global__ void __launch_bounds__(kKvThreads, 1)
     constexpr int NB = D / 64, W2 = D / 2, BQ = 64, NS = kv_stages<D>();
     constexpr int KP = 128 * D * 2, QP = BQ * D * 2;  // bytes of one plane of a K tile / a query tile
     constexpr int cVh = 0, cST = 64, cDPT = 192, cDV = 256, cDK = 256 + D;
+    const bool padded = plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *sKh = smem, *sKl = smem + KP, *sVl = smem + 2 * KP;  // V's hi plane sits in TMEM
@@ -278,9 +264,9 @@ __global__ void __launch_bounds__(kKvThreads, 1)
         if (elect_one()) {
             tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap), tma_prefetch_desc(&qmap), tma_prefetch_desc(&gmap);
             mbar_arrive_expect_tx(&sh->k_full, 3 * KP);
-            tma_load_4d(sKh, &kmap, &sh->k_full, 0, s0, g * NB, b);
-            tma_load_4d(sKl, &kmap, &sh->k_full, 0, s0, g * NB, B + b);
-            tma_load_4d(sVl, &vmap, &sh->k_full, 0, s0, g * NB, B + b);
+            load_head<NB>(sKh, &kmap, &sh->k_full, s0, g, b, 128 * 128, padded);
+            load_head<NB>(sKl, &kmap, &sh->k_full, s0, g, B + b, 128 * 128, padded);
+            load_head<NB>(sVl, &vmap, &sh->k_full, s0, g, B + b, 128 * 128, padded);
             int issued = 0;
             for (int it = 0; it < n_it; ++it, walk.next()) {
                 const int s = it % NS;
@@ -291,13 +277,13 @@ __global__ void __launch_bounds__(kKvThreads, 1)
                 // two steps ahead); dO's are released by dV and wanted a step later
                 if (it >= NS && !kwait(&sh->free_q[s], free_par, sh)) { kgive_up(sh, 21); break; }
                 mbar_arrive_expect_tx(&sh->full_q[s], 2 * QP);
-                tma_load_4d(st, &qmap, &sh->full_q[s], 0, row, h * NB, b);
-                tma_load_4d(st + QP, &qmap, &sh->full_q[s], 0, row, h * NB, B + b);
+                load_head<NB>(st, &qmap, &sh->full_q[s], row, h, b, 64 * 128, padded);
+                load_head<NB>(st + QP, &qmap, &sh->full_q[s], row, h, B + b, 64 * 128, padded);
                 ++issued;
                 if (it >= NS && !kwait(&sh->free_g[s], free_par, sh)) { kgive_up(sh, 21); break; }
                 mbar_arrive_expect_tx(&sh->full_g[s], 2 * QP);
-                tma_load_4d(st + 2 * QP, &gmap, &sh->full_g[s], 0, row, h * NB, b);
-                tma_load_4d(st + 3 * QP, &gmap, &sh->full_g[s], 0, row, h * NB, B + b);
+                load_head<NB>(st + 2 * QP, &gmap, &sh->full_g[s], row, h, b, 64 * 128, padded);
+                load_head<NB>(st + 3 * QP, &gmap, &sh->full_g[s], row, h, B + b, 64 * 128, padded);
                 ++issued;
             }
             if (sh->abort) {
@@ -463,11 +449,12 @@ __global__ void __launch_bounds__(kKvThreads, 1)
         const int tid = threadIdx.x & 127, set = threadIdx.x >> 7;
         const int key = s0 + tid;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        const long long wkv = (long long)p.n_kv_heads * D;
+        const int pd = plane_dim(p.dim_out);
+        const long long wkv = (long long)p.n_kv_heads * pd;
         {
             // V's hi plane -> TMEM, 16 words of the row per set
-            const long long off = ((long long)b * p.T + (key < p.T ? key : 0)) * wkv + (long long)g * D;
-            if (set * 16 < W2) row_to_tmem16(p.v_planes + off + set * 32, key < p.T, tmem + lane_base + cVh + set * 16);
+            const long long off = ((long long)b * p.T + (key < p.T ? key : 0)) * wkv + (long long)g * pd;
+            if (set * 16 < W2) row_to_tmem16(p.v_planes + off + set * 32, key < p.T ? (pd - set * 32) / 8 : 0, tmem + lane_base + cVh + set * 16);
             tmem_wait_st();
             tc_fence_before();
             mbar_arrive_warp(&sh->a_ready);
@@ -692,6 +679,7 @@ __global__ void __launch_bounds__(kKvThreads, 1)
     constexpr int NB = D / 64, W2 = D / 2, BN = 64;
     constexpr int QP = 128 * D * 2;  // bytes of one plane of the 128-row Q / dO tile
     constexpr int KP = BN * D * 2;   // bytes of one plane of a 64-key tile
+    const bool padded = plane_dim(p.dim_out) < D;
     constexpr int cQh = 0, cGh = 64, cS = 128, cDP = 256, cDQ = 384;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -736,29 +724,29 @@ __global__ void __launch_bounds__(kKvThreads, 1)
         if (elect_one()) {
             tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap), tma_prefetch_desc(&qmap), tma_prefetch_desc(&gmap);
             mbar_arrive_expect_tx(&sh->ql_full, 2 * QP);
-            tma_load_4d(sQl, &qmap, &sh->ql_full, 0, t0, h * NB, B + b);
-            tma_load_4d(sGl, &gmap, &sh->ql_full, 0, t0, h * NB, B + b);
+            load_head<NB>(sQl, &qmap, &sh->ql_full, t0, h, B + b, 128 * 128, padded);
+            load_head<NB>(sGl, &gmap, &sh->ql_full, t0, h, B + b, 128 * 128, padded);
             // the hi planes, bound for TMEM, are staged in K's slots 1 and 2 until the row threads have moved them:
             // one bulk copy each instead of a strided read per thread
             mbar_arrive_expect_tx(&sh->qh_full, 2 * QP);
-            tma_load_4d(sK + 2 * KP, &qmap, &sh->qh_full, 0, t0, h * NB, b);
-            tma_load_4d(sK + 4 * KP, &gmap, &sh->qh_full, 0, t0, h * NB, b);
+            load_head<NB>(sK + 2 * KP, &qmap, &sh->qh_full, t0, h, b, 128 * 128, padded);
+            load_head<NB>(sK + 4 * KP, &gmap, &sh->qh_full, t0, h, b, 128 * 128, padded);
             int n_k = 0, n_v = 0;  // tiles issued
             bool live = true;
             auto load_k = [&](int j) {
                 const int ks = j % kDqKSlots;
                 if (j >= kDqKSlots && !dwait(&sh->free_k[ks], (uint32_t)(((j / kDqKSlots) & 1) ^ 1), sh)) { dgive_up(sh, 31), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_k[ks], 2 * KP);
-                tma_load_4d(sK + ks * 2 * KP, &kmap, &sh->full_k[ks], 0, j * BN, g * NB, b);
-                tma_load_4d(sK + ks * 2 * KP + KP, &kmap, &sh->full_k[ks], 0, j * BN, g * NB, B + b);
+                load_head<NB>(sK + ks * 2 * KP, &kmap, &sh->full_k[ks], j * BN, g, b, 64 * 128, padded);
+                load_head<NB>(sK + ks * 2 * KP + KP, &kmap, &sh->full_k[ks], j * BN, g, B + b, 64 * 128, padded);
                 ++n_k;
             };
             auto load_v = [&](int j) {
                 const int vs = j % kDqVSlots;
                 if (j >= kDqVSlots && !dwait(&sh->free_v[vs], (uint32_t)(((j / kDqVSlots) & 1) ^ 1), sh)) { dgive_up(sh, 31), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v[vs], 2 * KP);
-                tma_load_4d(sV + vs * 2 * KP, &vmap, &sh->full_v[vs], 0, j * BN, g * NB, b);
-                tma_load_4d(sV + vs * 2 * KP + KP, &vmap, &sh->full_v[vs], 0, j * BN, g * NB, B + b);
+                load_head<NB>(sV + vs * 2 * KP, &vmap, &sh->full_v[vs], j * BN, g, b, 64 * 128, padded);
+                load_head<NB>(sV + vs * 2 * KP + KP, &vmap, &sh->full_v[vs], j * BN, g, B + b, 64 * 128, padded);
                 ++n_v;
             };
             load_k(0), load_v(0);
@@ -1113,7 +1101,7 @@ inline int launch_bwd_tc_d(const BwdMaps &m, const BwdParams &p, cudaStream_t st
 }  // namespace tcb
 
 inline size_t tc_bwd_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
-    return tcb::bwd_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).total_bytes;
+    return tcb::bwd_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim)).total_bytes;
 }
 
 }  // namespace zt

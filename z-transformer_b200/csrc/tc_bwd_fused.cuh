@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     static_assert(D == 64 || D == 128, "tile widths of this kernel");
     constexpr int NB = D / 64, W2 = D / 2, BQ = 64;
     constexpr int KP = 128 * D * 2, QP = BQ * D * 2;  // bytes of one plane of a K tile / a query tile
+    const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cVh = 0, cST = 64, cDPT = 128, cDQT = 192, cDV = 256, cDK = 256 + D;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sKh = smem, *sKl = smem + KP, *sVl = smem + 2 * KP;  // V's hi plane sits in TMEM
@@ -141,9 +142,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (elect_one() && !sh->abort) {
             tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap), tma_prefetch_desc(&qmap), tma_prefetch_desc(&gmap);
             mbar_arrive_expect_tx(&sh->k_full, 3 * KP);
-            tma_load_4d(sKh, &kmap, &sh->k_full, 0, s0, g * NB, b);
-            tma_load_4d(sKl, &kmap, &sh->k_full, 0, s0, g * NB, B + b);
-            tma_load_4d(sVl, &vmap, &sh->k_full, 0, s0, g * NB, B + b);
+            load_head<NB>(sKh, &kmap, &sh->k_full, s0, g, b, 128 * 128, padded);
+            load_head<NB>(sKl, &kmap, &sh->k_full, s0, g, B + b, 128 * 128, padded);
+            load_head<NB>(sVl, &vmap, &sh->k_full, s0, g, B + b, 128 * 128, padded);
             int n_ql = 0, n_gl = 0;  // tiles issued
             bool live = true;
             Walk wq = walk, wg = walk;
@@ -153,8 +154,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 if (j >= 2 && !fwait(&sh->free_q[s], (uint32_t)((((j >> 1) - 1) & 1)), sh)) { fgive_up(sh, 61), live = false; return; }
                 const int h = head0 + wq.hh, row = wq.qi * BQ;
                 mbar_arrive_expect_tx(&sh->full_q[s], 2 * QP);
-                tma_load_4d(sQ + s * 2 * QP, &qmap, &sh->full_q[s], 0, row, h * NB, b);
-                tma_load_4d(sQ + s * 2 * QP + QP, &qmap, &sh->full_q[s], 0, row, h * NB, B + b);
+                load_head<NB>(sQ + s * 2 * QP, &qmap, &sh->full_q[s], row, h, b, 64 * 128, padded);
+                load_head<NB>(sQ + s * 2 * QP + QP, &qmap, &sh->full_q[s], row, h, B + b, 64 * 128, padded);
                 ++n_ql, wq.next();
             };
             auto load_g = [&]() {  // dO tile of step n_gl
@@ -163,8 +164,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 if (j >= 1 && !fwait(&sh->free_g, (uint32_t)((j - 1) & 1), sh)) { fgive_up(sh, 61), live = false; return; }
                 const int h = head0 + wg.hh, row = wg.qi * BQ;
                 mbar_arrive_expect_tx(&sh->full_g, 2 * QP);
-                tma_load_4d(sG, &gmap, &sh->full_g, 0, row, h * NB, b);
-                tma_load_4d(sG + QP, &gmap, &sh->full_g, 0, row, h * NB, B + b);
+                load_head<NB>(sG, &gmap, &sh->full_g, row, h, b, 64 * 128, padded);
+                load_head<NB>(sG + QP, &gmap, &sh->full_g, row, h, B + b, 64 * 128, padded);
                 ++n_gl, wg.next();
             };
             // the tensor core frees dO's slot (dV) before Q's (dK of the next step): ask in that order
@@ -362,11 +363,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         const int lane = threadIdx.x & 31;
         const int key = s0 + tid;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        const long long wkv = (long long)p.n_kv_heads * D;
+        const int pd = PAD ? plane_dim(p.dim_out) : D;
+        const long long wkv = (long long)p.n_kv_heads * pd;
         {
             // V's hi plane -> TMEM, 16 words of the row per set
-            const long long off = ((long long)b * p.T + (key < p.T ? key : 0)) * wkv + (long long)g * D;
-            if (set * 16 < W2) row_to_tmem16(p.v_planes + off + set * 32, key < p.T, tmem + lane_base + cVh + set * 16);
+            const long long off = ((long long)b * p.T + (key < p.T ? key : 0)) * wkv + (long long)g * pd;
+            if (set * 16 < W2) row_to_tmem16(p.v_planes + off + set * 32, key < p.T ? (pd - set * 32) / 8 : 0, tmem + lane_base + cVh + set * 16);
             tmem_wait_st();
             tc_fence_before();
             mbar_arrive_warp(&sh->a_ready);
@@ -669,12 +671,12 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
                          const float2 *rope_t = nullptr, bool qkv_planes_kept = false, const PeerList *dq_peers = nullptr,
                          bool two_kernels = false) {
     using namespace tcb;
-    const int td = tc_tile_dim(dim);  // the kernels' D; the planes' head width
+    const int td = tc_tile_dim(dim), pd = tc::plane_dim(dim);  // the kernels' D; the planes' head width
     const bool fused = tc_bwd_takes_fused(dim, two_kernels, dq_peers);
     if (fused && rope_t) return refuse("internal: the fused backward does not rotate dq.");
-    const BwdWorkspace w = bwd_workspace(workspace, batch, T, n_heads, n_kv_heads, td);
+    const BwdWorkspace w = bwd_workspace(workspace, batch, T, n_heads, n_kv_heads, pd);
     const int group = n_heads / n_kv_heads;
-    const int wq = n_heads * td, wkv = n_kv_heads * td;
+    const int blocks = td / 64;
     // With the planes of q, k, v kept by the forward (their maxima and v's largest row norm beside them), only dout is
     // converted.  The header's last array holds the largest row norm of dout for the fused kernel, max |dS| (which its
     // dQ kernel finds) for the two kernels.
@@ -684,7 +686,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
         return refuse("could not clear the backward workspace header");
     }
     PassArgs pa{};
-    pa.dim = dim, pa.td = td;
+    pa.dim = dim, pa.pd = pd;
     {
         PassTensor &t = pass_add(pa, dout, batch, T, n_heads, group, w.part[3], w.amax_do, fused ? w.dsmax : nullptr, w.do_planes);
         t.o = out, t.delta = delta, t.rnorm = w.rnorm;
@@ -697,15 +699,15 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
     if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
     BwdMaps m;
-    bool maps = make_half_tile_map(&m.k128, w.k_planes, 2 * batch, T, wkv, td, 128) &&
-                make_half_tile_map(&m.v128, w.v_planes, 2 * batch, T, wkv, td, 128) &&
-                make_half_tile_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, wq, td, 64) &&
-                make_half_tile_map(&m.g64, w.do_planes, 2 * batch, T, wq, td, 64);
+    bool maps = make_head_map(&m.k128, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
+                make_head_map(&m.v128, w.v_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
+                make_head_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, n_heads, dim, blocks, 64) &&
+                make_head_map(&m.g64, w.do_planes, 2 * batch, T, n_heads, dim, blocks, 64);
     if (!fused)
-        maps = maps && make_half_tile_map(&m.k64, w.k_planes, 2 * batch, T, wkv, td, 64) &&
-               make_half_tile_map(&m.v64, w.v_planes, 2 * batch, T, wkv, td, 64) &&
-               make_half_tile_map(&m.q128, w.q_planes, 2 * batch, T, wq, td, 128) &&
-               make_half_tile_map(&m.g128, w.do_planes, 2 * batch, T, wq, td, 128);
+        maps = maps && make_head_map(&m.k64, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 64) &&
+               make_head_map(&m.v64, w.v_planes, 2 * batch, T, n_kv_heads, dim, blocks, 64) &&
+               make_head_map(&m.q128, w.q_planes, 2 * batch, T, n_heads, dim, blocks, 128) &&
+               make_head_map(&m.g128, w.do_planes, 2 * batch, T, n_heads, dim, blocks, 128);
     if (!maps) return refuse("the TMA tensor maps for the backward could not be encoded.");
     BwdParams p{};
     p.lse = lse, p.delta = delta;

@@ -848,7 +848,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     const int group = n_heads / n_kv_heads;
     const int wq = n_heads * td, wkv = n_kv_heads * td;
     PassArgs pa{};
-    pa.dim = dim, pa.td = td;
+    pa.dim = dim, pa.pd = td;
     uint32_t *rnmax = w.dsmax;  // (the header's last array)
     {
         PassTensor &t = pass_add(pa, dout, batch, T, n_heads, group, w.part[3], w.amax_do, rnmax, w.do_planes);

@@ -102,6 +102,18 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, u
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
+// Rows of one head, NB blocks of 64 columns, block_bytes apart in shared memory.  `padded`: the planes hold fewer columns a
+// head than the tile (make_head_map), a copy takes one block, and what lies beyond the head's columns arrives as zeros.
+template <int NB>
+__device__ __forceinline__ void load_head(uint8_t *dst, const CUtensorMap *map, uint64_t *bar, int row, int head, int plane, int block_bytes,
+                                          bool padded) {
+    if (!padded) {
+        tma_load_4d(dst, map, bar, 0, row, head * NB, plane);
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < NB; ++c) tma_load_4d(dst + c * block_bytes, map, bar, c * 64, row, head, plane);
+}
 // The same tile into L2 only: nothing lands in shared memory and nothing is signalled.
 __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1),
@@ -240,6 +252,17 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, bool a_mn_major, 
 // contraction, columns where they are N.  The padding beyond is zeros that only cost time: at 80 columns on a tile of 128,
 // three steps of eight in S and dP and three eighths of N in the products that leave in head columns.
 __host__ __device__ constexpr int head_steps(int dim) { return (dim + 15) >> 4; }
+// The columns of a head in the operand planes, which hold less than a tile where that is worth it: the rest of the tile then
+// never exists in memory, and copies fill it with zeros (load_head).  A quarter of the tile saved is (heads of 96: 863 ->
+// 823 us, of 72: 812 -> 770 at batch 4, T 2048, 16/4 heads, forward and backward; of 80, batch 4, T 1000: 319 -> 297; 4/2
+// heads of 32, T 256: 53 -> 47.5); an eighth is not (112: no change), nor are rows of 48 columns, 96 bytes that straddle
+// lines (0.9 % slower than rows of 64), nor tiles above 128 columns, where the copies that a narrow tile takes (one a block of
+// 64 columns) cost more than the bytes (136 on 192: 490 -> 510).
+__host__ __device__ constexpr int plane_dim(int dim) {
+    if (dim <= 64) return dim <= 32 ? 32 : 64;
+    if (dim <= 128) return dim <= 96 ? 16 * head_steps(dim) : 128;
+    return dim <= 192 ? 192 : 256;
+}
 // The variant of a kernel template that two flags choose.  (Kernels whose MMA-issuing threads are on the critical path have
 // the padded form as a variant of its own: the check of every step cost heads that fill their tile 0.9 %.)
 template <class F>
@@ -308,12 +331,12 @@ __device__ __forceinline__ float tf32_round(float x) {
 }  // namespace tc
 
 // ---- host: which shapes the tensor-core kernels take ------------------------------------------------
-// They have tiles of 64, 128, 192 and 256 columns; a head of any other width runs on the next wider tile.  The operand
-// planes carry every head zero-padded to the tile's width, outputs keep their own (rows leave in 16-byte chunks,
-// hence the multiple of four).  The padding costs at most half of the tensor work (head_dim 68 on 128 columns;
-// below 64 an MMA of half the width or depth costs the same clocks anyway), and what it replaces is the CUDA-core
+// They have tiles of 64, 128, 192 and 256 columns; a head of any other width runs on the next wider tile, zeros beyond its
+// columns (tc::plane_dim), outputs keep their own width (rows leave in 16-byte chunks, hence the multiple of four).  What
+// the MMAs of the padding cost is bounded (tc::head_steps; an MMA of half the width costs the same clocks anyway), and what
+// it replaces is the CUDA-core
 // kernels at a thirtieth of the rate: head_dim 80, batch 4, T 1000, 16/4 heads, forward and backward 7.6 ms there,
-// 0.45 ms here.  192 columns lie between because 132 ... 192 padded to 256 paid a third more MMAs, plane bytes and
+// 0.30 ms here.  192 columns lie between because 132 ... 192 padded to 256 paid a third more MMAs, plane bytes and
 // operand traffic for nothing: us on 256 -> on 192 columns, 16/4 heads of 192, forward and backward of batch 4, T 1024
 // 611 -> 526, forward of batch 4, T 2048 562 -> 486, a window of 512 rows at 3584 165 -> 128; 8/2 heads of 160,
 // batch 2, T 4096 1633 -> 1443.
@@ -375,6 +398,23 @@ inline bool make_half_tile_map(CUtensorMap *map, const void *base, int planes, l
     const cuuint64_t dims[4] = {64, (cuuint64_t)rows, (cuuint64_t)(width / 64), (cuuint64_t)planes};
     const cuuint64_t strides[3] = {(cuuint64_t)width * 2, 128, (cuuint64_t)rows * width * 2};
     const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, (cuuint32_t)(dim / 64), 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Tensor map over operand planes [planes, rows, heads, plane_dim(dim)] for tiles of `box_rows` rows and `blocks` blocks of
+// 64 columns.  Where a head fills its tile that is make_half_tile_map; elsewhere the innermost dimension ends with the head,
+// so that a box that reaches beyond it is filled with zeros, and a box is one block (tc::load_head).
+inline bool make_head_map(CUtensorMap *map, const void *base, int planes, long long rows, int heads, int dim, int blocks, int box_rows) {
+    const int td = tc_tile_dim(dim), pd = tc::plane_dim(dim);
+    if (pd == td) return make_half_tile_map(map, base, planes, rows, heads * td, blocks * 64, box_rows);
+    PFN_encodeTiled enc = get_encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)pd, (cuuint64_t)rows, (cuuint64_t)heads, (cuuint64_t)planes};
+    const cuuint64_t strides[3] = {(cuuint64_t)heads * pd * 2, (cuuint64_t)pd * 2, (cuuint64_t)rows * heads * pd * 2};
+    const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -29,7 +29,6 @@ namespace tcf16 {
 
 using namespace tc;
 using tcb::block_mult;
-using tcb::row_to_tmem;
 using tcb::split_pack;
 
 constexpr int kThreads = 320;  // 8 softmax warps (two sets of four), 1 TMA warp, 1 MMA warp
@@ -142,9 +141,8 @@ __device__ __forceinline__ float4 flush_sum4(const float *at, float f, bool firs
 // when the row is not the tensor's.
 struct FlushRow {
     float *lower, *upper;
-    int width;
-    template <int D>
-    __device__ __forceinline__ float *at(int c) const { return c < D / 2 ? lower + c : upper + (c - D / 2); }
+    int width, half;  // columns from `half` on are at upper
+    __device__ __forceinline__ float *at(int c) const { return c < half ? lower + c : upper + (c - half); }
 };
 // O's columns [0, D) of this thread's row, at TMEM `taddr`, into its running sum.
 template <int D>
@@ -158,7 +156,7 @@ __device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, f
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
             if (c + i >= row.width) break;
-            float *at = row.at<D>(c + i);
+            float *at = row.at(c + i);
             *reinterpret_cast<float4 *>(at) = flush_sum4(at, f, first, make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])));
         }
     }
@@ -170,6 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                   const __grid_constant__ CUtensorMap qmap, const Params p) {
     constexpr int NB = D / 64, W2 = D / 2, BN = 64;
     constexpr int KP = BN * D * 2;  // bytes of one plane of a key tile
+    const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cQh = 0, cQl = W2, cO0 = D, cS0 = 3 * D;  // O of set s at cO0 + s D, S/P of buffer i at cS0 + 64 i
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -230,8 +229,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             // the query tile's two planes, staged in V's first two slots until the row threads have moved
             // them into TMEM: one bulk copy each instead of a strided read per thread
             mbar_arrive_expect_tx(&sh->q_full, 4 * KP);
-            tma_load_4d(sV, &qmap, &sh->q_full, 0, t0, h * NB, b);
-            tma_load_4d(sV + 2 * KP, &qmap, &sh->q_full, 0, t0, h * NB, B + b);
+            load_head<NB>(sV, &qmap, &sh->q_full, t0, h, b, 128 * 128, padded);
+            load_head<NB>(sV + 2 * KP, &qmap, &sh->q_full, t0, h, B + b, 128 * 128, padded);
             int n_k = 0, n_v = 0;  // tiles issued
             bool live = true;
             const auto prefetch_next_q = [&]() {
@@ -243,23 +242,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (p.ahead <= 0 || lin >= gx * gy * gridDim.z) return;
                 const int nx = (int)(lin % gx), ny = (int)((lin / gx) % gy), nz = (int)(lin / (gx * gy));
                 const int nt0 = ((int)gx - 1 - nx) * 128;
-                tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, nz);
-                tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, B + nz);
+                if (!padded) {
+                    tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, nz);
+                    tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, B + nz);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NB; ++c) {
+                        tma_prefetch_l2_4d(&qmap, c * 64, nt0, ny, nz);
+                        tma_prefetch_l2_4d(&qmap, c * 64, nt0, ny, B + nz);
+                    }
+                }
             };
             auto load_k = [&](int j) {
                 const int s = j % 3;
                 if (j >= 3 && !fwait(&sh->free_k[s], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { fgive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_k[s], 2 * KP);
-                tma_load_4d(sK + s * 2 * KP, &kmap, &sh->full_k[s], 0, (jb + j) * BN, g * NB, b);
-                tma_load_4d(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], 0, (jb + j) * BN, g * NB, B + b);
+                load_head<NB>(sK + s * 2 * KP, &kmap, &sh->full_k[s], (jb + j) * BN, g, b, BN * 128, padded);
+                load_head<NB>(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], (jb + j) * BN, g, B + b, BN * 128, padded);
                 ++n_k;
             };
             auto load_v = [&](int j) {
                 const int s = j % 3;
                 if (j >= 3 && !fwait(&sh->free_v[s], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { fgive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v[s], 2 * KP);
-                tma_load_4d(sV + s * 2 * KP, &vmap, &sh->full_v[s], 0, (jb + j) * BN, g * NB, b);
-                tma_load_4d(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], 0, (jb + j) * BN, g * NB, B + b);
+                load_head<NB>(sV + s * 2 * KP, &vmap, &sh->full_v[s], (jb + j) * BN, g, b, BN * 128, padded);
+                load_head<NB>(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], (jb + j) * BN, g, B + b, BN * 128, padded);
                 ++n_v;
             };
             const int first = n_tiles < 3 ? n_tiles : 3;
@@ -372,17 +379,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         // where the sets keep flushed sums: set 0 in out, set 1 in the two planes of the query row, which this CTA alone
         // reads and has in TMEM by now (a forward that flushes keeps no planes for a backward)
-        FlushRow row0{nullptr, nullptr, p.dim_out}, row1{nullptr, nullptr, D};
+        const int pd = PAD ? plane_dim(p.dim_out) : D;  // a head in the planes
+        FlushRow row0{nullptr, nullptr, p.dim_out, pd / 2}, row1{nullptr, nullptr, p.dim_out, pd / 2};
         if (FLUSH && t < p.T) {
             row0.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
-            row0.upper = row0.lower + D / 2;
+            row0.upper = row0.lower + pd / 2;
             if (p.parts > 1) {  // (whose parts share the query rows: behind the parts' rows)
-                row1.lower = row0.lower + p.parts * p.out_part, row1.upper = row1.lower + D / 2;
-                row1.width = p.dim_out;
+                row1.lower = row0.lower + p.parts * p.out_part, row1.upper = row1.lower + pd / 2;
             } else {
-                __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * D + (long long)h * D;
+                __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * pd + (long long)h * pd;
                 row1.lower = reinterpret_cast<float *>(planes);
-                row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * D);
+                row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * pd);
             }
         }
         for (int j = set; ok && j < n_tiles; j += 2) {
@@ -492,11 +499,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int i = 0; i < 32; i += 4) {
                     const int col = set * (D / 2) + c + i;
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add0 && col < row0.width) o4 = flush_sum4(row0.at<D>(col), g0, false, o4);
+                    if (add0 && col < row0.width) o4 = flush_sum4(row0.at(col), g0, false, o4);
                     o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
                         float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
-                        if (add1 && col < row1.width) x4 = flush_sum4(row1.at<D>(col), g1, false, x4);
+                        if (add1 && col < row1.width) x4 = flush_sum4(row1.at(col), g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     const int ch = (set * (D / 2) + c + i) >> 2;
@@ -578,7 +585,7 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
 }  // namespace tcf16
 
 inline size_t tc_fwd16_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset = 0) {
-    return tcf16::workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim), q_offset).total_bytes;
+    return tcf16::workspace(nullptr, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim), q_offset).total_bytes;
 }
 
 inline bool tc_fwd16_supported(int batch, int T, int q_offset, int dim, const void *q, const void *k, const void *v, const void *out) {
@@ -599,28 +606,27 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
                            const float2 *rope = nullptr, bool in_backward_workspace = false, int variant = 0,
                            __half *out_planes = nullptr, const PeerList *out_peers = nullptr, int q_offset = 0) {
     using namespace tcb;
-    const int td = tc_tile_dim(dim);  // the kernel's D; the planes' head width
-    tcf16::Workspace w = tcf16::workspace(ws, batch, T, n_heads, n_kv_heads, td, q_offset);
+    const int td = tc_tile_dim(dim), pd = tc::plane_dim(dim);  // the kernel's D; the planes' head width
+    tcf16::Workspace w = tcf16::workspace(ws, batch, T, n_heads, n_kv_heads, pd, q_offset);
     if (in_backward_workspace) {
-        const BwdWorkspace bw = bwd_workspace(ws, batch, T, n_heads, n_kv_heads, td);
+        const BwdWorkspace bw = bwd_workspace(ws, batch, T, n_heads, n_kv_heads, pd);
         w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;
         w.vnmax = bw.vnmax;
         for (int i = 0; i < 3; ++i) w.part[i] = bw.part[i];
         w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes, w.parts = bw.parts;
     }
     const int group = n_heads / n_kv_heads;
-    const int wkv = n_kv_heads * td;
     const int n_seen = q_offset + T;  // key rows that some query row sees
     PassArgs pa{};
-    pa.dim = dim, pa.td = td;
+    pa.dim = dim, pa.pd = pd;
     pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
     pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
     pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     if (launch_pass(pa, stream)) return 1;
     CUtensorMap kmap, vmap, qmap;  // (the widest tile fetches K block by block, see attn_fwd_tc16x)
-    if (!make_half_tile_map(&kmap, w.k_planes, 2 * batch, n_seen, wkv, td > 128 ? 64 : td, 64) ||
-        !make_half_tile_map(&vmap, w.v_planes, 2 * batch, n_seen, wkv, td, 64) ||
-        !make_half_tile_map(&qmap, w.q_planes, 2 * batch, T, n_heads * td, td, 128))
+    if (!make_head_map(&kmap, w.k_planes, 2 * batch, n_seen, n_kv_heads, dim, td > 128 ? 1 : td / 64, 64) ||
+        !make_head_map(&vmap, w.v_planes, 2 * batch, n_seen, n_kv_heads, dim, td / 64, 64) ||
+        !make_head_map(&qmap, w.q_planes, 2 * batch, T, n_heads, dim, td / 64, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
     const int sms = split_sm_count();
     tcf16::Params p{};

@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                    const __grid_constant__ CUtensorMap qmap, const Params p) {
     constexpr int NB = D / 64, W2 = D / 2, BN = 64;
     constexpr int KP = BN * D * 2;  // bytes of one plane of a key tile; a ring slot is 2 KP (hi, lo)
+    const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cQh = 0, cO0 = D, cS0 = 3 * D;  // head s: Qh at cQh + s W2, O at cO0 + s D, S/P at cS0 + 64 s
     extern __shared__ __align__(1024) uint8_t smem_raw[];  // (the swizzled tiles need the alignment; checked below)
     uint8_t *sK = smem_raw, *sV = sK + 6 * KP, *sQl = sV + 4 * KP;  // sQl: Q lo of head A, of head B (2 KP each)
@@ -90,27 +91,27 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_prefetch_desc(&qmap), tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap);
             // the Q hi planes wait in V's two slots until the row threads have moved them into TMEM
             mbar_arrive_expect_tx(&sh->q_full, 4 * KP);
-            tma_load_4d(sV, &qmap, &sh->q_full, 0, t0, h0 * NB, b);
-            tma_load_4d(sV + 2 * KP, &qmap, &sh->q_full, 0, t0, (h0 + 1) * NB, b);
+            load_head<NB>(sV, &qmap, &sh->q_full, t0, h0, b, 128 * 128, padded);
+            load_head<NB>(sV + 2 * KP, &qmap, &sh->q_full, t0, h0 + 1, b, 128 * 128, padded);
             mbar_arrive_expect_tx(&sh->ql_full, 4 * KP);
-            tma_load_4d(sQl, &qmap, &sh->ql_full, 0, t0, h0 * NB, B + b);
-            tma_load_4d(sQl + 2 * KP, &qmap, &sh->ql_full, 0, t0, (h0 + 1) * NB, B + b);
+            load_head<NB>(sQl, &qmap, &sh->ql_full, t0, h0, B + b, 128 * 128, padded);
+            load_head<NB>(sQl + 2 * KP, &qmap, &sh->ql_full, t0, h0 + 1, B + b, 128 * 128, padded);
             int n_k = 0, n_v = 0;  // tiles issued
             bool live = true;
             auto load_k = [&](int j) {
                 const int s = j % 3;
                 if (j >= 3 && !gwait(&sh->free_k[s], (uint32_t)(((j / 3) & 1) ^ 1), sh)) { ggive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_k[s], 2 * KP);
-                tma_load_4d(sK + s * 2 * KP, &kmap, &sh->full_k[s], 0, j * BN, g * NB, b);
-                tma_load_4d(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], 0, j * BN, g * NB, B + b);
+                load_head<NB>(sK + s * 2 * KP, &kmap, &sh->full_k[s], j * BN, g, b, BN * 128, padded);
+                load_head<NB>(sK + s * 2 * KP + KP, &kmap, &sh->full_k[s], j * BN, g, B + b, BN * 128, padded);
                 ++n_k;
             };
             auto load_v = [&](int j) {
                 const int s = j & 1;
                 if (j >= 2 && !gwait(&sh->free_v[s], (uint32_t)(((j >> 1) & 1) ^ 1), sh)) { ggive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v[s], 2 * KP);
-                tma_load_4d(sV + s * 2 * KP, &vmap, &sh->full_v[s], 0, j * BN, g * NB, b);
-                tma_load_4d(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], 0, j * BN, g * NB, B + b);
+                load_head<NB>(sV + s * 2 * KP, &vmap, &sh->full_v[s], j * BN, g, b, BN * 128, padded);
+                load_head<NB>(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], j * BN, g, B + b, BN * 128, padded);
                 ++n_v;
             };
             for (int j = 0; j < 3 && j < n_tiles; ++j) load_k(j);
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        FlushRow row{nullptr, nullptr, p.dim_out};
+        FlushRow row{nullptr, nullptr, p.dim_out, D / 2};
         if (FLUSH && t < p.T) {
             row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row.upper = row.lower + D / 2;
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add && c + i < row.width) o4 = flush_sum4(row.at<D>(c + i), ff, false, o4);
+                    if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     const int ch = (c + i) >> 2;
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;

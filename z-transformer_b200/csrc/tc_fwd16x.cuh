@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         const float cs = p.scale_log2 / (mq * mk);
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        FlushRow row{nullptr, nullptr, p.dim_out};
+        FlushRow row{nullptr, nullptr, p.dim_out, D / 2};
         if (FLUSH && t < p.T) {
             row.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
             row.upper = row.lower + D / 2;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add && c + i < row.width) o4 = flush_sum4(row.at<D>(c + i), ff, false, o4);
+                    if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     const int ch = (c + i) >> 2;
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & 15)) << 4)) = o4;

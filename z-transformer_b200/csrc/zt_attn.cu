@@ -800,7 +800,7 @@ int check_proj(const void *workspace, size_t workspace_bytes, int batch, int T, 
 #ifndef ZT_NO_TC
 // The planes of x [batch][rows][width] with one scale per batch item: 64 columns count as a head of the pre-pass.
 void add_proj_planes(tcb::PassArgs &a, const float *x, int batch, int rows, int width, uint2 *part, uint32_t *amax, __half *planes) {
-    a.dim = 64, a.td = 64;
+    a.dim = 64, a.pd = 64;
     tcb::pass_add(a, x, batch, rows, width / 64, width / 64, part, amax, nullptr, planes);
 }
 #endif
@@ -880,7 +880,7 @@ int zt_attn_block_forward(const float *q, const float *k, const float *v, const 
     const uint32_t *from = nullptr;
     if (planes_written) {
         const RopeWorkspace rw = rope_workspace(rope_ws, batch, T, n_heads, n_kv_heads, dim);
-        from = tcb::bwd_workspace(rw.inner, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).amax_v;
+        from = tcb::bwd_workspace(rw.inner, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim)).amax_v;
     }
     return proj_forward_impl(ctx, wo, y, proj_workspace_, batch, T, kdim, d_model, s, from, n_kv_heads);
 #else
