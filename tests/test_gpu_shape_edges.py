@@ -26,6 +26,8 @@ def normal(oracle, shape, stream):
     (1, 1000, 4, 2, 64), (1, 700, 3, 3, 40), (2, 300, 8, 1, 128), (1, 1100, 2, 1, 72),
     # the 192-column tile: its narrowest and widest heads, several key tiles a block, more than one piece of a contraction
     (1, 385, 3, 3, 132), (2, 300, 4, 2, 192), (1, 1290, 2, 1, 188),
+    # more than one block an SM: the blocks go tile by tile through the sequences (and with odd ones among them)
+    (20, 130, 8, 4, 64), (30, 140, 3, 3, 128), (11, 260, 9, 3, 160), (40, 150, 4, 2, 96),
     # planes narrower than the tile, on either side of where they become so
     (1, 300, 4, 2, 32), (2, 200, 2, 1, 72), (1, 200, 2, 2, 96), (1, 200, 4, 2, 100),
 ])

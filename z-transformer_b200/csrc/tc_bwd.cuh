@@ -69,6 +69,7 @@ struct BwdParams {
     int dim_out;     // the tensors' head_dim, at most the tile's D
     const float2 *rope_t;  // null, or the (cos, sin) table transposed, [dim_out / 2][T]: dq leaves as R^T of what was computed
     float scale, scale_log2;
+    bool by_tile;       // (fused) blocks go through the sequences tile by tile, see tile_by_tile
     BwdParts parts;     // how the walk of a key tile is split; more than one part: dk, dv are the first part's,
     long long dkv_part; // and this many elements lie between two parts'
     float p_scale;  // P is multiplied by this power of two before its 16-bit split

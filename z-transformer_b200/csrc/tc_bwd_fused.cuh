@@ -61,7 +61,8 @@ __host__ __device__ constexpr size_t fused_smem_bytes() {
 
 // grid (n_kv_heads, ceil(T / 128), batch), 608 threads: 16 row warps, a TMA warp, two MMA warps.
 constexpr int kFusedThreads = (kKvRowWarps + 3) * 32;
-// PARTS: the walk is split (tc_split.cuh).  A variant of its own: the whole walk is 1 % slower with the code in it.
+// PARTS: the walk is split, or the blocks go tile by tile (tc_split.cuh).  A variant of its own: large launches are 1-2 % slower
+// with the code in it.
 template <int D, bool PARTS, bool PAD>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     attn_bwd_fused_tc(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
@@ -81,8 +82,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     FusedShared *sh = reinterpret_cast<FusedShared *>(sG + 2 * QP);
 
     const int warp = threadIdx.x >> 5;
-    const int g = blockIdx.x, kt = (int)blockIdx.y, b = PARTS ? (int)blockIdx.z / p.parts.n() : (int)blockIdx.z;
-    const int part = PARTS ? (int)blockIdx.z - b * p.parts.n() : 0;
+    // (the slowest index is the sequence, or the tile: see tile_by_tile)
+    const int g = blockIdx.x, kt = PARTS && p.by_tile ? (int)blockIdx.z : (int)blockIdx.y, bp = PARTS && p.by_tile ? (int)blockIdx.y : (int)blockIdx.z;
+    const int b = PARTS ? bp / p.parts.n() : bp, part = PARTS ? bp - b * p.parts.n() : 0;
     const int group = p.n_heads / p.n_kv_heads;
     const int s0 = kt * 128;
     // this CTA's part of the walk: heads [head0, head0 + n_heads_mine) and query tiles [qi0, n_q)
@@ -412,7 +414,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             const uint32_t acc = tmem + lane_base + (set < 2 ? cDV : cDK) + c0;
             const int j8 = lane & 7;
             const long long wo = (long long)p.n_kv_heads * p.dim_out;
-            const int mine = PARTS ? (int)blockIdx.z - b * p.parts.n() : 0;  // (`part`, without a register held for it)
+            const int mine = PARTS ? (int)(p.by_tile ? blockIdx.y : blockIdx.z) - b * p.parts.n() : 0;  // (`part`, without a register held for it)
             float *dst = (set < 2 ? p.dv : p.dk) + (PARTS ? mine * p.dkv_part : 0) + ((long long)b * p.T + (key - j8)) * wo + (long long)g * p.dim_out + c0 + 4 * j8;
             const float f = set < 2 ? 1.0f / (p.p_scale * mdo) : p.scale / (mq * cmin);
 #pragma unroll 1
@@ -641,9 +643,10 @@ inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, 
                               const BwdParams &p, cudaStream_t stream) {
     size_t smem = fused_smem_bytes<D>();
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused_tc<D, parts.value, pad.value>; }, p.parts.n() > 1, head_steps(p.dim_out) < D / 16);
+    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused_tc<D, parts.value, pad.value>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.T + 127) / 128), (unsigned)(p.batch * p.parts.n()));
+    const unsigned tiles = (unsigned)((p.T + 127) / 128), seqs = (unsigned)(p.batch * p.parts.n()), kv = (unsigned)p.n_kv_heads;
+    const dim3 grid = p.by_tile ? dim3(kv, seqs, tiles) : dim3(kv, tiles, seqs);
     return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
 }
 inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
@@ -726,6 +729,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     g_last_path = "tcgen05";
     if (fused) {
         p.parts = bwd_parts(batch, T, n_heads, n_kv_heads);
+        p.by_tile = tile_by_tile((long long)n_kv_heads * ((T + 127) / 128) * batch * p.parts.n(), kBwdTileWaves);
         if (p.parts.n() == 1) return tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream);
         const long long n = (long long)batch * T * n_kv_heads * dim;
         p.dk = w.parts, p.dv = w.parts + n, p.dkv_part = 2 * n;

@@ -52,6 +52,7 @@ struct Params {
     int q_offset;  // query row r stands at position q_offset + r of the keys: it sees keys 0 .. q_offset + r
     int parts;     // CTAs along a query tile's keys; with more than one, out and lse are the parts' (see tc_split.cuh):
     long long out_part, lse_part;  // elements from one part's to the next
+    bool by_tile;  // (one head a block) blocks go through the sequences tile by tile, see tile_by_tile
     bool flush;    // O leaves the tensor core's accumulator every kFlushKeyTiles key tiles (see flush_row)
     int dim_out;  // the tensors' head_dim, at most the tile's D
     int ahead;    // attn_fwd_tc16 prefetches the query tile of the block this many places on in launch order; 0: none
@@ -178,8 +179,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int warp = threadIdx.x >> 5;
     // launch order (x fastest): a head's query tiles, late (long) ones first.  (Starting the heads of a sequence
     // tile by tile instead, which would shorten the tail, measured 3 % slower.)
-    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;
-    const int h = blockIdx.y, b = (int)blockIdx.z / p.parts, part = (int)blockIdx.z - b * p.parts;
+    // Small launches have every head of every sequence along x instead, tile by tile (see tile_by_tile).
+    const int bx = p.by_tile ? (int)blockIdx.x / p.n_heads : 0;
+    const int qt = p.by_tile ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)gridDim.x - 1 - (int)blockIdx.x;
+    const int h = p.by_tile ? (int)blockIdx.x - bx * p.n_heads : (int)blockIdx.y, bp = (int)blockIdx.z + bx;
+    const int b = bp / p.parts, part = bp - b * p.parts;
     const int g = h / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
@@ -569,7 +573,8 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     const auto kernel = with_flags([](auto flush, auto pad) { return attn_fwd_tc16<D, flush.value, pad.value>; }, p.flush, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
+    const dim3 grid = p.by_tile ? tile_major_grid(p.n_heads, (p.T + 127) / 128, p.batch * p.parts, kFwdTileWaves)
+                                : dim3((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
     return launch_after("attn_fwd_tc16", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 
@@ -636,7 +641,6 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
     p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
     if (out_peers) p.out_peers = *out_peers;
-    p.ahead = sms;  // one CTA per SM
     p.scale_log2 = kLog2e / sqrtf((float)dim);
     p.parts = variant == 0 && !out_planes && p.out_peers.n == 0 ? fwd_parts(batch, T, n_heads, q_offset) : 1;
     const long long rows = (long long)batch * T * n_heads;
@@ -644,6 +648,8 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
         p.out = w.parts, p.out_part = rows * dim;
         p.lse = w.parts + p.parts * (q_offset > 0 ? 2 : 1) * p.out_part, p.lse_part = rows;
     }
+    p.by_tile = tile_by_tile((long long)((T + 127) / 128) * n_heads * batch * p.parts, kFwdTileWaves);
+    p.ahead = p.by_tile ? 0 : sms;  // one CTA per SM
     g_last_path = "tcgen05";
     // variant 0: two heads of a KV group per CTA (attn_fwd_tc16g) when the group has an even number of query heads
     // and that still gives every SM a CTA (half as many CTAs), one head per CTA (attn_fwd_tc16) otherwise; 1: one head

@@ -53,7 +53,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     // launch order (x fastest): the head pairs of a sequence, query tile by query tile, late (long) tiles first, so
     // that the last CTAs to start are the shortest (1.5 % faster than a head pair's tiles together)
     const int qt = (int)gridDim.y - 1 - (int)blockIdx.y;
-    const int h0 = 2 * (int)blockIdx.x, b = blockIdx.z;
+    // (the sequences are along z, or along x behind each other: see tile_by_tile)
+    const int pairs = p.n_heads / 2, bx = (int)blockIdx.x / pairs, h0 = 2 * ((int)blockIdx.x - bx * pairs), b = (int)blockIdx.z + bx;
     const int g = h0 / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
@@ -359,7 +360,7 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
     if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
     const auto kernel = with_flags([](auto flush, auto pad) { return attn_fwd_tc16g<D, flush.value, pad.value>; }, p.flush, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)(p.n_heads / 2), (unsigned)((p.T + 127) / 128), (unsigned)p.batch);
+    const dim3 grid = tile_major_grid(p.n_heads / 2, (p.T + 127) / 128, p.batch, kFwdTileWaves);
     return launch_after("attn_fwd_tc16g", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
 }
 

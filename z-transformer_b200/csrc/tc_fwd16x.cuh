@@ -65,8 +65,11 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 
     const int warp = threadIdx.x >> 5;
     // launch order (x fastest): a head's query tiles, late (long) ones first
-    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;
-    const int h = blockIdx.y, b = (int)blockIdx.z / p.parts, part = (int)blockIdx.z - b * p.parts;
+    // Small launches have every head of every sequence along x instead, tile by tile (see tile_by_tile).
+    const int bx = p.by_tile ? (int)blockIdx.x / p.n_heads : 0;
+    const int qt = p.by_tile ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)gridDim.x - 1 - (int)blockIdx.x;
+    const int h = p.by_tile ? (int)blockIdx.x - bx * p.n_heads : (int)blockIdx.y, bp = (int)blockIdx.z + bx;
+    const int b = bp / p.parts, part = bp - b * p.parts;
     const int g = h / (p.n_heads / p.n_kv_heads);
     const int t0 = qt * 128;
     const int rows_end = (t0 + 128 < p.T) ? t0 + 128 : p.T;
@@ -373,7 +376,8 @@ inline int launch_x_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
     const size_t smem = 3 * (size_t)(2 * 64 * D * 2) + sizeof(SharedX);  // K tile, V tile, Q lo
     const auto kernel = p.flush ? attn_fwd_tc16x<D, true> : attn_fwd_tc16x<D, false>;
     if (optin_smem((const void *)kernel, smem)) return 1;
-    const dim3 grid((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
+    const dim3 grid = p.by_tile ? tile_major_grid(p.n_heads, (p.T + 127) / 128, p.batch * p.parts, kFwdTileWaves)
+                                : dim3((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
     return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
 }
 

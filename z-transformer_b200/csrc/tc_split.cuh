@@ -19,6 +19,30 @@ inline int split_sm_count() {
     return d && d->sm_count > 0 ? d->sm_count : 148;  // (no device: a size query; a B200's count stands in)
 }
 
+// The order in which the blocks of a launch start (x fastest, then y, then z), where their walks differ in length.  Sequence by
+// sequence, blocks that run together share a sequence's operands in L2, which is worth 10 % of the backward at batch 8, T 4096;
+// but the last sequence's longest walks then start when the launch is nearly over, and with few blocks an SM that is what
+// the launch waits for: at batch 8, T 512, 32/8 heads of 64 the busiest SM of the backward had 1.6 times the average's work.
+// So launches of a few blocks an SM go tile by tile through all sequences, longest walks first: up to four in the backward, two
+// in the forward.  Us, by sequence -> by tile (blocks):
+//   backward  batch 8, T 512, 32/8 heads of 64 174 -> 139 (256), of 128 235 -> 194 (256); batch 4, T 1000, 16/4 heads of 80
+//             178 -> 127 (256, walks split); batch 8, T 768, of 128 393 -> 366 (384), T 1024 620 -> 602 (512), T 1536 no
+//             difference (768), T 2048 4 % slower (1024)
+//   forward   two heads a block: batch 4, T 1024, 16/4 heads of 128 72 -> 59 (256); batch 8, T 512, 32/8, with its
+//             pre-pass 149 -> 158 (512).  One head a block: batch 16, T 512, 12/4 heads 93 -> 103 (768).  Wide heads: batch
+//             2, T 1024, 16/4 heads of 256 102 -> 76 (256)
+// (One wave starts together, in whatever order.)
+constexpr int kFwdTileWaves = 2, kBwdTileWaves = 4;
+inline bool tile_by_tile(long long blocks, int waves) {
+    return blocks > split_sm_count() && blocks <= (long long)waves * split_sm_count();
+}
+// The grid for `across` blocks (heads, head pairs, KV heads) of each of `tiles` tiles of each of `seqs` sequences (times the
+// parts that a walk is split into): the sequences along z, or behind each other along x.
+inline dim3 tile_major_grid(int across, int tiles, int seqs, int waves) {
+    return tile_by_tile((long long)across * tiles * seqs, waves) ? dim3((unsigned)(across * seqs), (unsigned)tiles)
+                                                                 : dim3((unsigned)across, (unsigned)tiles, (unsigned)seqs);
+}
+
 // Parts of the forward along the keys.  A part should keep four key tiles of 64: fewer cost more in the part's own
 // prologue and in putting the rows together than they save.
 inline int fwd_parts(int batch, int T, int n_heads, int q_offset) {
