@@ -127,3 +127,24 @@ def test_projection_on_wide_tiles(zt, oracle, B, T, k, n):
     for got, ref in pairs + [(tdwo, ref_dwo)]:
         err = np.abs(got.cpu().numpy().astype(np.float64) - ref)
         assert float(np.where(np.isnan(err), np.inf, err).max()) <= 1e-4 * float(np.abs(ref).max())
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D", [(2, 70, 4, 2, 32), (1, 150, 4, 2, 96), (1, 140, 3, 3, 128), (1, 200, 2, 1, 160), (1, 90, 2, 2, 256)])
+def test_backward_takes_an_output_on_a_four_byte_boundary(zt, B, T, H, Hkv, D):
+    """Of out only the row sums with dout are wanted, so it need not start where the tensor copies of q, k, v and dout
+    do: an out at an odd offset of a larger buffer gives what the same values give in a buffer of their own (delta is the
+    same sum; dq, and above 128 columns dk and dv, are added in memory in no fixed order)."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v, do = (torch.randn((B, T, w * D), generator=gen, device="cuda") for w in (H, Hkv, Hkv, H))
+    ws = zt.BackwardWorkspace(B, T, H, Hkv, D)
+    out, lse = zt.attention_forward(q, k, v, H, Hkv, D, want_lse=True)
+    want = zt.attention_backward(q, k, v, out, lse, do, H, Hkv, D, workspace=ws)
+    for odd in (1, 2, 3):
+        moved = torch.empty(out.numel() + 4, device="cuda")[odd:odd + out.numel()].view(out.shape).copy_(out)
+        assert moved.data_ptr() % 16 == 4 * odd
+        got = zt.attention_backward(q, k, v, moved, lse, do, H, Hkv, D, workspace=ws)
+        torch.cuda.synchronize()
+        assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0
+        for name, a, b in zip(("dq", "dk", "dv"), got, want):
+            # two orders of at most ten f32 additions
+            assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max()), name

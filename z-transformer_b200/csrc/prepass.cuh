@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows_out = t.delta != nullptr, norms = rows_out || t.nmax != nullptr;
+    // (of a call's tensors `o` alone is not asked to start on a 16-byte boundary: nothing but its row sums is wanted)
+    const bool o_aligned = (reinterpret_cast<uintptr_t>(t.o) & 15u) == 0;
     const int n4 = a.dim >> 2, group = t.group, heads = t.heads;
     const long long first = (long long)w.b * t.rows * heads + w.g * group;  // the (sequence, group)'s first unit
     const float4 *xb = reinterpret_cast<const float4 *>(t.x) + first * n4 + li;
@@ -162,7 +164,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
                 const long long off = in ? (long long)at * n4 + LP * c : 0;
                 const uint32_t dst = slot0 + (uint32_t)((((step % S) * U + k) * NC + c) * 2 * kPassThreads * 16);
                 copy16_async(dst, xb + off, in);
-                if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
+                if (rows_out && o_aligned) copy16_async(dst + kPassThreads * 16, ob + off, in);
+                else if (rows_out) copy16_async_by4(dst + kPassThreads * 16, ob + off, in);
             }
         }
         copy_async_commit();

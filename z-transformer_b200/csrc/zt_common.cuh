@@ -242,6 +242,13 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool
     const int bytes = in ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+// The same from a source on a 4-byte boundary only.
+__device__ __forceinline__ void copy16_async_by4(uint32_t dst, const void *src, bool in) {
+    const int bytes = in ? 4 : 0;
+#pragma unroll
+    for (int i = 0; i < 16; i += 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + i), "l"(static_cast<const char *>(src) + i), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING>  // all but the PENDING latest groups of this thread have landed
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
