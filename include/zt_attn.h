@@ -100,7 +100,7 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
  *  - zt_attn_reserve sizes it for a shape up front -- the place for it is where the reference's
  *    holder sizes its own eleven buffers (device.Attn.init, src/cuda/device.zig:221-299; that
  *    function already calls zt_attn_dim_ok).  After zt_attn_reserve(batch, T, ...) no call of
- *    that shape or a smaller one allocates.  (No counterpart in the reference, whose kernels need
+ *    that shape, or of fewer rows or sequences with the same heads, allocates.  (No counterpart in the reference, whose kernels need
  *    no scratch.)
  *  - while `stream` is being captured into a CUDA graph a call that would have to grow the arena
  *    is refused (return 1) instead of allocating inside the capture: reserve first;
@@ -109,6 +109,10 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
  *    overwrite the first one's operand planes.  Calls queued on one stream are safe.  The batched
  *    calls that take a caller workspace (_keep, backward_batched, _rope_, decode) do not touch it. */
 int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim);
+/* Bytes zt_attn_reserve makes the arena hold for a shape (on the current device; without one, on a B200).  At least
+ * zt_attn_backward_workspace_bytes of the shape and of every one with fewer rows or sequences: a shorter sequence can
+ * use MORE scratch, because its work may be split into partial results where a longer one has blocks enough. */
+size_t zt_attn_reserve_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim);
 /* Bytes the current device's arena holds now (0 before its first use). */
 size_t zt_attn_arena_bytes(void);
 
@@ -146,8 +150,11 @@ int zt_attn_forward_batched(const float *q, const float *k, const float *v, floa
 /* Batched backward that consumes the forward's out and lse instead of
  * recomputing them (autograd.attentionBackward, src/autograd.zig:636-842, is the
  * arithmetic it must match).  delta is caller scratch [batch, T, n_heads].
- * dq, dk, dv are assigned.  workspace/workspace_bytes: see
- * zt_attn_backward_workspace_bytes; may be NULL/0 when that returns 0.
+ * dq, dk, dv are assigned.  workspace/workspace_bytes: zt_attn_backward_workspace_bytes says with how much the
+ * call is at its best, which does not grow with T alone (a short sequence may be split into partial results).  What
+ * it cannot do without does: a workspace sized for the longest sequence serves every shorter one.  Less than that
+ * is refused, except for sequences under 128 rows and widths other than 32, 64, 96, 128, 192 and 256: these
+ * run on the CUDA cores then (as all shapes do for which the query returns 0), NULL/0 included.
  * The workspace holds the 16-bit operand planes of q, k, v, dout;
  * at head_dim 192 and 256 it also holds the planes of P and dS of as many heads as fit in about 2 GiB
  * (at least one KV group's: 8 T^2 bytes a head), because the backward at those widths writes them to

@@ -127,6 +127,23 @@ def test_newer_extension_refusals(zt):
     L.zt_attn_set_verbose(1)
 
 
+@pytest.mark.parametrize("H,Hkv,D", [(32, 8, 128), (4, 2, 128), (4, 2, 32), (16, 4, 80), (8, 8, 64), (32, 8, 256), (8, 2, 192), (3, 1, 160)])
+def test_reserving_a_shape_covers_every_shorter_one(zt, H, Hkv, D):
+    """The scratch of a split is not monotone in T: 32/8 heads of 128 want more at 2304 rows than at 2432.  What
+    zt_attn_reserve holds for a shape has to cover all of them (both queries stand in a B200 where there is no device)."""
+    L = zt.lib.load()
+    lengths = sorted({*range(1, 130, 9), *range(128, 4097, 64), *range(1000, 4000, 333)})
+    want = {(b, t): L.zt_attn_backward_workspace_bytes(b, t, H, Hkv, D) for b in (1, 2, 3) for t in lengths}
+    if (H, Hkv, D) == (32, 8, 128):
+        assert want[1, 2304] > want[1, 2432]
+    worst = 0
+    for t in lengths:
+        worst = max(worst, want[1, t])
+        assert L.zt_attn_reserve_bytes(1, t, H, Hkv, D) >= worst, t
+        assert L.zt_attn_reserve_bytes(3, t, H, Hkv, D) >= max(n for (b, s), n in want.items() if s <= t), t
+    assert L.zt_attn_reserve_bytes(1, 0, H, Hkv, D) == 0 and L.zt_attn_reserve_bytes(1, 64, H, Hkv, 31) == 0
+
+
 def test_no_cpu_fallback_without_a_device(zt):
     """A well-formed call on a machine without a GPU is refused, never computed on the host."""
     import torch

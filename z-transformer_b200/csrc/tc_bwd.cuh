@@ -1026,8 +1026,10 @@ struct BwdWorkspace {
     float *rnorm;  // [batch, T, n_heads]
     __half *qs_planes;  // the row-scaled copy of q's planes (the fused and the wide-head backward read it for dK)
     uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
-    float *parts;       // partial results of a split forward, then of a split backward (tc_split.cuh)
-    size_t total_bytes;
+    // partial results of a split forward, then of a split backward (tc_split.cuh): behind everything else, so that a
+    // workspace of base_bytes does for a call that is not split
+    float *parts;
+    size_t base_bytes, total_bytes;
 };
 
 inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim) {
@@ -1048,6 +1050,7 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.rnorm = reinterpret_cast<float *>(c + off), off += up((size_t)batch * T * n_heads * sizeof(float));
     w.qs_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
+    w.base_bytes = off;
     const size_t pf = fwd_parts_floats(batch, T, n_heads, dim, 0), pb = dim <= 128 ? bwd_parts_floats(batch, T, n_heads, n_kv_heads, dim) : 0;
     w.parts = reinterpret_cast<float *>(c + off), off += up((pf > pb ? pf : pb) * sizeof(float));
     w.total_bytes = off;
@@ -1101,8 +1104,11 @@ inline int launch_bwd_tc_d(const BwdMaps &m, const BwdParams &p, cudaStream_t st
 
 }  // namespace tcb
 
-inline size_t tc_bwd_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
-    return tcb::bwd_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim)).total_bytes;
+// What the backward up to 128 columns wants, must have, and can want at this shape or a shorter one.
+inline WorkspaceNeed tc_bwd_workspace_need(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+    const tcb::BwdWorkspace w = tcb::bwd_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim));
+    const size_t pf = fwd_parts_floats_bound(tc::plane_dim(dim)), pb = bwd_parts_floats_bound(batch, T, n_heads, tc::plane_dim(dim));
+    return {w.base_bytes, w.total_bytes, w.base_bytes + ((pf > pb ? pf : pb) * sizeof(float) + 1023) / 1024 * 1024};
 }
 
 }  // namespace zt

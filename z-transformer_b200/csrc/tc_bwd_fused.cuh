@@ -669,7 +669,7 @@ inline bool tc_bwd_takes_fused(int dim, bool two_kernels, const PeerList *dq_pee
 // dq is first written.
 // rope_t: only with the two-kernel form (the fused kernel's dq takes its rotation in a pass of its own, by the caller).
 inline int launch_bwd_tc(const float *q, const float *k, const float *v, const float *out, const float *dout,
-                         const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
+                         const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, size_t workspace_bytes, int batch, int T,
                          int n_heads, int n_kv_heads, int dim, cudaStream_t stream, const float2 *rope = nullptr,
                          const float2 *rope_t = nullptr, bool qkv_planes_kept = false, const PeerList *dq_peers = nullptr,
                          bool two_kernels = false) {
@@ -729,6 +729,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     g_last_path = "tcgen05";
     if (fused) {
         p.parts = bwd_parts(batch, T, n_heads, n_kv_heads);
+        if (p.parts.n() > 1 && w.base_bytes + bwd_parts_floats(batch, T, n_heads, n_kv_heads, pd) * sizeof(float) > workspace_bytes) p.parts = BwdParts{1, 1};
         p.by_tile = tile_by_tile((long long)n_kv_heads * ((T + 127) / 128) * batch * p.parts.n(), kBwdTileWaves);
         if (p.parts.n() == 1) return tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream);
         const long long n = (long long)batch * T * n_kv_heads * dim;

@@ -784,7 +784,7 @@ constexpr size_t kScratchLimit = (size_t)16 << 30;   // one KV group's planes be
 
 struct WideWorkspace {
     tcb::BwdWorkspace base;   // the fused backward's layout first: the forward may have left q, k, v planes there
-    __half *p_planes, *ds_planes;
+    __half *p_planes, *ds_planes;  // where base has its partial results: a forward has put those together by then
     int Tp, unit_cap;
     size_t total_bytes;
 };
@@ -800,18 +800,21 @@ inline int wide_unit_cap(int batch, int T, int n_heads, int n_kv_heads) {
     return (int)(cap < all ? cap : all);
 }
 
-inline WideWorkspace wide_workspace(void *ws, int batch, int T, int n_heads, int n_kv_heads, int td) {
+// The layout in a workspace of `bytes`: a chunk takes as many heads as fit, one KV group's at least.
+inline WideWorkspace wide_workspace(void *ws, size_t bytes, int batch, int T, int n_heads, int n_kv_heads, int td) {
     WideWorkspace w{};
     w.base = tcb::bwd_workspace(ws, batch, T, n_heads, n_kv_heads, td);
-    auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
+    const int group = n_heads / n_kv_heads;
     w.Tp = (T + 127) / 128 * 128;
     w.unit_cap = wide_unit_cap(batch, T, n_heads, n_kv_heads);
+    const size_t half = (size_t)2 * w.Tp * w.Tp * sizeof(__half);  // P's two planes of a head, or dS's (a multiple of 64 KB)
+    const size_t fit = bytes > w.base.base_bytes ? (bytes - w.base.base_bytes) / (2 * half) / group * group : 0;
+    if (fit < (size_t)w.unit_cap) w.unit_cap = fit < (size_t)group ? group : (int)fit;
     char *c = static_cast<char *>(ws);
-    size_t off = w.base.total_bytes;
-    const size_t planes = (size_t)2 * w.unit_cap * w.Tp * w.Tp * sizeof(__half);
-    w.p_planes = reinterpret_cast<__half *>(c + off), off += up(planes);
-    w.ds_planes = reinterpret_cast<__half *>(c + off), off += up(planes);
-    w.total_bytes = off;
+    w.p_planes = reinterpret_cast<__half *>(c + w.base.base_bytes);
+    w.ds_planes = reinterpret_cast<__half *>(c + w.base.base_bytes + w.unit_cap * half);
+    w.total_bytes = w.base.base_bytes + 2 * w.unit_cap * half;
+    if (w.total_bytes < w.base.total_bytes) w.total_bytes = w.base.total_bytes;
     return w;
 }
 
@@ -829,21 +832,28 @@ inline size_t wide_smem_bytes() { return (size_t)kStages * kSB + sizeof(WideShar
 
 }  // namespace tcw
 
-inline size_t tc_bwd_wide_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
-    if (tcw::wide_unit_cap(batch, T, n_heads, n_kv_heads) == 0) return 0;
-    return tcw::wide_workspace(nullptr, batch, T, n_heads, n_kv_heads, tc_tile_dim(dim)).total_bytes;
+// What the backward above 128 columns wants, must have, and can want at this shape or a shorter one (all 0: not taken).
+inline WorkspaceNeed tc_bwd_wide_workspace_need(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+    if (tcw::wide_unit_cap(batch, T, n_heads, n_kv_heads) == 0) return {0, 0, 0};
+    const int td = tc_tile_dim(dim), group = n_heads / n_kv_heads;
+    const tcw::WideWorkspace w = tcw::wide_workspace(nullptr, SIZE_MAX, batch, T, n_heads, n_kv_heads, td);
+    const size_t unit = (size_t)8 * w.Tp * w.Tp, all = unit * batch * n_heads;
+    size_t planes = unit * group > tcw::kScratchBudget ? unit * group : tcw::kScratchBudget;
+    if (planes > all) planes = all;
+    const size_t parts = (fwd_parts_floats_bound(td) * sizeof(float) + 1023) / 1024 * 1024;
+    return {w.base.base_bytes + unit * group, w.total_bytes, w.base.base_bytes + (planes > parts ? planes : parts)};
 }
 
 // delta (= sum_j dout out, per row) is formed here; dq, dk, dv are assigned.  `out` may alias dq: it has been read when
 // dq is first written.
 inline int launch_bwd_wide(const float *q, const float *k, const float *v, const float *out, const float *dout,
-                           const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, int batch, int T,
+                           const float *lse, float *delta, float *dq, float *dk, float *dv, void *workspace, size_t workspace_bytes, int batch, int T,
                            int n_heads, int n_kv_heads, int dim, cudaStream_t stream, bool qkv_planes_kept = false,
                            bool tile_scores = false) {
     using namespace tcb;
     using namespace tcw;
     const int td = tc_tile_dim(dim);
-    const WideWorkspace ww = wide_workspace(workspace, batch, T, n_heads, n_kv_heads, td);
+    const WideWorkspace ww = wide_workspace(workspace, workspace_bytes, batch, T, n_heads, n_kv_heads, td);
     const BwdWorkspace &w = ww.base;
     const int group = n_heads / n_kv_heads;
     const int wq = n_heads * td, wkv = n_kv_heads * td;

@@ -348,6 +348,12 @@ inline bool tc_takes_dim(int dim) { return dim % 4 == 0 && dim >= 32 && dim <= 2
 // against 111 us at 2 rows already.
 constexpr int kTcForwardMinKeys = 33;
 
+// Bytes of a caller's scratch: without which a call cannot run, with which it runs at its best, and the most that this shape
+// or one of fewer rows or sequences runs best with.
+struct WorkspaceNeed {
+    size_t least, best, bound;
+};
+
 // ---- host: tensor maps through the driver entry point (no link-time libcuda dependency) ---------
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                     const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,

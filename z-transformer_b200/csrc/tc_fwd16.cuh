@@ -544,8 +544,8 @@ struct Workspace {
     uint32_t *vnmax;  // (in the backward's layout: the largest row norm of v, which the backward wants; else null)
     uint2 *part[3];   // the pre-pass's slots
     __half *q_planes, *k_planes, *v_planes;
-    float *parts;     // of a forward split along the keys
-    size_t total_bytes;
+    float *parts;     // of a forward split along the keys: behind everything else
+    size_t base_bytes, total_bytes;
 };
 
 inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset = 0) {
@@ -561,6 +561,7 @@ inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_h
     w.q_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
     w.k_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
+    w.base_bytes = off;
     w.parts = reinterpret_cast<float *>(c + off), off += up(fwd_parts_floats(batch, T, n_heads, dim, q_offset) * sizeof(float));
     w.total_bytes = off;
     return w;
@@ -606,7 +607,8 @@ inline bool tc_fwd16_supported(int batch, int T, int q_offset, int dim, const vo
 // q_offset: the query rows are a window of the sequence that starts there (batch 1; k and v hold at least q_offset + T
 // rows, of which the later ones are not read).
 // out_planes (optional): where the kernel also leaves out as f16 hi/lo planes, [2][batch][T][n_heads * dim] halves.
-inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float *out, float *lse, void *ws,
+// ws_bytes: at least the layout's bytes without the parts; a forward that has no room for them is not split.
+inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float *out, float *lse, void *ws, size_t ws_bytes,
                            int batch, int T, int n_heads, int n_kv_heads, int dim, cudaStream_t stream,
                            const float2 *rope = nullptr, bool in_backward_workspace = false, int variant = 0,
                            __half *out_planes = nullptr, const PeerList *out_peers = nullptr, int q_offset = 0) {
@@ -619,6 +621,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
         w.vnmax = bw.vnmax;
         for (int i = 0; i < 3; ++i) w.part[i] = bw.part[i];
         w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes, w.parts = bw.parts;
+        w.base_bytes = bw.base_bytes;
     }
     const int group = n_heads / n_kv_heads;
     const int n_seen = q_offset + T;  // key rows that some query row sees
@@ -643,6 +646,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     if (out_peers) p.out_peers = *out_peers;
     p.scale_log2 = kLog2e / sqrtf((float)dim);
     p.parts = variant == 0 && !out_planes && p.out_peers.n == 0 ? fwd_parts(batch, T, n_heads, q_offset) : 1;
+    if (p.parts > 1 && w.base_bytes + fwd_parts_floats(batch, T, n_heads, pd, q_offset) * sizeof(float) > ws_bytes) p.parts = 1;
     const long long rows = (long long)batch * T * n_heads;
     if (p.parts > 1) {
         p.out = w.parts, p.out_part = rows * dim;

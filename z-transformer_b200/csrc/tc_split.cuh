@@ -95,6 +95,15 @@ inline size_t bwd_parts_floats(int batch, int T, int n_heads, int n_kv_heads, in
     return n < 2 ? 0 : (size_t)n * 2 * batch * T * n_kv_heads * dim;
 }
 
+// Neither number grows with the shape -- a shorter sequence may be split where a longer one is not -- so a scratch that is to
+// serve every smaller shape too takes these, which do: the blocks that a split ends at, times what one of them writes.
+inline size_t fwd_parts_floats_bound(int dim) { return (size_t)split_sm_count() * 128 * (2 * (size_t)dim + 1); }
+inline size_t bwd_parts_floats_bound(int batch, int T, int n_heads, int dim) {
+    const size_t by_blocks = (size_t)4 * split_sm_count() * 128 * dim;
+    const size_t by_steps = (size_t)n_heads * ((T + 63) / 64) / 4 * 2 * batch * T * dim;  // (a part keeps four steps)
+    return by_steps < by_blocks ? by_steps : by_blocks;
+}
+
 // out, lse <- the forward's parts.  A warp per (row, head).
 __global__ void __launch_bounds__(256) fwd_join_kernel(const float *__restrict__ part, const float *__restrict__ part_lse,
                                                        float *__restrict__ out, float *__restrict__ lse, long long rows, int dim,

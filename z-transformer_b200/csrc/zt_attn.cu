@@ -111,7 +111,7 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
             return refuse("this shape needs %zu bytes of the per-device arena, which would have to grow while the "
                           "stream is being captured: call zt_attn_reserve for the shape before the capture.", need);
         if (arena)
-            return launch_fwd_tc16(q, k, v, out, lse, arena, batch, T, n_heads, n_kv_heads, dim, stream, nullptr, false,
+            return launch_fwd_tc16(q, k, v, out, lse, arena, need, batch, T, n_heads, n_kv_heads, dim, stream, nullptr, false,
                                    path == 6 ? 1 : (path == 7 ? 2 : 0), nullptr, nullptr, q_offset);
     }
     if ((path == 0 || path == 2 || path == 6 || path == 7 || path == 8) &&
@@ -129,16 +129,24 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
     return launch_fwd_simt(p, batch, stream);
 }
 
-static size_t backward_workspace(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+// A caller's workspace for the tensor-core backward (all 0 where there is none).  A split of the work and, above 128 columns,
+// how many heads go through memory together take what room there is beyond `least`, which grows with the shape: a workspace
+// sized for the longest sequence serves the shorter ones, although some of them would use more if they had it.
+static WorkspaceNeed backward_need(int batch, int T, int n_heads, int n_kv_heads, int dim) {
 #ifndef ZT_NO_TC
-    if (tc_takes_dim(dim)) {
-        if (dim <= 128) return tc_bwd_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
-        // wider heads: the planes of the fused form, then a row-scaled copy of Q's and the planes of P and dS
-        return tc_bwd_wide_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
-    }
+    if (tc_takes_dim(dim))
+        return dim <= 128 ? tc_bwd_workspace_need(batch, T, n_heads, n_kv_heads, dim) : tc_bwd_wide_workspace_need(batch, T, n_heads, n_kv_heads, dim);
 #endif
-    (void)batch, (void)n_heads, (void)n_kv_heads;
-    return 0;
+    (void)batch, (void)T, (void)n_heads, (void)n_kv_heads;
+    return {0, 0, 0};
+}
+// Without a workspace, or with less than `least`, these shapes run on the CUDA cores instead of being refused: widths between
+// the tiles' and sequences shorter than a tile of query rows.
+static bool workspace_optional(int T, int dim) {
+    return T < 128 || !(dim == 32 || dim == 64 || dim == 96 || dim == 128 || dim == 192 || dim == 256);
+}
+static size_t required_workspace(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+    return workspace_optional(T, dim) ? 0 : backward_need(batch, T, n_heads, n_kv_heads, dim).least;
 }
 
 // The forward-for-training call (zt_attn_forward_batched_keep) leaves the f16 planes of q, k, v in the backward's
@@ -213,19 +221,18 @@ static int backward_impl(const float *q, const float *k, const float *v, const f
                          int n_kv_heads, int dim, cudaStream_t stream, bool kept = false,
                          const PeerList *dq_peers = nullptr) {
 #ifndef ZT_NO_TC
-    if (g_path.load() != 1 && workspace &&
-        workspace_bytes >= backward_workspace(batch, T, n_heads, n_kv_heads, dim) &&
+    const size_t least = backward_need(batch, T, n_heads, n_kv_heads, dim).least;
+    if (g_path.load() != 1 && workspace && workspace_bytes >= least &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
         n_kv_heads <= tcb::kPrepassMaxGroups && tcb::tc_bwd_supported(batch, T, dim, q, k, v, dout, dq, dk, dv)) {
-        return launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads,
+        return launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, workspace_bytes, batch, T, n_heads, n_kv_heads,
                              dim, stream, nullptr, nullptr, kept, dq_peers, g_path.load() == 8);
     }
-    const size_t wide_need = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
-    if (g_path.load() != 1 && workspace && wide_need > 0 && workspace_bytes >= wide_need &&
+    if (g_path.load() != 1 && workspace && least > 0 && workspace_bytes >= least &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
         !(dq_peers && dq_peers->n > 0) &&
         tcw::tc_bwd_wide_supported(batch, T, n_heads, n_kv_heads, dim, q, k, v, dout, dq, dk, dv)) {
-        return launch_bwd_wide(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, batch, T, n_heads, n_kv_heads, dim,
+        return launch_bwd_wide(q, k, v, out, dout, lse, delta, dq, dk, dv, workspace, workspace_bytes, batch, T, n_heads, n_kv_heads, dim,
                                stream, kept, g_path.load() == 8);
     }
 #endif
@@ -334,22 +341,27 @@ int zt_attn_tc_saturated(unsigned int *host_count) {
     return 0;
 }
 
+size_t zt_attn_reserve_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+    if (batch < 1 || T < 1 || n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads != 0 || !zt_attn_dim_ok(dim)) return 0;
+    size_t need = kArenaBytes;  // the decode-shaped forward's partial results
+#ifndef ZT_NO_TC
+    if (n_kv_heads <= tcb::kPrepassMaxGroups && tc_takes_dim(dim)) {
+        // (a shorter sequence, or a window of this one, may be split where this one is not)
+        const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim) + fwd_parts_floats_bound(tc::plane_dim(dim)) * sizeof(float);
+        const size_t b = backward_need(batch, T, n_heads, n_kv_heads, dim).bound;
+        need = f > need ? f : need;
+        need = b > need ? b : need;
+    }
+#endif
+    return need;
+}
+
 int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     g_last_error[0] = 0;
     if (batch < 1 || batch > 65535) return refuse("batch %d is not launchable (1 .. 65535).", batch);
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     if (need_device()) return 1;
-    size_t need = kArenaBytes;  // the decode-shaped forward's partial results
-#ifndef ZT_NO_TC
-    if (n_kv_heads <= tcb::kPrepassMaxGroups && tc_takes_dim(dim)) {
-        // (and, for windows of the sequence, the partial rows of a forward that is split until every SM has a block)
-        const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim) +
-                         (size_t)split_sm_count() * 128 * (2 * tc_tile_dim(dim) + 1) * sizeof(float);
-        const size_t b = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
-        need = f > need ? f : need;
-        need = b > need ? b : need;
-    }
-#endif
+    const size_t need = zt_attn_reserve_bytes(batch, T, n_heads, n_kv_heads, dim);
     bool in_capture = false;
     if (!device_arena(need, nullptr, &in_capture))
         return refuse("the per-device arena of %zu bytes could not be allocated.", need);
@@ -466,7 +478,7 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
     if (need_device()) return 1;
     cudaStream_t s = (cudaStream_t)stream;
     // the arena must hold the backward's planes (at least the forward's): grown, if at all, before any launch
-    const size_t need = backward_workspace(1, T, n_heads, n_kv_heads, dim);
+    const size_t need = backward_need(1, T, n_heads, n_kv_heads, dim).best;
     bool in_capture = false;
     void *arena = need ? device_arena(need, s, &in_capture) : nullptr;
     if (in_capture)
@@ -521,12 +533,12 @@ static int forward_keep_impl(const float *q, const float *k, const float *v, flo
     cudaStream_t s = (cudaStream_t)stream;
     if (workspace) drop_kept_planes(workspace);
 #ifndef ZT_NO_TC
-    const size_t need = backward_workspace(batch, T, n_heads, n_kv_heads, dim);
+    const size_t need = backward_need(batch, T, n_heads, n_kv_heads, dim).least;
     const int keep_path = g_path.load();
     if ((keep_path == 0 || keep_path == 6 || keep_path == 7 || keep_path == 8) && need > 0 && workspace && workspace_bytes >= need &&
         (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
         tc_fwd16_supported(batch, T, 0, dim, q, k, v, out)) {
-        if (launch_fwd_tc16(q, k, v, out, lse, workspace, batch, T, n_heads, n_kv_heads, dim, s, nullptr, true,
+        if (launch_fwd_tc16(q, k, v, out, lse, workspace, workspace_bytes, batch, T, n_heads, n_kv_heads, dim, s, nullptr, true,
                             keep_path == 6 ? 1 : (keep_path == 7 ? 2 : 0), nullptr, out_peers))
             return 1;
         const unsigned long long token = note_kept_planes(workspace, batch, T, n_heads, n_kv_heads, dim);
@@ -563,7 +575,7 @@ int zt_attn_forward_batched_keep_peers(const float *q, const float *k, const flo
 size_t zt_attn_backward_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     if (batch < 1 || T < 1 || n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads != 0 || !zt_attn_dim_ok(dim))
         return 0;
-    return backward_workspace(batch, T, n_heads, n_kv_heads, dim);
+    return backward_need(batch, T, n_heads, n_kv_heads, dim).best;
 }
 
 static int backward_kept_impl(const float *q, const float *k, const float *v, const float *out,
@@ -575,9 +587,10 @@ static int backward_kept_impl(const float *q, const float *k, const float *v, co
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     if (!q || !k || !v || !out || !lse || !dout || !dq || !dk || !dv || !delta)
         return refuse("a null device pointer was passed.");
-    const size_t need = zt_attn_backward_workspace_bytes(batch, T, n_heads, n_kv_heads, dim);
+    const size_t need = required_workspace(batch, T, n_heads, n_kv_heads, dim);
     if (need > 0 && (!workspace || workspace_bytes < need))
-        return refuse("the backward needs %zu bytes of workspace, %zu were given.", need, workspace_bytes);
+        return refuse("the backward needs %zu bytes of workspace (%zu to run at its best), %zu were given.", need,
+                      zt_attn_backward_workspace_bytes(batch, T, n_heads, n_kv_heads, dim), workspace_bytes);
     if (need > 0 && (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
         return refuse("the backward workspace must be 256-byte aligned.");
     if (need_device()) return 1;
@@ -629,9 +642,10 @@ struct RopeWorkspace {
     float2 *table_t;       // the same, [dim / 2][T]
     float *q_rot, *k_rot;  // rotated copies, used only off the fused path
     void *inner;           // the tensor-core kernels' workspace (operand planes)
-    size_t inner_bytes, total_bytes;
+    size_t inner_bytes;    // (of a workspace of `bytes`)
+    size_t least_bytes, total_bytes;
 };
-RopeWorkspace rope_workspace(void *base, int batch, int T, int n_heads, int n_kv_heads, int dim) {
+RopeWorkspace rope_workspace(void *base, size_t bytes, int batch, int T, int n_heads, int n_kv_heads, int dim) {
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     RopeWorkspace w{};
     char *c = static_cast<char *>(base);
@@ -641,9 +655,9 @@ RopeWorkspace rope_workspace(void *base, int batch, int T, int n_heads, int n_kv
     w.q_rot = reinterpret_cast<float *>(c + off), off += up((size_t)batch * T * n_heads * dim * sizeof(float));
     w.k_rot = reinterpret_cast<float *>(c + off), off += up((size_t)batch * T * n_kv_heads * dim * sizeof(float));
     w.inner = c + off;
-    w.inner_bytes = backward_workspace(batch, T, n_heads, n_kv_heads, dim);  // >= the forward's planes
-    off += up(w.inner_bytes);
-    w.total_bytes = off;
+    w.inner_bytes = bytes > off ? bytes - off : 0;
+    w.least_bytes = off + required_workspace(batch, T, n_heads, n_kv_heads, dim);
+    w.total_bytes = off + up(backward_need(batch, T, n_heads, n_kv_heads, dim).best);
     return w;
 }
 int check_rope_call(const void *workspace, size_t workspace_bytes, size_t need, int pos, double theta) {
@@ -659,7 +673,7 @@ int check_rope_call(const void *workspace, size_t workspace_bytes, size_t need, 
 size_t zt_attn_rope_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     if (batch < 1 || T < 1 || n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads != 0 || !zt_attn_dim_ok(dim))
         return 0;
-    return rope_workspace(nullptr, batch, T, n_heads, n_kv_heads, dim).total_bytes;
+    return rope_workspace(nullptr, 0, batch, T, n_heads, n_kv_heads, dim).total_bytes;
 }
 
 // zt_attn_forward_rope_batched; with out_planes the tensor-core kernel also leaves out as f16 planes there and
@@ -674,20 +688,20 @@ static int forward_rope_impl(const float *q, const float *k, const float *v, flo
     if (batch < 1 || batch > 65535) return refuse("batch %d is not launchable (1 .. 65535).", batch);
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     if (!q || !k || !v || !out) return refuse("a null device pointer was passed.");
-    const RopeWorkspace w = rope_workspace(workspace, batch, T, n_heads, n_kv_heads, dim);
-    if (check_rope_call(workspace, workspace_bytes, w.total_bytes, pos, theta)) return 1;
+    const RopeWorkspace w = rope_workspace(workspace, workspace_bytes, batch, T, n_heads, n_kv_heads, dim);
+    if (check_rope_call(workspace, workspace_bytes, w.least_bytes, pos, theta)) return 1;
     if (need_device()) return 1;
     cudaStream_t s = (cudaStream_t)stream;
     drop_kept_planes(w.inner);
     if (launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
 #ifndef ZT_NO_TC
+    const size_t least = backward_need(batch, T, n_heads, n_kv_heads, dim).least;
     // (the pre-pass rotates four elements at a time: a head's halves must be multiples of four)
     if ((g_path.load() == 0 || g_path.load() == 8) && n_kv_heads <= tcb::kPrepassMaxGroups && dim % 8 == 0 &&
-        tc_fwd16_supported(batch, T, 0, dim, q, k, v, out) &&
-        w.inner_bytes >= tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim)) {
+        tc_fwd16_supported(batch, T, 0, dim, q, k, v, out) && least > 0 && w.inner_bytes >= least) {
         // the planes (rotated q and k among them) go where the backward keeps its own: the rope backward that
         // follows with the same workspace, tensors, pos and theta converts only dout
-        if (launch_fwd_tc16(q, k, v, out, lse, w.inner, batch, T, n_heads, n_kv_heads, dim, s, w.table, true, 0, out_planes)) return 1;
+        if (launch_fwd_tc16(q, k, v, out, lse, w.inner, w.inner_bytes, batch, T, n_heads, n_kv_heads, dim, s, w.table, true, 0, out_planes)) return 1;
         const unsigned long long token = note_kept_planes(w.inner, batch, T, n_heads, n_kv_heads, dim, true, pos, theta);
         if (host_token) *host_token = token;
         if (planes_written) *planes_written = out_planes != nullptr;
@@ -718,8 +732,8 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     if (!q || !k || !v || !out || !lse || !dout || !dq || !dk || !dv || !delta)
         return refuse("a null device pointer was passed.");
-    const RopeWorkspace w = rope_workspace(workspace, batch, T, n_heads, n_kv_heads, dim);
-    if (check_rope_call(workspace, workspace_bytes, w.total_bytes, pos, theta)) return 1;
+    const RopeWorkspace w = rope_workspace(workspace, workspace_bytes, batch, T, n_heads, n_kv_heads, dim);
+    if (check_rope_call(workspace, workspace_bytes, w.least_bytes, pos, theta)) return 1;
     if (need_device()) return 1;
     cudaStream_t s = (cudaStream_t)stream;
     const bool kept = take_kept_planes(w.inner, token, batch, T, n_heads, n_kv_heads, dim, true, pos, theta);
@@ -730,13 +744,14 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     if (launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
     bool fused = false, dq_in_kernel = false;
 #ifndef ZT_NO_TC
-    fused = g_path.load() != 1 && w.inner_bytes > 0 && dim % 8 == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
+    const size_t least = backward_need(batch, T, n_heads, n_kv_heads, dim).least;
+    fused = g_path.load() != 1 && least > 0 && w.inner_bytes >= least && dim % 8 == 0 && n_kv_heads <= tcb::kPrepassMaxGroups &&
             tcb::tc_bwd_supported(batch, T, dim, q, k, v, dout, dq, dk, dv);
     // the dQ kernel's epilogue rotates whole 16- or 32-column pieces: only where a head's half is made of them;
     // and the fused backward adds partial sums into dq, which can only be rotated once they are complete
     const bool two_kernels = g_path.load() == 8;
     dq_in_kernel = fused && (dim == 32 || dim == 64 || dim == 128) && !tc_bwd_takes_fused(dim, two_kernels, nullptr);
-    if (fused && launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, w.inner, batch, T, n_heads, n_kv_heads, dim, s,
+    if (fused && launch_bwd_tc(q, k, v, out, dout, lse, delta, dq, dk, dv, w.inner, w.inner_bytes, batch, T, n_heads, n_kv_heads, dim, s,
                                w.table, dq_in_kernel ? w.table_t : nullptr, kept, nullptr, two_kernels))
         return 1;
 #endif
@@ -879,7 +894,7 @@ int zt_attn_block_forward(const float *q, const float *k, const float *v, const 
         return 1;
     const uint32_t *from = nullptr;
     if (planes_written) {
-        const RopeWorkspace rw = rope_workspace(rope_ws, batch, T, n_heads, n_kv_heads, dim);
+        const RopeWorkspace rw = rope_workspace(rope_ws, rope_ws_bytes, batch, T, n_heads, n_kv_heads, dim);
         from = tcb::bwd_workspace(rw.inner, batch, T, n_heads, n_kv_heads, tc::plane_dim(dim)).amax_v;
     }
     return proj_forward_impl(ctx, wo, y, proj_workspace_, batch, T, kdim, d_model, s, from, n_kv_heads);
