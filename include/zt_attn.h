@@ -16,9 +16,10 @@
  *     zt_attn_forward_batched take no workspace; their scratch (the 16-bit
  *     operand planes of q, k, v, dout: up to 4 bytes per element of those
  *     tensors, or 16 MiB for a decode-shaped call) lives in one per-device
- *     arena.  See "The per-device arena" below for when it allocates, how to
+ *     arena, or is taken and given back in the order of the call's stream.  See
+ *     "Scratch" below for which call does what, when either allocates, how to
  *     make that never happen mid-run (zt_attn_reserve) and what calls that
- *     share it must not do;
+ *     share the arena must not do;
  *   - return 0: the work was enqueued on `stream` (no synchronisation);
  *     return 1: refused, with the reason on stderr and in zt_attn_last_error();
  *     nothing was launched and no buffer was touched;
@@ -70,8 +71,10 @@ size_t zt_attn_bwd_dkdv_shmem(int dim);
  * n_heads > 65535; group_q outside [1, 64] or dim*group_q > 1024;
  * q_offset < 0, n_keys < 1 or q_offset > n_keys - T; max_tile < 1.
  * A decode-shaped call (T == 1) splits the context over many blocks and keeps
- * its partial results in a per-device arena of 16 MiB that is allocated once,
- * on the first such call on that device. */
+ * its partial results in the per-device arena (16 MiB at least, allocated on the
+ * first call on that device that needs it).  Every other call of more than 32
+ * keys whose head width is a multiple of four keeps operand planes: see
+ * "Scratch". */
 int zt_attn_forward(const float *q, const float *k, const float *v, float *out, int T, int n_heads,
                     int n_kv_heads, int dim, int group_q, int max_tile, int q_offset, int n_keys,
                     zt_stream_t stream);
@@ -91,26 +94,38 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
 /* Extensions                                                                 */
 /* ------------------------------------------------------------------------- */
 
-/* The per-device arena.  zt_attn_forward, zt_attn_backward and zt_attn_forward_batched have no
- * workspace argument (the reference's signatures have none, src/cuda/device.zig:69-105), so their
- * scratch comes from an arena this library keeps per device.  Rules:
+/* Scratch.  zt_attn_forward, zt_attn_backward and zt_attn_forward_batched have no workspace
+ * argument (the reference's signatures have none, src/cuda/device.zig:69-105).
+ *
+ * Windows (q_offset > 0 or n_keys > T), sequences under 128 rows, and head widths other than 32, 64,
+ * 96, 128, 192 and 256 take theirs with cudaMallocFromPoolAsync on the call's stream, from a pool of
+ * the library's own per device, and give it back behind their launches.  Nothing is shared: such
+ * calls may overlap on the GPU (several streams and threads) and need no preparation to be captured
+ * (inside a capture the memory is the graph's own, so such a graph has memory nodes: it can
+ * be instantiated once at a time and not become a child graph).  The pool keeps up to 2 GiB between
+ * calls, or what zt_attn_reserve asked for, and gives back the rest when the device is waited for.
+ * Where there is no memory to be had they run on the CUDA cores, which need none.
+ *
+ * Decode-shaped calls (T == 1) and whole sequences of at least 128 rows at those six widths take
+ * theirs from an arena this library keeps per device.  Rules:
  *  - it is allocated (cudaMalloc) by the first call on a device that needs it and grows when a
  *    later call needs more; it never shrinks, and an outgrown arena is kept until the process ends
  *    (work queued earlier may still be using it), so growth costs memory, never correctness;
  *  - zt_attn_reserve sizes it for a shape up front -- the place for it is where the reference's
  *    holder sizes its own eleven buffers (device.Attn.init, src/cuda/device.zig:221-299; that
- *    function already calls zt_attn_dim_ok).  After zt_attn_reserve(batch, T, ...) no call of
+ *    function already calls zt_attn_dim_ok); it makes the pool hold what windows take, too.  After zt_attn_reserve(batch, T, ...) no call of
  *    that shape, or of fewer rows or sequences with the same heads, allocates.  (No counterpart in the reference, whose kernels need
  *    no scratch.)
  *  - while `stream` is being captured into a CUDA graph a call that would have to grow the arena
  *    is refused (return 1) instead of allocating inside the capture: reserve first;
- *  - every call on a device shares the arena: two calls that use it must not overlap on the GPU
- *    (different streams or host threads without an ordering between them) -- the second would
- *    overwrite the first one's operand planes.  Calls queued on one stream are safe.  The batched
+ *  - these calls share the arena: two of them must not overlap on the GPU (different streams or
+ *    host threads without an ordering between them) -- the second would overwrite the first one's
+ *    operand planes.  Calls queued on one stream are safe.  The batched
  *    calls that take a caller workspace (_keep, backward_batched, _rope_, decode) do not touch it. */
 int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim);
-/* Bytes zt_attn_reserve makes the arena hold for a shape (on the current device; without one, on a B200).  At least
- * zt_attn_backward_workspace_bytes of the shape and of every one with fewer rows or sequences: a shorter sequence can
+/* The most scratch that a call of this shape, of a window of it, or of fewer rows or sequences takes: what
+ * zt_attn_reserve makes the arena hold for whole sequences, where they use it (on the current device; without one, on a
+ * B200).  At least zt_attn_backward_workspace_bytes of the shape and of every one with fewer rows or sequences: a shorter sequence can
  * use MORE scratch, because its work may be split into partial results where a longer one has blocks enough. */
 size_t zt_attn_reserve_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim);
 /* Bytes the current device's arena holds now (0 before its first use). */

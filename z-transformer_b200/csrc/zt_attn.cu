@@ -31,6 +31,14 @@ namespace zt {
 constexpr int kMinDim = 32, kMaxDim = 256;  // src/cuda/attn_kernels.cu:147-148
 constexpr size_t kArenaBytes = 16u << 20;
 
+static bool is_capturing(cudaStream_t stream) {
+    // (the legacy default stream cannot be captured, and asking about it would itself disturb a capture running on another
+    // stream)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (stream != nullptr && cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();
+    return cap != cudaStreamCaptureStatusNone;
+}
+
 // One arena per device for the entry points that take no workspace argument (the reference's own two, and
 // the batched forward): created on the first call that needs scratch on that device, or by zt_attn_reserve.
 // It only ever grows, and an arena that has been outgrown is retired, not freed: a launch queued earlier, or a
@@ -39,7 +47,7 @@ constexpr size_t kArenaBytes = 16u << 20;
 // step -- allocates on its first step (or in zt_attn_reserve) and never again.
 // Growth is refused (nullptr, with the reason recorded) while `stream` is being captured into a CUDA graph:
 // an allocation inside a capture would break it, and the caller can size the arena beforehand.
-// Every call on a device shares the arena: calls that use it must not overlap on the GPU (see zt_attn.h).
+// The calls that use it share it: they must not overlap on the GPU (see zt_attn.h).
 static void *device_arena(size_t need, cudaStream_t stream, bool *refused_in_capture = nullptr,
                           size_t *held_now = nullptr) {
     static void *arena[64] = {};
@@ -54,11 +62,7 @@ static void *device_arena(size_t need, cudaStream_t stream, bool *refused_in_cap
     }
     if (need < kArenaBytes) need = kArenaBytes;
     if (held[dev] < need) {
-        // (the legacy default stream cannot be captured, and asking about it would itself disturb a capture
-        // running on another stream)
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (stream != nullptr && cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();
-        if (cap != cudaStreamCaptureStatusNone) {
+        if (is_capturing(stream)) {
             if (refused_in_capture) *refused_in_capture = true;
             return nullptr;
         }
@@ -71,6 +75,73 @@ static void *device_arena(size_t need, cudaStream_t stream, bool *refused_in_cap
     }
     return arena[dev];
 }
+
+// Scratch of one call, in the order of its stream: taken before the call's launches, given back behind them.  For the calls
+// that could do without any -- on the CUDA cores -- and therefore share nothing with each other: they may run on several streams
+// and threads at once, and be captured, without a word to the library.  The memory comes from a pool of the library's own per
+// device that keeps up to kPoolKeeps bytes (or what zt_attn_reserve asks for) between calls and gives back the rest whenever
+// the device is waited for; inside a capture it is the graph's own.  A pair of driver calls each:
+// 77 rows of 32/8 heads of 128 take 17.1 us in a run of calls either way, a first call by itself 31.2 us where the arena's
+// took 29.0.
+constexpr size_t kPoolKeeps = (size_t)2 << 30;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    bool tried = false;
+    size_t keeps = 0, mapped = 0;
+};
+// The current device's pool; with `map`, `map` bytes of it are there for good.
+static cudaMemPool_t device_pool(size_t map = 0) {
+    static DevicePool table[64];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    DevicePool &d = table[dev];
+    if (d.tried && map <= d.mapped) return d.pool;
+    // (a capture, this thread's or another's, must neither make these calls fail nor be broken by them)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!d.tried) {
+        d.tried = true;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice, props.location.id = dev;
+        if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) d.pool = nullptr;
+    }
+    unsigned long long keep = map > kPoolKeeps ? map : kPoolKeeps;
+    if (d.pool && d.keeps < keep && cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) d.keeps = keep;
+    cudaStream_t s = nullptr;
+    void *ptr = nullptr;
+    if (d.pool && map > d.mapped && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) {
+        if (cudaMallocFromPoolAsync(&ptr, map, d.pool, s) == cudaSuccess && cudaFreeAsync(ptr, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess)
+            d.mapped = map;
+        cudaStreamDestroy(s);
+    }
+    cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return d.pool;
+}
+class StreamScratch {
+  public:
+    StreamScratch(size_t need, cudaStream_t stream) : stream_(stream) {
+        if (need == 0) return;
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (is_capturing(stream)) e = cudaMallocAsync(&ptr_, need, stream);
+        else if (cudaMemPool_t pool = device_pool()) e = cudaMallocFromPoolAsync(&ptr_, need, pool, stream);
+        if (e != cudaSuccess) ptr_ = nullptr, cudaGetLastError();
+    }
+    ~StreamScratch() {
+        if (ptr_ && cudaFreeAsync(ptr_, stream_) != cudaSuccess) cudaGetLastError();
+    }
+    StreamScratch(const StreamScratch &) = delete;
+    StreamScratch &operator=(const StreamScratch &) = delete;
+    void *get() const { return ptr_; }  // null: there is none to be had
+
+  private:
+    void *ptr_ = nullptr;
+    cudaStream_t stream_;
+};
 
 static inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -92,6 +163,11 @@ static int need_device() {
     return 0;
 }
 
+// Without a workspace, or with less than `least`, these shapes run on the CUDA cores instead of being refused: widths between
+// the tiles' and sequences shorter than a tile of query rows.
+static bool workspace_optional(int T, int dim) {
+    return T < 128 || !(dim == 32 || dim == 64 || dim == 96 || dim == 128 || dim == 192 || dim == 256);
+}
 static int forward_impl(const float *q, const float *k, const float *v, float *out, float *lse,
                         int batch, int T, int n_heads, int n_kv_heads, int dim, int q_offset,
                         int n_keys, cudaStream_t stream) {
@@ -103,10 +179,13 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
     if ((path == 0 || path == 6 || path == 7 || path == 8) && n_kv_heads <= tcb::kPrepassMaxGroups &&
         tc_fwd16_supported(batch, T, q_offset, dim, q, k, v, out)) {
         // The f16-split forward keeps its operand planes in the per-device arena (no entry point
-        // of the forward takes a workspace); see device_arena for when that allocates.
+        // of the forward takes a workspace); see device_arena for when that allocates.  Windows and the shapes that can
+        // do without scratch have some of their own for the call.
         const size_t need = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim, q_offset);
+        const bool own = q_offset != 0 || n_keys != T || workspace_optional(T, dim);
+        const StreamScratch scratch(own ? need : 0, stream);
         bool in_capture = false;
-        void *arena = device_arena(need, stream, &in_capture);
+        void *arena = own ? scratch.get() : device_arena(need, stream, &in_capture);
         if (in_capture)
             return refuse("this shape needs %zu bytes of the per-device arena, which would have to grow while the "
                           "stream is being captured: call zt_attn_reserve for the shape before the capture.", need);
@@ -139,11 +218,6 @@ static WorkspaceNeed backward_need(int batch, int T, int n_heads, int n_kv_heads
 #endif
     (void)batch, (void)T, (void)n_heads, (void)n_kv_heads;
     return {0, 0, 0};
-}
-// Without a workspace, or with less than `least`, these shapes run on the CUDA cores instead of being refused: widths between
-// the tiles' and sequences shorter than a tile of query rows.
-static bool workspace_optional(int T, int dim) {
-    return T < 128 || !(dim == 32 || dim == 64 || dim == 96 || dim == 128 || dim == 192 || dim == 256);
 }
 static size_t required_workspace(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     return workspace_optional(T, dim) ? 0 : backward_need(batch, T, n_heads, n_kv_heads, dim).least;
@@ -341,19 +415,24 @@ int zt_attn_tc_saturated(unsigned int *host_count) {
     return 0;
 }
 
+// The most scratch that a forward and a backward of this shape, a window of it, or a shorter sequence takes.
+static void scratch_bounds(int batch, int T, int n_heads, int n_kv_heads, int dim, size_t *forward, size_t *backward) {
+    *forward = *backward = 0;
+#ifndef ZT_NO_TC
+    if (n_kv_heads > tcb::kPrepassMaxGroups || !tc_takes_dim(dim)) return;
+    // (a shorter sequence, or a window of this one, may be split where this one is not)
+    *forward = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim) + fwd_parts_floats_bound(tc::plane_dim(dim)) * sizeof(float);
+    *backward = backward_need(batch, T, n_heads, n_kv_heads, dim).bound;
+#endif
+    (void)batch, (void)T, (void)n_heads;
+}
+static size_t most(size_t a, size_t b) { return a > b ? a : b; }
+
 size_t zt_attn_reserve_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     if (batch < 1 || T < 1 || n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads != 0 || !zt_attn_dim_ok(dim)) return 0;
-    size_t need = kArenaBytes;  // the decode-shaped forward's partial results
-#ifndef ZT_NO_TC
-    if (n_kv_heads <= tcb::kPrepassMaxGroups && tc_takes_dim(dim)) {
-        // (a shorter sequence, or a window of this one, may be split where this one is not)
-        const size_t f = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim) + fwd_parts_floats_bound(tc::plane_dim(dim)) * sizeof(float);
-        const size_t b = backward_need(batch, T, n_heads, n_kv_heads, dim).bound;
-        need = f > need ? f : need;
-        need = b > need ? b : need;
-    }
-#endif
-    return need;
+    size_t f, b;
+    scratch_bounds(batch, T, n_heads, n_kv_heads, dim, &f, &b);
+    return most(kArenaBytes, most(f, b));  // (16 MiB: the decode-shaped forward's partial results)
 }
 
 int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim) {
@@ -361,10 +440,16 @@ int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim) {
     if (batch < 1 || batch > 65535) return refuse("batch %d is not launchable (1 .. 65535).", batch);
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     if (need_device()) return 1;
-    const size_t need = zt_attn_reserve_bytes(batch, T, n_heads, n_kv_heads, dim);
+    size_t f, b, f_short, b_short;
+    scratch_bounds(batch, T, n_heads, n_kv_heads, dim, &f, &b);
+    scratch_bounds(batch, T < 127 ? T : 127, n_heads, n_kv_heads, dim, &f_short, &b_short);
+    // the arena serves whole sequences of the widths and lengths that cannot do without; the pool serves windows and the rest
+    const bool own = workspace_optional(T, dim);
+    const size_t need = own ? kArenaBytes : most(kArenaBytes, most(f, b));
     bool in_capture = false;
     if (!device_arena(need, nullptr, &in_capture))
         return refuse("the per-device arena of %zu bytes could not be allocated.", need);
+    device_pool(most(f, own ? b : b_short));  // (as far as it goes: what it serves has a form that needs no scratch)
     return 0;
 }
 
@@ -477,10 +562,12 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
         return refuse("a null device pointer was passed.");
     if (need_device()) return 1;
     cudaStream_t s = (cudaStream_t)stream;
-    // the arena must hold the backward's planes (at least the forward's): grown, if at all, before any launch
+    // the scratch must hold the backward's planes (at least the forward's): the arena grows, if at all, before any launch
     const size_t need = backward_need(1, T, n_heads, n_kv_heads, dim).best;
+    const bool own = workspace_optional(T, dim);
+    const StreamScratch scratch(own ? need : 0, s);
     bool in_capture = false;
-    void *arena = need ? device_arena(need, s, &in_capture) : nullptr;
+    void *arena = own ? scratch.get() : need ? device_arena(need, s, &in_capture) : nullptr;
     if (in_capture)
         return refuse("this shape needs %zu bytes of the per-device arena, which would have to grow while the "
                       "stream is being captured: call zt_attn_reserve for the shape before the capture.", need);
