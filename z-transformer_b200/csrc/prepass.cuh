@@ -133,7 +133,9 @@ __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int bl
 // LP lanes hold a unit, NC float4 each.  The loads run kStages - 1 steps of U units ahead through slots of shared memory
 // that belong to one thread each (so nothing but the thread's own copies is waited for): held in registers instead,
 // the loads of a step would stall on the arithmetic of the step before (heads of 256, batch 8, T 1024: 4.1 TB/s against 5.4).
-template <int LP, int NC>
+// O4: the tensor that dout is multiplied with starts on a 4-byte boundary only (of a call's tensors it alone may, because
+// nothing but its row sums is wanted).  A variant of its own: asked per copy it cost every backward 0.4 us.
+template <int LP, int NC, bool O4>
 __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_constant__ PassArgs a) {
     constexpr int NG = kPassThreads / LP, U = 1, S = kStatsStages;
     extern __shared__ __align__(16) float4 ring[];  // [S][U][NC][2][kPassThreads]
@@ -142,8 +144,6 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows_out = t.delta != nullptr, norms = rows_out || t.nmax != nullptr;
-    // (of a call's tensors `o` alone is not asked to start on a 16-byte boundary: nothing but its row sums is wanted)
-    const bool o_aligned = (reinterpret_cast<uintptr_t>(t.o) & 15u) == 0;
     const int n4 = a.dim >> 2, group = t.group, heads = t.heads;
     const long long first = (long long)w.b * t.rows * heads + w.g * group;  // the (sequence, group)'s first unit
     const float4 *xb = reinterpret_cast<const float4 *>(t.x) + first * n4 + li;
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
                 const long long off = in ? (long long)at * n4 + LP * c : 0;
                 const uint32_t dst = slot0 + (uint32_t)((((step % S) * U + k) * NC + c) * 2 * kPassThreads * 16);
                 copy16_async(dst, xb + off, in);
-                if (rows_out && o_aligned) copy16_async(dst + kPassThreads * 16, ob + off, in);
-                else if (rows_out) copy16_async_by4(dst + kPassThreads * 16, ob + off, in);
+                if (rows_out && O4) copy16_async_by4(dst + kPassThreads * 16, ob + off, in);
+                else if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
             }
         }
         copy_async_commit();
@@ -452,12 +452,14 @@ inline void pass_fill(PassArgs &a, float *dst, long long n) {
 // Both launches.  The tensors with an f32 source come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     long long blocks = 0, stats = 0;
+    bool o4 = false;
     a.n_stats = 0;
     for (int i = 0; i < a.n; ++i) {
         PassTensor &t = a.t[i];
         t.first = (int)blocks;
         blocks += (long long)t.batch * (t.heads / t.group) * t.slots;
         if (t.x) a.n_stats = i + 1, stats = blocks;
+        o4 |= (reinterpret_cast<uintptr_t>(t.o) & 15u) != 0;
     }
     a.fill_first[0] = (int)blocks;
     for (int f = 0; f < a.n_fill; ++f) {
@@ -471,8 +473,9 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     const auto both = [&](auto lanes, auto chunks) -> int {
         constexpr int LP = lanes.value, NC = chunks.value;
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
-        if (optin_smem((const void *)pass_stats_kernel<LP, NC>, smem)) return 1;
-        rc = launch_pdl("pass_stats_kernel", pass_stats_kernel<LP, NC>, gs, th, smem, stream, a);
+        const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
+        if (optin_smem((const void *)stats_kernel, smem)) return 1;
+        rc = launch_pdl("pass_stats_kernel", stats_kernel, gs, th, smem, stream, a);
         return rc ? rc : launch_pdl("pass_planes_kernel", pass_planes_kernel<LP, NC>, gp, th, 0, stream, a);
     };
     using std::integral_constant;
