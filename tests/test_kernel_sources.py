@@ -1,0 +1,46 @@
+"""Rules of the kernel sources that no run can be trusted to show."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "z-transformer_b200", "csrc")
+
+
+def sources():
+    return {f: open(os.path.join(CSRC, f)).read() for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh"))}
+
+
+def block(text, start):
+    """The brace-balanced body that opens after `start`."""
+    depth, i = 0, text.index("{", start)
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            return text[i:j + 1]
+    raise AssertionError("unbalanced")
+
+
+def kernels():
+    for name, text in sources().items():
+        for m in re.finditer(r"__global__ void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\s*\(([^;{]*?)\)\s*\{", text):
+            yield name, m[1], m[2], block(text, m.start())
+
+
+def test_overlapped_kernels_read_their_predecessors_results_with_plain_loads():
+    """A kernel that calls pdl_wait() is resident while the launch before it still writes.  Loads through the read-only path
+    may be moved ahead of the wait, so such kernels take no const __restrict__ pointer, and __ldg only reads what is at
+    least two launches old: the caller's tensors, the rope table, kept planes, and in the attention kernels (behind
+    both launches of the pre-pass) the first launch's row sums."""
+    overlapped = [(f, name, args, body) for f, name, args, body in kernels() if "pdl_wait()" in body]
+    assert len(overlapped) >= 12
+    older = {"reinterpret_cast<const uint2 *>(src", "reinterpret_cast<const float4 *>(t.x + at[k] * a.dim", "src + ch", "src + h4 + ch",
+             "cs", "cs + 1", "p.lse", "p.delta", "p.rnorm"}
+    for f, name, args, body in overlapped:
+        assert not re.search(r"const [\w ]*\*\s*__restrict__", args), name
+        for operand in re.findall(r"__ldg\(((?:[^()]|\([^()]*\))*)", body):
+            assert any(operand.strip().startswith(o) for o in older), (name, operand)
+        if f == "prepass.cuh":
+            assert "__ldg(p.rnorm" not in body and "__ldg(t.rnorm" not in body, name
+    # helpers of these kernels: V's planes come from the launch just before
+    assert "__ldg" not in block(sources()["tc_bwd.cuh"], sources()["tc_bwd.cuh"].index("void row_to_tmem16("))

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     PassTops tops{};
     const auto row_rel = [&](long long at) -> float {
         float cq, rel;
-        ds_row_scale(__ldg(t.rnorm + at), tops.dn, tops.vn, cq, rel);
+        ds_row_scale(t.rnorm[at], tops.dn, tops.vn, cq, rel);
         return rel;
     };
     // (the first units' loads go out before the maxima are waited for: many blocks have no second units)
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
             for (int k = 0; k < U; ++k) {
                 int r;
                 at[k] = locate(u0 + k * NG + gi, r);
-                rn[k] = __ldg(t.rnorm + (at[k] < 0 ? 0 : at[k]));
+                rn[k] = t.rnorm[at[k] < 0 ? 0 : at[k]];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const int col = (li + LP * c) * 4;

@@ -191,13 +191,14 @@ __host__ __device__ constexpr size_t kv_smem_bytes() {
 }
 
 // 16 packed-half words of one row from global memory into TMEM columns [taddr, taddr + 16).
-// (`chunks`: how many of the four 16-byte chunks are the row's; zeros beyond)
+// (`chunks`: how many of the four 16-byte chunks are the row's; zeros beyond.  Plain loads: the launch before may have
+// written the row, see pdl_wait.)
 __device__ __forceinline__ void row_to_tmem16(const __half *src, int chunks, uint32_t taddr) {
     uint32_t r[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (i / 4 < chunks) v = __ldg(reinterpret_cast<const uint4 *>(src) + i / 4);
+        if (i / 4 < chunks) v = *(reinterpret_cast<const uint4 *>(src) + i / 4);
         r[i] = v.x, r[i + 1] = v.y, r[i + 2] = v.z, r[i + 3] = v.w;
     }
     tmem_st16(taddr, r);

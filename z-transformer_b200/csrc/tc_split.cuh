@@ -105,9 +105,8 @@ inline size_t bwd_parts_floats_bound(int batch, int T, int n_heads, int dim) {
 }
 
 // out, lse <- the forward's parts.  A warp per (row, head).
-__global__ void __launch_bounds__(256) fwd_join_kernel(const float *__restrict__ part, const float *__restrict__ part_lse,
-                                                       float *__restrict__ out, float *__restrict__ lse, long long rows, int dim,
-                                                       int parts) {
+__global__ void __launch_bounds__(256) fwd_join_kernel(const float *part, const float *part_lse, float *out, float *lse, long long rows,
+                                                       int dim, int parts) {
     pdl_wait();
     pdl_launch();
     const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -141,8 +140,8 @@ inline int launch_fwd_join(const float *part, const float *part_lse, float *out,
 
 // dk, dv <- the backward's parts, each [2][batch][T][width] (dk, then dv).  A range of query tiles that lies before the
 // key tile wrote nothing.
-__global__ void __launch_bounds__(256) bwd_join_kernel(const float *__restrict__ part, float *__restrict__ dk, float *__restrict__ dv,
-                                                       int batch, int T, int width, BwdParts parts) {
+__global__ void __launch_bounds__(256) bwd_join_kernel(const float *part, float *dk, float *dv, int batch, int T, int width,
+                                                       BwdParts parts) {
     pdl_wait();
     pdl_launch();
     const long long n4 = (long long)batch * T * width / 4;

@@ -94,7 +94,9 @@ inline void prof_end(int idx, const char *name, cudaStream_t stream) {
 // kernel launched this way calls pdl_wait() in every block before it touches global memory -- it returns once the
 // kernel before has completed and its writes are visible, so the stream's order is what it always was -- and
 // pdl_launch() as soon as its own successor may be set up.  On a chain of 5-10 us kernels this takes 1-2 us off
-// each gap.
+// each gap.  What the kernel before has written is read by plain loads only: __ldg, and pointers that are const and
+// __restrict__, promise that the data does not change while the kernel runs, which lets the compiler move them ahead of
+// the wait.  (Data of earlier launches is older than the kernel: the one before lets it be set up only after its own wait.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
