@@ -44,3 +44,14 @@ def test_overlapped_kernels_read_their_predecessors_results_with_plain_loads():
             assert "__ldg(p.rnorm" not in body and "__ldg(t.rnorm" not in body, name
     # helpers of these kernels: V's planes come from the launch just before
     assert "__ldg" not in block(sources()["tc_bwd.cuh"], sources()["tc_bwd.cuh"].index("void row_to_tmem16("))
+
+
+def test_aligned_cluster_barriers_are_reached_by_whole_warps():
+    """barrier.cluster.*.aligned wants all threads of a warp to execute it together; code before it may end in one thread."""
+    n = 0
+    for name, text in sources().items():
+        for m in re.finditer(r"barrier\.cluster\.(?:arrive|wait)[.\w]*\.aligned", text):
+            body = text[text.rindex("__device__", 0, m.start()):m.start()]
+            assert "__syncwarp();" in body, (name, m[0])
+            n += 1
+    assert n == 2

@@ -49,7 +49,10 @@ __device__ __forceinline__ void cluster_arrive() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();  // (.aligned: the whole warp together, also where what lies before it was a single thread's)
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // A float of block `rank`'s shared memory, at the place that `addr` has in this block's.
 __device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
     float v;
