@@ -76,13 +76,15 @@ __device__ __forceinline__ void count_bad_sequences(const DecodeParams &p) {
 constexpr float kNoKey = -3.402823466e38f;  // the running maximum before the first key
 constexpr float kDecodeLazy = 8.f;          // a maximum moves when it is outgrown by 2^8
 
+// Blocks an SM holds, from a register estimate (q and accumulators: 8 floats per chunk per head).
+__host__ __device__ constexpr int decode_blocks_per_sm(int nch, int gp) { return gp * nch * 8 + 56 > 128 ? 1 : 2; }
+
 template <int LPK, int NCH, int GP>
 struct DecodeCfg {
     // Keys a lane group takes per step: at most as many (key, head) pairs as it has lanes, and 128 bytes a thread.
     static constexpr int kUnroll = (4 / NCH < 1 ? 1 : 4 / NCH) * GP > LPK ? LPK / GP : (4 / NCH < 1 ? 1 : 4 / NCH);
-    // Blocks per SM from a register estimate (q and accumulators: 8 floats per chunk per head), stages from what is left
-    // of shared memory (96 KB or 192 KB a block).
-    static constexpr int kMinBlocks = GP * NCH * 8 + 56 > 128 ? 1 : 2;
+    // Stages from what is left of shared memory (96 KB or 192 KB a block).
+    static constexpr int kMinBlocks = decode_blocks_per_sm(NCH, GP);
     static constexpr int kStageBytes = kDecodeThreads * kUnroll * NCH * 2 * 16;
     static constexpr int kFit = (kMinBlocks == 2 ? 96 : 192) * 1024 / kStageBytes;
     static constexpr int kStages = kFit > 8 ? 8 : kFit;
@@ -449,8 +451,8 @@ struct DecodePlan {
 
 // The split is a pure function of the shape and of the current device's SM count, so the
 // workspace-size query and the launch agree (both made with the same device current).  The
-// chunk is as large as keeps roughly four waves of blocks in flight (two blocks per SM),
-// between 128 and 1024 keys.  Without a device (a size query on a machine with none) the
+// chunk is as large as keeps roughly eight blocks an SM in the launch, between 128 and 1024
+// keys.  Without a device (a size query on a machine with none) the
 // count of a B200, 148, stands in.
 inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads, int dim) {
     DecodePlan pl{};
@@ -462,7 +464,8 @@ inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads,
     pl.nch = (chunks4 + pl.lpk - 1) / pl.lpk;
     const long long units = (long long)batch * n_kv_heads * pl.n_sub;
     const DeviceInfo *di = device_info();
-    const long long target_blocks = 4LL * 2 * (di && di->sm_count > 0 ? di->sm_count : 148);
+    const int sms = di && di->sm_count > 0 ? di->sm_count : 148;
+    const long long target_blocks = 8LL * sms;
     long long want = (target_blocks + units - 1) / units;
     if (want < 1) want = 1;
     long long chunk = (n_ctx + want - 1) / want;
@@ -471,14 +474,21 @@ inline DecodePlan decode_plan(int batch, int n_ctx, int n_heads, int n_kv_heads,
     if (chunk > 1024) chunk = 1024;
     pl.chunk = (int)chunk;
     pl.max_chunks = (n_ctx + pl.chunk - 1) / pl.chunk;
-    // One launch where clusters of at most eight blocks find an SM slot each at once (two blocks an SM) and a block's
-    // share stays below 768 keys; 32/8 heads of 128, us a call: one sequence, 512 keys 6.9 against 12.9, 2048 keys 11.1
+    // One launch where clusters of at most eight blocks find an SM slot each at once and a block's share stays below 768
+    // keys; 32/8 heads of 128, us a call: one sequence, 512 keys 6.9 against 12.9, 2048 keys 11.1
     // against 18.4, 8192 keys 39.4 against 35.6; four sequences, 2048 keys 19.4 against 30.7; sixteen (a second wave of
     // clusters), 512 keys 34.0 against 27.5.  (Clusters of sixteen start late: 36.7 where eight take 19.4.)
-    const long long slots = target_blocks / 4;
-    long long cs = 1;
-    while (cs < kMaxCluster && 2 * cs * units <= slots && n_ctx > 64 * cs) cs *= 2;
-    pl.cluster = (cs * units <= slots && n_ctx <= 768 * cs) ? (int)cs : 0;
+    // Where an SM holds one block only, clusters of up to two waves serve what one wave's share is too long for: 32/8 heads
+    // of 256, four sequences of 4096 keys 75 against 93, sixteen of 1024 keys 56 against 75.  What fits one wave is better
+    // off with it: four of 1024 keys 16.8 in one wave, 33.2 in two; eight of 256 keys 12.4 and 17.3.
+    const int per_sm = decode_blocks_per_sm(pl.nch, pl.gp);
+    const auto clusters_in = [&](long long slots) -> int {
+        long long cs = 1;
+        while (cs < kMaxCluster && 2 * cs * units <= slots && n_ctx > 64 * cs) cs *= 2;
+        return cs * units <= slots && n_ctx <= 768 * cs ? (int)cs : 0;
+    };
+    pl.cluster = clusters_in((long long)per_sm * sms);
+    if (pl.cluster == 0 && per_sm == 1) pl.cluster = clusters_in(2LL * sms);
     pl.ml_bytes = (size_t)batch * n_heads * pl.max_chunks * sizeof(float2);
     pl.ml_bytes = (pl.ml_bytes + 255) / 256 * 256;
     pl.acc_bytes = (size_t)batch * n_heads * pl.max_chunks * dim * sizeof(float);
