@@ -148,3 +148,14 @@ def test_backward_takes_an_output_on_a_four_byte_boundary(zt, B, T, H, Hkv, D):
         for name, a, b in zip(("dq", "dk", "dv"), got, want):
             # two orders of at most ten f32 additions
             assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max()), name
+
+
+def test_a_flag_whose_truth_raises(zt):
+    """want_lse is asked for its truth in native code: what it raises is what the caller sees."""
+    q, k, v = (torch.randn((1, 40, w * 32), device="cuda") for w in (2, 1, 1))
+    both = np.array([True, False])
+    with pytest.raises(ValueError):
+        zt.attention_forward(q, k, v, 2, 1, 32, want_lse=both)
+    nk = torch.full((1,), 40, dtype=torch.int32, device="cuda")
+    with pytest.raises(ValueError):
+        zt.decode_attention(q[:, 0].contiguous(), k, v, nk, 2, 1, 32, workspace=zt.DecodeWorkspace(1, 40, 2, 1, 32), want_lse=both)

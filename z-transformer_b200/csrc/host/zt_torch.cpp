@@ -98,10 +98,12 @@ PyObject *attention_forward(PyObject *, PyObject *const *args, Py_ssize_t n_args
     bool ok;
     void *keep = scratch(args[7], keep_bytes, *s.q, &ok);
     if (!ok) return none();
+    const int want_lse = PyObject_IsTrue(args[6]);
+    if (want_lse < 0) return nullptr;
     const bool keeps = args[7] != Py_None;
     const c10::cuda::CUDAGuard guard(s.q->device());
     const at::Tensor out = at::empty(s.q->sizes(), s.q->options());
-    const at::Tensor lse = PyObject_IsTrue(args[6]) == 1 ? at::empty({s.B, s.T, s.H}, s.q->options()) : at::Tensor();
+    const at::Tensor lse = want_lse ? at::empty({s.B, s.T, s.H}, s.q->options()) : at::Tensor();
     unsigned long long token = 0;
     const zt_stream_t stream = stream_of(*s.q);
     const int rc = without_gil([&] {
@@ -231,9 +233,11 @@ PyObject *decode(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     bool ok;
     void *ws = scratch(args[7], bytes, *q, &ok);
     if (!ok || !ws) return none();
+    const int want_lse = PyObject_IsTrue(args[10]);
+    if (want_lse < 0) return nullptr;
     const c10::cuda::CUDAGuard guard(q->device());
     const at::Tensor out = given ? *given : at::empty(q->sizes(), q->options());
-    const at::Tensor lse = PyObject_IsTrue(args[10]) == 1 ? at::empty({B, (int64_t)H}, q->options()) : at::Tensor();
+    const at::Tensor lse = want_lse ? at::empty({B, (int64_t)H}, q->options()) : at::Tensor();
     const zt_stream_t stream = stream_of(*q);
     const int rc = without_gil([&] {
         return zt_attn_decode(in(q), in(k), in(v), nk->const_data_ptr<int>(), out_of(out), lse.defined() ? out_of(lse) : nullptr, ws, bytes,
