@@ -266,7 +266,8 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
  *                     weightGrad accumulates into the layer's gradient (:958-972) -- zero it for a fresh one.
  * Both take a caller workspace of zt_proj_workspace_bytes(batch, T, k, n) bytes (256-byte aligned) and allocate
  * nothing.  Refusals: batch or T < 1; k or n not a multiple of 64 (there is no CUDA-core form of these calls);
- * a missing, short or misaligned workspace; a device that is not sm_100. */
+ * a missing, short or misaligned workspace; a tensor that does not start on a 16-byte boundary; a device that
+ * is not sm_100. */
 size_t zt_proj_workspace_bytes(int batch, int T, int k, int n);
 int zt_proj_forward(const float *ctx, const float *wo, float *y, void *workspace, size_t workspace_bytes, int batch,
                     int T, int k, int n, zt_stream_t stream);

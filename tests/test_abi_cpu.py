@@ -144,6 +144,22 @@ def test_reserving_a_shape_covers_every_shorter_one(zt, H, Hkv, D):
     assert L.zt_attn_reserve_bytes(1, 0, H, Hkv, D) == 0 and L.zt_attn_reserve_bytes(1, 64, H, Hkv, 31) == 0
 
 
+def test_projection_refuses_tensors_off_a_sixteen_byte_boundary(zt):
+    """Its kernels read and write four floats at a time: refused on the host, whichever tensor it is."""
+    L = zt.lib.load()
+    L.zt_attn_set_verbose(0)
+    room = 1 << 30
+    for bad in range(3):
+        t = [4096 + 4 * (i == bad) for i in range(3)]
+        assert L.zt_proj_forward(*t, 4096, room, 1, 8, 64, 64, None) == 1 and "16-byte" in zt.lib.last_error()
+        assert L.zt_attn_block_forward(4096, 4096, 4096, t[1], t[0], 4096, t[2], 4096, room, 4096, room, 1, 8, 2, 1, 32, 64, 0, 10000.0, None,
+                                       None) == 1 and "16-byte" in zt.lib.last_error()
+    for bad in range(5):
+        t = [4096 + 8 * (i == bad) for i in range(5)]
+        assert L.zt_proj_backward(*t, 4096, room, 1, 8, 64, 64, None) == 1 and "16-byte" in zt.lib.last_error()
+    L.zt_attn_set_verbose(1)
+
+
 def test_no_cpu_fallback_without_a_device(zt):
     """A well-formed call on a machine without a GPU is refused, never computed on the host."""
     import torch

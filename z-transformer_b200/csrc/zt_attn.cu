@@ -24,6 +24,7 @@
 #include "tc_bwd_fused.cuh"
 #endif
 
+#include <initializer_list>
 #include <mutex>
 
 namespace zt {
@@ -880,7 +881,7 @@ ProjWorkspace proj_workspace(void *base, int batch, int T, int k, int n) {
     w.total_bytes = off;
     return w;
 }
-int check_proj(const void *workspace, size_t workspace_bytes, int batch, int T, int k, int n) {
+int check_proj(std::initializer_list<const void *> tensors, const void *workspace, size_t workspace_bytes, int batch, int T, int k, int n) {
     if (batch < 1 || batch > 65535) return refuse("batch %d is not launchable (1 .. 65535).", batch);
     if (T < 1) return refuse("T %d is not launchable.", T);
     if (k < 64 || n < 64 || k % 64 != 0 || n % 64 != 0)
@@ -890,6 +891,8 @@ int check_proj(const void *workspace, size_t workspace_bytes, int batch, int T, 
     if (!workspace || workspace_bytes < need)
         return refuse("the projection needs %zu bytes of workspace, %zu were given.", need, workspace_bytes);
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return refuse("the projection workspace must be 256-byte aligned.");
+    for (const void *t : tensors)  // (read and written four floats at a time)
+        if (!aligned16(t)) return refuse("the projection's tensors must be 16-byte aligned.");
     if (need_device()) return 1;
 #ifdef ZT_NO_TC
     return refuse("this build has no tensor-core kernels.");
@@ -957,7 +960,7 @@ int zt_proj_forward(const float *ctx, const float *w, float *y, void *workspace,
                     int k, int n, zt_stream_t stream) {
     g_last_error[0] = 0;
     if (!ctx || !w || !y) return refuse("a null device pointer was passed.");
-    if (check_proj(workspace, workspace_bytes, batch, T, k, n)) return 1;
+    if (check_proj({ctx, w, y}, workspace, workspace_bytes, batch, T, k, n)) return 1;
     return proj_forward_impl(ctx, w, y, workspace, batch, T, k, n, (cudaStream_t)stream, nullptr, 0);
 }
 
@@ -971,7 +974,7 @@ int zt_attn_block_forward(const float *q, const float *k, const float *v, const 
     if (batch < 1 || batch > 65535) return refuse("batch %d is not launchable (1 .. 65535).", batch);
     if (check_geometry(T, n_heads, n_kv_heads, dim)) return 1;
     const int kdim = n_heads * dim;
-    if (check_proj(proj_workspace_, proj_workspace_bytes, batch, T, kdim, d_model)) return 1;
+    if (check_proj({ctx, wo, y}, proj_workspace_, proj_workspace_bytes, batch, T, kdim, d_model)) return 1;
     cudaStream_t s = (cudaStream_t)stream;
 #ifndef ZT_NO_TC
     const ProjWorkspace pw = proj_workspace(proj_workspace_, batch, T, kdim, d_model);
@@ -995,7 +998,7 @@ int zt_proj_backward(const float *ctx, const float *w, const float *dy, float *d
                      size_t workspace_bytes, int batch, int T, int k, int n, zt_stream_t stream) {
     g_last_error[0] = 0;
     if (!ctx || !w || !dy || !dctx || !dw) return refuse("a null device pointer was passed.");
-    if (check_proj(workspace, workspace_bytes, batch, T, k, n)) return 1;
+    if (check_proj({ctx, w, dy, dctx, dw}, workspace, workspace_bytes, batch, T, k, n)) return 1;
 #ifndef ZT_NO_TC
     cudaStream_t s = (cudaStream_t)stream;
     const ProjWorkspace ws = proj_workspace(workspace, batch, T, k, n);
