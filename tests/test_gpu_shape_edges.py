@@ -159,3 +159,81 @@ def test_a_flag_whose_truth_raises(zt):
     nk = torch.full((1,), 40, dtype=torch.int32, device="cuda")
     with pytest.raises(ValueError):
         zt.decode_attention(q[:, 0].contiguous(), k, v, nk, 2, 1, 32, workspace=zt.DecodeWorkspace(1, 40, 2, 1, 32), want_lse=both)
+
+
+@pytest.mark.parametrize("path,T,q_offset,H,Hkv,D", [
+    # two heads a block, whose row sums leave the accumulator on the way: forced, the planes as wide as the tile and narrower
+    (7, 129, 2900, 2, 1, 128), (7, 300, 2100, 4, 1, 72), (7, 70, 1500, 4, 2, 64), (7, 33, 5, 2, 1, 96),
+    # and where enough blocks make it the default
+    (0, 1200, 1100, 32, 8, 64),
+])
+def test_windows_two_heads_a_block(zt, oracle, path, T, q_offset, H, Hkv, D):
+    n_keys = q_offset + T
+    q = normal(oracle, (T, H * D), 0)
+    k, v = (normal(oracle, (n_keys, Hkv * D), i) for i in (1, 2))
+    holder = zt.Attn(n_keys, H, Hkv, D)
+    for name, x in (("q", q), ("k", k), ("v", v)):
+        holder.upload(getattr(holder, name), x)
+    L = zt.lib.load()
+    L.zt_attn_set_path(path)
+    try:
+        L.zt_attn_profile(1)
+        holder.forward_at(1, 64, q_offset, n_keys, T)
+        torch.cuda.synchronize()
+        names = kernels_timed(zt)
+    finally:
+        L.zt_attn_profile(0)
+        L.zt_attn_set_path(0)
+    assert "attn_fwd_tc16g" in names and zt.lib.tc_status() == 0
+    ref = oracle.attention_forward_at(q, k, v, H, Hkv, D, q_offset, n_keys, threads=8)
+    got = holder.out[: q.size].view(q.shape)
+    close(got, ref, "window")
+    assert float(np.linalg.norm(got.cpu().numpy() - ref) / np.linalg.norm(ref)) <= 5e-6
+
+
+def kernels_timed(zt):
+    """Names of the kernels timed since zt_attn_profile(1)."""
+    import ctypes
+    buf = ctypes.create_string_buffer(4096)
+    zt.lib.load().zt_attn_profile_read(buf, 4096)
+    return {line.split()[0] for line in buf.value.decode().splitlines()}
+
+
+@pytest.mark.parametrize("D", [160, 192, 256])
+def test_wide_heads_tile_by_tile(zt, oracle, D):
+    """More blocks than SMs and at most twice as many, odd numbers of heads and tiles: the wide forward goes tile by tile."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    T, H, Hkv = 260, 9, 3  # 27 blocks a sequence
+    B = sms // 27 + 2
+    assert sms < 27 * B <= 2 * sms
+    q, k, v = (normal(oracle, (B, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv)))
+    o, lse = zt.attention_forward(*(torch.from_numpy(x).cuda() for x in (q, k, v)), H, Hkv, D, want_lse=True)
+    torch.cuda.synchronize()
+    assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0
+    for b in range(B):
+        ro, rl = oracle.attention_forward(q[b], k[b], v[b], H, Hkv, D, want_lse=True, threads=8)
+        close(o[b], ro, f"out[{b}]"), close(lse[b], rl, f"lse[{b}]")
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D", [(2, 70, 4, 2, 40), (1, 200, 2, 1, 80), (1, 150, 3, 1, 96), (1, 33, 2, 2, 100), (2, 129, 4, 2, 160),
+                                         (1, 260, 2, 1, 192), (1, 90, 2, 1, 252)])
+def test_earlier_backward_forms_at_widths_between_the_tiles(zt, oracle, B, T, H, Hkv, D):
+    """zt_attn_set_path(8): the two-kernel backward, and the scores that load every operand per tile, on padded heads."""
+    q, k, v, do = (normal(oracle, (B, T, w * D), i) for i, w in enumerate((H, Hkv, Hkv, H)))
+    tq, tk, tv, tdo = (torch.from_numpy(x).cuda() for x in (q, k, v, do))
+    L = zt.lib.load()
+    L.zt_attn_set_path(8)
+    try:
+        o, lse = zt.attention_forward(tq, tk, tv, H, Hkv, D, want_lse=True)
+        L.zt_attn_profile(1)
+        grads = zt.attention_backward(tq, tk, tv, o, lse, tdo, H, Hkv, D)
+        torch.cuda.synchronize()
+        names = kernels_timed(zt)
+    finally:
+        L.zt_attn_profile(0)
+        L.zt_attn_set_path(0)
+    assert ("attn_bwd_dq_tc" if D <= 128 else "bwd_wide_scores") in names and zt.lib.tc_status() == 0
+    for b in range(B):
+        ref = oracle.attention_backward(q[b], k[b], v[b], do[b], H, Hkv, D, threads=4)
+        for name, got, want in zip(("dq", "dk", "dv"), grads, ref):
+            close(got[b], want, f"{name}[{b}]")
