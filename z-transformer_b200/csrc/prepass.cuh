@@ -130,15 +130,15 @@ __device__ __forceinline__ PassUnit pass_locate(const PassArgs &a, int n, int bl
     return w;
 }
 
-// LP lanes hold a unit, NC float4 each.  The loads run kStages - 1 steps of U units ahead through slots of shared memory
+// LP lanes hold a unit, NC float4 each.  The loads run kStatsStages - 1 units ahead through slots of shared memory
 // that belong to one thread each (so nothing but the thread's own copies is waited for): held in registers instead,
 // the loads of a step would stall on the arithmetic of the step before (heads of 256, batch 8, T 1024: 4.1 TB/s against 5.4).
 // O4: the tensor that dout is multiplied with starts on a 4-byte boundary only (of a call's tensors it alone may, because
 // nothing but its row sums is wanted).  A variant of its own: asked per copy it cost every backward 0.4 us.
 template <int LP, int NC, bool O4>
 __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_constant__ PassArgs a) {
-    constexpr int NG = kPassThreads / LP, U = 1, S = kStatsStages;
-    extern __shared__ __align__(16) float4 ring[];  // [S][U][NC][2][kPassThreads]
+    constexpr int NG = kPassThreads / LP, S = kStatsStages;
+    extern __shared__ __align__(16) float4 ring[];  // [S][NC][2][kPassThreads]
     __shared__ float red[2][kPassThreads / 32];
     const PassUnit w = pass_locate(a, a.n_stats, (int)blockIdx.x);
     const PassTensor &t = a.t[w.z];
@@ -149,24 +149,21 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     const float4 *xb = reinterpret_cast<const float4 *>(t.x) + first * n4 + li;
     const float4 *ob = reinterpret_cast<const float4 *>(rows_out ? t.o : t.x) + first * n4 + li;
     const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(ring + threadIdx.x);
-    const int stride = t.slots * NG * U, n_steps = (w.units - w.slot * NG * U + stride - 1) / stride;
-    const auto place = [&](int step, int k) -> int {  // the unit's index within the (sequence, group), or -1
-        const int u = step * stride + (w.slot * U + k) * NG + gi;
+    const int stride = t.slots * NG, n_steps = (w.units - w.slot * NG + stride - 1) / stride;
+    const auto place = [&](int step) -> int {  // the unit's index within the (sequence, group), or -1
+        const int u = step * stride + w.slot * NG + gi;
         return u < w.units ? (u / group) * (heads - group) + u : -1;  // r heads + (u - r group)
     };
     const auto fetch = [&](int step) {
+        const int at = place(step);
 #pragma unroll
-        for (int k = 0; k < U; ++k) {
-            const int at = place(step, k);
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const bool in = step < n_steps && at >= 0 && li + LP * c < n4;
-                const long long off = in ? (long long)at * n4 + LP * c : 0;
-                const uint32_t dst = slot0 + (uint32_t)((((step % S) * U + k) * NC + c) * 2 * kPassThreads * 16);
-                copy16_async(dst, xb + off, in);
-                if (rows_out && O4) copy16_async_by4(dst + kPassThreads * 16, ob + off, in);
-                else if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
-            }
+        for (int c = 0; c < NC; ++c) {
+            const bool in = step < n_steps && at >= 0 && li + LP * c < n4;
+            const long long off = in ? (long long)at * n4 + LP * c : 0;
+            const uint32_t dst = slot0 + (uint32_t)(((step % S) * NC + c) * 2 * kPassThreads * 16);
+            copy16_async(dst, xb + off, in);
+            if (rows_out && O4) copy16_async_by4(dst + kPassThreads * 16, ob + off, in);
+            else if (rows_out) copy16_async(dst + kPassThreads * 16, ob + off, in);
         }
         copy_async_commit();
     };
@@ -177,38 +174,29 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     float amax = 0.f, nmax = 0.f;
     for (int step = 0; step < n_steps; ++step) {
         copy_async_wait<S - 2>();
-        float sq[U], de[U];
+        float sq = 0.f, de = 0.f;
 #pragma unroll
-        for (int k = 0; k < U; ++k) {
-            sq[k] = 0.f, de[k] = 0.f;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const float4 *at = ring + (((step % S) * U + k) * NC + c) * 2 * kPassThreads + threadIdx.x;
-                const float4 x = at[0];
-                amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-                sq[k] = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq[k]))));
-                if (rows_out) {
-                    const float4 o = at[kPassThreads];
-                    de[k] = fmaf(x.x, o.x, fmaf(x.y, o.y, fmaf(x.z, o.z, fmaf(x.w, o.w, de[k]))));
-                }
+        for (int c = 0; c < NC; ++c) {
+            const float4 *at = ring + ((step % S) * NC + c) * 2 * kPassThreads + threadIdx.x;
+            const float4 x = at[0];
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+            sq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq))));
+            if (rows_out) {
+                const float4 o = at[kPassThreads];
+                de = fmaf(x.x, o.x, fmaf(x.y, o.y, fmaf(x.z, o.z, fmaf(x.w, o.w, de))));
             }
         }
         fetch(step + S - 1);
         if (!norms) continue;
 #pragma unroll
-        for (int off = LP / 2; off > 0; off >>= 1)
-#pragma unroll
-            for (int k = 0; k < U; ++k) {
-                sq[k] += __shfl_xor_sync(0xffffffffu, sq[k], off);
-                if (rows_out) de[k] += __shfl_xor_sync(0xffffffffu, de[k], off);
-            }
-#pragma unroll
-        for (int k = 0; k < U; ++k) {
-            const float norm = sqrtf(sq[k]);
-            nmax = fmaxf(nmax, norm);
-            const int at = place(step, k);
-            if (rows_out && li == 0 && at >= 0) t.delta[first + at] = de[k], t.rnorm[first + at] = norm;
+        for (int off = LP / 2; off > 0; off >>= 1) {
+            sq += __shfl_xor_sync(0xffffffffu, sq, off);
+            if (rows_out) de += __shfl_xor_sync(0xffffffffu, de, off);
         }
+        const float norm = sqrtf(sq);
+        nmax = fmaxf(nmax, norm);
+        const int at = place(step);
+        if (rows_out && li == 0 && at >= 0) t.delta[first + at] = de, t.rnorm[first + at] = norm;
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {

@@ -38,7 +38,6 @@ using tcb::block_mult;
 using tcb::kDsBound;
 using tcb::ds_group_scale;
 using tcb::ds_row_scale;
-using tcb::pow2_for;
 using tcb::split_pack;
 
 constexpr int kStages = 3;

@@ -7,7 +7,6 @@
 // protocol mistake costs a wrong answer and a status word, never a hung GPU.
 #pragma once
 
-
 #include <cuda.h>
 #include <cuda_runtime.h>
 
