@@ -113,9 +113,9 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
  *    (work queued earlier may still be using it), so growth costs memory, never correctness;
  *  - zt_attn_reserve sizes it for a shape up front -- the place for it is where the reference's
  *    holder sizes its own eleven buffers (device.Attn.init, src/cuda/device.zig:221-299; that
- *    function already calls zt_attn_dim_ok); it makes the pool hold what windows take, too.  After zt_attn_reserve(batch, T, ...) no call of
- *    that shape, or of fewer rows or sequences with the same heads, allocates.  (No counterpart in the reference, whose kernels need
- *    no scratch.)
+ *    function already calls zt_attn_dim_ok); it makes the pool hold what windows take, too.  After
+ *    zt_attn_reserve(batch, T, ...) no call of that shape, or of fewer rows or sequences with the
+ *    same heads, allocates.  (No counterpart in the reference, whose kernels need no scratch.)
  *  - while `stream` is being captured into a CUDA graph a call that would have to grow the arena
  *    is refused (return 1) instead of allocating inside the capture: reserve first;
  *  - these calls share the arena: two of them must not overlap on the GPU (different streams or
@@ -124,9 +124,10 @@ int zt_attn_backward(const float *q, const float *k, const float *v, const float
  *    calls that take a caller workspace (_keep, backward_batched, _rope_, decode) do not touch it. */
 int zt_attn_reserve(int batch, int T, int n_heads, int n_kv_heads, int dim);
 /* The most scratch that a call of this shape, of a window of it, or of fewer rows or sequences takes: what
- * zt_attn_reserve makes the arena hold for whole sequences, where they use it (on the current device; without one, on a
- * B200).  At least zt_attn_backward_workspace_bytes of the shape and of every one with fewer rows or sequences: a shorter sequence can
- * use MORE scratch, because its work may be split into partial results where a longer one has blocks enough. */
+ * zt_attn_reserve makes the arena hold for whole sequences, where they use it (on the current device;
+ * without one, on a B200).  At least zt_attn_backward_workspace_bytes of the shape and of every one with
+ * fewer rows or sequences: a shorter sequence can use MORE scratch, because its work may be split into
+ * partial results where a longer one has blocks enough. */
 size_t zt_attn_reserve_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim);
 /* Bytes the current device's arena holds now (0 before its first use). */
 size_t zt_attn_arena_bytes(void);
@@ -171,7 +172,7 @@ int zt_attn_forward_batched(const float *q, const float *k, const float *v, floa
  * is refused, except for sequences under 128 rows and widths other than 32, 64, 96, 128, 192 and 256: these
  * run on the CUDA cores then (as all shapes do for which the query returns 0), NULL/0 included.
  * The workspace holds the 16-bit operand planes of q, k, v, dout;
- * at head_dim 192 and 256 it also holds the planes of P and dS of as many heads as fit in about 2 GiB
+ * above head_dim 128 it also holds the planes of P and dS of as many heads as fit in about 2 GiB
  * (at least one KV group's: 8 T^2 bytes a head), because the backward at those widths writes them to
  * memory between its launches; there dq, dk, dv are sums added in memory in no fixed order, equal run to
  * run to rounding only. */

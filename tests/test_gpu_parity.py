@@ -527,7 +527,7 @@ TC_BWD_WIDE_SHAPES = [  # B, T, H, Hkv, D, keep -- head_dim 256, and 192 zero-pa
 @pytest.mark.parametrize("B,T,H,Hkv,D,keep", TC_BWD_WIDE_SHAPES)
 def test_wide_head_backward_matches_oracle(zt, dev, oracle, B, T, H, Hkv, D, keep):
     """head_dim 192 and 256: P and dS go through memory as operand planes (bwd_wide_scores), dQ, dK, dV are three
-    products over them (gemm_tri).  With and without the planes of q, k, v that the forward leaves in the workspace."""
+    products over them (wide_products).  With and without the planes of q, k, v that the forward leaves in the workspace."""
     q = oracle.fill_normal((B, T, H * D), 61, 0)
     k = oracle.fill_normal((B, T, Hkv * D), 61, 1)
     v = oracle.fill_normal((B, T, Hkv * D), 61, 2)

@@ -8,14 +8,13 @@
 //   pass_planes_kernel   reads the slots of its (sequence, group) -- at most 1024 of them --, publishes the maxima for
 //                        the attention kernels, and writes the planes (rotating q and k on the way where rope is asked
 //                        for), the row-scaled copy of q's planes for dK, and the zeros of outputs that are summed in memory.
-// Both work on units, one head of one row, held by 8, 16 or 32 lanes; a lane has four units in flight.  A block's units
-// belong to one (sequence, group), of which its blocks take turns: blocks that run together read and write one stretch
-// of memory, not a stretch each (the first
-// pass at T 4096, heads of 128: 460 us, with the turns 417).  The split into blocks aims at 2048 blocks per tensor (14 an SM; 4096 and 1024 were
-// 1-2 % slower, 512 more) of at least eight units a lane group.
+// Both work on units, one head of one row, held by 8, 16 or 32 lanes.  A lane of the first launch has three units under way, of
+// the second four (two where it holds two or three chunks of one).  A block's units belong to one (sequence, group), of which its blocks take turns: blocks that run together read and write one stretch of memory, not a
+// stretch each (the first launch at T 4096, heads of 128: 460 us, with the turns 417).  The split into blocks is in pass_add.
 // Before (one kernel per quantity: two for the planes, one each for delta, v's norms, dout's norms, the row-scaled
-// copy, and up to four memsets; 13 launches a step where there are 6 now): batch 8, T 512, 32/8 heads of 64, forward
-// and backward, 175 us, now 115; T 1024, heads of 256, 740 us, now 540; T 4096, heads of 128, 1370 us, now 1270.
+// copy, and up to four memsets; 13 launches a step where there are 6 now), us a step: batch 8, T 512, 32/8 heads of 64, forward
+// and backward, 175, now 106; T 1024, heads of 256, 740, now 582; T 4096, heads of 128, 1370, now 1350 (all under the
+// step's clock, 1.5 GHz at the last).
 #pragma once
 
 #include <cuda_fp16.h>
@@ -425,8 +424,12 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
     t.x = x, t.batch = batch, t.rows = rows, t.heads = heads, t.group = group;
     t.part = part, t.amax = amax, t.nmax = nmax, t.planes = planes;
     const long long bg = (long long)batch * (heads / group), units = (long long)rows * group;
+    // 2048 blocks a tensor, 14 an SM (4096 and 1024 were 1-2 % slower, 512 more), of at least 256 units at 32 columns, 128 up
+    // to 64 and 64 beyond: eight units a lane group where 32 lanes hold one, two at 80 and 96 columns and four at 192, whose
+    // units are held by 8 and 16 lanes.  Eight there too is 1-2 % of a large step faster (8 sequences of 512, 16/4 heads of 96,
+    // 223 -> 220 us) and costs a small one up to a quarter (one of 500, 8/2 heads of 80, 69 -> 87).
     const int lanes = a.dim <= 32 ? 8 : (a.dim <= 64 ? 16 : 32);
-    const long long step = (long long)kPassThreads / lanes * 8;  // eight units a lane group at least
+    const long long step = (long long)kPassThreads / lanes * 8;
     long long slots = kPassTargetBlocks / bg;
     slots = slots > kPassMaxSlots ? kPassMaxSlots : (slots < 1 ? 1 : slots);
     const long long most = (units + step - 1) / step;

@@ -1,4 +1,4 @@
-// Causal GQA attention backward at head_dim 192 and 256 (132 ... 252 zero-padded to the next of them) on the tensor cores.
+// Causal GQA attention backward above head_dim 128, on tiles of 192 and 256 columns, on the tensor cores.
 //
 // What it computes: autograd.attentionBackward (src/autograd.zig:636-842) for a batch, as tc_bwd.cuh does:
 //     P = exp(S - lse),  dP = dO V^T,  dS = P (dP - delta),  dV = P^T dO,  dK = scale dS^T Q,  dQ = scale dS K

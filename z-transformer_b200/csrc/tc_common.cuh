@@ -333,18 +333,19 @@ __device__ __forceinline__ float tf32_round(float x) {
 // They have tiles of 64, 128, 192 and 256 columns; a head of any other width runs on the next wider tile, zeros beyond its
 // columns (tc::plane_dim), outputs keep their own width (rows leave in 16-byte chunks, hence the multiple of four).  What
 // the MMAs of the padding cost is bounded (tc::head_steps; an MMA of half the width costs the same clocks anyway), and what
-// it replaces is the CUDA-core
-// kernels at a thirtieth of the rate: head_dim 80, batch 4, T 1000, 16/4 heads, forward and backward 7.6 ms there,
-// 0.30 ms here.  192 columns lie between because 132 ... 192 padded to 256 paid a third more MMAs, plane bytes and
+// it replaces is the CUDA-core kernels at a thirtieth of the rate: head_dim 80, batch 4, T 1000, 16/4 heads, forward and
+// backward 7.6 ms there, 0.24 ms here.  192 columns lie between because 132 ... 192 padded to 256 paid a third more MMAs, plane bytes and
 // operand traffic for nothing: us on 256 -> on 192 columns, 16/4 heads of 192, forward and backward of batch 4, T 1024
 // 611 -> 526, forward of batch 4, T 2048 562 -> 486, a window of 512 rows at 3584 165 -> 128; 8/2 heads of 160,
 // batch 2, T 4096 1633 -> 1443.
 inline int tc_tile_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : (dim <= 192 ? 192 : 256)); }
 inline bool tc_takes_dim(int dim) { return dim % 4 == 0 && dim >= 32 && dim <= 256; }
-// Keys from which the forward goes to the tensor cores: up to 32 the CUDA-core forward is one launch of one row and one
-// key tile and the quicker of the two (32/8 heads of 128: 17 us against 28 at 32 rows, 29.5 against 28.5 at 48, 57
-// against 31 at 127; a key tile more costs it 13 us, however few the rows).  The backward has no such line: 47
-// against 111 us at 2 rows already.
+// Keys from which the forward goes to the tensor cores.  Up to 32 the CUDA-core forward is one launch of one row tile and one
+// key tile, needs no scratch, and is the quicker of the two for narrow heads and small batches: us there and on the tensor
+// cores at 32 rows, 4/2 heads of 32 8.5 and 11.7 (64 sequences 10.5 and 24.9), 8/2 of 64 12.5 and 14.4, 32/8 of 128 18.8
+// and 17.4 (8 sequences 26.9 and 32.9, 64 157 and 114), 16/4 of 256 31.1 and 23.5.  A key tile more costs it 13 us, however few the
+// rows: 32/8 heads of 128 take it 29.5 at 48 rows and 57 at 127, where 77 rows are 17.1 here.  The backward has no such line:
+// at 2 rows 32.5 us against 119 (32/8 heads of 128) and 16.9 against 34.1 (4/2 of 32).
 constexpr int kTcForwardMinKeys = 33;
 
 // Bytes of a caller's scratch: without which a call cannot run, with which it runs at its best, and the most that this shape

@@ -3,8 +3,9 @@
 // with the arithmetic of the attention kernels: f32 operands as f16 hi/lo planes times a power of two, every
 // product as three kind::f16 MMAs (hi.hi + hi.lo + lo.hi), f32 accumulation in TMEM.
 //
-// One kernel, gemm_f16split_tc<A_MN, B_MN>, C[M, N] = A . B over a contraction range, 128 x 128 output tiles,
-// 64-deep steps through a ring of three shared-memory stages (A and B tiles, hi and lo: 64 KB a stage):
+// C[M, N] = A . B over a contraction range, in 64-deep steps, by one of two kernels: gemm_f16split_tc<A_MN, B_MN>, a CTA per
+// 128 x 128 output tile and a ring of three shared-memory stages (A and B tiles, hi and lo: 64 KB a stage), and for
+// products that fill the chip gemm_f16split_wide<A_MN, B_MN> on 128 x 256 tiles (below):
 //   forward     y    = ctx . w        A = ctx planes, rows x K, K-major;      B = w planes, K x N, N-major
 //   inputGrad   dctx = dy . w^T       A = dy planes, rows x N, K-major;       B = w planes read as N x K^T, K-major
 //   weightGrad  dw  += ctx^T . dy     A = ctx planes read as K x rows^T, M-major; B = dy planes, rows x N, N-major
@@ -15,7 +16,7 @@
 // keeps that drift below the f32 rounding of the answer; weightGrad's contraction runs over the rows of ONE
 // sequence per piece, which is also what makes its scale uniform.
 // 6 warps: TMA producer, MMA issuer, four epilogue warps (a thread per output row; rows leave through shared
-// memory, a row per store instruction).  Every wait is bounded and raises g_tc_status when it gives up.
+// memory, a row per store instruction, or regrouped among eight lanes).  Every wait is bounded and raises g_tc_status when it gives up.
 #pragma once
 
 #include "tc_bwd.cuh"
