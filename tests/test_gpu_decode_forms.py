@@ -61,3 +61,27 @@ def test_clusters(zt, oracle, B, n_ctx, H, Hkv, D):
 def test_many_sequences_of_short_prefixes(zt, oracle):
     """More (sequence, KV head) pairs than places for clusters: two launches of few chunks each."""
     check(zt, oracle, 200, 16, 8, 64, [1 + (37 * i) % 200 for i in range(98)] + [0, 201], 2)
+
+
+def test_static_scratch_in_two_launches(zt, oracle):
+    """zt_attn_decode_static over the built-in scratch: the two-launch form's results and count, twice over its own leftovers."""
+    import ctypes
+    L = zt.lib.load()
+    H, Hkv, D = 4, 2, 64
+    n_keys = [LONG, 0, 129, 5000, LONG + 1, 1]
+    B = len(n_keys)
+    k, v = (torch.from_numpy(oracle.fill_normal((B, LONG, Hkv * D), 52, i)).cuda() for i in (1, 2))
+    nk = torch.tensor(n_keys, dtype=torch.int32, device="cuda")
+    for seed in (0, 3):
+        q = torch.from_numpy(oracle.fill_normal((B, H * D), 52, seed)).cuda()
+        want, want_lse = zt.decode_attention(q, k, v, nk, H, Hkv, D, workspace=zt.DecodeWorkspace(B, LONG, H, Hkv, D), want_lse=True)
+        out, lse = torch.full_like(q, 9.0), torch.full((B, H), 9.0, device="cuda")
+        before = zt.lib.launch_count()
+        assert L.zt_attn_decode_static(*(x.data_ptr() for x in (q, k, v, nk, out, lse)), B, LONG, H, Hkv, D,
+                                       torch.cuda.current_stream().cuda_stream) == 0, zt.lib.last_error()
+        assert zt.lib.launch_count() - before == 2
+        torch.cuda.synchronize()
+        bad = ctypes.c_int(-1)
+        assert L.zt_attn_decode_status(None, ctypes.byref(bad)) == 0 and bad.value == 2
+        for a, b in ((out, want), (lse, want_lse)):
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))

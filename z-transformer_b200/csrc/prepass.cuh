@@ -13,7 +13,7 @@
 // stretch each (the first launch at T 4096, heads of 128: 460 us, with the turns 417).  The split into blocks is in pass_add.
 // Before (one kernel per quantity: two for the planes, one each for delta, v's norms, dout's norms, the row-scaled
 // copy, and up to four memsets; 13 launches a step where there are 6 now), us a step: batch 8, T 512, 32/8 heads of 64, forward
-// and backward, 175, now 106; T 1024, heads of 256, 740, now 582; T 4096, heads of 128, 1370, now 1350 (all under the
+// and backward, 175, now 106; T 1024, heads of 256, 740, now 582; T 4096, heads of 128, 1370, now 1310-1350 (all under the
 // step's clock, 1.5 GHz at the last).
 #pragma once
 
