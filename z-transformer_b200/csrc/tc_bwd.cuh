@@ -102,7 +102,7 @@ struct BwdParams {
 //    walked head by head, and after each head the accumulators are added to dk/dv in memory
 //    (a rounded f32 add by the row threads) and restarted from zero, so no large partial sum
 //    sits in TMEM while further terms arrive.  The tiles beyond them are flushed every
-//    kFlushTiles query tiles for the same reason, which keeps the error flat in T.
+//    kFlushRows query rows for the same reason, which keeps the error flat in T.
 //    (Before the periodic flushes, with a flush only per head: 12-26 of 524288 dk/dv elements
 //    outside the tolerance at T = 4096; with them: none.)
 // The bound on dS.  dS leaves the row threads as a pair of f16 pieces, so it must stay inside the f16 range;
@@ -111,16 +111,17 @@ struct BwdParams {
 // arrived in dout from spreading through the accumulators of a whole CTA -- and a clamp that fires is counted
 // in g_tc_saturated (zt_attn_tc_saturated), which every test asserts to be zero.
 constexpr float kDsBound = 65000.f;
-constexpr int kFlushTiles = 8;  // query tiles of 64 rows between flushes (512 rows)
-constexpr int kDiagTiles = 2;   // query tiles that overlap a 128-key tile
-// An iterator: step `it` is (head hh of the group, query tile qi); `flush` says the accumulators are
+constexpr int kFlushRows = 512;  // query rows between flushes
+// An iterator: step `it` is (head hh of the group, query tile qi of ROWS rows); `flush` says the accumulators are
 // flushed after it, `fresh` that they restart from zero at it.  No divisions per step: every role of
 // the kernel walks it in lockstep.
-struct Walk {
+template <int ROWS>
+struct WalkOf {
+    static constexpr int kFlushTiles = kFlushRows / ROWS, kDiagTiles = 128 / ROWS;  // (the latter overlap a 128-key tile)
     int group, qi0, nd, na;  // nd diagonal tiles (<= kDiagTiles); na steps over the tiles beyond them
     int it, hh, qi, cnt;     // cnt: steps since the last flush, while it < na
     bool flush, fresh;
-    __device__ __forceinline__ Walk(int group_, int per_head, int qi0_, int n_q) : group(group_), qi0(qi0_) {
+    __device__ __forceinline__ WalkOf(int group_, int per_head, int qi0_, int n_q) : group(group_), qi0(qi0_) {
         nd = per_head < kDiagTiles ? per_head : kDiagTiles;
         na = (per_head - nd) * group;
         it = 0, hh = 0, cnt = 0;
@@ -148,6 +149,7 @@ struct Walk {
         set_flush();
     }
 };
+using Walk = WalkOf<64>;
 
 // ---------------------------------------------------------------------------------------------------
 // dK, dV.  grid (ceil(T / 128), n_kv_heads, batch), 576 threads: 16 row warps, a TMA warp, an MMA warp.
@@ -1082,7 +1084,7 @@ inline bool tc_bwd_supported(int batch, int T, int dim, const void *q, const voi
 }
 
 struct BwdMaps {
-    CUtensorMap k128, v128, q64, g64;   // dK/dV kernel: 128-key K and V tiles, 64-row Q and dO tiles
+    CUtensorMap k128, v128, q64, g64;   // dK/dV and fused kernels: 128-key K and V tiles, Q and dO tiles of a step's rows
     CUtensorMap k64, v64, q128, g128;   // dQ kernel: 64-key K and V tiles, 128-row Q and dO tiles
 };
 

@@ -1,5 +1,5 @@
-// The backward at tile widths 64 and 128 (every head_dim up to 128, padded to them) as ONE tensor-core kernel: dK, dV and dQ from one
-// computation of S^T and dP^T.
+// The backward at tile width 128 (head_dim 68 to 128, padded to it) as ONE tensor-core kernel: dK, dV and dQ from one
+// computation of S^T and dP^T.  (Narrower heads: tc_bwd_fused64.cuh.)
 //
 // tc_bwd.cuh computes S and dP twice: once in the dK/dV kernel (a CTA per 128 keys, query tiles walked) and
 // once in the dQ kernel (a CTA per 128 query rows, key tiles walked) -- 7 products issued for 5 credited.  Here
@@ -27,7 +27,7 @@
 //    sum_t (dS cq(t)) (Q / rel(t)) with one scale, dQ^T's column t leaves times 1 / cq(t).
 #pragma once
 
-#include "tc_bwd_wide.cuh"
+#include "tc_bwd_fused64.cuh"
 
 namespace zt {
 namespace tcf {
@@ -53,23 +53,19 @@ __device__ __forceinline__ void fgive_up(FusedShared *sh, int code) {
     sh->abort = code;
     atomicMax(&g_tc_status, code);
 }
-// K hi, K lo, V lo; dS hi + lo (32 KB); two Q slots and one dO slot (each 32 KB at head_dim 128)
-template <int D>
-__host__ __device__ constexpr size_t fused_smem_bytes() {
-    return 3 * (size_t)(128 * D * 2) + 2 * (size_t)(128 * 128) + 6 * (size_t)(64 * D * 2) + sizeof(FusedShared);
-}
+// K hi, K lo, V lo; dS hi + lo (32 KB); two Q slots and one dO slot (each 32 KB)
+constexpr size_t kFusedSmem = 3 * (size_t)(128 * 128 * 2) + 2 * (size_t)(128 * 128) + 6 * (size_t)(64 * 128 * 2) + sizeof(FusedShared);
 
 // grid (n_kv_heads, ceil(T / 128), batch), 608 threads: 16 row warps, a TMA warp, two MMA warps.
 constexpr int kFusedThreads = (kKvRowWarps + 3) * 32;
 // PARTS: the walk is split, or the blocks go tile by tile (tc_split.cuh).  A variant of its own: large launches are 1-2 % slower
 // with the code in it.
-template <int D, bool PARTS, bool PAD>
+template <bool PARTS, bool PAD>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     attn_bwd_fused_tc(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                       const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap gmap,
                       const BwdParams p) {
-    static_assert(D == 64 || D == 128, "tile widths of this kernel");
-    constexpr int NB = D / 64, W2 = D / 2, BQ = 64;
+    constexpr int D = 128, NB = D / 64, W2 = D / 2, BQ = 64;
     constexpr int KP = 128 * D * 2, QP = BQ * D * 2;  // bytes of one plane of a K tile / a query tile
     const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cVh = 0, cST = 64, cDPT = 128, cDQT = 192, cDV = 256, cDK = 256 + D;
@@ -280,12 +276,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             if (!ok) fgive_up(sh, 62);
             tc_fence_after();
             const uint64_t bvl = desc_kmajor(smem_u32(sVl));
-            // dQ^T's A operand is the K tile read M-major: M = the head's columns.  At 128 columns that is the two
-            // 64-column blocks of one plane (16 KB apart), and a product is the usual three terms.  At 64 columns M
-            // would be 64, half a tensor-core tile: instead the hi plane and the lo plane (KP apart) are read as ONE
-            // 128-row operand, so that accumulator rows 0..63 hold Kh^T dS and rows 64..127 Kl^T dS; with dS hi and
-            // dS lo as the two B operands that is all four terms in two MMAs, and the read-out adds the two halves.
-            const uint64_t mkh = desc_mnmajor_16b(smem_u32(sKh), D == 128 ? 128 * 128 : KP);
+            // dQ^T's A operand is the K tile read M-major: M = the head's columns, two 64-column blocks of one plane (16 KB apart)
+            const uint64_t mkh = desc_mnmajor_16b(smem_u32(sKh), 128 * 128);
             const uint64_t mkl = desc_mnmajor_16b(smem_u32(sKl), 128 * 128);
             const uint64_t mdh = desc_mnmajor_16b(smem_u32(sDS), DSP), mdl = desc_mnmajor_16b(smem_u32(sDS) + DSP, DSP);
             const uint32_t q_u32 = smem_u32(sQ), g_u32 = smem_u32(sG);
@@ -316,7 +308,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                     const uint64_t ddh = desc_advance(mdh, kk * 2048), ddl = desc_advance(mdl, kk * 2048);
                     mma_ss_f16(tmem + cDQT, dkh, ddh, id_q, kk > 0);
                     mma_ss_f16(tmem + cDQT, dkh, ddl, id_q, 1);
-                    if (D == 128) mma_ss_f16(tmem + cDQT, dkl, ddh, id_q, 1);
+                    mma_ss_f16(tmem + cDQT, dkl, ddh, id_q, 1);
                 }
             };
             int n_flush = 0;
@@ -487,8 +479,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 }
             }
             // now r[4 q4 + e] = dQ^T[head column 4 (lane / 4) + e of this warp's 32][query row 16 set + 4 q4 + (lane & 3)]
-            // (at 64 columns the accumulator's rows 64..127 are the K lo half of the same columns: both halves add)
-            const int d0 = ((warp & 3) * 32 + (lane & ~3)) & (D - 1);
+            const int d0 = (warp & 3) * 32 + (lane & ~3);
             if (d0 < p.dim_out) {
                 const long long wq = (long long)p.n_heads * p.dim_out;
 #pragma unroll
@@ -638,21 +629,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     if (warp == kKvRowWarps + 1) tmem_dealloc(tmem, 512);
 }
 
-template <int D>
-inline int launch_bwd_fused_d(const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
-                              const BwdParams &p, cudaStream_t stream) {
-    size_t smem = fused_smem_bytes<D>();
-    if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: it allocates all of TMEM
-    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused_tc<D, parts.value, pad.value>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < D / 16);
-    if (optin_smem((const void *)kernel, smem)) return 1;
+inline int launch_bwd_fused(const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
+                            const BwdParams &p, cudaStream_t stream) {
+    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused_tc<parts.value, pad.value>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < 8);
+    if (optin_smem((const void *)kernel, kFusedSmem)) return 1;
     const unsigned tiles = (unsigned)((p.T + 127) / 128), seqs = (unsigned)(p.batch * p.parts.n()), kv = (unsigned)p.n_kv_heads;
     const dim3 grid = p.by_tile ? dim3(kv, seqs, tiles) : dim3(kv, tiles, seqs);
-    return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), smem, stream, k128, v128, qs64, g64, p);
-}
-inline int launch_bwd_fused(int td, const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs64, const CUtensorMap &g64,
-                            const BwdParams &p, cudaStream_t stream) {
-    return td == 64 ? launch_bwd_fused_d<64>(k128, v128, qs64, g64, p, stream)
-                    : launch_bwd_fused_d<128>(k128, v128, qs64, g64, p, stream);
+    return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), kFusedSmem, stream, k128, v128, qs64, g64, p);
 }
 
 }  // namespace tcf
@@ -701,11 +684,12 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     }
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
     if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
+    const int rows = fused ? bwd_step_rows(dim) : 64;  // of a query tile
     BwdMaps m;
     bool maps = make_head_map(&m.k128, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
                 make_head_map(&m.v128, w.v_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
-                make_head_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, n_heads, dim, blocks, 64) &&
-                make_head_map(&m.g64, w.do_planes, 2 * batch, T, n_heads, dim, blocks, 64);
+                make_head_map(&m.q64, fused ? w.qs_planes : w.q_planes, 2 * batch, T, n_heads, dim, blocks, rows) &&
+                make_head_map(&m.g64, w.do_planes, 2 * batch, T, n_heads, dim, blocks, rows);
     if (!fused)
         maps = maps && make_head_map(&m.k64, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 64) &&
                make_head_map(&m.v64, w.v_planes, 2 * batch, T, n_kv_heads, dim, blocks, 64) &&
@@ -728,14 +712,15 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     p.p_scale = ldexpf(1.0f, 10);
     g_last_path = "tcgen05";
     if (fused) {
-        p.parts = bwd_parts(batch, T, n_heads, n_kv_heads);
+        p.parts = bwd_parts(batch, T, n_heads, n_kv_heads, dim);
         if (p.parts.n() > 1 && w.base_bytes + bwd_parts_floats(batch, T, n_heads, n_kv_heads, pd) * sizeof(float) > workspace_bytes) p.parts = BwdParts{1, 1};
         p.by_tile = tile_by_tile((long long)n_kv_heads * ((T + 127) / 128) * batch * p.parts.n(), kBwdTileWaves);
-        if (p.parts.n() == 1) return tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream);
+        const auto launch = td == 64 ? tcf::launch_bwd_fused64 : tcf::launch_bwd_fused;
+        if (p.parts.n() == 1) return launch(m.k128, m.v128, m.q64, m.g64, p, stream);
         const long long n = (long long)batch * T * n_kv_heads * dim;
         p.dk = w.parts, p.dv = w.parts + n, p.dkv_part = 2 * n;
-        if (tcf::launch_bwd_fused(td, m.k128, m.v128, m.q64, m.g64, p, stream)) return 1;
-        return launch_bwd_join(w.parts, dk, dv, batch, T, n_kv_heads * dim, p.parts, stream);
+        if (launch(m.k128, m.v128, m.q64, m.g64, p, stream)) return 1;
+        return launch_bwd_join(w.parts, dk, dv, batch, T, n_kv_heads * dim, p.parts, rows, stream);
     }
     return td == 64 ? launch_bwd_tc_d<64>(m, p, stream) : launch_bwd_tc_d<128>(m, p, stream);
 }

@@ -119,6 +119,22 @@ __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap *map, int c
                  "r"(c2), "r"(c3)
                  : "memory");
 }
+// A tile of this CTA's shared memory added to (tma_add_4d) or written over (tma_store_4d) a tensor in memory; what of the box
+// lies beyond the tensor is left out.  The source is read, and the tensor changed, some time after the call: see the two waits,
+// which are for the copies of the calling thread that tma_commit has closed a group of.
+__device__ __forceinline__ void tma_add_4d(const CUtensorMap *map, const void *src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(map),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, const void *src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(map), "r"(c0),
+                 "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // sources are free again
+__device__ __forceinline__ void tma_wait_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }       // the tensors have changed
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -425,6 +441,19 @@ inline bool make_head_map(CUtensorMap *map, const void *base, int planes, long l
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Tensor map over f32 rows of heads, [batch, rows, heads, dim], for tma_store_4d and tma_add_4d of 32 columns x box_rows rows
+// of one head (128-byte swizzle): what a head does not have of the columns is left out.  dim a multiple of four.
+inline bool make_out_map(CUtensorMap *map, float *base, long long batch, long long rows, int heads, int dim, int box_rows) {
+    PFN_encodeTiled enc = get_encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)dim, (cuuint64_t)heads, (cuuint64_t)rows, (cuuint64_t)batch};
+    const cuuint64_t strides[3] = {(cuuint64_t)dim * 4, (cuuint64_t)heads * dim * 4, (cuuint64_t)rows * heads * dim * 4};
+    const cuuint32_t box[4] = {32, 1, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace zt

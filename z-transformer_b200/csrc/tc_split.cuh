@@ -60,30 +60,36 @@ inline size_t fwd_parts_floats(int batch, int T, int n_heads, int dim, int q_off
     return n < 2 ? 0 : n * rows * ((q_offset > 0 ? 2 : 1) * (size_t)dim + 1);
 }
 
-// Parts of the backward's walk: heads x ranges of query tiles.  A step is a query tile of 64 rows of one head.
+// Parts of the backward's walk: heads x ranges of query tiles.  A step is a query tile of bwd_step_rows rows of one head.
+constexpr int bwd_step_rows(int dim) { return dim <= 64 ? 128 : 64; }
 struct BwdParts {
     int heads, ranges;
     __host__ __device__ int n() const { return heads * ranges; }
 };
-// The split with the shortest schedule, in steps: a launch ends with its longest block, or once all blocks' steps have been
-// shared out with half a block left over at the end (the walks are of all lengths, longest first); a block costs three
-// steps beside its walk, putting the parts together two and their traffic one per 45 blocks.  Parts keep four steps of
-// the longest walk, and a launch two blocks an SM (which bounds the partial results: 38 MB at most).
-inline BwdParts bwd_parts(int batch, int T, int n_heads, int n_kv_heads) {
-    const int group = n_heads / n_kv_heads, tiles = (T + 63) / 64, sms = split_sm_count();
+// The split with the shortest schedule, in steps (about 3 us each, 64 rows at 128 columns or 128 at 64): a launch ends with
+// its longest block, or once all blocks' steps have been shared out with half a block left over at the end (the walks are of
+// all lengths, longest first); a block costs three steps beside its walk (two at 64 columns, where several share an SM),
+// putting the parts together two and their traffic one per 45 blocks (at 64 columns, whose parts are half as large,
+// one and a half and one per 90).  Parts keep 256 rows of the longest walk, and a launch two blocks an SM (which bounds the
+// partial results: 38 MB at most).  At 64 columns, us a step unsplit / split as this does (heads x ranges): batch 4, T 1000, 16/4
+// heads 210 / 180 (2 x 1); one sequence, 32/8 heads, T 1000 180 / 122 (4 x 1), T 2048 332 / 246 (2 x 1); 8/2 heads, T 512 87 / 53 (4 x 2).
+inline BwdParts bwd_parts(int batch, int T, int n_heads, int n_kv_heads, int dim) {
+    const int rows = bwd_step_rows(dim), group = n_heads / n_kv_heads, tiles = (T + rows - 1) / rows, sms = split_sm_count();
     const long long key_tiles = (T + 127) / 128, ctas = n_kv_heads * key_tiles * batch;
-    const double walks = (double)group * (tiles * key_tiles - key_tiles * (key_tiles - 1)) * n_kv_heads * batch;  // all blocks' steps
+    const double walks = (double)group * (tiles * key_tiles - key_tiles * (key_tiles - 1) / 2 * (128 / rows)) * n_kv_heads * batch;  // all blocks' steps
+    const bool narrow = rows == 128;
+    const double block = narrow ? 2 : 3, join = narrow ? 1.5 : 2, traffic = narrow ? 90 : 45;
     BwdParts best{1, 1};
     if (ctas > 2 * sms) return best;
     double best_cost = 0.;
     for (int h = 1; h <= group; ++h) {
         if (group % h != 0) continue;
-        for (int r = 1; r == 1 || r <= tiles / 2; ++r) {
+        for (int r = 1; r == 1 || r * 128 <= tiles * rows; ++r) {
             const int n = h * r;
-            if (n > 1 && (n * ctas > 2 * sms || (long long)group * tiles < 4LL * n)) break;
-            const double longest = (double)(group / h) * ((tiles + r - 1) / r) + 3, shared = (walks + 3. * n * ctas) / sms + longest / 2;
+            if (n > 1 && (n * ctas > 2 * sms || (long long)group * tiles * rows < 256LL * n)) break;
+            const double longest = (double)(group / h) * ((tiles + r - 1) / r) + 3, shared = (walks + block * n * ctas) / sms + longest / 2;
             double cost = n * ctas <= sms || longest > shared ? longest : shared;
-            if (n > 1) cost += 2 + n * ctas / 45.;
+            if (n > 1) cost += join + n * ctas / traffic;
             // (of equals the split by heads: a part of a range also flushes its accumulators once per head)
             if ((h == 1 && r == 1) || cost <= best_cost) best = BwdParts{h, r}, best_cost = cost;
         }
@@ -91,7 +97,7 @@ inline BwdParts bwd_parts(int batch, int T, int n_heads, int n_kv_heads) {
     return best;
 }
 inline size_t bwd_parts_floats(int batch, int T, int n_heads, int n_kv_heads, int dim) {
-    const int n = bwd_parts(batch, T, n_heads, n_kv_heads).n();
+    const int n = bwd_parts(batch, T, n_heads, n_kv_heads, dim).n();
     return n < 2 ? 0 : (size_t)n * 2 * batch * T * n_kv_heads * dim;
 }
 
@@ -100,7 +106,7 @@ inline size_t bwd_parts_floats(int batch, int T, int n_heads, int n_kv_heads, in
 inline size_t fwd_parts_floats_bound(int dim) { return (size_t)split_sm_count() * 128 * (2 * (size_t)dim + 1); }
 inline size_t bwd_parts_floats_bound(int batch, int T, int n_heads, int dim) {
     const size_t by_blocks = (size_t)4 * split_sm_count() * 128 * dim;
-    const size_t by_steps = (size_t)n_heads * ((T + 63) / 64) / 4 * 2 * batch * T * dim;  // (a part keeps four steps)
+    const size_t by_steps = (size_t)n_heads * ((T + 63) / 64) / 4 * 2 * batch * T * dim;  // (a part keeps 256 rows)
     return by_steps < by_blocks ? by_steps : by_blocks;
 }
 
@@ -141,14 +147,14 @@ inline int launch_fwd_join(const float *part, const float *part_lse, float *out,
 // dk, dv <- the backward's parts, each [2][batch][T][width] (dk, then dv).  A range of query tiles that lies before the
 // key tile wrote nothing.
 __global__ void __launch_bounds__(256) bwd_join_kernel(const float *part, float *dk, float *dv, int batch, int T, int width,
-                                                       BwdParts parts) {
+                                                       BwdParts parts, int rows) {
     pdl_wait();
     pdl_launch();
     const long long n4 = (long long)batch * T * width / 4;
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= n4) return;
     const int t = (int)(i * 4 / width % T);
-    const int per_head = (T + 63) / 64 - t / 128 * 2, per = (per_head + parts.ranges - 1) / parts.ranges;
+    const int per_head = (T + rows - 1) / rows - t / 128 * (128 / rows), per = (per_head + parts.ranges - 1) / parts.ranges;
     const float4 *src = reinterpret_cast<const float4 *>(part);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     for (int s = 0; s < parts.n(); ++s) {
@@ -159,10 +165,10 @@ __global__ void __launch_bounds__(256) bwd_join_kernel(const float *part, float 
     }
     reinterpret_cast<float4 *>(dk)[i] = a, reinterpret_cast<float4 *>(dv)[i] = b;
 }
-inline int launch_bwd_join(const float *part, float *dk, float *dv, int batch, int T, int width, BwdParts parts, cudaStream_t stream) {
+inline int launch_bwd_join(const float *part, float *dk, float *dv, int batch, int T, int width, BwdParts parts, int rows, cudaStream_t stream) {
     const long long n4 = (long long)batch * T * width / 4;
     return launch_pdl("bwd_join_kernel", bwd_join_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, part, dk, dv, batch, T,
-                      width, parts);
+                      width, parts, rows);
 }
 
 }  // namespace zt
