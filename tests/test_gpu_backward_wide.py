@@ -1,0 +1,27 @@
+"""The backward of heads above 128 columns against float64, where a tile of a product is one unit (up to 1024 keys; dQ is stored) and
+where it is several (added to a zeroed dq): lengths around the tiles and that line, odd numbers of heads, padded heads.  Tolerance in
+the 2-norm, as in the 64-column backward's test: 6e-7 for the operands, 4e-8 for each addition to a truncating accumulator: at most 48
+of a score's contraction and 192 of a product's piece."""
+import pytest
+import torch
+
+from test_gpu_backward64 import gradients
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [
+    (1, 64, 2, 1, 256), (1, 128, 4, 4, 192), (3, 129, 3, 1, 160), (2, 700, 6, 2, 132), (1, 1000, 4, 1, 256), (5, 1024, 3, 3, 256),
+    (1, 1025, 4, 2, 192), (2, 1300, 3, 1, 256),
+])
+def test_gradients_against_float64(zt, B, T, H, G, D):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(13)
+    q, k, v, do = (torch.randn((B, T, w * D), device="cuda", generator=gen) for w in (H, G, G, H))
+    ws = zt.BackwardWorkspace(B, T, H, G, D)
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    got = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=ws.token != 0)
+    torch.cuda.synchronize()
+    assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+    for name, x, ref in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
+        assert float((x.double() - ref).norm()) <= (6e-7 + 4e-8 * 240) * float(ref.norm()), name

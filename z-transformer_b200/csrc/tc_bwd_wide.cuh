@@ -44,6 +44,7 @@ constexpr int kStages = 3;
 constexpr int kTB = 128 * 64 * 2;  // bytes of one plane of an operand tile
 constexpr int kSB = 4 * kTB;       // a stage: A hi, A lo, B hi, B lo
 constexpr int kScoreThreads = 10 * 32;  // TMA producer, MMA issuer, eight epilogue warps
+constexpr int kResThreads = 18 * 32;    // TMA producer, MMA issuer, sixteen row warps
 constexpr int kTriThreads = 6 * 32;     // TMA producer, MMA issuer, four epilogue warps
 constexpr int kPiece = 1024;            // contraction depth of one unit of wide_products
 
@@ -263,11 +264,14 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
 // 64 columns, hi and lo: 32 KB) through a ring of three; per key tile, S (4 blocks x 12 MMAs of N = 128) into one
 // 128-column accumulator, then dP into the other.  Against bwd_wide_scores every operand byte of the query side
 // is loaded once per CTA instead of once per tile: half the traffic from L2, which is what bounds both.
-// The eight epilogue warps read S as soon as it is complete (P, kept in registers, goes to memory while dP's
+// The sixteen row warps, a thread per query row and 32 of the tile's keys, read S as soon as it is complete (P, kept in registers, goes to memory while dP's
 // MMAs run), then dP (dS goes out while the next tile's S runs): the accumulators are single, and free again as
 // soon as they have been read.  No shared memory is left for staging rows, so a tile's rows reach memory from
 // registers: four lanes exchange 4 x 4 blocks of 16-byte chunks, and an instruction writes 64-byte runs of 8 rows.
-// grid (units of the chunk, query tiles), 320 threads.
+// grid (units of the chunk, query tiles), 576 threads.
+// With eight row warps of 64 keys a thread their splitting and storing, in series between S and dP, was longer than a tile's MMAs:
+// us, eight -> sixteen, one sequence of T 700, 8/2 heads of 160 48 -> 39; 2 of T 3000, 16/4 of 192 594 -> 521; batch 8, T 1024,
+// 32/8 of 256 623 -> 606 (the planes' DRAM traffic next).
 // ---------------------------------------------------------------------------------------------------
 struct ResShared {
     uint64_t full[4], freed[4], qh_full, ql_full, a_ready, s_full, s_free, dp_full, dp_free;
@@ -320,7 +324,7 @@ template <int D>
 __host__ __device__ constexpr int res_slots() { return D == 256 ? 3 : 4; }
 
 template <int D>
-__global__ void __launch_bounds__(kScoreThreads, 1)
+__global__ void __launch_bounds__(kResThreads, 1)
     bwd_wide_scores_res(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                         const __grid_constant__ CUtensorMap gmap, const __grid_constant__ CUtensorMap vmap, const WideParams p) {
     constexpr int NB = D / 64, NR = res_slots<D>();
@@ -345,9 +349,9 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
     if (threadIdx.x == 0) {
         for (int i = 0; i < NR; ++i) mbar_init(&sh->full[i], 1), mbar_init(&sh->freed[i], 1);
         mbar_init(&sh->qh_full, 1), mbar_init(&sh->ql_full, 1);
-        mbar_init(&sh->a_ready, 8);
-        mbar_init(&sh->s_full, 1), mbar_init(&sh->s_free, 8);
-        mbar_init(&sh->dp_full, 1), mbar_init(&sh->dp_free, 8);
+        mbar_init(&sh->a_ready, 16);
+        mbar_init(&sh->s_full, 1), mbar_init(&sh->s_free, 16);
+        mbar_init(&sh->dp_full, 1), mbar_init(&sh->dp_free, 16);
         sh->abort = (smem_u32(smem_raw) & 1023u) ? 90 : 0;
         if (sh->abort) atomicMax(&g_tc_status, 90);
         mbar_fence_init();
@@ -444,28 +448,27 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         }
         __syncwarp();
     } else {
-        // ------------------------------------------------------------------ a thread per query row and 64 of a
-        // tile's 128 keys: warps 2..5 the first 64, warps 6..9 the others
+        // ------------------------------------------------------------------ a thread per query row and 32 of the tile's 128 keys
         const int lane = threadIdx.x & 31;
         const int lane_grp = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int quarter = (warp - 2) >> 2;
         const int row = lane_grp * 32 + lane;
         const uint32_t lane_base = (uint32_t)(lane_grp * 32) << 16;
         const int t = m0 + row;
         bool ok = true;
         {
-            // this row's hi plane of Q (warps 2..5) or of dO (warps 6..9) -> TMEM, out of the 128-byte-swizzled staging tiles
+            // this row's hi plane of Q (even quarters) or of dO (odd ones), every other block of it, -> TMEM, out of the 128-byte-swizzled staging tiles
             if (!__all_sync(0xffffffffu, rwait(&sh->qh_full, 0, sh))) rgive_up(sh, 95), ok = false;
-            const uint8_t *src = (half ? sGl : sQl) + row * 128;
+            const uint8_t *src = (quarter & 1 ? sGl : sQl) + row * 128;
 #pragma unroll 1
-            for (int blk = 0; blk < NB; ++blk) {
+            for (int blk = quarter >> 1; blk < NB; blk += 2) {
                 uint32_t r[32];
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const uint4 v4 = *reinterpret_cast<const uint4 *>(src + blk * BT + ((c ^ (row & 7)) << 4));
                     r[4 * c] = v4.x, r[4 * c + 1] = v4.y, r[4 * c + 2] = v4.z, r[4 * c + 3] = v4.w;
                 }
-                tmem_st32(tmem + lane_base + (half ? cGh : cQh) + blk * 32, r);
+                tmem_st32(tmem + lane_base + (quarter & 1 ? cGh : cQh) + blk * 32, r);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -483,26 +486,24 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         const float dels = (t < p.T && !ZT_DEFECT(13)) ? __ldg(p.delta + ridx) * cq / p.p_scale : 0.f;
         bool saturated = false;
         const long long plane = (long long)p.Tp * p.Tp;
-        // the quad's first row, this thread's 64 columns, of the unit's hi planes (lo: unit_cap planes further)
-        __half *p_hi = p.p_planes + (long long)u * plane + (long long)(m0 + (row & ~3)) * p.Tp + half * 64;
-        __half *d_hi = p.ds_planes + (long long)u * plane + (long long)(m0 + (row & ~3)) * p.Tp + half * 64;
+        // the quad's first row, this thread's 32 columns, of the unit's hi planes (lo: unit_cap planes further)
+        __half *p_hi = p.p_planes + (long long)u * plane + (long long)(m0 + (row & ~3)) * p.Tp + quarter * 32;
+        __half *d_hi = p.ds_planes + (long long)u * plane + (long long)(m0 + (row & ~3)) * p.Tp + quarter * 32;
         const long long lo_off = (long long)p.unit_cap * plane;
         for (int n = 0; ok && n < n_tiles; ++n) {
             const int n0 = n * 128;
             const bool diag = (n == m) || (m0 + 128 > p.T);
-            float pr[64];
+            float pr[32];
             if (!__all_sync(0xffffffffu, rwait(&sh->s_full, (uint32_t)(n & 1), sh))) { rgive_up(sh, 96); ok = false; break; }
             tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 64; c += 32) {
+            {
                 uint32_t rs[32];
-                tmem_ld32(tmem + lane_base + cS + half * 64 + c, rs);
+                tmem_ld32(tmem + lane_base + cS + quarter * 32, rs);
                 tmem_wait_ld();
-                if (c == 32) {  // S has been read: the next tile's may overwrite it
-                    tc_fence_before();
-                    mbar_arrive_warp_relaxed(&sh->s_free);
-                }
-                const int key0 = n0 + half * 64 + c;
+                // S has been read: the next tile's may overwrite it
+                tc_fence_before();
+                mbar_arrive_warp_relaxed(&sh->s_free);
+                const int key0 = n0 + quarter * 32;
                 uint32_t ph[16], pl[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
@@ -510,38 +511,35 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
                     for (int e = 0; e < 2; ++e) {
                         const int key = key0 + i + e;
                         const bool vis = !diag || ((key <= t || ZT_DEFECT(11)) && key < p.T && t < p.T);
-                        pr[c + i + e] = vis ? ex2(__uint_as_float(rs[i + e]) * cs - lse2) : 0.f;
+                        pr[i + e] = vis ? ex2(__uint_as_float(rs[i + e]) * cs - lse2) : 0.f;
                     }
-                    split_pack(pr[c + i], pr[c + i + 1], ph[i >> 1], pl[i >> 1]);
+                    split_pack(pr[i], pr[i + 1], ph[i >> 1], pl[i >> 1]);
                 }
-                store_rows_quad(p_hi + n0 + c, p.Tp, ph, lane);
-                store_rows_quad(p_hi + lo_off + n0 + c, p.Tp, pl, lane);
+                store_rows_quad(p_hi + n0, p.Tp, ph, lane);
+                store_rows_quad(p_hi + lo_off + n0, p.Tp, pl, lane);
             }
             if (!__all_sync(0xffffffffu, rwait(&sh->dp_full, (uint32_t)(n & 1), sh))) { rgive_up(sh, 97); ok = false; break; }
             tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 64; c += 32) {
+            {
                 uint32_t rd[32];
-                tmem_ld32(tmem + lane_base + cDP + half * 64 + c, rd);
+                tmem_ld32(tmem + lane_base + cDP + quarter * 32, rd);
                 tmem_wait_ld();
-                if (c == 32) {
-                    tc_fence_before();
-                    mbar_arrive_warp_relaxed(&sh->dp_free);
-                }
+                tc_fence_before();
+                mbar_arrive_warp_relaxed(&sh->dp_free);
                 uint32_t dh[16], dl[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
                     float dv[2];
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const float x = pr[c + i + e] * (__uint_as_float(rd[i + e]) * c1 - dels);  // (pr is zero where masked)
+                        const float x = pr[i + e] * (__uint_as_float(rd[i + e]) * c1 - dels);  // (pr is zero where masked)
                         saturated |= !(fabsf(x) <= kDsBound);
                         dv[e] = fminf(fmaxf(x, -kDsBound), kDsBound);
                     }
                     split_pack(dv[0], dv[1], dh[i >> 1], dl[i >> 1]);
                 }
-                store_rows_quad(d_hi + n0 + c, p.Tp, dh, lane);
-                store_rows_quad(d_hi + lo_off + n0 + c, p.Tp, dl, lane);
+                store_rows_quad(d_hi + n0, p.Tp, dh, lane);
+                store_rows_quad(d_hi + lo_off + n0, p.Tp, dl, lane);
             }
         }
         if (__any_sync(0xffffffffu, saturated) && lane == 0) atomicAdd(&g_tc_saturated, 1u);
@@ -561,12 +559,16 @@ inline size_t res_smem_bytes() { return (size_t)(2 * D / 64 + 2 * res_slots<D>()
 //           times scale / (cq(t) mk).
 //   dK, dV  A = dS or P planes read M-major (rows are the contraction index: query rows); contraction over query rows
 //           [max(m * 128, piece * 1024), min(Tp, (piece + 1) * 1024)); every head of a group adds into its KV head.
-// Every tile is added to the output (red.global.add.v4.f32), which the pre-pass has zeroed.
+// dQ's tiles are stored where one unit holds a tile's whole contraction (T up to 1024); every other tile is added to the output
+// (red.global.add.v4.f32), which the pre-pass has zeroed.
 // A unit is one (product, head of the chunk, piece, tile): nine steps of MMAs on average at T 1024, about as long as its
 // prologue and epilogue together when each was a block of its own.  So a block walks its share of the units with two
 // accumulators in TMEM (all 512 columns), loads run ahead across units, and a unit's epilogue -- straight from TMEM to
 // memory, rows regrouped among eight lanes -- runs under the next one's MMAs.  A head's tiles are consecutive units:
-// blocks that run together share its operands in L2.
+// blocks that run together share its operands in L2.  Where a tile is one unit (T up to 1024) so are those of its three products,
+// in turn, and dS is still in L2 when the second of its two products reads it; longest first, and the other way round in every
+// second head, so that what a block gets by its stride is neither always long nor always short.  (With pieces this was 5 % slower,
+// T 3000: 789 -> 827.)  Batch 8, T 1024, 32/8 heads of 256, with dQ stored instead of added: 775 -> 687.
 // Us, three launches of a block per unit -> this: batch 8, T 1024, 32/8 heads of 256 809 -> 777 (bound by DRAM: the planes are
 // 3 GB written and read there); forward and backward at batch 4, T 300, 8/2 heads 129 -> 111, one sequence of T 500, 4/2
 // heads of 160 130 -> 102.
@@ -590,10 +592,19 @@ __device__ __forceinline__ void tgive_up(TriShared *sh, int code) {
 struct TriUnit {
     int which, u, m0, b, h, k_begin, n_steps;  // which: 0 dQ, 1 dK, 2 dV; n_steps <= 0: nothing to do
     __device__ __forceinline__ TriUnit(const WideParams &p, int i) {
-        const int nt = p.Tp / 128, m = i % nt, r = i / nt % (p.units * p.pieces);
-        which = i / (nt * p.units * p.pieces);
-        u = r / p.pieces;
-        const int piece = r - u * p.pieces, ug = p.unit0 + u;
+        const int nt = p.Tp / 128;
+        int m, piece = 0;
+        if (p.pieces == 1) {
+            u = i / (3 * nt);
+            const int at = i - u * 3 * nt, r = u & 1 ? 3 * nt - 1 - at : at, level = r / 3;
+            which = r - 3 * level;
+            m = which == 0 ? nt - 1 - level : level;
+        } else {
+            const int r = i / nt % (p.units * p.pieces);
+            which = i / (nt * p.units * p.pieces);
+            m = i % nt, u = r / p.pieces, piece = r - u * p.pieces;
+        }
+        const int ug = p.unit0 + u;
         b = ug / p.n_heads, h = ug - b * p.n_heads;
         m0 = m * 128;
         k_begin = piece * kPiece;
@@ -726,6 +737,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
             tc_fence_after();
             const long long ld = (long long)(w.which == 0 ? p.n_heads : p.n_kv_heads) * p.dim_out;
             const int row0 = t - j8;  // the first of this lane's eight rows
+            const bool whole = w.which == 0 && p.pieces == 1;
             float *dst = (w.which == 0 ? p.dq : w.which == 1 ? p.dk : p.dv) + ((long long)w.b * p.T + row0) * ld +
                          (long long)(w.which == 0 ? w.h : g) * p.dim_out + 4 * j8;
 #pragma unroll 1
@@ -759,10 +771,12 @@ __global__ void __launch_bounds__(kTriThreads, 1)
                 }
                 if (c + 4 * j8 < p.dim_out) {  // (a padded tile's upper columns are not the tensor's)
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (row0 + e < p.T)
-                            tcb::red_add_v4(dst + (long long)e * ld + c, make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]),
-                                                                                    __uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3])));
+                    for (int e = 0; e < 8; ++e) {
+                        if (row0 + e >= p.T) continue;
+                        const float4 a = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3]));
+                        if (whole) *reinterpret_cast<float4 *>(dst + (long long)e * ld + c) = a;
+                        else tcb::red_add_v4(dst + (long long)e * ld + c, a);
+                    }
                 }
             }
             ++n;
@@ -868,7 +882,8 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         pass_add(pa, k, batch, T, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes);
         pass_add(pa, v, batch, T, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     }
-    pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
+    const int pieces = (ww.Tp + kPiece - 1) / kPiece;
+    if (pieces > 1) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);  // (a whole contraction's dQ is stored)
     pass_fill(pa, dk, (long long)batch * T * n_kv_heads * dim);
     pass_fill(pa, dv, (long long)batch * T * n_kv_heads * dim);
     if (launch_pass_backward(pa, w, true, true, qkv_planes_kept, stream)) return 1;
@@ -904,7 +919,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     p.dim_out = dim, p.td = td;
     p.unit_cap = cap;
     p.dq = dq, p.dk = dk, p.dv = dv;
-    p.pieces = (Tp + kPiece - 1) / kPiece;
+    p.pieces = pieces;
     p.scale = 1.0f / sqrtf((float)dim), p.scale_log2 = kLog2e / sqrtf((float)dim);
     p.p_scale = ldexpf(1.0f, 10);
     g_last_path = "tcgen05";
@@ -918,7 +933,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
             if (launch_after("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
         } else {
             const dim3 gs((unsigned)units, (unsigned)nt);
-            if (launch_after("bwd_wide_scores_res", scores, gs, dim3(kScoreThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores_res", scores, gs, dim3(kResThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
         }
         p.units = units;
         const long long n_units = 3LL * nt * units * p.pieces;
