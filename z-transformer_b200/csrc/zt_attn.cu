@@ -19,6 +19,7 @@
 #include "tc_fwd16.cuh"
 #include "tc_fwd16g.cuh"
 #include "tc_fwd16x.cuh"
+#include "tc_fwd_short.cuh"
 #include "tc_gemm.cuh"
 #include "tc_bwd_wide.cuh"
 #include "tc_bwd_fused.cuh"
@@ -184,12 +185,17 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
         // do without scratch have some of their own for the call.
         const size_t need = tc_fwd16_workspace_bytes(batch, T, n_heads, n_kv_heads, dim, q_offset);
         const bool own = q_offset != 0 || n_keys != T || workspace_optional(T, dim);
+        // Up to 128 keys need no planes.  (A shape that takes the device's arena asks for it all the same: inside a capture that may
+        // have to be refused.)
+        const bool brief = path == 0 && tc_fwd_short_takes(batch, T, q_offset, dim);
+        if (brief && own) return launch_fwd_short(q, k, v, out, lse, batch, T, q_offset, n_keys, n_heads, n_kv_heads, dim, stream);
         const StreamScratch scratch(own ? need : 0, stream);
         bool in_capture = false;
         void *arena = own ? scratch.get() : device_arena(need, stream, &in_capture);
         if (in_capture)
             return refuse("this shape needs %zu bytes of the per-device arena, which would have to grow while the "
                           "stream is being captured: call zt_attn_reserve for the shape before the capture.", need);
+        if (arena && brief) return launch_fwd_short(q, k, v, out, lse, batch, T, q_offset, n_keys, n_heads, n_kv_heads, dim, stream);
         if (arena)
             return launch_fwd_tc16(q, k, v, out, lse, arena, need, batch, T, n_heads, n_kv_heads, dim, stream, nullptr, false,
                                    path == 6 ? 1 : (path == 7 ? 2 : 0), nullptr, nullptr, q_offset);
