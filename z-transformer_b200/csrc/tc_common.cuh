@@ -132,6 +132,10 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, const void 
                  "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
                  : "memory");
 }
+// `bytes` of this CTA's shared memory to global memory (both 16-byte aligned, a multiple of 16 bytes), waited for in the same way.
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tma_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }  // sources are free again
 __device__ __forceinline__ void tma_wait_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }       // the tensors have changed

@@ -631,9 +631,9 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
     pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     if (launch_pass(pa, stream)) return 1;
-    CUtensorMap kmap, vmap, qmap;  // (the widest tile fetches K block by block, see attn_fwd_tc16x)
+    CUtensorMap kmap, vmap, qmap;  // (the widest tiles fetch K block by block and V by 16 keys, see attn_fwd_tc16x)
     if (!make_head_map(&kmap, w.k_planes, 2 * batch, n_seen, n_kv_heads, dim, td > 128 ? 1 : td / 64, 64) ||
-        !make_head_map(&vmap, w.v_planes, 2 * batch, n_seen, n_kv_heads, dim, td / 64, 64) ||
+        !make_head_map(&vmap, w.v_planes, 2 * batch, n_seen, n_kv_heads, dim, td / 64, td > 128 ? 16 : 64) ||
         !make_head_map(&qmap, w.q_planes, 2 * batch, T, n_heads, dim, td / 64, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
     const int sms = split_sm_count();

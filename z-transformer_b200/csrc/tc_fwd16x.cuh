@@ -13,11 +13,14 @@
 //          next tile is fetched into it while the later blocks are still being read.  So S(j+1) can follow
 //          S(j) at once although there is room for one K tile only.
 //   MMA    S(0) S(1) | P.V(0) S(2) | P.V(1) S(3) | ...: the softmax of tile j+1 runs under P.V(j) and S(j+2).
-//          V(j+1) is fetched while S(j+2) runs.
+//          V(j+1) is fetched 16 keys after 16 keys, each piece as soon as the MMAs of P.V(j) on the one before it have
+//          retired: a tile took 5100 clocks with V fetched as a whole while S(j+2) ran, against 4000 of MMAs.
+// With the rows leaving as bulk copies (below): us, batch 8, T 1024, 32/8 heads of 256 650 -> 594; one sequence of T 700, 8/2 heads
+// of 160 41 -> 36; 2 sequences of T 4096, 32/8 of 256 1695 -> 1663.
 // Per 64-key tile the tensor core issues 12 MMAs of N = 64 per block for S and 12 of N = D for P.V: heads of 132 to 192
 // columns on a tile of 192 issue three quarters of what they cost padded to 256.
 // The Q hi tile reaches TMEM through V's slot (TMA, then the row threads); the rows leave through the K and V
-// slots, a row in two store instructions.  Every wait is bounded; a wait that gives up raises g_tc_status.
+// slots, a bulk copy a row.  Every wait is bounded; a wait that gives up raises g_tc_status.
 //
 // The backward at these widths: tc_bwd_wide.cuh.
 #pragma once
@@ -30,7 +33,7 @@ namespace tcf16 {
 constexpr int kThreadsX = 6 * 32;
 
 struct SharedX {
-    uint64_t full_k[4], free_k[4], full_v, free_v;
+    uint64_t full_k[4], free_k[4], full_v[4], free_v[4];
     uint64_t a_ready, q_full, ql_full, s_full[2], p_full[2], pv_done, staged, all_done;
     uint32_t tmem_base;
     volatile int abort;
@@ -47,7 +50,7 @@ __device__ __forceinline__ void xgive_up(SharedX *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-// kmap: K planes with a box of ONE 64-column block x 64 keys; vmap: V planes, the head's D / 64 blocks x 64 keys; qmap:
+// kmap: K planes with a box of ONE 64-column block x 64 keys; vmap: V planes, the head's D / 64 blocks x 16 keys; qmap:
 // Q planes, the head's blocks x 128 rows.
 template <int D, bool FLUSH>
 __global__ void __launch_bounds__(kThreadsX, 1)
@@ -56,10 +59,11 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     constexpr int NB = D / 64, BN = 64;
     constexpr int KB = BN * 128;        // bytes of one 64-column block of one plane of a key tile (8 KB)
     constexpr int KP = NB * KB;         // one plane of a key tile (32 KB at 256 columns); a K or V tile is 2 KP
+    constexpr int VB = NB * 16 * 128;   // one plane of 16 keys of a V tile (8 KB at 256 columns)
     constexpr int QB = 128 * 128;       // one block of one plane of the 128-row query tile (16 KB)
     constexpr int cQh = 0, cO = 128, cS0 = 384;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // K: block c of the tile at sK + c * 2 KB (hi, then lo); V: hi plane, lo plane; Q lo: NB blocks
+    // K: block c of the tile at sK + c * 2 KB (hi, then lo); V: 16 keys c of the tile at sV + c * 2 VB (hi, then lo); Q lo: NB blocks
     uint8_t *sK = smem_raw, *sV = sK + 2 * KP, *sQl = sV + 2 * KP;
     SharedX *sh = reinterpret_cast<SharedX *>(sQl + NB * QB);
 
@@ -90,7 +94,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NB; ++i) mbar_init(&sh->full_k[i], 1), mbar_init(&sh->free_k[i], 1);
-        mbar_init(&sh->full_v, 1), mbar_init(&sh->free_v, 1);
+        for (int i = 0; i < BN / 16; ++i) mbar_init(&sh->full_v[i], 1), mbar_init(&sh->free_v[i], 1);
         mbar_init(&sh->a_ready, 4);
         mbar_init(&sh->q_full, 1), mbar_init(&sh->ql_full, 1);
         for (int i = 0; i < 2; ++i) mbar_init(&sh->s_full[i], 1), mbar_init(&sh->p_full[i], 4);
@@ -121,7 +125,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             tma_load_4d(sV, &qmap, &sh->q_full, 0, t0, h * NB, b);
             mbar_arrive_expect_tx(&sh->ql_full, NB * QB);
             tma_load_4d(sQl, &qmap, &sh->ql_full, 0, t0, h * NB, B + b);
-            int n_k = 0, n_v = 0;  // K blocks and V tiles issued
+            int n_k = 0, n_v = 0;  // K blocks and V pieces issued
             bool live = true;
             auto load_k_block = [&](int j, int c) {
                 if (j >= 1 && !xwait(&sh->free_k[c], (uint32_t)((j - 1) & 1), sh)) { xgive_up(sh, 61), live = false; return; }
@@ -131,11 +135,13 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 ++n_k;
             };
             auto load_v = [&](int j) {
-                if (j >= 1 && !xwait(&sh->free_v, (uint32_t)((j - 1) & 1), sh)) { xgive_up(sh, 61), live = false; return; }
-                mbar_arrive_expect_tx(&sh->full_v, 2 * KP);
-                tma_load_4d(sV, &vmap, &sh->full_v, 0, (jb + j) * BN, g * NB, b);
-                tma_load_4d(sV + KP, &vmap, &sh->full_v, 0, (jb + j) * BN, g * NB, B + b);
-                ++n_v;
+                for (int c = 0; c < BN / 16; ++c) {
+                    if (j >= 1 && !xwait(&sh->free_v[c], (uint32_t)((j - 1) & 1), sh)) { xgive_up(sh, 61), live = false; return; }
+                    mbar_arrive_expect_tx(&sh->full_v[c], 2 * VB);
+                    tma_load_4d(sV + c * 2 * VB, &vmap, &sh->full_v[c], 0, (jb + j) * BN + c * 16, g * NB, b);
+                    tma_load_4d(sV + c * 2 * VB + VB, &vmap, &sh->full_v[c], 0, (jb + j) * BN + c * 16, g * NB, B + b);
+                    ++n_v;
+                }
             };
             for (int c = 0; c < NB; ++c) load_k_block(0, c);
             if (!xwait(&sh->a_ready, 0, sh)) xgive_up(sh, 61), live = false;  // V's slot holds Q hi until then
@@ -148,7 +154,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 // let the copies in flight land before the CTA's shared memory goes away
                 mbar_wait(&sh->q_full, 0), mbar_wait(&sh->ql_full, 0);
                 for (int i = (n_k > NB ? n_k - NB : 0); i < n_k; ++i) mbar_wait(&sh->full_k[i % NB], (uint32_t)((i / NB) & 1));
-                if (n_v > 0) mbar_wait(&sh->full_v, (uint32_t)((n_v - 1) & 1));
+                for (int i = (n_v > 4 ? n_v - 4 : 0); i < n_v; ++i) mbar_wait(&sh->full_v[i & 3], (uint32_t)((i >> 2) & 1));
             }
         }
         __syncwarp();
@@ -186,31 +192,34 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 mma_commit(&sh->s_full[j & 1]);
                 return true;
             };
-            // P.V of tile j
-            auto issue_pv = [&](int j) {
+            // P.V of tile j, 16 keys after 16 keys of the contraction
+            auto issue_pv = [&](int j) -> bool {
                 const bool fresh = j == 0 || (FLUSH && j % kFlushKeyTiles == 0);  // (O was flushed before tile j)
-                const uint64_t mvh = desc_mnmajor_16b(v_u32, BN * 128), mvl = desc_mnmajor_16b(v_u32 + KP, BN * 128);
                 const uint32_t cS = cS0 + (j & 1) * BN;
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
+                    if (!xwait(&sh->full_v[kk], (uint32_t)(j & 1), sh)) return false;
+                    tc_fence_after();
                     const uint32_t ac = (uint32_t)(32 * (kk >> 1) + (kk & 1) * 8);
-                    const uint64_t dvh = desc_advance(mvh, kk * 2048), dvl = desc_advance(mvl, kk * 2048);
+                    const uint64_t dvh = desc_mnmajor_16b(v_u32 + (uint32_t)(kk * 2 * VB), 16 * 128);
+                    const uint64_t dvl = desc_mnmajor_16b(v_u32 + (uint32_t)(kk * 2 * VB + VB), 16 * 128);
                     mma_ts_f16(tmem + cO, tmem + cS + ac, dvh, id_o, (!fresh || kk > 0) ? 1 : 0);
                     mma_ts_f16(tmem + cO, tmem + cS + ac, dvl, id_o, 1);
                     mma_ts_f16(tmem + cO, tmem + cS + ac + 16, dvh, id_o, 1);
+                    mma_commit(&sh->free_v[kk]);
                 }
-                mma_commit(&sh->free_v);
                 mma_commit(&sh->pv_done);
+                return true;
             };
             if (ok && !issue_qk(0)) { xgive_up(sh, 63); ok = false; }
             if (ok && n_tiles > 1 && !issue_qk(1)) { xgive_up(sh, 63); ok = false; }
             for (int j = 0; ok && j < n_tiles; ++j) {
-                if (!xwait(&sh->p_full[j & 1], (uint32_t)((j >> 1) & 1), sh) || !xwait(&sh->full_v, (uint32_t)(j & 1), sh)) {
+                if (!xwait(&sh->p_full[j & 1], (uint32_t)((j >> 1) & 1), sh)) {
                     xgive_up(sh, 64);
                     break;
                 }
                 tc_fence_after();
-                issue_pv(j);
+                if (!issue_pv(j)) { xgive_up(sh, 64); break; }
                 if (j == n_tiles - 1) mma_commit(&sh->all_done);  // once, after the last P.V
                 if (j + 2 < n_tiles && !issue_qk(j + 2)) { xgive_up(sh, 63); break; }  // over the P tile P.V(j) has just read
             }
@@ -320,16 +329,19 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             xgive_up(sh, 68);
             ok = false;
         }
-        // The rows go to global memory through shared memory (the K and V slots are idle once all_done completes):
-        // 128 rows of 4 D bytes; a row in two store instructions instead of 32.
-        // (16-byte chunk c of row r sits at chunk c ^ (r & 15): a row is a multiple of sixteen chunks)
+        // The rows go to global memory through shared memory (idle once all_done completes), each by its own thread as one bulk
+        // copy: the stores of a warp that went through all rows, two instructions a row, took 7500 clocks.  (Rows 16 bytes
+        // apart from a multiple of 128, so that eight threads' chunks lie in different banks.)  A row that goes to more
+        // places than out goes by such stores all the same.
+        constexpr int RS = D * 4 + 16;
         uint8_t *stage = smem_raw;
+        const bool plain = p.o_planes == nullptr && p.out_peers.n == 0;
         if (ok) {
             tc_fence_after();
             const float inv = l == 0.f ? 0.f : 1.f / (l * mv);  // l, like O, carries kPScale (0: a part without a key the row sees)
             const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
-            uint8_t *srow = stage + tid * (D * 4);
+            uint8_t *srow = stage + tid * RS;
 #pragma unroll 1
             for (int c = 0; c < D; c += 32) {
                 uint32_t ra[32];
@@ -340,14 +352,20 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
                     if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
-                    const int ch = (c + i) >> 2;
-                    *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & 15)) << 4)) = o4;
+                    *reinterpret_cast<float4 *>(srow + (c + i) * 4) = o4;
                 }
             }
             if (p.lse && t < p.T) p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
         }
+        if (plain) {
+            fence_async_smem();
+            if (FLUSH) asm volatile("fence.proxy.async.global;" ::: "memory");  // (the row's running sum was written by plain stores)
+            if (ok && t < p.T) bulk_store(p.out + part * p.out_part + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out, stage + tid * RS, (uint32_t)p.dim_out * 4);
+            tma_commit();
+            tma_wait_read();
+        }
         mbar_arrive_warp(&sh->staged);
-        if (__all_sync(0xffffffffu, xwait(&sh->staged, 0, sh)) && !sh->abort) {
+        if (!plain && __all_sync(0xffffffffu, xwait(&sh->staged, 0, sh)) && !sh->abort) {
             const long long wo = (long long)p.n_heads * p.dim_out;
             const float mo = p.o_planes ? out_plane_mult(p, b) : 1.f;
             // a warp stores its 32 rows; a row is 48 or 64 chunks: two instructions
@@ -358,7 +376,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 for (int half = 0; half < 2; ++half) {
                     const int ch = half * 32 + lane;
                     if (ch >= D / 4) continue;
-                    const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * (D * 4) + ((ch ^ (r & 15)) << 4));
+                    const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * RS + ch * 16);
                     if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
                         store_out4(p, part * p.out_part + ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
                 }
