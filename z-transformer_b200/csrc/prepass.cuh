@@ -1,7 +1,7 @@
 // The pre-pass of the tensor-core kernels: f32 tensors -> f16 hi/lo operand planes with a power-of-two scale per
 // (sequence, group of heads), and beside them what the backward wants to know about the rows of dout.
 //
-// Two launches for all tensors of a call, both bound by HBM (or, for small calls, by launch latency):
+// Two launches for all tensors of a call (one for a small forward: pass_one_kernel), both bound by HBM (or, for small calls, by launch latency):
 //   pass_stats_kernel    reads every tensor once.  Per block: max |x| and, where asked, the largest row norm; per row of
 //                        dout its norm and delta = sum_j dout out.  A block leaves its two maxima in a slot of its own
 //                        (no atomics and nothing to clear beforehand).
@@ -261,6 +261,25 @@ __device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long p
     *reinterpret_cast<uint2 *>(qs) = hw, *reinterpret_cast<uint2 *>(qs + plane) = lw;
 }
 
+// What four elements of the planes stand for.
+__device__ __forceinline__ float4 join_split4(uint2 h, uint2 l) {
+    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h.x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
+    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l.x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l.y));
+    return make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y);
+}
+// Block blk's part of the zeros of outputs that are summed in memory.
+template <int THREADS>
+__device__ __forceinline__ void pass_fill_block(const PassArgs &a, int blk) {
+    int f = 0;
+    while (f + 1 < a.n_fill && blk >= a.fill_first[f + 1]) ++f;
+    const long long i0 = (long long)(blk - a.fill_first[f]) * kFillPerBlock;
+#pragma unroll
+    for (int k = 0; k < kFillPerBlock / THREADS; ++k) {
+        const long long i = i0 + k * THREADS + threadIdx.x;
+        if (i < a.fill_n4[f]) a.fill[f][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
 // LP lanes hold a unit of the planes (pd columns), NC chunks of four columns each.
 template <int LP, int NC>
 __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
@@ -269,14 +288,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     pdl_launch();
     const int blk = (int)blockIdx.x;
     if (blk >= a.fill_first[0]) {
-        int f = 0;
-        while (f + 1 < a.n_fill && blk >= a.fill_first[f + 1]) ++f;
-        const long long i0 = (long long)(blk - a.fill_first[f]) * kFillPerBlock;
-#pragma unroll
-        for (int k = 0; k < kFillPerBlock / kPassThreads; ++k) {
-            const long long i = i0 + k * kPassThreads + threadIdx.x;
-            if (i < a.fill_n4[f]) a.fill[f][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        pass_fill_block<kPassThreads>(a, blk);
         return;
     }
     __shared__ uint4 red[kPassThreads / 32];
@@ -326,11 +338,9 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                 ds_row_scale(rn[k], tops.dn, tops.vn, cq, rel);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h[k][c].y));
-                    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l[k][c].y));
                     // (a sum of the two pieces splits into these very pieces again)
                     if (at[k] >= 0 && (li + LP * c) * 4 < a.pd)
-                        store_split4(nullptr, t.qs + at[k] * a.pd + (li + LP * c) * 4, plane, make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y), 1.f, rel);
+                        store_split4(nullptr, t.qs + at[k] * a.pd + (li + LP * c) * 4, plane, join_split4(h[k][c], l[k][c]), 1.f, rel);
                 }
             }
             u0 += stride;
@@ -412,6 +422,87 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
 }
 
+// ---- the one launch of small forwards ---------------------------------------------------------------
+// Both launches in one, for forwards whose every (sequence, group) fits the registers of a block: 16 float4 a thread.  A block reads
+// its group's rows once, all loads under way together, knows the maxima after one barrier and writes the planes out of
+// registers: a launch less in a chain that is nothing but launches.  Us, forward of one sequence of 256, 16/16 heads of 64 20.7 -> 15.8, of
+// 12 of 128, 8/8 heads of 192 34.1 -> 20.6, forward and backward of one of 256, 4/2 heads of 32 44.1 -> 41.8.
+// (A backward's dout, whose block has out to read and q's planes to copy as well, took longer so than in two launches: forward and
+// backward of 64 rows, 32/8 heads of 128, 70 -> 77.)
+constexpr int kOneThreads = 512, kOneChunks = 16;
+template <int LP, int NC>
+__host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (kOneChunks / NC); }
+
+template <int LP, int NC>
+__global__ void __launch_bounds__(kOneThreads, 1) pass_one_kernel(const __grid_constant__ PassArgs a) {
+    constexpr int NG = kOneThreads / LP, U = kOneChunks / NC;
+    __shared__ uint32_t red[2][kOneThreads / 32];
+    pdl_wait();
+    pdl_launch();
+    const int blk = (int)blockIdx.x;
+    const PassUnit w = pass_locate(a, a.n, blk);
+    const PassTensor &t = a.t[w.z];
+    const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
+    const long long plane = (long long)t.batch * t.rows * t.heads * a.pd;
+    const int n4 = a.dim >> 2;
+    // this lane group's units, as places beyond the (sequence, group)'s first; -1: none
+    const long long first = (long long)w.b * t.rows * t.heads + w.g * t.group;
+    int place[U];
+    {
+        int r = gi / t.group, i = gi - r * t.group;
+        const int dr = NG / t.group, di = NG - dr * t.group;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            place[k] = r < t.rows ? r * t.heads + i : -1;
+            r += dr, i += di;
+            if (i >= t.group) i -= t.group, ++r;
+        }
+    }
+    float4 x[U][NC];
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int ch = li + LP * c;
+            x[k][c] = place[k] >= 0 && ch < n4 ? reinterpret_cast<const float4 *>(t.x + (first + place[k]) * a.dim)[ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    float amax = 0.f, nmax = 0.f;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        float sq = 0.f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const float4 v = x[k][c];
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
+        }
+        if (!t.nmax) continue;
+#pragma unroll
+        for (int off = LP / 2; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        nmax = fmaxf(nmax, sqrtf(sq));
+    }
+    // (f32 bit patterns of non-negative numbers order like integers)
+    const uint32_t wa = __reduce_max_sync(0xffffffffu, __float_as_uint(amax)), wn = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));
+    if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5] = wa, red[1][threadIdx.x >> 5] = wn;
+    __syncthreads();
+    const uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kOneThreads / 32 - 1)]);
+    const uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kOneThreads / 32 - 1)]);
+    if (threadIdx.x == 0) {
+        t.amax[w.bg] = top;
+        if (t.nmax) t.nmax[w.bg] = dn;
+    }
+    const float m = block_mult(top);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        const long long at = first + place[k];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int col = (li + LP * c) * 4;
+            if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, nullptr, plane, x[k][c], m, 1.f);
+        }
+    }
+}
+
 // ---- host side --------------------------------------------------------------------------------------
 // Slots of one tensor of `bg` (sequence, group) pairs: what pass_slots() below can ask for.
 inline size_t pass_part_bytes(size_t bg) { return (bg > (size_t)kPassTargetBlocks ? bg : (size_t)kPassTargetBlocks) * sizeof(uint2); }
@@ -440,6 +531,25 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
 inline void pass_fill(PassArgs &a, float *dst, long long n) {
     a.fill[a.n_fill] = reinterpret_cast<float4 *>(dst), a.fill_n4[a.n_fill++] = n / 4;
 }
+// Whether one launch takes the call: `units` units a (sequence, group) at most, nothing rotated, nothing but planes and maxima wanted.
+inline bool pass_takes_one(const PassArgs &a, int units) {
+    for (int i = 0; i < a.n; ++i) {
+        const PassTensor &t = a.t[i];
+        if ((long long)t.rows * t.group > units || !t.x || !t.planes || t.delta || t.rope || t.qs) return false;
+    }
+    return a.n_fill == 0;
+}
+template <int LP, int NC>
+inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
+    long long blocks = 0;
+    for (int i = 0; i < a.n; ++i) {
+        PassTensor &t = a.t[i];
+        t.slots = 1, t.first = (int)blocks;
+        blocks += (long long)t.batch * (t.heads / t.group);
+    }
+    if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
+    return launch_pdl("pass_one_kernel", pass_one_kernel<LP, NC>, dim3((unsigned)blocks), dim3(kOneThreads), 0, stream, a);
+}
 // Both launches.  The tensors with an f32 source come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     long long blocks = 0, stats = 0;
@@ -463,6 +573,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     // lanes x chunks of four columns that a unit takes: the tightest that holds it
     const auto both = [&](auto lanes, auto chunks) -> int {
         constexpr int LP = lanes.value, NC = chunks.value;
+        if (pass_takes_one(a, pass_one_units<LP, NC>())) return launch_pass_one<LP, NC>(a, stream);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
