@@ -18,9 +18,9 @@
 // 16 row warps, a thread per key row and 32 of the step's query columns, at 80 registers a thread.
 // TMEM: V hi 32 (of 64), S^T/P^T 128, dP^T/dS^T 128, dQ 64, dV 64, dK 64 = 512 columns.  Shared memory: K hi/lo, V lo 48 KB,
 // dS^T hi/lo 64 KB, two Q slots and one dO slot of 32 KB each, 16 KB on the way out = 224 KB.
-// Measured (us, before -> after, this kernel): 32/8 heads of 64, batch 8, T 512 139 -> 103, T 4096, batch 1 643 -> 448; heads
-// of 32, batch 8, T 512 121 -> 94.  Error against 64 bits (2-norm, relative; T 1000, 8/2 heads of 64): dq 8.3e-7 -> 4.7e-7, dk
-// 1.2e-6 -> 8.0e-7, dv 9.5e-7 -> 6.9e-7.
+// Measured (us, before -> after, this kernel): 32/8 heads of 64, batch 8, T 512 139 -> 104, T 4096, batch 1 643 -> 448; heads
+// of 32, batch 8, T 512 121 -> 94.  Error against 64 bits (2-norm, relative; T 1000, 8/2 heads of 64): dq 8.0e-7 -> 5.7e-7, dk
+// 1.07e-6 -> 8.6e-7, dv 8.2e-7 -> 7.5e-7.
 #pragma once
 
 #include "tc_bwd_wide.cuh"
@@ -80,6 +80,8 @@ __device__ __forceinline__ void split_pack2(float2 v, uint32_t &hw, uint32_t &lw
     hw = *reinterpret_cast<const uint32_t *>(&hh);
     lw = pack_half2(lo.x, lo.y);
 }
+// The power of two at or below a normal x > 0; 0 for 0.
+__device__ __forceinline__ float pow2_of(float x) { return __uint_as_float(__float_as_uint(x) & 0x7f800000u); }
 // x with its magnitude cut to `bound` (> 0); the bound itself for a NaN
 __device__ __forceinline__ float clamp_abs(float x, float bound) {
     float r;
@@ -234,26 +236,25 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 tc_fence_after();
                 return true;
             };
-            // S^T(j) = K Q~^T.  (The tensor core adds with truncation, of the accumulator's last bits: here and below the two small
-            // terms of a product go first, while there is little to truncate.)
+            // S^T(j) = K Q~^T, its terms in the forward's order: the tensor core adds with truncation, and where the softmax is saturated
+            // what dP and delta leave of each other is as good as this S agrees with the one that delta's P came from.  (Small terms
+            // first here too: dq missed 1e-4 of its largest value by a quarter on scores that rise with the key, T 512, heads of 32.)
             auto issue_st = [&](int j) {
                 const uint32_t qh = q_u32 + (uint32_t)((j & 1) * 2 * QP);
                 const uint64_t bqh = desc_kmajor(qh), bql = desc_kmajor(qh + QP);
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                     if (PAD && kk >= steps) break;
-                    mma_ss_f16(tmem + cST, desc_advance(bkh, kk * 32), desc_advance(bql, kk * 32), id_s, kk > 0);
-                    mma_ss_f16(tmem + cST, desc_advance(bkl, kk * 32), desc_advance(bqh, kk * 32), id_s, 1);
-                }
-#pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    if (PAD && kk >= steps) break;
-                    mma_ss_f16(tmem + cST, desc_advance(bkh, kk * 32), desc_advance(bqh, kk * 32), id_s, 1);
+                    const uint64_t dkh = desc_advance(bkh, kk * 32), dqh = desc_advance(bqh, kk * 32);
+                    mma_ss_f16(tmem + cST, dkh, dqh, id_s, kk > 0);
+                    mma_ss_f16(tmem + cST, desc_advance(bkl, kk * 32), dqh, id_s, 1);
+                    mma_ss_f16(tmem + cST, dkh, desc_advance(bql, kk * 32), id_s, 1);
                 }
                 mma_commit(&sh->st_full);
             };
             // dV(j) += P^T dO: P^T's 16-column windows hold hi halves in their first 8 columns, lo in the last 8.
             // Waits for P^T(j) and for dO(j); `restart`: the accumulators were flushed after step j-1.
+            // (Here and in the other products the two small terms go first, while there is little to truncate.)
             int n_flush = 0;
             auto issue_dv = [&](int j, bool restart, bool flush_after) -> bool {
                 if (!fwait(&sh->p_ready, (uint32_t)(j & 1), sh) || !fwait(&sh->full_g, (uint32_t)(j & 1), sh)) return false;
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
         // lane, fetched and worked out a step ahead.  (Done by the row threads, a value each, the loads' latency stood at the
         // head of every step and the arithmetic took a sixth of their instructions.)
         const int lane = threadIdx.x & 31;
-        const float lse_shift = log2f(p.p_scale), ndel_unit = 1.0f / (p.p_scale * unit);
+        const float lse_shift = log2f(p.p_scale), ndel_unit = 1.0f / (p.p_scale * pow2_of(unit));
         float lse[4], rn[4], de[4];
         int t0 = walk.qi * BQ + lane;
         const auto load = [&]() {
@@ -428,15 +429,16 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
         // columns [col, col + 32) of TMEM, this lane's row times f, into `out`
         const auto take = [&](uint32_t col, float f, uint64_t *freed) {
             uint32_t r[32];
+            __syncwarp();  // (the whole warp: tcgen05.ld and its wait are warp-aligned)
             tmem_ld32(tmem + lane_base + col, r);
             if (lane == 0) tma_wait_read();
+            __syncwarp();
             tmem_wait_ld();
             if (freed) {
                 // (the tensor core may go on while the columns are still on their way)
                 tc_fence_before();
                 mbar_arrive_warp_relaxed(freed);
             }
-            __syncwarp();
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const float2 a = mul2(floats2(r[4 * c], r[4 * c + 1]), make_float2(f, f)), d = mul2(floats2(r[4 * c + 2], r[4 * c + 3]), make_float2(f, f));
@@ -509,8 +511,10 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             tc_fence_before();
             mbar_arrive_warp(&sh->a_ready);
         }
-        // dS = P (dP - delta) cq(t): the row threads keep P csc(t), whose factor beside cq(t) leaves with the units of dP and delta
-        const float dp_unit = cmin / mdo / mv / (p.p_scale * unit);
+        // dS = P (dP - delta) cq(t): the row threads keep P times csc(t)'s power of two, which beside cq(t) leaves with the units of
+        // dP and delta.  (Powers of two only: dP and delta nearly cancel where the softmax is saturated, and a unit rounded once for
+        // each of them left 1e-7 of delta there.)
+        const float dp_unit = cmin / mdo / mv / (p.p_scale * pow2_of(unit));
         const float2 dp_unit2 = make_float2(dp_unit, dp_unit);
         float ds_top = 0.f;
         for (int it = 0; it < n_it; ++it, walk.next()) {
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                             p0.x = vis(t) ? p0.x : 0.f, p0.y = vis(t + 1) ? p0.y : 0.f;
                             p1.x = vis(t + 2) ? p1.x : 0.f, p1.y = vis(t + 3) ? p1.y : 0.f;
                         }
-                        pr[k] = mul2(p0, make_float2(c.x, c.y)), pr[k + 1] = mul2(p1, make_float2(c.z, c.w));
+                        pr[k] = mul2(p0, make_float2(pow2_of(c.x), pow2_of(c.y))), pr[k + 1] = mul2(p1, make_float2(pow2_of(c.z), pow2_of(c.w)));
                         split_pack2(p0, ph[2 * i4], pl[2 * i4]);
                         split_pack2(p1, ph[2 * i4 + 1], pl[2 * i4 + 1]);
                     }
