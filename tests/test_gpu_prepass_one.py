@@ -1,0 +1,38 @@
+"""The one-launch pre-pass of small forwards at the sizes where its two forms begin and end (units of a sequence's group of heads:
+rows times heads): outputs against float64, and gradients from the planes it leaves.  Tolerances are those of the short forward's and
+the backwards' tests."""
+import pytest
+import torch
+
+from test_gpu_backward64 import gradients
+from test_gpu_forward_short import forward64
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,T,H,G,D,one", [
+    (3, 64, 8, 2, 32, True), (1, 65, 8, 2, 32, True), (1, 256, 4, 1, 32, True), (1, 257, 4, 1, 32, False),     # 256 and 1024 units
+    (2, 128, 3, 3, 64, True), (1, 129, 3, 3, 64, True), (1, 170, 6, 2, 60, True), (1, 171, 6, 2, 64, False),   # 128 and 512
+    (1, 64, 2, 2, 96, True), (5, 106, 3, 1, 80, True), (1, 107, 3, 1, 80, False),                              # 64 and 320
+    (1, 64, 4, 1, 128, True), (1, 65, 4, 1, 128, False), (7, 53, 3, 1, 192, True), (1, 54, 3, 1, 160, False),  # 64, 256; 32, 160
+    (2, 128, 2, 2, 256, True), (1, 129, 2, 2, 200, False),                                                     # 32, 128
+])
+def test_planes_of_small_forwards(zt, B, T, H, G, D, one):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(17)
+    q, k, v, do = (torch.randn((B, T, w * D), device="cuda", generator=gen) * c for w, c in zip((H, G, G, H), (1, 1, 1e3, 1e-3)))
+    ws = zt.BackwardWorkspace(B, T, H, G, D)
+    zt.lib.profile(True)
+    zt.lib.profile_read()
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    launched = zt.lib.profile_read()
+    zt.lib.profile(False)
+    assert ("pass_one_kernel" in launched) == one and ("pass_planes_kernel" in launched) != one
+    got = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=ws.token != 0)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+    ref, ref_lse = forward64(q, k, v, H, G, D, 0)
+    assert float((out.double() - ref).norm()) <= 3e-6 * float(ref.norm())
+    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 1e-5
+    for name, x, r in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
+        assert float((x.double() - r).norm()) <= (6e-7 + 4e-8 * 240) * float(r.norm()), name

@@ -429,13 +429,15 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
 // 12 of 128, 8/8 heads of 192 34.1 -> 20.6, forward and backward of one of 256, 4/2 heads of 32 44.1 -> 41.8.
 // (A backward's dout, whose block has out to read and q's planes to copy as well, took longer so than in two launches: forward and
 // backward of 64 rows, 32/8 heads of 128, 70 -> 77.)
-constexpr int kOneThreads = 512, kOneChunks = 16;
-template <int LP, int NC>
-__host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (kOneChunks / NC); }
+// Two forms: of 16 float4 a thread, and of 4, with three blocks an SM: forward and backward of 7 sequences of 87, 16/16 heads of 32,
+// took 38.8 in two launches, 41.6 with the former alone, 36.3 with the latter.
+constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4;
+template <int LP, int NC, int CHUNKS>
+__host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (CHUNKS / NC); }
 
-template <int LP, int NC>
-__global__ void __launch_bounds__(kOneThreads, 1) pass_one_kernel(const __grid_constant__ PassArgs a) {
-    constexpr int NG = kOneThreads / LP, U = kOneChunks / NC;
+template <int LP, int NC, int CHUNKS>
+__global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_one_kernel(const __grid_constant__ PassArgs a) {
+    constexpr int NG = kOneThreads / LP, U = CHUNKS / NC;
     __shared__ uint32_t red[2][kOneThreads / 32];
     pdl_wait();
     pdl_launch();
@@ -539,7 +541,7 @@ inline bool pass_takes_one(const PassArgs &a, int units) {
     }
     return a.n_fill == 0;
 }
-template <int LP, int NC>
+template <int LP, int NC, int CHUNKS>
 inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
     long long blocks = 0;
     for (int i = 0; i < a.n; ++i) {
@@ -548,7 +550,7 @@ inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
         blocks += (long long)t.batch * (t.heads / t.group);
     }
     if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
-    return launch_pdl("pass_one_kernel", pass_one_kernel<LP, NC>, dim3((unsigned)blocks), dim3(kOneThreads), 0, stream, a);
+    return launch_pdl("pass_one_kernel", pass_one_kernel<LP, NC, CHUNKS>, dim3((unsigned)blocks), dim3(kOneThreads), 0, stream, a);
 }
 // Both launches.  The tensors with an f32 source come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
@@ -573,7 +575,8 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     // lanes x chunks of four columns that a unit takes: the tightest that holds it
     const auto both = [&](auto lanes, auto chunks) -> int {
         constexpr int LP = lanes.value, NC = chunks.value;
-        if (pass_takes_one(a, pass_one_units<LP, NC>())) return launch_pass_one<LP, NC>(a, stream);
+        if (pass_takes_one(a, pass_one_units<LP, NC, kOneFew>())) return launch_pass_one<LP, NC, kOneFew>(a, stream);
+        if (pass_takes_one(a, pass_one_units<LP, NC, kOneMost>())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
