@@ -68,7 +68,7 @@ struct BwdParts {
 };
 // The split with the shortest schedule, in steps (about 3 us each, 64 rows at 128 columns or 128 at 64): a launch ends with
 // its longest block, or once all blocks' steps have been shared out with half a block left over at the end (the walks are of
-// all lengths, longest first); a block costs three steps beside its walk (two at 64 columns, where several share an SM),
+// all lengths, longest first); a block costs three steps beside its walk (two at 64 columns, whose tiles are half as large),
 // putting the parts together two and their traffic one per 45 blocks (at 64 columns, whose parts are half as large,
 // one and a half and one per 90).  Parts keep 256 rows of the longest walk, and a launch two blocks an SM (which bounds the
 // partial results: 38 MB at most).  At 64 columns, us a step unsplit / split as this does (heads x ranges): batch 4, T 1000, 16/4
