@@ -55,3 +55,20 @@ def test_aligned_cluster_barriers_are_reached_by_whole_warps():
             assert "__syncwarp();" in body, (name, m[0])
             n += 1
     assert n == 2
+
+
+def test_aligned_tensor_memory_instructions_are_reached_by_whole_warps():
+    """tcgen05.alloc, dealloc, ld, st and their waits are .sync.aligned: all threads of a warp execute them together.  They follow
+    code that ends lane by lane (rows past the sequence, columns past the head, one lane's arrival), so the wrapper
+    brings the warp together itself, and nothing but the wrappers issues them; a wait comes straight after the ones it is for or a
+    vote of the whole warp."""
+    text = sources()
+    names = []
+    for name, t in text.items():
+        for m in re.finditer(r"tcgen05\.(?:alloc|dealloc|ld|st)[.\w:]*\.sync\.aligned", t):
+            assert name == "tc_common.cuh", name
+            start = t.rindex("__device__", 0, m.start())
+            names.append(re.match(r"__device__ __forceinline__ void (\w+)\(", t[start:])[1])
+            body = t[start:m.start()]
+            assert re.match(r"[^{]*\{\s*__syncwarp\(\);", body), names[-1]
+    assert sorted(names) == ["tmem_alloc", "tmem_dealloc", "tmem_ld16", "tmem_ld32", "tmem_st16", "tmem_st32", "tmem_st8"]
