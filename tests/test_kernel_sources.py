@@ -72,3 +72,21 @@ def test_aligned_tensor_memory_instructions_are_reached_by_whole_warps():
             body = t[start:m.start()]
             assert re.match(r"[^{]*\{\s*__syncwarp\(\);", body), names[-1]
     assert sorted(names) == ["tmem_alloc", "tmem_dealloc", "tmem_ld16", "tmem_ld32", "tmem_st16", "tmem_st32", "tmem_st8"]
+
+
+def test_tensor_memory_is_allocated_before_the_next_launch_is_let_in():
+    """A successor that is let in may take tensor memory of its own and then wait for this grid to end, so a block has its own by
+    then: a barrier of the block lies between tmem_alloc and pdl_launch.  (A block without work, which returns, has none to wait for.)"""
+    n = 0
+    for f, name, args, body in kernels():
+        if "tmem_alloc(" not in body or "pdl_launch();" not in body:
+            continue
+        n, body = n + 1, re.sub(r"//[^\n]*", "", body)
+        for m in re.finditer(r"pdl_launch\(\);", body):
+            depth, end = 1, m.end()  # of the braces that the call stands in
+            while depth and end < len(body):
+                depth += {"{": 1, "}": -1}.get(body[end], 0)
+                end += 1
+            if not body[m.end():end - 1].rstrip().endswith("return;") or end >= len(body):
+                assert re.search(r"tmem_alloc\(.*__syncthreads\(\);", body[:m.start()], re.S), (f, name)
+    assert n == 11

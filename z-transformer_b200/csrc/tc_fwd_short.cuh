@@ -63,7 +63,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
     const bool in = li * 4 < p.dim;
 
     pdl_wait();
-    pdl_launch();
     float4 x[3][NP];
     {
         const float *q = p.q + ((long long)b * p.T * p.n_heads + h) * p.dim + li * 4;
@@ -85,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
         if (sh->abort) atomicMax(&g_tc_status, 30);
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(&sh->tmem_base, 256);
+    if (warp == 1) tmem_alloc(&sh->tmem_base, 256);
 #pragma unroll
     for (int z = 0; z < 3; ++z) {
         float top = 0.f;
@@ -98,6 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_launch();  // (only now that the block has its TMEM: a successor that took more of it ahead of its own pdl_wait would wait for this grid)
     const uint32_t tmem = sh->tmem_base;
     float mult[3];
 #pragma unroll
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
             *reinterpret_cast<float4 *>(out + (long long)t * p.n_heads * p.dim) = *reinterpret_cast<const float4 *>(sQ + t * (D * 4) + ((li ^ (t & (LP - 1))) << 4));
         }
     }
-    if (warp == 0) tmem_dealloc(tmem, 256);
+    if (warp == 1) tmem_dealloc(tmem, 256);
 }
 
 template <int D>
