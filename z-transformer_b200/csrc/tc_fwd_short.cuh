@@ -4,10 +4,13 @@
 // magnitude of every (sequence, KV group), which sets the planes' scale, and one for the planes.  A short prompt is nothing but
 // the latency of that chain.  Here a block has one head's whole q, k and v in registers (a tile of 128 rows each), so that it
 // knows their maxima after one barrier, splits them itself and leaves the operands in shared memory as TMA would have:
-//   S = Ql.Kh + Qh.Kl + Qh.Kh      one accumulator of 128 x (keys, up to a multiple of 16)
+//   S = Qh.Kh + Qh.Kl + Ql.Kh      one accumulator of 128 x (keys, up to a multiple of 16)
 //   P = exp(S - max) 2^7           four warps a 32-column quarter of S, a row's maximum and sum put together through shared memory
 //   O = Pl.Vh + Ph.Vl + Ph.Vh      P in TMEM over S, V read N-major
-// with the arithmetic of attn_fwd_tc16 (three-term split on f16 pieces, f32 accumulators), the small terms of a step first.
+// with the arithmetic of attn_fwd_tc16 (three-term split on f16 pieces, f32 accumulators).  S's terms are added in its order, which is
+// the backwards' too: the tensor core truncates, and a backward that adds S otherwise than the forward whose out and log-sum-exp it
+// is given finds another P (T 128, scores that rise with the key, dq against float64, small terms first -> so: heads of 32 2.8e-6 ->
+// 1.1e-6, of 128 2.3e-6 -> 1.7e-6).  O's small terms go first, while there is little to truncate.
 // Every query head converts its KV head's k and v again; a group's heads run side by side, and even several waves of blocks, each
 // of which does so, are faster than the planes' two launches: us, planes -> this, one prompt of 77, 32/8 heads of 128 17.0 -> 8.3, of 40,
 // 4/2 of 32 12.9 -> 5.1; 8 prompts of 100, 32/8 of 128 42 -> 21, 16 of 128 70 -> 46; 16 of 128, 32/8 of 64 43 -> 29.
@@ -129,9 +132,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
 #pragma unroll 1
             for (int kk = 0; kk < steps; ++kk) {
                 const uint32_t o = (uint32_t)((kk >> 2) * BT + (kk & 3) * 32);
-                mma_ss_f16(tmem + cS, desc_advance(ql, o), desc_advance(kh, o), id_s, kk > 0);
+                mma_ss_f16(tmem + cS, desc_advance(qh, o), desc_advance(kh, o), id_s, kk > 0);
                 mma_ss_f16(tmem + cS, desc_advance(qh, o), desc_advance(kl, o), id_s, 1);
-                mma_ss_f16(tmem + cS, desc_advance(qh, o), desc_advance(kh, o), id_s, 1);
+                mma_ss_f16(tmem + cS, desc_advance(ql, o), desc_advance(kh, o), id_s, 1);
             }
             mma_commit(&sh->s_full);
         }
