@@ -106,7 +106,8 @@ inline size_t bwd_parts_floats(int batch, int T, int n_heads, int n_kv_heads, in
 inline size_t fwd_parts_floats_bound(int dim) { return (size_t)split_sm_count() * 128 * (2 * (size_t)dim + 1); }
 inline size_t bwd_parts_floats_bound(int batch, int T, int n_heads, int dim) {
     const size_t by_blocks = (size_t)4 * split_sm_count() * 128 * dim;
-    const size_t by_steps = (size_t)n_heads * ((T + 63) / 64) / 4 * 2 * batch * T * dim;  // (a part keeps 256 rows)
+    const int rows = bwd_step_rows(dim);
+    const size_t by_steps = (size_t)n_heads * ((T + rows - 1) / rows) * rows / 256 * 2 * batch * T * dim;  // (a part keeps 256 rows of whole steps)
     return by_steps < by_blocks ? by_steps : by_blocks;
 }
 
