@@ -25,3 +25,9 @@ def test_gradients_against_float64(zt, B, T, H, G, D):
     assert zt.lib.last_path() == "tcgen05" and zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
     for name, x, ref in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
         assert float((x.double() - ref).norm()) <= (6e-7 + 4e-8 * 240) * float(ref.norm()), name
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [(23, 100, 4, 2, 160), (23, 256, 2, 1, 256), (15, 380, 3, 1, 192), (12, 1024, 4, 2, 132)])
+def test_units_of_the_products_in_turn(zt, B, T, H, G, D):
+    """Enough heads for a head's units of the three products to go in turn (45 of them on 148 SMs at these lengths, 89 of up to 128 rows)."""
+    test_gradients_against_float64(zt, B, T, H, G, D)

@@ -75,6 +75,7 @@ struct WideParams {
     int dim_out, td;                   // the tensors' head_dim, the planes' (192 or 256)
     int unit0, unit_cap;               // the chunk: units (b * n_heads + h) from unit0; planes allocated for unit_cap
     int units, pieces;                 // wide_products: units of the chunk, pieces of kPiece along one head's contraction
+    bool in_turn;                      // and the order of its units (products_in_turn)
     float scale, scale_log2, p_scale;
 };
 
@@ -565,10 +566,11 @@ inline size_t res_smem_bytes() { return (size_t)(2 * D / 64 + 2 * res_slots<D>()
 // prologue and epilogue together when each was a block of its own.  So a block walks its share of the units with two
 // accumulators in TMEM (all 512 columns), loads run ahead across units, and a unit's epilogue -- straight from TMEM to
 // memory, rows regrouped among eight lanes -- runs under the next one's MMAs.  A head's tiles are consecutive units:
-// blocks that run together share its operands in L2.  Where a tile is one unit (T up to 1024) so are those of its three products,
-// in turn, and dS is still in L2 when the second of its two products reads it; longest first, and the other way round in every
-// second head, so that what a block gets by its stride is neither always long nor always short.  (With pieces this was 5 % slower,
-// T 3000: 789 -> 827.)  Batch 8, T 1024, 32/8 heads of 256, with dQ stored instead of added: 775 -> 687.
+// blocks that run together share its operands in L2.  Where a tile is one unit (T up to 1024) and
+// products_in_turn allows it, so are those of its three products, in turn, and dS is still in L2 when the second of its two products reads it;
+// longest first, and the other way round in every second head, so that what a block gets by its stride is neither always long nor
+// always short.  (With pieces this was 5 % slower, T 3000: 789 -> 827.)  Batch 8, T 1024, 32/8 heads of 256, in the order of the
+// products / in turn: 773 / 702 (and 785 with dQ added instead of stored).
 // Us, three launches of a block per unit -> this: batch 8, T 1024, 32/8 heads of 256 809 -> 777 (bound by DRAM: the planes are
 // 3 GB written and read there); forward and backward at batch 4, T 300, 8/2 heads 129 -> 111, one sequence of T 500, 4/2
 // heads of 160 130 -> 102.
@@ -589,12 +591,23 @@ __device__ __forceinline__ void tgive_up(TriShared *sh, int code) {
     sh->abort = code;
     atomicMax(&g_tc_status, code);
 }
+// Whether a head's units of the three products go in turn: where no block gets much more than the others.  The units repeat every two
+// heads, 6 nt of them; a block finds its next one `blocks` further on, which moves its place in that period by `drift`, so few
+// rounds leave it among the long ones (T 1024, 36 heads on 148 blocks: 25 % above the order of the products), and it is as good once
+// they have gone through three fifths of the period.  Us, in the order of the products / in turn, heads of 192 and of 256 columns:
+// T 1024, 16 heads 53.8 / 61.2 and 62 / 71, 32 88.5 / 91.6 and 99 / 101, 64 156 / 154 and 191 / 188, 256 637 / 560 and 773 / 702; T 500, 32
+// 32.4 / 35.2 and 38.2 / 41.5, 64 59.5 / 55.9 and 70.8 / 67.0.
+__host__ __device__ inline bool products_in_turn(int pieces, int nt, int heads, int blocks) {
+    const int place = blocks % (6 * nt), drift = place < 6 * nt - place ? place : 6 * nt - place;
+    return pieces == 1 && 5LL * heads * drift >= 6LL * blocks;
+}
+
 struct TriUnit {
     int which, u, m0, b, h, k_begin, n_steps;  // which: 0 dQ, 1 dK, 2 dV; n_steps <= 0: nothing to do
-    __device__ __forceinline__ TriUnit(const WideParams &p, int i) {
+    __host__ __device__ __forceinline__ TriUnit(const WideParams &p, int i) {
         const int nt = p.Tp / 128;
         int m, piece = 0;
-        if (p.pieces == 1) {
+        if (p.in_turn) {
             u = i / (3 * nt);
             const int at = i - u * 3 * nt, r = u & 1 ? 3 * nt - 1 - at : at, level = r / 3;
             which = r - 3 * level;
@@ -938,6 +951,7 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         p.units = units;
         const long long n_units = 3LL * nt * units * p.pieces;
         const dim3 gp((unsigned)(n_units < split_sm_count() ? n_units : split_sm_count()));
+        p.in_turn = products_in_turn(p.pieces, nt, units, split_sm_count());
         if (launch_after("wide_products", products, gp, dim3(kTriThreads), smem_t, stream, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
             return 1;
     }
