@@ -36,3 +36,12 @@ def test_planes_of_small_forwards(zt, B, T, H, G, D, one):
     assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 1e-5
     for name, x, r in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
         assert float((x.double() - r).norm()) <= (6e-7 + 4e-8 * 240) * float(r.norm()), name
+
+
+@pytest.mark.parametrize("B,T,H,G,D,one", [
+    (36, 64, 16, 4, 64, True), (64, 64, 16, 4, 64, False),   # a quarter of the room in use: four waves of blocks
+    (20, 33, 32, 4, 32, True), (24, 33, 32, 4, 32, False),   # 0.107 of it: 1.7 waves
+    (64, 103, 16, 4, 64, True), (64, 60, 16, 16, 128, True)  # two fifths and more: any number
+])
+def test_planes_of_small_forwards_in_many_blocks(zt, B, T, H, G, D, one):
+    test_planes_of_small_forwards(zt, B, T, H, G, D, one)

@@ -541,6 +541,24 @@ inline bool pass_takes_one(const PassArgs &a, int units) {
     }
     return a.n_fill == 0;
 }
+inline int pass_sm_count() {
+    const DeviceInfo *d = device_info();
+    return d ? d->sm_count : 0;
+}
+// Whether it pays in the form of 16 float4 a thread, where a block has an SM to itself however few units its (sequence, group) has -- and
+// with a group of query heads k's and v's have few.  Two fifths of the room in use pay for any number of blocks; below that the fewer the
+// fewer waves.  Us, forward and backward of heads of 64, two launches / one: 16/4 heads, T 64 (a quarter in use), batch 32 81 / 79,
+// 64 138 / 144, 256 445 / 474; T 100 (0.39), 64 175 / 172, 256 576 / 584; 32/8, T 120 (0.47), 64 357 / 351, 256 1240 / 1235; 32/4 heads
+// of 32, T 33 (0.11), 4 40 / 39, 64 173 / 181, 256 591 / 630.
+inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
+    long long blocks = 0, held = 0;
+    for (int i = 0; i < a.n; ++i) {
+        const PassTensor &t = a.t[i];
+        blocks += (long long)t.batch * (t.heads / t.group), held += (long long)t.batch * t.rows * t.heads;
+    }
+    const long long room = blocks * units;
+    return 5 * held >= 2 * room || (double)blocks * room <= 16. * held * sms;
+}
 template <int LP, int NC, int CHUNKS>
 inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
     long long blocks = 0;
@@ -576,7 +594,8 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     const auto both = [&](auto lanes, auto chunks) -> int {
         constexpr int LP = lanes.value, NC = chunks.value;
         if (pass_takes_one(a, pass_one_units<LP, NC, kOneFew>())) return launch_pass_one<LP, NC, kOneFew>(a, stream);
-        if (pass_takes_one(a, pass_one_units<LP, NC, kOneMost>())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
+        constexpr int most = pass_one_units<LP, NC, kOneMost>();
+        if (pass_takes_one(a, most) && pass_one_pays(a, most, pass_sm_count())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
