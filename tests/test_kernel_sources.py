@@ -61,17 +61,35 @@ def test_aligned_tensor_memory_instructions_are_reached_by_whole_warps():
     """tcgen05.alloc, dealloc, ld, st and their waits are .sync.aligned: all threads of a warp execute them together.  They follow
     code that ends lane by lane (rows past the sequence, columns past the head, one lane's arrival), so the wrapper
     brings the warp together itself, and nothing but the wrappers issues them; a wait comes straight after the ones it is for or a
-    vote of the whole warp."""
+    vote of the whole warp.  A wrapper that does not (_joined) is called behind a vote, with no branch of a lane's own in between."""
     text = sources()
-    names = []
+    names, joined = [], []
     for name, t in text.items():
         for m in re.finditer(r"tcgen05\.(?:alloc|dealloc|ld|st)[.\w:]*\.sync\.aligned", t):
             assert name == "tc_common.cuh", name
             start = t.rindex("__device__", 0, m.start())
             names.append(re.match(r"__device__ __forceinline__ void (\w+)\(", t[start:])[1])
+            if names[-1].endswith("_joined"):
+                joined.append(names[-1])
+                continue
             body = t[start:m.start()]
             assert re.match(r"[^{]*\{\s*__syncwarp\(\);", body), names[-1]
-    assert sorted(names) == ["tmem_alloc", "tmem_dealloc", "tmem_ld16", "tmem_ld32", "tmem_st16", "tmem_st32", "tmem_st8"]
+    assert sorted(n.removesuffix("_joined") for n in names) == ["tmem_alloc", "tmem_dealloc", "tmem_ld16", "tmem_ld32", "tmem_st16", "tmem_st32", "tmem_st8"]
+    for n in joined:
+        assert re.search(r"void %s\([^{]*\{\s*__syncwarp\(\);\s*%s\(taddr, r\);" % (n.removesuffix("_joined"), n), text["tc_common.cuh"]), n
+    uniform = {"if (diag)", "for (int c = 0; c < D; c += 32)", "for (int i = 0; i < 32; ++i)"}
+    calls = 0
+    for name, t in text.items():
+        if name == "tc_common.cuh":
+            continue
+        for m in re.finditer(r"tmem_\w+_joined\(", t):
+            calls += 1
+            vote = max(t.rfind(x, 0, m.start()) for x in ("__all_sync(", "__any_sync(", "__syncwarp();"))
+            between = t[t.index("\n", vote):m.start()]
+            between = re.sub(r"//[^\n]*", "", between)
+            branches = re.findall(r"\b(?:if|for|while|switch) \([^\n]*?\)(?= |$)", between, re.M)
+            assert set(branches) <= uniform and "break" not in between.split("}", 1)[-1], (name, branches)
+    assert calls == 24
 
 
 def test_tensor_memory_is_allocated_before_the_next_launch_is_let_in():

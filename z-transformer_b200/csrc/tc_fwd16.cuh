@@ -406,8 +406,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int s0 = (jb + j) * BN;
             const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
-            tmem_ld32(tmem + lane_base + cS, r0);
-            tmem_ld32(tmem + lane_base + cS + 32, r1);
+            tmem_ld32_joined(tmem + lane_base + cS, r0);
+            tmem_ld32_joined(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
             float mt = -INFINITY;
             if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
@@ -422,7 +422,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (ZT_DEFECT(3) && j > 0) factor = 1.f;
             l *= factor;
             const bool flush = FLUSH && j > 1 && (j >> 1) % kFlushKeyTiles == 0;
-            if (j > 1 && (flush || __any_sync(0xffffffffu, factor != 1.f))) {
+            const bool moved = __any_sync(0xffffffffu, factor != 1.f);
+            if (j > 1 && (flush || moved)) {
                 // this set's O may only be touched once its previous P.V (tile j-2) has retired
                 if (!__all_sync(0xffffffffu, fwait(&sh->pv_done[set], (uint32_t)(((j >> 1) - 1) & 1), sh))) {
                     fgive_up(sh, 46);
@@ -434,15 +435,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const bool first = m_flushed == -INFINITY;
                     flush_row<D>(tmem + lane_base + cO, set == 0 ? row0 : row1, first ? 0.f : ex2(m_flushed - m_old), first);
                     m_flushed = m_old;
+                    __syncwarp();  // (rows past the sequence were not summed)
                 } else {
 #pragma unroll 1
                     for (int c = 0; c < D; c += 32) {
                         uint32_t r[32];
-                        tmem_ld32(tmem + lane_base + cO + c, r);
+                        tmem_ld32_joined(tmem + lane_base + cO + c, r);
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * factor);
-                        tmem_st32(tmem + lane_base + cO + c, r);
+                        tmem_st32_joined(tmem + lane_base + cO + c, r);
                     }
                 }
             }
@@ -452,11 +454,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             {
                 uint32_t ph[16], pl[16];
                 psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
-                tmem_st16(tmem + lane_base + cS, ph);
-                tmem_st16(tmem + lane_base + cS + 16, pl);
+                tmem_st16_joined(tmem + lane_base + cS, ph);
+                tmem_st16_joined(tmem + lane_base + cS + 16, pl);
                 psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
-                tmem_st16(tmem + lane_base + cS + 32, ph);
-                tmem_st16(tmem + lane_base + cS + 48, pl);
+                tmem_st16_joined(tmem + lane_base + cS + 32, ph);
+                tmem_st16_joined(tmem + lane_base + cS + 48, pl);
             }
             l += psum;
             tmem_wait_st();
