@@ -46,3 +46,11 @@ def test_gradients_against_float64(zt, B, T, H, G, D, scale):
         assert float((x.double() - ref).norm()) <= (6e-7 + 4e-8 * n) * float(ref.norm()), name
     again = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws)
     assert torch.equal(got[1], again[1]) and torch.equal(got[2], again[2])  # (sums of dk and dv are made in the order of the walk)
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [
+    (1, 33, 4, 2, 32), (2, 48, 8, 2, 64), (3, 63, 3, 3, 36), (5, 64, 16, 16, 60), (1, 64, 32, 4, 64),  # (the last one: split by heads)
+    (64, 37, 32, 4, 32), (40, 64, 16, 4, 40), (1, 65, 8, 2, 64),  # (tile by tile; sequence by sequence; the first of steps of 128)
+])
+def test_steps_of_64_rows(zt, B, T, H, G, D):
+    test_gradients_against_float64(zt, B, T, H, G, D, (1, 1, 1, 1))

@@ -684,7 +684,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     }
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
     if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
-    const int rows = fused ? bwd_step_rows(dim) : 64;  // of a query tile
+    const int rows = fused && td == 64 ? tcf::fused64_rows(T) : 64;  // of a query tile
     BwdMaps m;
     bool maps = make_head_map(&m.k128, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
                 make_head_map(&m.v128, w.v_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&
@@ -720,7 +720,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
         const long long n = (long long)batch * T * n_kv_heads * dim;
         p.dk = w.parts, p.dv = w.parts + n, p.dkv_part = 2 * n;
         if (launch(m.k128, m.v128, m.q64, m.g64, p, stream)) return 1;
-        return launch_bwd_join(w.parts, dk, dv, batch, T, n_kv_heads * dim, p.parts, rows, stream);
+        return launch_bwd_join(w.parts, dk, dv, batch, T, n_kv_heads * dim, p.parts, bwd_step_rows(dim), stream);
     }
     return td == 64 ? launch_bwd_tc_d<64>(m, p, stream) : launch_bwd_tc_d<128>(m, p, stream);
 }

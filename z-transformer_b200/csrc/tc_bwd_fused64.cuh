@@ -2,7 +2,7 @@
 // 128 query rows instead of 64.
 //
 // A head of 64 columns leaves half of what a 128-column head fills: with steps of 64 rows the row threads' hand-offs, not
-// the tensor core, were what a step took (5500 clocks of it, 35 % of them with the tensor pipe active).  Here a step is a
+// the tensor core, were what a step took (5500 clocks; the tensor pipe was active for 29 % of a launch at batch 8, T 512).  Here a step is a
 // tile of 128 x 128 scores:
 //  * S^T and dP^T are MMAs of N = 128, which cost 64 clocks where two of N = 64 cost 106, and a step's barriers,
 //    polls and row constants serve twice the elements;
@@ -15,12 +15,18 @@
 //    broadcast LDS.128 is two wavefronts, and a step is bound by shared memory: 2800 wavefronts of the row threads' and
 //    about 3900 of the tensor core's operands, as 128 bytes a clock);
 //  * the row threads' arithmetic is paired (fma.rn.f32x2).
-// 16 row warps, a thread per key row and 32 of the step's query columns, at 80 registers a thread.
+// 16 row warps, a thread per key row and 32 of the step's query columns, at 80 registers a thread (all that 768 threads leave; the
+// variants for split walks and padded heads spill 16 to 24 bytes).
+// Sequences of up to 64 rows have half a step: ROWS = 64, a step of 128 x 64 scores, 16 query columns a row thread.  (Us, this kernel, steps
+// of 128 -> of 64 rows: T 64, batch 64, 16/4 heads of 64 53.5 -> 45.5, one sequence of 16/16 heads of 32 14.8 -> 12.8; T 33, batch 256,
+// 32/4 heads of 32 266 -> 208.  With T 129 to 192, whose second step is as empty, -10 to +10 %: those keep steps of 128.)
 // TMEM: V hi 32 (of 64), S^T/P^T 128, dP^T/dS^T 128, dQ 64, dV 64, dK 64 = 512 columns.  Shared memory: K hi/lo, V lo 48 KB,
 // dS^T hi/lo 64 KB, two Q slots and one dO slot of 32 KB each, 16 KB on the way out = 224 KB.
 // Measured (us, before -> after, this kernel): 32/8 heads of 64, batch 8, T 512 139 -> 104, T 4096, batch 1 643 -> 448; heads
-// of 32, batch 8, T 512 121 -> 94.  Error against 64 bits (2-norm, relative; T 1000, 8/2 heads of 64): dq 8.0e-7 -> 5.7e-7, dk
-// 1.07e-6 -> 8.6e-7, dv 8.2e-7 -> 7.5e-7.
+// of 32, batch 8, T 512 121 -> 94.  Error against 64 bits (2-norm, relative, N(0, 1); batch 2, T 512, 8/2 heads of 64): dq 8.0e-7 -> 5.8e-7, dk
+// 9.2e-7 -> 6.9e-7, dv 7.3e-7 -> 6.2e-7.  (dQ sums three of the four products of the pieces where the kernel before it had all four: with
+// lo.lo as well, 32 MMAs for 24, its error is the same to 1 %.  What moves it is dP's small terms going first; with its large ones
+// first dq 7.2e-7.  Where the softmax is saturated on a few keys, dP and delta cancel and either order is within 9 % of the kernel before.)
 #pragma once
 
 #include "tc_bwd_wide.cuh"
@@ -95,14 +101,14 @@ constexpr int kFused64Threads = (kKvRowWarps + 8) * 32, kReadWarps = 4;
 constexpr size_t kFused64Smem = 3 * (size_t)(128 * 64 * 2) + 2 * (size_t)(128 * 128 * 2) + 6 * (size_t)(128 * 64 * 2) +
                                 kReadWarps * 4096 + sizeof(Fused64Shared);
 
-// PARTS, PAD: as in attn_bwd_fused_tc.
-template <bool PARTS, bool PAD>
+// PARTS, PAD: as in attn_bwd_fused_tc.  ROWS: query rows of a step, 128, or 64 for sequences that have no more.
+template <bool PARTS, bool PAD, int ROWS>
 __global__ void __launch_bounds__(kFused64Threads, 1)
     attn_bwd_fused64_tc(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                         const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap gmap,
                         const __grid_constant__ CUtensorMap dqmap, const __grid_constant__ CUtensorMap dkmap,
                         const __grid_constant__ CUtensorMap dvmap, const BwdParams p) {
-    constexpr int D = 64, BQ = 128, BR = 128 * 128;  // BR: bytes of 128 rows of 64 halves, every operand block's size
+    constexpr int D = 64, BQ = ROWS, BR = 128 * 128;  // BR: bytes of 128 rows of 64 halves, every operand block's size
     constexpr int KP = BR, QP = BR, DSP = 2 * BR;    // one plane of K, of a query tile, of dS^T (two blocks of 64 query columns)
     const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cVh = 0, cST = 64, cDPT = 192, cDQ = 320, cDV = 384, cDK = 448;
@@ -123,7 +129,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
     // this CTA's part of the walk: heads [head0, head0 + n_heads_mine) and query tiles [qi0, n_q)
     const int n_heads_mine = PARTS ? group / p.parts.heads : group;
     const int head0 = PARTS ? g * group + part / p.parts.ranges * n_heads_mine : g * group;
-    int n_q = (p.T + BQ - 1) / BQ, qi0 = kt;
+    int n_q = (p.T + BQ - 1) / BQ, qi0 = kt * (128 / BQ);
     if (PARTS && p.parts.ranges > 1) {
         const int per = (n_q - qi0 + p.parts.ranges - 1) / p.parts.ranges;
         qi0 += part % p.parts.ranges * per;
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
         mbar_init(&sh->p_ready, kKvRowWarps);
         mbar_init(&sh->ds_ready, kKvRowWarps);
         mbar_init(&sh->dq_done, 1);
-        mbar_init(&sh->dq_free, kReadWarps);
+        mbar_init(&sh->dq_free, BQ / 32);
         mbar_init(&sh->ld_ready, 1);
         mbar_init(&sh->flush_ready, 2);  // (dK's issuer and dV's)
         mbar_init(&sh->dv_free, kReadWarps), mbar_init(&sh->dk_free, kReadWarps);
@@ -189,7 +195,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 const int j = n_ql, s = j & 1;
                 // (its slot was last read by dK(j - 2))
                 if (j >= 2 && !fwait(&sh->free_q[s], (uint32_t)((((j >> 1) - 1) & 1)), sh)) { fgive_up(sh, 71), live = false; return; }
-                mbar_arrive_expect_tx(&sh->full_q[s], 2 * QP);
+                mbar_arrive_expect_tx(&sh->full_q[s], 2 * BQ * 128);
                 load_head<1>(sQ + s * 2 * QP, &qmap, &sh->full_q[s], wq.qi * BQ, head0 + wq.hh, b, BR, padded);
                 load_head<1>(sQ + s * 2 * QP + QP, &qmap, &sh->full_q[s], wq.qi * BQ, head0 + wq.hh, B + b, BR, padded);
                 ++n_ql, wq.next();
@@ -198,7 +204,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 const int j = n_gl;
                 // (the one slot was last read by dV(j - 1) and dP^T(j - 1))
                 if (j >= 1 && !fwait(&sh->free_g, (uint32_t)((j - 1) & 1), sh)) { fgive_up(sh, 71), live = false; return; }
-                mbar_arrive_expect_tx(&sh->full_g, 2 * QP);
+                mbar_arrive_expect_tx(&sh->full_g, 2 * BQ * 128);
                 load_head<1>(sG, &gmap, &sh->full_g, wg.qi * BQ, head0 + wg.hh, b, BR, padded);
                 load_head<1>(sG + QP, &gmap, &sh->full_g, wg.qi * BQ, head0 + wg.hh, B + b, BR, padded);
                 ++n_gl, wg.next();
@@ -382,12 +388,13 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
         // head of every step and the arithmetic took a sixth of their instructions.)
         const int lane = threadIdx.x & 31;
         const float lse_shift = log2f(p.p_scale), ndel_unit = 1.0f / (p.p_scale * pow2_of(unit));
-        float lse[4], rn[4], de[4];
+        constexpr int NR = BQ / 32;
+        float lse[NR], rn[NR], de[NR];
         int t0 = walk.qi * BQ + lane;
         const auto load = [&]() {
             t0 = walk.qi * BQ + lane;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NR; ++i) {
                 const int t = t0 + i * 32;
                 const long long idx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + head0 + walk.hh;
                 lse[i] = __ldg(p.lse + idx), rn[i] = __ldg(p.rnorm + idx), de[i] = __ldg(p.delta + idx);
@@ -395,9 +402,9 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
         };
         load();
         for (int it = 0; it < n_it; ++it) {
-            float csc[4], nlse[4], ndel[4];
+            float csc[NR], nlse[NR], ndel[NR];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NR; ++i) {
                 const bool in = t0 + i * 32 < p.T;
                 float cq, rel;
                 ds_row_scale(rn[i], rn_bits, vn_bits, cq, rel);
@@ -413,7 +420,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 break;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NR; ++i) {
                 const int r = i * 32 + lane;
                 sh->csc[r] = csc[i], sh->nlse[r] = nlse[i], sh->ndel[r] = ndel[i];
             }
@@ -454,7 +461,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             // this lane's query row of the step: 1 / (the scale of dS)
             const int t0 = walk.qi * BQ + q32;
             float fq = 0.f;
-            if (t0 + lane < p.T) {
+            if (q32 < BQ && t0 + lane < p.T) {
                 float cq, rel;
                 ds_row_scale(__ldg(p.rnorm + ((long long)b * p.T + t0 + lane) * p.n_heads + head0 + walk.hh), rn_bits, vn_bits, cq, rel);
                 fq = dq_unit / cq;
@@ -480,6 +487,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 }
                 ++n_flush;
             }
+            if (q32 >= BQ) continue;  // (no query rows of the step)
             if (!__all_sync(0xffffffffu, fwait(&sh->dq_done, (uint32_t)(it & 1), sh))) {
                 fgive_up(sh, 76);
                 break;
@@ -498,6 +506,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
     } else {
         // ------------------------------------------------------------------ one thread per key row and
         // 32 of the step's query columns: set `set` handles columns [32 set, 32 set + 32)
+        constexpr int CW = BQ / 4;
         const int tid = threadIdx.x & 127, set = threadIdx.x >> 7;
         const int lane = threadIdx.x & 31;
         const int key = s0 + tid;
@@ -524,16 +533,16 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                 break;
             }
             tc_fence_after();
-            const uint32_t wS = tmem + lane_base + cST + set * 32;
-            const uint32_t wP = tmem + lane_base + cDPT + set * 32;
-            float2 pr[16];
+            const uint32_t wS = tmem + lane_base + cST + set * CW;
+            const uint32_t wP = tmem + lane_base + cDPT + set * CW;
+            float2 pr[CW / 2];
             {
-                const float4 *csc = reinterpret_cast<const float4 *>(sh->csc + set * 32);
-                const float4 *nlse = reinterpret_cast<const float4 *>(sh->nlse + set * 32);
-                const int q_first = walk.qi * BQ, t0 = q_first + set * 32;
+                const float4 *csc = reinterpret_cast<const float4 *>(sh->csc + set * CW);
+                const float4 *nlse = reinterpret_cast<const float4 *>(sh->nlse + set * CW);
+                const int q_first = walk.qi * BQ, t0 = q_first + set * CW;
                 const bool plain = (q_first >= s0 + 127 || ZT_DEFECT(11)) && q_first + BQ <= p.T && s0 + 128 <= p.T;
 #pragma unroll
-                for (int w = 0; w < 2; ++w) {
+                for (int w = 0; w < CW / 16; ++w) {
                     uint32_t rs[16], ph[8], pl[8];
                     tmem_ld16(wS + 16 * w, rs);
                     tmem_wait_ld();
@@ -570,10 +579,10 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             {
                 // The values go to the tensor core twice: over dP^T, and as a row of dQ's A operand -- key row `tid`, four 16-byte
                 // chunks of its 128 bytes in the block of 64 query columns that they belong to, 128-byte swizzled.
-                uint8_t *row_h = sDS + (set >> 1) * BR + tid * 128;
-                const float4 *ndel = reinterpret_cast<const float4 *>(sh->ndel + set * 32);
+                uint8_t *row_h = sDS + (set * CW >> 6) * BR + tid * 128;
+                const float4 *ndel = reinterpret_cast<const float4 *>(sh->ndel + set * CW);
 #pragma unroll
-                for (int w = 0; w < 2; ++w) {
+                for (int w = 0; w < CW / 16; ++w) {
                     uint32_t rd[16];
                     tmem_ld16(wP + 16 * w, rd);
                     tmem_wait_ld();
@@ -596,7 +605,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                     if (w == 0 && it >= 1) free = __all_sync(0xffffffffu, fwait(&sh->dq_done, (uint32_t)((it - 1) & 1), sh));
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
-                        const int at = ((4 * (set & 1) + 2 * w + c) ^ (tid & 7)) << 4;
+                        const int at = (((set * CW & 63) / 8 + 2 * w + c) ^ (tid & 7)) << 4;
                         *reinterpret_cast<uint4 *>(row_h + at) = make_uint4(th[4 * c], th[4 * c + 1], th[4 * c + 2], th[4 * c + 3]);
                         *reinterpret_cast<uint4 *>(row_h + DSP + at) = make_uint4(tl[4 * c], tl[4 * c + 1], tl[4 * c + 2], tl[4 * c + 3]);
                     }
@@ -618,6 +627,9 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
     if (warp == kKvRowWarps + 1) tmem_dealloc(tmem, 512);
 }
 
+// Query rows of a step.  (One variant at 64 for whole and split walks, padded and whole heads.)
+inline int fused64_rows(int T) { return T <= 64 ? 64 : 128; }
+
 inline int launch_bwd_fused64(const CUtensorMap &k128, const CUtensorMap &v128, const CUtensorMap &qs128, const CUtensorMap &g128,
                               const BwdParams &p, cudaStream_t stream) {
     CUtensorMap dqmap, dkmap, dvmap;
@@ -626,7 +638,8 @@ inline int launch_bwd_fused64(const CUtensorMap &k128, const CUtensorMap &v128, 
         !make_out_map(&dkmap, p.dk, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32) ||
         !make_out_map(&dvmap, p.dv, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32))
         return refuse("the TMA tensor maps for the backward's gradients could not be encoded.");
-    const auto kernel = with_flags([](auto parts, auto pad) { return attn_bwd_fused64_tc<parts.value, pad.value>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < 4);
+    const auto kernel = fused64_rows(p.T) == 64 ? attn_bwd_fused64_tc<true, true, 64>
+                                  : with_flags([](auto parts, auto pad) { return attn_bwd_fused64_tc<parts.value, pad.value, 128>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < 4);
     if (optin_smem((const void *)kernel, kFused64Smem)) return 1;
     const unsigned tiles = (unsigned)((p.T + 127) / 128), seqs = (unsigned)(p.batch * p.parts.n()), kv = (unsigned)p.n_kv_heads;
     const dim3 grid = p.by_tile ? dim3(kv, seqs, tiles) : dim3(kv, tiles, seqs);

@@ -60,7 +60,8 @@ inline size_t fwd_parts_floats(int batch, int T, int n_heads, int dim, int q_off
     return n < 2 ? 0 : n * rows * ((q_offset > 0 ? 2 : 1) * (size_t)dim + 1);
 }
 
-// Parts of the backward's walk: heads x ranges of query tiles.  A step is a query tile of bwd_step_rows rows of one head.
+// Parts of the backward's walk: heads x ranges of query tiles.  A step is a query tile of bwd_step_rows rows of one head.  (Of one
+// tile, where all there are is 64 rows at 64 columns.)
 constexpr int bwd_step_rows(int dim) { return dim <= 64 ? 128 : 64; }
 struct BwdParts {
     int heads, ranges;
