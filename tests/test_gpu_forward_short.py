@@ -40,24 +40,6 @@ def test_against_float64(zt, B, T, H, G, D, scale):
     assert torch.equal(out, zt.attention_forward(q, k, v, H, G, D))
 
 
-@pytest.mark.parametrize("B,T,H,G,D,one", [
-    (256, 33, 32, 1, 32, True), (257, 33, 32, 1, 32, False), (129, 64, 64, 2, 32, False),  # the planes: waves of 32-column heads, groups of 32
-    (129, 65, 64, 2, 32, True), (129, 64, 64, 2, 36, True), (129, 40, 64, 4, 32, True),
-])
-def test_many_heads_of_one_group(zt, B, T, H, G, D, one):
-    gen = torch.Generator(device="cuda")
-    gen.manual_seed(19)
-    q, k, v = (torch.randn((B, T, w * D), device="cuda", generator=gen) for w in (H, G, G))
-    n0 = zt.lib.launch_count()
-    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True)
-    assert (zt.lib.launch_count() - n0 == 1) == one
-    torch.cuda.synchronize()
-    assert zt.lib.tc_status() == 0
-    ref, ref_lse = forward64(q, k, v, H, G, D, 0)
-    assert float((out.double() - ref).norm()) <= 3e-6 * float(ref.norm())
-    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 1e-5
-
-
 @pytest.mark.parametrize("t,off,D", [(1, 40, 64), (16, 17, 128), (50, 78, 80), (20, 100, 32)])
 def test_windows_of_short_prompts(zt, t, off, D):
     H, G = 8, 2

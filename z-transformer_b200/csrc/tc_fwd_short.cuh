@@ -231,14 +231,9 @@ inline int launch_d(const Params &p, int batch, cudaStream_t stream) {
 
 }  // namespace tcshort
 
-// Which forwards take it: every key in one tile, heads of up to 128 columns.  (Not where every one of 32 query heads or more converts the
-// same k and v again, these are rows of 32 columns or less, half of the tile's rows are empty and there are waves of blocks: us, planes ->
-// this, T 33, 64/1 heads of 32, batch 128 234 -> 227, 256 467 -> 479, 1024 1811 -> 1896; 32/1, 2048 1844 -> 1897; 16 query heads a group,
-// 1938 -> 1907; 64/1 heads of 48, 1024 1962 -> 1952; T 100, 64/1 of 32, 256 649 -> 637.)
-inline bool tc_fwd_short_takes(int batch, int T, int q_offset, int n_heads, int n_kv_heads, int dim) {
-    const int keys = q_offset + T;
-    const bool again = n_heads / n_kv_heads >= 32 && dim <= 32 && keys <= 64 && (long long)n_heads * batch > 8192;
-    return keys <= tcshort::kMaxKeys && dim <= 128 && batch <= 65535 && !again;
+// Which forwards take it: every key in one tile, heads of up to 128 columns.
+inline bool tc_fwd_short_takes(int batch, int T, int q_offset, int dim) {
+    return q_offset + T <= tcshort::kMaxKeys && dim <= 128 && batch <= 65535;
 }
 
 // (after tc_fwd16_supported)  k and v hold n_keys rows a sequence, of which those from q_offset + T on are not read.

@@ -187,7 +187,7 @@ static int forward_impl(const float *q, const float *k, const float *v, float *o
         const bool own = q_offset != 0 || n_keys != T || workspace_optional(T, dim);
         // Up to 128 keys need no planes.  (A shape that takes the device's arena asks for it all the same: inside a capture that may
         // have to be refused.)
-        const bool brief = path == 0 && tc_fwd_short_takes(batch, T, q_offset, n_heads, n_kv_heads, dim);
+        const bool brief = path == 0 && tc_fwd_short_takes(batch, T, q_offset, dim);
         if (brief && own) return launch_fwd_short(q, k, v, out, lse, batch, T, q_offset, n_keys, n_heads, n_kv_heads, dim, stream);
         const StreamScratch scratch(own ? need : 0, stream);
         bool in_capture = false;
