@@ -12,8 +12,8 @@
 //  * dQ, dK and dV leave by TMA (a reduction in memory), read out of TMEM by four warps of their own.  As
 //    red.global.add.v4 the 32 KB of a step's dQ took 4300 clocks of an SM, 8 bytes a clock, and a flush of dK and dV 8000;
 //  * the constants of a step's query rows are worked out by a warp of their own, a step ahead, and are three a row (a
-//    broadcast LDS.128 is two wavefronts, and a step is bound by shared memory: 2800 wavefronts of the row threads' and
-//    about 3900 of the tensor core's operands, as 128 bytes a clock);
+//    broadcast LDS.128 is two wavefronts, and a step is bound by shared memory: 2500 wavefronts of loads and stores, 3200 of
+//    the tensor core's operands and 770 of the copies', at 128 bytes a clock);
 //  * the row threads' arithmetic is paired (fma.rn.f32x2).
 // 16 row warps, a thread per key row and 32 of the step's query columns, at 80 registers a thread (all that 768 threads leave; the
 // variants for split walks and padded heads spill 16 to 24 bytes).

@@ -231,7 +231,10 @@ inline int launch_d(const Params &p, int batch, cudaStream_t stream) {
 
 }  // namespace tcshort
 
-// Which forwards take it: every key in one tile, heads of up to 128 columns.
+// Which forwards take it: every key in one tile, heads of up to 128 columns, for any number of blocks.  At its far end every one of a group's
+// query heads converts the same k and v again: us, planes -> this, T 33, heads of 32, batch 2048, 32/8 heads 1978 -> 1950, 32/2 1938 -> 1907,
+// 32/1 1844 -> 1897; 64/1, batch 128 234 -> 227, 256 467 -> 479, 1024 1811 -> 1896; 64/1 heads of 48 1962 -> 1952; T 100, 64/1 of 32, batch
+// 256 649 -> 637.  (What 32 query heads a group lose beyond 8192 blocks is not worth a scratch, which leaves memory nodes in a graph.)
 inline bool tc_fwd_short_takes(int batch, int T, int q_offset, int dim) {
     return q_offset + T <= tcshort::kMaxKeys && dim <= 128 && batch <= 65535;
 }
