@@ -39,9 +39,11 @@ def test_planes_of_small_forwards(zt, B, T, H, G, D, one):
 
 
 @pytest.mark.parametrize("B,T,H,G,D,one", [
-    (36, 64, 16, 4, 64, True), (64, 64, 16, 4, 64, False),   # a quarter of the room in use: four waves of blocks
-    (20, 33, 32, 4, 32, True), (24, 33, 32, 4, 32, False),   # 0.107 of it: 1.7 waves
-    (64, 103, 16, 4, 64, True), (64, 60, 16, 16, 128, True)  # two fifths and more: any number
+    (36, 64, 16, 4, 64, True), (64, 64, 16, 4, 64, False),     # a quarter of the room in use, groups of four: five waves of blocks
+    (64, 78, 16, 4, 64, True), (128, 78, 16, 4, 64, False),    # 0.305: 7.4
+    (9, 33, 32, 4, 32, True), (24, 33, 32, 4, 32, False),      # 0.107, groups of eight: 0.9
+    (64, 130, 16, 16, 64, True), (128, 130, 16, 16, 64, False),  # 0.254, no groups: 29
+    (128, 103, 16, 4, 64, True), (64, 60, 16, 16, 128, True),  # two fifths: any number; the form of 4 float4
 ])
 def test_planes_of_small_forwards_in_many_blocks(zt, B, T, H, G, D, one):
     test_planes_of_small_forwards(zt, B, T, H, G, D, one)

@@ -543,21 +543,25 @@ inline bool pass_takes_one(const PassArgs &a, int units) {
 }
 inline int pass_sm_count() {
     const DeviceInfo *d = device_info();
-    return d ? d->sm_count : 0;
+    return d && d->sm_count > 0 ? d->sm_count : 148;
 }
-// Whether it pays in the form of 16 float4 a thread, where a block has an SM to itself however few units its (sequence, group) has -- and
-// with a group of query heads k's and v's have few.  Two fifths of the room in use pay for any number of blocks; below that the fewer the
-// fewer waves.  Us, forward and backward of heads of 64, two launches / one: 16/4 heads, T 64 (a quarter in use), batch 32 81 / 79,
-// 64 138 / 144, 256 445 / 474; T 100 (0.39), 64 175 / 172, 256 576 / 584; 32/8, T 120 (0.47), 64 357 / 351, 256 1240 / 1235; 32/4 heads
-// of 32, T 33 (0.11), 4 40 / 39, 64 173 / 181, 256 591 / 630.
+// Whether it pays in the form of 16 float4 a thread, where a block has an SM to itself however few units its (sequence, group) has: a wave
+// takes 4.5 us almost empty and 7 full, and what the two launches take goes with the bytes, so the emptier the blocks the fewer waves pay; with
+// groups of query heads k's and v's blocks are the empty ones, without them the two launches have small blocks as well.  Us, forward's
+// pre-pass in two launches / one, by the room in use and the waves: 16/4 heads of 64, T 48 (0.19) 3.9 waves 24 / 23.4, 5.2 27.5 / 31, 20.8
+// 70 / 95; T 64 (0.25) 3.9 27 / 25, 10.4 46 / 55; T 80 (0.31) 5.2 38 / 33, 10.4 58 / 58, 20.8 96 / 103; T 100 (0.39) 10.4 69 / 62, 20.8
+// 112 / 109; 16/16 heads of 40, T 130 (0.25) 15.6 79 / 77, 41.5 156 / 186; of 64, T 160 (0.31) 20.8 109 / 102, 41.5 177 / 196; of 96, T 70
+// (0.22) 20.8 104 / 78, 41.5 145 / 149; from two fifths on one launch was the faster for any number of waves.
 inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
     long long blocks = 0, held = 0;
+    bool groups = false;
     for (int i = 0; i < a.n; ++i) {
         const PassTensor &t = a.t[i];
         blocks += (long long)t.batch * (t.heads / t.group), held += (long long)t.batch * t.rows * t.heads;
+        groups |= t.group > 1;
     }
-    const long long room = blocks * units;
-    return 5 * held >= 2 * room || (double)blocks * room <= 16. * held * sms;
+    const double in_use = (double)held / ((double)blocks * units), waves = (double)blocks / sms;
+    return in_use >= 0.4 || waves <= (groups ? 80. : 450.) * in_use * in_use;
 }
 template <int LP, int NC, int CHUNKS>
 inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
