@@ -183,12 +183,12 @@ int zt_attn_backward_batched(const float *q, const float *k, const float *v, con
 size_t zt_attn_backward_workspace_bytes(int batch, int T, int n_heads, int n_kv_heads, int dim);
 
 /* The forward of a training step: zt_attn_forward_batched, except that the 16-bit operand planes of
- * q, k, v it builds are written into the backward's workspace and kept there, and *host_token
+ * k, v it builds are written into the backward's workspace and kept there, and *host_token
  * (a host pointer, may be NULL) receives a token for them: non-zero when planes were kept, 0 when not
  * (a workspace that is NULL, short or misaligned, or a shape the tensor-core kernels do not take:
  * this is then the ordinary forward).  This call takes nothing from the per-device arena.
- * zt_attn_backward_batched_kept, given the same workspace, shape and that token, converts only dout
- * (a quarter less pre-pass traffic per step).  The token is the caller's statement that q, k, v have
+ * zt_attn_backward_batched_kept, given the same workspace, shape and that token, converts only q and
+ * dout (q's planes are the backward's alone: the forward splits the rows itself).  The token is the caller's statement that q, k, v have
  * not been written since the forward; the library never infers that from pointer values.  A token is
  * good for one backward; any other call that writes the workspace (another forward_keep, a plain
  * backward) retires it, and a retired or mismatched token is refused (return 1), never silently
@@ -240,7 +240,7 @@ int zt_attn_backward_batched_kept_peers(const float *q, const float *k, const fl
  *             src/autograd.zig:851-874, applied to the attention gradients), dv as usual; out and
  *             lse are the rope forward's.
  * Both take a caller workspace of zt_attn_rope_workspace_bytes(...) bytes (256-byte aligned; never
- * 0) and allocate nothing.  The forward keeps its operand planes (rotated q and k among them) in that
+ * 0) and allocate nothing.  The forward keeps its operand planes (rotated k among them) in that
  * workspace and reports a token through *host_token (may be NULL) exactly as
  * zt_attn_forward_batched_keep does; the backward takes it back (`token`; 0 converts everything
  * again) under the same rules, pos and theta included.  Refusals: those of the batched calls, plus

@@ -1,0 +1,83 @@
+"""The forwards that split the query rows themselves, against float64: one head a block, two, wide heads, walks split along the keys and
+windows whose sums leave the accumulators; rows far smaller than their neighbours, whole tensors far from one; and the backward
+that reads q after the forward, its gradient written over it.  Tolerance in the 2-norm: operands of 22 bits and at most 48 truncated
+additions (half of 2^-23 each) give S 3e-6 of its size at 256 columns, half of that at 128; O is truncated 12 times a key tile at
+two thirds of its final size on average, 4e-8 each."""
+import pytest
+import torch
+
+from test_gpu_backward64 import gradients
+from test_gpu_forward_short import forward64
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(B, T, H, G, D, scale, spread):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(29)
+    q, k, v, do = (torch.randn((B, T, w * D), device="cuda", generator=gen) * c for w, c in zip((H, G, G, H), (*scale, 1.0)))
+    if spread:  # every row by a power of two of its own, the largest 1
+        q *= 2.0 ** -torch.randint(0, spread, (B, T, 1), device="cuda", generator=gen).float()
+    return q, k, v, do
+
+
+def bound(D, keys):
+    return (1.5e-6 if D <= 128 else 3e-6) + 12 * -(-keys // 64) * 4e-8
+
+
+@pytest.mark.parametrize("B,T,H,G,D,scale,spread", [
+    (1, 129, 4, 2, 32, (1, 1, 1), 30), (3, 200, 3, 3, 60, (1, 1, 1), 0), (2, 161, 6, 2, 80, (1, 1, 1), 30),   # one head a block
+    (1, 1100, 2, 1, 128, (1, 1, 1), 0),                                                                      # split along the keys
+    (20, 200, 8, 2, 64, (1, 1, 1), 30), (30, 130, 12, 2, 100, (1, 1, 1), 0), (13, 257, 8, 2, 128, (1, 1, 1), 30),  # two heads a block
+    (2, 131, 3, 1, 160, (1, 1, 1), 30), (1, 300, 4, 2, 192, (1, 1, 1), 0), (2, 129, 2, 2, 256, (1, 1, 1), 30),     # wide heads
+    (1, 200, 4, 2, 128, (1e-25, 1e25, 1), 30), (20, 200, 8, 2, 64, (1e20, 1e-20, 1e-20), 0), (1, 200, 2, 1, 256, (1e-30, 1, 1), 0),
+])
+def test_against_float64(zt, B, T, H, G, D, scale, spread):
+    q, k, v, do = inputs(B, T, H, G, D, scale, spread)
+    ws = zt.BackwardWorkspace(B, T, H, G, D)
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0 and zt.lib.last_path() == "tcgen05"
+    ref, ref_lse = forward64(q, k, v, H, G, D, 0)
+    assert float((out.double() - ref).norm()) <= bound(D, T) * float(ref.norm())
+    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5
+    if scale != (1, 1, 1):
+        return
+    got = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=True)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+    for name, x, r in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
+        assert float((x.double() - r).norm()) <= 1e-5 * float(r.norm()), name  # (what the calls are measured to)
+
+
+@pytest.mark.parametrize("t,off,H,G,D", [(130, 1200, 3, 3, 64), (200, 2100, 8, 2, 128), (40, 1500, 2, 1, 256), (600, 1400, 32, 8, 64)])
+def test_windows(zt, t, off, H, G, D):
+    attn = zt.Attn(off + t, H, G, D)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    for x in (attn.q, attn.k, attn.v):
+        x.normal_(generator=gen)
+    attn.forward_at(1, 64, off, off + t, t)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0
+    q, k, v = attn.q[: t * H * D].view(1, t, H * D), attn.k.view(1, -1, G * D), attn.v.view(1, -1, G * D)
+    ref = forward64(q, k, v, H, G, D, off)[0]
+    assert float((attn.out[: t * H * D].double().view_as(ref) - ref).norm()) <= bound(D, 1024) * float(ref.norm())  # (flushed every 16 tiles)
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [(2, 200, 4, 2, 64), (1, 300, 8, 2, 128), (1, 1100, 2, 1, 256)])
+def test_gradient_of_q_over_q(zt, B, T, H, G, D):
+    q, k, v, do = inputs(B, T, H, G, D, (1, 1, 1), 0)
+    ws = zt.BackwardWorkspace(B, T, H, G, D)
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    token = ws.token
+    want = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=True)
+    zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    assert ws.token > token
+    dk, dv, delta = torch.empty_like(k), torch.empty_like(v), torch.empty_like(lse)
+    assert zt.lib.load().zt_attn_backward_batched_kept(
+        *(x.data_ptr() for x in (q, k, v, out, lse, do, q, dk, dv, delta, ws.buf)), ws.nbytes, B, T, H, G, D,
+        torch.cuda.current_stream().cuda_stream, ws.token) == 0, zt.lib.last_error()
+    torch.cuda.synchronize()
+    for a, b in zip((q, dk, dv), want):  # (sums that are made in memory come in no fixed order)
+        assert float((a.double() - b.double()).norm()) <= 1e-6 * float(b.double().norm())

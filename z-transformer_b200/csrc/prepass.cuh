@@ -86,17 +86,16 @@ constexpr int kPassTargetBlocks = 2048, kPassMaxSlots = 1024, kPassMaxTensors = 
 constexpr int kFillPerBlock = 4096;  // float4
 
 struct PassTensor {
-    const float *x;          // [batch][rows][heads * dim]; null: no f32 source, see q_planes
+    const float *x;          // [batch][rows][heads * dim]
     const float *o;          // with delta: the tensor it is formed with
     float *delta, *rnorm;    // [batch][rows][heads], or null
     __half *planes;          // [2][batch][rows][heads * pd], or null
-    uint2 *part;             // [batch * groups][slots] (max |x|, largest row norm) as f32 bit patterns
+    uint2 *part;             // [batch * groups][slots] (max |x|, largest row norm) as f32 bit patterns; null: amax is known already
     uint32_t *amax, *nmax;   // [batch * groups]: where the maxima are published; nmax null: not wanted
+    uint32_t *clear;         // [batch * groups] words set to zero, or null
     const float2 *rope;      // null, or the (cos, sin) table [rows][dim / 2]: x is rotated on its way into the planes
-    // the copy of the planes with row t times rel(t) (ds_row_scale, from rnorm and the largest row norms of dout and v),
-    // or null; made from x's planes as they pass, or from q_planes where x is null
+    // the planes with row t times rel(t) (ds_row_scale, from rnorm and the largest row norms of dout and v), or null
     __half *qs;
-    const __half *q_planes;
     const uint2 *dn_part, *vn_part;  // dout's slots; v's, or null: v's norms are published already
     const uint32_t *vn_final;
     int dn_slots, vn_slots;
@@ -110,6 +109,7 @@ struct PassArgs {
     long long fill_n4[3];
     int fill_first[4];  // first block of each region; [n_fill]: one past the last
     int n, n_stats, n_fill, dim, pd;  // dim: columns of a head in the tensors; pd: in the planes (plane_dim)
+    int q_units;                      // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
 };
 
 struct PassUnit {  // where a block stands
@@ -218,7 +218,9 @@ struct PassTops {
 };
 __device__ __forceinline__ PassTops pass_tops(const PassTensor &t, int bg, uint4 *red) {
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (t.x) {
+    if (t.part == nullptr) {
+        m.x = t.amax[bg];
+    } else {
         const uint2 *part = t.part + (long long)bg * t.slots;
         for (int i = threadIdx.x; i < t.slots; i += kPassThreads) {
             const uint2 v = part[i];
@@ -247,26 +249,14 @@ __device__ __forceinline__ PassTops pass_tops(const PassTensor &t, int bg, uint4
     return PassTops{m.x, m.y, m.z, m.w};
 }
 
-// Four elements times m into the planes at `hi` (null: not wanted) and, times rel as well, into the row-scaled copy.
-__device__ __forceinline__ void store_split4(__half *hi, __half *qs, long long plane, float4 v, float m, float rel) {
+// Four elements times m into the planes at `hi`.
+__device__ __forceinline__ void store_split4(__half *hi, long long plane, float4 v, float m) {
     uint2 hw, lw;
     split_pack(v.x * m, v.y * m, hw.x, lw.x);
     split_pack(v.z * m, v.w * m, hw.y, lw.y);
-    if (hi) *reinterpret_cast<uint2 *>(hi) = hw, *reinterpret_cast<uint2 *>(hi + plane) = lw;
-    if (qs == nullptr) return;
-    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&hw.x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&hw.y));
-    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&lw.x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&lw.y));
-    split_pack((h0.x + l0.x) * rel, (h0.y + l0.y) * rel, hw.x, lw.x);
-    split_pack((h1.x + l1.x) * rel, (h1.y + l1.y) * rel, hw.y, lw.y);
-    *reinterpret_cast<uint2 *>(qs) = hw, *reinterpret_cast<uint2 *>(qs + plane) = lw;
+    *reinterpret_cast<uint2 *>(hi) = hw, *reinterpret_cast<uint2 *>(hi + plane) = lw;
 }
 
-// What four elements of the planes stand for.
-__device__ __forceinline__ float4 join_split4(uint2 h, uint2 l) {
-    const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&h.x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
-    const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&l.x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&l.y));
-    return make_float4(h0.x + l0.x, h0.y + l0.y, h1.x + l1.x, h1.y + l1.y);
-}
 // Block blk's part of the zeros of outputs that are summed in memory.
 template <int THREADS>
 __device__ __forceinline__ void pass_fill_block(const PassArgs &a, int blk) {
@@ -302,59 +292,22 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
         return u < w.units ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
     };
     PassTops tops{};
-    const auto row_rel = [&](long long at) -> float {
+    const auto row_rel = [&](float norm) -> float {
         float cq, rel;
-        ds_row_scale(t.rnorm[at], tops.dn, tops.vn, cq, rel);
+        ds_row_scale(norm, tops.dn, tops.vn, cq, rel);
         return rel;
     };
     // (the first units' loads go out before the maxima are waited for: many blocks have no second units)
     const int stride = t.slots * NG * U;
-    if (t.x == nullptr) {
-        uint2 h[U][NC], l[U][NC];
-        float rn[U];
-        long long at[U];
-        const auto load = [&](int u0) {
-#pragma unroll
-            for (int k = 0; k < U; ++k) {
-                int r;
-                at[k] = locate(u0 + k * NG + gi, r);
-                rn[k] = t.rnorm[at[k] < 0 ? 0 : at[k]];
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int col = (li + LP * c) * 4;
-                    const __half *src = t.q_planes + (at[k] < 0 ? 0 : at[k]) * a.pd + (col < a.pd ? col : 0);
-                    h[k][c] = __ldg(reinterpret_cast<const uint2 *>(src));
-                    l[k][c] = __ldg(reinterpret_cast<const uint2 *>(src + plane));
-                }
-            }
-        };
-        int u0 = w.slot * NG * U;
-        load(u0);
-        tops = pass_tops(t, w.bg, red);
-        for (; u0 < w.units;) {
-#pragma unroll
-            for (int k = 0; k < U; ++k) {
-                float cq, rel;
-                ds_row_scale(rn[k], tops.dn, tops.vn, cq, rel);
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    // (a sum of the two pieces splits into these very pieces again)
-                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd)
-                        store_split4(nullptr, t.qs + at[k] * a.pd + (li + LP * c) * 4, plane, join_split4(h[k][c], l[k][c]), 1.f, rel);
-                }
-            }
-            u0 += stride;
-            if (u0 < w.units) load(u0);
-        }
-        return;
-    }
     float4 x[U][NC];
+    float norm[U];
     long long at[U];
     const auto load = [&](int u0) {
 #pragma unroll
         for (int k = 0; k < U; ++k) {
             int r;
             at[k] = locate(u0 + k * NG + gi, r);
+            norm[k] = t.qs && at[k] >= 0 ? t.rnorm[at[k]] : 0.f;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const int ch = li + LP * c;
@@ -365,20 +318,22 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     int u0 = w.slot * NG * U;
     if (t.rope == nullptr) load(u0);
     tops = pass_tops(t, w.bg, red);
-    if (w.slot == 0 && threadIdx.x == 0) {
+    if (w.slot == 0 && threadIdx.x == 0 && t.part) {
         t.amax[w.bg] = tops.amax;
         if (t.nmax) t.nmax[w.bg] = tops.nmax;
+        if (t.clear) t.clear[w.bg] = 0u;
     }
     const float m = block_mult(tops.amax);
+    __half *const planes = t.qs ? t.qs : t.planes;
     if (t.rope == nullptr) {
         for (; u0 < w.units;) {
 #pragma unroll
             for (int k = 0; k < U; ++k) {
-                const float rel = t.qs && at[k] >= 0 ? row_rel(at[k]) : 1.f;
+                const float rel = t.qs ? row_rel(norm[k]) : 1.f;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const long long to = at[k] * a.pd + (li + LP * c) * 4;
-                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd) store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, x[k][c], m, rel);
+                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd) store_split4(planes + to, plane, x[k][c], m * rel);
                 }
             }
             u0 += stride;
@@ -395,10 +350,9 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
             int r;
             const long long at = locate(u0 + k * NG + gi, r);
             if (at < 0) break;
-            const float rel = t.qs ? row_rel(at) : 1.f;
+            const float rel = t.qs ? row_rel(t.rnorm[at]) : 1.f;
             const auto put = [&](int col, float4 v) {
-                const long long to = at * a.pd + col;
-                store_split4(t.planes ? t.planes + to : nullptr, t.qs ? t.qs + to : nullptr, plane, v, m, rel);
+                store_split4(planes + at * a.pd + col, plane, v, m * rel);
             };
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
@@ -407,12 +361,8 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
                     const float4 *src = reinterpret_cast<const float4 *>(t.x + at * a.dim);
                     const float4 lo = __ldg(src + ch), hi = __ldg(src + h4 + ch);
                     const float4 *cs = reinterpret_cast<const float4 *>(t.rope + (long long)r * half) + 2 * ch;
-                    const float4 p = __ldg(cs), q = __ldg(cs + 1);  // four (cos, sin) pairs
                     float4 lr, hr;
-                    lr.x = rope_elem(lo.x, hi.x, make_float2(p.x, p.y), false, false), hr.x = rope_elem(hi.x, lo.x, make_float2(p.x, p.y), true, false);
-                    lr.y = rope_elem(lo.y, hi.y, make_float2(p.z, p.w), false, false), hr.y = rope_elem(hi.y, lo.y, make_float2(p.z, p.w), true, false);
-                    lr.z = rope_elem(lo.z, hi.z, make_float2(q.x, q.y), false, false), hr.z = rope_elem(hi.z, lo.z, make_float2(q.x, q.y), true, false);
-                    lr.w = rope_elem(lo.w, hi.w, make_float2(q.z, q.w), false, false), hr.w = rope_elem(hi.w, lo.w, make_float2(q.z, q.w), true, false);
+                    rope_chunk(lo, hi, __ldg(cs), __ldg(cs + 1), lr, hr);
                     put(ch * 4, lr), put(half + ch * 4, hr);
                 } else if (ch >= n4 && ch * 4 < a.pd) {
                     put(ch * 4, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -492,6 +442,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     if (threadIdx.x == 0) {
         t.amax[w.bg] = top;
         if (t.nmax) t.nmax[w.bg] = dn;
+        if (t.clear) t.clear[w.bg] = 0u;
     }
     const float m = block_mult(top);
 #pragma unroll
@@ -500,7 +451,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const int col = (li + LP * c) * 4;
-            if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, nullptr, plane, x[k][c], m, 1.f);
+            if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, plane, x[k][c], m);
         }
     }
 }
@@ -509,7 +460,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
 // Slots of one tensor of `bg` (sequence, group) pairs: what pass_slots() below can ask for.
 inline size_t pass_part_bytes(size_t bg) { return (bg > (size_t)kPassTargetBlocks ? bg : (size_t)kPassTargetBlocks) * sizeof(uint2); }
 
-// Adds a tensor (x or q_planes set by the caller afterwards where they are not plain) to the launch.
+// Adds a tensor to the launch.
 inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, int heads, int group, uint2 *part, uint32_t *amax,
                             uint32_t *nmax, __half *planes) {
     PassTensor &t = a.t[a.n++];
@@ -534,10 +485,12 @@ inline void pass_fill(PassArgs &a, float *dst, long long n) {
     a.fill[a.n_fill] = reinterpret_cast<float4 *>(dst), a.fill_n4[a.n_fill++] = n / 4;
 }
 // Whether one launch takes the call: `units` units a (sequence, group) at most, nothing rotated, nothing but planes and maxima wanted.
+// (The line is drawn by the group's query rows, although the forward reads those itself.)
 inline bool pass_takes_one(const PassArgs &a, int units) {
+    if (a.q_units > units) return false;
     for (int i = 0; i < a.n; ++i) {
         const PassTensor &t = a.t[i];
-        if ((long long)t.rows * t.group > units || !t.x || !t.planes || t.delta || t.rope || t.qs) return false;
+        if ((long long)t.rows * t.group > units || !t.part || t.delta || t.rope || t.qs) return false;
     }
     return a.n_fill == 0;
 }
@@ -553,8 +506,9 @@ inline int pass_sm_count() {
 // 112 / 109; 16/16 heads of 40, T 130 (0.25) 15.6 79 / 77, 41.5 156 / 186; of 64, T 160 (0.31) 20.8 109 / 102, 41.5 177 / 196; of 96, T 70
 // (0.22) 20.8 104 / 78, 41.5 145 / 149; from two fifths on one launch was the faster for any number of waves.
 inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
-    long long blocks = 0, held = 0;
-    bool groups = false;
+    const long long bg = (long long)a.t[0].batch * (a.t[0].heads / a.t[0].group);
+    long long blocks = a.q_units ? bg : 0, held = bg * a.q_units;
+    bool groups = a.q_units > a.t[0].rows;
     for (int i = 0; i < a.n; ++i) {
         const PassTensor &t = a.t[i];
         blocks += (long long)t.batch * (t.heads / t.group), held += (long long)t.batch * t.rows * t.heads;
@@ -574,7 +528,7 @@ inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
     if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
     return launch_pdl("pass_one_kernel", pass_one_kernel<LP, NC, CHUNKS>, dim3((unsigned)blocks), dim3(kOneThreads), 0, stream, a);
 }
-// Both launches.  The tensors with an f32 source come first in a.t.
+// Both launches (or the second alone, for zeros).  The tensors whose maxima are wanted come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     long long blocks = 0, stats = 0;
     bool o4 = false;
@@ -583,7 +537,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
         PassTensor &t = a.t[i];
         t.first = (int)blocks;
         blocks += (long long)t.batch * (t.heads / t.group) * t.slots;
-        if (t.x) a.n_stats = i + 1, stats = blocks;
+        if (t.part) a.n_stats = i + 1, stats = blocks;
         o4 |= (reinterpret_cast<uintptr_t>(t.o) & 15u) != 0;
     }
     a.fill_first[0] = (int)blocks;
@@ -603,7 +557,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
-        rc = launch_pdl("pass_stats_kernel", stats_kernel, gs, th, smem, stream, a);
+        rc = stats ? launch_pdl("pass_stats_kernel", stats_kernel, gs, th, smem, stream, a) : 0;
         return rc ? rc : launch_pdl("pass_planes_kernel", pass_planes_kernel<LP, NC>, gp, th, 0, stream, a);
     };
     using std::integral_constant;

@@ -42,6 +42,14 @@ __device__ __forceinline__ float rope_elem(float mine, float other, float2 cs, b
     return fmaf(mine, cs.x, other * s);
 }
 
+// Four elements of a head's lower half and their partners, rotated; p and q hold their four (cos, sin) pairs.
+__device__ __forceinline__ void rope_chunk(float4 lo, float4 hi, float4 p, float4 q, float4 &lr, float4 &hr) {
+    lr.x = rope_elem(lo.x, hi.x, make_float2(p.x, p.y), false, false), hr.x = rope_elem(hi.x, lo.x, make_float2(p.x, p.y), true, false);
+    lr.y = rope_elem(lo.y, hi.y, make_float2(p.z, p.w), false, false), hr.y = rope_elem(hi.y, lo.y, make_float2(p.z, p.w), true, false);
+    lr.z = rope_elem(lo.z, hi.z, make_float2(q.x, q.y), false, false), hr.z = rope_elem(hi.z, lo.z, make_float2(q.x, q.y), true, false);
+    lr.w = rope_elem(lo.w, hi.w, make_float2(q.z, q.w), false, false), hr.w = rope_elem(hi.w, lo.w, make_float2(q.z, q.w), true, false);
+}
+
 // out = R x (transpose = 0) or R^T x (transpose = 1) for x [batch][rows][width]; may run in place: a thread
 // owns both elements of a pair.  grid over batch * rows * width / 2 pairs.
 __global__ void __launch_bounds__(256) rope_apply_kernel(const float *x, float *out, const float2 *__restrict__ table,

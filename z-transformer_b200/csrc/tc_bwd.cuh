@@ -1027,7 +1027,7 @@ struct BwdWorkspace {
     uint32_t *amax_q, *amax_k, *amax_v, *amax_do, *vnmax, *dsmax;  // six [batch, n_kv_heads] arrays, in this order
     __half *q_planes, *do_planes, *k_planes, *v_planes;
     float *rnorm;  // [batch, T, n_heads]
-    __half *qs_planes;  // the row-scaled copy of q's planes (the fused and the wide-head backward read it for dK)
+    __half *qs_planes;  // q's planes with their rows scaled: what the fused and the wide-head backward read (q_planes: the two kernels)
     uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
     // partial results of a split forward, then of a split backward (tc_split.cuh): behind everything else, so that a
     // workspace of base_bytes does for a call that is not split
@@ -1060,18 +1060,28 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
     return w;
 }
 
-// The pre-pass of a backward: a.t[0] is dout and, unless their planes were kept, a.t[1 .. 3] are q, k, v.  want_qs: the
-// row-scaled copy of q's planes, want_q: q's planes themselves.
-inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs, bool want_q, bool kept, cudaStream_t stream) {
-    if (!kept && !want_q) a.t[1].planes = nullptr;
+// The pre-pass of a backward: a.t[0] is dout, a.t[1] q, a.t[2] and a.t[3] k and v, unless the forward has kept the planes of
+// these two and the maxima of all three.  want_qs: q's planes have their rows scaled.
+inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs, bool kept, cudaStream_t stream) {
+    const PassTensor &g = a.t[0];
+    PassTensor &t = a.t[1];
+    if (kept) t.part = nullptr;
     if (want_qs) {
-        const PassTensor &g = a.t[0];
-        PassTensor &t = kept ? pass_add(a, nullptr, g.batch, g.rows, g.heads, g.group, nullptr, nullptr, nullptr, nullptr) : a.t[1];
         t.qs = w.qs_planes, t.rnorm = w.rnorm, t.dn_part = g.part, t.dn_slots = g.slots;
-        if (kept) t.q_planes = w.q_planes, t.vn_final = w.vnmax;
+        if (kept) t.vn_final = w.vnmax;
         else t.vn_part = a.t[3].part, t.vn_slots = a.t[3].slots;
     }
-    return launch_pass(a, stream);
+    // (a caller's q may be where its gradient goes, as long as nothing is zeroed before q has been read)
+    const char *q0 = reinterpret_cast<const char *>(t.x), *q1 = q0 + (size_t)t.batch * t.rows * t.heads * a.dim * sizeof(float);
+    bool apart = true;
+    for (int f = 0; f < a.n_fill; ++f) {
+        const char *f0 = reinterpret_cast<const char *>(a.fill[f]);
+        apart = apart && (f0 >= q1 || f0 + a.fill_n4[f] * sizeof(float4) <= q0);
+    }
+    if (apart) return launch_pass(a, stream);
+    PassArgs zeros = a;
+    a.n_fill = 0, zeros.n = 0;
+    return launch_pass(a, stream) || launch_pass(zeros, stream);
 }
 
 inline bool tc_bwd_supported(int batch, int T, int dim, const void *q, const void *k, const void *v,

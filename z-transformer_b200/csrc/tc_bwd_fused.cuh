@@ -663,7 +663,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
     const BwdWorkspace w = bwd_workspace(workspace, batch, T, n_heads, n_kv_heads, pd);
     const int group = n_heads / n_kv_heads;
     const int blocks = td / 64;
-    // With the planes of q, k, v kept by the forward (their maxima and v's largest row norm beside them), only dout is
+    // With the planes of k, v kept by the forward (all maxima and v's largest row norm beside them), only q and dout are
     // converted.  The header's last array holds the largest row norm of dout for the fused kernel, max |dS| (which its
     // dQ kernel finds) for the two kernels.
     const size_t n_amax = (size_t)batch * n_kv_heads;
@@ -677,13 +677,13 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
         PassTensor &t = pass_add(pa, dout, batch, T, n_heads, group, w.part[3], w.amax_do, fused ? w.dsmax : nullptr, w.do_planes);
         t.o = out, t.delta = delta, t.rnorm = w.rnorm;
     }
+    pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
     if (!qkv_planes_kept) {
-        pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
         pass_add(pa, k, batch, T, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
         pass_add(pa, v, batch, T, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     }
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
-    if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
+    if (launch_pass_backward(pa, w, fused, qkv_planes_kept, stream)) return 1;
     const int rows = fused && td == 64 ? tcf::fused64_rows(T) : 64;  // of a query tile
     BwdMaps m;
     bool maps = make_head_map(&m.k128, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&

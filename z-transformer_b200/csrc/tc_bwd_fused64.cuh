@@ -634,9 +634,9 @@ inline int launch_bwd_fused64(const CUtensorMap &k128, const CUtensorMap &v128, 
                               const BwdParams &p, cudaStream_t stream) {
     CUtensorMap dqmap, dkmap, dvmap;
     const long long kv_batch = p.parts.n() > 1 ? (2LL * p.parts.n() - 1) * p.batch : p.batch;
-    if (!make_out_map(&dqmap, p.dq, p.batch, p.T, p.n_heads, p.dim_out, 32) ||
-        !make_out_map(&dkmap, p.dk, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32) ||
-        !make_out_map(&dvmap, p.dv, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32))
+    if (!make_row_map(&dqmap, p.dq, p.batch, p.T, p.n_heads, p.dim_out, 32) ||
+        !make_row_map(&dkmap, p.dk, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32) ||
+        !make_row_map(&dvmap, p.dv, kv_batch, p.T, p.n_kv_heads, p.dim_out, 32))
         return refuse("the TMA tensor maps for the backward's gradients could not be encoded.");
     const auto kernel = fused64_rows(p.T) == 64 ? attn_bwd_fused64_tc<true, true, 64>
                                   : with_flags([](auto parts, auto pad) { return attn_bwd_fused64_tc<parts.value, pad.value, 128>; }, p.parts.n() > 1 || p.by_tile, head_steps(p.dim_out) < 4);

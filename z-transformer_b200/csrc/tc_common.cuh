@@ -467,16 +467,16 @@ inline bool make_head_map(CUtensorMap *map, const void *base, int planes, long l
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor map over f32 rows of heads, [batch, rows, heads, dim], for tma_store_4d and tma_add_4d of 32 columns x box_rows rows
-// of one head (128-byte swizzle): what a head does not have of the columns is left out.  dim a multiple of four.
-inline bool make_out_map(CUtensorMap *map, float *base, long long batch, long long rows, int heads, int dim, int box_rows) {
+// Tensor map over f32 rows of heads, [batch, rows, heads, dim], for copies of 32 columns x box_rows rows of one head (128-byte
+// swizzle) either way: what a head does not have of the columns is left out, or arrives as zeros.  dim a multiple of four.
+inline bool make_row_map(CUtensorMap *map, const float *base, long long batch, long long rows, int heads, int dim, int box_rows) {
     PFN_encodeTiled enc = get_encode_tiled();
     if (!enc) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)dim, (cuuint64_t)heads, (cuuint64_t)rows, (cuuint64_t)batch};
     const cuuint64_t strides[3] = {(cuuint64_t)dim * 4, (cuuint64_t)heads * dim * 4, (cuuint64_t)rows * heads * dim * 4};
     const cuuint32_t box[4] = {32, 1, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

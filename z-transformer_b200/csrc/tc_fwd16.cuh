@@ -6,7 +6,7 @@
 // an f16 term is half a TF32 MMA, operands take half the bytes (three K and three V tiles, hi and
 // lo, fit in shared memory), and two S tiles and two O accumulators fit in TMEM.
 //
-//   the pre-pass             (prepass.cuh) q, k, v -> f16 hi/lo planes with a power-of-two scale
+//   the pre-pass             (prepass.cuh) k, v -> f16 hi/lo planes with a power-of-two scale
 //                            per (sequence, KV group), in a workspace.
 //   TMA warp        K and V hi/lo tiles of 64 keys, a ring of three slots each: a K tile is free
 //                   once its S has retired, two tiles before its V.
@@ -42,11 +42,14 @@ struct Shared {
     volatile int abort;
     float fin_m[2][128], fin_l[2][128];  // each set's reference maximum and sum, for the final merge
     float fin_f[2][128];                 // what has been flushed of its O is relative to this maximum (-inf: nothing)
+    float q_top[2][128];                 // max |q| of each half of a row's columns
 };
 
 struct Params {
-    const __half *q_planes;                     // [2][B][T][H*D]
-    const uint32_t *amax_q, *amax_k, *amax_v;   // [B, Hkv]
+    const uint32_t *amax_k, *amax_v;            // [B, Hkv]
+    uint32_t *amax_q;                           // [B, Hkv]: takes the maximum of every query row (cleared before); null: not wanted
+    const float2 *rope;                         // null, or the (cos, sin) table [T][dim_out / 2] to rotate the query rows with
+    float *flush_rows;                          // [B, T, H, dim_out]: where attn_fwd_tc16 keeps its second set's flushed sums
     float *out, *lse;                           // lse may be null
     int batch, T, n_heads, n_kv_heads;
     int q_offset;  // query row r stands at position q_offset + r of the keys: it sees keys 0 .. q_offset + r
@@ -138,12 +141,10 @@ __device__ __forceinline__ float4 flush_sum4(const float *at, float f, bool firs
     o.x = fmaf(g.x, f, o.x), o.y = fmaf(g.y, f, o.y), o.z = fmaf(g.z, f, o.z), o.w = fmaf(g.w, f, o.w);
     return o;
 }
-// Where a row's running sum is kept: columns [0, D/2) and [D/2, D); `width` columns of it (the rest are padding), null
-// when the row is not the tensor's.
+// Where a row's running sum is kept, null when the row is not the tensor's; `width` columns of it (the rest are padding).
 struct FlushRow {
-    float *lower, *upper;
-    int width, half;  // columns from `half` on are at upper
-    __device__ __forceinline__ float *at(int c) const { return c < half ? lower + c : upper + (c - half); }
+    float *sums;
+    int width;
 };
 // O's columns [0, D) of this thread's row, at TMEM `taddr`, into its running sum.
 template <int D>
@@ -153,15 +154,102 @@ __device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, f
         uint32_t r[32];
         tmem_ld32(taddr + c, r);
         tmem_wait_ld();
-        if (row.lower == nullptr) continue;
+        if (row.sums == nullptr) continue;
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
             if (c + i >= row.width) break;
-            float *at = row.at(c + i);
+            float *at = row.sums + c + i;
             *reinterpret_cast<float4 *>(at) = flush_sum4(at, f, first, make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])));
         }
     }
 }
+
+// The query tile.  A tile is read by one CTA only (by the few parts of a split one), so the rows come as the caller's f32 and become
+// the two pieces here, between shared memory and the MMAs' operands: no planes of q are written and read again, and no
+// launch before this one has to know q's maxima, so a small launch has its rows in place before the pre-pass ends.  Every row has
+// a power of two of its own, which its thread takes out of the scores.  It costs a CTA about 1500 clocks before its first MMA (3500
+// while a thread converted a row by itself).  Us, forward and backward, q's planes from the pre-pass -> rows: one sequence of 256, 4/2
+// heads of 32 42.1 -> 39.1; batch 8, T 512, 32/8 heads of 64 255 -> 241; batch 4, T 1000, 16/4 of 80 248 -> 236; batch 8, T 1024, 32/8
+// of 256 2580 -> 2410; T 4096, of 128 11970 -> 11640.
+constexpr int kQBlock = 128 * 128;  // 32 columns of the tile's 128 rows, as TMA lands them: 128 bytes a row, swizzled
+template <int D>
+__device__ __forceinline__ void load_q(uint8_t *tile, const CUtensorMap *map, uint64_t *bar, int row, int head, int b) {
+#pragma unroll
+    for (int c = 0; c < D / 32; ++c) tma_load_4d(tile + c * kQBlock, map, bar, c * 32, head, row, b);
+}
+// Four columns of a row, whose bytes are its thread's alone.
+__device__ __forceinline__ float4 *q_at(uint8_t *tile, int row, int chunk) {
+    return reinterpret_cast<float4 *>(tile + (chunk >> 3) * kQBlock + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
+}
+// Rotates columns of the row in place: chunks [first, last) of the head's lower half (h4 chunks) and their partners, by the row's
+// (cos, sin) pairs.
+__device__ __forceinline__ void rotate_q(uint8_t *tile, int row, const float2 *angles, int h4, int first, int last) {
+    for (int ch = first; ch < last; ++ch) {
+        const float4 lo = *q_at(tile, row, ch), hi = *q_at(tile, row, h4 + ch);
+        const float4 *cs = reinterpret_cast<const float4 *>(angles) + 2 * ch;
+        float4 a, b;
+        rope_chunk(lo, hi, cs[0], cs[1], a, b);
+        *q_at(tile, row, ch) = a, *q_at(tile, row, h4 + ch) = b;
+    }
+}
+__device__ __forceinline__ float max_abs4(float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); }
+// The pieces of 32 columns times m: packed pairs of the hi ones, then of the lo ones.
+template <class X>
+__device__ __forceinline__ void split_q32(const X &column4, float m, uint32_t (&h)[16], uint32_t (&l)[16]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float4 x = column4(c);
+        split_pack(x.x * m, x.y * m, h[2 * c], l[2 * c]);
+        split_pack(x.z * m, x.w * m, h[2 * c + 1], l[2 * c + 1]);
+    }
+}
+// The lo pieces of the tile's 32 columns `block` into the K-major tile of halves that an MMA reads: half of a block of 64 columns.
+__device__ __forceinline__ void store_q_lo(uint8_t *tile, int row, int block, const uint32_t (&l)[16]) {
+    uint8_t *at = tile + (block >> 1) * kQBlock + row * 128;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4 *>(at + ((((block & 1) * 4 + c) ^ (row & 7)) << 4)) = make_uint4(l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]);
+}
+// A head's query row by two threads, which take a half of its columns each, out of their CTA's 256 (the barrier): hi pieces at TMEM `hi`,
+// lo pieces at TMEM `lo` or, where LO_SMEM, over the tile (the rows have been read by then: a half goes where the row's columns
+// of either thread were).  Returns the row's maximum; `tops` holds the halves'.
+template <int D, bool LO_SMEM>
+__device__ __forceinline__ float convert_q(uint8_t *tile, int set, int row, const float2 *angles, int dim, float (*tops)[128], uint32_t hi, uint32_t lo) {
+    if (angles) {
+        const int h4 = dim >> 3, mid = h4 >> 1;
+        rotate_q(tile, row, angles, h4, set ? mid : 0, set ? h4 : mid);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    float4 x[D / 8];
+    float top = 0.f;
+#pragma unroll
+    for (int c = 0; c < D / 8; ++c) x[c] = *q_at(tile, row, set * (D / 8) + c), top = fmaxf(top, max_abs4(x[c]));
+    tops[set][row] = top;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    top = fmaxf(top, tops[set ^ 1][row]);
+    const float m = block_mult(__float_as_uint(top));
+#pragma unroll
+    for (int cb = 0; cb < D / 64; ++cb) {
+        uint32_t qh[16], ql[16];
+        split_q32([&](int c) { return x[cb * 8 + c]; }, m, qh, ql);
+        tmem_st16(hi + set * (D / 4) + cb * 16, qh);
+        if (LO_SMEM) store_q_lo(tile, row, set * (D / 64) + cb, ql);
+        else tmem_st16(lo + set * (D / 4) + cb * 16, ql);
+    }
+    tmem_wait_st();
+    if (LO_SMEM) fence_async_smem();
+    tc_fence_before();
+    return top;
+}
+// The tile's maximum into its (sequence, KV group)'s, for the backward.
+__device__ __forceinline__ void publish_q_top(const Params &p, int bg, float row_top) {
+    if (p.amax_q == nullptr) return;
+    const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(row_top));
+    if ((threadIdx.x & 31) == 0) atomicMax(p.amax_q + bg, top);
+}
+// What turns a row's scores into log2 units.  (One division after the other: a row of tiny values may have a scale whose
+// product with k's is beyond f32.)
+__device__ __forceinline__ float score_scale(const Params &p, float mq, float mk) { return p.scale_log2 / mq / mk; }
 
 template <int D, bool FLUSH, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -219,43 +307,30 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    pdl_wait();
-    pdl_launch();
-
-    const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
-    const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+    // (the query rows are older than the launch before this one, for whose planes and maxima pdl_wait() waits)
 
     if (warp == 8) {
         // ------------------------------------------------------------------ TMA producer
         // K of tile j is free again once S(j) has retired, two tiles before its V: rings of their own
         if (elect_one()) {
             tma_prefetch_desc(&qmap), tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap);
-            // the query tile's two planes, staged in V's first two slots until the row threads have moved
-            // them into TMEM: one bulk copy each instead of a strided read per thread
+            // the query tile waits in V's first two slots until the row threads have its pieces in TMEM
             mbar_arrive_expect_tx(&sh->q_full, 4 * KP);
-            load_head<NB>(sV, &qmap, &sh->q_full, t0, h, b, 128 * 128, padded);
-            load_head<NB>(sV + 2 * KP, &qmap, &sh->q_full, t0, h, B + b, 128 * 128, padded);
+            load_q<D>(sV, &qmap, &sh->q_full, t0, h, b);
+            pdl_wait();
+            pdl_launch();
             int n_k = 0, n_v = 0;  // tiles issued
             bool live = true;
             const auto prefetch_next_q = [&]() {
                 // The query tile of the CTA that will start when one of the running ones ends (`ahead` blocks on in
-                // launch order, about the number of SMs), into L2: its planes were written once by the pre-pass and
-                // would otherwise come from DRAM, under load, before that CTA's first MMA can go out.
+                // launch order, about the number of SMs), into L2: it would otherwise come from DRAM, under load, before
+                // that CTA's first MMA can go out.
                 const long long gx = gridDim.x, gy = gridDim.y;
                 const long long lin = blockIdx.x + gx * (blockIdx.y + gy * blockIdx.z) + p.ahead;
                 if (p.ahead <= 0 || lin >= gx * gy * gridDim.z) return;
                 const int nx = (int)(lin % gx), ny = (int)((lin / gx) % gy), nz = (int)(lin / (gx * gy));
                 const int nt0 = ((int)gx - 1 - nx) * 128;
-                if (!padded) {
-                    tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, nz);
-                    tma_prefetch_l2_4d(&qmap, 0, nt0, ny * NB, B + nz);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < NB; ++c) {
-                        tma_prefetch_l2_4d(&qmap, c * 64, nt0, ny, nz);
-                        tma_prefetch_l2_4d(&qmap, c * 64, nt0, ny, B + nz);
-                    }
-                }
+                for (int c = 0; c < p.dim_out; c += 32) tma_prefetch_l2_4d(&qmap, c, ny, nt0, nz / p.parts);
             };
             auto load_k = [&](int j) {
                 const int s = j % 3;
@@ -359,42 +434,26 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int t = t0 + tid, pos = p.q_offset + t;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         bool ok = true;
+        float top;  // max |q| of the row
         {
-            // this thread's row of Q's hi (set 0) or lo (set 1) plane, out of the 128-byte-swizzled staging tile
             if (!__all_sync(0xffffffffu, fwait(&sh->q_full, 0, sh))) fgive_up(sh, 49), ok = false;
-            const uint8_t *src = sV + set * 2 * KP + tid * 128;
-#pragma unroll
-            for (int kb = 0; kb < NB; ++kb) {
-                uint32_t r[32];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 v4 = *reinterpret_cast<const uint4 *>(src + kb * (128 * 128) + ((c ^ (tid & 7)) << 4));
-                    r[4 * c] = v4.x, r[4 * c + 1] = v4.y, r[4 * c + 2] = v4.z, r[4 * c + 3] = v4.w;
-                }
-                tmem_st32(tmem + lane_base + (set == 0 ? cQh : cQl) + kb * 32, r);
-            }
-            tmem_wait_st();
-            tc_fence_before();
+            const float2 *angles = p.rope ? p.rope + (long long)(t < p.T ? t : 0) * (p.dim_out >> 1) : nullptr;
+            top = convert_q<D, false>(sV, set, tid, angles, p.dim_out, sh->q_top, tmem + lane_base + cQh, tmem + lane_base + cQl);
             mbar_arrive_warp(&sh->a_ready);
         }
-        const float cs = p.scale_log2 / (mq * mk);
+        pdl_wait();
+        const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+        if (set == 0) publish_q_top(p, b * p.n_kv_heads + g, top);
+        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        // where the sets keep flushed sums: set 0 in out, set 1 in the two planes of the query row, which this CTA alone
-        // reads and has in TMEM by now (a forward that flushes keeps no planes for a backward)
-        const int pd = PAD ? plane_dim(p.dim_out) : D;  // a head in the planes
-        FlushRow row0{nullptr, nullptr, p.dim_out, pd / 2}, row1{nullptr, nullptr, p.dim_out, pd / 2};
+        // where the sets keep flushed sums: set 0 in out, set 1 in rows of its own
+        FlushRow row0{nullptr, p.dim_out}, row1{nullptr, p.dim_out};
         if (FLUSH && t < p.T) {
-            row0.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
-            row0.upper = row0.lower + pd / 2;
-            if (p.parts > 1) {  // (whose parts share the query rows: behind the parts' rows)
-                row1.lower = row0.lower + p.parts * p.out_part, row1.upper = row1.lower + pd / 2;
-            } else {
-                __half *planes = const_cast<__half *>(p.q_planes) + ((long long)b * p.T + t) * p.n_heads * pd + (long long)h * pd;
-                row1.lower = reinterpret_cast<float *>(planes);
-                row1.upper = reinterpret_cast<float *>(planes + (long long)B * p.T * p.n_heads * pd);
-            }
+            const long long at = (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out;
+            row0.sums = p.out + part * p.out_part + at;
+            row1.sums = p.parts > 1 ? row0.sums + p.parts * p.out_part : p.flush_rows + at;  // (parts': behind the parts' rows)
         }
         for (int j = set; ok && j < n_tiles; j += 2) {
             if (!__all_sync(0xffffffffu, fwait(&sh->s_full[set], (uint32_t)((j >> 1) & 1), sh))) {
@@ -491,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float inv = lsum == 0.f ? 0.f : 1.f / (lsum * mv);  // lsum, like O, carries kPScale
             const float f0 = w0 * inv, f1 = w1 * inv;
             const float s0 = sh->fin_f[0][tid], s1 = sh->fin_f[1][tid];
-            const bool add0 = FLUSH && s0 != -INFINITY && row0.lower != nullptr, add1 = FLUSH && s1 != -INFINITY && row1.lower != nullptr;
+            const bool add0 = FLUSH && s0 != -INFINITY && row0.sums != nullptr, add1 = FLUSH && s1 != -INFINITY && row1.sums != nullptr;
             const float g0 = add0 ? ex2(s0 - m0) : 0.f, g1 = add1 ? ex2(s1 - m1) : 0.f;
             // set s merges columns [s D/2, (s+1) D/2) of the row
             uint8_t *srow = sK + tid * (D * 4);
@@ -505,11 +564,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int i = 0; i < 32; i += 4) {
                     const int col = set * (D / 2) + c + i;
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add0 && col < row0.width) o4 = flush_sum4(row0.at(col), g0, false, o4);
+                    if (add0 && col < row0.width) o4 = flush_sum4(row0.sums + col, g0, false, o4);
                     o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
                         float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
-                        if (add1 && col < row1.width) x4 = flush_sum4(row1.at(col), g1, false, x4);
+                        if (add1 && col < row1.width) x4 = flush_sum4(row1.sums + col, g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     const int ch = (set * (D / 2) + c + i) >> 2;
@@ -545,7 +604,8 @@ struct Workspace {
     uint32_t *amax_q, *amax_k, *amax_v;
     uint32_t *vnmax;  // (in the backward's layout: the largest row norm of v, which the backward wants; else null)
     uint2 *part[3];   // the pre-pass's slots
-    __half *q_planes, *k_planes, *v_planes;
+    float *flush_rows;  // (see Params)
+    __half *k_planes, *v_planes;
     float *parts;     // of a forward split along the keys: behind everything else
     size_t base_bytes, total_bytes;
 };
@@ -554,13 +614,13 @@ inline Workspace workspace(void *base, int batch, int T, int n_heads, int n_kv_h
     Workspace w{};
     const size_t n_amax = (size_t)batch * n_kv_heads;
     auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
-    const size_t qh = (size_t)2 * batch * T * n_heads * dim * sizeof(__half);
+    const size_t rows = (size_t)batch * T * n_heads * dim * sizeof(float);
     const size_t kh = (size_t)2 * batch * (q_offset + T) * n_kv_heads * dim * sizeof(__half);
     char *c = static_cast<char *>(base);
     w.amax_q = reinterpret_cast<uint32_t *>(c), w.amax_k = w.amax_q + n_amax, w.amax_v = w.amax_k + n_amax;
     size_t off = up(3 * n_amax * sizeof(uint32_t));
     for (int i = 0; i < 3; ++i) w.part[i] = reinterpret_cast<uint2 *>(c + off), off += up(tcb::pass_part_bytes(n_amax));
-    w.q_planes = reinterpret_cast<__half *>(c + off), off += up(qh);
+    w.flush_rows = reinterpret_cast<float *>(c + off), off += up(rows);
     w.k_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.v_planes = reinterpret_cast<__half *>(c + off), off += up(kh);
     w.base_bytes = off;
@@ -622,25 +682,29 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
         w.amax_q = bw.amax_q, w.amax_k = bw.amax_k, w.amax_v = bw.amax_v;
         w.vnmax = bw.vnmax;
         for (int i = 0; i < 3; ++i) w.part[i] = bw.part[i];
-        w.q_planes = bw.q_planes, w.k_planes = bw.k_planes, w.v_planes = bw.v_planes, w.parts = bw.parts;
+        w.k_planes = bw.k_planes, w.v_planes = bw.v_planes, w.parts = bw.parts;
         w.base_bytes = bw.base_bytes;
     }
     const int group = n_heads / n_kv_heads;
     const int n_seen = q_offset + T;  // key rows that some query row sees
     PassArgs pa{};
-    pa.dim = dim, pa.pd = pd;
-    pass_add(pa, q, batch, T, n_heads, group, w.part[0], w.amax_q, nullptr, w.q_planes).rope = rope;
-    pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes).rope = rope;
+    pa.dim = dim, pa.pd = pd, pa.q_units = T * group;
+    {
+        PassTensor &t = pass_add(pa, k, batch, n_seen, n_kv_heads, 1, w.part[1], w.amax_k, nullptr, w.k_planes);
+        t.rope = rope;
+        if (in_backward_workspace) t.clear = w.amax_q;
+    }
     pass_add(pa, v, batch, n_seen, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     if (launch_pass(pa, stream)) return 1;
     CUtensorMap kmap, vmap, qmap;  // (the widest tiles fetch K block by block and V by 16 keys, see attn_fwd_tc16x)
     if (!make_head_map(&kmap, w.k_planes, 2 * batch, n_seen, n_kv_heads, dim, td > 128 ? 1 : td / 64, 64) ||
         !make_head_map(&vmap, w.v_planes, 2 * batch, n_seen, n_kv_heads, dim, td / 64, td > 128 ? 16 : 64) ||
-        !make_head_map(&qmap, w.q_planes, 2 * batch, T, n_heads, dim, td / 64, 128))
+        !make_row_map(&qmap, q, batch, T, n_heads, dim, 128))
         return refuse("the TMA tensor maps for the forward could not be encoded.");
     const int sms = split_sm_count();
     tcf16::Params p{};
-    p.q_planes = w.q_planes, p.amax_q = w.amax_q, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
+    p.amax_q = in_backward_workspace ? w.amax_q : nullptr, p.amax_k = w.amax_k, p.amax_v = w.amax_v;
+    p.rope = rope, p.flush_rows = q_offset > 0 ? w.flush_rows : nullptr;
     p.out = out, p.lse = lse;
     p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
     p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;

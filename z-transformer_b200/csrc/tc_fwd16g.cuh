@@ -10,7 +10,7 @@
 //         (an SS MMA), which is what makes room for the second head;
 //   MMA   S_A(0) S_B(0) | P.V_A(j) S_A(j+1) P.V_B(j) S_B(j+1) | ...: a head's next S goes out behind its P.V,
 //         so its softmax runs under the other head's MMAs, as with the parity split;
-//   smem  K ring of three slots, V ring of two, two Q lo planes (224 KB at head_dim 128).
+//   smem  K ring of three slots, V ring of two, the lo pieces of two query tiles (224 KB at head_dim 128).
 // One accumulator per head: no merge at the end.  Needs an even number of query heads per KV group.
 #pragma once
 
@@ -21,9 +21,10 @@ namespace tcf16 {
 
 struct SharedG {
     uint64_t full_k[3], free_k[3], full_v[2], free_v[2];
-    uint64_t a_ready, q_full, ql_full, s_full[2], p_full[2], pv_done[2], staged[2], all_done;
+    uint64_t a_ready[2], q_full[2], s_full[2], p_full[2], pv_done[2], staged[2], all_done;
     uint32_t tmem_base;
     volatile int abort;
+    float q_top[2][2][128];  // of a head: max |q| of each half of a row's columns
 };
 __device__ __forceinline__ bool gwait(uint64_t *bar, uint32_t parity, SharedG *sh) {
     for (uint32_t i = 0; i < (1u << 20); ++i) {
@@ -46,8 +47,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool padded = PAD && plane_dim(p.dim_out) < D;  // the planes are narrower than the tile
     constexpr int cQh = 0, cO0 = D, cS0 = 3 * D;  // head s: Qh at cQh + s W2, O at cO0 + s D, S/P at cS0 + 64 s
     extern __shared__ __align__(1024) uint8_t smem_raw[];  // (the swizzled tiles need the alignment; checked below)
-    uint8_t *sK = smem_raw, *sV = sK + 6 * KP, *sQl = sV + 4 * KP;  // sQl: Q lo of head A, of head B (2 KP each)
-    SharedG *sh = reinterpret_cast<SharedG *>(sQl + 4 * KP);
+    // Behind K's ring: head s's f32 query tile at sQ + s 4 KP, of which its lo pieces take the first half over and V's slot s the other.
+    uint8_t *sK = smem_raw, *sQ = sK + 6 * KP;
+    SharedG *sh = reinterpret_cast<SharedG *>(sQ + 8 * KP);
 
     const int warp = threadIdx.x >> 5;
     // launch order (x fastest): the head pairs of a sequence, query tile by query tile, late (long) tiles first, so
@@ -64,11 +66,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x == 0) {
         for (int i = 0; i < 3; ++i) mbar_init(&sh->full_k[i], 1), mbar_init(&sh->free_k[i], 1);
         for (int i = 0; i < 2; ++i) mbar_init(&sh->full_v[i], 1), mbar_init(&sh->free_v[i], 1);
-        mbar_init(&sh->a_ready, 8);
-        mbar_init(&sh->q_full, 1), mbar_init(&sh->ql_full, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh->s_full[i], 1), mbar_init(&sh->p_full[i], 4), mbar_init(&sh->pv_done[i], 1);
             mbar_init(&sh->staged[i], 4);
+            mbar_init(&sh->q_full[i], 1), mbar_init(&sh->a_ready[i], 8);
         }
         mbar_init(&sh->all_done, 1);
         sh->abort = (smem_u32(smem_raw) & 1023u) ? 40 : 0;
@@ -80,23 +81,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    pdl_wait();
-    pdl_launch();
-
-    const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
-    const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+    // (the query rows are older than the launch before this one, for whose planes and maxima pdl_wait() waits)
 
     if (warp == 8) {
         // ------------------------------------------------------------------ TMA producer
         if (elect_one() && !sh->abort) {
             tma_prefetch_desc(&qmap), tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap);
-            // the Q hi planes wait in V's two slots until the row threads have moved them into TMEM
-            mbar_arrive_expect_tx(&sh->q_full, 4 * KP);
-            load_head<NB>(sV, &qmap, &sh->q_full, t0, h0, b, 128 * 128, padded);
-            load_head<NB>(sV + 2 * KP, &qmap, &sh->q_full, t0, h0 + 1, b, 128 * 128, padded);
-            mbar_arrive_expect_tx(&sh->ql_full, 4 * KP);
-            load_head<NB>(sQl, &qmap, &sh->ql_full, t0, h0, B + b, 128 * 128, padded);
-            load_head<NB>(sQl + 2 * KP, &qmap, &sh->ql_full, t0, h0 + 1, B + b, 128 * 128, padded);
+            for (int i = 0; i < 2; ++i) {
+                mbar_arrive_expect_tx(&sh->q_full[i], 4 * KP);
+                load_q<D>(sQ + i * 4 * KP, &qmap, &sh->q_full[i], t0, h0 + i, b);
+            }
+            pdl_wait();
+            pdl_launch();
             int n_k = 0, n_v = 0;  // tiles issued
             bool live = true;
             auto load_k = [&](int j) {
@@ -111,20 +107,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int s = j & 1;
                 if (j >= 2 && !gwait(&sh->free_v[s], (uint32_t)(((j >> 1) & 1) ^ 1), sh)) { ggive_up(sh, 41), live = false; return; }
                 mbar_arrive_expect_tx(&sh->full_v[s], 2 * KP);
-                load_head<NB>(sV + s * 2 * KP, &vmap, &sh->full_v[s], j * BN, g, b, BN * 128, padded);
-                load_head<NB>(sV + s * 2 * KP + KP, &vmap, &sh->full_v[s], j * BN, g, B + b, BN * 128, padded);
+                load_head<NB>(sQ + (2 + 4 * s) * KP, &vmap, &sh->full_v[s], j * BN, g, b, BN * 128, padded);
+                load_head<NB>(sQ + (3 + 4 * s) * KP, &vmap, &sh->full_v[s], j * BN, g, B + b, BN * 128, padded);
                 ++n_v;
             };
             for (int j = 0; j < 3 && j < n_tiles; ++j) load_k(j);
-            if (!gwait(&sh->a_ready, 0, sh)) ggive_up(sh, 41), live = false;
-            for (int j = 0; live && j < 2 && j < n_tiles; ++j) load_v(j);
+            for (int j = 0; live && j < 2 && j < n_tiles; ++j) {
+                if (!gwait(&sh->a_ready[j], 0, sh)) ggive_up(sh, 41), live = false;
+                else load_v(j);
+            }
             for (int j = 2; live && j < n_tiles; ++j) {
                 if (j + 1 < n_tiles) load_k(j + 1);
                 if (live) load_v(j);
             }
             if (sh->abort) {
                 // let the copies in flight land before the CTA's shared memory goes away
-                mbar_wait(&sh->q_full, 0), mbar_wait(&sh->ql_full, 0);
+                mbar_wait(&sh->q_full[0], 0), mbar_wait(&sh->q_full[1], 0);
                 for (int j = (n_k > 3 ? n_k - 3 : 0); j < n_k; ++j) mbar_wait(&sh->full_k[j % 3], (uint32_t)((j / 3) & 1));
                 for (int j = (n_v > 2 ? n_v - 2 : 0); j < n_v; ++j) mbar_wait(&sh->full_v[j & 1], (uint32_t)((j >> 1) & 1));
             }
@@ -136,15 +134,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             constexpr uint32_t id_s = idesc_f16(128, BN, false, false);
             const int steps = PAD ? head_steps(p.dim_out) : D / 16;
             const uint32_t id_o = idesc_f16(128, 16 * steps, false, true);
-            bool ok = gwait(&sh->a_ready, 0, sh) && gwait(&sh->ql_full, 0, sh);
-            if (!ok) ggive_up(sh, 42);
-            tc_fence_after();
-            const uint32_t k_u32 = smem_u32(sK), v_u32 = smem_u32(sV);
+            bool ok = true;
+            const uint32_t k_u32 = smem_u32(sK), q_u32 = smem_u32(sQ);
             // S of head `hd`, tile j (K tile j has landed: the caller waited)
             auto issue_qk = [&](int hd, int j) {
                 const uint32_t kh = k_u32 + (uint32_t)((j % 3) * 2 * KP);
                 const uint64_t bkh = desc_kmajor(kh), bkl = desc_kmajor(kh + KP);
-                const uint64_t bql = desc_kmajor(smem_u32(sQl) + (uint32_t)(hd * 2 * KP));
+                const uint64_t bql = desc_kmajor(q_u32 + (uint32_t)(hd * 4 * KP));
                 const uint32_t cS = cS0 + hd * BN, cQ = cQh + hd * W2;
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
@@ -167,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // P.V of head `hd`, tile j (V tile j has landed)
             auto issue_pv = [&](int hd, int j) {
                 const bool fresh = j == 0 || (FLUSH && j % kFlushKeyTiles == 0);  // (O was flushed before tile j)
-                const uint32_t vh = v_u32 + (uint32_t)((j & 1) * 2 * KP);
+                const uint32_t vh = q_u32 + (uint32_t)((2 + 4 * (j & 1)) * KP);
                 const uint64_t mvh = desc_mnmajor_16b(vh, BN * 128), mvl = desc_mnmajor_16b(vh + KP, BN * 128);
                 const uint32_t cS = cS0 + hd * BN, cO = cO0 + hd * D;
 #pragma unroll
@@ -181,8 +177,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (hd == 1) mma_commit(&sh->free_v[j & 1]);
                 mma_commit(&sh->pv_done[hd]);
             };
-            if (ok && !k_landed(0)) { ggive_up(sh, 43); ok = false; }
-            if (ok) issue_qk(0, 0), issue_qk(1, 0);
+            for (int hd = 0; ok && hd < 2; ++hd) {
+                if (!gwait(&sh->a_ready[hd], 0, sh) || !k_landed(0)) { ggive_up(sh, 42); ok = false; }
+                else issue_qk(hd, 0);
+            }
             for (int j = 0; ok && j < n_tiles; ++j) {
                 const uint32_t par = (uint32_t)(j & 1);
                 if (!gwait(&sh->p_full[0], par, sh) || !gwait(&sh->full_v[j & 1], (uint32_t)((j >> 1) & 1), sh)) { ggive_up(sh, 44); break; }
@@ -209,33 +207,27 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int t = t0 + tid, pos = p.q_offset + t;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         bool ok = true;
+        float top = 0.f;  // max |q| of the row
         {
-            // this thread's row of its head's Q hi plane, out of the 128-byte-swizzled staging tile
-            if (!__all_sync(0xffffffffu, gwait(&sh->q_full, 0, sh))) ggive_up(sh, 49), ok = false;
-            const uint8_t *src = sV + set * 2 * KP + tid * 128;
+            // both sets take one head's rows, then the other's: the first head's S runs under the second's conversion
+            const float2 *angles = p.rope ? p.rope + (long long)(t < p.T ? t : 0) * (p.dim_out >> 1) : nullptr;
 #pragma unroll
-            for (int kb = 0; kb < NB; ++kb) {
-                uint32_t r[32];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 v4 = *reinterpret_cast<const uint4 *>(src + kb * (128 * 128) + ((c ^ (tid & 7)) << 4));
-                    r[4 * c] = v4.x, r[4 * c + 1] = v4.y, r[4 * c + 2] = v4.z, r[4 * c + 3] = v4.w;
-                }
-                tmem_st32(tmem + lane_base + cQh + set * W2 + kb * 32, r);
+            for (int hd = 0; hd < 2; ++hd) {
+                if (!__all_sync(0xffffffffu, gwait(&sh->q_full[hd], 0, sh))) ggive_up(sh, 49), ok = false;
+                const float x = convert_q<D, true>(sQ + hd * 4 * KP, set, tid, angles, p.dim_out, sh->q_top[hd], tmem + lane_base + cQh + hd * W2, 0u);
+                if (hd == set) top = x;
+                mbar_arrive_warp(&sh->a_ready[hd]);
             }
-            tmem_wait_st();
-            tc_fence_before();
-            mbar_arrive_warp(&sh->a_ready);
         }
-        const float cs = p.scale_log2 / (mq * mk);
+        pdl_wait();
+        const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+        publish_q_top(p, b * p.n_kv_heads + g, top);
+        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        FlushRow row{nullptr, nullptr, p.dim_out, D / 2};
-        if (FLUSH && t < p.T) {
-            row.lower = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
-            row.upper = row.lower + D / 2;
-        }
+        FlushRow row{nullptr, p.dim_out};
+        if (FLUSH && t < p.T) row.sums = p.out + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
         for (int j = 0; ok && j < n_tiles; ++j) {
             if (!__all_sync(0xffffffffu, gwait(&sh->s_full[set], (uint32_t)(j & 1), sh))) {
                 ggive_up(sh, 45);
@@ -316,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
-            const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
+            const bool add = FLUSH && m_flushed != -INFINITY && row.sums != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * (D * 4);
 #pragma unroll 1
@@ -327,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
+                    if (add && c + i < row.width) o4 = flush_sum4(row.sums + c + i, ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     const int ch = (c + i) >> 2;
                     *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;

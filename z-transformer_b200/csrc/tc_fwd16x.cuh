@@ -19,7 +19,7 @@
 // of 160 41 -> 36; 2 sequences of T 4096, 32/8 of 256 1695 -> 1663.
 // Per 64-key tile the tensor core issues 12 MMAs of N = 64 per block for S and 12 of N = D for P.V: heads of 132 to 192
 // columns on a tile of 192 issue three quarters of what they cost padded to 256.
-// The Q hi tile reaches TMEM through V's slot (TMA, then the row threads); the rows leave through the K and V
+// The query tile lands as f32 in V's slot and where Q lo goes, and is split by the row threads; the rows leave through the K and V
 // slots, a bulk copy a row.  Every wait is bounded; a wait that gives up raises g_tc_status.
 //
 // The backward at these widths: tc_bwd_wide.cuh.
@@ -34,7 +34,7 @@ constexpr int kThreadsX = 6 * 32;
 
 struct SharedX {
     uint64_t full_k[4], free_k[4], full_v[4], free_v[4];
-    uint64_t a_ready, q_full, ql_full, s_full[2], p_full[2], pv_done, staged, all_done;
+    uint64_t a_ready, q_full, s_full[2], p_full[2], pv_done, staged, all_done;
     uint32_t tmem_base;
     volatile int abort;
 };
@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     constexpr int KB = BN * 128;        // bytes of one 64-column block of one plane of a key tile (8 KB)
     constexpr int KP = NB * KB;         // one plane of a key tile (32 KB at 256 columns); a K or V tile is 2 KP
     constexpr int VB = NB * 16 * 128;   // one plane of 16 keys of a V tile (8 KB at 256 columns)
-    constexpr int QB = 128 * 128;       // one block of one plane of the 128-row query tile (16 KB)
+    constexpr int QB = 128 * 128;       // one block of the lo pieces of the 128-row query tile (16 KB)
+    static_assert(QB == kQBlock && KP * 2 == NB * QB, "the f32 query tile fills V's slot and Q lo");
     constexpr int cQh = 0, cO = 128, cS0 = 384;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // K: block c of the tile at sK + c * 2 KB (hi, then lo); V: 16 keys c of the tile at sV + c * 2 VB (hi, then lo); Q lo: NB blocks
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         for (int i = 0; i < NB; ++i) mbar_init(&sh->full_k[i], 1), mbar_init(&sh->free_k[i], 1);
         for (int i = 0; i < BN / 16; ++i) mbar_init(&sh->full_v[i], 1), mbar_init(&sh->free_v[i], 1);
         mbar_init(&sh->a_ready, 4);
-        mbar_init(&sh->q_full, 1), mbar_init(&sh->ql_full, 1);
+        mbar_init(&sh->q_full, 1);
         for (int i = 0; i < 2; ++i) mbar_init(&sh->s_full[i], 1), mbar_init(&sh->p_full[i], 4);
         mbar_init(&sh->pv_done, 1);
         mbar_init(&sh->staged, 4);
@@ -110,21 +111,17 @@ __global__ void __launch_bounds__(kThreadsX, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    pdl_wait();
-    pdl_launch();
-
-    const float mq = block_mult(p.amax_q[b * p.n_kv_heads + g]), mk = block_mult(p.amax_k[b * p.n_kv_heads + g]);
-    const float mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+    // (the query rows are older than the launch before this one, for whose planes and maxima pdl_wait() waits)
 
     if (warp == 4) {
         // ------------------------------------------------------------------ TMA producer
         if (elect_one() && !sh->abort) {
             tma_prefetch_desc(&qmap), tma_prefetch_desc(&kmap), tma_prefetch_desc(&vmap);
-            // the Q hi plane waits in V's slot until the row threads have moved it into TMEM
-            mbar_arrive_expect_tx(&sh->q_full, NB * QB);
-            tma_load_4d(sV, &qmap, &sh->q_full, 0, t0, h * NB, b);
-            mbar_arrive_expect_tx(&sh->ql_full, NB * QB);
-            tma_load_4d(sQl, &qmap, &sh->ql_full, 0, t0, h * NB, B + b);
+            // the query tile: the lower half of its columns in V's slot, the upper where Q lo goes
+            mbar_arrive_expect_tx(&sh->q_full, 2 * NB * QB);
+            load_q<D>(sV, &qmap, &sh->q_full, t0, h, b);
+            pdl_wait();
+            pdl_launch();
             int n_k = 0, n_v = 0;  // K blocks and V pieces issued
             bool live = true;
             auto load_k_block = [&](int j, int c) {
@@ -144,7 +141,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 }
             };
             for (int c = 0; c < NB; ++c) load_k_block(0, c);
-            if (!xwait(&sh->a_ready, 0, sh)) xgive_up(sh, 61), live = false;  // V's slot holds Q hi until then
+            if (!xwait(&sh->a_ready, 0, sh)) xgive_up(sh, 61), live = false;  // V's slot holds query columns until then
             if (live) load_v(0);
             for (int j = 1; live && j < n_tiles; ++j) {
                 for (int c = 0; live && c < NB; ++c) load_k_block(j, c);
@@ -152,7 +149,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             }
             if (sh->abort) {
                 // let the copies in flight land before the CTA's shared memory goes away
-                mbar_wait(&sh->q_full, 0), mbar_wait(&sh->ql_full, 0);
+                mbar_wait(&sh->q_full, 0);
                 for (int i = (n_k > NB ? n_k - NB : 0); i < n_k; ++i) mbar_wait(&sh->full_k[i % NB], (uint32_t)((i / NB) & 1));
                 for (int i = (n_v > 4 ? n_v - 4 : 0); i < n_v; ++i) mbar_wait(&sh->full_v[i & 3], (uint32_t)((i >> 2) & 1));
             }
@@ -164,7 +161,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             constexpr uint32_t id_s = idesc_f16(128, BN, false, false);
             const int steps = head_steps(p.dim_out);
             const uint32_t id_o = idesc_f16(128, 16 * steps, false, true);
-            bool ok = xwait(&sh->a_ready, 0, sh) && xwait(&sh->ql_full, 0, sh);
+            bool ok = xwait(&sh->a_ready, 0, sh);
             if (!ok) xgive_up(sh, 62);
             tc_fence_after();
             const uint32_t k_u32 = smem_u32(sK), v_u32 = smem_u32(sV), ql_u32 = smem_u32(sQl);
@@ -231,32 +228,39 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         const int t = t0 + tid, pos = p.q_offset + t;
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         bool ok = true;
+        float top = 0.f;  // max |q| of the row
         {
-            // this thread's row of the Q hi plane, out of the 128-byte-swizzled staging tile
+            // this thread's row: the hi pieces into TMEM, the lo ones where the upper columns were, which are in registers by then
             if (!__all_sync(0xffffffffu, xwait(&sh->q_full, 0, sh))) xgive_up(sh, 69), ok = false;
-            const uint8_t *src = sV + tid * 128;
-#pragma unroll 1
-            for (int kb = 0; kb < NB; ++kb) {
-                uint32_t r[32];
+            if (p.rope && t < p.T) rotate_q(sV, tid, p.rope + (long long)t * (p.dim_out >> 1), p.dim_out >> 3, 0, p.dim_out >> 3);
+            float4 upper[D / 8];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 v4 = *reinterpret_cast<const uint4 *>(src + kb * QB + ((c ^ (tid & 7)) << 4));
-                    r[4 * c] = v4.x, r[4 * c + 1] = v4.y, r[4 * c + 2] = v4.z, r[4 * c + 3] = v4.w;
-                }
-                tmem_st32(tmem + lane_base + cQh + kb * 32, r);
+            for (int c = 0; c < D / 8; ++c) {
+                upper[c] = *q_at(sV, tid, D / 8 + c);
+                top = fmaxf(top, fmaxf(max_abs4(upper[c]), max_abs4(*q_at(sV, tid, c))));
+            }
+            const float mq = block_mult(__float_as_uint(top));
+#pragma unroll
+            for (int cb = 0; cb < D / 32; ++cb) {
+                uint32_t qh[16], ql[16];
+                if (cb < D / 64) split_q32([&](int c) { return *q_at(sV, tid, cb * 8 + c); }, mq, qh, ql);
+                else split_q32([&](int c) { return upper[(cb - D / 64) * 8 + c]; }, mq, qh, ql);
+                tmem_st16(tmem + lane_base + cQh + cb * 16, qh);
+                store_q_lo(sQl, tid, cb, ql);
             }
             tmem_wait_st();
+            fence_async_smem();
             tc_fence_before();
             mbar_arrive_warp(&sh->a_ready);
         }
-        const float cs = p.scale_log2 / (mq * mk);
+        pdl_wait();
+        const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
+        publish_q_top(p, b * p.n_kv_heads + g, top);
+        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        FlushRow row{nullptr, nullptr, p.dim_out, D / 2};
-        if (FLUSH && t < p.T) {
-            row.lower = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
-            row.upper = row.lower + D / 2;
-        }
+        FlushRow row{nullptr, p.dim_out};
+        if (FLUSH && t < p.T) row.sums = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
         for (int j = 0; ok && j < n_tiles; ++j) {
             if (!__all_sync(0xffffffffu, xwait(&sh->s_full[j & 1], (uint32_t)((j >> 1) & 1), sh))) {
                 xgive_up(sh, 65);
@@ -341,7 +345,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         if (ok) {
             tc_fence_after();
             const float inv = l == 0.f ? 0.f : 1.f / (l * mv);  // l, like O, carries kPScale (0: a part without a key the row sees)
-            const bool add = FLUSH && m_flushed != -INFINITY && row.lower != nullptr;
+            const bool add = FLUSH && m_flushed != -INFINITY && row.sums != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
             uint8_t *srow = stage + tid * RS;
 #pragma unroll 1
@@ -352,7 +356,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
+                    if (add && c + i < row.width) o4 = flush_sum4(row.sums + c + i, ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     *reinterpret_cast<float4 *>(srow + (c + i) * 4) = o4;
                 }

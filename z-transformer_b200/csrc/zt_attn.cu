@@ -230,9 +230,9 @@ static size_t required_workspace(int batch, int T, int n_heads, int n_kv_heads, 
     return workspace_optional(T, dim) ? 0 : backward_need(batch, T, n_heads, n_kv_heads, dim).least;
 }
 
-// The forward-for-training call (zt_attn_forward_batched_keep) leaves the f16 planes of q, k, v in the backward's
+// The forward-for-training call (zt_attn_forward_batched_keep) leaves the f16 planes of k, v in the backward's
 // workspace and hands the caller a token; a backward that is given the token back (zt_attn_backward_batched_kept)
-// converts only dout.  The library keeps one record per (device, workspace) of which token is current, for which
+// converts only q and dout.  The library keeps one record per (device, workspace) of which token is current, for which
 // shape; a token is good for one backward, and any other call that writes the workspace retires it.  Nothing is
 // ever inferred from pointer values of q, k, v: reuse happens only when the caller asks for it.
 namespace {
@@ -793,8 +793,8 @@ static int forward_rope_impl(const float *q, const float *k, const float *v, flo
     // (the pre-pass rotates four elements at a time: a head's halves must be multiples of four)
     if ((g_path.load() == 0 || g_path.load() == 8) && n_kv_heads <= tcb::kPrepassMaxGroups && dim % 8 == 0 &&
         tc_fwd16_supported(batch, T, 0, dim, q, k, v, out) && least > 0 && w.inner_bytes >= least) {
-        // the planes (rotated q and k among them) go where the backward keeps its own: the rope backward that
-        // follows with the same workspace, tensors, pos and theta converts only dout
+        // the planes (rotated k among them) go where the backward keeps its own: the rope backward that
+        // follows with the same workspace, tensors, pos and theta converts only q and dout
         if (launch_fwd_tc16(q, k, v, out, lse, w.inner, w.inner_bytes, batch, T, n_heads, n_kv_heads, dim, s, w.table, true, 0, out_planes)) return 1;
         const unsigned long long token = note_kept_planes(w.inner, batch, T, n_heads, n_kv_heads, dim, true, pos, theta);
         if (host_token) *host_token = token;

@@ -41,7 +41,7 @@ def _head_config(n_heads, n_kv_heads, head_dim):
 
 class BackwardWorkspace:
     """Caller-owned scratch of the batched backward for one (batch, T, heads, dim) shape.  Handed to
-    attention_forward as `keep`, it also carries the forward's operand planes of q, k, v over to the backward."""
+    attention_forward as `keep`, it also carries the forward's operand planes of k, v over to the backward."""
 
     def __init__(self, batch, t, n_heads, n_kv_heads, head_dim, device="cuda"):
         import torch
@@ -53,7 +53,7 @@ class BackwardWorkspace:
 
 def attention_forward(q, k, v, n_heads, n_kv_heads, head_dim, *, want_lse=False, keep=None):
     """Batched attention.forward.  q [B, T, H*D] (or [T, H*D]); returns out (and lse [B, T, H]).
-    keep: a BackwardWorkspace of this shape; the forward's operand planes of q, k, v are left in it, and a
+    keep: a BackwardWorkspace of this shape; the forward's operand planes of k, v are left in it, and a
     backward given it with kept=True (the caller's word that q, k, v were not written in between) skips
     converting them again."""
     if keep is None or keep.shape == (*q.shape[:2], n_heads, n_kv_heads, head_dim):
