@@ -81,3 +81,34 @@ def test_gradient_of_q_over_q(zt, B, T, H, G, D):
     torch.cuda.synchronize()
     for a, b in zip((q, dk, dv), want):  # (sums that are made in memory come in no fixed order)
         assert float((a.double() - b.double()).norm()) <= 1e-6 * float(b.double().norm())
+
+
+def rotated(x, heads, D, pos, theta):
+    """x in float64 with its heads rotated as src/rope.zig does."""
+    B, T, _ = x.shape
+    i = torch.arange(D // 2, dtype=torch.float64, device=x.device)
+    angle = (pos + torch.arange(T, dtype=torch.float64, device=x.device))[:, None] / theta ** (2 * i / D)
+    c, s = angle.cos()[None, :, None], angle.sin()[None, :, None]
+    lo, hi = x.double().view(B, T, heads, 2, D // 2).unbind(3)
+    return torch.stack((lo * c - hi * s, hi * c + lo * s), 3).reshape(B, T, heads * D)
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [
+    (1, 200, 4, 2, 64), (1, 140, 6, 2, 80), (12, 300, 8, 2, 64), (40, 130, 3, 1, 40),  # one head a block; two blocks an SM
+    (14, 257, 8, 2, 128), (20, 130, 8, 4, 96), (1, 150, 4, 2, 256), (1, 300, 2, 1, 160),  # two heads; wide heads
+])
+def test_rotated_rows_and_the_planes_of_out(zt, B, T, H, G, D):
+    q, k, v, _ = inputs(B, T, H, G, D, (1, 1, 1), 0)
+    out, lse = zt.attention_forward_rope(q, k, v, H, G, D, pos=5, want_lse=True)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0
+    theta = zt.ops.ROPE_THETA
+    ref, ref_lse = forward64(rotated(q, H, D, 5, theta), rotated(k, G, D, 5, theta), v.double(), H, G, D, 0)
+    assert float((out.double() - ref).norm()) <= (bound(D, T) + 1e-6) * float(ref.norm())  # (a rotation is an f32 product sum)
+    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5
+    if H * D % 64:
+        return
+    wo = torch.randn(H * D, 64, device="cuda") / (H * D) ** 0.5
+    block = zt.AttentionBlock(B, T, H, G, D, 64)
+    y, y2 = (block.forward(q, k, v, wo, fused=f) for f in (True, False))
+    assert float((y - y2).abs().max()) <= 1e-6 * float(y2.abs().max())

@@ -71,13 +71,52 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
-// (a, b) -> packed h pair and packed l pair: one paired conversion each way instead of two single ones
-__device__ __forceinline__ void split_pack(float a, float b, uint32_t &hw, uint32_t &lw) {
-    const __half2 hh = __floats2half2_rn(a, b);
-    const float2 back = __half22float2(hh);
-    hw = *reinterpret_cast<const uint32_t *>(&hh);
-    lw = pack_half2(a - back.x, b - back.y);
+// Two f32 operations an instruction, each rounded as the single one is.
+__device__ __forceinline__ uint64_t pair2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
+__device__ __forceinline__ float2 unpair2(uint64_t r) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair2(a.x, a.y)), "l"(pair2(b.x, b.y)), "l"(pair2(c.x, c.y)));
+    return unpair2(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair2(a.x, a.y)), "l"(pair2(b.x, b.y)));
+    return unpair2(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair2(a.x, a.y)), "l"(pair2(b.x, b.y)));
+    return unpair2(r);
+}
+__device__ __forceinline__ float2 floats2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// x with its magnitude cut to `bound` (> 0); the bound itself for a NaN
+__device__ __forceinline__ float clamp_abs(float x, float bound) {
+    float r;
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(bound));
+    return r;
+}
+// v -> packed h pair and packed l pair, two values an instruction but for the way back
+__device__ __forceinline__ void split_pack(float2 v, uint32_t &hw, uint32_t &lw) {
+    const __half2 hh = __floats2half2_rn(v.x, v.y);
+    const float2 lo = fma2(__half22float2(hh), make_float2(-1.f, -1.f), v);
+    hw = *reinterpret_cast<const uint32_t *>(&hh);
+    lw = pack_half2(lo.x, lo.y);
+}
+__device__ __forceinline__ void split_pack(float a, float b, uint32_t &hw, uint32_t &lw) { split_pack(make_float2(a, b), hw, lw); }
 
 // ---- the two launches -------------------------------------------------------------------------------
 constexpr int kPrepassMaxGroups = 256;

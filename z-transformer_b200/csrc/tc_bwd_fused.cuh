@@ -40,7 +40,7 @@ struct FusedShared {
     uint64_t k_full, a_ready, st_full, dp_full, p_ready, ds_ready, dq_done, dq_free, ld_ready, flush_ready, flush_done, all_done;
     uint32_t tmem_base;
     volatile int abort;
-    float lse2[2][64], dels[2][64], csc[2][64], c1c[2][64];  // [buffer][query row of the step]
+    float nlse[2][64], ndel[2][64], csc[2][64], c1c[2][64];  // [buffer][query row of the step]
 };
 __device__ __forceinline__ bool fwait(uint64_t *bar, uint32_t parity, FusedShared *sh) {
     for (uint32_t i = 0; i < (1u << 20); ++i) {
@@ -371,22 +371,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         const float lse_shift = log2f(p.p_scale);
         const float inv_dov = 1.0f / (mdo * mv * p.p_scale);
         // Per query row of a step (fetched one step ahead by the first 64 threads of each set, published
-        // through shared memory): set 0 lse, set 1 delta cq / p_scale, set 2 the factor that turns K Q~^T into
+        // through shared memory): set 0 -lse, set 1 -delta cq / p_scale, set 2 the factor that turns K Q~^T into
         // log2-domain scores (scale_log2 cq / (mq mk cmin)), set 3 the factor of dP^T (cq / (mdo mv p_scale)).
         auto fetch = [&](const Walk &w, int it) -> float {
             if (tid >= 64 || it >= n_it) return 0.f;
             const int t = w.qi * BQ + tid;
             if (t >= p.T) return 0.f;
             const long long idx = ((long long)b * p.T + t) * p.n_heads + head0 + w.hh;
-            if (set == 0) return __ldg(p.lse + idx) * kLog2e - lse_shift;
+            if (set == 0) return lse_shift - __ldg(p.lse + idx) * kLog2e;
             float cq, rel;
             ds_row_scale(__ldg(p.rnorm + idx), rn_bits, vn_bits, cq, rel);
-            if (set == 1) return ZT_DEFECT(13) ? 0.f : __ldg(p.delta + idx) * cq / p.p_scale;
+            if (set == 1) return ZT_DEFECT(13) ? 0.f : -(__ldg(p.delta + idx) * cq / p.p_scale);
             if (set == 2) return cs_over_cmin * cq;
             return cq * inv_dov;
         };
         auto publish = [&](int it, float v) {
-            if (tid < 64) (set == 0 ? sh->lse2 : set == 1 ? sh->dels : set == 2 ? sh->csc : sh->c1c)[it & 1][tid] = v;
+            if (tid < 64) (set == 0 ? sh->nlse : set == 1 ? sh->ndel : set == 2 ? sh->csc : sh->c1c)[it & 1][tid] = v;
             mbar_arrive_warp(&sh->ld_ready);
         };
         Walk ahead = walk;  // one step ahead of `walk`
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         ahead.next();
         int n_flush = 0;
         bool ok = true;
-        bool saturated = false;
+        float ds_top = 0.f;
         auto flush_now = [&]() -> bool {
             if (!__all_sync(0xffffffffu, fwait(&sh->flush_ready, (uint32_t)(n_flush & 1), sh))) {
                 fgive_up(sh, 66);
@@ -506,34 +506,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             tc_fence_after();
             const uint32_t wS = tmem + lane_base + cST + set * 16;
             const uint32_t wP = tmem + lane_base + cDPT + set * 16;
-            const float *lse2 = sh->lse2[it & 1] + set * 16, *csc = sh->csc[it & 1] + set * 16;
-            float pr[16];
+            const float2 *nlse = reinterpret_cast<const float2 *>(sh->nlse[it & 1] + set * 16), *csc = reinterpret_cast<const float2 *>(sh->csc[it & 1] + set * 16);
+            float2 pr[8];
             {
                 uint32_t rs[16];
                 tmem_ld16(wS, rs);
                 tmem_wait_ld();
                 uint32_t ph[8], pl[8];
                 const int q_first = walk.qi * BQ;
-                if ((q_first >= s0 + 127 || ZT_DEFECT(11)) && q_first + BQ <= p.T && s0 + 128 <= p.T) {
+                const bool plain = (q_first >= s0 + 127 || ZT_DEFECT(11)) && q_first + BQ <= p.T && s0 + 128 <= p.T;
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
+                for (int i = 0; i < 8; ++i) {
+                    const float2 x = fma2(floats2(rs[2 * i], rs[2 * i + 1]), csc[i], nlse[i]);
+                    pr[i] = make_float2(ex2(x.x), ex2(x.y));
+                }
+                if (!plain) {
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) pr[i + e] = ex2(__uint_as_float(rs[i + e]) * csc[i + e] - lse2[i + e]);
-                        split_pack(pr[i], pr[i + 1], ph[i >> 1], pl[i >> 1]);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const int t = t0 + i + e;
-                            const bool vis = (key <= t || ZT_DEFECT(11)) && (t < p.T) && (key < p.T);
-                            const float pe = ex2(__uint_as_float(rs[i + e]) * csc[i + e] - lse2[i + e]);
-                            pr[i + e] = vis ? pe : 0.f;
-                        }
-                        split_pack(pr[i], pr[i + 1], ph[i >> 1], pl[i >> 1]);
+                    for (int i = 0; i < 8; ++i) {
+                        const auto vis = [&](int t) { return (key <= t || ZT_DEFECT(11)) && t < p.T && key < p.T; };
+                        pr[i].x = vis(t0 + 2 * i) ? pr[i].x : 0.f, pr[i].y = vis(t0 + 2 * i + 1) ? pr[i].y : 0.f;
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) split_pack(pr[i], ph[i], pl[i]);
                 tmem_st8(wS, ph);
                 tmem_st8(wS + 8, pl);
             }
@@ -560,21 +555,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             }
             tc_fence_after();
             {
-                const float *c1c = sh->c1c[it & 1] + set * 16, *dels = sh->dels[it & 1] + set * 16;
+                const float2 *c1c = reinterpret_cast<const float2 *>(sh->c1c[it & 1] + set * 16), *ndel = reinterpret_cast<const float2 *>(sh->ndel[it & 1] + set * 16);
                 uint32_t rd[16];
                 tmem_ld16(wP, rd);
                 tmem_wait_ld();
                 uint32_t dh[8], dl[8];
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    float dv[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float x = pr[i + e] * (__uint_as_float(rd[i + e]) * c1c[i + e] - dels[i + e]);
-                        saturated |= !(fabsf(x) <= kDsBound);
-                        dv[e] = fminf(fmaxf(x, -kDsBound), kDsBound);
-                    }
-                    split_pack(dv[0], dv[1], dh[i >> 1], dl[i >> 1]);
+                for (int i = 0; i < 8; ++i) {
+                    float2 x = mul2(pr[i], fma2(floats2(rd[2 * i], rd[2 * i + 1]), c1c[i], ndel[i]));
+                    x.x = clamp_abs(x.x, kDsBound), x.y = clamp_abs(x.y, kDsBound);
+                    ds_top = max3(ds_top, fabsf(x.x), fabsf(x.y));
+                    split_pack(x, dh[i], dl[i]);
                 }
                 tmem_st8(wP, dh);
                 tmem_st8(wP + 8, dl);
@@ -622,7 +613,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                 flush_now();
             }
         }
-        if (__any_sync(0xffffffffu, saturated) && lane == 0) atomicAdd(&g_tc_saturated, 1u);
+        if (__any_sync(0xffffffffu, ds_top >= kDsBound) && lane == 0) atomicAdd(&g_tc_saturated, 1u);
     }
     tc_fence_before();
     __syncthreads();
@@ -635,7 +626,7 @@ inline int launch_bwd_fused(const CUtensorMap &k128, const CUtensorMap &v128, co
     if (optin_smem((const void *)kernel, kFusedSmem)) return 1;
     const unsigned tiles = (unsigned)((p.T + 127) / 128), seqs = (unsigned)(p.batch * p.parts.n()), kv = (unsigned)p.n_kv_heads;
     const dim3 grid = p.by_tile ? dim3(kv, seqs, tiles) : dim3(kv, tiles, seqs);
-    return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), kFusedSmem, stream, k128, v128, qs64, g64, p);
+    return launch_after("attn_bwd_fused_tc", kernel, grid, dim3(kFusedThreads), kFusedSmem, stream, 1, k128, v128, qs64, g64, p);
 }
 
 }  // namespace tcf

@@ -57,44 +57,8 @@ __device__ __forceinline__ void fgive_up(Fused64Shared *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-// Two f32 operations an instruction.
-__device__ __forceinline__ uint64_t pair2(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpair2(uint64_t r) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-    return v;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair2(a.x, a.y)), "l"(pair2(b.x, b.y)), "l"(pair2(c.x, c.y)));
-    return unpair2(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair2(a.x, a.y)), "l"(pair2(b.x, b.y)));
-    return unpair2(r);
-}
-__device__ __forceinline__ float2 floats2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
-// split_pack with the subtraction of the two low pieces as one instruction
-__device__ __forceinline__ void split_pack2(float2 v, uint32_t &hw, uint32_t &lw) {
-    const __half2 hh = __floats2half2_rn(v.x, v.y);
-    const float2 lo = fma2(__half22float2(hh), make_float2(-1.f, -1.f), v);
-    hw = *reinterpret_cast<const uint32_t *>(&hh);
-    lw = pack_half2(lo.x, lo.y);
-}
 // The power of two at or below a normal x > 0; 0 for 0.
 __device__ __forceinline__ float pow2_of(float x) { return __uint_as_float(__float_as_uint(x) & 0x7f800000u); }
-// x with its magnitude cut to `bound` (> 0); the bound itself for a NaN
-__device__ __forceinline__ float clamp_abs(float x, float bound) {
-    float r;
-    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(bound));
-    return r;
-}
-
 // grid (n_kv_heads, ceil(T / 128), batch), 768 threads: 16 row warps, a TMA warp, two MMA warps, a warp for the rows'
 // constants, four warps that read accumulators out.
 constexpr int kFused64Threads = (kKvRowWarps + 8) * 32, kReadWarps = 4;
@@ -560,8 +524,8 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                             p1.x = vis(t + 2) ? p1.x : 0.f, p1.y = vis(t + 3) ? p1.y : 0.f;
                         }
                         pr[k] = mul2(p0, make_float2(pow2_of(c.x), pow2_of(c.y))), pr[k + 1] = mul2(p1, make_float2(pow2_of(c.z), pow2_of(c.w)));
-                        split_pack2(p0, ph[2 * i4], pl[2 * i4]);
-                        split_pack2(p1, ph[2 * i4 + 1], pl[2 * i4 + 1]);
+                        split_pack(p0, ph[2 * i4], pl[2 * i4]);
+                        split_pack(p1, ph[2 * i4 + 1], pl[2 * i4 + 1]);
                     }
                     tmem_st8(wS + 16 * w, ph);
                     tmem_st8(wS + 16 * w + 8, pl);
@@ -595,9 +559,9 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
                         float2 x1 = mul2(fma2(floats2(rd[i + 2], rd[i + 3]), dp_unit2, make_float2(n.z, n.w)), pr[k + 1]);
                         x0.x = clamp_abs(x0.x, kDsBound), x0.y = clamp_abs(x0.y, kDsBound);
                         x1.x = clamp_abs(x1.x, kDsBound), x1.y = clamp_abs(x1.y, kDsBound);
-                        ds_top = fmaxf(fmaxf(ds_top, fmaxf(fabsf(x0.x), fabsf(x0.y))), fmaxf(fabsf(x1.x), fabsf(x1.y)));
-                        split_pack2(x0, th[2 * i4], tl[2 * i4]);
-                        split_pack2(x1, th[2 * i4 + 1], tl[2 * i4 + 1]);
+                        ds_top = max3(max3(ds_top, fabsf(x0.x), fabsf(x0.y)), fabsf(x1.x), fabsf(x1.y));
+                        split_pack(x0, th[2 * i4], tl[2 * i4]);
+                        split_pack(x1, th[2 * i4 + 1], tl[2 * i4 + 1]);
                     }
                     tmem_st8(wP + 16 * w, th);
                     tmem_st8(wP + 16 * w + 8, tl);
@@ -643,7 +607,7 @@ inline int launch_bwd_fused64(const CUtensorMap &k128, const CUtensorMap &v128, 
     if (optin_smem((const void *)kernel, kFused64Smem)) return 1;
     const unsigned tiles = (unsigned)((p.T + 127) / 128), seqs = (unsigned)(p.batch * p.parts.n()), kv = (unsigned)p.n_kv_heads;
     const dim3 grid = p.by_tile ? dim3(kv, seqs, tiles) : dim3(kv, tiles, seqs);
-    return launch_after("attn_bwd_fused64_tc", kernel, grid, dim3(kFused64Threads), kFused64Smem, stream, k128, v128, qs128, g128, dqmap, dkmap, dvmap, p);
+    return launch_after("attn_bwd_fused64_tc", kernel, grid, dim3(kFused64Threads), kFused64Smem, stream, 1, k128, v128, qs128, g128, dqmap, dkmap, dvmap, p);
 }
 
 }  // namespace tcf

@@ -39,6 +39,11 @@ using tcb::kDsBound;
 using tcb::ds_group_scale;
 using tcb::ds_row_scale;
 using tcb::split_pack;
+using tcb::fma2;
+using tcb::mul2;
+using tcb::max3;
+using tcb::floats2;
+using tcb::clamp_abs;
 
 constexpr int kStages = 3;
 constexpr int kTB = 128 * 64 * 2;  // bytes of one plane of an operand tile
@@ -485,7 +490,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         const float lse2 = (t < p.T) ? __ldg(p.lse + ridx) * kLog2e - log2f(p.p_scale) : 0.f;
         const float c1 = cq / (mdo * mv * p.p_scale);
         const float dels = (t < p.T && !ZT_DEFECT(13)) ? __ldg(p.delta + ridx) * cq / p.p_scale : 0.f;
-        bool saturated = false;
+        float ds_top = 0.f;
         const long long plane = (long long)p.Tp * p.Tp;
         // the quad's first row, this thread's 32 columns, of the unit's hi planes (lo: unit_cap planes further)
         __half *p_hi = p.p_planes + (long long)u * plane + (long long)(m0 + (row & ~3)) * p.Tp + quarter * 32;
@@ -494,7 +499,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         for (int n = 0; ok && n < n_tiles; ++n) {
             const int n0 = n * 128;
             const bool diag = (n == m) || (m0 + 128 > p.T);
-            float pr[32];
+            float2 pr[16];
             if (!__all_sync(0xffffffffu, rwait(&sh->s_full, (uint32_t)(n & 1), sh))) { rgive_up(sh, 96); ok = false; break; }
             tc_fence_after();
             {
@@ -507,15 +512,19 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 const int key0 = n0 + quarter * 32;
                 uint32_t ph[16], pl[16];
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int key = key0 + i + e;
-                        const bool vis = !diag || ((key <= t || ZT_DEFECT(11)) && key < p.T && t < p.T);
-                        pr[i + e] = vis ? ex2(__uint_as_float(rs[i + e]) * cs - lse2) : 0.f;
-                    }
-                    split_pack(pr[i], pr[i + 1], ph[i >> 1], pl[i >> 1]);
+                for (int i = 0; i < 16; ++i) {
+                    const float2 x = fma2(floats2(rs[2 * i], rs[2 * i + 1]), make_float2(cs, cs), make_float2(-lse2, -lse2));
+                    pr[i] = make_float2(ex2(x.x), ex2(x.y));
                 }
+                if (diag) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const auto vis = [&](int key) { return (key <= t || ZT_DEFECT(11)) && key < p.T && t < p.T; };
+                        pr[i].x = vis(key0 + 2 * i) ? pr[i].x : 0.f, pr[i].y = vis(key0 + 2 * i + 1) ? pr[i].y : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) split_pack(pr[i], ph[i], pl[i]);
                 store_rows_quad(p_hi + n0, p.Tp, ph, lane);
                 store_rows_quad(p_hi + lo_off + n0, p.Tp, pl, lane);
             }
@@ -529,21 +538,18 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 mbar_arrive_warp_relaxed(&sh->dp_free);
                 uint32_t dh[16], dl[16];
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float dv[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float x = pr[i + e] * (__uint_as_float(rd[i + e]) * c1 - dels);  // (pr is zero where masked)
-                        saturated |= !(fabsf(x) <= kDsBound);
-                        dv[e] = fminf(fmaxf(x, -kDsBound), kDsBound);
-                    }
-                    split_pack(dv[0], dv[1], dh[i >> 1], dl[i >> 1]);
+                for (int i = 0; i < 16; ++i) {
+                    // (pr is zero where masked)
+                    float2 x = mul2(pr[i], fma2(floats2(rd[2 * i], rd[2 * i + 1]), make_float2(c1, c1), make_float2(-dels, -dels)));
+                    x.x = clamp_abs(x.x, kDsBound), x.y = clamp_abs(x.y, kDsBound);
+                    ds_top = max3(ds_top, fabsf(x.x), fabsf(x.y));
+                    split_pack(x, dh[i], dl[i]);
                 }
                 store_rows_quad(d_hi + n0, p.Tp, dh, lane);
                 store_rows_quad(d_hi + lo_off + n0, p.Tp, dl, lane);
             }
         }
-        if (__any_sync(0xffffffffu, saturated) && lane == 0) atomicAdd(&g_tc_saturated, 1u);
+        if (__any_sync(0xffffffffu, ds_top >= kDsBound) && lane == 0) atomicAdd(&g_tc_saturated, 1u);
     }
     tc_fence_before();
     __syncthreads();
@@ -943,16 +949,16 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
         p.unit0 = unit0;
         if (tile_scores) {
             const dim3 gs((unsigned)(nt * (nt + 1) / 2), (unsigned)units);
-            if (launch_after("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores", bwd_wide_scores, gs, dim3(kScoreThreads), smem, stream, 1, q_k, k_k, g_k, v_k, p)) return 1;
         } else {
             const dim3 gs((unsigned)units, (unsigned)nt);
-            if (launch_after("bwd_wide_scores_res", scores, gs, dim3(kResThreads), smem_r, stream, q_k, k_k, g_k, v_k, p)) return 1;
+            if (launch_after("bwd_wide_scores_res", scores, gs, dim3(kResThreads), smem_r, stream, 1, q_k, k_k, g_k, v_k, p)) return 1;
         }
         p.units = units;
         const long long n_units = 3LL * nt * units * p.pieces;
         const dim3 gp((unsigned)(n_units < split_sm_count() ? n_units : split_sm_count()));
         p.in_turn = products_in_turn(p.pieces, nt, units, split_sm_count());
-        if (launch_after("wide_products", products, gp, dim3(kTriThreads), smem_t, stream, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
+        if (launch_after("wide_products", products, gp, dim3(kTriThreads), smem_t, stream, 1, ds_k, ds_m, p_m, k_n, qs_n, g_n, p, (int)n_units))
             return 1;
     }
     return 0;

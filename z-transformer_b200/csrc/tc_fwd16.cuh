@@ -30,6 +30,10 @@ namespace tcf16 {
 using namespace tc;
 using tcb::block_mult;
 using tcb::split_pack;
+using tcb::fma2;
+using tcb::add2;
+using tcb::max3;
+using tcb::floats2;
 
 constexpr int kThreads = 320;  // 8 softmax warps (two sets of four), 1 TMA warp, 1 MMA warp
 constexpr float kPScale = 128.0f;  // 2^7: P is multiplied by it before its 16-bit split (the 7.0f in the kernels)
@@ -99,32 +103,37 @@ __device__ __forceinline__ void fgive_up(Shared *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-// The row work on 32 score columns, in two forms chosen per tile (the same for every thread of the CTA): a tile
-// that ends before the query tile begins needs no mask.  P comes out already multiplied by kPScale (the scale
-// rides in the exponent: `off` is the reference maximum minus log2 kPScale), split into packed f16 pairs.
-template <bool MASK>
-__device__ __forceinline__ float row_max32(const uint32_t (&r)[32], int key0, int t, float m) {
+// The row work on 32 score columns.  A softmax's warps share their schedulers' slots with each other and with the warp that issues the
+// MMAs, so it is paired (f32x2, three-operand maxima): ten instructions for two columns where there were fourteen.  Us of the forward,
+// before -> after: 512 rows at 3584 keys, 32/8 heads of 128 103 -> 99; batch 8, T 512, of 128 94 -> 86 (with the rows' way out, send_row).
+// Columns beyond the `visible` first one take no part: a tile needs this only where it reaches beyond the first of a warp's rows.
+__device__ __forceinline__ void mask32(uint32_t (&r)[32], int visible) {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-        if (!MASK || key0 + i <= t) m = fmaxf(m, __uint_as_float(r[i]));
-    return m;
+        if (i > visible) r[i] = 0xff800000u;
 }
-template <bool MASK>
-__device__ __forceinline__ float row_exp32(const uint32_t (&r)[32], int key0, int t, float cs, float off,
-                                           uint32_t (&ph)[16], uint32_t (&pl)[16]) {
-    float sum = 0.f;
+__device__ __forceinline__ float row_max32(const uint32_t (&r)[32], float m) {
+    float n = -INFINITY;  // (a chain of its own)
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+        m = max3(m, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+        n = max3(n, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+    }
+    return fmaxf(m, n);
+}
+// P comes out already multiplied by kPScale (the scale rides in the exponent: `off` is the reference maximum minus log2 kPScale), split into
+// packed f16 pairs.
+__device__ __forceinline__ float row_exp32(const uint32_t (&r)[32], float cs, float off, uint32_t (&ph)[16], uint32_t (&pl)[16]) {
+    const float2 cs2 = make_float2(cs, cs), off2 = make_float2(-off, -off);
+    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
-        float pe[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            pe[e] = ex2(__uint_as_float(r[i + e]) * cs - off);
-            if (MASK && key0 + i + e > t) pe[e] = 0.f;
-            sum += pe[e];
-        }
-        split_pack(pe[0], pe[1], ph[i >> 1], pl[i >> 1]);
+        const float2 x = fma2(floats2(r[i], r[i + 1]), cs2, off2);
+        const float2 pe = make_float2(ex2(x.x), ex2(x.y));
+        sum = add2(sum, pe);
+        split_pack(pe, ph[i >> 1], pl[i >> 1]);
     }
-    return sum;
+    return sum.x + sum.y;
 }
 
 // The tensor core adds into its f32 accumulator with truncation, which over n key tiles of 64 costs O about
@@ -210,6 +219,17 @@ __device__ __forceinline__ void store_q_lo(uint8_t *tile, int row, int block, co
     for (int c = 0; c < 4; ++c)
         *reinterpret_cast<uint4 *>(at + ((((block & 1) * 4 + c) ^ (row & 7)) << 4)) = make_uint4(l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]);
 }
+// A finished row, or a part of it, from its thread's staging row in shared memory to `dst`, as one bulk copy: nothing of the warp waits
+// for it but the end of the block.  (FLUSH: the row's running sum was written there by plain stores.)
+template <bool FLUSH>
+__device__ __forceinline__ void send_row(float *dst, const uint8_t *staged, int columns, bool wanted) {
+    fence_async_smem();
+    if (FLUSH) asm volatile("fence.proxy.async.global;" ::: "memory");
+    if (wanted && columns > 0) bulk_store(dst, staged, (uint32_t)columns * 4);
+    tma_commit();
+    tma_wait_read();
+}
+
 // A head's query row by two threads, which take a half of its columns each, out of their CTA's 256 (the barrier): hi pieces at TMEM `hi`,
 // lo pieces at TMEM `lo` or, where LO_SMEM, over the tile (the rows have been read by then: a half goes where the row's columns
 // of either thread were).  Returns the row's maximum; `tops` holds the halves'.
@@ -247,9 +267,9 @@ __device__ __forceinline__ void publish_q_top(const Params &p, int bg, float row
     const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(row_top));
     if ((threadIdx.x & 31) == 0) atomicMax(p.amax_q + bg, top);
 }
-// What turns a row's scores into log2 units.  (One division after the other: a row of tiny values may have a scale whose
-// product with k's is beyond f32.)
-__device__ __forceinline__ float score_scale(const Params &p, float mq, float mk) { return p.scale_log2 / mq / mk; }
+// What turns a row's scores into log2 units, more than zero.  (One division after the other: a row of tiny values may have a scale
+// whose product with k's is beyond f32.)
+__device__ __forceinline__ float score_scale(float scale_log2, float mq, float mk) { return fmaxf(scale_log2 / mq / mk, 1.17549435e-38f); }
 
 template <int D, bool FLUSH, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -444,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         pdl_wait();
         const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
         if (set == 0) publish_q_top(p, b * p.n_kv_heads + g, top);
-        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
+        const float cs = score_scale(p.scale_log2, block_mult(__float_as_uint(top)), mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
@@ -463,15 +483,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_after();
             const int s0 = (jb + j) * BN;
-            const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
+            const bool diag = (s0 + BN - 1 > p.q_offset + t0 + (warp & 3) * 32) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32_joined(tmem + lane_base + cS, r0);
             tmem_ld32_joined(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
-            float mt = -INFINITY;
-            if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
-            else mt = row_max32<false>(r1, s0 + 32, pos, row_max32<false>(r0, s0, pos, mt));
-            mt *= cs;  // cs > 0
+            if (diag) mask32(r0, pos - s0), mask32(r1, pos - s0 - 32);
+            const float mt = row_max32(r1, row_max32(r0, -INFINITY)) * cs;  // cs > 0
             float factor = 1.f;
             const float m_old = m_ref;
             if ((mt > m_ref + kRescaleThreshold || m_ref == -INFINITY) && mt != -INFINITY) {
@@ -512,10 +530,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             float psum;
             {
                 uint32_t ph[16], pl[16];
-                psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
+                psum = row_exp32(r0, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 16, pl);
-                psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
+                psum += row_exp32(r1, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS + 32, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 48, pl);
             }
@@ -528,15 +546,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         sh->fin_m[set][tid] = m_ref;
         sh->fin_l[set][tid] = l;
         sh->fin_f[set][tid] = m_flushed;
+        if (FLUSH) asm volatile("fence.proxy.async.global;" ::: "memory");  // (each set sends columns of the row that the other has summed, too)
         asm volatile("bar.sync 1, 256;" ::: "memory");  // the 256 softmax threads
         if (ok && !__all_sync(0xffffffffu, fwait(&sh->all_done, 0, sh))) {
             fgive_up(sh, 48);
             ok = false;
         }
-        // The merged rows go to global memory through shared memory (K's slots: every tile has been consumed
-        // once all_done completes): a thread owns a row in TMEM, and 32 rows per store instruction would cost
-        // 32 memory transactions each; written back a row (or two) per instruction they cost four.
-        constexpr int CH = D / 4;  // 16-byte chunks per row; chunk c of row r sits at chunk c ^ (r & (CH - 1))
+        // The merged rows go to global memory through shared memory (K's slots: every tile has been consumed once all_done
+        // completes), a half row of each thread as one bulk copy.  A row that goes to more places than out goes by stores, a row
+        // (or two) an instruction.
+        constexpr int RS = D * 4 + 16;  // (eight threads' chunks lie in different banks)
+        const bool plain = p.o_planes == nullptr && p.out_peers.n == 0;
+        uint8_t *srow = sK + tid * RS;
         if (ok) {
             tc_fence_after();
             const bool two = n_tiles > 1;  // set 1 has an accumulator only then
@@ -553,7 +574,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool add0 = FLUSH && s0 != -INFINITY && row0.sums != nullptr, add1 = FLUSH && s1 != -INFINITY && row1.sums != nullptr;
             const float g0 = add0 ? ex2(s0 - m0) : 0.f, g1 = add1 ? ex2(s1 - m1) : 0.f;
             // set s merges columns [s D/2, (s+1) D/2) of the row
-            uint8_t *srow = sK + tid * (D * 4);
 #pragma unroll 1
             for (int c = 0; c < D / 2; c += 32) {
                 uint32_t ra[32], rb[32];
@@ -571,15 +591,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                         if (add1 && col < row1.width) x4 = flush_sum4(row1.sums + col, g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
-                    const int ch = (set * (D / 2) + c + i) >> 2;
-                    *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;
+                    *reinterpret_cast<float4 *>(srow + col * 4) = o4;
                 }
             }
             if (set == 0 && p.lse && t < p.T)
                 p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (mm + log2f(lsum) - 7.0f) * kLn2;
         }
+        if (plain) {
+            const int c0 = set * (D / 2), mine = p.dim_out - c0 < D / 2 ? p.dim_out - c0 : D / 2;
+            send_row<FLUSH>(p.out + part * p.out_part + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out + c0, srow + c0 * 4, mine, ok && t < p.T);
+        }
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (!sh->abort) {
+        if (!plain && !sh->abort) {
+            constexpr int CH = D / 4;  // 16-byte chunks per row
             constexpr int RPI = 32 / CH;  // rows per store instruction
             const int lane = threadIdx.x & 31;
             const int ch = lane & (CH - 1);
@@ -588,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 4
             for (int i = 0; i < 16; i += RPI) {
                 const int r = warp * 16 + i + lane / CH;
-                const float4 o4 = *reinterpret_cast<const float4 *>(sK + r * (D * 4) + ((ch ^ (r & (CH - 1))) << 4));
+                const float4 o4 = *reinterpret_cast<const float4 *>(sK + r * RS + ch * 16);
                 if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
                     store_out4(p, part * p.out_part + ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
             }
@@ -638,7 +662,7 @@ inline int launch_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid = p.by_tile ? tile_major_grid(p.n_heads, (p.T + 127) / 128, p.batch * p.parts, kFwdTileWaves)
                                 : dim3((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
-    return launch_after("attn_fwd_tc16", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16", kernel, grid, dim3(kThreads), smem, stream, 1, kmap, vmap, qmap, p);
 }
 
 // (tc_fwd16x.cuh)

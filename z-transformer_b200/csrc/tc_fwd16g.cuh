@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         pdl_wait();
         const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
         publish_q_top(p, b * p.n_kv_heads + g, top);
-        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
+        const float cs = score_scale(p.scale_log2, block_mult(__float_as_uint(top)), mk);
         const uint32_t cS = cS0 + set * BN, cO = cO0 + set * D;
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
@@ -236,15 +236,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_after();
             const int s0 = j * BN;
-            const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
+            const bool diag = (s0 + BN - 1 > p.q_offset + t0 + (warp & 3) * 32) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32_joined(tmem + lane_base + cS, r0);
             tmem_ld32_joined(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
-            float mt = -INFINITY;
-            if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
-            else mt = row_max32<false>(r1, s0 + 32, pos, row_max32<false>(r0, s0, pos, mt));
-            mt *= cs;  // cs > 0
+            if (diag) mask32(r0, pos - s0), mask32(r1, pos - s0 - 32);
+            const float mt = row_max32(r1, row_max32(r0, -INFINITY)) * cs;  // cs > 0
             float factor = 1.f;
             const float m_old = m_ref;
             if ((mt > m_ref + kRescaleThreshold || m_ref == -INFINITY) && mt != -INFINITY) {
@@ -285,10 +283,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             float psum;
             {
                 uint32_t ph[16], pl[16];
-                psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
+                psum = row_exp32(r0, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 16, pl);
-                psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
+                psum += row_exp32(r1, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS + 32, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 48, pl);
             }
@@ -301,16 +299,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             ggive_up(sh, 48);
             ok = false;
         }
-        // The head's rows go to global memory through shared memory (the rings are idle once all_done completes):
-        // head A's in the first 4 KP bytes, head B's in the next; a row per store instruction instead of 32.
-        constexpr int CH = D / 4;  // 16-byte chunks per row; chunk c of row r sits at chunk c ^ (r & (CH - 1))
-        uint8_t *stage = smem_raw + set * 4 * KP;
+        // The head's rows go to global memory through shared memory (the rings are idle once all_done completes), as in
+        // attn_fwd_tc16: 6400 clocks of a CTA by stores of whole rows.
+        constexpr int RS = D * 4 + 16;
+        const bool plain = p.o_planes == nullptr && p.out_peers.n == 0;
+        uint8_t *stage = smem_raw + set * 128 * RS, *srow = stage + tid * RS;
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / (l * mv);  // l, like O, carries kPScale
             const bool add = FLUSH && m_flushed != -INFINITY && row.sums != nullptr;
             const float ff = add ? ex2(m_flushed - m_ref) : 0.f;
-            uint8_t *srow = stage + tid * (D * 4);
 #pragma unroll 1
             for (int c = 0; c < D; c += 32) {
                 uint32_t ra[32];
@@ -321,14 +319,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
                     if (add && c + i < row.width) o4 = flush_sum4(row.sums + c + i, ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
-                    const int ch = (c + i) >> 2;
-                    *reinterpret_cast<float4 *>(srow + ((ch ^ (tid & (CH - 1))) << 4)) = o4;
+                    *reinterpret_cast<float4 *>(srow + (c + i) * 4) = o4;
                 }
             }
             if (p.lse && t < p.T) p.lse[((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
         }
+        if (plain) send_row<FLUSH>(p.out + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out, srow, p.dim_out, ok && t < p.T);
         mbar_arrive_warp(&sh->staged[set]);
-        if (__all_sync(0xffffffffu, gwait(&sh->staged[set], 0, sh)) && !sh->abort) {
+        if (!plain && __all_sync(0xffffffffu, gwait(&sh->staged[set], 0, sh)) && !sh->abort) {
+            constexpr int CH = D / 4;  // 16-byte chunks per row
             constexpr int RPI = 32 / CH;  // rows per store instruction
             const int ch = lane & (CH - 1);
             const long long wo = (long long)p.n_heads * p.dim_out;
@@ -336,7 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 4
             for (int i = 0; i < 32; i += RPI) {
                 const int r = (warp & 3) * 32 + i + lane / CH;
-                const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * (D * 4) + ((ch ^ (r & (CH - 1))) << 4));
+                const float4 o4 = *reinterpret_cast<const float4 *>(stage + r * RS + ch * 16);
                 if (t0 + r < p.T && ch * 4 < p.dim_out)  // (a padded tile's upper columns are not the tensor's)
                     store_out4(p, ((long long)b * p.T + t0 + r) * wo + (long long)h * p.dim_out + ch * 4, o4, mo);
             }
@@ -355,7 +354,7 @@ inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
     const auto kernel = with_flags([](auto flush, auto pad) { return attn_fwd_tc16g<D, flush.value, pad.value>; }, p.flush, head_steps(p.dim_out) < D / 16);
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid = tile_major_grid(p.n_heads / 2, (p.T + 127) / 128, p.batch, kFwdTileWaves);
-    return launch_after("attn_fwd_tc16g", kernel, grid, dim3(kThreads), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16g", kernel, grid, dim3(kThreads), smem, stream, 1, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

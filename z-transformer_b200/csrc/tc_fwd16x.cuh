@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         pdl_wait();
         const float mk = block_mult(p.amax_k[b * p.n_kv_heads + g]), mv = block_mult(p.amax_v[b * p.n_kv_heads + g]);
         publish_q_top(p, b * p.n_kv_heads + g, top);
-        const float cs = score_scale(p, block_mult(__float_as_uint(top)), mk);
+        const float cs = score_scale(p.scale_log2, block_mult(__float_as_uint(top)), mk);
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         FlushRow row{nullptr, p.dim_out};
@@ -270,15 +270,13 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             tc_fence_after();
             const int s0 = (jb + j) * BN;
             const uint32_t cS = cS0 + (j & 1) * BN;
-            const bool diag = (s0 + BN - 1 > p.q_offset + t0) && !ZT_DEFECT(1);
+            const bool diag = (s0 + BN - 1 > p.q_offset + t0 + warp * 32) && !ZT_DEFECT(1);
             uint32_t r0[32], r1[32];
             tmem_ld32_joined(tmem + lane_base + cS, r0);
             tmem_ld32_joined(tmem + lane_base + cS + 32, r1);
             tmem_wait_ld();
-            float mt = -INFINITY;
-            if (diag) mt = row_max32<true>(r1, s0 + 32, pos, row_max32<true>(r0, s0, pos, mt));
-            else mt = row_max32<false>(r1, s0 + 32, pos, row_max32<false>(r0, s0, pos, mt));
-            mt *= cs;  // cs > 0
+            if (diag) mask32(r0, pos - s0), mask32(r1, pos - s0 - 32);
+            const float mt = row_max32(r1, row_max32(r0, -INFINITY)) * cs;  // cs > 0
             float factor = 1.f;
             const float m_old = m_ref;
             if ((mt > m_ref + kRescaleThreshold || m_ref == -INFINITY) && mt != -INFINITY) {
@@ -319,10 +317,10 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             float psum;
             {
                 uint32_t ph[16], pl[16];
-                psum = diag ? row_exp32<true>(r0, s0, pos, cs, off, ph, pl) : row_exp32<false>(r0, s0, pos, cs, off, ph, pl);
+                psum = row_exp32(r0, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 16, pl);
-                psum += diag ? row_exp32<true>(r1, s0 + 32, pos, cs, off, ph, pl) : row_exp32<false>(r1, s0 + 32, pos, cs, off, ph, pl);
+                psum += row_exp32(r1, cs, off, ph, pl);
                 tmem_st16_joined(tmem + lane_base + cS + 32, ph);
                 tmem_st16_joined(tmem + lane_base + cS + 48, pl);
             }
@@ -363,13 +361,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
             }
             if (p.lse && t < p.T) p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (m_ref + log2f(l) - 7.0f) * kLn2;
         }
-        if (plain) {
-            fence_async_smem();
-            if (FLUSH) asm volatile("fence.proxy.async.global;" ::: "memory");  // (the row's running sum was written by plain stores)
-            if (ok && t < p.T) bulk_store(p.out + part * p.out_part + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out, stage + tid * RS, (uint32_t)p.dim_out * 4);
-            tma_commit();
-            tma_wait_read();
-        }
+        if (plain) send_row<FLUSH>(p.out + part * p.out_part + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out, stage + tid * RS, p.dim_out, ok && t < p.T);
         mbar_arrive_warp(&sh->staged);
         if (!plain && __all_sync(0xffffffffu, xwait(&sh->staged, 0, sh)) && !sh->abort) {
             const long long wo = (long long)p.n_heads * p.dim_out;
@@ -402,7 +394,7 @@ inline int launch_x_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid = p.by_tile ? tile_major_grid(p.n_heads, (p.T + 127) / 128, p.batch * p.parts, kFwdTileWaves)
                                 : dim3((unsigned)((p.T + 127) / 128), (unsigned)p.n_heads, (unsigned)(p.batch * p.parts));
-    return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, kmap, vmap, qmap, p);
+    return launch_after("attn_fwd_tc16x", kernel, grid, dim3(kThreadsX), smem, stream, 1, kmap, vmap, qmap, p);
 }
 
 }  // namespace tcf16

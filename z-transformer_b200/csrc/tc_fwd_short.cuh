@@ -147,13 +147,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
     const int row = (warp & 3) * 32 + lane, quarter = warp >> 2, key0 = quarter * 32, pos = ZT_DEFECT(1) ? n_keys - 1 : p.q_offset + row;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const bool some = key0 < kn;
-    const float cs = p.scale_log2 / (mult[0] * mult[1]);
+    const float cs = tcf16::score_scale(p.scale_log2, mult[0], mult[1]);
     uint32_t r[32];
     float m = -INFINITY;
     if (some) {
         tmem_ld32(tmem + lane_base + cS + key0, r);
         tmem_wait_ld();
-        m = tcf16::row_max32<true>(r, key0, pos, m) * cs;
+        tcf16::mask32(r, pos - key0);
+        m = tcf16::row_max32(r, m) * cs;
     }
     sh->m[quarter][row] = m;
     __syncthreads();
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_short(const Params p) {
     float sum = 0.f;
     if (some) {
         uint32_t ph[16], pl[16];
-        sum = tcf16::row_exp32<true>(r, key0, pos, cs, off, ph, pl);
+        sum = tcf16::row_exp32(r, cs, off, ph, pl);
         tmem_st16(tmem + lane_base + cS + key0, ph);
         tmem_st16(tmem + lane_base + cS + key0 + 16, pl);
         tmem_wait_st();
@@ -226,7 +227,7 @@ template <int D>
 inline int launch_d(const Params &p, int batch, cudaStream_t stream) {
     const size_t smem = (size_t)6 * (D / 64) * 128 * 128 + sizeof(Shared);
     if (optin_smem((const void *)attn_fwd_short<D>, smem)) return 1;
-    return launch_after("attn_fwd_short", attn_fwd_short<D>, dim3((unsigned)p.n_heads, (unsigned)batch), dim3(kThreads), smem, stream, p);
+    return launch_after("attn_fwd_short", attn_fwd_short<D>, dim3((unsigned)p.n_heads, (unsigned)batch), dim3(kThreads), smem, stream, 1, p);
 }
 
 }  // namespace tcshort

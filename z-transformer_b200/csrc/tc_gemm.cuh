@@ -417,12 +417,12 @@ inline int launch_gemm(const CUtensorMap &amap, const CUtensorMap &bmap, const G
         const size_t smem = (size_t)kWideStages * 6 * (128 * 64 * 2) + sizeof(GemmWideShared);
         if (optin_smem((const void *)gemm_f16split_wide<A_MN, B_MN>, smem)) return 1;
         const dim3 grid((unsigned)(wide < sms ? wide : sms));
-        return launch_after("gemm_f16split_wide", gemm_f16split_wide<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, amap, bmap, p, (int)wide);
+        return launch_after("gemm_f16split_wide", gemm_f16split_wide<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, 1, amap, bmap, p, (int)wide);
     }
     const size_t smem = gemm_smem_bytes();
     if (optin_smem((const void *)gemm_f16split_tc<A_MN, B_MN>, smem)) return 1;
     const dim3 grid((unsigned)((p.m_rows + 127) / 128), (unsigned)((p.n_cols + 127) / 128), (unsigned)(p.batch * p.pieces));
-    return launch_after("gemm_f16split_tc", gemm_f16split_tc<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, amap, bmap, p);
+    return launch_after("gemm_f16split_tc", gemm_f16split_tc<A_MN, B_MN>, grid, dim3(kGemmThreads), smem, stream, 1, amap, bmap, p);
 }
 
 }  // namespace tcg

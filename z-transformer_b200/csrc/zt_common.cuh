@@ -198,11 +198,12 @@ inline int launch_pdl_cluster(const char *name, void (*kernel)(P...), dim3 grid,
 // A longer grid set up early starts as the SMs fall free, one by one, and its blocks then walk their tiles out of step
 // with the neighbours they share them with in L2: forward and backward at T 32768 took 4 % longer that way, and
 // batch 8, T 512, heads of 64 still 1.6 %.
+// `per_sm`: blocks that an SM holds.
 template <typename... P, typename... A>
-inline int launch_after(const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline int launch_after(const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int per_sm,
                         const A &...args) {
     const DeviceInfo *d = device_info();
-    if (d && (long long)grid.x * grid.y * grid.z <= d->sm_count) return launch_pdl(name, kernel, grid, block, smem, stream, args...);
+    if (d && (long long)grid.x * grid.y * grid.z <= (long long)per_sm * d->sm_count) return launch_pdl(name, kernel, grid, block, smem, stream, args...);
     const int pi = prof_begin(stream);
     kernel<<<grid, block, smem, stream>>>(args...);
     prof_end(pi, name, stream);
