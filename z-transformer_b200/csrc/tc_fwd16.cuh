@@ -105,7 +105,8 @@ __device__ __forceinline__ void fgive_up(Shared *sh, int code) {
 
 // The row work on 32 score columns.  A softmax's warps share their schedulers' slots with each other and with the warp that issues the
 // MMAs, so it is paired (f32x2, three-operand maxima): ten instructions for two columns where there were fourteen.  Us of the forward,
-// before -> after: 512 rows at 3584 keys, 32/8 heads of 128 103 -> 99; batch 8, T 512, of 128 94 -> 86 (with the rows' way out, send_row).
+// before -> after: 4 of T 2000, 12/4 heads of 64 77 -> 70, 16 of 300, 4/2 of 48 16.7 -> 14.7 (attn_fwd_tc16n); 512 rows at 3584 keys, 32/8 of
+// 128 103 -> 99 (with the rows' way out, send_row).
 // Columns beyond the `visible` first one take no part: a tile needs this only where it reaches beyond the first of a warp's rows.
 __device__ __forceinline__ void mask32(uint32_t (&r)[32], int visible) {
 #pragma unroll
@@ -673,6 +674,8 @@ inline int launch_x_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CU
 template <int D>
 inline int launch_g_d(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p,
                       cudaStream_t stream);
+// (tc_fwd16n.cuh)
+inline int launch_n(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, Params p, int sms, cudaStream_t stream);
 
 }  // namespace tcf16
 
@@ -750,8 +753,14 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     // per CTA; 2: two heads per CTA whatever the number of CTAs (the group must be even).
     const long long pair_ctas = (long long)((T + 127) / 128) * (n_heads / 2) * batch;
     const bool pairs = td <= 128 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
+    const long long blocks = (long long)((T + 127) / 128) * n_heads * batch;
+    // Up to 64 columns, with more than a CTA an SM: two an SM (attn_fwd_tc16n).  Below, one tile at a time, two softmax sets in turn are the
+    // quicker.  (Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to: 1200 rows at 1100 keys, 32/8
+    // heads of 64 take 84 us there and 68 here.)
+    const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
     int rc;
-    if (td == 256) rc = tcf16::launch_x_d<256>(kmap, vmap, qmap, p, stream);
+    if (narrow) rc = tcf16::launch_n(kmap, vmap, qmap, p, sms, stream);
+    else if (td == 256) rc = tcf16::launch_x_d<256>(kmap, vmap, qmap, p, stream);
     else if (td == 192) rc = tcf16::launch_x_d<192>(kmap, vmap, qmap, p, stream);
     else if (pairs) rc = td == 64 ? tcf16::launch_g_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_g_d<128>(kmap, vmap, qmap, p, stream);
     else rc = td == 64 ? tcf16::launch_d<64>(kmap, vmap, qmap, p, stream) : tcf16::launch_d<128>(kmap, vmap, qmap, p, stream);

@@ -18,6 +18,7 @@
 #include "tc_fwd.cuh"
 #include "tc_fwd16.cuh"
 #include "tc_fwd16g.cuh"
+#include "tc_fwd16n.cuh"
 #include "tc_fwd16x.cuh"
 #include "tc_fwd_short.cuh"
 #include "tc_gemm.cuh"
