@@ -105,7 +105,7 @@ __device__ __forceinline__ void fgive_up(Shared *sh, int code) {
 
 // The row work on 32 score columns.  A softmax's warps share their schedulers' slots with each other and with the warp that issues the
 // MMAs, so it is paired (f32x2, three-operand maxima): ten instructions for two columns where there were fourteen.  Us of the forward,
-// before -> after: 4 of T 2000, 12/4 heads of 64 77 -> 70, 16 of 300, 4/2 of 48 16.7 -> 14.7 (attn_fwd_tc16n); 512 rows at 3584 keys, 32/8 of
+// before -> after: 512 rows at 3584 keys, 32/8 of
 // 128 103 -> 99 (with the rows' way out, send_row).
 // Columns beyond the `visible` first one take no part: a tile needs this only where it reaches beyond the first of a warp's rows.
 __device__ __forceinline__ void mask32(uint32_t (&r)[32], int visible) {
@@ -213,8 +213,8 @@ __device__ __forceinline__ void split_q32(const X &column4, float m, uint32_t (&
         split_pack(x.z * m, x.w * m, h[2 * c + 1], l[2 * c + 1]);
     }
 }
-// The lo pieces of the tile's 32 columns `block` into the K-major tile of halves that an MMA reads: half of a block of 64 columns.
-__device__ __forceinline__ void store_q_lo(uint8_t *tile, int row, int block, const uint32_t (&l)[16]) {
+// One piece each of the tile's 32 columns `block` into the K-major tile of halves that an MMA reads: half of a block of 64 columns.
+__device__ __forceinline__ void store_q_piece(uint8_t *tile, int row, int block, const uint32_t (&l)[16]) {
     uint8_t *at = tile + (block >> 1) * kQBlock + row * 128;
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -254,7 +254,7 @@ __device__ __forceinline__ float convert_q(uint8_t *tile, int set, int row, cons
         uint32_t qh[16], ql[16];
         split_q32([&](int c) { return x[cb * 8 + c]; }, m, qh, ql);
         tmem_st16(hi + set * (D / 4) + cb * 16, qh);
-        if (LO_SMEM) store_q_lo(tile, row, set * (D / 64) + cb, ql);
+        if (LO_SMEM) store_q_piece(tile, row, set * (D / 64) + cb, ql);
         else tmem_st16(lo + set * (D / 4) + cb * 16, ql);
     }
     tmem_wait_st();
@@ -755,8 +755,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     const bool pairs = td <= 128 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
     const long long blocks = (long long)((T + 127) / 128) * n_heads * batch;
     // Up to 64 columns, with more than a CTA an SM: two an SM (attn_fwd_tc16n).  Below, one tile at a time, two softmax sets in turn are the
-    // quicker.  (Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to: 1200 rows at 1100 keys, 32/8
-    // heads of 64 take 84 us there and 68 here.)
+    // quicker.  (Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to.)
     const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
     int rc;
     if (narrow) rc = tcf16::launch_n(kmap, vmap, qmap, p, sms, stream);

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
                 if (cb < D / 64) split_q32([&](int c) { return *q_at(sV, tid, cb * 8 + c); }, mq, qh, ql);
                 else split_q32([&](int c) { return upper[(cb - D / 64) * 8 + c]; }, mq, qh, ql);
                 tmem_st16(tmem + lane_base + cQh + cb * 16, qh);
-                store_q_lo(sQl, tid, cb, ql);
+                store_q_piece(sQl, tid, cb, ql);
             }
             tmem_wait_st();
             fence_async_smem();
