@@ -44,23 +44,6 @@ struct DecodeParams {
     float scale_log2;
 };
 
-// ---- thread-block clusters ----------------------------------------------------------------------
-__device__ __forceinline__ void cluster_arrive() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-    __syncwarp();  // (.aligned: the whole warp together, also where what lies before it was a single thread's)
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// A float of block `rank`'s shared memory, at the place that `addr` has in this block's.
-__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
-    float v;
-    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n"
-                 : "=f"(v) : "r"(addr), "r"(rank) : "memory");
-    return v;
-}
-
 // How many sequences name no valid prefix: counted by one block, so that nothing has to be cleared beforehand.
 __device__ __forceinline__ void count_bad_sequences(const DecodeParams &p) {
     __shared__ int total;

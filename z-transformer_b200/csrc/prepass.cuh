@@ -148,6 +148,7 @@ struct PassArgs {
     long long fill_n4[3];
     int fill_first[4];  // first block of each region; [n_fill]: one past the last
     int n, n_stats, n_fill, dim, pd;  // dim: columns of a head in the tensors; pd: in the planes (plane_dim)
+    int cluster;                      // of the one-launch form: blocks per (sequence, group)
     int q_units;                      // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
 };
 
@@ -411,6 +412,27 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
 }
 
+// A block's two maxima -> its cluster's.  Leaves the cluster's barrier arrived at, to be waited for at the end of the kernel: nobody's shared
+// memory may go away while others read it.  So the words read are stored again, behind which the block meets, before it arrives: a load whose
+// value nothing waits for could still be on its way when the block that it reads has left.
+__device__ __forceinline__ void cluster_tops(int cluster, uint32_t &top, uint32_t &norm) {
+    __shared__ float mine[2];
+    __shared__ uint32_t all[2];
+    if (threadIdx.x == 0) mine[0] = __uint_as_float(top), mine[1] = __uint_as_float(norm);
+    cluster_arrive();
+    cluster_wait();
+    if (threadIdx.x < 32) {
+        const int from = (int)threadIdx.x < cluster ? (int)threadIdx.x : 0;
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(mine);
+        const uint32_t x = __reduce_max_sync(0xffffffffu, __float_as_uint(ld_cluster(at, from)));
+        const uint32_t y = __reduce_max_sync(0xffffffffu, __float_as_uint(ld_cluster(at + 4u, from)));
+        if (threadIdx.x == 0) all[0] = x, all[1] = y;
+    }
+    __syncthreads();
+    cluster_arrive();
+    top = all[0], norm = all[1];
+}
+
 // ---- the one launch of small forwards ---------------------------------------------------------------
 // Both launches in one, for forwards whose every (sequence, group) fits the registers of a block: 16 float4 a thread.  A block reads
 // its group's rows once, all loads under way together, knows the maxima after one barrier and writes the planes out of
@@ -420,7 +442,11 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
 // backward of 64 rows, 32/8 heads of 128, 70 -> 77.)
 // Two forms: of 16 float4 a thread, and of 4, with three blocks an SM: forward and backward of 7 sequences of 87, 16/16 heads of 32,
 // took 38.8 in two launches, 41.6 with the former alone, 36.3 with the latter.
-constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4;
+// A (sequence, group) of k or v that is more than a block's goes to a cluster of at most eight, which puts its maxima together through
+// distributed shared memory.  Us a forward, two launches -> a cluster a group: one of T 150, 8/2 heads of 128 17.5 -> 12.6; of 700, 32/8 of
+// 128 41.3 -> 33.3; of 2048, 8/2 of 64 52.1 -> 46.1; 2 of 400, 12/4 of 32 23.6 -> 17.6; 8 of 512, 32/8 of 64 67.8 -> 59.2; 16 of 1024,
+// 16/16 of 64 219 -> 198; 8 of 1024, 32/8 of 256 no change.  (Sixteen blocks a cluster: one of 4096, 32/8 of 128 319 -> 325.)
+constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4, kOneCluster = 8;
 template <int LP, int NC, int CHUNKS>
 __host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (CHUNKS / NC); }
 
@@ -430,7 +456,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     __shared__ uint32_t red[2][kOneThreads / 32];
     pdl_wait();
     pdl_launch();
-    const int blk = (int)blockIdx.x;
+    const int blk = (int)blockIdx.x / a.cluster, rank = (int)blockIdx.x - blk * a.cluster;
     const PassUnit w = pass_locate(a, a.n, blk);
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
@@ -440,7 +466,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     const long long first = (long long)w.b * t.rows * t.heads + w.g * t.group;
     int place[U];
     {
-        int r = gi / t.group, i = gi - r * t.group;
+        int r = (rank * NG * U + gi) / t.group, i = rank * NG * U + gi - r * t.group;
         const int dr = NG / t.group, di = NG - dr * t.group;
 #pragma unroll
         for (int k = 0; k < U; ++k) {
@@ -476,9 +502,10 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     const uint32_t wa = __reduce_max_sync(0xffffffffu, __float_as_uint(amax)), wn = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));
     if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5] = wa, red[1][threadIdx.x >> 5] = wn;
     __syncthreads();
-    const uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kOneThreads / 32 - 1)]);
-    const uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kOneThreads / 32 - 1)]);
-    if (threadIdx.x == 0) {
+    uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kOneThreads / 32 - 1)]);
+    uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kOneThreads / 32 - 1)]);
+    if (a.cluster > 1) cluster_tops(a.cluster, top, dn);  // (whose end is waited for below)
+    if (threadIdx.x == 0 && rank == 0) {
         t.amax[w.bg] = top;
         if (t.nmax) t.nmax[w.bg] = dn;
         if (t.clear) t.clear[w.bg] = 0u;
@@ -493,6 +520,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
             if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, plane, x[k][c], m);
         }
     }
+    if (a.cluster > 1) cluster_wait();
 }
 
 // ---- host side --------------------------------------------------------------------------------------
@@ -523,16 +551,20 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
 inline void pass_fill(PassArgs &a, float *dst, long long n) {
     a.fill[a.n_fill] = reinterpret_cast<float4 *>(dst), a.fill_n4[a.n_fill++] = n / 4;
 }
-// Whether one launch takes the call: `units` units a (sequence, group) at most, nothing rotated, nothing but planes and maxima wanted.
-// (The line is drawn by the group's query rows, although the forward reads those itself.)
-inline bool pass_takes_one(const PassArgs &a, int units) {
-    if (a.q_units > units) return false;
+// The blocks that a (sequence, group) of the one-launch form needs at `units` units each; 0: the form does not take the call, because a tensor
+// is rotated, or more than planes and maxima are wanted.
+inline long long pass_one_blocks(const PassArgs &a, int units) {
+    long long most = 1;
     for (int i = 0; i < a.n; ++i) {
         const PassTensor &t = a.t[i];
-        if ((long long)t.rows * t.group > units || !t.part || t.delta || t.rope || t.qs) return false;
+        if (!t.part || t.delta || t.rope || t.qs) return 0;
+        const long long blocks = ((long long)t.rows * t.group + units - 1) / units;
+        if (blocks > most) most = blocks;
     }
-    return a.n_fill == 0;
+    return a.n_fill == 0 ? most : 0;
 }
+// Whether a single block does.  (The line is drawn by the group's query rows, although the forward reads those itself.)
+inline bool pass_takes_one(const PassArgs &a, int units) { return a.q_units <= units && pass_one_blocks(a, units) == 1; }
 inline int pass_sm_count() {
     const DeviceInfo *d = device_info();
     return d && d->sm_count > 0 ? d->sm_count : 148;
@@ -557,15 +589,18 @@ inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
     return in_use >= 0.4 || waves <= (groups ? 80. : 450.) * in_use * in_use;
 }
 template <int LP, int NC, int CHUNKS>
-inline int launch_pass_one(PassArgs &a, cudaStream_t stream) {
+inline int launch_pass_one(PassArgs &a, cudaStream_t stream, const char *name = "pass_one_kernel", int cluster = 1) {
     long long blocks = 0;
+    a.cluster = cluster;
     for (int i = 0; i < a.n; ++i) {
         PassTensor &t = a.t[i];
         t.slots = 1, t.first = (int)blocks;
         blocks += (long long)t.batch * (t.heads / t.group);
     }
-    if (blocks > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
-    return launch_pdl("pass_one_kernel", pass_one_kernel<LP, NC, CHUNKS>, dim3((unsigned)blocks), dim3(kOneThreads), 0, stream, a);
+    if (blocks * cluster > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
+    const auto kernel = pass_one_kernel<LP, NC, CHUNKS>;
+    const dim3 grid((unsigned)(blocks * cluster)), th(kOneThreads);
+    return cluster > 1 ? launch_pdl_cluster(name, kernel, grid, th, 0, stream, cluster, a) : launch_pdl(name, kernel, grid, th, 0, stream, a);
 }
 // Both launches (or the second alone, for zeros).  The tensors whose maxima are wanted come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
@@ -593,6 +628,11 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
         if (pass_takes_one(a, pass_one_units<LP, NC, kOneFew>())) return launch_pass_one<LP, NC, kOneFew>(a, stream);
         constexpr int most = pass_one_units<LP, NC, kOneMost>();
         if (pass_takes_one(a, most) && pass_one_pays(a, most, pass_sm_count())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
+        // (clusters go under the name of the second of the two launches, whose work they do)
+        long long c = pass_one_blocks(a, pass_one_units<LP, NC, kOneFew>());
+        if (c > 0 && c <= kOneCluster) return launch_pass_one<LP, NC, kOneFew>(a, stream, "pass_planes_kernel", (int)c);
+        c = pass_one_blocks(a, most);
+        if (c > 0 && c <= kOneCluster) return launch_pass_one<LP, NC, kOneMost>(a, stream, "pass_planes_kernel", (int)c);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;

@@ -237,6 +237,23 @@ struct PeerList {
     int n;
 };
 
+// ---- thread-block clusters ----------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();  // (.aligned: the whole warp together, also where what lies before it was a single thread's)
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A float of block `rank`'s shared memory, at the place that `addr` has in this block's.
+__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
+    float v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}\n"
+                 : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
