@@ -148,7 +148,7 @@ struct PassArgs {
     long long fill_n4[3];
     int fill_first[4];  // first block of each region; [n_fill]: one past the last
     int n, n_stats, n_fill, dim, pd;  // dim: columns of a head in the tensors; pd: in the planes (plane_dim)
-    int cluster;                      // of the one-launch form: blocks per (sequence, group)
+    int cluster, per;                 // of the one-launch forms: blocks per (sequence, group); units that a lane group of a backward's takes
     int q_units;                      // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
 };
 
@@ -523,6 +523,113 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     if (a.cluster > 1) cluster_wait();
 }
 
+// ---- the one launch of a small backward whose k and v were kept -------------------------------------------
+// dout's statistics and planes, q's row-scaled planes and the zeros.  A (sequence, group) is a cluster's, of at most eight blocks, which holds its
+// rows of dout in shared memory: they are read once, all copies under way together, beside the zeros; out passes by; the maxima are put
+// together through distributed shared memory; then the planes leave and q, fetched ahead, follows.  Bound by latency: a launch less in the
+// chain.  Us, forward and backward, two launches -> this: one of T 256, 4/2 heads of 32 51 -> 45; 4 of 256, 16/16 of 64 55 -> 44.6; 4 of 100,
+// 4/2 of 32 32 -> 29.5; 64 of 100, 8/2 of 64 82.6 -> 78.8; 16 of 512, 16/16 of 64 269 -> 263; 16 of 300, 32/8 of 32 205 -> 203.
+// Where a group is more than 160 KB its phases, one after the other, take longer than two launches do: one of 1000, 32/8 of 64 105 -> 111,
+// 8 of 512 207 -> 209; and so for wider heads: one of 150, 8/2 of 128 67 -> 68, 8 of 256, 32/8 of 128 182 -> 191.
+constexpr int kBackThreads = 512, kBackSteps = 20;  // 8 KB of dout a step
+template <int LP>
+__global__ void __launch_bounds__(kBackThreads, 2) pass_backward_kernel(const __grid_constant__ PassArgs a) {
+    constexpr int NG = kBackThreads / LP, S = kPassUnroll;
+    extern __shared__ __align__(16) float4 held[];  // [a.per][kBackThreads], a thread's own; then [a.per][NG] norms
+    __shared__ uint32_t red[2][kBackThreads / 32];
+    pdl_wait();
+    pdl_launch();
+    const PassTensor &t = a.t[0], &tq = a.t[1];
+    const int bg = (int)blockIdx.x / a.cluster, rank = (int)blockIdx.x - bg * a.cluster;
+    const int groups = t.heads / t.group, b = bg / groups, g = bg - b * groups, units = t.rows * t.group;
+    const int gi = threadIdx.x / LP, li = threadIdx.x % LP, n4 = a.dim >> 2;
+    const long long first = (long long)b * t.rows * t.heads + g * t.group, plane = (long long)t.batch * t.rows * t.heads * a.pd;
+    float *norms = reinterpret_cast<float *>(held + a.per * kBackThreads) + gi;
+    const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(held + threadIdx.x);
+    const int u0 = rank * a.per * NG + gi;
+    const auto place = [&](int k) -> long long {  // of the block's k-th unit of this lane group; -1: none
+        const int u = u0 + k * NG;
+        return k < a.per && u < units ? first + (u / t.group) * (t.heads - t.group) + u : -1;
+    };
+    for (int k = 0; k < a.per; ++k) {
+        const long long at = place(k);
+        const bool in = at >= 0 && li < n4;
+        copy16_async(slot0 + (uint32_t)(k * kBackThreads * 16), reinterpret_cast<const float4 *>(t.x) + (in ? at * n4 + li : 0), in);
+    }
+    copy_async_commit();
+    const auto load = [&](const float *x, int k0, float4 (&r)[S]) {
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const long long at = place(k0 + s);
+            r[s] = at >= 0 && li < n4 ? reinterpret_cast<const float4 *>(x)[at * n4 + li] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float4 r[S];
+    load(t.o, 0, r);
+    for (int f = 0; f < a.n_fill; ++f) {  // this block's share of the zeros
+        const long long n = (a.fill_n4[f] + gridDim.x - 1) / gridDim.x, i0 = n * blockIdx.x, i1 = i0 + n < a.fill_n4[f] ? i0 + n : a.fill_n4[f];
+        for (long long i = i0 + threadIdx.x; i < i1; i += kBackThreads) a.fill[f][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    copy_async_wait<0>();
+    float amax = 0.f, nmax = 0.f;
+    for (int k0 = 0; k0 < a.per; k0 += S) {
+        float sq[S], de[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            sq[s] = de[s] = 0.f;
+            if (k0 + s >= a.per) continue;
+            const float4 x = held[(k0 + s) * kBackThreads + threadIdx.x], o = r[s];
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+            sq[s] = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
+            de[s] = fmaf(x.x, o.x, fmaf(x.y, o.y, fmaf(x.z, o.z, x.w * o.w)));
+        }
+        if (k0 + S < a.per) load(t.o, k0 + S, r);
+        else load(tq.x, 0, r);  // (q's first rows, for behind the barrier)
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+#pragma unroll
+            for (int off = LP / 2; off > 0; off >>= 1) {
+                sq[s] += __shfl_xor_sync(0xffffffffu, sq[s], off);
+                de[s] += __shfl_xor_sync(0xffffffffu, de[s], off);
+            }
+            const float norm = sqrtf(sq[s]);
+            nmax = fmaxf(nmax, norm);
+            const long long at = place(k0 + s);
+            if (li == 0 && at >= 0) t.delta[at] = de[s], t.rnorm[at] = norm, norms[(k0 + s) * NG] = norm;
+        }
+    }
+    // (f32 bit patterns of non-negative numbers order like integers)
+    const uint32_t wa = __reduce_max_sync(0xffffffffu, __float_as_uint(amax)), wn = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));
+    if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5] = wa, red[1][threadIdx.x >> 5] = wn;
+    __syncthreads();
+    uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kBackThreads / 32 - 1)]);
+    uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kBackThreads / 32 - 1)]);
+    if (a.cluster > 1) cluster_tops(a.cluster, top, dn);  // (whose end is waited for below)
+    if (threadIdx.x == 0 && rank == 0) t.amax[bg] = top, t.nmax[bg] = dn;
+    const float m = block_mult(top), mq = block_mult(tq.amax[bg]);
+    const uint32_t vn = tq.vn_final[bg];
+    const bool in_planes = li * 4 < a.pd;
+    for (int k = 0; k < a.per; ++k) {
+        const long long at = place(k);
+        if (at >= 0 && in_planes) store_split4(t.planes + at * a.pd + li * 4, plane, held[k * kBackThreads + threadIdx.x], m);
+    }
+    for (int k0 = 0; k0 < a.per; k0 += S) {
+        float4 x[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s) x[s] = r[s];
+        if (k0 + S < a.per) load(tq.x, k0 + S, r);
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const long long at = place(k0 + s);
+            if (at < 0 || !in_planes) continue;
+            float cq, rel;
+            ds_row_scale(norms[(k0 + s) * NG], dn, vn, cq, rel);
+            store_split4(tq.qs + at * a.pd + li * 4, plane, x[s], mq * rel);
+        }
+    }
+    if (a.cluster > 1) cluster_wait();
+}
+
 // ---- host side --------------------------------------------------------------------------------------
 // Slots of one tensor of `bg` (sequence, group) pairs: what pass_slots() below can ask for.
 inline size_t pass_part_bytes(size_t bg) { return (bg > (size_t)kPassTargetBlocks ? bg : (size_t)kPassTargetBlocks) * sizeof(uint2); }
@@ -601,6 +708,26 @@ inline int launch_pass_one(PassArgs &a, cudaStream_t stream, const char *name = 
     const auto kernel = pass_one_kernel<LP, NC, CHUNKS>;
     const dim3 grid((unsigned)(blocks * cluster)), th(kOneThreads);
     return cluster > 1 ? launch_pdl_cluster(name, kernel, grid, th, 0, stream, cluster, a) : launch_pdl(name, kernel, grid, th, 0, stream, a);
+}
+// The one launch of a backward (dout in a.t[0], q in a.t[1]); -1: not taken, because more is wanted, the rows are too many or too wide, or out
+// starts on a 4-byte boundary.
+inline int launch_pass_backward_one(PassArgs &a, cudaStream_t stream) {
+    const PassTensor &t = a.t[0], &q = a.t[1];
+    if (a.n != 2 || a.pd > 64 || q.part || !q.qs || q.rope || !t.delta || !t.nmax || (reinterpret_cast<uintptr_t>(t.o) & 15u) != 0) return -1;
+    const int ng = kBackThreads / (a.pd <= 32 ? 8 : 16);
+    const long long bg = (long long)t.batch * (t.heads / t.group), steps = ((long long)t.rows * t.group + ng - 1) / ng;
+    if (steps > kBackSteps || bg * kOneCluster > 0x7fffffffLL) return -1;
+    // blocks of eight steps, or as many as give every SM one
+    long long c = (steps + 7) / 8, fill = (pass_sm_count() + bg - 1) / bg;
+    if (c < fill) c = fill;
+    if (c > steps) c = steps;
+    if (c > kOneCluster) c = kOneCluster;
+    a.cluster = (int)c, a.per = (int)((steps + c - 1) / c);
+    const size_t smem = (size_t)a.per * (kBackThreads * sizeof(float4) + ng * sizeof(float));
+    const auto kernel = a.pd <= 32 ? pass_backward_kernel<8> : pass_backward_kernel<16>;
+    if (optin_smem((const void *)kernel, smem)) return 1;
+    const dim3 grid((unsigned)(bg * c)), th(kBackThreads);
+    return c > 1 ? launch_pdl_cluster("pass_backward_kernel", kernel, grid, th, smem, stream, (int)c, a) : launch_pdl("pass_backward_kernel", kernel, grid, th, smem, stream, a);
 }
 // Both launches (or the second alone, for zeros).  The tensors whose maxima are wanted come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {

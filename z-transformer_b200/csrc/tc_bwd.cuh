@@ -1071,14 +1071,21 @@ inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs
         if (kept) t.vn_final = w.vnmax;
         else t.vn_part = a.t[3].part, t.vn_slots = a.t[3].slots;
     }
-    // (a caller's q may be where its gradient goes, as long as nothing is zeroed before q has been read)
-    const char *q0 = reinterpret_cast<const char *>(t.x), *q1 = q0 + (size_t)t.batch * t.rows * t.heads * a.dim * sizeof(float);
-    bool apart = true;
-    for (int f = 0; f < a.n_fill; ++f) {
-        const char *f0 = reinterpret_cast<const char *>(a.fill[f]);
-        apart = apart && (f0 >= q1 || f0 + a.fill_n4[f] * sizeof(float4) <= q0);
+    // (a caller's q may be where its gradient goes, as long as nothing is zeroed before q has been read; out may too, which the first of two
+    // launches has read)
+    const size_t bytes = (size_t)t.batch * t.rows * t.heads * a.dim * sizeof(float);
+    const auto apart = [&](const float *x) {
+        const char *x0 = reinterpret_cast<const char *>(x);
+        for (int f = 0; f < a.n_fill; ++f) {
+            const char *f0 = reinterpret_cast<const char *>(a.fill[f]);
+            if (f0 < x0 + bytes && f0 + a.fill_n4[f] * sizeof(float4) > x0) return false;
+        }
+        return true;
+    };
+    if (apart(t.x)) {
+        const int rc = kept && want_qs && apart(g.o) && apart(g.x) ? launch_pass_backward_one(a, stream) : -1;
+        return rc >= 0 ? rc : launch_pass(a, stream);
     }
-    if (apart) return launch_pass(a, stream);
     PassArgs zeros = a;
     a.n_fill = 0, zeros.n = 0;
     return launch_pass(a, stream) || launch_pass(zeros, stream);
