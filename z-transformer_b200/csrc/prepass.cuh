@@ -139,6 +139,7 @@ struct PassTensor {
     const uint32_t *vn_final;
     int dn_slots, vn_slots;
     int batch, rows, heads, group;  // heads per row, heads per group
+    uint32_t per_head;              // what a unit's index is divided by `group` with (pass_row)
     int slots;                      // blocks per (sequence, group)
     int first;                      // first block of this tensor
 };
@@ -152,6 +153,11 @@ struct PassArgs {
     int q_units;                      // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
 };
 
+// The row of a (sequence, group)'s unit u.  (A product with 2^32 / group rounded up, which is exact where pass_add has found it so: two divisions a
+// step were a fifth of the first launch's time: us, batch 8, T 4096, 32/8 heads of 128, 345 -> 279, the second launch 611 -> 556.)
+__device__ __forceinline__ int pass_row(const PassTensor &t, int u) {
+    return t.per_head ? (int)__umulhi((uint32_t)u, t.per_head) : t.group == 1 ? u : u / t.group;
+}
 struct PassUnit {  // where a block stands
     int z, bg, slot, b, g, units;
 };
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_stats_kernel(const __grid_c
     const int stride = t.slots * NG, n_steps = (w.units - w.slot * NG + stride - 1) / stride;
     const auto place = [&](int step) -> int {  // the unit's index within the (sequence, group), or -1
         const int u = step * stride + w.slot * NG + gi;
-        return u < w.units ? (u / group) * (heads - group) + u : -1;  // r heads + (u - r group)
+        return u < w.units ? pass_row(t, u) * (heads - group) + u : -1;  // r heads + (u - r group)
     };
     const auto fetch = [&](int step) {
         const int at = place(step);
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     const long long plane = (long long)t.batch * t.rows * t.heads * a.pd;
     const int n4 = a.dim >> 2;
     const auto locate = [&](int u, int &r) -> long long {
-        r = u / t.group;
+        r = pass_row(t, u);
         return u < w.units ? ((long long)w.b * t.rows + r) * t.heads + w.g * t.group + (u - r * t.group) : -1;
     };
     PassTops tops{};
@@ -549,7 +555,7 @@ __global__ void __launch_bounds__(kBackThreads, 2) pass_backward_kernel(const __
     const int u0 = rank * a.per * NG + gi;
     const auto place = [&](int k) -> long long {  // of the block's k-th unit of this lane group; -1: none
         const int u = u0 + k * NG;
-        return k < a.per && u < units ? first + (u / t.group) * (t.heads - t.group) + u : -1;
+        return k < a.per && u < units ? first + pass_row(t, u) * (t.heads - t.group) + u : -1;
     };
     for (int k = 0; k < a.per; ++k) {
         const long long at = place(k);
@@ -641,6 +647,8 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
     t = PassTensor{};
     t.x = x, t.batch = batch, t.rows = rows, t.heads = heads, t.group = group;
     t.part = part, t.amax = amax, t.nmax = nmax, t.planes = planes;
+    // (exact up to u with u times what the rounding up added, less than group, below 2^32; the last block's lanes look a step further)
+    if (group > 1 && ((unsigned long long)rows * group + (1u << 20)) * (unsigned)group < (1ull << 32)) t.per_head = (uint32_t)(((1ull << 32) + group - 1) / group);
     const long long bg = (long long)batch * (heads / group), units = (long long)rows * group;
     // 2048 blocks a tensor, 14 an SM (4096 and 1024 were 1-2 % slower, 512 more), of at least 256 units at 32 columns, 128 up
     // to 64 and 64 beyond: eight units a lane group where 32 lanes hold one, two at 80 and 96 columns and four at 192, whose
