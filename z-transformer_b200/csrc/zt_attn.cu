@@ -804,8 +804,7 @@ static int forward_rope_impl(const float *q, const float *k, const float *v, flo
     }
 #endif
     // off the fused path: rotate into the workspace, then the ordinary forward
-    if (launch_rope_apply(q, w.q_rot, w.table, batch, T, n_heads * dim, dim, false, s)) return 1;
-    if (launch_rope_apply(k, w.k_rot, w.table, batch, T, n_kv_heads * dim, dim, false, s)) return 1;
+    if (launch_rope_apply(q, w.q_rot, n_heads, k, w.k_rot, n_kv_heads, w.table, batch, T, dim, false, s)) return 1;
     return forward_impl(w.q_rot, w.k_rot, v, out, lse, batch, T, n_heads, n_kv_heads, dim, 0, T, s);
 }
 
@@ -851,8 +850,7 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
         return 1;
 #endif
     if (!fused) {
-        if (launch_rope_apply(q, w.q_rot, w.table, batch, T, n_heads * dim, dim, false, s)) return 1;
-        if (launch_rope_apply(k, w.k_rot, w.table, batch, T, n_kv_heads * dim, dim, false, s)) return 1;
+        if (launch_rope_apply(q, w.q_rot, n_heads, k, w.k_rot, n_kv_heads, w.table, batch, T, dim, false, s)) return 1;
         // (the wide heads take the unfused tensor-core form, which wants the inner workspace)
         const bool wide = dim > 128 || dim % 8 != 0;
         if (backward_impl(w.q_rot, w.k_rot, v, out, lse, delta, dout, dq, dk, dv, wide ? w.inner : nullptr,
@@ -861,8 +859,8 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
     }
     // the gradients of the unrotated q and k: R^T.  The tensor-core dQ kernel applies it as it writes dq; dk
     // (a quarter of dq's bytes here, flushed from its accumulator many times) takes a pass in place.
-    if (!dq_in_kernel && launch_rope_apply(dq, dq, w.table, batch, T, n_heads * dim, dim, true, s)) return 1;
-    return launch_rope_apply(dk, dk, w.table, batch, T, n_kv_heads * dim, dim, true, s);
+    if (dq_in_kernel) return launch_rope_single(dk, dk, w.table, batch, T, n_kv_heads * dim, dim, true, s);
+    return launch_rope_apply(dq, dq, n_heads, dk, dk, n_kv_heads, w.table, batch, T, dim, true, s);
 }
 
 // ---- the projection after attention: y = ctx . wo, and its gradients ------------------------------------------
