@@ -1,7 +1,9 @@
 // The pre-pass of the tensor-core kernels: f32 tensors -> f16 hi/lo operand planes with a power-of-two scale per
 // (sequence, group of heads), and beside them what the backward wants to know about the rows of dout.
 //
-// Two launches for all tensors of a call (one for a small forward: pass_one_kernel), both bound by HBM (or, for small calls, by launch latency):
+// A forward's are k and v (its kernels split the query rows themselves); a backward's dout and q, and k and v where the forward has not kept
+// them.  One launch where a block or a cluster holds a (sequence, group)'s rows (pass_one_kernel, pass_backward_kernel), else two for all
+// tensors of a call, bound by HBM (or, for small calls, by launch latency):
 //   pass_stats_kernel    reads every tensor once.  Per block: max |x| and, where asked, the largest row norm; per row of
 //                        dout its norm and delta = sum_j dout out.  A block leaves its two maxima in a slot of its own
 //                        (no atomics and nothing to clear beforehand).

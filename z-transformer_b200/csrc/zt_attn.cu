@@ -835,7 +835,8 @@ int zt_attn_backward_rope_batched(const float *q, const float *k, const float *v
         return refuse("token %llu is not the current one of this workspace for this shape, pos and theta: the planes "
                       "it stood for are gone (pass 0 to convert q, k, v again).", token);
     drop_kept_planes(w.inner);
-    if (launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
+    // (kept planes were made with the very table, which lies where the forward has left it)
+    if (!kept && launch_rope_table(w.table, w.table_t, T, dim, pos, theta, s)) return 1;
     bool fused = false, dq_in_kernel = false;
 #ifndef ZT_NO_TC
     const size_t least = backward_need(batch, T, n_heads, n_kv_heads, dim).least;
