@@ -10,7 +10,7 @@ def per_head(rows, group):
     return 0
 
 
-@pytest.mark.parametrize("group", [2, 3, 4, 5, 6, 7, 8, 12, 17, 31, 33, 64, 100, 511, 1000, 4093])
+@pytest.mark.parametrize("group", [2, 3, 4, 5, 6, 7, 8, 12, 17, 31, 33, 64, 100, 511, 1000, 2000])
 def test_rows_by_a_product(group):
     m = per_head(1, group)
     most = (1 << 32) // group - (1 << 20)  # units of the largest sequence that the rule admits
