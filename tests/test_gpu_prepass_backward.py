@@ -48,4 +48,5 @@ def test_one_launch(zt, B, T, H, G, D):
 
 def test_two_launches(zt):
     assert not step(zt, 1, 641, 2, 2, 64) and not step(zt, 1, 1281, 1, 1, 32) and not step(zt, 1, 70, 4, 2, 68)
+    assert not step(zt, 130, 257, 8, 8, 64)  # (two blocks for each of 1040 (sequence, group)s: more than dout's slots)
     assert not step(zt, 2, 90, 4, 2, 64, out_shift=1) and not step(zt, 2, 90, 4, 2, 64, out_is_dq=True)

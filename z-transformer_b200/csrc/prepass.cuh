@@ -420,25 +420,16 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
 }
 
-// A block's two maxima -> its cluster's.  Leaves the cluster's barrier arrived at, to be waited for at the end of the kernel: nobody's shared
-// memory may go away while others read it.  So the words read are stored again, behind which the block meets, before it arrives: a load whose
-// value nothing waits for could still be on its way when the block that it reads has left.
-__device__ __forceinline__ void cluster_tops(int cluster, uint32_t &top, uint32_t &norm) {
-    __shared__ float mine[2];
-    __shared__ uint32_t all[2];
-    if (threadIdx.x == 0) mine[0] = __uint_as_float(top), mine[1] = __uint_as_float(norm);
+// A block's two maxima -> its cluster's, through `slots` in global memory, one a block: behind the barrier nothing of a block is read by another, so
+// that each may leave when its own work is done.  (Through distributed shared memory, which holds every block until the others have read,
+// a suite of calls ended with an illegal address twice in some twenty runs, each time in a projection's pre-pass.)
+__device__ __forceinline__ void cluster_tops(uint2 *slots, int rank, int cluster, uint32_t &top, uint32_t &norm) {
+    if (threadIdx.x == 0) slots[rank] = make_uint2(top, norm);
     cluster_arrive();
     cluster_wait();
-    if (threadIdx.x < 32) {
-        const int from = (int)threadIdx.x < cluster ? (int)threadIdx.x : 0;
-        const uint32_t at = (uint32_t)__cvta_generic_to_shared(mine);
-        const uint32_t x = __reduce_max_sync(0xffffffffu, __float_as_uint(ld_cluster(at, from)));
-        const uint32_t y = __reduce_max_sync(0xffffffffu, __float_as_uint(ld_cluster(at + 4u, from)));
-        if (threadIdx.x == 0) all[0] = x, all[1] = y;
-    }
-    __syncthreads();
-    cluster_arrive();
-    top = all[0], norm = all[1];
+    const int lane = (int)threadIdx.x & 31;
+    const uint2 v = __ldcg(slots + (lane < cluster ? lane : 0));  // (from L2, where the others' words are)
+    top = __reduce_max_sync(0xffffffffu, v.x), norm = __reduce_max_sync(0xffffffffu, v.y);
 }
 
 // ---- the one launch of small forwards ---------------------------------------------------------------
@@ -450,8 +441,8 @@ __device__ __forceinline__ void cluster_tops(int cluster, uint32_t &top, uint32_
 // backward of 64 rows, 32/8 heads of 128, 70 -> 77.)
 // Two forms: of 16 float4 a thread, and of 4, with three blocks an SM: forward and backward of 7 sequences of 87, 16/16 heads of 32,
 // took 38.8 in two launches, 41.6 with the former alone, 36.3 with the latter.
-// A (sequence, group) of k or v that is more than a block's goes to a cluster of at most eight, which puts its maxima together through
-// distributed shared memory.  Us a forward, two launches -> a cluster a group: one of T 150, 8/2 heads of 128 17.5 -> 12.6; of 700, 32/8 of
+// A (sequence, group) of k or v that is more than a block's goes to a cluster of at most eight, which puts its maxima together behind
+// one barrier (cluster_tops).  Us a forward, two launches -> a cluster a group: one of T 150, 8/2 heads of 128 17.5 -> 12.6; of 700, 32/8 of
 // 128 41.3 -> 33.3; of 2048, 8/2 of 64 52.1 -> 46.1; 2 of 400, 12/4 of 32 23.6 -> 17.6; 8 of 512, 32/8 of 64 67.8 -> 59.2; 16 of 1024,
 // 16/16 of 64 219 -> 198; 8 of 1024, 32/8 of 256 no change.  (Sixteen blocks a cluster: one of 4096, 32/8 of 128 319 -> 325.)
 constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4, kOneCluster = 8;
@@ -512,7 +503,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     __syncthreads();
     uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kOneThreads / 32 - 1)]);
     uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kOneThreads / 32 - 1)]);
-    if (a.cluster > 1) cluster_tops(a.cluster, top, dn);  // (whose end is waited for below)
+    if (a.cluster > 1) cluster_tops(t.part + (long long)w.bg * a.cluster, rank, a.cluster, top, dn);
     if (threadIdx.x == 0 && rank == 0) {
         t.amax[w.bg] = top;
         if (t.nmax) t.nmax[w.bg] = dn;
@@ -528,13 +519,12 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
             if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, plane, x[k][c], m);
         }
     }
-    if (a.cluster > 1) cluster_wait();
 }
 
 // ---- the one launch of a small backward whose k and v were kept -------------------------------------------
 // dout's statistics and planes, q's row-scaled planes and the zeros.  A (sequence, group) is a cluster's, of at most eight blocks, which holds its
 // rows of dout in shared memory: they are read once, all copies under way together, beside the zeros; out passes by; the maxima are put
-// together through distributed shared memory; then the planes leave and q, fetched ahead, follows.  Bound by latency: a launch less in the
+// together behind a cluster's barrier; then the planes leave and q, fetched ahead, follows.  Bound by latency: a launch less in the
 // chain.  Us, forward and backward, two launches -> this: one of T 256, 4/2 heads of 32 51 -> 45; 4 of 256, 16/16 of 64 55 -> 44.6; 4 of 100,
 // 4/2 of 32 32 -> 29.5; 64 of 100, 8/2 of 64 82.6 -> 78.8; 16 of 512, 16/16 of 64 269 -> 263; 16 of 300, 32/8 of 32 205 -> 203.
 // Where a group is more than 160 KB its phases, one after the other, take longer than two launches do: one of 1000, 32/8 of 64 105 -> 111,
@@ -612,7 +602,7 @@ __global__ void __launch_bounds__(kBackThreads, 2) pass_backward_kernel(const __
     __syncthreads();
     uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kBackThreads / 32 - 1)]);
     uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kBackThreads / 32 - 1)]);
-    if (a.cluster > 1) cluster_tops(a.cluster, top, dn);  // (whose end is waited for below)
+    if (a.cluster > 1) cluster_tops(t.part + (long long)bg * a.cluster, rank, a.cluster, top, dn);
     if (threadIdx.x == 0 && rank == 0) t.amax[bg] = top, t.nmax[bg] = dn;
     const float m = block_mult(top), mq = block_mult(tq.amax[bg]);
     const uint32_t vn = tq.vn_final[bg];
@@ -635,7 +625,6 @@ __global__ void __launch_bounds__(kBackThreads, 2) pass_backward_kernel(const __
             store_split4(tq.qs + at * a.pd + li * 4, plane, x[s], mq * rel);
         }
     }
-    if (a.cluster > 1) cluster_wait();
 }
 
 // ---- host side --------------------------------------------------------------------------------------
@@ -723,15 +712,16 @@ inline int launch_pass_one(PassArgs &a, cudaStream_t stream, const char *name = 
 // starts on a 4-byte boundary.
 inline int launch_pass_backward_one(PassArgs &a, cudaStream_t stream) {
     const PassTensor &t = a.t[0], &q = a.t[1];
-    if (a.n != 2 || a.pd > 64 || q.part || !q.qs || q.rope || !t.delta || !t.nmax || (reinterpret_cast<uintptr_t>(t.o) & 15u) != 0) return -1;
+    if (a.n != 2 || a.pd > 64 || q.part || !q.qs || q.rope || !t.part || !t.delta || !t.nmax || (reinterpret_cast<uintptr_t>(t.o) & 15u) != 0) return -1;
     const int ng = kBackThreads / (a.pd <= 32 ? 8 : 16);
     const long long bg = (long long)t.batch * (t.heads / t.group), steps = ((long long)t.rows * t.group + ng - 1) / ng;
-    if (steps > kBackSteps || bg * kOneCluster > 0x7fffffffLL) return -1;
+    if (steps > kBackSteps) return -1;
     // blocks of eight steps, or as many as give every SM one
     long long c = (steps + 7) / 8, fill = (pass_sm_count() + bg - 1) / bg;
     if (c < fill) c = fill;
     if (c > steps) c = steps;
     if (c > kOneCluster) c = kOneCluster;
+    if (c > 1 && bg * c > kPassTargetBlocks) return -1;  // (the slots that dout has)
     a.cluster = (int)c, a.per = (int)((steps + c - 1) / c);
     const size_t smem = (size_t)a.per * (kBackThreads * sizeof(float4) + ng * sizeof(float));
     const auto kernel = a.pd <= 32 ? pass_backward_kernel<8> : pass_backward_kernel<16>;
@@ -765,11 +755,14 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
         if (pass_takes_one(a, pass_one_units<LP, NC, kOneFew>())) return launch_pass_one<LP, NC, kOneFew>(a, stream);
         constexpr int most = pass_one_units<LP, NC, kOneMost>();
         if (pass_takes_one(a, most) && pass_one_pays(a, most, pass_sm_count())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
-        // (clusters go under the name of the second of the two launches, whose work they do)
+        // (clusters go under the name of the second of the two launches, whose work they do; every block has a slot of its tensor's)
+        long long bg = 0;
+        for (int i = 0; i < a.n; ++i) bg = std::max(bg, (long long)a.t[i].batch * (a.t[i].heads / a.t[i].group));
+        const auto fits = [&](long long c) { return c > 0 && c <= kOneCluster && bg * c <= kPassTargetBlocks; };
         long long c = pass_one_blocks(a, pass_one_units<LP, NC, kOneFew>());
-        if (c > 0 && c <= kOneCluster) return launch_pass_one<LP, NC, kOneFew>(a, stream, "pass_planes_kernel", (int)c);
+        if (fits(c)) return launch_pass_one<LP, NC, kOneFew>(a, stream, "pass_planes_kernel", (int)c);
         c = pass_one_blocks(a, most);
-        if (c > 0 && c <= kOneCluster) return launch_pass_one<LP, NC, kOneMost>(a, stream, "pass_planes_kernel", (int)c);
+        if (fits(c)) return launch_pass_one<LP, NC, kOneMost>(a, stream, "pass_planes_kernel", (int)c);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
