@@ -50,7 +50,12 @@ def test_against_float64(zt, B, T, H, G, D, scale, spread):
         assert float((x.double() - r).norm()) <= 1e-5 * float(r.norm()), name  # (what the calls are measured to)
 
 
-@pytest.mark.parametrize("t,off,H,G,D", [(130, 1200, 3, 3, 64), (200, 2100, 8, 2, 128), (40, 1500, 2, 1, 256), (600, 1400, 32, 8, 64)])
+@pytest.mark.parametrize("t,off,H,G,D", [
+    (130, 1200, 3, 3, 64), (200, 2100, 8, 2, 128), (40, 1500, 2, 1, 256), (600, 1400, 32, 8, 64),
+    # as many tiles as no accumulator is flushed after, and one more: one head a block, two, wide heads; narrow ones; rows that are not a warp's
+    (519, 1529, 32, 32, 128), (519, 1530, 32, 32, 100), (1223, 313, 16, 16, 36), (1001, 1100, 16, 16, 60), (1025, 999, 32, 8, 100), (603, 421, 32, 32, 192),
+    (603, 422, 32, 32, 164),
+])
 def test_windows(zt, t, off, H, G, D):
     attn = zt.Attn(off + t, H, G, D)
     gen = torch.Generator(device="cuda")

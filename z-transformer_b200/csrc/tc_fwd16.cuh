@@ -60,7 +60,7 @@ struct Params {
     int parts;     // CTAs along a query tile's keys; with more than one, out and lse are the parts' (see tc_split.cuh):
     long long out_part, lse_part;  // elements from one part's to the next
     bool by_tile;  // (one head a block) blocks go through the sequences tile by tile, see tile_by_tile
-    bool flush;    // O leaves the tensor core's accumulator every kFlushKeyTiles key tiles (see flush_row)
+    bool flush;    // of a window whose accumulators take more than kFlushKeyTiles key tiles: O leaves them after every so many (see flush_row)
     int dim_out;  // the tensors' head_dim, at most the tile's D
     int ahead;    // attn_fwd_tc16 prefetches the query tile of the block this many places on in launch order; 0: none
     float scale_log2;
@@ -151,11 +151,27 @@ __device__ __forceinline__ float4 flush_sum4(const float *at, float f, bool firs
     o.x = fmaf(g.x, f, o.x), o.y = fmaf(g.y, f, o.y), o.z = fmaf(g.z, f, o.z), o.w = fmaf(g.w, f, o.w);
     return o;
 }
-// Where a row's running sum is kept, null when the row is not the tensor's; `width` columns of it (the rest are padding).
+// Where a row's running sum is kept, null when the row is not the tensor's; `width` columns of it (the rest are padding).  The sums are their
+// threads' own, so a warp's lie in its rows of the tensor as they come -- the lanes' first four columns, then their next four -- and an
+// instruction covers 512 bytes in a stretch or two.  (Each in its own row, an instruction touched 32 lines: 10000 clocks a flush and 17000 at a
+// block's end of 143000 in all, 512 rows at 3584 keys, 32/8 heads of 128.  Us, the kernel there 93.8 -> 86.4; 2000 rows at 8000, 8/2 heads of 128
+// 243 -> 200; in attn_fwd_tc16g 2048 at 2000, 32/8 of 128 297 -> 249.)
 struct FlushRow {
-    float *sums;
-    int width;
+    float *sums;  // the warp's first row
+    int width, stride, rows;  // columns of a row; from a row to the next; the warp's that are the tensor's
+    uint32_t per;             // 2^20 over the row's float4, rounded up: i, below 32 rows of at most 64, is divided by them exactly
+    __device__ __forceinline__ float *at(int col) const {
+        const int i = (col >> 2) * rows + (int)(threadIdx.x & 31), r = (int)(((uint32_t)i * per) >> 20);
+        return sums + (long long)r * stride + (i - r * (width >> 2)) * 4;
+    }
 };
+// For the warp whose rows of head h begin with t0, in `tensor` [B, T, H, dim_out].
+__device__ __forceinline__ FlushRow flush_row_at(const Params &p, float *tensor, int b, int t0, int h) {
+    const int rows = p.T - t0 < 32 ? p.T - t0 : 32;
+    FlushRow w{nullptr, p.dim_out, p.n_heads * p.dim_out, rows, (1u << 20) / (uint32_t)(p.dim_out >> 2) + 1u};
+    if ((int)(threadIdx.x & 31) < rows) w.sums = tensor + (((long long)b * p.T + t0) * p.n_heads + h) * p.dim_out;
+    return w;
+}
 // O's columns [0, D) of this thread's row, at TMEM `taddr`, into its running sum.
 template <int D>
 __device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, float f, bool first) {
@@ -168,7 +184,7 @@ __device__ __forceinline__ void flush_row(uint32_t taddr, const FlushRow &row, f
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
             if (c + i >= row.width) break;
-            float *at = row.sums + c + i;
+            float *at = row.at(c + i);
             *reinterpret_cast<float4 *>(at) = flush_sum4(at, f, first, make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])));
         }
     }
@@ -225,7 +241,10 @@ __device__ __forceinline__ void store_q_piece(uint8_t *tile, int row, int block,
 template <bool FLUSH>
 __device__ __forceinline__ void send_row(float *dst, const uint8_t *staged, int columns, bool wanted) {
     fence_async_smem();
-    if (FLUSH) asm volatile("fence.proxy.async.global;" ::: "memory");
+    if (FLUSH) {  // (the sums of the warp's rows lie in each other's)
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        __syncwarp();
+    }
     if (wanted && columns > 0) bulk_store(dst, staged, (uint32_t)columns * 4);
     tma_commit();
     tma_wait_read();
@@ -470,11 +489,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
         // where the sets keep flushed sums: set 0 in out, set 1 in rows of its own
-        FlushRow row0{nullptr, p.dim_out}, row1{nullptr, p.dim_out};
-        if (FLUSH && t < p.T) {
-            const long long at = (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out;
-            row0.sums = p.out + part * p.out_part + at;
-            row1.sums = p.parts > 1 ? row0.sums + p.parts * p.out_part : p.flush_rows + at;  // (parts': behind the parts' rows)
+        FlushRow row0{}, row1{};
+        if (FLUSH) {
+            float *rows = p.out + part * p.out_part;
+            row0 = flush_row_at(p, rows, b, t0 + (warp & 3) * 32, h);
+            row1 = flush_row_at(p, p.parts > 1 ? rows + p.parts * p.out_part : p.flush_rows, b, t0 + (warp & 3) * 32, h);  // (parts': behind the parts' rows)
         }
         for (int j = set; ok && j < n_tiles; j += 2) {
             if (!__all_sync(0xffffffffu, fwait(&sh->s_full[set], (uint32_t)((j >> 1) & 1), sh))) {
@@ -585,11 +604,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int i = 0; i < 32; i += 4) {
                     const int col = set * (D / 2) + c + i;
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add0 && col < row0.width) o4 = flush_sum4(row0.sums + col, g0, false, o4);
+                    if (add0 && col < row0.width) o4 = flush_sum4(row0.at(col), g0, false, o4);
                     o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
                         float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
-                        if (add1 && col < row1.width) x4 = flush_sum4(row1.sums + col, g1, false, x4);
+                        if (add1 && col < row1.width) x4 = flush_sum4(row1.at(col), g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     *reinterpret_cast<float4 *>(srow + col * 4) = o4;
@@ -598,6 +617,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (set == 0 && p.lse && t < p.T)
                 p.lse[part * p.lse_part + ((long long)b * p.T + t) * p.n_heads + h] = (mm + log2f(lsum) - 7.0f) * kLn2;
         }
+        if (FLUSH) asm volatile("bar.sync 1, 256;" ::: "memory");  // (either set has read sums out of the rows that the other sends to)
         if (plain) {
             const int c0 = set * (D / 2), mine = p.dim_out - c0 < D / 2 ? p.dim_out - c0 : D / 2;
             send_row<FLUSH>(p.out + part * p.out_part + (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out + c0, srow + c0 * 4, mine, ok && t < p.T);
@@ -734,7 +754,7 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     p.rope = rope, p.flush_rows = q_offset > 0 ? w.flush_rows : nullptr;
     p.out = out, p.lse = lse;
     p.batch = batch, p.T = T, p.n_heads = n_heads, p.n_kv_heads = n_kv_heads;
-    p.dim_out = dim, p.q_offset = q_offset, p.flush = q_offset > 0;
+    p.dim_out = dim, p.q_offset = q_offset;
     p.o_planes = out_planes, p.o_plane_stride = (long long)batch * T * n_heads * dim;
     if (out_peers) p.out_peers = *out_peers;
     p.scale_log2 = kLog2e / sqrtf((float)dim);
@@ -757,6 +777,10 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     // Up to 64 columns, with more than a CTA an SM: two an SM (attn_fwd_tc16n).  Below, one tile at a time, two softmax sets in turn are the
     // quicker.  (Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to.)
     const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
+    // An accumulator that takes no more than kFlushKeyTiles tiles is never flushed: the variant without, whose end has no sums to look for.  (A CTA of one head
+    // gives its tiles to two accumulators in turn up to 128 columns.)  Us, 100 rows at 1700 keys, 12/4 heads of 96 20.2 -> 19.6, 200 at 3000 29.9 -> 29.0.
+    const int tiles = (n_seen + 63) / 64, per = (tiles + p.parts - 1) / p.parts;
+    p.flush = q_offset > 0 && per > tcf16::kFlushKeyTiles * (td <= 128 && (narrow || !pairs) ? 2 : 1);
     int rc;
     if (narrow) rc = tcf16::launch_n(kmap, vmap, qmap, p, sms, stream);
     else if (td == 256) rc = tcf16::launch_x_d<256>(kmap, vmap, qmap, p, stream);

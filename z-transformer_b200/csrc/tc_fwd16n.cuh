@@ -216,7 +216,8 @@ __device__ __forceinline__ void fwd16n_block(const CUtensorMap &kmap, const CUte
         // of the tiles of either parity: the reference maximum, the sum, the reference maximum of what has been flushed, and where that is kept
         float m_of[2] = {-INFINITY, -INFINITY}, l_of[2] = {0.f, 0.f}, f_of[2] = {-INFINITY, -INFINITY};
         const long long row_at = (((long long)b * p.T + t) * p.n_heads + h) * p.dim_out;
-        const FlushRow row0{FLUSH && t < p.T ? p.out + row_at : nullptr, p.dim_out}, row1{FLUSH && t < p.T ? p.flush_rows + row_at : nullptr, p.dim_out};
+        FlushRow row0{}, row1{};
+        if (FLUSH) row0 = flush_row_at(p, p.out, b, t0 + warp * 32, h), row1 = flush_row_at(p, p.flush_rows, b, t0 + warp * 32, h);
         const auto softmax = [&](int j, auto parity) -> bool {
             constexpr int s = parity.value;
             float &m_ref = m_of[s], &l = l_of[s], &m_flushed = f_of[s];
@@ -310,11 +311,11 @@ __device__ __forceinline__ void fwd16n_block(const CUtensorMap &kmap, const CUte
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add0 && c + i < row0.width) o4 = flush_sum4(row0.sums + c + i, g0, false, o4);
+                    if (add0 && c + i < row0.width) o4 = flush_sum4(row0.at(c + i), g0, false, o4);
                     o4.x *= f0, o4.y *= f0, o4.z *= f0, o4.w *= f0;
                     if (two && w1 != 0.f) {
                         float4 x4 = make_float4(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1]), __uint_as_float(rb[i + 2]), __uint_as_float(rb[i + 3]));
-                        if (add1 && c + i < row1.width) x4 = flush_sum4(row1.sums + c + i, g1, false, x4);
+                        if (add1 && c + i < row1.width) x4 = flush_sum4(row1.at(c + i), g1, false, x4);
                         o4.x += x4.x * f1, o4.y += x4.y * f1, o4.z += x4.z * f1, o4.w += x4.w * f1;
                     }
                     *reinterpret_cast<float4 *>(srow + (c + i) * 4) = o4;

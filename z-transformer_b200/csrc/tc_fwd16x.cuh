@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(kThreadsX, 1)
         const float cs = score_scale(p.scale_log2, block_mult(__float_as_uint(top)), mk);
         float m_ref = -INFINITY, l = 0.f;
         float m_flushed = -INFINITY;  // the reference maximum of what has been flushed
-        FlushRow row{nullptr, p.dim_out};
-        if (FLUSH && t < p.T) row.sums = p.out + part * p.out_part + ((long long)b * p.T + t) * p.n_heads * p.dim_out + (long long)h * p.dim_out;
+        FlushRow row{};
+        if (FLUSH) row = flush_row_at(p, p.out + part * p.out_part, b, t0 + warp * 32, h);
         for (int j = 0; ok && j < n_tiles; ++j) {
             if (!__all_sync(0xffffffffu, xwait(&sh->s_full[j & 1], (uint32_t)((j >> 1) & 1), sh))) {
                 xgive_up(sh, 65);
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kThreadsX, 1)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     float4 o4 = make_float4(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1]), __uint_as_float(ra[i + 2]), __uint_as_float(ra[i + 3]));
-                    if (add && c + i < row.width) o4 = flush_sum4(row.sums + c + i, ff, false, o4);
+                    if (add && c + i < row.width) o4 = flush_sum4(row.at(c + i), ff, false, o4);
                     o4.x *= inv, o4.y *= inv, o4.z *= inv, o4.w *= inv;
                     *reinterpret_cast<float4 *>(srow + (c + i) * 4) = o4;
                 }
