@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             for (int i = 0; i < NR; ++i) {
                 const int t = t0 + i * 32;
                 const long long idx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + head0 + walk.hh;
-                lse[i] = __ldg(p.lse + idx), rn[i] = __ldg(p.rnorm + idx), de[i] = __ldg(p.delta + idx);
+                lse[i] = __ldg(p.lse + idx), rn[i] = p.rnorm[idx], de[i] = p.delta[idx];  // (the sums may be the launch before's, pass_backward_kernel: plain loads)
             }
         };
         load();
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             float fq = 0.f;
             if (q32 < BQ && t0 + lane < p.T) {
                 float cq, rel;
-                ds_row_scale(__ldg(p.rnorm + ((long long)b * p.T + t0 + lane) * p.n_heads + head0 + walk.hh), rn_bits, vn_bits, cq, rel);
+                ds_row_scale(p.rnorm[((long long)b * p.T + t0 + lane) * p.n_heads + head0 + walk.hh], rn_bits, vn_bits, cq, rel);
                 fq = dq_unit / cq;
             }
             if (walk.flush) {
