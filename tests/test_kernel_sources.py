@@ -111,3 +111,18 @@ def test_tensor_memory_is_allocated_before_the_next_launch_is_let_in():
             if not body[m.end():end - 1].rstrip().endswith("return;") or end >= len(body):
                 assert re.search(r"tmem_alloc\(.*__syncthreads\(\);", body[:m.start()], re.S), (f, name)
     assert n == 11
+
+
+def test_rotated_query_rows_are_fenced_before_their_tile_is_copied_over():
+    """rotate_q writes the query tile by ordinary stores, and bulk copies land there once a_ready has completed: an mbarrier's arrival
+    orders no ordinary store before a bulk copy, so a proxy fence that runs wherever rows were rotated lies before it."""
+    n = 0
+    for name, text in sources().items():
+        for m in re.finditer(r"(?<!void )rotate_q\(", text):
+            n += 1
+            end = text.index("mbar_arrive_warp(&sh->a_ready", m.end())
+            if text.rfind("convert_q(uint8_t", 0, m.start()) > text.rfind("__global__", 0, m.start()):
+                end = text.index("\n}\n", m.end())  # (its callers arrive)
+            fences = re.findall(r"^ *(if \([^\n]*\) )?fence_async_smem\(\);", text[m.end():end], re.M)
+            assert any(f in ("", "if (LO_SMEM || angles) ") for f in fences), name
+    assert n == 3

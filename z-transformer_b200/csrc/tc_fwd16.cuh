@@ -277,7 +277,7 @@ __device__ __forceinline__ float convert_q(uint8_t *tile, int set, int row, cons
         else tmem_st16(lo + set * (D / 4) + cb * 16, ql);
     }
     tmem_wait_st();
-    if (LO_SMEM) fence_async_smem();
+    if (LO_SMEM || angles) fence_async_smem();  // (what was written over the tile, before the copies that land there next)
     tc_fence_before();
     return top;
 }
