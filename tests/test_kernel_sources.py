@@ -110,7 +110,11 @@ def test_tensor_memory_is_allocated_before_the_next_launch_is_let_in():
                 end += 1
             if not body[m.end():end - 1].rstrip().endswith("return;") or end >= len(body):
                 assert re.search(r"tmem_alloc\(.*__syncthreads\(\);", body[:m.start()], re.S), (f, name)
-    assert n == 11
+    assert n == 12
+    # no other kernel has tensor memory, and none takes it in a function that this does not look into
+    for name, text in sources().items():
+        inside = sum(body.count("tmem_alloc(") for f, _, _, body in kernels() if f == name)
+        assert text.count("tmem_alloc(") == inside + (name == "tc_common.cuh"), name
 
 
 def test_rotated_query_rows_are_fenced_before_their_tile_is_copied_over():

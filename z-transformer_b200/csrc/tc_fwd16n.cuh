@@ -43,9 +43,10 @@ __device__ __forceinline__ void ngive_up(SharedN *sh, int code) {
     atomicMax(&g_tc_status, code);
 }
 
-// A block's work.  (Every block of a launch has its tensor memory before it lets the next launch in, as in the other kernels.)
 template <bool FLUSH, bool PAD>
-__device__ __forceinline__ void fwd16n_block(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, const Params &p) {
+__global__ void __launch_bounds__(kThreadsN, 2)
+    attn_fwd_tc16n(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
+                   const __grid_constant__ CUtensorMap qmap, const Params p) {
     constexpr int D = 64, BN = 64;
     constexpr int KP = BN * D * 2;  // bytes of one plane of a key tile; a ring slot is 2 KP (hi, lo)
     constexpr int cO0 = 0, cS0 = 128;  // O of the tiles of parity s at cO0 + 64 s, S/P at cS0 + 64 s
@@ -341,13 +342,6 @@ __device__ __forceinline__ void fwd16n_block(const CUtensorMap &kmap, const CUte
     tc_fence_before();
     __syncthreads();
     if (warp == 5) tmem_dealloc(tmem, 256);
-}
-
-template <bool FLUSH, bool PAD>
-__global__ void __launch_bounds__(kThreadsN, 2)
-    attn_fwd_tc16n(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
-                   const __grid_constant__ CUtensorMap qmap, const __grid_constant__ Params p) {
-    fwd16n_block<FLUSH, PAD>(kmap, vmap, qmap, p);
 }
 
 inline int launch_n(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUtensorMap &qmap, Params p, int sms, cudaStream_t stream) {
