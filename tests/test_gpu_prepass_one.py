@@ -1,11 +1,13 @@
 """The one-launch pre-pass of small forwards at the sizes where its two forms begin and end (units of a sequence's group of heads:
 rows times heads): outputs against float64, and gradients from the planes it leaves.  Tolerances are those of the short forward's and
-the backwards' tests."""
+the backwards' tests.  Where pass_one_kernel ends, a form of pass_planes_kernel goes on that holds the rows in clusters of blocks, still
+in one launch; where that ends, pass_stats_kernel goes before pass_planes_kernel."""
 import pytest
 import torch
 
 from test_gpu_backward64 import gradients
 from test_gpu_forward_short import forward64
+from test_gpu_query_rows import bound
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +49,36 @@ def test_planes_of_small_forwards(zt, B, T, H, G, D, one):
 ])
 def test_planes_of_small_forwards_in_many_blocks(zt, B, T, H, G, D, one):
     test_planes_of_small_forwards(zt, B, T, H, G, D, one)
+
+
+ONE, HELD, TWO = {"pass_one_kernel"}, {"pass_planes_kernel"}, {"pass_stats_kernel", "pass_planes_kernel"}
+
+
+@pytest.mark.parametrize("B,T,H,G,D,launched", [
+    (1, 256, 4, 1, 32, ONE), (1, 257, 4, 1, 32, HELD), (1, 170, 6, 2, 60, ONE), (1, 171, 6, 2, 64, HELD), (1, 107, 3, 1, 80, HELD),
+    (1, 65, 4, 1, 128, HELD), (1, 54, 3, 1, 160, HELD), (64, 64, 16, 4, 64, HELD), (24, 33, 32, 4, 32, HELD),
+    # the clusters' sizes: eight blocks of 4 float4 a thread, three of 16, eight of these, and more
+    (1, 256, 1, 1, 256, HELD), (1, 257, 1, 1, 256, HELD), (1, 1024, 1, 1, 256, HELD), (1, 1025, 1, 1, 256, TWO),
+    (2, 1280, 1, 1, 160, HELD), (2, 1281, 1, 1, 160, TWO), (1, 2049, 1, 1, 128, TWO),
+    # and their slots, 2048 a tensor
+    (128, 129, 8, 8, 64, HELD), (150, 140, 16, 16, 64, TWO),
+])
+def test_the_launches_of_a_forwards_pre_pass(zt, B, T, H, G, D, launched):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(B + T)
+    q, k, v, do = (torch.randn((B, T, w * D), device="cuda", generator=gen) * c for w, c in zip((H, G, G, H), (1, 1, 1e3, 1e-3)))
+    ws = zt.BackwardWorkspace(B, T, H, G, D)
+    zt.lib.profile(True)
+    zt.lib.profile_read()
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+    names = {x for x in zt.lib.profile_read() if x.startswith("pass_")}
+    zt.lib.profile(False)
+    assert names == launched
+    got = zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=ws.token != 0)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+    ref, ref_lse = forward64(q, k, v, H, G, D, 0)
+    assert float((out.double() - ref).norm()) <= bound(D, T) * float(ref.norm())
+    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5
+    for name, x, r in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
+        assert float((x.double() - r).norm()) <= 1e-5 * float(r.norm()), name

@@ -45,7 +45,8 @@ def test_overlapped_kernels_read_their_predecessors_results_with_plain_loads():
             assert not re.search(r"__ldg\(p\.(?:delta|rnorm)", body), name
         if f == "prepass.cuh":
             assert "__ldg(p.rnorm" not in body and "__ldg(t.rnorm" not in body, name
-    # helpers of these kernels: V's planes come from the launch just before
+    # helpers of these kernels: V's planes come from the launch just before, and what a pre-pass of one launch reads may too
+    assert "__ldg" not in block(sources()["prepass.cuh"], sources()["prepass.cuh"].index("void pass_held("))
     assert "__ldg" not in block(sources()["tc_bwd.cuh"], sources()["tc_bwd.cuh"].index("void row_to_tmem16("))
 
 
@@ -130,3 +131,22 @@ def test_rotated_query_rows_are_fenced_before_their_tile_is_copied_over():
             fences = re.findall(r"^ *(if \([^\n]*\) )?fence_async_smem\(\);", text[m.end():end], re.M)
             assert any(f in ("", "if (LO_SMEM || angles) ") for f in fences), name
     assert n == 3
+
+
+def test_launches_go_under_their_kernels_names():
+    """What a launch is recorded as (profiles, error messages) is the name of the kernel that runs."""
+    n = 0
+    defined = {name for _, name, _, _ in kernels()}
+    for f, text in sources().items():
+        for m in re.finditer(r"\blaunch_(?:pdl|pdl_cluster|after|pass_held)\(\"(\w+)\", (\w+)", text):
+            n += 1
+            if m[2] in defined:
+                assert m[1] == m[2], (f, m[0])
+            else:  # a variable: every kernel it may be has that name
+                rest = text[m.end():].split("dim3")[0]
+                picked = re.findall(r"\w+(?=<)", rest) if rest.startswith(" ?") else re.findall(r"\b%s = ([^;]*);" % m[2], text)
+                assert picked and all(m[1] in x for x in picked), (f, m[0])
+        for m in re.finditer(r"ZT_LAUNCH\(\"(\w+)\", \w+,\s*\((\w+)", text):
+            n += 1
+            assert m[1] == m[2], (f, m[0])
+    assert n >= 20

@@ -2,8 +2,8 @@
 // (sequence, group of heads), and beside them what the backward wants to know about the rows of dout.
 //
 // A forward's are k and v (its kernels split the query rows themselves); a backward's dout and q, and k and v where the forward has not kept
-// them.  One launch where a block or a cluster holds a (sequence, group)'s rows (pass_one_kernel, pass_backward_kernel), else two for all
-// tensors of a call, bound by HBM (or, for small calls, by launch latency):
+// them.  One launch where a block or a cluster holds a (sequence, group)'s rows (pass_one_kernel, the forms of pass_planes_kernel that
+// hold them, pass_backward_kernel), else two for all tensors of a call, bound by HBM (or, for small calls, by launch latency):
 //   pass_stats_kernel    reads every tensor once.  Per block: max |x| and, where asked, the largest row norm; per row of
 //                        dout its norm and delta = sum_j dout out.  A block leaves its two maxima in a slot of its own
 //                        (no atomics and nothing to clear beforehand).
@@ -420,9 +420,14 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
 }
 
+// ---- the one launch of small forwards ---------------------------------------------------------------
+// Of the one-launch forms: threads of a block, float4 that a thread of either form holds, blocks of a cluster at most.
+constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4, kOneCluster = 8;
+template <int LP, int NC, int CHUNKS>
+__host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (CHUNKS / NC); }
+
 // A block's two maxima -> its cluster's, through `slots` in global memory, one a block: behind the barrier nothing of a block is read by another, so
-// that each may leave when its own work is done.  (Through distributed shared memory, which holds every block until the others have read,
-// a suite of calls ended with an illegal address twice in some twenty runs, each time in a projection's pre-pass.)
+// that each may leave when its own work is done.
 __device__ __forceinline__ void cluster_tops(uint2 *slots, int rank, int cluster, uint32_t &top, uint32_t &norm) {
     if (threadIdx.x == 0) slots[rank] = make_uint2(top, norm);
     cluster_arrive();
@@ -432,30 +437,13 @@ __device__ __forceinline__ void cluster_tops(uint2 *slots, int rank, int cluster
     top = __reduce_max_sync(0xffffffffu, v.x), norm = __reduce_max_sync(0xffffffffu, v.y);
 }
 
-// ---- the one launch of small forwards ---------------------------------------------------------------
-// Both launches in one, for forwards whose every (sequence, group) fits the registers of a block: 16 float4 a thread.  A block reads
-// its group's rows once, all loads under way together, knows the maxima after one barrier and writes the planes out of
-// registers: a launch less in a chain that is nothing but launches.  Us, forward of one sequence of 256, 16/16 heads of 64 20.7 -> 15.8, of
-// 12 of 128, 8/8 heads of 192 34.1 -> 20.6, forward and backward of one of 256, 4/2 heads of 32 44.1 -> 41.8.
-// (A backward's dout, whose block has out to read and q's planes to copy as well, took longer so than in two launches: forward and
-// backward of 64 rows, 32/8 heads of 128, 70 -> 77.)
-// Two forms: of 16 float4 a thread, and of 4, with three blocks an SM: forward and backward of 7 sequences of 87, 16/16 heads of 32,
-// took 38.8 in two launches, 41.6 with the former alone, 36.3 with the latter.
-// A (sequence, group) of k or v that is more than a block's goes to a cluster of at most eight, which puts its maxima together behind
-// one barrier (cluster_tops).  Us a forward, two launches -> a cluster a group: one of T 150, 8/2 heads of 128 17.5 -> 12.6; of 700, 32/8 of
-// 128 41.3 -> 33.3; of 2048, 8/2 of 64 52.1 -> 46.1; 2 of 400, 12/4 of 32 23.6 -> 17.6; 8 of 512, 32/8 of 64 67.8 -> 59.2; 16 of 1024,
-// 16/16 of 64 219 -> 198; 8 of 1024, 32/8 of 256 no change.  (Sixteen blocks a cluster: one of 4096, 32/8 of 128 319 -> 325.)
-constexpr int kOneThreads = 512, kOneMost = 16, kOneFew = 4, kOneCluster = 8;
+// The pre-pass of a (sequence, group) that a block, or a cluster of `cluster` blocks, holds in registers, CHUNKS float4 a thread: it reads the
+// group's rows once, all loads under way together, knows the maxima after one barrier and writes the planes out of registers.
+// `blk`: the block's, or its cluster's, place among the launch's.
 template <int LP, int NC, int CHUNKS>
-__host__ __device__ constexpr int pass_one_units() { return kOneThreads / LP * (CHUNKS / NC); }
-
-template <int LP, int NC, int CHUNKS>
-__global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_one_kernel(const __grid_constant__ PassArgs a) {
+__device__ __forceinline__ void pass_held(const PassArgs &a, int blk, int rank, int cluster) {
     constexpr int NG = kOneThreads / LP, U = CHUNKS / NC;
     __shared__ uint32_t red[2][kOneThreads / 32];
-    pdl_wait();
-    pdl_launch();
-    const int blk = (int)blockIdx.x / a.cluster, rank = (int)blockIdx.x - blk * a.cluster;
     const PassUnit w = pass_locate(a, a.n, blk);
     const PassTensor &t = a.t[w.z];
     const int gi = threadIdx.x / LP, li = threadIdx.x % LP;
@@ -503,7 +491,7 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
     __syncthreads();
     uint32_t top = __reduce_max_sync(0xffffffffu, red[0][threadIdx.x & (kOneThreads / 32 - 1)]);
     uint32_t dn = __reduce_max_sync(0xffffffffu, red[1][threadIdx.x & (kOneThreads / 32 - 1)]);
-    if (a.cluster > 1) cluster_tops(t.part + (long long)w.bg * a.cluster, rank, a.cluster, top, dn);
+    if (cluster > 1) cluster_tops(t.part + (long long)w.bg * cluster, rank, cluster, top, dn);
     if (threadIdx.x == 0 && rank == 0) {
         t.amax[w.bg] = top;
         if (t.nmax) t.nmax[w.bg] = dn;
@@ -519,6 +507,31 @@ __global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_o
             if (place[k] >= 0 && col < a.pd) store_split4(t.planes + at * a.pd + col, plane, x[k][c], m);
         }
     }
+}
+
+// Both launches in one, for forwards whose every (sequence, group) fits the registers of a block, 16 float4 a thread: a launch less in a chain
+// that is nothing but launches.  Us, forward of one sequence of 256, 16/16 heads of 64 20.7 -> 15.8, of 12 of 128, 8/8 heads of
+// 192 34.1 -> 20.6, forward and backward of one of 256, 4/2 heads of 32 44.1 -> 41.8.
+// Two forms: of 16 float4 a thread, and of 4, with three blocks an SM: forward and backward of 7 sequences of 87, 16/16 heads of 32,
+// took 38.8 in two launches, 41.6 with the former alone, 36.3 with the latter.
+template <int LP, int NC, int CHUNKS>
+__global__ void __launch_bounds__(kOneThreads, CHUNKS == kOneFew ? 3 : 1) pass_one_kernel(const __grid_constant__ PassArgs a) {
+    pdl_wait();
+    pdl_launch();
+    pass_held<LP, NC, CHUNKS>(a, (int)blockIdx.x, 0, 1);
+}
+
+// The planes without a first launch, where a cluster of up to eight blocks holds a (sequence, group)'s rows: k's and v's beyond what
+// pass_one_kernel takes.  Us a forward, two launches -> a cluster a group: one of T 150, 8/2 heads of 128 17.5 -> 12.6; of 700, 32/8 of
+// 128 41.3 -> 33.3; of 2048, 8/2 of 64 52.1 -> 46.1; 2 of 400, 12/4 of 32 23.6 -> 17.6; 8 of 512, 32/8 of 64 67.8 -> 59.2; 16 of 1024,
+// 16/16 of 64 219 -> 198; 8 of 1024, 32/8 of 256 no change; by single blocks, 64 of 64, 16/4 of 64 40.5 -> 34.9.  (Sixteen blocks a
+// cluster: one of 4096, 32/8 of 128 319 -> 325.)
+template <int LP, int NC, int HELD>
+__global__ void __launch_bounds__(kOneThreads, HELD == kOneFew ? 3 : 1) pass_planes_kernel(const __grid_constant__ PassArgs a) {
+    pdl_wait();
+    pdl_launch();
+    const int at = (int)blockIdx.x / a.cluster;
+    pass_held<LP, NC, HELD>(a, at, (int)blockIdx.x - at * a.cluster, a.cluster);
 }
 
 // ---- the one launch of a small backward whose k and v were kept -------------------------------------------
@@ -694,8 +707,9 @@ inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
     const double in_use = (double)held / ((double)blocks * units), waves = (double)blocks / sms;
     return in_use >= 0.4 || waves <= (groups ? 80. : 450.) * in_use * in_use;
 }
-template <int LP, int NC, int CHUNKS>
-inline int launch_pass_one(PassArgs &a, cudaStream_t stream, const char *name = "pass_one_kernel", int cluster = 1) {
+// Blocks that hold their (sequence, group)s' rows, `cluster` of them one.
+template <typename Kernel>
+inline int launch_pass_held(const char *name, Kernel kernel, PassArgs &a, int cluster, cudaStream_t stream) {
     long long blocks = 0;
     a.cluster = cluster;
     for (int i = 0; i < a.n; ++i) {
@@ -704,7 +718,6 @@ inline int launch_pass_one(PassArgs &a, cudaStream_t stream, const char *name = 
         blocks += (long long)t.batch * (t.heads / t.group);
     }
     if (blocks * cluster > 0x7fffffffLL) return refuse("the operand planes of this shape need more blocks than a launch can have.");
-    const auto kernel = pass_one_kernel<LP, NC, CHUNKS>;
     const dim3 grid((unsigned)(blocks * cluster)), th(kOneThreads);
     return cluster > 1 ? launch_pdl_cluster(name, kernel, grid, th, 0, stream, cluster, a) : launch_pdl(name, kernel, grid, th, 0, stream, a);
 }
@@ -752,17 +765,17 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
     // lanes x chunks of four columns that a unit takes: the tightest that holds it
     const auto both = [&](auto lanes, auto chunks) -> int {
         constexpr int LP = lanes.value, NC = chunks.value;
-        if (pass_takes_one(a, pass_one_units<LP, NC, kOneFew>())) return launch_pass_one<LP, NC, kOneFew>(a, stream);
-        constexpr int most = pass_one_units<LP, NC, kOneMost>();
-        if (pass_takes_one(a, most) && pass_one_pays(a, most, pass_sm_count())) return launch_pass_one<LP, NC, kOneMost>(a, stream);
-        // (clusters go under the name of the second of the two launches, whose work they do; every block has a slot of its tensor's)
+        constexpr int few = pass_one_units<LP, NC, kOneFew>(), most = pass_one_units<LP, NC, kOneMost>();
+        if (pass_takes_one(a, few)) return launch_pass_held("pass_one_kernel", pass_one_kernel<LP, NC, kOneFew>, a, 1, stream);
+        if (pass_takes_one(a, most) && pass_one_pays(a, most, pass_sm_count())) return launch_pass_held("pass_one_kernel", pass_one_kernel<LP, NC, kOneMost>, a, 1, stream);
+        // (every block of a cluster has a slot of its tensor's)
         long long bg = 0;
         for (int i = 0; i < a.n; ++i) bg = std::max(bg, (long long)a.t[i].batch * (a.t[i].heads / a.t[i].group));
         const auto fits = [&](long long c) { return c > 0 && c <= kOneCluster && bg * c <= kPassTargetBlocks; };
-        long long c = pass_one_blocks(a, pass_one_units<LP, NC, kOneFew>());
-        if (fits(c)) return launch_pass_one<LP, NC, kOneFew>(a, stream, "pass_planes_kernel", (int)c);
+        long long c = pass_one_blocks(a, few);
+        if (fits(c)) return launch_pass_held("pass_planes_kernel", pass_planes_kernel<LP, NC, kOneFew>, a, (int)c, stream);
         c = pass_one_blocks(a, most);
-        if (fits(c)) return launch_pass_one<LP, NC, kOneMost>(a, stream, "pass_planes_kernel", (int)c);
+        if (fits(c)) return launch_pass_held("pass_planes_kernel", pass_planes_kernel<LP, NC, kOneMost>, a, (int)c, stream);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;

@@ -114,7 +114,7 @@ inline int launch_rope_apply(const float *q, float *q_out, int n_heads, const fl
     const auto blocks = [&](int heads) { return (int)(((long long)heads * (head_dim / 8) + 255) / 256); };
     if (head_dim % 8 == 0 && (all & 15u) == 0 && blocks(n_heads) + blocks(n_kv_heads) <= 65535) {
         const RopeTensor a{q, q_out, n_heads, blocks(n_heads)}, b{k, k_out, n_kv_heads, blocks(n_kv_heads)};
-        return ZT_LAUNCH("rope_apply_kernel", stream,
+        return ZT_LAUNCH("rope_apply4_kernel", stream,
                          (rope_apply4_kernel<<<dim3((unsigned)(batch * rows), (unsigned)(a.blocks + b.blocks)), 256, 0, stream>>>(
                              a, b, table, rows, head_dim / 2, transpose ? 1 : 0)));
     }
