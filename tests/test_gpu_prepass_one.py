@@ -61,7 +61,7 @@ ONE, HELD, TWO = {"pass_one_kernel"}, {"pass_planes_kernel"}, {"pass_stats_kerne
     (1, 256, 1, 1, 256, HELD), (1, 257, 1, 1, 256, HELD), (1, 1024, 1, 1, 256, HELD), (1, 1025, 1, 1, 256, TWO),
     (2, 1280, 1, 1, 160, HELD), (2, 1281, 1, 1, 160, TWO), (1, 2049, 1, 1, 128, TWO),
     # and their slots, 2048 a tensor
-    (128, 129, 8, 8, 64, HELD), (150, 140, 16, 16, 64, TWO),
+    (128, 129, 32, 8, 64, HELD), (150, 140, 16, 16, 64, TWO),
 ])
 def test_the_launches_of_a_forwards_pre_pass(zt, B, T, H, G, D, launched):
     gen = torch.Generator(device="cuda")
@@ -82,3 +82,24 @@ def test_the_launches_of_a_forwards_pre_pass(zt, B, T, H, G, D, launched):
     assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5
     for name, x, r in zip(("dq", "dk", "dv"), got, gradients(q, k, v, do, H, G, D)):
         assert float((x.double() - r).norm()) <= 1e-5 * float(r.norm()), name
+
+
+@pytest.mark.parametrize("B,T,k,n,launched", [
+    (1, 128, 128, 128, ONE), (1, 600, 64, 576, HELD), (3, 600, 64, 576, HELD), (1, 4096, 64, 4096, HELD),
+    # two tensors that need different numbers of blocks: in the form of 4 float4 a thread, and in that of 16 too
+    (1, 641, 64, 576, HELD), (1, 1300, 128, 1088, TWO), (12, 300, 512, 64, TWO),
+])
+def test_a_projections_pre_pass(zt, B, T, k, n, launched):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(B + T)
+    ctx, w = torch.randn((B, T, k), device="cuda", generator=gen) * 1e2, torch.randn((k, n), device="cuda", generator=gen) * 1e-2
+    zt.lib.profile(True)
+    zt.lib.profile_read()
+    y = zt.proj_forward(ctx, w)
+    torch.cuda.synchronize()
+    names = {x for x in zt.lib.profile_read() if x.startswith("pass_")}
+    zt.lib.profile(False)
+    assert names == launched and zt.lib.tc_status() == 0
+    ref = ctx.double() @ w.double()
+    # two operands of 22 bits, and three truncated additions (half of 2^-23 on average) for every 16 of the contraction
+    assert float((y.double() - ref).norm()) <= (2 * 2.0 ** -22 + 3 * (k // 16) * 2.0 ** -24) * float(ref.norm())

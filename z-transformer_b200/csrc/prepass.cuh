@@ -670,17 +670,21 @@ inline PassTensor &pass_add(PassArgs &a, const float *x, int batch, int rows, in
 inline void pass_fill(PassArgs &a, float *dst, long long n) {
     a.fill[a.n_fill] = reinterpret_cast<float4 *>(dst), a.fill_n4[a.n_fill++] = n / 4;
 }
-// The blocks that a (sequence, group) of the one-launch form needs at `units` units each; 0: the form does not take the call, because a tensor
-// is rotated, or more than planes and maxima are wanted.
+// The blocks that a (sequence, group) of the one-launch forms needs at `units` units each; 0: the forms do not take the call, because a tensor
+// is rotated, or more than planes and maxima are wanted, or the tensors need different numbers of blocks.  A cluster has as many for one
+// tensor as for the other, so that some would have no unit, and no launch has such blocks: twice in some twenty runs of a suite of
+// calls an illegal address ended one of two projections whose clusters had them (the maxima met in distributed shared memory then).  No
+// cause has been found, in those blocks or elsewhere.
 inline long long pass_one_blocks(const PassArgs &a, int units) {
-    long long most = 1;
+    long long need = 0;
     for (int i = 0; i < a.n; ++i) {
         const PassTensor &t = a.t[i];
         if (!t.part || t.delta || t.rope || t.qs) return 0;
         const long long blocks = ((long long)t.rows * t.group + units - 1) / units;
-        if (blocks > most) most = blocks;
+        if (need && blocks != need) return 0;
+        need = blocks;
     }
-    return a.n_fill == 0 ? most : 0;
+    return a.n_fill == 0 ? need : 0;
 }
 // Whether a single block does.  (The line is drawn by the group's query rows, although the forward reads those itself.)
 inline bool pass_takes_one(const PassArgs &a, int units) { return a.q_units <= units && pass_one_blocks(a, units) == 1; }
@@ -721,6 +725,20 @@ inline int launch_pass_held(const char *name, Kernel kernel, PassArgs &a, int cl
     const dim3 grid((unsigned)(blocks * cluster)), th(kOneThreads);
     return cluster > 1 ? launch_pdl_cluster(name, kernel, grid, th, 0, stream, cluster, a) : launch_pdl(name, kernel, grid, th, 0, stream, a);
 }
+// Blocks of a (sequence, group) of `steps` steps in a backward's one launch, and the steps that each takes: eight steps a block, or as many blocks as
+// give every SM one.  Every block has a step.
+struct PassBackPlan {
+    int cluster, per;
+};
+inline PassBackPlan pass_backward_plan(long long steps, long long bg, int sms) {
+    long long c = (steps + 7) / 8;
+    const long long fill = (sms + bg - 1) / bg;
+    if (c < fill) c = fill;
+    if (c > steps) c = steps;
+    if (c > kOneCluster) c = kOneCluster;
+    const long long per = (steps + c - 1) / c;
+    return PassBackPlan{(int)((steps + per - 1) / per), (int)per};
+}
 // The one launch of a backward (dout in a.t[0], q in a.t[1]); -1: not taken, because more is wanted, the rows are too many or too wide, or out
 // starts on a 4-byte boundary.
 inline int launch_pass_backward_one(PassArgs &a, cudaStream_t stream) {
@@ -729,18 +747,15 @@ inline int launch_pass_backward_one(PassArgs &a, cudaStream_t stream) {
     const int ng = kBackThreads / (a.pd <= 32 ? 8 : 16);
     const long long bg = (long long)t.batch * (t.heads / t.group), steps = ((long long)t.rows * t.group + ng - 1) / ng;
     if (steps > kBackSteps) return -1;
-    // blocks of eight steps, or as many as give every SM one
-    long long c = (steps + 7) / 8, fill = (pass_sm_count() + bg - 1) / bg;
-    if (c < fill) c = fill;
-    if (c > steps) c = steps;
-    if (c > kOneCluster) c = kOneCluster;
-    if (c > 1 && bg * c > kPassTargetBlocks) return -1;  // (the slots that dout has)
-    a.cluster = (int)c, a.per = (int)((steps + c - 1) / c);
+    const PassBackPlan plan = pass_backward_plan(steps, bg, pass_sm_count());
+    if (plan.cluster > 1 && bg * plan.cluster > kPassTargetBlocks) return -1;  // (the slots that dout has)
+    const int c = a.cluster = plan.cluster;
+    a.per = plan.per;
     const size_t smem = (size_t)a.per * (kBackThreads * sizeof(float4) + ng * sizeof(float));
     const auto kernel = a.pd <= 32 ? pass_backward_kernel<8> : pass_backward_kernel<16>;
     if (optin_smem((const void *)kernel, smem)) return 1;
     const dim3 grid((unsigned)(bg * c)), th(kBackThreads);
-    return c > 1 ? launch_pdl_cluster("pass_backward_kernel", kernel, grid, th, smem, stream, (int)c, a) : launch_pdl("pass_backward_kernel", kernel, grid, th, smem, stream, a);
+    return c > 1 ? launch_pdl_cluster("pass_backward_kernel", kernel, grid, th, smem, stream, c, a) : launch_pdl("pass_backward_kernel", kernel, grid, th, smem, stream, a);
 }
 // Both launches (or the second alone, for zeros).  The tensors whose maxima are wanted come first in a.t.
 inline int launch_pass(PassArgs &a, cudaStream_t stream) {
