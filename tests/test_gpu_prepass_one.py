@@ -62,6 +62,8 @@ ONE, HELD, TWO = {"pass_one_kernel"}, {"pass_planes_kernel"}, {"pass_stats_kerne
     (2, 1280, 1, 1, 160, HELD), (2, 1281, 1, 1, 160, TWO), (1, 2049, 1, 1, 128, TWO),
     # and their slots, 2048 a tensor
     (128, 129, 32, 8, 64, HELD), (150, 140, 16, 16, 64, TWO),
+    # single blocks of 16 float4 a thread, where those of 4 have no slots: full enough or not
+    (65, 100, 16, 8, 256, HELD), (130, 45, 24, 8, 256, TWO), (128, 130, 16, 16, 64, TWO),
 ])
 def test_the_launches_of_a_forwards_pre_pass(zt, B, T, H, G, D, launched):
     gen = torch.Generator(device="cuda")

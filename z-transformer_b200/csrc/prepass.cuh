@@ -686,7 +686,8 @@ inline long long pass_one_blocks(const PassArgs &a, int units) {
     }
     return a.n_fill == 0 ? need : 0;
 }
-// Whether a single block does.  (The line is drawn by the group's query rows, although the forward reads those itself.)
+// Whether pass_one_kernel does.  (Its line is still the one drawn when the launch converted the query rows as well, which count although the
+// forward reads those itself, and so is pass_one_pays: beyond them the forms of pass_planes_kernel take over.)
 inline bool pass_takes_one(const PassArgs &a, int units) { return a.q_units <= units && pass_one_blocks(a, units) == 1; }
 inline int pass_sm_count() {
     const DeviceInfo *d = device_info();
@@ -710,6 +711,20 @@ inline bool pass_one_pays(const PassArgs &a, int units, int sms) {
     }
     const double in_use = (double)held / ((double)blocks * units), waves = (double)blocks / sms;
     return in_use >= 0.4 || waves <= (groups ? 80. : 450.) * in_use * in_use;
+}
+// The same of pass_planes_kernel's form of 16, for k and v alone (a cluster's blocks are two thirds full at least; a single block, which comes
+// here where two or more of 4 float4 would have too few slots, may be almost empty).  Us a forward, two launches / one, 16/16 heads, by the
+// room in use: of 64, 128 sequences, 0.25 217 / 270, 0.39 279 / 309, 0.50 314 / 332, 0.59 417 / 424, 0.78 589 / 566, 1 676 / 633; of 32, 0.50 528 /
+// 537, 0.68 833 / 810; of 128, 64 sequences, 0.39 136 / 149, 0.50 149 / 161, 0.70 239 / 235; where a unit is two or three chunks a
+// lane, earlier: of 96, 0.31 131 / 123; of 192, 0.25 115 / 123, 0.41 161 / 145; of 256, 0.31 134 / 142, 0.47 159 / 155.
+// (Few blocks: a launch less is all that counts.)
+inline bool pass_held_pays(const PassArgs &a, int units, long long cluster, int chunks, int sms) {
+    long long blocks = 0, held = 0;
+    for (int i = 0; i < a.n; ++i) {
+        const PassTensor &t = a.t[i];
+        blocks += (long long)t.batch * (t.heads / t.group) * cluster, held += (long long)t.batch * t.rows * t.heads;
+    }
+    return blocks <= sms || (double)held >= (chunks == 1 ? 0.64 : 0.4) * blocks * units;
 }
 // Blocks that hold their (sequence, group)s' rows, `cluster` of them one.
 template <typename Kernel>
@@ -790,7 +805,7 @@ inline int launch_pass(PassArgs &a, cudaStream_t stream) {
         long long c = pass_one_blocks(a, few);
         if (fits(c)) return launch_pass_held("pass_planes_kernel", pass_planes_kernel<LP, NC, kOneFew>, a, (int)c, stream);
         c = pass_one_blocks(a, most);
-        if (fits(c)) return launch_pass_held("pass_planes_kernel", pass_planes_kernel<LP, NC, kOneMost>, a, (int)c, stream);
+        if (fits(c) && pass_held_pays(a, most, c, NC, pass_sm_count())) return launch_pass_held("pass_planes_kernel", pass_planes_kernel<LP, NC, kOneMost>, a, (int)c, stream);
         const size_t smem = (size_t)kStatsStages * NC * 2 * kPassThreads * sizeof(float4);
         const auto stats_kernel = o4 ? pass_stats_kernel<LP, NC, true> : pass_stats_kernel<LP, NC, false>;
         if (optin_smem((const void *)stats_kernel, smem)) return 1;
