@@ -117,3 +117,21 @@ def test_rotated_rows_and_the_planes_of_out(zt, B, T, H, G, D):
     block = zt.AttentionBlock(B, T, H, G, D, 64)
     y, y2 = (block.forward(q, k, v, wo, fused=f) for f in (True, False))
     assert float((y - y2).abs().max()) <= 1e-6 * float(y2.abs().max())
+
+
+@pytest.mark.parametrize("B,T,H,G,D,kernel", [
+    # more than a block an SM and fewer than two: by the length; from two on whatever it is
+    (1, 1536, 16, 16, 64, "attn_fwd_tc16n"), (1, 1537, 16, 16, 64, "attn_fwd_tc16"), (1, 3001, 8, 2, 40, "attn_fwd_tc16"), (3, 1537, 8, 4, 64, "attn_fwd_tc16n"),
+])
+def test_long_sequences_in_few_blocks(zt, B, T, H, G, D, kernel):
+    q, k, v, _ = inputs(B, T, H, G, D, (1, 1, 1), 0)
+    zt.lib.profile(True)
+    zt.lib.profile_read()
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True)
+    torch.cuda.synchronize()
+    names = {x for x in zt.lib.profile_read() if x.startswith("attn_")}
+    zt.lib.profile(False)
+    assert names == {kernel} and zt.lib.tc_status() == 0
+    ref, ref_lse = forward64(q, k, v, H, G, D, 0)
+    assert float((out.double() - ref).norm()) <= bound(D, T) * float(ref.norm())
+    assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5

@@ -775,8 +775,14 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     const bool pairs = td <= 128 && group % 2 == 0 && (variant == 2 || (variant == 0 && pair_ctas >= sms));
     const long long blocks = (long long)((T + 127) / 128) * n_heads * batch;
     // Up to 64 columns, with more than a CTA an SM: two an SM (attn_fwd_tc16n).  Below, one tile at a time, two softmax sets in turn are the
-    // quicker.  (Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to.)
-    const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
+    // quicker; and up to two CTAs an SM, whose launch ends with its longest walk, for long sequences too.  Us, one head a CTA / two CTAs an
+    // SM: 160 CTAs, T 1000 26.4 / 23.8, 2000 192 CTAs 36.8 / 39.4, 3000 192 46.1 / 51.9, 288 53.6 / 57.3, 4500 288 75.6 / 91.1, 7000 220
+    // 91 / 123; T 1400 176 30.2 / 30.4, 264 36.5 / 33.7; T 700 288 30.8 / 23.2.  (A window's walks are all of a length: 1400 rows at 3000
+    // keys, 176 CTAs, 112.8 / 112.6.  Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to.  Us, two heads a
+    // CTA / two CTAs an SM: 1200 rows at 1100 keys, 32/8 heads of 64 85 / 78, 1500 at 2500, of 56 162 / 155, 1300 at 6000 309 / 304,
+    // 4000 at 4000, 16/4 287 / 306, 2200 at 9000, 32/8 503 / 531.)
+    const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset == 0 && blocks < 2LL * sms && T > 1536) &&
+                        !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
     // An accumulator that takes no more than kFlushKeyTiles tiles is never flushed: the variant without, whose end has no sums to look for.  (A CTA of one head
     // gives its tiles to two accumulators in turn up to 128 columns.)  Us, 100 rows at 1700 keys, 12/4 heads of 96 20.2 -> 19.6, 200 at 3000 29.9 -> 29.0.
     const int tiles = (n_seen + 63) / 64, per = (tiles + p.parts - 1) / p.parts;

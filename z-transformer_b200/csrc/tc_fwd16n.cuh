@@ -14,7 +14,7 @@
 // by half and more: T 512, 16/16 heads 6.2e-7 -> 8.6e-7, T 2000 1.25e-6 -> 2.2e-6.)
 // Us of the kernel, the forms before (one or two heads a CTA, whichever took the call) -> this: batch 8, T 512, 32/8 heads 64 -> 53; 2 of T
 // 3000, 16/16 heads 146 -> 103; 4 of 2000, 12/4 113 -> 76; 8 of 700, 12/4 54 -> 35; 64 of 256, 12/4 100 -> 72; 16 of 130, 16/16 of 32
-// columns 35 -> 21; one of 2048, 16/16 39.3 -> 42, the call 58 -> 52.  (Two heads a CTA, one CTA an SM, with two S buffers each and the next
+// columns 35 -> 21.  (Two heads a CTA, one CTA an SM, with two S buffers each and the next
 // tiles' rows split ahead: 64 -> 54, 146 -> 121, 113 -> 87.)
 #pragma once
 
