@@ -349,12 +349,14 @@ inline int launch_n(const CUtensorMap &kmap, const CUtensorMap &vmap, const CUte
     const auto kernel = with_flags([](auto flush, auto pad) { return attn_fwd_tc16n<flush.value, pad.value>; }, p.flush, head_steps(p.dim_out) < 4);
     if (optin_smem((const void *)kernel, smem)) return 1;
     const unsigned tiles = (unsigned)((p.T + 127) / 128), heads = (unsigned)p.n_heads, seqs = (unsigned)p.batch;
-    // Tile by tile up to four waves, where the tail counts, and to eight where the planes of k and v of all sequences stay in L2 (two halves of
-    // 63 MB), else sequence by sequence.  Us by tile / by sequence (with one accumulator): 16/16 heads, 2 of T 3000 (768 blocks) 93 / 110; 12/4, 4 of 2000
-    // (768) 70 / 81; 32/8, 8 of 1024 (2048 blocks, 34 MB) 110 / 124; 16/16 of 32 columns, 4 of 4096 (2048, 67 MB) 376 / 340; 32/8, 64 of
-    // 140 (4096) 144 / 129, 16 of 1024 (4096) 283 / 255, 8 of 4096 (8192) 1449 / 1397; few long ones lose a little, 2 of 8000 1308 / 1357.
+    // Tile by tile up to eight blocks an SM, where the tail counts, and beyond where the planes of k and v of all sequences stay in L2 (two
+    // halves of 63 MB), else sequence by sequence.  Us a forward, back to back for most of a second, by tile / by sequence: 16/16 heads, 2 of T
+    // 3000 (5 blocks an SM) 130 / 162; 12/4, 4 of 2000 (5) 89 / 108; 64 MB of planes: 32/8, 2 of 8192 (28) 1513 / 1567, 12/4, 16 of 2048 (21)
+    // 383 / 386, 32/8 of 32 columns, 100 of 300 (65) 356 / 382; 128 MB: 32/8, 8 of 4096 (55) 1742 / 1688, 16/4, 32 of 2048 (55) 1014 /
+    // 976, 16/16, 8 of 2048 (14) 329 / 319, 2 of 8000 (14) 841 / 867, 32/8, 64 of 512 (55) 456 / 468, one of 32768 11124 / 11117; 256 MB:
+    // 16/16 of 32 columns, 16 of 4096 (55) 1606 / 1431.
     const long long blocks = (long long)tiles * heads * seqs, kv = 8LL * p.batch * (p.q_offset + p.T) * p.n_kv_heads * plane_dim(p.dim_out);
-    p.by_tile = blocks <= 8LL * sms || (blocks <= 16LL * sms && kv <= (48LL << 20));
+    p.by_tile = blocks <= 8LL * sms || kv <= (64LL << 20);
     return launch_after("attn_fwd_tc16n", kernel, p.by_tile ? dim3(heads * seqs * tiles) : dim3(tiles, heads, seqs), dim3(kThreadsN), smem, stream, 2, kmap, vmap, qmap, p);
 }
 
