@@ -135,7 +135,8 @@ struct PassTensor {
     uint32_t *amax, *nmax;   // [batch * groups]: where the maxima are published; nmax null: not wanted
     uint32_t *clear;         // [batch * groups] words set to zero, or null
     const float2 *rope;      // null, or the (cos, sin) table [rows][dim / 2]: x is rotated on its way into the planes
-    // the planes with row t times rel(t) (ds_row_scale, from rnorm and the largest row norms of dout and v), or null
+    // the planes with row t times rel(t) (ds_row_scale, from rnorm and the largest row norms of dout and v), or null; together with `planes`
+    // above 128 columns only
     __half *qs;
     const uint2 *dn_part, *vn_part;  // dout's slots; v's, or null: v's norms are published already
     const uint32_t *vn_final;
@@ -320,7 +321,7 @@ __device__ __forceinline__ void pass_fill_block(const PassArgs &a, int blk) {
 
 // LP lanes hold a unit of the planes (pd columns), NC chunks of four columns each.
 template <int LP, int NC>
-__global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_constant__ PassArgs a) {
+__global__ void __launch_bounds__(kPassThreads, LP * NC > 32 ? 3 : 0) pass_planes_kernel(const __grid_constant__ PassArgs a) {
     constexpr int NG = kPassThreads / LP, U = (kPassUnroll + NC - 1) / NC;
     pdl_wait();
     pdl_launch();
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
     }
     const float m = block_mult(tops.amax);
     __half *const planes = t.qs ? t.qs : t.planes;
+    const bool both = LP * NC > 32 && t.qs && t.planes;  // (the wide heads' q)
     if (t.rope == nullptr) {
         for (; u0 < w.units;) {
 #pragma unroll
@@ -381,7 +383,9 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const long long to = at[k] * a.pd + (li + LP * c) * 4;
-                    if (at[k] >= 0 && (li + LP * c) * 4 < a.pd) store_split4(planes + to, plane, x[k][c], m * rel);
+                    if (at[k] < 0 || (li + LP * c) * 4 >= a.pd) continue;
+                    store_split4(planes + to, plane, x[k][c], m * rel);
+                    if (both) store_split4(t.planes + to, plane, x[k][c], m);
                 }
             }
             u0 += stride;
@@ -401,6 +405,7 @@ __global__ void __launch_bounds__(kPassThreads) pass_planes_kernel(const __grid_
             const float rel = t.qs ? row_rel(t.rnorm[at]) : 1.f;
             const auto put = [&](int col, float4 v) {
                 store_split4(planes + at * a.pd + col, plane, v, m * rel);
+                if (both) store_split4(t.planes + at * a.pd + col, plane, v, m);
             };
 #pragma unroll
             for (int c = 0; c < NC; ++c) {

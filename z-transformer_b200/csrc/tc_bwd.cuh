@@ -1027,7 +1027,7 @@ struct BwdWorkspace {
     uint32_t *amax_q, *amax_k, *amax_v, *amax_do, *vnmax, *dsmax;  // six [batch, n_kv_heads] arrays, in this order
     __half *q_planes, *do_planes, *k_planes, *v_planes;
     float *rnorm;  // [batch, T, n_heads]
-    __half *qs_planes;  // q's planes with their rows scaled: what the fused and the wide-head backward read (q_planes: the two kernels)
+    __half *qs_planes;  // q's planes with their rows scaled: for the fused backward and the wide heads' dK (q_planes: the wide heads' scores, the two kernels)
     uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
     // partial results of a split forward, then of a split backward (tc_split.cuh): behind everything else, so that a
     // workspace of base_bytes does for a call that is not split
@@ -1061,11 +1061,12 @@ inline BwdWorkspace bwd_workspace(void *base, int batch, int T, int n_heads, int
 }
 
 // The pre-pass of a backward: a.t[0] is dout, a.t[1] q, a.t[2] and a.t[3] k and v, unless the forward has kept the planes of
-// these two and the maxima of all three.  want_qs: q's planes have their rows scaled.
-inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs, bool kept, cudaStream_t stream) {
+// these two and the maxima of all three.  want_qs: q's planes with their rows scaled; want_q: q's planes as they are.
+inline int launch_pass_backward(PassArgs &a, const BwdWorkspace &w, bool want_qs, bool want_q, bool kept, cudaStream_t stream) {
     const PassTensor &g = a.t[0];
     PassTensor &t = a.t[1];
     if (kept) t.part = nullptr;
+    if (!want_q) t.planes = nullptr;
     if (want_qs) {
         t.qs = w.qs_planes, t.rnorm = w.rnorm, t.dn_part = g.part, t.dn_slots = g.slots;
         if (kept) t.vn_final = w.vnmax;

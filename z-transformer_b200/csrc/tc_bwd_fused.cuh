@@ -674,7 +674,7 @@ inline int launch_bwd_tc(const float *q, const float *k, const float *v, const f
         pass_add(pa, v, batch, T, n_kv_heads, 1, w.part[2], w.amax_v, w.vnmax, w.v_planes);
     }
     if (fused) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);
-    if (launch_pass_backward(pa, w, fused, qkv_planes_kept, stream)) return 1;
+    if (launch_pass_backward(pa, w, fused, !fused, qkv_planes_kept, stream)) return 1;
     const int rows = fused && td == 64 ? tcf::fused64_rows(T) : 64;  // of a query tile
     BwdMaps m;
     bool maps = make_head_map(&m.k128, w.k_planes, 2 * batch, T, n_kv_heads, dim, blocks, 128) &&

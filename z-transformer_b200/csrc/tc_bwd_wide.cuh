@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
         const long long ridx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + h;
         float cq = 1.f, rel = 1.f;
         if (t < p.T) ds_row_scale(__ldg(p.rnorm + ridx), p.rnmax[b * p.n_kv_heads + g], p.vnmax[b * p.n_kv_heads + g], cq, rel);
-        const float cs = p.scale_log2 / (mq * mk * rel);  // (Q's rows are scaled)
+        const float cs = p.scale_log2 / (mq * mk);
         // P leaves times p_scale: the factor rides in the exponent
         const float lse2 = (t < p.T) ? __ldg(p.lse + ridx) * kLog2e - log2f(p.p_scale) : 0.f;
         const float c1 = cq / (mdo * mv * p.p_scale);  // (P carries p_scale; dS must not)
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         const long long ridx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + h;
         float cq = 1.f, rel = 1.f;
         if (t < p.T) ds_row_scale(__ldg(p.rnorm + ridx), p.rnmax[bg], p.vnmax[bg], cq, rel);
-        const float cs = p.scale_log2 / (mq * mk * rel);  // (Q's rows are scaled)
+        const float cs = p.scale_log2 / (mq * mk);
         const float lse2 = (t < p.T) ? __ldg(p.lse + ridx) * kLog2e - log2f(p.p_scale) : 0.f;
         const float c1 = cq / (mdo * mv * p.p_scale);
         const float dels = (t < p.T && !ZT_DEFECT(13)) ? __ldg(p.delta + ridx) * cq / p.p_scale : 0.f;
@@ -905,12 +905,12 @@ inline int launch_bwd_wide(const float *q, const float *k, const float *v, const
     if (pieces > 1) pass_fill(pa, dq, (long long)batch * T * n_heads * dim);  // (a whole contraction's dQ is stored)
     pass_fill(pa, dk, (long long)batch * T * n_kv_heads * dim);
     pass_fill(pa, dv, (long long)batch * T * n_kv_heads * dim);
-    if (launch_pass_backward(pa, w, true, qkv_planes_kept, stream)) return 1;
+    if (launch_pass_backward(pa, w, true, true, qkv_planes_kept, stream)) return 1;
     const int Tp = ww.Tp, cap = ww.unit_cap;
     CUtensorMap q_k, k_k, g_k, v_k;      // K-major 128-row tiles of one 64-column block: the scores' operands
     CUtensorMap k_n, qs_n, g_n;          // N-major tiles (64 contraction rows x the head's 256 columns): B of the three products
     CUtensorMap ds_k, ds_m, p_m;         // the planes: K-major A (dQ), M-major A (dK, dV)
-    if (!make_half_tile_map(&q_k, w.qs_planes, 2 * batch, T, wq, 64, 128) ||
+    if (!make_half_tile_map(&q_k, w.q_planes, 2 * batch, T, wq, 64, 128) ||
         !make_half_tile_map(&k_k, w.k_planes, 2 * batch, T, wkv, 64, 128) ||
         !make_half_tile_map(&g_k, w.do_planes, 2 * batch, T, wq, 64, 128) ||
         !make_half_tile_map(&v_k, w.v_planes, 2 * batch, T, wkv, 64, 128) ||
