@@ -105,3 +105,36 @@ def test_a_projections_pre_pass(zt, B, T, k, n, launched):
     ref = ctx.double() @ w.double()
     # two operands of 22 bits, and three truncated additions (half of 2^-23 on average) for every 16 of the contraction
     assert float((y.double() - ref).norm()) <= (2 * 2.0 ** -22 + 3 * (k // 16) * 2.0 ** -24) * float(ref.norm())
+
+
+def test_clusters_in_a_captured_graph(zt):
+    """A step whose pre-passes are clusters, forward and backward, and a projection's, recorded once and replayed on other inputs."""
+    B, T, H, G, D = 2, 200, 6, 2, 64
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    q, k, v, do = (torch.randn((B, T, w * D), device="cuda", generator=gen) for w in (H, G, G, H))
+    ctx, w = torch.randn((1, 600, 64), device="cuda", generator=gen), torch.randn((64, 576), device="cuda", generator=gen)
+    ws, pws = zt.BackwardWorkspace(B, T, H, G, D), zt.ProjWorkspace(1, 600, 64, 576)
+
+    def step():
+        out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True, keep=ws)
+        return (out, lse, *zt.attention_backward(q, k, v, out, lse, do, H, G, D, workspace=ws, kept=True), zt.proj_forward(ctx, w, workspace=pws))
+
+    zt.lib.profile(True)
+    zt.lib.profile_read()
+    step()
+    names = {x for x in zt.lib.profile_read() if x.startswith("pass_")}
+    zt.lib.profile(False)
+    assert names == {"pass_planes_kernel", "pass_backward_kernel"}
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    for _ in range(2):
+        for x in (q, k, v, do, ctx, w):
+            x.normal_(generator=gen)
+        graph.replay()
+        got = [x.clone() for x in captured]
+        torch.cuda.synchronize()
+        assert zt.lib.tc_status() == 0 and zt.lib.tc_saturated() == 0
+        for a, b in zip(got, step()):  # (sums that are made in memory come in no fixed order)
+            assert float((a.double() - b.double()).norm()) <= 1e-6 * float(b.double().norm())

@@ -135,3 +135,34 @@ def test_long_sequences_in_few_blocks(zt, B, T, H, G, D, kernel):
     ref, ref_lse = forward64(q, k, v, H, G, D, 0)
     assert float((out.double() - ref).norm()) <= bound(D, T) * float(ref.norm())
     assert float((lse.double().view_as(ref_lse) - ref_lse).abs().max()) <= 2e-5
+
+
+@pytest.mark.parametrize("B,T,H,G,D", [
+    (1, 200, 4, 2, 128), (1, 140, 6, 2, 80), (1, 1100, 2, 1, 128),  # one head a block, split along the keys
+    (20, 200, 8, 2, 64), (24, 130, 12, 4, 40),                      # two blocks an SM
+    (13, 257, 8, 2, 128), (2, 131, 3, 1, 160), (1, 300, 2, 2, 256),  # two heads, wide heads
+])
+def test_rows_that_are_not_numbers(zt, B, T, H, G, D):
+    """A NaN or an infinity in one query row of one head makes that row's output NaN and changes no bit of any other: a row's scale is its own.
+    A NaN in a key's row reaches the queries that see the key, in its group's heads, and none before them."""
+    q, k, v, _ = inputs(B, T, H, G, D, (1, 1, 1), 0)
+    out, lse = zt.attention_forward(q, k, v, H, G, D, want_lse=True)
+    spoilt = q.clone()
+    spoilt[0, 70, 3] = float("nan")
+    spoilt[B - 1, T - 2, H * D - 1] = float("inf")
+    got, got_lse = zt.attention_forward(spoilt, k, v, H, G, D, want_lse=True)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0
+    hit = torch.zeros(B, T, H, dtype=torch.bool, device="cuda")
+    hit[0, 70, 0] = hit[B - 1, T - 2, H - 1] = True
+    rows, rows0 = got.view(B, T, H, D), out.view(B, T, H, D)
+    assert rows[hit].isnan().all() and torch.equal(rows[~hit], rows0[~hit])
+    assert torch.equal(got_lse.view(B, T, H)[~hit], lse.view(B, T, H)[~hit])
+    spoilt = k.clone()
+    spoilt[B - 1, 90, G * D - 2] = float("nan")
+    got = zt.attention_forward(q, spoilt, v, H, G, D).view(B, T, H, D)
+    torch.cuda.synchronize()
+    assert zt.lib.tc_status() == 0
+    hit.zero_()
+    hit[B - 1, 90:, H - H // G:] = True
+    assert got[hit].isnan().all() and torch.equal(got[~hit], rows0[~hit])

@@ -1,5 +1,5 @@
-"""What the one-launch pre-passes are planned to be (csrc/prepass.cuh, compiled here; without a device it takes a B200's 148 SMs): a cluster has a
-unit, or a step, for each of its blocks, whichever tensor they convert."""
+"""What the pre-passes' launches are planned to be (csrc/prepass.cuh, compiled here; without a device it takes a B200's 148 SMs): a cluster has a
+unit, or a step, for each of its blocks, whichever tensor they convert; a unit's row, where it is taken by a product, is the division's."""
 import os
 import shutil
 import subprocess
@@ -51,6 +51,36 @@ int main() {
 }
 """
 
+ROWS = r"""
+#include "prepass.cuh"
+using namespace zt::tcb;
+int main() {
+    long long products = 0, divisions = 0, bad = 0;
+    const int groups[] = {1, 2, 3, 4, 5, 6, 7, 8, 12, 17, 31, 33, 64, 100, 511, 1000, 2000, 65535};
+    for (int group : groups)
+        // up to the longest that units are counted of in 31 bits, on both sides of where the product ends
+        for (long long rows : {1ll, 2ll, 127ll, 1000ll, 65536ll, ((1ll << 32) / group - (1ll << 20)) / group - 1, ((1ll << 32) / group - (1ll << 20)) / group,
+                               ((1ll << 32) / group - (1ll << 20)) / group + 1, 0x7fffffffll / group}) {
+            if (rows < 1 || rows * group > 0x7fffffffll) continue;
+            PassArgs a{};
+            a.dim = a.pd = 32;
+            static uint2 part[1];
+            static uint32_t amax[1];
+            const PassTensor &t = pass_add(a, nullptr, 1, (int)rows, group, group, part, amax, nullptr, nullptr);
+            (t.per_head ? products : divisions) += 1;
+            // a block's lanes ask for units beyond the last, as far as a step of all blocks: those only have to be beyond it, too
+            const long long units = rows * group, step = (long long)t.slots * kPassThreads / 8 * kPassUnroll;
+            for (long long r : {0ll, 1ll, 2ll, rows / 3, rows / 2, rows - 2, rows - 1})
+                for (long long u : {r * group - 1, r * group, r * group + 1, r * group + group - 1})
+                    if (u >= 0 && u < units && pass_row(t, (int)u) != u / group && bad++ < 5) printf("%lld x %d: unit %lld\n", rows, group, u);
+            for (long long u : {units, units + 1, units + step - 1})
+                if (u <= 0x7fffffffll && pass_row(t, (int)u) < rows && bad++ < 5) printf("%lld x %d: unit %lld, beyond\n", rows, group, u);
+        }
+    printf("%lld products, %lld divisions, %lld bad\n", products, divisions, bad);
+    return bad > 0 || products < 40 || divisions < 10;
+}
+"""
+
 
 def run(tmp_path, program):
     src = tmp_path / "program.cu"
@@ -63,3 +93,7 @@ def run(tmp_path, program):
 
 def test_every_block_of_a_cluster_has_work(tmp_path):
     run(tmp_path, CLUSTERS)
+
+
+def test_a_units_row_is_the_divisions(tmp_path):
+    run(tmp_path, ROWS)

@@ -158,8 +158,8 @@ struct PassArgs {
 
 // The row of a (sequence, group)'s unit u.  (A product with 2^32 / group rounded up, which is exact where pass_add has found it so: two divisions a
 // step were a fifth of the first launch's time: us, batch 8, T 4096, 32/8 heads of 128, 345 -> 279, the second launch 611 -> 556.)
-__device__ __forceinline__ int pass_row(const PassTensor &t, int u) {
-    return t.per_head ? (int)__umulhi((uint32_t)u, t.per_head) : t.group == 1 ? u : u / t.group;
+__host__ __device__ __forceinline__ int pass_row(const PassTensor &t, int u) {
+    return t.per_head ? (int)(((unsigned long long)(uint32_t)u * t.per_head) >> 32) : t.group == 1 ? u : u / t.group;
 }
 struct PassUnit {  // where a block stands
     int z, bg, slot, b, g, units;
