@@ -3,8 +3,8 @@
 //
 // Written in Python the same work took 10-20 us a call (a torch.Size per shape compared, a device context, a ctypes call
 // of a dozen converted arguments), more than the kernels of a small step: a decode step of one sequence was 37 us of
-// host time over 20 us of kernels.  Here it is a few us plus the launches, of 2-3 us each: 2.7 us an append, 4.2 a short decode
-// step, 4.7 a forward of one launch, 8.7 of three (9.9 with scratch of its own), 13.1 a backward (one output to four allocated).
+// host time over 20 us of kernels.  Here it is a few us plus the launches: 2.7 us an append, 4.2 a short decode step, 6.0 a
+// forward of one launch, 6.5 of two (8.5 with its planes kept and the log-sum-exp), 13.4 a backward of three (one output to four allocated).
 //
 // Every function answers None when the arguments are not the plain case it handles (wrong shapes, types or devices
 // included) and False when the library refused the call; the Python caller then takes its own path, which raises the

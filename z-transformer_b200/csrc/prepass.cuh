@@ -11,12 +11,11 @@
 //                        the attention kernels, and writes the planes (rotating q and k on the way where rope is asked
 //                        for), the row-scaled copy of q's planes for dK, and the zeros of outputs that are summed in memory.
 // Both work on units, one head of one row, held by 8, 16 or 32 lanes.  A lane of the first launch has three units under way, of
-// the second four (two where it holds two or three chunks of one).  A block's units belong to one (sequence, group), of which its blocks take turns: blocks that run together read and write one stretch of memory, not a
-// stretch each (the first launch at T 4096, heads of 128: 460 us, with the turns 417).  The split into blocks is in pass_add.
-// Before (one kernel per quantity: two for the planes, one each for delta, v's norms, dout's norms, the row-scaled
-// copy, and up to four memsets; 13 launches a step where there are 6 now), us a step: batch 8, T 512, 32/8 heads of 64, forward
-// and backward, 175, now 106; T 1024, heads of 256, 740, now 582; T 4096, heads of 128, 1370, now 1310-1350 (all under the
-// step's clock, 1.5 GHz at the last).
+// the second four (two where it holds two or three chunks of one).  A block's units belong to one (sequence, group), of which its
+// blocks take turns: blocks that run together read and write one stretch of memory, not a stretch each (the first launch of a step at
+// T 4096, heads of 128, when it read q too: 460 us, with the turns 417).  The split into blocks is in pass_add.
+// Us of a step's pre-passes, forward and backward with k and v kept: batch 8, T 512, 32/8 heads of 64 66; T 1024, heads of 256,
+// 410 (its q goes into two pairs of planes); T 4096, heads of 128, 830 for 4.6 GB read and written, 700 at the copy rate.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -153,7 +152,7 @@ struct PassArgs {
     int fill_first[4];  // first block of each region; [n_fill]: one past the last
     int n, n_stats, n_fill, dim, pd;  // dim: columns of a head in the tensors; pd: in the planes (plane_dim)
     int cluster, per;                 // of the one-launch forms: blocks per (sequence, group); units that a lane group of a backward's takes
-    int q_units;                      // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
+    int q_units;  // of a forward: rows times heads of a (sequence, group)'s queries, which no launch here reads (see pass_takes_one)
 };
 
 // The row of a (sequence, group)'s unit u.  (A product with 2^32 / group rounded up, which is exact where pass_add has found it so: two divisions a

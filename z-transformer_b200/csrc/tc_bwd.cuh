@@ -1027,7 +1027,8 @@ struct BwdWorkspace {
     uint32_t *amax_q, *amax_k, *amax_v, *amax_do, *vnmax, *dsmax;  // six [batch, n_kv_heads] arrays, in this order
     __half *q_planes, *do_planes, *k_planes, *v_planes;
     float *rnorm;  // [batch, T, n_heads]
-    __half *qs_planes;  // q's planes with their rows scaled: for the fused backward and the wide heads' dK (q_planes: the wide heads' scores, the two kernels)
+    // q's planes with their rows scaled, for the fused backward and the wide heads' dK (q_planes: for the wide heads' scores and the two kernels)
+    __half *qs_planes;
     uint2 *part[4];     // the pre-pass's slots: q, k, v, dout
     // partial results of a split forward, then of a split backward (tc_split.cuh): behind everything else, so that a
     // workspace of base_bytes does for a call that is not split

@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(kFused64Threads, 1)
             for (int i = 0; i < NR; ++i) {
                 const int t = t0 + i * 32;
                 const long long idx = ((long long)b * p.T + (t < p.T ? t : 0)) * p.n_heads + head0 + walk.hh;
-                lse[i] = __ldg(p.lse + idx), rn[i] = p.rnorm[idx], de[i] = p.delta[idx];  // (the sums may be the launch before's, pass_backward_kernel: plain loads)
+                // (the row sums may be the launch before's, pass_backward_kernel's: plain loads)
+                lse[i] = __ldg(p.lse + idx), rn[i] = p.rnorm[idx], de[i] = p.delta[idx];
             }
         };
         load();

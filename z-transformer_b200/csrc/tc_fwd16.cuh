@@ -778,9 +778,9 @@ inline int launch_fwd_tc16(const float *q, const float *k, const float *v, float
     // quicker; and up to two CTAs an SM, whose launch ends with its longest walk, for long sequences too.  Us, one head a CTA / two CTAs an
     // SM: 160 CTAs, T 1000 26.4 / 23.8, 2000 192 CTAs 36.8 / 39.4, 3000 192 46.1 / 51.9, 288 53.6 / 57.3, 4500 288 75.6 / 91.1, 7000 220
     // 91 / 123; T 1400 176 30.2 / 30.4, 264 36.5 / 33.7; T 700 288 30.8 / 23.2.  (A window's walks are all of a length: 1400 rows at 3000
-    // keys, 176 CTAs, 112.8 / 112.6.  Windows of fewer than two waves of pairs stay with two heads a CTA, which a test holds them to.  Us, two heads a
-    // CTA / two CTAs an SM: 1200 rows at 1100 keys, 32/8 heads of 64 85 / 78, 1500 at 2500, of 56 162 / 155, 1300 at 6000 309 / 304,
-    // 4000 at 4000, 16/4 287 / 306, 2200 at 9000, 32/8 503 / 531.)
+    // keys, 176 CTAs, 112.8 / 112.6.)  Windows of fewer than two waves of pairs stay with two heads a CTA: neither is the quicker throughout.
+    // Us, two heads a CTA / two CTAs an SM: 1200 rows at 1100 keys, 32/8 heads of 64 85 / 78, 1500 at 2500, of 56 162 / 155, 1300 at
+    // 6000 309 / 304, 4000 at 4000, 16/4 287 / 306, 2200 at 9000, 32/8 503 / 531.  (The shortest lose by it; a test holds 1200 at 1100 there.)
     const bool narrow = td == 64 && variant == 0 && p.parts == 1 && blocks > sms && !(q_offset == 0 && blocks < 2LL * sms && T > 1536) &&
                         !(q_offset > 0 && pairs && pair_ctas < 2LL * sms);
     // An accumulator that takes no more than kFlushKeyTiles tiles is never flushed: the variant without, whose end has no sums to look for.  (A CTA of one head
